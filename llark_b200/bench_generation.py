@@ -236,7 +236,7 @@ def op_table(records, ctx, peaks):
             continue  # already inside `linear`
         ms = e0.elapsed_time(e1)
         if name == "linear":
-            name = "linear_rows" if shape[0] <= 8 and ops.linear_rows_pays(*shape) else "linear_tcgen05"
+            name = "linear_rows" if shape[0] <= ops.LINEAR_FEW_MAX else "linear_tcgen05"
         if name == "gemm":
             name = "gemm_tcgen05"
         d = agg.setdefault(name, {"calls": 0, "ms": 0.0, "bytes": 0, "flops": 0.0, "roof_ms": 0.0})

@@ -14,7 +14,7 @@
 // The smem ring has kStages stages of (A 16 KB + B 32 KB); the two TMEM accumulator stages let the MMA
 // of tile i+1 overlap the epilogue of tile i. Operands may be K-major or MN-major (dgrad/wgrad read the
 // weights / activations in place, no transposes), selected per operand through the UMMA descriptors.
-#include "common.cuh"
+#include "skinny.cuh"
 #include "../../include/llark_b200.h"
 #include <cuda.h>
 #include <mutex>
@@ -1254,6 +1254,27 @@ extern "C" int llark_gemm_ex(const void* A, int a_mn_major, long long lda, const
     const int vec = c_fp32 ? 4 : 8;
     if ((ldc % vec) != 0 || (reinterpret_cast<uintptr_t>(C) & 15) != 0) return LLARK_EINVAL;
     if (R && ((ldr % vec) != 0 || (reinterpret_cast<uintptr_t>(R) & 15) != 0)) return LLARK_EINVAL;
+
+    // Few rows: 256-row tiles would be mostly padding and, for the widths of one layer, occupy 16 to 86 of the 148 SMs; the
+    // product is a stream of B instead.
+    if (M <= skinny::kMaxRows && !a_mn_major && !b_mn_major && !in_fp32 && max_ctas == 0 &&
+        (!ep || ep->kind == LLARK_EPI_NONE || ep->kind == LLARK_EPI_ROPE) && skinny::fits(A, lda, B, ldb, K)) {
+        skinny::Args a = {};
+        a.A = (const __nv_bfloat16*)A, a.lda = lda, a.W = (const __nv_bfloat16*)B, a.ldw = ldb;
+        a.C = C, a.ldc = ldc, a.c_fp32 = c_fp32, a.bias = bias, a.bias_fp32 = bias_fp32, a.R = R, a.ldr = ldr;
+        a.M = M, a.N = N, a.K = K;
+        if (ep && ep->kind == LLARK_EPI_ROPE) {
+            a.act = skinny::kActRope;
+            a.rope_cos = (const __nv_bfloat16*)ep->a, a.rope_sin = (const __nv_bfloat16*)ep->b;
+            a.rope_S = ep->i0, a.rope_cols = ep->i1;
+        }
+        cudaError_t e = skinny::launch(a, stream);
+        if (e != cudaSuccess) {
+            g_last_cuda_error = (int)e;
+            return LLARK_ECUDA;
+        }
+        return LLARK_OK;
+    }
 
     static int dbg_split = -1;
     if (dbg_split < 0) {

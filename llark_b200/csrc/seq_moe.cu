@@ -21,7 +21,7 @@
 //   llark_seq_moe_up        act[pos] = silu(W_gate,e x) * (W_up,e x), or relu(W_up,e x)^2 for experts without a gate;
 //                           x = the entry's token row
 //   llark_seq_moe_down      z[pos]   = W_down,e act[pos]                 fp32
-#include "common.cuh"
+#include "skinny.cuh"
 
 namespace llark {
 extern thread_local int g_last_cuda_error;
@@ -587,9 +587,31 @@ static void launch_rows(const T* A, long long lda, const int* perm, int top, con
         grouped_rows_kernel<T, TC, MODE, 8><<<grid, 256, 0, st>>>(A, lda, perm, top, W, C, N, tiles, meta, N, K, vec_ok, up);
 }
 
+// bf16 rows in 16-byte pieces, whatever their number: the few-rows product of skinny.cu over the tile list
+static int launch_few(const void* A, long long lda, const int* perm, int top, const void* W, void* C, long long ldc, int c_fp32,
+                      const int* tiles, const int* meta, int max_tiles, int n_rows, int K, int mode, UpArgs up, cudaStream_t st) {
+    skinny::Args a = {};
+    a.A = (const bf16_t*)A, a.lda = lda, a.W = (const bf16_t*)W, a.ldw = K;
+    a.C = C, a.ldc = ldc, a.c_fp32 = c_fp32;
+    a.N = n_rows, a.K = K;
+    a.act = mode == kSiluGlu ? skinny::kActSiluGlu : mode == kClampGlu ? skinny::kActClampGlu
+            : mode == kRelu2 ? skinny::kActRelu2 : skinny::kActNone;
+    a.limit = up.limit, a.slope = up.slope, a.in_wts = up.in_wts;
+    a.tiles = tiles, a.meta = meta, a.max_tiles = max_tiles, a.perm = perm, a.top = top;
+    cudaError_t e = skinny::launch(a, st);
+    if (e != cudaSuccess) {
+        g_last_cuda_error = (int)e;
+        return LLARK_ECUDA;
+    }
+    return LLARK_OK;
+}
+
 template <typename T, int MODE>
 static int launch_up(const void* x, long long ldx, const int* perm, int top, const void* w, void* act, const int* tiles,
                      const int* meta, int max_tiles, int n_ent, int ff, int K, UpArgs up, cudaStream_t st) {
+    constexpr bool dual = MODE == kSiluGlu || MODE == kClampGlu;
+    if (sizeof(T) == 2 && skinny::fits(x, ldx, w, K, K))
+        return launch_few(x, ldx, perm, top, w, act, ff, 0, tiles, meta, max_tiles, dual ? 2 * ff : ff, K, MODE, up, st);
     if (n_ent <= kRowsRouteMaxEntries) {  // a handful of rows per expert: stream the weights once
         const int vec = 16 / (int)sizeof(T);
         const int vec_ok = (K % vec == 0) && (ldx % vec == 0) &&
@@ -621,6 +643,8 @@ extern "C" int llark_seq_moe_up(const void* x, long long ldx, const int* perm, i
 extern "C" int llark_seq_moe_down(const void* act, const void* w_down, float* z, const int* tiles, const int* meta,
                                   int max_tiles, int n_ent, int C, int ff, int act_fp32, cudaStream_t st) {
     if (max_tiles <= 0 || ff <= 0 || C <= 0 || !act || !w_down || !z || !tiles || !meta) return LLARK_EINVAL;
+    if (!act_fp32 && skinny::fits(act, ff, w_down, ff, ff))
+        return launch_few(act, ff, nullptr, 1, w_down, z, C, 1, tiles, meta, max_tiles, C, ff, kPlain, UpArgs{}, st);
     if (n_ent <= kRowsRouteMaxEntries) {
         const int esz = act_fp32 ? 4 : 2, vec = 16 / esz;
         const int vec_ok = (ff % vec == 0) &&

@@ -28,7 +28,7 @@
 //                           clamped gated unit)
 #include <initializer_list>
 
-#include "common.cuh"
+#include "skinny.cuh"
 
 namespace llark {
 extern thread_local int g_last_cuda_error;
@@ -1345,6 +1345,22 @@ extern "C" int llark_linear_rows(const void* A, long long lda, const void* W, lo
         return LLARK_EINVAL;
     if (in_fp32 && !c_fp32) return LLARK_EINVAL;
     const ActArg act{act_kind, act_limit, act_slope};
+    if (!in_fp32 && M <= skinny::kMaxRows && skinny::fits(A, lda, W, ldw, K)) {
+        skinny::Args a = {};
+        a.A = (const bf16_t*)A, a.lda = lda, a.W = (const bf16_t*)W, a.ldw = ldw;
+        a.C = C, a.ldc = ldc, a.c_fp32 = c_fp32, a.bias = bias, a.bias_fp32 = 1;
+        a.M = M, a.N = N, a.K = K;
+        a.act = act_kind == LLARK_ACT_RELU2 ? skinny::kActRelu2
+                : act_kind == LLARK_ACT_RELU_GLU ? skinny::kActReluGlu
+                : act_kind == LLARK_ACT_CLAMP_GLU ? skinny::kActClampGlu : skinny::kActNone;
+        a.limit = act_limit, a.slope = act_slope;
+        cudaError_t e = skinny::launch(a, st);
+        if (e != cudaSuccess) {
+            g_last_cuda_error = (int)e;
+            return LLARK_ECUDA;
+        }
+        return LLARK_OK;
+    }
     if (in_fp32)
         launch_rows<float, float>(A, lda, W, ldw, C, ldc, bias, M, N, K, act, st);
     else if (c_fp32)

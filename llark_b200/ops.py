@@ -481,19 +481,11 @@ def _actf(dtype):
     return int(dtype == torch.float32)
 
 
-# rows up to which a linear can be the weight-streaming kernel (the activations then sit in L1 / L2, the op is a pure read
-# of the weight matrix; linear_rows_pays says when it is); otherwise the tcgen05 GEMM core (bf16, at least one 64-wide tile in N and K, rows that TMA can
-# address) or the tiled SIMT kernel (fp32 mode, small or odd shapes)
+# rows up to which a linear is a stream of its weights (csrc/skinny.cu: bf16, 16-byte rows; up to LINEAR_ROWS_MAX also fp32 and
+# rows that are not); otherwise the tcgen05 GEMM core (bf16, at least one 64-wide tile in N and K, rows that TMA can address)
+# or the tiled SIMT kernel (fp32 mode, small or odd shapes)
 LINEAR_ROWS_MAX = 8
-
-
-def linear_rows_pays(M, N, K):
-    """Whether the weight-streaming kernel beats the tcgen05 core at M <= LINEAR_ROWS_MAX rows. Two rows ride on one read of a
-    weight; beyond that its FMAs grow with M N K, while the core takes a fixed time plus one that grows with K (measured on a
-    B200: rows 8 us + M N K / 4.1e6 us, core 16 us + K / 220 us, the launch included)."""
-    return M <= 2 or M * N * K < 32500000 + 18300 * K
-
-
+LINEAR_FEW_MAX = 64
 LINEAR_STATS = {"rows": 0, "tcgen05": 0, "simt": 0}
 LINEAR_ACTS = {None: 0, "relu2": 1, "relu_glu": 2, "clamp_glu": 3}
 PAIRED_ACTS = ("relu_glu", "clamp_glu")  # two columns of the product, a gate and its up column, make one of the result
@@ -523,7 +515,8 @@ def linear(a, w, bias=None, out_dtype=None, out=None, act=None, act_limit=0.0, a
     if bias is not None:
         _req(bias, torch.float32)
     vec = 4 if c_fp32 else 8
-    rows = M <= LINEAR_ROWS_MAX and (in_fp32 or linear_rows_pays(M, N, K))
+    rows = (M <= LINEAR_ROWS_MAX and in_fp32) or (M <= LINEAR_FEW_MAX and not in_fp32 and K % 8 == 0 and a.stride(0) % 8 == 0
+                                                  and w.stride(0) % 8 == 0 and (a.data_ptr() | w.data_ptr()) % 16 == 0)
     tc = (not rows and not in_fp32 and not (c_fp32 and paired) and K >= 64 and N >= 64 and K % 8 == 0 and a.stride(0) % 8 == 0
           and w.stride(0) % 8 == 0 and out.stride(0) % vec == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
           and out.data_ptr() % 16 == 0)

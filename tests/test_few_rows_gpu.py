@@ -1,0 +1,82 @@
+"""Products with few rows (csrc/skinny.cu) at the edges of their tiles: tokens 1 / 8 | 9 / 16 | 17 / 32 | 33 / 64 (the kernels' groups),
+weight rows that fill no tile, K of one slice, of a ragged last slice and of a cluster of eight, every epilogue, and the routed form
+with empty and full experts."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+BF16, F32, F64 = torch.bfloat16, torch.float32, torch.float64
+
+
+def _rel(a, b):
+    return ((a.to(F64) - b).norm() / b.norm()).item()
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("N,K", [(64, 64), (72, 136), (1000, 2048), (4096, 4096), (333, 8)])
+def test_products_and_epilogues(M, N, K):
+    from llark_b200 import ops
+
+    torch.manual_seed(M + N + K)
+    x, w = (torch.randn(M, K, device="cuda") * 0.5).to(BF16), (torch.randn(N, K, device="cuda") * 0.5).to(BF16)
+    b = torch.randn(N, device="cuda")
+    z = x.to(F64) @ w.to(F64).t()
+    # fp32 results: products of bf16 numbers are exact, so only the order and the cut of K fp32 additions shows: at most
+    # K * 2^-24 relative to the terms' norm, sqrt(K) of it in practice; the tensor cores' truncating adders measure 2e-6
+    assert _rel(ops.linear(x, w, bias=b, out_dtype=F32), z + b.to(F64)) < (5e-7 if M <= 8 else 5e-6)
+    # bf16 results: one rounding to eight bits, at most 2^-8 of a value
+    assert _rel(ops.linear(x, w, act="relu2"), torch.relu(z) ** 2) < 2.0 ** -8
+    assert ops.LINEAR_STATS["rows"] > 0
+    if N % 2 == 0:
+        v = z + b.to(F64)
+        assert _rel(ops.linear(x, w, bias=b, act="relu_glu"), torch.relu(v[:, 0::2]) * v[:, 1::2]) < 2.0 ** -8
+        g, u = z[:, 0::2].clamp(max=7.0), z[:, 1::2].clamp(-7.0, 7.0)
+        assert _rel(ops.linear(x, w, act="clamp_glu", act_limit=7.0), g * torch.sigmoid(1.702 * g) * (u + 1)) < 2.0 ** -8
+    if N % 8 == 0:
+        r = torch.randn(M, N, device="cuda").to(BF16)
+        assert _rel(ops.gemm(x, w, residual=r, bias=b.to(BF16)), z + r.to(F64) + b.to(BF16).to(F64)) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("M", [1, 5, 16, 33, 64])
+def test_rotation_in_the_epilogue_is_that_of_the_op(M):
+    from llark_b200 import ops
+
+    torch.manual_seed(M)
+    H, K = 512, 1024
+    x, w = (torch.randn(M, K, device="cuda") * 0.5).to(BF16), (torch.randn(3 * H, K, device="cuda") * 0.1).to(BF16)
+    cos, sin = torch.randn(16, 128, device="cuda").to(BF16), torch.randn(16, 128, device="cuda").to(BF16)
+    for S in (1, 7):
+        want = ops.gemm(x, w)
+        ops.rope_(want, cos, sin, S, H // 128, 128)  # rotates the q and the k heads of the packed projection
+        assert torch.equal(ops.gemm(x, w, rope=(cos, sin, S, 2 * H)), want)
+
+
+@pytest.mark.parametrize("T,C,ff,E,top,kind", [(1, 64, 64, 4, 2, "silu"), (9, 136, 72, 8, 3, "silu"), (70, 256, 128, 2, 1, "clamp"),
+                                                (33, 128, 200, 16, 4, "relu2"), (300, 512, 256, 8, 4, "silu")])
+def test_routed_experts(T, C, ff, E, top, kind):
+    from llark_b200 import ops
+
+    torch.manual_seed(T + C)
+    up = ff if kind == "relu2" else 2 * ff
+    wu, wd = torch.randn(E, up, C, device="cuda").mul(C ** -0.5).to(BF16), torch.randn(E, C, ff, device="cuda").mul(ff ** -0.5).to(BF16)
+    x = torch.randn(T, C, device="cuda").to(BF16)
+    hot = max(top, E // 2)  # the other experts get nothing
+    ids = torch.stack([torch.randperm(hot, device="cuda")[:top] for _ in range(T)]).to(torch.int32)
+    wts = torch.rand(T, top, device="cuda") if kind == "clamp" else None
+    z, pos = ops.seq_moe_experts(x, ids, wu, wd, gated=kind != "relu2", in_wts=wts, limit=7.0 if kind == "clamp" else None)
+    got = z[pos.long()].view(T, top, C)
+    want = torch.empty(T, top, C, device="cuda", dtype=F64)
+    for t in range(T):
+        for k in range(top):
+            e = int(ids[t, k])
+            u = wu[e].to(F64) @ x[t].to(F64)
+            if kind == "clamp":
+                u = u * wts[t, k].to(F64)
+                g, v = u[0::2].clamp(max=7.0), u[1::2].clamp(-7.0, 7.0)
+                h = g * torch.sigmoid(ops.GLU_SLOPE * g) * (v + 1)
+            elif kind == "silu":
+                h = torch.nn.functional.silu(u[:ff]) * u[ff:]
+            else:
+                h = torch.relu(u) ** 2
+            want[t, k] = wd[e].to(F64) @ h
+    assert _rel(got, want) < 2.0 ** -8  # the units are rounded to eight bits between the two products
