@@ -7,7 +7,7 @@ OBJ := $(patsubst llark_b200/csrc/%.cu,build/%.o,$(SRC))
 LIB := llark_b200/libllark_b200.so
 
 # the subset a native checkpoint of a layer-list decoder needs: GEMM core, decode linears, generation-path ops
-SERVE_OBJ := build/gemm_tcgen05.o build/gemv.o build/skinny.o build/seq_ops.o build/seq_mixers.o build/seq_swa_mma.o build/seq_delta.o \
+SERVE_OBJ := build/gemm_tcgen05.o build/gemv.o build/skinny.o build/attn_step.o build/seq_ops.o build/seq_mixers.o build/seq_swa_mma.o build/seq_delta.o \
              build/seq_latent.o build/seq_moe.o build/seq_decay.o
 LIB_SERVE := llark_b200/libllark_serve.so
 
@@ -19,6 +19,8 @@ build/%.o: llark_b200/csrc/%.cu llark_b200/csrc/common.cuh include/llark_b200.h
 	$(NVCC) $(NVFLAGS) -c $< -o $@ 2> build/$*.ptxas.log || (cat build/$*.ptxas.log; exit 1)
 
 build/skinny.o build/gemv.o build/gemm_tcgen05.o build/seq_ops.o build/seq_moe.o: llark_b200/csrc/skinny.cuh
+
+build/attn_step.o build/attention.o build/seq_mixers.o: llark_b200/csrc/attn_step.cuh
 
 # the ALiBi instantiation #includes the attention source: rebuild it when that changes
 build/attention_tc_alibi.o: llark_b200/csrc/attention_tc.cu

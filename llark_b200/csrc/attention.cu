@@ -8,7 +8,7 @@
 // online softmax in fp32, exp2 with pre-scaled log2e) that serve S > 4096 and `LLARK_ATTN_TC=0`, the dO.O row-sum
 // prep kernel of the backward pass, and the single-token decode kernel of the KV-cache path. The default path for
 // S <= 4096 is the tcgen05 / TMEM / TMA implementation in attention_tc.cu (same contract, same tests).
-#include "common.cuh"
+#include "attn_step.cuh"
 #include <stdlib.h>
 #include "../../include/llark_b200.h"
 
@@ -640,7 +640,20 @@ using namespace llark;
 extern "C" int llark_attn_decode(const void* q, const void* k_cache, const void* v_cache, const int* lens, void* out,
                                  int B, int s_max, int n_heads, int head_dim, float scale, cudaStream_t st) {
     if (head_dim != HD || B <= 0 || s_max <= 0 || s_max > DEC_MAX_LEN || n_heads <= 0 || !lens) return LLARK_EINVAL;
-    dim3 grid(n_heads, B);
+    if (attnstep::fits(B, n_heads, n_heads, HD, q, k_cache, v_cache)) {
+        attnstep::Args a = {};
+        a.q = (const __nv_bfloat16*)q, a.k = (const __nv_bfloat16*)k_cache, a.v = (const __nv_bfloat16*)v_cache;
+        a.out = (__nv_bfloat16*)out, a.out_ld = (long long)n_heads * HD;
+        a.B = B, a.H = a.G = n_heads, a.D = HD;
+        a.lens = lens, a.cap = s_max, a.scale = scale, a.out_scale = 1.f;
+        cudaError_t e = attnstep::launch(a, st);
+        if (e != cudaSuccess) {
+            g_last_cuda_error = (int)e;
+            return LLARK_ECUDA;
+        }
+        return LLARK_OK;
+    }
+    dim3 grid(n_heads, B);  // rows that are not on 16-byte boundaries
     attn_decode_kernel<<<grid, 128, 0, st>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k_cache,
                                              (const __nv_bfloat16*)v_cache, lens, (__nv_bfloat16*)out, s_max, n_heads,
                                              scale * LOG2E);

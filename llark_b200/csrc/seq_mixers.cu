@@ -18,7 +18,7 @@
 //                           f = low + (1 - low) * sigmoid(f_pre), q = silu(q_pre); fp32 state [slot, H, D, E]; long
 //                           prompts run as chunks in three passes (local states, llark_seq_glr_combine, outputs)
 //   llark_seq_head_rmsnorm  per-head RMS norm of the recurrence's output
-#include "common.cuh"
+#include "attn_step.cuh"
 
 namespace llark {
 extern thread_local int g_last_cuda_error;
@@ -1070,6 +1070,25 @@ extern "C" int llark_seq_swa_attn(const void* qn, const void* kn, const void* vv
         return LLARK_EINVAL;
     if (!from_ring_only && (!kn || !vv)) return LLARK_EINVAL;
     if ((size_t)(D + 8 * 32 + 16 + 9 * E) * sizeof(float) > 48 * 1024) return LLARK_EINVAL;
+    if (!act_fp32 && from_ring_only && D == E && attnstep::fits(n_tok, H, G, D, qn, kring, vring)) {
+        // decode steps read a key head's store once for all its query heads; the block-per-head kernel below is for steps that
+        // bring keys of their own, fp32 and other head sizes
+        attnstep::Args a = {};
+        a.q = (const bf16_t*)qn, a.k = (const bf16_t*)kring, a.v = (const bf16_t*)vring;
+        a.out = (bf16_t*)out, a.out_ld = out_ld;
+        a.B = n_tok, a.H = H, a.G = G, a.D = D;
+        a.tok_seq = tok_seq, a.cu = cu, a.pos0 = pos0, a.slot = slot;
+        a.cap = cap, a.window = window, a.chunk = chunk;
+        a.scale_h = scale_h, a.softcap = softcap, a.out_scale = out_scale;
+        a.sink = sink, a.gate = gate, a.gate_ld = gate_ld, a.gate_per_head = gate_per_head;
+        a.vfreq = vfreq, a.v_interleaved = v_interleaved;
+        cudaError_t e = attnstep::launch(a, st);
+        if (e != cudaSuccess) {
+            g_last_cuda_error = (int)e;
+            return LLARK_ECUDA;
+        }
+        return LLARK_OK;
+    }
     return act_fp32 ? launch_swa<float>(qn, kn, vv, kring, vring, gate, gate_ld, scale_h, out, tok_seq, cu, pos0, slot,
                                         n_tok, H, G, D, E, window, cap, from_ring_only, sink, gate_per_head, chunk,
                                         softcap, vfreq, v_interleaved, out_ld, out_scale, st)
