@@ -1,0 +1,511 @@
+// Matrix recurrences of prompts, 16 tokens at a time as products on the tensor cores. Per head and request S is [D, E] and
+//
+//     S_t = diag(d_t) S_(t-1) + p_t u_t^T,     o_t = S_t^T q_t,
+//
+// with u_t = v_t (HGRN2: d = f, p = 1 - f; state-space layers) or, for the gated delta rules, u_t = v_t - S_(t-1)^T z_t, z = d . k
+// and p = beta k. With b_t the product of d over the block's tokens up to t and w_s,t = p_s . d_(s+1) ... d_t (elementwise):
+//
+//     S_t^T x = S_0^T (b_t . x) + sum_(s <= t) (w_s,t x) u_s
+//
+// so a block of 16 tokens needs, beside S_0: Q' = b_t . q_t, Z' = b_(t-1) . z_t, the 16 x 16 matrices A[t, s] = w_s,t q_t (s <= t) and
+// L[t, s] = w_s,(t-1) z_t (s < t), P = w_s,15 and b_15. Every product of decays is taken as such, front to back (never as a quotient of
+// two of them), so nothing overflows however small a decay is. The correction u solves (1 + L) U = V - Z' S_0; with T = (1 + L)^-1,
+// Z = T Z', Q = Q' - A Z and A' = A T both the outputs and U are direct functions of S_0 and V:
+//
+//     O = Q S_0 + A' V,    U = T V - Z S_0,    S = diag(b_15) S_0 + P^T U.
+//
+//   chunk_prep_kernel   all of that which does not depend on S: a warp per block of tokens and head, every block at once, fp32
+//   chunk_scan_kernel   the walk over the blocks: a warp keeps 16 columns of S, transposed, in registers that are directly the A
+//                       operand of S^T Q^T. Every product as three TF32 products of split operands (x = hi + lo without lo lo:
+//                       2^-21 relative). The tensor cores cut their sums instead of rounding them, so chains are kept short (8
+//                       products) and a block's update of S starts from zero and is added with an FMA.
+//
+// The token-by-token kernels (seq_mixers.cu, seq_delta.cu) walk a chain of shared-memory reads and FMAs per token and stay for short
+// steps, other sizes and the general rule. What bounds this: the tensor cores' mma.sync rate on one chain of blocks per head and 16
+// columns. Measured on a B200: see the launchers.
+#include "common.cuh"
+
+namespace llark {
+extern thread_local int g_last_cuda_error;
+namespace chunk {
+
+constexpr int C = 16;  // tokens per block
+
+enum { kGlr = 0, kPaired = 1, kPlain = 2 };  // where q, d, p, z come from: HGRN2 columns; prepared vectors, with / without correction
+
+__host__ __device__ constexpr int block_floats(int D, bool correct) {  // Z | Q | P | b | T | A'
+    return (correct ? 3 : 2) * C * D + D + (correct ? 2 : 1) * C * C;
+}
+
+__device__ __forceinline__ float sigmoidf_(float z) { return 1.0f / (1.0f + expf(-z)); }
+
+template <int N> struct Vec { float v[N]; };
+template <int N> __device__ __forceinline__ Vec<N> ldv(const float* p) {
+    Vec<N> r;
+    if constexpr (N == 4) {
+        const float4 f = *reinterpret_cast<const float4*>(p);
+        r.v[0] = f.x, r.v[1] = f.y, r.v[2] = f.z, r.v[3] = f.w;
+    } else {
+        const float2 f = *reinterpret_cast<const float2*>(p);
+        r.v[0] = f.x, r.v[1] = f.y;
+    }
+    return r;
+}
+template <int N> __device__ __forceinline__ void stv(float* p, const Vec<N>& r) {
+    if constexpr (N == 4)
+        *reinterpret_cast<float4*>(p) = make_float4(r.v[0], r.v[1], r.v[2], r.v[3]);
+    else
+        *reinterpret_cast<float2*>(p) = make_float2(r.v[0], r.v[1]);
+}
+template <int N> __device__ __forceinline__ float dot(const Vec<N>& a, const Vec<N>& b) {
+    float s = a.v[0] * b.v[0];
+#pragma unroll
+    for (int i = 1; i < N; ++i) s = fmaf(a.v[i], b.v[i], s);
+    return s;
+}
+
+// 32 values per lane -> lane i holds the sum of value i over the lanes (31 shuffles)
+__device__ __forceinline__ float reduce32(float (&v)[32], int lane) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+            const bool up = lane & o;
+            const float send = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    return v[0];
+}
+
+struct PrepArgs {
+    const float* src;  // kGlr: columns of the fused projection; else the prepared vectors [n_tok, H, 5, D] = q, z, d, -p, p
+    long long ld;
+    int q_off, f_off;
+    const float* lower;
+    float* ws;         // [n_seq, chunks, H] blocks
+    const int* cu;
+    int H, c0, chunks;
+};
+
+template <int D, int MODE>
+__global__ void __launch_bounds__(128)
+chunk_prep_kernel(const PrepArgs p) {
+    constexpr int N = D / 32;
+    constexpr bool CORRECT = MODE == kPaired;
+    constexpr int kFlat = CORRECT ? 256 : 160;
+    __shared__ float flat_[4][kFlat], sT_[4][CORRECT ? C * C : 1];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int h = blockIdx.y * 4 + warp, b = blockIdx.z, c = p.c0 + blockIdx.x;
+    const int row_b = p.cu[b], left = p.cu[b + 1] - row_b - c * C;
+    if (h >= p.H || left <= 0) return;  // no barrier of the block below
+    const int cnt = left < C ? left : C;
+    const long long row0 = row_b + c * C;
+    float* flat = flat_[warp];
+    float* out = p.ws + (((long long)b * p.chunks + blockIdx.x) * p.H + h) * block_floats(D, CORRECT);
+    float* oZ = out;
+    float* oQ = out + (CORRECT ? C * D : 0);
+    float* oP = oQ + C * D;
+    float* oB = oP + C * D;
+    float* oT = oB + D;
+    float* oA = oT + (CORRECT ? C * C : 0);
+    const int d0 = lane * N;
+    Vec<N> low, cum, w[C], zb[CORRECT ? C : 1];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        cum.v[i] = 1.f;
+        low.v[i] = MODE == kGlr && p.lower ? p.lower[h * D + d0 + i] : 0.f;
+    }
+    float v[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = 0.f;
+    constexpr int G = 4;  // tokens whose rows are requested together
+#pragma unroll
+    for (int t0 = 0; t0 < C; t0 += G) {
+        Vec<N> q[G], d[G], pp[G], z[CORRECT ? G : 1];
+#pragma unroll
+        for (int i = 0; i < G; ++i) {
+            const int t = t0 + i;
+            if (t < cnt) {
+                if (MODE == kGlr) {
+                    const float* r = p.src + (row0 + t) * p.ld + (long long)h * D + d0;
+                    q[i] = ldv<N>(r + p.q_off);
+                    d[i] = ldv<N>(r + p.f_off);
+                } else {
+                    const float* r = p.src + ((row0 + t) * p.H + h) * 5 * D + d0;
+                    q[i] = ldv<N>(r);
+                    d[i] = ldv<N>(r + 2 * D);
+                    pp[i] = ldv<N>(r + 4 * D);
+                    if (CORRECT) z[CORRECT ? i : 0] = ldv<N>(r + D);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < G; ++i) {
+            const int t = t0 + i;
+#pragma unroll
+            for (int e = 0; e < N; ++e) {
+                if (t >= cnt) {  // nothing read, nothing written, nothing lost
+                    q[i].v[e] = pp[i].v[e] = 0.f;
+                    d[i].v[e] = 1.f;
+                    if (CORRECT) z[CORRECT ? i : 0].v[e] = 0.f;
+                } else if (MODE == kGlr) {
+                    const float x = q[i].v[e];
+                    q[i].v[e] = x * sigmoidf_(x);
+                    d[i].v[e] = low.v[e] + (1.0f - low.v[e]) * sigmoidf_(d[i].v[e]);
+                    pp[i].v[e] = 1.0f - d[i].v[e];
+                }
+            }
+            auto put = [&](int idx, float x) {
+                v[idx & 31] = x;
+                if ((idx & 31) == 31) flat[idx - 31 + lane] = reduce32(v, lane);
+            };
+            if (CORRECT) {
+#pragma unroll
+                for (int e = 0; e < N; ++e) zb[CORRECT ? t : 0].v[e] = z[CORRECT ? i : 0].v[e] * cum.v[e];
+#pragma unroll
+                for (int s = 0; s < t; ++s) put(t * t + s, dot(z[CORRECT ? i : 0], w[s]));  // L[t, s]
+            }
+#pragma unroll
+            for (int s = 0; s < t; ++s)
+#pragma unroll
+                for (int e = 0; e < N; ++e) w[s].v[e] *= d[i].v[e];
+            w[t] = pp[i];
+#pragma unroll
+            for (int s = 0; s <= t; ++s) put(CORRECT ? t * t + t + s : t * (t + 1) / 2 + s, dot(q[i], w[s]));  // A[t, s]
+            Vec<N> qb;
+#pragma unroll
+            for (int e = 0; e < N; ++e) {
+                cum.v[e] *= d[i].v[e];
+                qb.v[e] = q[i].v[e] * cum.v[e];
+            }
+            stv<N>(oQ + t * D + d0, qb);
+        }
+    }
+    if (!CORRECT) flat[128 + lane] = reduce32(v, lane);  // entries 128 .. 135, and left-overs behind them
+#pragma unroll
+    for (int s = 0; s < C; ++s) stv<N>(oP + s * D + d0, w[s]);
+    stv<N>(oB + d0, cum);
+    __syncwarp();
+    if (!CORRECT) {
+#pragma unroll
+        for (int i = 0; i < C * C; i += 32) {
+            const int t = (i + lane) >> 4, s = (i + lane) & 15;
+            oA[i + lane] = s <= t ? flat[t * (t + 1) / 2 + s] : 0.f;
+        }
+        return;
+    }
+    // ---- T = (1 + L)^-1 and A' = A T, a column per lane (both halves of the warp do the same)
+    float* sT = sT_[warp];
+    {
+        const int j = lane & 15;
+        float col[C];
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+            float a = 0.f;
+#pragma unroll
+            for (int k = 0; k < i; ++k) a = fmaf(flat[i * i + k], col[k], a);
+            col[i] = i == j ? 1.f : (i > j ? -a : 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+            float a = 0.f;
+#pragma unroll
+            for (int k = 0; k <= i; ++k) a = fmaf(flat[i * i + i + k], col[k], a);
+            if (lane < 16) {
+                sT[i * C + j] = col[i];
+                oT[i * C + j] = col[i];
+                oA[i * C + j] = a;
+            }
+        }
+    }
+    __syncwarp();
+    // ---- Z = T Z' (from the last token back, so that the rows it reads are still Z'), Q = Q' - A Z
+#pragma unroll
+    for (int t = C - 1; t > 0; --t)
+#pragma unroll
+        for (int s = 0; s < t; ++s) {
+            const float f = sT[t * C + s];
+#pragma unroll
+            for (int e = 0; e < N; ++e) zb[CORRECT ? t : 0].v[e] = fmaf(f, zb[CORRECT ? s : 0].v[e], zb[CORRECT ? t : 0].v[e]);
+        }
+#pragma unroll
+    for (int t = 0; t < C; ++t) {
+        stv<N>(oZ + t * D + d0, zb[CORRECT ? t : 0]);
+        Vec<N> qb = ldv<N>(oQ + t * D + d0);  // this thread's own
+#pragma unroll
+        for (int s = 0; s <= t; ++s) {
+            const float f = flat[t * t + t + s];
+#pragma unroll
+            for (int e = 0; e < N; ++e) qb.v[e] = fmaf(-f, zb[CORRECT ? s : 0].v[e], qb.v[e]);
+        }
+        stv<N>(oQ + t * D + d0, qb);
+    }
+}
+
+// ------------------------------------------------------------------------------------------------ the walk
+// x = hi + lo + (what neither holds, < 2^-21 |x|), both representable in TF32
+__device__ __forceinline__ void split(float x, uint32_t& hi, uint32_t& lo) {
+    hi = __float_as_uint(x) & 0xffffe000u;
+    lo = __float_as_uint(x - __uint_as_float(hi)) & 0xffffe000u;
+}
+__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+struct FragA {
+    uint32_t hi[4], lo[4];
+    __device__ __forceinline__ void set(float x0, float x1, float x2, float x3) {
+        split(x0, hi[0], lo[0]);
+        split(x1, hi[1], lo[1]);
+        split(x2, hi[2], lo[2]);
+        split(x3, hi[3], lo[3]);
+    }
+};
+struct FragB {
+    uint32_t hi[2], lo[2];
+    __device__ __forceinline__ void set(float x0, float x1) {
+        split(x0, hi[0], lo[0]);
+        split(x1, hi[1], lo[1]);
+    }
+};
+__device__ __forceinline__ void copy16(float* dst, const float* src, bool live) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+
+struct ScanArgs {
+    const float* ws;
+    const float* v;    // value of token row r, head h, channel e at v[r * v_ld + h * E + e]
+    long long v_ld;
+    float *state, *o;  // [slots, H, D, E], [n_tok, H * E]
+    const int *cu, *slot;
+    int H, E, c0, chunks;
+};
+
+// shared memory of a stage, in floats: Z [16][D + 8] | Q [16][D + 8] | P [16][PP] | b [D] | T [16][20] | A' [16][20] | V [16][cols + 8]
+template <int D, bool CORRECT> struct Layout {
+    static constexpr int DS = D + 8, PP = CORRECT ? D + 4 : D + 8, TS = C + 4;  // pitches without bank conflicts for their reads
+    static constexpr int Q = CORRECT ? C * DS : 0, P = Q + C * DS, B = P + C * PP, T = B + D, A = T + (CORRECT ? C * TS : 0), V = A + C * TS;
+    __host__ __device__ static constexpr int stage(int cols) { return V + C * (cols + 8); }
+};
+
+template <int D, bool CORRECT>
+__global__ void __launch_bounds__(256)
+chunk_scan_kernel(const ScanArgs p) {
+    constexpr int NT = D / 8;
+    typedef Layout<D, CORRECT> Y;
+    constexpr int M = CORRECT ? 2 : 1;  // Q alone, or Q and Z
+    extern __shared__ __align__(16) float sm[];
+    const int cols = (blockDim.x >> 5) * 16, VS = cols + 8;
+    const int stage_floats = Y::stage(cols);
+    const int h = blockIdx.y, b = blockIdx.z;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+    const int e0 = blockIdx.x * cols, wc = warp * 16;
+    const int row_b = p.cu[b], n = p.cu[b + 1] - row_b;
+    int nblk = (n + C - 1) / C - p.c0;
+    if (nblk <= 0) return;
+    if (nblk > p.chunks) nblk = p.chunks;
+    float* st = p.state + ((long long)p.slot[b] * p.H + h) * (long long)D * p.E + e0 + wc;
+    const float* wsb = p.ws + ((long long)b * p.chunks * p.H + h) * block_floats(D, CORRECT);
+    const long long ws_step = (long long)p.H * block_floats(D, CORRECT);
+    float S[NT][4];  // rows g, g + 8 (columns of S) x entries d = 8 nt + 2 t4, + 1
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) S[nt][c] = st[(long long)(8 * nt + 2 * t4 + (c & 1)) * p.E + g + (c >> 1) * 8];
+
+    auto fetch = [&](int k, float* dst) {
+        const float* s = wsb + k * ws_step;
+        auto rows = [&](float* to, int pitch) {  // 16 rows of D
+            for (int i = threadIdx.x; i < C * (D / 4); i += blockDim.x)
+                copy16(to + (i / (D / 4)) * pitch + (i % (D / 4)) * 4, s + i * 4, true);
+            s += C * D;
+        };
+        auto square = [&](float* to) {
+            for (int i = threadIdx.x; i < C * C / 4; i += blockDim.x) copy16(to + (i >> 2) * Y::TS + (i & 3) * 4, s + i * 4, true);
+            s += C * C;
+        };
+        if (CORRECT) rows(dst, Y::DS);
+        rows(dst + Y::Q, Y::DS);
+        rows(dst + Y::P, Y::PP);
+        for (int i = threadIdx.x; i < D / 4; i += blockDim.x) copy16(dst + Y::B + i * 4, s + i * 4, true);
+        s += D;
+        if (CORRECT) square(dst + Y::T);
+        square(dst + Y::A);
+        const int r0 = (p.c0 + k) * C, q = cols / 4;
+        for (int i = threadIdx.x; i < C * q; i += blockDim.x) {
+            const int t = i / q, e = (i % q) * 4;
+            const bool live = r0 + t < n;
+            copy16(dst + Y::V + t * VS + e, p.v + (live ? (long long)(row_b + r0 + t) * p.v_ld + h * p.E + e0 + e : 0), live);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0, sm);
+    for (int k = 0; k < nblk; ++k) {
+        const float* x = sm + (k & 1) * stage_floats;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();  // this block is here, and everybody is done with the one before
+        if (k + 1 < nblk) fetch(k + 1, sm + ((k + 1) & 1) * stage_floats);
+        // ---- S^T Q^T (and S^T Z^T), V^T A'^T (and V^T T^T)
+        float hh[M][2][2][4] = {}, xx[M][2][4] = {};  // leading products in two chains, the small ones in a third
+#pragma unroll
+        for (int kk = 0; kk < NT; ++kk) {
+            FragA a;
+            a.set(S[kk][0], S[kk][2], S[kk][1], S[kk][3]);  // slot t4 <-> entry 2 t4, slot t4 + 4 <-> entry 2 t4 + 1
+            FragB f[M][2];
+#pragma unroll
+            for (int m = 0; m < M; ++m)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const float2 y = *reinterpret_cast<const float2*>(x + (m == 0 ? Y::Q : 0) + (8 * j + g) * Y::DS + 8 * kk + 2 * t4);
+                    f[m][j].set(y.x, y.y);
+                }
+#pragma unroll
+            for (int m = 0; m < M; ++m)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) mma_tf32(hh[m][j][kk & 1], a.hi, f[m][j].hi);
+#pragma unroll
+            for (int m = 0; m < M; ++m)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) mma_tf32(xx[m][j], a.lo, f[m][j].hi);
+#pragma unroll
+            for (int m = 0; m < M; ++m)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) mma_tf32(xx[m][j], a.hi, f[m][j].lo);
+        }
+        FragA av[2];
+        float vv[M][2][4] = {};
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+            const float* vp = x + Y::V + (8 * ks + t4) * VS + wc + g;
+            av[ks].set(vp[0], vp[8], vp[4 * VS], vp[4 * VS + 8]);
+#pragma unroll
+            for (int m = 0; m < M; ++m)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    if (j < ks) continue;  // above the diagonal
+                    const float* tp = x + (m == 0 ? Y::A : Y::T) + (8 * j + g) * Y::TS + 8 * ks + t4;
+                    FragB f;
+                    f.set(tp[0], tp[4]);
+                    mma_tf32(vv[m][j], av[ks].lo, f.hi);
+                    mma_tf32(vv[m][j], av[ks].hi, f.lo);
+                    mma_tf32(vv[m][j], av[ks].hi, f.hi);
+                }
+        }
+        // ---- outputs: rows g, g + 8 are channels, columns 2 t4, 2 t4 + 1 of group j are tokens
+        const int r0 = (p.c0 + k) * C;
+        float* op = p.o + (long long)(row_b + r0) * p.H * p.E + (long long)h * p.E + e0 + wc + g;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int t = 8 * j + 2 * t4 + (c & 1);
+                if (r0 + t < n)
+                    op[(long long)t * p.H * p.E + (c >> 1) * 8] = (hh[0][j][0][c] + hh[0][j][1][c]) + (xx[0][j][c] + vv[0][j][c]);
+            }
+        // ---- S <- b S + P^T U
+        FragA au[2];
+        if (CORRECT) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                float u[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) u[c] = vv[M - 1][j][c] - ((hh[M - 1][j][0][c] + hh[M - 1][j][1][c]) + xx[M - 1][j][c]);
+                au[j].set(u[0], u[2], u[1], u[3]);  // slot t4 <-> token 2 t4, slot t4 + 4 <-> token 2 t4 + 1
+            }
+        }
+#pragma unroll
+        for (int n0 = 0; n0 < NT; n0 += 4) {
+            float acc[4][4] = {};
+#pragma unroll
+            for (int ks = 0; ks < 2; ++ks) {
+                const FragA& a = CORRECT ? au[ks] : av[ks];
+                FragB f[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float* pp = x + Y::P + (8 * ks + (CORRECT ? 2 * t4 : t4)) * Y::PP + 8 * (n0 + i) + g;
+                    f[i].set(pp[0], pp[(CORRECT ? 1 : 4) * Y::PP]);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) mma_tf32(acc[i], a.lo, f[i].hi);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) mma_tf32(acc[i], a.hi, f[i].lo);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) mma_tf32(acc[i], a.hi, f[i].hi);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float2 bb = *reinterpret_cast<const float2*>(x + Y::B + 8 * (n0 + i) + 2 * t4);
+                S[n0 + i][0] = fmaf(S[n0 + i][0], bb.x, acc[i][0]);
+                S[n0 + i][1] = fmaf(S[n0 + i][1], bb.y, acc[i][1]);
+                S[n0 + i][2] = fmaf(S[n0 + i][2], bb.x, acc[i][2]);
+                S[n0 + i][3] = fmaf(S[n0 + i][3], bb.y, acc[i][3]);
+            }
+        }
+    }
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) st[(long long)(8 * nt + 2 * t4 + (c & 1)) * p.E + g + (c >> 1) * 8] = S[nt][c];
+}
+
+// ------------------------------------------------------------------------------------------------ host
+static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+template <int D, int MODE>
+static int run(PrepArgs a, ScanArgs s, int n_seq, int max_len, cudaStream_t st) {
+    constexpr bool CORRECT = MODE == kPaired;
+    // columns of S per CTA: few heads and requests are spread over the SMs, many share the blocks' operands
+    const long long heads = (long long)n_seq * a.H;
+    int cols = 32;
+    while (cols < 128 && s.E % (2 * cols) == 0 && heads * (s.E / cols) > 148 * 4) cols *= 2;
+    const int smem = 2 * Layout<D, CORRECT>::stage(cols) * (int)sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(chunk_scan_kernel<D, CORRECT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    for (int c0 = 0; c0 * C < max_len && e == cudaSuccess; c0 += a.chunks) {
+        const int left = (max_len + C - 1) / C - c0, nc = left < a.chunks ? left : a.chunks;
+        a.c0 = s.c0 = c0;
+        chunk_prep_kernel<D, MODE><<<dim3(nc, (a.H + 3) / 4, n_seq), 128, 0, st>>>(a);
+        chunk_scan_kernel<D, CORRECT><<<dim3(s.E / cols, a.H, n_seq), cols * 2, smem, st>>>(s);
+        e = cudaGetLastError();
+    }
+    if (e != cudaSuccess) {
+        g_last_cuda_error = (int)e;
+        return LLARK_ECUDA;
+    }
+    return LLARK_OK;
+}
+
+}  // namespace chunk
+}  // namespace llark
+
+using namespace llark;
+
+extern "C" long long llark_seq_chunk_block_bytes(int D, int correct) { return 4LL * chunk::block_floats(D, correct != 0); }
+
+static bool bad_sizes(int n_seq, int max_len, int H, int D, int E, int chunks) {
+    return n_seq <= 0 || n_seq > 65535 || max_len <= 0 || H <= 0 || H > 65535 || (D != 64 && D != 128) || E <= 0 || E % 32 || chunks <= 0;
+}
+
+extern "C" int llark_seq_glr_chunks(const float* src, long long ld, int q_off, int f_off, int v_off, const float* lower, float* state,
+                                    float* o, float* ws, int chunks, const int* cu, const int* slot, int n_seq, int max_len, int H,
+                                    int D, int E, cudaStream_t st) {
+    if (bad_sizes(n_seq, max_len, H, D, E, chunks) || !src || !state || !o || !ws || !cu || !slot || ld % 4 || q_off % 4 || f_off % 4 ||
+        v_off % 4 || !chunk::aligned16(src) || !chunk::aligned16(ws))
+        return LLARK_EINVAL;
+    const chunk::PrepArgs a = {src, ld, q_off, f_off, lower, ws, cu, H, 0, chunks};
+    const chunk::ScanArgs s = {ws, src + v_off, ld, state, o, cu, slot, H, E, 0, chunks};
+    return D == 64 ? chunk::run<64, chunk::kGlr>(a, s, n_seq, max_len, st) : chunk::run<128, chunk::kGlr>(a, s, n_seq, max_len, st);
+}
+
+extern "C" int llark_seq_delta_chunks(const float* vec, const float* v, long long v_ld, float* state, float* o, float* ws, int chunks,
+                                      const int* cu, const int* slot, int n_seq, int max_len, int H, int D, int E, int correct,
+                                      cudaStream_t st) {
+    if (bad_sizes(n_seq, max_len, H, D, E, chunks) || !vec || !v || !state || !o || !ws || !cu || !slot || v_ld % 4 ||
+        !chunk::aligned16(vec) || !chunk::aligned16(v) || !chunk::aligned16(ws))
+        return LLARK_EINVAL;
+    const chunk::PrepArgs a = {vec, 0, 0, 0, nullptr, ws, cu, H, 0, chunks};
+    const chunk::ScanArgs s = {ws, v, v_ld, state, o, cu, slot, H, E, 0, chunks};
+    if (correct)
+        return D == 64 ? chunk::run<64, chunk::kPaired>(a, s, n_seq, max_len, st) : chunk::run<128, chunk::kPaired>(a, s, n_seq, max_len, st);
+    return D == 64 ? chunk::run<64, chunk::kPlain>(a, s, n_seq, max_len, st) : chunk::run<128, chunk::kPlain>(a, s, n_seq, max_len, st);
+}

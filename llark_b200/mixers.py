@@ -403,7 +403,7 @@ class GatedDeltaRule:
         cv = ops.seq_conv_act(pin[:, :w.n_conv], w.conv, cache.view(self.h_carry), st, silu=True)
         vec = ops.seq_delta_prep(ops.DELTA_GATED, cv[:, :GD], cv[:, GD:2 * GD], dec, pin[:, w.b_off:], w.H, w.G, w.D,
                                  dec_bias=w.dt_bias, rate_log=w.rate_log)
-        o = ops.seq_delta_scan(vec, cv[:, 2 * GD:], cache.view(self.h_state), st, w.H, w.D, w.E)
+        o = ops.seq_delta_scan(vec, cv[:, 2 * GD:], cache.view(self.h_state), st, w.H, w.D, w.E, paired=True)
         on = ops.seq_head_norm_gate(o, w.norm, w.H, w.E, self.eps, self.act, gate=gate)
         return ops.linear(on, w.w_o, out_dtype=F32)
 
@@ -488,7 +488,7 @@ class ScalarGatedDeltaRule(_OneBranch):
         cv = ops.seq_conv_act(pin[:, :w.n_conv], w.conv, cache.view(self.h_carry), st, silu=True)
         vec = ops.seq_delta_prep(ops.DELTA_GATED_SCALAR, cv[:, :GD], cv[:, GD:2 * GD], pin[:, w.a_off:w.a_off + w.H],
                                  pin[:, w.b_off:w.b_off + w.H], w.H, w.G, w.D, dec_bias=w.dt_bias, rate_log=w.rate_log)
-        o = ops.seq_delta_scan(vec, cv[:, 2 * GD:], cache.view(self.h_state), st, w.H, w.D, w.E)
+        o = ops.seq_delta_scan(vec, cv[:, 2 * GD:], cache.view(self.h_state), st, w.H, w.D, w.E, paired=True)
         on = ops.seq_head_norm_gate(o, w.norm, w.H, w.E, self.eps, self.act, gate=pin[:, w.g_off:w.n_in], gate_silu=True)
         return ops.linear(on, w.w_o, out_dtype=F32)
 

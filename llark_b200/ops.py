@@ -772,6 +772,20 @@ def seq_kv_ring_write(kn, vv, kring, vring, st, cap):
 
 GLR_CHUNK = 256        # rows per work item when a long prompt is scanned in chunks
 GLR_CHUNK_MIN_LEN = 512  # shortest longest-request of a step that is scanned in chunks
+# Steps whose longest request brings this many tokens take the tensor-core walk of csrc/seq_chunk.cu (blocks of 16 tokens) where its
+# sizes allow; its workspace holds up to SCAN_BLOCK_BYTES (less than L2, so that the walk finds there what was prepared)
+SCAN_BLOCK_MIN_LEN = 16
+SCAN_BLOCK_BYTES = 96 << 20
+
+
+def _scan_blocks(st, H, D, E, correct, tensors, offsets=()):
+    """(workspace, blocks of a request it holds) when the block walk takes these sizes and pointers, else None."""
+    if (st.max_len < SCAN_BLOCK_MIN_LEN or D not in (64, 128) or E % 32 or any(x % 4 for x in offsets)
+            or any(t.data_ptr() % 16 or t.stride(0) % 4 for t in tensors)):
+        return None
+    per = lib().llark_seq_chunk_block_bytes(D, int(correct)) * H * st.n_seq
+    n = max(1, min((st.max_len + 15) // 16, SCAN_BLOCK_BYTES // per))
+    return torch.empty(n * per, device=st.device, dtype=torch.uint8), n
 
 
 def seq_glr_scan(src, q_off, f_off, v_off, lower, state, st, H, D, E):
@@ -781,6 +795,12 @@ def seq_glr_scan(src, q_off, f_off, v_off, lower, state, st, H, D, E):
     _req(src, torch.float32), _req(state, torch.float32)
     o = torch.empty((st.n_tok, H * E), device=src.device, dtype=torch.float32)
     L = lib()
+    blocks = _scan_blocks(st, H, D, E, False, (src,), (q_off, f_off, v_off))
+    if blocks is not None:
+        ws, n = blocks
+        check(L.llark_seq_glr_chunks(_p(src), src.stride(0), q_off, f_off, v_off, _p(lower), _p(state), _p(o), _p(ws), n, _p(st.cu),
+                                     _p(st.slot), st.n_seq, st.max_len, H, D, E, _stream()), "seq_glr_chunks")
+        return o
     if st.max_len < GLR_CHUNK_MIN_LEN:
         check(L.llark_seq_glr_scan(_p(src), src.stride(0), q_off, f_off, v_off, _p(lower), _p(state), _p(state), None,
                                    _p(o), _p(st.cu), _p(st.lens_dev), _p(st.slot), _p(st.slot), st.n_seq, H, D, E,
@@ -952,11 +972,18 @@ def seq_delta_prep(rule, q, k, dec, mix, H, G, D, dec_bias=None, rate_log=None, 
     return vec
 
 
-def seq_delta_scan(vec, v, state, st, H, D, E, correct=True):
+def seq_delta_scan(vec, v, state, st, H, D, E, correct=True, paired=False):
     """vec fp32 [n_tok, H, 5, D], v fp32 [n_tok, H*E] (column slice fine), state fp32 [slots, H, D, E] (updated) ->
-    o fp32 [n_tok, H*E]. correct=False: the rule has no correction term (DELTA_STATE_SPACE)."""
+    o fp32 [n_tok, H*E]. correct=False: the rule has no correction term (DELTA_STATE_SPACE). paired: the fourth vector is the fifth
+    with its sign changed (DELTA_GATED, DELTA_GATED_SCALAR)."""
     _req(vec, torch.float32), _req(v, torch.float32), _req(state, torch.float32)
     o = torch.empty((st.n_tok, H * E), device=v.device, dtype=torch.float32)
+    blocks = _scan_blocks(st, H, D, E, correct, (vec, v)) if paired or not correct else None
+    if blocks is not None:
+        ws, n = blocks
+        check(lib().llark_seq_delta_chunks(_p(vec), _p(v), v.stride(0), _p(state), _p(o), _p(ws), n, _p(st.cu), _p(st.slot), st.n_seq,
+                                           st.max_len, H, D, E, int(correct), _stream()), "seq_delta_chunks")
+        return o
     check(lib().llark_seq_delta_scan(_p(vec), _p(v), v.stride(0), _p(state), _p(o), _p(st.cu), _p(st.slot), st.n_seq,
                                      st.n_tok, H, D, E, int(correct), _stream()), "seq_delta_scan")
     return o

@@ -1,0 +1,82 @@
+"""The block walk of matrix recurrences (csrc/seq_chunk.cu) against 64 bits and against the token-by-token kernels: requests of one token,
+around a block of 16, several passes of its workspace, decays from nothing left to nothing lost, states that were there before, both
+head sizes and all three sources."""
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+F32, F64 = torch.float32, torch.float64
+
+
+def _layout(lens, slots, dev="cuda"):
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    ints = lambda v: torch.tensor(v, device=dev, dtype=torch.int32)  # noqa: E731
+    return types.SimpleNamespace(n_tok=cu[-1], n_seq=len(lens), max_len=max(lens), cu=ints(cu), slot=ints(slots), lens_dev=ints(lens),
+                                 device=dev, cu_host=cu)
+
+
+def _walk(q, d, z, p, v, S, correct):
+    """One request in 64 bits: vectors [T, H, D], values [T, H, E], state [H, D, E]."""
+    out = []
+    for t in range(q.shape[0]):
+        u = v[t] - (torch.einsum("hde,hd->he", S, z[t]) if correct else 0)
+        S = d[t][..., None] * S + p[t][..., None] * u[:, None]
+        out.append(torch.einsum("hde,hd->he", S, q[t]))
+    return torch.stack(out), S
+
+
+@pytest.mark.parametrize("kind", ["hgrn2", "gated", "plain"])
+@pytest.mark.parametrize("lens,H,D,E,bytes_", [([16], 1, 128, 128, None), ([1, 17, 40], 5, 128, 64, None), ([33, 15, 2], 3, 64, 96, None),
+                                               ([200, 70], 2, 128, 128, 1)])
+def test_against_64_bits(kind, lens, H, D, E, bytes_, monkeypatch):
+    from llark_b200 import ops
+
+    if bytes_:
+        monkeypatch.setattr(ops, "SCAN_BLOCK_BYTES", bytes_)  # a workspace of one block per request: a pass per 16 tokens
+    torch.manual_seed(sum(lens) + H + D)
+    dev, n = "cuda", sum(lens)
+    slots = torch.randperm(len(lens) + 1)[:len(lens)].tolist()
+    st = _layout(lens, slots)
+    S0 = torch.randn(len(lens) + 1, H, D, E, device=dev)
+    state = S0.clone()
+    # decays of every kind: channels that keep next to nothing, that keep nearly everything, and anything between
+    x = torch.randn(n, H, D, device=dev) * 3 + torch.linspace(-12, 8, D, device=dev)
+    if kind == "hgrn2":
+        ld = 2 * H * D + H * E
+        src = torch.randn(n, ld, device=dev)
+        src[:, H * D:2 * H * D] = x.reshape(n, -1)
+        lower = torch.rand(H * D, device=dev) * (torch.rand(H * D, device=dev) > 0.3)
+        o = ops.seq_glr_scan(src, 0, H * D, 2 * H * D, lower, state, st, H, D, E)
+        s = src.to(F64)
+        q = torch.nn.functional.silu(s[:, :H * D]).view(n, H, D)
+        lo = lower.to(F64)
+        d = (lo + (1 - lo) * torch.sigmoid(s[:, H * D:2 * H * D])).view(n, H, D)
+        z, p, v = None, 1 - d, s[:, 2 * H * D:].reshape(n, H, E)
+    else:
+        unit = lambda t: t / t.norm(dim=-1, keepdim=True)  # noqa: E731
+        q, k = unit(torch.randn(n, H, D, device=dev)), unit(torch.randn(n, H, D, device=dev) + 0.5)
+        d, beta = torch.sigmoid(x), torch.rand(n, H, 1, device=dev)
+        v = torch.randn(n, H * E + 4, device=dev)[:, 4:]  # a column slice
+        z, p = (k * d, beta * k) if kind == "gated" else (torch.zeros_like(k), k)
+        vec = torch.stack([q, z, d, -p if kind == "gated" else torch.zeros_like(p), p], dim=2).contiguous()
+        o = ops.seq_delta_scan(vec, v, state, st, H, D, E, correct=kind == "gated", paired=kind == "gated")
+        monkeypatch.setattr(ops, "SCAN_BLOCK_MIN_LEN", 1 << 30)
+        old_state = S0.clone()
+        old = ops.seq_delta_scan(vec, v, old_state, st, H, D, E, correct=kind == "gated")
+        q, z, d, p = (t.to(F64) for t in (q, z, d, p))
+        v = v.to(F64).reshape(n, H, E)
+    for b, ln in enumerate(lens):
+        at = slice(st.cu_host[b], st.cu_host[b] + ln)
+        want, S = _walk(q[at], d[at], z[at] if z is not None else None, p[at], v[at], S0[slots[b]].to(F64), kind == "gated")
+        rel = lambda a, w: ((a.to(F64) - w).norm() / w.norm()).item()  # noqa: E731
+        eo, es = rel(o.view(n, H, E)[at], want), rel(state[slots[b]], S)
+        # 2^-21 of a product from the split, sums of up to 128 + 16 of them: 2e-6 of the terms' norm at most
+        assert eo < 2e-6 and es < 2e-6, (b, eo, es)
+        if kind != "hgrn2":
+            assert eo < max(2 * rel(old.view(n, H, E)[at], want), 1e-6) and es < max(2 * rel(old_state[slots[b]], S), 1e-6)
+    rest = [s for s in range(len(lens) + 1) if s not in slots]
+    assert torch.equal(state[rest], S0[rest])  # nobody else's state was touched
