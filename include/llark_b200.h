@@ -403,17 +403,17 @@ int llark_seq_glr_scan(const float* src, long long ld, int q_off, int f_off, int
 int llark_seq_glr_combine(const float* state, float* chunk_state, const float* chunk_decay, const int* seq_item0,
                           const int* slot, int n_seq, int H, int D, int E, cudaStream_t stream);
 /* The same recurrences of prompts on the tensor cores, 16 tokens at a time (D 64 or 128, E a multiple of 32, every row and offset a
- * multiple of 16 bytes): _glr_chunks on the projection's columns as llark_seq_glr_scan, _delta_chunks on the vectors of
- * llark_seq_delta_prep with (correct = 1: the fourth vector is minus the fifth) or without the correction term. state [slots, H, D, E]
- * is read and written back. ws: n_seq * chunks * H blocks of llark_seq_chunk_block_bytes; any chunks >= 1 does, longer requests are
- * walked in as many passes. */
+ * multiple of 16 bytes): _glr_chunks on the projection's columns as llark_seq_glr_scan; _delta_chunks on what llark_seq_delta_prep
+ * reads, rules 0, 2 and 3 of it. state [slots, H, D, E] is read and written back. ws: n_seq * chunks * H blocks of
+ * llark_seq_chunk_block_bytes (correct = 0 for HGRN2 and rule 3); any chunks >= 1 does, longer requests are walked in more passes. */
 long long llark_seq_chunk_block_bytes(int D, int correct);
 int llark_seq_glr_chunks(const float* src, long long ld, int q_off, int f_off, int v_off, const float* lower, float* state, float* o,
                          float* ws, int chunks, const int* cu, const int* slot, int n_seq, int max_len, int H, int D, int E,
                          cudaStream_t stream);
-int llark_seq_delta_chunks(const float* vec, const float* v, long long v_ld, float* state, float* o, float* ws, int chunks,
-                           const int* cu, const int* slot, int n_seq, int max_len, int H, int D, int E, int correct,
-                           cudaStream_t stream);
+int llark_seq_delta_chunks(int rule, const float* q, long long q_ld, const float* k, long long k_ld, const float* dec, long long dec_ld,
+                           const float* dec_bias, const float* rate_log, const float* mix, long long mix_ld, float unit_eps,
+                           const float* v, long long v_ld, float* state, float* o, float* ws, int chunks, const int* cu,
+                           const int* slot, int n_seq, int max_len, int H, int G, int D, int E, cudaStream_t stream);
 int llark_seq_head_rmsnorm(const float* x, const float* w, void* out, long long n_rows, int E, float eps, int act_fp32,
                            cudaStream_t stream);
 

@@ -14,16 +14,21 @@
 //
 //     O = Q S_0 + A' V,    U = T V - Z S_0,    S = diag(b_15) S_0 + P^T U.
 //
-//   chunk_prep_kernel   all of that which does not depend on S: a warp per block of tokens and head, every block at once, fp32
-//   chunk_scan_kernel   the walk over the blocks: a warp keeps 16 columns of S, transposed, in registers that are directly the A
-//                       operand of S^T Q^T. Every product as three TF32 products of split operands (x = hi + lo without lo lo:
-//                       2^-21 relative). The tensor cores cut their sums instead of rounding them, so chains are kept short (8
-//                       products) and a block's update of S starts from zero and is added with an FMA.
+//   chunk_prep_kernel   all of that which does not depend on S, from the projections: a warp per block of tokens and head, every
+//                       block at once, fp32
+//   chunk_scan_kernel   the walk over the blocks: two warps keep 16 columns of S, transposed, half of the rows each, in registers
+//                       that are directly the A operand of S^T Q^T; their partial results meet in shared memory. Every product as
+//                       three TF32 products of split operands (x = hi + lo without lo lo: 2^-21 relative). The tensor cores cut
+//                       their sums instead of rounding them, so chains are kept short (4 products) and a block's update of S
+//                       starts from zero and is added with an FMA.
 //
 // The token-by-token kernels (seq_mixers.cu, seq_delta.cu) walk a chain of shared-memory reads and FMAs per token and stay for short
-// steps, other sizes and the general rule. What bounds this: the tensor cores' mma.sync rate on one chain of blocks per head and 16
-// columns. Measured on a B200: see the launchers.
+// steps, other sizes and the general rule. What bounds this: one chain of blocks per head and 16 columns, in which a warp issues some
+// 750 instructions per block (100 of them products at 8 cycles each). With one warp for all rows the walk took 1.6 times as long: one
+// warp per scheduler waits for its own results two thirds of the time.
 #include "common.cuh"
+
+#include <utility>
 
 namespace llark {
 extern thread_local int g_last_cuda_error;
@@ -31,7 +36,7 @@ namespace chunk {
 
 constexpr int C = 16;  // tokens per block
 
-enum { kGlr = 0, kPaired = 1, kPlain = 2 };  // where q, d, p, z come from: HGRN2 columns; prepared vectors, with / without correction
+enum { kChannel = 0, kGlr = 1, kScalar = 2, kState = 3 };  // gated delta with a decay per channel / HGRN2 / with one decay / state space
 
 __host__ __device__ constexpr int block_floats(int D, bool correct) {  // Z | Q | P | b | T | A'
     return (correct ? 3 : 2) * C * D + D + (correct ? 2 : 1) * C * C;
@@ -77,23 +82,36 @@ __device__ __forceinline__ float reduce32(float (&v)[32], int lane) {
     return v[0];
 }
 
+template <int I> struct Const {
+    static constexpr int value = I;
+    __host__ __device__ constexpr operator int() const { return I; }
+};
+// f(0), f(1), .. f(N - 1) with constants: what indexes registers has to be known at compile time
+template <typename F, int... I> __device__ __forceinline__ void each_(F&& f, std::integer_sequence<int, I...>) {
+    (f(Const<I>{}), ...);
+}
+template <int N, typename F> __device__ __forceinline__ void each(F&& f) { each_(f, std::make_integer_sequence<int, N>{}); }
+
+__device__ __forceinline__ float softplusf_(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
+// 1 / (1 + e^-z) with the fast reciprocal (2 ulp)
+__device__ __forceinline__ float sigmoid_fast(float z) { return __fdividef(1.0f, 1.0f + expf(-z)); }
+
 struct PrepArgs {
-    const float* src;  // kGlr: columns of the fused projection; else the prepared vectors [n_tok, H, 5, D] = q, z, d, -p, p
-    long long ld;
-    int q_off, f_off;
-    const float* lower;
-    float* ws;         // [n_seq, chunks, H] blocks
+    const float *q, *k, *dec, *mix;  // k, mix: not with kGlr (dec = f there); mix: not with kState
+    long long q_ld, k_ld, dec_ld, mix_ld;
+    const float *bias, *rate_log;    // of the decay; kGlr: bias = the lower bound (or NULL), no rate
+    float unit_eps;
+    float* ws;                       // [n_seq, chunks, H] blocks
     const int* cu;
-    int H, c0, chunks;
+    int H, G, c0, chunks;
 };
 
-template <int D, int MODE>
-__global__ void __launch_bounds__(128)
+template <int D, int SRC>
+__global__ void __launch_bounds__(128, 4)
 chunk_prep_kernel(const PrepArgs p) {
     constexpr int N = D / 32;
-    constexpr bool CORRECT = MODE == kPaired;
-    constexpr int kFlat = CORRECT ? 256 : 160;
-    __shared__ float flat_[4][kFlat], sT_[4][CORRECT ? C * C : 1];
+    constexpr bool CORRECT = SRC == kChannel || SRC == kScalar;
+    __shared__ float flat_[4][CORRECT ? 256 : 160], sT_[4][CORRECT ? C * C : 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h = blockIdx.y * 4 + warp, b = blockIdx.z, c = p.c0 + blockIdx.x;
     const int row_b = p.cu[b], left = p.cu[b + 1] - row_b - c * C;
@@ -108,70 +126,110 @@ chunk_prep_kernel(const PrepArgs p) {
     float* oB = oP + C * D;
     float* oT = oB + D;
     float* oA = oT + (CORRECT ? C * C : 0);
-    const int d0 = lane * N;
-    Vec<N> low, cum, w[C], zb[CORRECT ? C : 1];
+    const int d0 = lane * N, g = SRC == kGlr ? h : h / (p.H / p.G);
+    const float* qp = p.q + row0 * p.q_ld + (long long)g * D + d0;
+    const float* kp = SRC == kGlr ? nullptr : p.k + row0 * p.k_ld + (long long)g * D + d0;
+    const bool wide = SRC == kChannel || SRC == kGlr;  // a decay per channel
+    const float* dp = p.dec + row0 * p.dec_ld + (wide ? (long long)h * D + d0 : h);
+    const float rate = SRC == kGlr ? 0.f : expf(p.rate_log[h]);
+    Vec<N> low, cum;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
         cum.v[i] = 1.f;
-        low.v[i] = MODE == kGlr && p.lower ? p.lower[h * D + d0 + i] : 0.f;
+        low.v[i] = wide && p.bias ? p.bias[h * D + d0 + i] : 0.f;
     }
-    float v[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = 0.f;
-    constexpr int G = 4;  // tokens whose rows are requested together
-#pragma unroll
-    for (int t0 = 0; t0 < C; t0 += G) {
-        Vec<N> q[G], d[G], pp[G], z[CORRECT ? G : 1];
-#pragma unroll
-        for (int i = 0; i < G; ++i) {
-            const int t = t0 + i;
-            if (t < cnt) {
-                if (MODE == kGlr) {
-                    const float* r = p.src + (row0 + t) * p.ld + (long long)h * D + d0;
-                    q[i] = ldv<N>(r + p.q_off);
-                    d[i] = ldv<N>(r + p.f_off);
-                } else {
-                    const float* r = p.src + ((row0 + t) * p.H + h) * 5 * D + d0;
-                    q[i] = ldv<N>(r);
-                    d[i] = ldv<N>(r + 2 * D);
-                    pp[i] = ldv<N>(r + 4 * D);
-                    if (CORRECT) z[CORRECT ? i : 0] = ldv<N>(r + D);
-                }
+    // numbers of a token: lane t keeps those of token t
+    float beta = 0.f, decay = 1.f, step = 0.f, rq = 0.f, rk = 0.f;
+    if (!wide || CORRECT) {
+        const int t = lane & 15;
+        if (t < cnt) {
+            if (CORRECT) beta = sigmoidf_(p.mix[(row0 + t) * p.mix_ld + h]);
+            if (!wide) {
+                step = softplusf_(dp[t * p.dec_ld] + p.bias[h]);
+                decay = expf(-rate * step);
             }
         }
-#pragma unroll
-        for (int i = 0; i < G; ++i) {
-            const int t = t0 + i;
+    }
+    float v[32];
+    if (CORRECT) {  // squared norms of q (lanes 0 .. 15) and k (16 .. 31)
+        each<C>([&](auto T) {
+            constexpr int t = T;
+            v[t] = v[t + 16] = 0.f;
+            if (t < cnt) {
+                const Vec<N> q = ldv<N>(qp + t * p.q_ld), k = ldv<N>(kp + t * p.k_ld);
+                v[t] = dot(q, q);
+                v[t + 16] = dot(k, k);
+            }
+        });
+        const float n2 = 1.0f / sqrtf(reduce32(v, lane) + p.unit_eps);
+        rq = n2 / sqrtf((float)D);
+        rk = __shfl_down_sync(0xffffffffu, n2, 16);  // of lanes 0 .. 15
+    }
+    Vec<N> w[C];
+    constexpr int G = 2;  // tokens whose rows are requested together
+    each<C / G>([&](auto T0) {
+        constexpr int t0 = T0 * G;
+        Vec<N> q[G], d[G], pp[G], z[G];
+        each<G>([&](auto I) {
+            constexpr int i = I, t = t0 + i;
+            if (t < cnt) {
+                q[i] = ldv<N>(qp + t * p.q_ld);
+                if (SRC != kGlr) pp[i] = ldv<N>(kp + t * p.k_ld);
+                if (wide) d[i] = ldv<N>(dp + t * p.dec_ld);
+            }
+        });
+        each<G>([&](auto I) {
+            constexpr int i = I, t = t0 + i;
+            float fb = 0.f, fd = 1.f, fs = 0.f, fq = 1.f, fk = 1.f;
+            if (CORRECT) {
+                fb = __shfl_sync(0xffffffffu, beta, t);
+                fq = __shfl_sync(0xffffffffu, rq, t);
+                fk = __shfl_sync(0xffffffffu, rk, t);
+            }
+            if (!wide) fd = __shfl_sync(0xffffffffu, decay, t);
+            if (SRC == kState) fs = __shfl_sync(0xffffffffu, step, t);
 #pragma unroll
             for (int e = 0; e < N; ++e) {
                 if (t >= cnt) {  // nothing read, nothing written, nothing lost
-                    q[i].v[e] = pp[i].v[e] = 0.f;
+                    q[i].v[e] = pp[i].v[e] = z[i].v[e] = 0.f;
                     d[i].v[e] = 1.f;
-                    if (CORRECT) z[CORRECT ? i : 0].v[e] = 0.f;
-                } else if (MODE == kGlr) {
+                } else if (SRC == kGlr) {
                     const float x = q[i].v[e];
-                    q[i].v[e] = x * sigmoidf_(x);
-                    d[i].v[e] = low.v[e] + (1.0f - low.v[e]) * sigmoidf_(d[i].v[e]);
+                    q[i].v[e] = x * sigmoid_fast(x);
+                    d[i].v[e] = low.v[e] + (1.0f - low.v[e]) * sigmoid_fast(d[i].v[e]);
                     pp[i].v[e] = 1.0f - d[i].v[e];
+                } else if (SRC == kState) {
+                    d[i].v[e] = fd;
+                    pp[i].v[e] *= fs;
+                } else {
+                    if (wide) d[i].v[e] = expf(-rate * softplusf_(d[i].v[e] + low.v[e]));
+                    else d[i].v[e] = fd;
+                    const float kh = pp[i].v[e] * fk;
+                    q[i].v[e] *= fq;
+                    z[i].v[e] = kh * d[i].v[e];
+                    pp[i].v[e] = fb * kh;
                 }
             }
-            auto put = [&](int idx, float x) {
+            auto put = [&](auto IDX, float x) {
+                constexpr int idx = decltype(IDX)::value;
                 v[idx & 31] = x;
-                if ((idx & 31) == 31) flat[idx - 31 + lane] = reduce32(v, lane);
+                if constexpr ((idx & 31) == 31) flat[idx - 31 + lane] = reduce32(v, lane);
             };
-            if (CORRECT) {
+            if constexpr (CORRECT) {
+                Vec<N> zb;
 #pragma unroll
-                for (int e = 0; e < N; ++e) zb[CORRECT ? t : 0].v[e] = z[CORRECT ? i : 0].v[e] * cum.v[e];
-#pragma unroll
-                for (int s = 0; s < t; ++s) put(t * t + s, dot(z[CORRECT ? i : 0], w[s]));  // L[t, s]
+                for (int e = 0; e < N; ++e) zb.v[e] = z[i].v[e] * cum.v[e];
+                stv<N>(oZ + t * D + d0, zb);
+                each<t>([&](auto S) { put(Const<t * t + S>{}, dot(z[i], w[S])); });  // L[t, s]
             }
+            each<t>([&](auto S) {
 #pragma unroll
-            for (int s = 0; s < t; ++s)
-#pragma unroll
-                for (int e = 0; e < N; ++e) w[s].v[e] *= d[i].v[e];
+                for (int e = 0; e < N; ++e) w[S].v[e] *= d[i].v[e];
+            });
             w[t] = pp[i];
-#pragma unroll
-            for (int s = 0; s <= t; ++s) put(CORRECT ? t * t + t + s : t * (t + 1) / 2 + s, dot(q[i], w[s]));  // A[t, s]
+            each<t + 1>([&](auto S) {  // A[t, s]
+                put(Const<(CORRECT ? t * t + t + S : t * (t + 1) / 2 + S)>{}, dot(q[i], w[S]));
+            });
             Vec<N> qb;
 #pragma unroll
             for (int e = 0; e < N; ++e) {
@@ -179,66 +237,64 @@ chunk_prep_kernel(const PrepArgs p) {
                 qb.v[e] = q[i].v[e] * cum.v[e];
             }
             stv<N>(oQ + t * D + d0, qb);
-        }
-    }
-    if (!CORRECT) flat[128 + lane] = reduce32(v, lane);  // entries 128 .. 135, and left-overs behind them
-#pragma unroll
-    for (int s = 0; s < C; ++s) stv<N>(oP + s * D + d0, w[s]);
+        });
+    });
+    each<C>([&](auto S) { stv<N>(oP + S * D + d0, w[S]); });
     stv<N>(oB + d0, cum);
-    __syncwarp();
-    if (!CORRECT) {
+    if constexpr (!CORRECT) {
+        flat[128 + lane] = reduce32(v, lane);  // entries 128 .. 135, and left-overs behind them
+        __syncwarp();
 #pragma unroll
         for (int i = 0; i < C * C; i += 32) {
             const int t = (i + lane) >> 4, s = (i + lane) & 15;
             oA[i + lane] = s <= t ? flat[t * (t + 1) / 2 + s] : 0.f;
         }
-        return;
-    }
-    // ---- T = (1 + L)^-1 and A' = A T, a column per lane (both halves of the warp do the same)
-    float* sT = sT_[warp];
-    {
-        const int j = lane & 15;
-        float col[C];
-#pragma unroll
-        for (int i = 0; i < C; ++i) {
-            float a = 0.f;
-#pragma unroll
-            for (int k = 0; k < i; ++k) a = fmaf(flat[i * i + k], col[k], a);
-            col[i] = i == j ? 1.f : (i > j ? -a : 0.f);
+    } else {
+        __syncwarp();
+        // ---- T = (1 + L)^-1 and A' = A T, a column per lane (both halves of the warp do the same)
+        float* sT = sT_[warp];
+        {
+            const int j = lane & 15;
+            float col[C];
+            each<C>([&](auto I) {
+                constexpr int i = I;
+                float a = 0.f;
+                each<i>([&](auto K) { a = fmaf(flat[i * i + K], col[K], a); });
+                col[i] = i == j ? 1.f : (i > j ? -a : 0.f);
+            });
+            each<C>([&](auto I) {
+                constexpr int i = I;
+                float a = 0.f;
+                each<i + 1>([&](auto K) { a = fmaf(flat[i * i + i + K], col[K], a); });
+                if (lane < 16) {
+                    sT[i * C + j] = col[i];
+                    oT[i * C + j] = col[i];
+                    oA[i * C + j] = a;
+                }
+            });
         }
+        __syncwarp();
+        // ---- Z = T Z' (from the last token back, so that the rows it reads are still Z'), Q = Q' - A Z; rows of this thread's own
+        each<C>([&](auto T) { w[T] = ldv<N>(oZ + T * D + d0); });
+        each<C>([&](auto R) {
+            constexpr int t = C - 1 - R;
+            each<t>([&](auto S) {
+                const float f = sT[t * C + S];
 #pragma unroll
-        for (int i = 0; i < C; ++i) {
-            float a = 0.f;
+                for (int e = 0; e < N; ++e) w[t].v[e] = fmaf(f, w[S].v[e], w[t].v[e]);
+            });
+        });
+        each<C>([&](auto T) {
+            constexpr int t = T;
+            stv<N>(oZ + t * D + d0, w[t]);
+            Vec<N> qb = ldv<N>(oQ + t * D + d0);
+            each<t + 1>([&](auto S) {
+                const float f = flat[t * t + t + S];
 #pragma unroll
-            for (int k = 0; k <= i; ++k) a = fmaf(flat[i * i + i + k], col[k], a);
-            if (lane < 16) {
-                sT[i * C + j] = col[i];
-                oT[i * C + j] = col[i];
-                oA[i * C + j] = a;
-            }
-        }
-    }
-    __syncwarp();
-    // ---- Z = T Z' (from the last token back, so that the rows it reads are still Z'), Q = Q' - A Z
-#pragma unroll
-    for (int t = C - 1; t > 0; --t)
-#pragma unroll
-        for (int s = 0; s < t; ++s) {
-            const float f = sT[t * C + s];
-#pragma unroll
-            for (int e = 0; e < N; ++e) zb[CORRECT ? t : 0].v[e] = fmaf(f, zb[CORRECT ? s : 0].v[e], zb[CORRECT ? t : 0].v[e]);
-        }
-#pragma unroll
-    for (int t = 0; t < C; ++t) {
-        stv<N>(oZ + t * D + d0, zb[CORRECT ? t : 0]);
-        Vec<N> qb = ldv<N>(oQ + t * D + d0);  // this thread's own
-#pragma unroll
-        for (int s = 0; s <= t; ++s) {
-            const float f = flat[t * t + t + s];
-#pragma unroll
-            for (int e = 0; e < N; ++e) qb.v[e] = fmaf(-f, zb[CORRECT ? s : 0].v[e], qb.v[e]);
-        }
-        stv<N>(oQ + t * D + d0, qb);
+                for (int e = 0; e < N; ++e) qb.v[e] = fmaf(-f, w[S].v[e], qb.v[e]);
+            });
+            stv<N>(oQ + t * D + d0, qb);
+        });
     }
 }
 
@@ -292,23 +348,27 @@ template <int D, bool CORRECT> struct Layout {
 template <int D, bool CORRECT>
 __global__ void __launch_bounds__(256)
 chunk_scan_kernel(const ScanArgs p) {
-    constexpr int NT = D / 8;
+    constexpr int NT = D / 16;  // groups of eight rows of S that a warp keeps: half of them
     typedef Layout<D, CORRECT> Y;
     constexpr int M = CORRECT ? 2 : 1;  // Q alone, or Q and Z
     extern __shared__ __align__(16) float sm[];
-    const int cols = (blockDim.x >> 5) * 16, VS = cols + 8;
+    const int cols = (blockDim.x >> 6) * 16, VS = cols + 8;
     const int stage_floats = Y::stage(cols);
     const int h = blockIdx.y, b = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
-    const int e0 = blockIdx.x * cols, wc = warp * 16;
+    const int half = warp & 1, e0 = blockIdx.x * cols, wc = (warp >> 1) * 16;
     const int row_b = p.cu[b], n = p.cu[b + 1] - row_b;
     int nblk = (n + C - 1) / C - p.c0;
     if (nblk <= 0) return;
     if (nblk > p.chunks) nblk = p.chunks;
-    float* st = p.state + ((long long)p.slot[b] * p.H + h) * (long long)D * p.E + e0 + wc;
+    const int hd = half * (D / 2);
+    // partial results that the two warps of a column group hand each other: [2][warps][32] float4 of outputs, [warps][2][32] of U
+    float4* xo = reinterpret_cast<float4*>(sm + 2 * stage_floats);
+    float4* xu = xo + 2 * blockDim.x;
+    float* st = p.state + ((long long)p.slot[b] * p.H + h) * (long long)D * p.E + (long long)hd * p.E + e0 + wc;
     const float* wsb = p.ws + ((long long)b * p.chunks * p.H + h) * block_floats(D, CORRECT);
     const long long ws_step = (long long)p.H * block_floats(D, CORRECT);
-    float S[NT][4];  // rows g, g + 8 (columns of S) x entries d = 8 nt + 2 t4, + 1
+    float S[NT][4];  // rows g, g + 8 (columns of S) x entries d = hd + 8 nt + 2 t4, + 1
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -340,13 +400,28 @@ chunk_scan_kernel(const ScanArgs p) {
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    // The outputs of eight tokens: this warp finishes tokens 8 half .. 8 half + 7 of a block, one block later (the other warp's part
+    // is then there without a wait of its own). Rows g, g + 8 are channels, columns 2 t4, 2 t4 + 1 tokens.
+    float mine[4];
+    auto finish = [&](int k) {
+        const int r0 = (p.c0 + k) * C + 8 * half;
+        const float4 o4 = xo[(k & 1) * blockDim.x + (warp ^ 1) * 32 + lane];
+        const float other[4] = {o4.x, o4.y, o4.z, o4.w};
+        float* op = p.o + (long long)(row_b + r0) * p.H * p.E + (long long)h * p.E + e0 + wc + g;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int t = 2 * t4 + (c & 1);
+            if (r0 + t < n) op[(long long)t * p.H * p.E + (c >> 1) * 8] = mine[c] + other[c];
+        }
+    };
     fetch(0, sm);
     for (int k = 0; k < nblk; ++k) {
         const float* x = sm + (k & 1) * stage_floats;
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();  // this block is here, and everybody is done with the one before
         if (k + 1 < nblk) fetch(k + 1, sm + ((k + 1) & 1) * stage_floats);
-        // ---- S^T Q^T (and S^T Z^T), V^T A'^T (and V^T T^T)
+        if (k) finish(k - 1);
+        // ---- this warp's rows of S^T Q^T (and S^T Z^T)
         float hh[M][2][2][4] = {}, xx[M][2][4] = {};  // leading products in two chains, the small ones in a third
 #pragma unroll
         for (int kk = 0; kk < NT; ++kk) {
@@ -357,7 +432,7 @@ chunk_scan_kernel(const ScanArgs p) {
             for (int m = 0; m < M; ++m)
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
-                    const float2 y = *reinterpret_cast<const float2*>(x + (m == 0 ? Y::Q : 0) + (8 * j + g) * Y::DS + 8 * kk + 2 * t4);
+                    const float2 y = *reinterpret_cast<const float2*>(x + (m == 0 ? Y::Q : 0) + (8 * j + g) * Y::DS + hd + 8 * kk + 2 * t4);
                     f[m][j].set(y.x, y.y);
                 }
 #pragma unroll
@@ -373,45 +448,58 @@ chunk_scan_kernel(const ScanArgs p) {
 #pragma unroll
                 for (int j = 0; j < 2; ++j) mma_tf32(xx[m][j], a.hi, f[m][j].lo);
         }
+        // ---- and, for tokens 8 half .. 8 half + 7, V^T A'^T (and V^T T^T); nothing above the diagonal
         FragA av[2];
-        float vv[M][2][4] = {};
+        float vv[M][4] = {};
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) {
             const float* vp = x + Y::V + (8 * ks + t4) * VS + wc + g;
             av[ks].set(vp[0], vp[8], vp[4 * VS], vp[4 * VS + 8]);
+            if (ks <= half) {  // the same for the whole warp
 #pragma unroll
-            for (int m = 0; m < M; ++m)
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    if (j < ks) continue;  // above the diagonal
-                    const float* tp = x + (m == 0 ? Y::A : Y::T) + (8 * j + g) * Y::TS + 8 * ks + t4;
+                for (int m = 0; m < M; ++m) {
+                    const float* tp = x + (m == 0 ? Y::A : Y::T) + (8 * half + g) * Y::TS + 8 * ks + t4;
                     FragB f;
                     f.set(tp[0], tp[4]);
-                    mma_tf32(vv[m][j], av[ks].lo, f.hi);
-                    mma_tf32(vv[m][j], av[ks].hi, f.lo);
-                    mma_tf32(vv[m][j], av[ks].hi, f.hi);
+                    mma_tf32(vv[m], av[ks].lo, f.hi);
+                    mma_tf32(vv[m], av[ks].hi, f.lo);
+                    mma_tf32(vv[m], av[ks].hi, f.hi);
                 }
+            }
         }
-        // ---- outputs: rows g, g + 8 are channels, columns 2 t4, 2 t4 + 1 of group j are tokens
-        const int r0 = (p.c0 + k) * C;
-        float* op = p.o + (long long)(row_b + r0) * p.H * p.E + (long long)h * p.E + e0 + wc + g;
+        float part[2][4];
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
+            for (int c = 0; c < 4; ++c) part[j][c] = (hh[0][j][0][c] + hh[0][j][1][c]) + xx[0][j][c];
+        {
+            float give[4];
+#pragma unroll
             for (int c = 0; c < 4; ++c) {
-                const int t = 8 * j + 2 * t4 + (c & 1);
-                if (r0 + t < n)
-                    op[(long long)t * p.H * p.E + (c >> 1) * 8] = (hh[0][j][0][c] + hh[0][j][1][c]) + (xx[0][j][c] + vv[0][j][c]);
+                mine[c] = (half ? part[1][c] : part[0][c]) + vv[0][c];
+                give[c] = half ? part[0][c] : part[1][c];
             }
+            xo[(k & 1) * blockDim.x + warp * 32 + lane] = make_float4(give[0], give[1], give[2], give[3]);
+        }
         // ---- S <- b S + P^T U
         FragA au[2];
         if (CORRECT) {
+            float u[2][4];
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                float u[4];
 #pragma unroll
-                for (int c = 0; c < 4; ++c) u[c] = vv[M - 1][j][c] - ((hh[M - 1][j][0][c] + hh[M - 1][j][1][c]) + xx[M - 1][j][c]);
-                au[j].set(u[0], u[2], u[1], u[3]);  // slot t4 <-> token 2 t4, slot t4 + 4 <-> token 2 t4 + 1
+                for (int c = 0; c < 4; ++c) {
+                    u[j][c] = -((hh[M - 1][j][0][c] + hh[M - 1][j][1][c]) + xx[M - 1][j][c]);
+                    if (j == half) u[j][c] += vv[M - 1][c];
+                }
+                xu[(warp * 2 + j) * 32 + lane] = make_float4(u[j][0], u[j][1], u[j][2], u[j][3]);
+            }
+            asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp >> 1)) : "memory");  // the two warps of these columns
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const float4 y = xu[((warp ^ 1) * 2 + j) * 32 + lane];
+                // slot t4 <-> token 2 t4, slot t4 + 4 <-> token 2 t4 + 1; the same sum in both warps
+                au[j].set(u[j][0] + y.x, u[j][2] + y.z, u[j][1] + y.y, u[j][3] + y.w);
             }
         }
 #pragma unroll
@@ -423,7 +511,7 @@ chunk_scan_kernel(const ScanArgs p) {
                 FragB f[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const float* pp = x + Y::P + (8 * ks + (CORRECT ? 2 * t4 : t4)) * Y::PP + 8 * (n0 + i) + g;
+                    const float* pp = x + Y::P + (8 * ks + (CORRECT ? 2 * t4 : t4)) * Y::PP + hd + 8 * (n0 + i) + g;
                     f[i].set(pp[0], pp[(CORRECT ? 1 : 4) * Y::PP]);
                 }
 #pragma unroll
@@ -435,7 +523,7 @@ chunk_scan_kernel(const ScanArgs p) {
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const float2 bb = *reinterpret_cast<const float2*>(x + Y::B + 8 * (n0 + i) + 2 * t4);
+                const float2 bb = *reinterpret_cast<const float2*>(x + Y::B + hd + 8 * (n0 + i) + 2 * t4);
                 S[n0 + i][0] = fmaf(S[n0 + i][0], bb.x, acc[i][0]);
                 S[n0 + i][1] = fmaf(S[n0 + i][1], bb.y, acc[i][1]);
                 S[n0 + i][2] = fmaf(S[n0 + i][2], bb.x, acc[i][2]);
@@ -443,6 +531,8 @@ chunk_scan_kernel(const ScanArgs p) {
             }
         }
     }
+    __syncthreads();
+    finish(nblk - 1);
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -452,20 +542,20 @@ chunk_scan_kernel(const ScanArgs p) {
 // ------------------------------------------------------------------------------------------------ host
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-template <int D, int MODE>
+template <int D, int SRC>
 static int run(PrepArgs a, ScanArgs s, int n_seq, int max_len, cudaStream_t st) {
-    constexpr bool CORRECT = MODE == kPaired;
+    constexpr bool CORRECT = SRC == kChannel || SRC == kScalar;
     // columns of S per CTA: few heads and requests are spread over the SMs, many share the blocks' operands
     const long long heads = (long long)n_seq * a.H;
     int cols = 32;
-    while (cols < 128 && s.E % (2 * cols) == 0 && heads * (s.E / cols) > 148 * 4) cols *= 2;
-    const int smem = 2 * Layout<D, CORRECT>::stage(cols) * (int)sizeof(float);
+    while (cols < 64 && s.E % (2 * cols) == 0 && heads * (s.E / cols) > 148 * 4) cols *= 2;
+    const int threads = cols * 4, smem = (2 * Layout<D, CORRECT>::stage(cols) + 4 * threads * 4) * (int)sizeof(float);
     cudaError_t e = cudaFuncSetAttribute(chunk_scan_kernel<D, CORRECT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     for (int c0 = 0; c0 * C < max_len && e == cudaSuccess; c0 += a.chunks) {
         const int left = (max_len + C - 1) / C - c0, nc = left < a.chunks ? left : a.chunks;
         a.c0 = s.c0 = c0;
-        chunk_prep_kernel<D, MODE><<<dim3(nc, (a.H + 3) / 4, n_seq), 128, 0, st>>>(a);
-        chunk_scan_kernel<D, CORRECT><<<dim3(s.E / cols, a.H, n_seq), cols * 2, smem, st>>>(s);
+        chunk_prep_kernel<D, SRC><<<dim3(nc, (a.H + 3) / 4, n_seq), 128, 0, st>>>(a);
+        chunk_scan_kernel<D, CORRECT><<<dim3(s.E / cols, a.H, n_seq), threads, smem, st>>>(s);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) {
@@ -492,20 +582,24 @@ extern "C" int llark_seq_glr_chunks(const float* src, long long ld, int q_off, i
     if (bad_sizes(n_seq, max_len, H, D, E, chunks) || !src || !state || !o || !ws || !cu || !slot || ld % 4 || q_off % 4 || f_off % 4 ||
         v_off % 4 || !chunk::aligned16(src) || !chunk::aligned16(ws))
         return LLARK_EINVAL;
-    const chunk::PrepArgs a = {src, ld, q_off, f_off, lower, ws, cu, H, 0, chunks};
+    const chunk::PrepArgs a = {src + q_off, nullptr, src + f_off, nullptr, ld, 0, ld, 0, lower, nullptr, 0.f, ws, cu, H, H, 0, chunks};
     const chunk::ScanArgs s = {ws, src + v_off, ld, state, o, cu, slot, H, E, 0, chunks};
     return D == 64 ? chunk::run<64, chunk::kGlr>(a, s, n_seq, max_len, st) : chunk::run<128, chunk::kGlr>(a, s, n_seq, max_len, st);
 }
 
-extern "C" int llark_seq_delta_chunks(const float* vec, const float* v, long long v_ld, float* state, float* o, float* ws, int chunks,
-                                      const int* cu, const int* slot, int n_seq, int max_len, int H, int D, int E, int correct,
-                                      cudaStream_t st) {
-    if (bad_sizes(n_seq, max_len, H, D, E, chunks) || !vec || !v || !state || !o || !ws || !cu || !slot || v_ld % 4 ||
-        !chunk::aligned16(vec) || !chunk::aligned16(v) || !chunk::aligned16(ws))
+extern "C" int llark_seq_delta_chunks(int rule, const float* q, long long q_ld, const float* k, long long k_ld, const float* dec,
+                                      long long dec_ld, const float* dec_bias, const float* rate_log, const float* mix,
+                                      long long mix_ld, float unit_eps, const float* v, long long v_ld, float* state, float* o,
+                                      float* ws, int chunks, const int* cu, const int* slot, int n_seq, int max_len, int H, int G,
+                                      int D, int E, cudaStream_t st) {
+    if (bad_sizes(n_seq, max_len, H, D, E, chunks) || (rule != 0 && rule != 2 && rule != 3) || G <= 0 || H % G || !q || !k || !dec ||
+        !dec_bias || !rate_log || (!mix && rule != 3) || !v || !state || !o || !ws || !cu || !slot || q_ld % 4 || k_ld % 4 || v_ld % 4 ||
+        !chunk::aligned16(q) || !chunk::aligned16(k) || !chunk::aligned16(v) || !chunk::aligned16(ws) ||
+        (rule == 0 && (dec_ld % 4 || !chunk::aligned16(dec))))
         return LLARK_EINVAL;
-    const chunk::PrepArgs a = {vec, 0, 0, 0, nullptr, ws, cu, H, 0, chunks};
+    const chunk::PrepArgs a = {q, k, dec, mix, q_ld, k_ld, dec_ld, mix_ld, dec_bias, rate_log, unit_eps, ws, cu, H, G, 0, chunks};
     const chunk::ScanArgs s = {ws, v, v_ld, state, o, cu, slot, H, E, 0, chunks};
-    if (correct)
-        return D == 64 ? chunk::run<64, chunk::kPaired>(a, s, n_seq, max_len, st) : chunk::run<128, chunk::kPaired>(a, s, n_seq, max_len, st);
-    return D == 64 ? chunk::run<64, chunk::kPlain>(a, s, n_seq, max_len, st) : chunk::run<128, chunk::kPlain>(a, s, n_seq, max_len, st);
+#define LLARK_CHUNKS(SRC_) (D == 64 ? chunk::run<64, SRC_>(a, s, n_seq, max_len, st) : chunk::run<128, SRC_>(a, s, n_seq, max_len, st))
+    return rule == 0 ? LLARK_CHUNKS(chunk::kChannel) : rule == 2 ? LLARK_CHUNKS(chunk::kScalar) : LLARK_CHUNKS(chunk::kState);
+#undef LLARK_CHUNKS
 }

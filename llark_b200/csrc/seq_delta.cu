@@ -66,42 +66,76 @@ __global__ void conv_act_kernel(const float* __restrict__ src, long long ld, con
     }
 }
 
-// Prompts: a thread walks TB consecutive rows of one channel with the last TAPS-1 inputs in registers, so every input is
-// read once (the per-row kernel reads it TAPS times) and the accesses of a warp are adjacent channels of one row. The
-// window is rebuilt wherever a request starts inside the run of rows.
-template <int TAPS, int TB>
-__global__ void conv_act_rows_kernel(const float* __restrict__ src, long long ld, const float* __restrict__ w,
-                                     const float* __restrict__ carry, const int* __restrict__ tok_seq,
-                                     const int* __restrict__ cu, const int* __restrict__ slot, float* __restrict__ out,
-                                     int n_tok, int n_ch, int silu, const float* __restrict__ bias) {
-    const int c = blockIdx.y * blockDim.x + threadIdx.x;
+// Prompts: a thread takes TB consecutive rows of V adjacent channels. Inside a request (nearly always) it requests all of them and
+// the TAPS-1 rows before at once and reads every input once; a run of rows in which a request starts or ends goes row by row.
+// Memory-bound: 5297 rows x 6144 channels 53 us (82 with one channel per thread and one row at a time; 40 us of traffic).
+template <int TAPS, int TB, int V>
+__global__ void __launch_bounds__(128)
+conv_act_rows_kernel(const float* __restrict__ src, long long ld, const float* __restrict__ w,
+                     const float* __restrict__ carry, const int* __restrict__ tok_seq,
+                     const int* __restrict__ cu, const int* __restrict__ slot, float* __restrict__ out,
+                     int n_tok, int n_ch, int silu, const float* __restrict__ bias) {
+    const int c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
     if (c >= n_ch) return;
     const int t0 = blockIdx.x * TB;
-    float wr[TAPS], win[TAPS > 1 ? TAPS - 1 : 1];
+    float wr[V][TAPS], b0[V];
 #pragma unroll
-    for (int j = 0; j < TAPS; ++j) wr[j] = w[(long long)c * TAPS + j];
-    const float b0 = bias ? bias[c] : 0.f;
-    for (int i = 0; i < TB && t0 + i < n_tok; ++i) {
-        const int t = t0 + i;
-        const int b = tok_seq[t];
-        const int local = t - cu[b];
-        if (i == 0 || local < TAPS - 1) {
-            const float* cr = carry + (long long)slot[b] * (TAPS - 1) * n_ch;
+    for (int x = 0; x < V; ++x) {
 #pragma unroll
-            for (int j = 0; j < TAPS - 1; ++j) {
-                const int s = local - (TAPS - 1) + j;
-                win[j] = s >= 0 ? src[(long long)(t - local + s) * ld + c] : cr[(long long)(TAPS - 1 + s) * n_ch + c];
-            }
+        for (int j = 0; j < TAPS; ++j) wr[x][j] = w[(long long)(c + x) * TAPS + j];
+        b0[x] = bias ? bias[c + x] : 0.f;
+    }
+    auto load = [&](const float* p, float (&v)[V]) {
+        if constexpr (V == 4) {
+            const float4 f = *reinterpret_cast<const float4*>(p);
+            v[0] = f.x, v[1] = f.y, v[2] = f.z, v[3] = f.w;
+        } else {
+            v[0] = p[0];
         }
-        const float cur = src[(long long)t * ld + c];
-        float acc = b0;
+    };
+    auto finish = [&](int t, const float (&acc)[V]) {
+        float r[V];
 #pragma unroll
-        for (int j = 0; j < TAPS - 1; ++j) acc = fmaf(wr[j], win[j], acc);
-        acc = fmaf(wr[TAPS - 1], cur, acc);
-        out[(long long)t * n_ch + c] = silu ? acc * sigmoidf_(acc) : acc;
+        for (int x = 0; x < V; ++x) r[x] = silu ? acc[x] * sigmoidf_(acc[x]) : acc[x];
+        float* p = out + (long long)t * n_ch + c;
+        if constexpr (V == 4)
+            *reinterpret_cast<float4*>(p) = make_float4(r[0], r[1], r[2], r[3]);
+        else
+            p[0] = r[0];
+    };
+    const int b = tok_seq[t0], local0 = t0 - cu[b];
+    if (local0 >= TAPS - 1 && t0 + TB <= cu[b + 1]) {
+        float in[TB + TAPS - 1][V];
 #pragma unroll
-        for (int j = 0; j + 1 < TAPS - 1; ++j) win[j] = win[j + 1];
-        if (TAPS > 1) win[TAPS - 2] = cur;
+        for (int i = 0; i < TB + TAPS - 1; ++i) load(src + (long long)(t0 - (TAPS - 1) + i) * ld + c, in[i]);
+#pragma unroll
+        for (int i = 0; i < TB; ++i) {
+            float acc[V];
+#pragma unroll
+            for (int x = 0; x < V; ++x) {
+                acc[x] = b0[x];
+#pragma unroll
+                for (int j = 0; j < TAPS; ++j) acc[x] = fmaf(wr[x][j], in[i + j][x], acc[x]);
+            }
+            finish(t0 + i, acc);
+        }
+        return;
+    }
+    for (int t = t0; t < t0 + TB && t < n_tok; ++t) {
+        const int bt = tok_seq[t], local = t - cu[bt];
+        const float* cr = carry + (long long)slot[bt] * (TAPS - 1) * n_ch + c;
+        float acc[V];
+#pragma unroll
+        for (int x = 0; x < V; ++x) acc[x] = b0[x];
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) {
+            const int s = local - (TAPS - 1) + j;
+            float v[V];
+            load(s >= 0 ? src + (long long)(t - local + s) * ld + c : cr + (long long)(TAPS - 1 + s) * n_ch, v);
+#pragma unroll
+            for (int x = 0; x < V; ++x) acc[x] = fmaf(wr[x][j], v[x], acc[x]);
+        }
+        finish(t, acc);
     }
 }
 
@@ -111,7 +145,8 @@ __global__ void conv_carry_kernel(const float* __restrict__ src, long long ld, f
     const int b = blockIdx.x;
     const int r0 = cu[b], n = cu[b + 1] - r0;
     float* cr = carry + (long long)slot[b] * (taps - 1) * n_ch;
-    for (int c = threadIdx.x; c < n_ch; c += blockDim.x)
+    const int c = blockIdx.y * blockDim.x + threadIdx.x;
+    if (c < n_ch)
         for (int k = 0; k < taps - 1; ++k) {  // ascending: entry k + n >= k is read before it is rewritten
             const int s = n - (taps - 1) + k;
             cr[(long long)k * n_ch + c] = s >= 0 ? src[(long long)(r0 + s) * ld + c] : cr[(long long)(taps - 1 + s) * n_ch + c];
@@ -554,17 +589,22 @@ extern "C" int llark_seq_conv_act(const float* src, long long ld, const float* w
     while (th < n_ch && th < 256) th <<= 1;
     const int inline_carry = n_tok == n_seq;  // every request brings one token
     if (!inline_carry && n_tok >= 64 && taps >= 2 && taps <= 4) {
-        constexpr int TB = 16;
-        dim3 grid((n_tok + TB - 1) / TB, (n_ch + 127) / 128);
-        if (taps == 2)
-            conv_act_rows_kernel<2, TB><<<grid, 128, 0, st>>>(src, ld, w, carry, tok_seq, cu, slot, out, n_tok, n_ch, silu,
-                                                              bias);
-        else if (taps == 3)
-            conv_act_rows_kernel<3, TB><<<grid, 128, 0, st>>>(src, ld, w, carry, tok_seq, cu, slot, out, n_tok, n_ch, silu,
-                                                              bias);
-        else
-            conv_act_rows_kernel<4, TB><<<grid, 128, 0, st>>>(src, ld, w, carry, tok_seq, cu, slot, out, n_tok, n_ch, silu,
-                                                              bias);
+        const bool vec = n_ch % 4 == 0 && ld % 4 == 0 &&
+                         ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(carry)) & 15) == 0;
+#define LLARK_ROWS(T_, TB_, V_)                                                                                              \
+    conv_act_rows_kernel<T_, TB_, V_><<<dim3((n_tok + TB_ - 1) / TB_, (n_ch + 128 * V_ - 1) / (128 * V_)), 128, 0, st>>>(    \
+        src, ld, w, carry, tok_seq, cu, slot, out, n_tok, n_ch, silu, bias)
+#define LLARK_TAPS(TB_, V_)            \
+    if (taps == 2) LLARK_ROWS(2, TB_, V_); \
+    else if (taps == 3) LLARK_ROWS(3, TB_, V_); \
+    else LLARK_ROWS(4, TB_, V_)
+        if (vec) {
+            LLARK_TAPS(8, 4);
+        } else {
+            LLARK_TAPS(16, 1);
+        }
+#undef LLARK_TAPS
+#undef LLARK_ROWS
     } else {
         // few rows (decode): the channels are spread over blocks too, so that a handful of tokens still fills the GPU
         int gy = (n_ch + th - 1) / th;
@@ -574,7 +614,7 @@ extern "C" int llark_seq_conv_act(const float* src, long long ld, const float* w
     }
     int rc = check_launch();
     if (rc != LLARK_OK || inline_carry || taps == 1) return rc;
-    conv_carry_kernel<<<n_seq, th, 0, st>>>(src, ld, carry, cu, slot, n_ch, taps);
+    conv_carry_kernel<<<dim3(n_seq, (n_ch + 127) / 128), 128, 0, st>>>(src, ld, carry, cu, slot, n_ch, taps);
     return check_launch();
 }
 

@@ -401,9 +401,8 @@ class GatedDeltaRule:
         dec = ops.linear(low[:, :w.ra], w.a2, out_dtype=F32)
         gate = ops.linear(low[:, w.ra:], w.g2, out_dtype=F32)
         cv = ops.seq_conv_act(pin[:, :w.n_conv], w.conv, cache.view(self.h_carry), st, silu=True)
-        vec = ops.seq_delta_prep(ops.DELTA_GATED, cv[:, :GD], cv[:, GD:2 * GD], dec, pin[:, w.b_off:], w.H, w.G, w.D,
-                                 dec_bias=w.dt_bias, rate_log=w.rate_log)
-        o = ops.seq_delta_scan(vec, cv[:, 2 * GD:], cache.view(self.h_state), st, w.H, w.D, w.E, paired=True)
+        o = ops.seq_delta_rule(ops.DELTA_GATED, cv[:, :GD], cv[:, GD:2 * GD], cv[:, 2 * GD:], dec, pin[:, w.b_off:],
+                               cache.view(self.h_state), st, w.H, w.G, w.D, w.E, dec_bias=w.dt_bias, rate_log=w.rate_log)
         on = ops.seq_head_norm_gate(o, w.norm, w.H, w.E, self.eps, self.act, gate=gate)
         return ops.linear(on, w.w_o, out_dtype=F32)
 
@@ -486,9 +485,9 @@ class ScalarGatedDeltaRule(_OneBranch):
         w = self.w
         GD = w.G * w.D
         cv = ops.seq_conv_act(pin[:, :w.n_conv], w.conv, cache.view(self.h_carry), st, silu=True)
-        vec = ops.seq_delta_prep(ops.DELTA_GATED_SCALAR, cv[:, :GD], cv[:, GD:2 * GD], pin[:, w.a_off:w.a_off + w.H],
-                                 pin[:, w.b_off:w.b_off + w.H], w.H, w.G, w.D, dec_bias=w.dt_bias, rate_log=w.rate_log)
-        o = ops.seq_delta_scan(vec, cv[:, 2 * GD:], cache.view(self.h_state), st, w.H, w.D, w.E, paired=True)
+        o = ops.seq_delta_rule(ops.DELTA_GATED_SCALAR, cv[:, :GD], cv[:, GD:2 * GD], cv[:, 2 * GD:], pin[:, w.a_off:w.a_off + w.H],
+                               pin[:, w.b_off:w.b_off + w.H], cache.view(self.h_state), st, w.H, w.G, w.D, w.E, dec_bias=w.dt_bias,
+                               rate_log=w.rate_log)
         on = ops.seq_head_norm_gate(o, w.norm, w.H, w.E, self.eps, self.act, gate=pin[:, w.g_off:w.n_in], gate_silu=True)
         return ops.linear(on, w.w_o, out_dtype=F32)
 
@@ -873,9 +872,8 @@ class StateSpaceDuality(_OneBranch):
         cv = ops.seq_conv_act(pin[:, inner:inner + w.n_conv], w.conv, cache.view(self.h_carry), st, silu=True,
                               bias=w.conv_b)
         xs, write, read = cv[:, :inner], cv[:, inner:inner + GN], cv[:, inner + GN:]
-        vec = ops.seq_delta_prep(ops.DELTA_STATE_SPACE, read, write, step, None, w.H, w.G, w.N, dec_bias=w.dt_bias,
-                                 rate_log=w.rate_log)
-        o = ops.seq_delta_scan(vec, xs, cache.view(self.h_state), st, w.H, w.N, w.E, correct=False)
+        o = ops.seq_delta_rule(ops.DELTA_STATE_SPACE, read, write, xs, step, None, cache.view(self.h_state), st, w.H, w.G, w.N, w.E,
+                               dec_bias=w.dt_bias, rate_log=w.rate_log)
         y = ops.seq_skip_gate_group_norm(o, xs, w.skip, gate, w.norm, w.H, w.E, w.NG, self.eps, self.act)
         return ops.linear(y, w.w_o, out_dtype=F32)
 

@@ -972,20 +972,35 @@ def seq_delta_prep(rule, q, k, dec, mix, H, G, D, dec_bias=None, rate_log=None, 
     return vec
 
 
-def seq_delta_scan(vec, v, state, st, H, D, E, correct=True, paired=False):
+def seq_delta_scan(vec, v, state, st, H, D, E, correct=True):
     """vec fp32 [n_tok, H, 5, D], v fp32 [n_tok, H*E] (column slice fine), state fp32 [slots, H, D, E] (updated) ->
-    o fp32 [n_tok, H*E]. correct=False: the rule has no correction term (DELTA_STATE_SPACE). paired: the fourth vector is the fifth
-    with its sign changed (DELTA_GATED, DELTA_GATED_SCALAR)."""
+    o fp32 [n_tok, H*E]. correct=False: the rule has no correction term (DELTA_STATE_SPACE)."""
     _req(vec, torch.float32), _req(v, torch.float32), _req(state, torch.float32)
     o = torch.empty((st.n_tok, H * E), device=v.device, dtype=torch.float32)
-    blocks = _scan_blocks(st, H, D, E, correct, (vec, v)) if paired or not correct else None
-    if blocks is not None:
-        ws, n = blocks
-        check(lib().llark_seq_delta_chunks(_p(vec), _p(v), v.stride(0), _p(state), _p(o), _p(ws), n, _p(st.cu), _p(st.slot), st.n_seq,
-                                           st.max_len, H, D, E, int(correct), _stream()), "seq_delta_chunks")
-        return o
     check(lib().llark_seq_delta_scan(_p(vec), _p(v), v.stride(0), _p(state), _p(o), _p(st.cu), _p(st.slot), st.n_seq,
                                      st.n_tok, H, D, E, int(correct), _stream()), "seq_delta_scan")
+    return o
+
+
+def seq_delta_rule(rule, q, k, v, dec, mix, state, st, H, G, D, E, dec_bias=None, rate_log=None, unit_eps=1e-6):
+    """seq_delta_prep and seq_delta_scan in one: o fp32 [n_tok, H*E] from the projections, state updated. Prompts of every rule but
+    DELTA_GENERALIZED take the block walk, which prepares what it needs itself."""
+    correct = rule != DELTA_STATE_SPACE
+    blocks = None
+    if rule != DELTA_GENERALIZED:
+        blocks = _scan_blocks(st, H, D, E, correct, (q, k, v) + ((dec,) if rule == DELTA_GATED else ()))
+    if blocks is None:
+        vec = seq_delta_prep(rule, q, k, dec, mix, H, G, D, dec_bias=dec_bias, rate_log=rate_log, unit_eps=unit_eps)
+        return seq_delta_scan(vec, v, state, st, H, D, E, correct=correct)
+    _req(q, torch.float32), _req(k, torch.float32), _req(v, torch.float32), _req(dec, torch.float32), _req(state, torch.float32)
+    if mix is not None:
+        _req(mix, torch.float32)
+    ws, n = blocks
+    o = torch.empty((st.n_tok, H * E), device=v.device, dtype=torch.float32)
+    check(lib().llark_seq_delta_chunks(int(rule), _p(q), q.stride(0), _p(k), k.stride(0), _p(dec), dec.stride(0), _p(dec_bias),
+                                       _p(rate_log), _p(mix), mix.stride(0) if mix is not None else 0, float(unit_eps), _p(v),
+                                       v.stride(0), _p(state), _p(o), _p(ws), n, _p(st.cu), _p(st.slot), st.n_seq, st.max_len, H, G,
+                                       D, E, _stream()), "seq_delta_chunks")
     return o
 
 

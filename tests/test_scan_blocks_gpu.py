@@ -29,7 +29,7 @@ def _walk(q, d, z, p, v, S, correct):
     return torch.stack(out), S
 
 
-@pytest.mark.parametrize("kind", ["hgrn2", "gated", "plain"])
+@pytest.mark.parametrize("kind", ["hgrn2", "scalar", "channel", "state"])
 @pytest.mark.parametrize("lens,H,D,E,bytes_", [([16], 1, 128, 128, None), ([1, 17, 40], 5, 128, 64, None), ([33, 15, 2], 3, 64, 96, None),
                                                ([200, 70], 2, 128, 128, 1)])
 def test_against_64_bits(kind, lens, H, D, E, bytes_, monkeypatch):
@@ -57,21 +57,31 @@ def test_against_64_bits(kind, lens, H, D, E, bytes_, monkeypatch):
         d = (lo + (1 - lo) * torch.sigmoid(s[:, H * D:2 * H * D])).view(n, H, D)
         z, p, v = None, 1 - d, s[:, 2 * H * D:].reshape(n, H, E)
     else:
-        unit = lambda t: t / t.norm(dim=-1, keepdim=True)  # noqa: E731
-        q, k = unit(torch.randn(n, H, D, device=dev)), unit(torch.randn(n, H, D, device=dev) + 0.5)
-        d, beta = torch.sigmoid(x), torch.rand(n, H, 1, device=dev)
-        v = torch.randn(n, H * E + 4, device=dev)[:, 4:]  # a column slice
-        z, p = (k * d, beta * k) if kind == "gated" else (torch.zeros_like(k), k)
-        vec = torch.stack([q, z, d, -p if kind == "gated" else torch.zeros_like(p), p], dim=2).contiguous()
-        o = ops.seq_delta_scan(vec, v, state, st, H, D, E, correct=kind == "gated", paired=kind == "gated")
+        rule = {"scalar": ops.DELTA_GATED_SCALAR, "channel": ops.DELTA_GATED, "state": ops.DELTA_STATE_SPACE}[kind]
+        G = 1 if H % 2 else H // 2  # heads share keys
+        wide = torch.randn(n, 2 * G * D + H * E + 4, device=dev)  # column slices, as the mixers hand them over
+        q, k, v = wide[:, :G * D], wide[:, G * D:2 * G * D] + 0.3, wide[:, 2 * G * D + 4:]
+        dec = x.reshape(n, -1) if kind == "channel" else x[:, :, 5].contiguous()
+        mix, rate_log, bias = torch.randn(n, H, device=dev), torch.randn(H, device=dev), torch.randn(dec.shape[1], device=dev)
+        args = (rule, q, k, v, dec, None if kind == "state" else mix)
+        o = ops.seq_delta_rule(*args, state, st, H, G, D, E, dec_bias=bias, rate_log=rate_log)
         monkeypatch.setattr(ops, "SCAN_BLOCK_MIN_LEN", 1 << 30)
         old_state = S0.clone()
-        old = ops.seq_delta_scan(vec, v, old_state, st, H, D, E, correct=kind == "gated")
-        q, z, d, p = (t.to(F64) for t in (q, z, d, p))
+        old = ops.seq_delta_rule(*args, old_state, st, H, G, D, E, dec_bias=bias, rate_log=rate_log)
+        q, k = (t.to(F64).reshape(n, G, D).repeat_interleave(H // G, 1) for t in (q, k))
         v = v.to(F64).reshape(n, H, E)
+        step = torch.nn.functional.softplus(dec.to(F64) + bias.to(F64))
+        step = step.view(n, H, D) if kind == "channel" else step[:, :, None]
+        d = torch.exp(-torch.exp(rate_log.to(F64))[:, None] * step).expand(n, H, D)
+        if kind == "state":
+            z, p = None, step * k
+        else:
+            unit = lambda t: t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)  # noqa: E731
+            q, k = unit(q) / D ** 0.5, unit(k)
+            z, p = k * d, torch.sigmoid(mix.to(F64))[:, :, None] * k
     for b, ln in enumerate(lens):
         at = slice(st.cu_host[b], st.cu_host[b] + ln)
-        want, S = _walk(q[at], d[at], z[at] if z is not None else None, p[at], v[at], S0[slots[b]].to(F64), kind == "gated")
+        want, S = _walk(q[at], d[at], z[at] if z is not None else None, p[at], v[at], S0[slots[b]].to(F64), kind in ("scalar", "channel"))
         rel = lambda a, w: ((a.to(F64) - w).norm() / w.norm()).item()  # noqa: E731
         eo, es = rel(o.view(n, H, E)[at], want), rel(state[slots[b]], S)
         # 2^-21 of a product from the split, sums of up to 128 + 16 of them: 2e-6 of the terms' norm at most
