@@ -72,6 +72,8 @@ class FlatBuckets:
             view = self.params[o:o + k].view(p.shape)
             view.copy_(p.data)  # converts when cast_to_bf16 admitted another storage dtype
             p.data = view
+        self._views = {}  # fused views asked for before: (name, shape, span) -> view of params
+        self._order = None  # the parameters in module order, as is_same() saw them last
         self.grads_attached = False
         # set by the fused optimizer step: the bucket's contents have been consumed, so the next backward
         # OVERWRITES instead of accumulating (saves zeroing 13 GB per optimizer step)
@@ -87,8 +89,39 @@ class FlatBuckets:
                 return False
         return True
 
+    @staticmethod
+    def _walk(module):
+        """(module's name in its parent, parameter's name, parameter) of the whole tree."""
+        found, seen, stack = [], set(), [("", module)]
+        while stack:
+            name, m = stack.pop()
+            if m in seen:
+                continue
+            seen.add(m)
+            found.extend((name, k, p) for k, p in m._parameters.items() if p is not None)
+            stack.extend(c for c in m._modules.items() if c[1] is not None)
+        return found
+
+    def note_order(self, module):
+        self._order = [(n, k, p, p.requires_grad, p.data_ptr(), p.shape, p.dtype) for n, k, p in self._walk(module)]
+
+    def is_same(self, module):
+        """Whether `module` holds the very parameters that is_current() accepted last, under their names, where and as they
+        were: one walk over the tree (named_parameters() puts every full name together: most of a small decode step)."""
+        found = self._walk(module)
+        return (self._order is not None and len(found) == len(self._order)
+                and all(p is q and n == m and k == l and p.requires_grad == r and p.data_ptr() == a and p.shape == s and p.dtype == t
+                        for (n, k, p), (m, l, q, r, a, s, t) in zip(found, self._order)))
+
     def pview(self, name, shape=None, span=1):
         """View of `span` consecutive parameters starting at `name` (fused q|k|v, gate|up)."""
+        key = (name, shape, span)
+        t = self._views.get(key)
+        if t is None:
+            t = self._views[key] = self._pview(name, shape, span)
+        return t
+
+    def _pview(self, name, shape, span):
         o, k = self.offsets[name]
         if span == 1:
             t = self.params[o:o + k]
@@ -202,6 +235,13 @@ class LlamaEngine:
         return [(n, p) for n, p in self.lm.named_parameters()]
 
     def ensure_packed(self):
+        if self.flat is not None and self.flat.is_same(self.lm):
+            return self.flat
+        flat = self._ensure_packed()
+        flat.note_order(self.lm)
+        return flat
+
+    def _ensure_packed(self):
         named = self._named()
         dev = named[0][1].device
         if dev.type != "cuda":
@@ -449,9 +489,6 @@ class LlamaEngine:
         cos_t, sin_t = cos[t:], sin[t:]  # row 0 of these views is position t: with S = 1 every row reads it
         cache.lens.fill_(t + 1)
         rstd = torch.empty(B, device=dev, dtype=torch.float32)
-        # up to 8 rows the linears are weight-streaming GEMVs (csrc/gemv.cu); LLARK_DECODE_GEMV=0 keeps the GEMM core
-        skinny = B <= 8 and os.environ.get("LLARK_DECODE_GEMV", "1") != "0"
-        lin = ops.gemv if skinny else ops.gemm
         for l in range(L):
             pfx = f"model.layers.{l}."
             Wqkv = flat.pview(pfx + "self_attn.q_proj.weight", (3 * H, H), span=3)
@@ -459,23 +496,23 @@ class LlamaEngine:
             Wgu = flat.pview(pfx + "mlp.gate_proj.weight", (2 * I, H), span=2)
             Wd = flat.pview(pfx + "mlp.down_proj.weight", (H, I))
             xn1 = ops.rmsnorm_fwd(x, flat.pview(pfx + "input_layernorm.weight"), eps, rstd=rstd)
-            if self.fuse_epilogues and D == 128 and not skinny:
+            if self.fuse_epilogues and D == 128:
                 qkv = ops.gemm(xn1, Wqkv, rope=(cos_t, sin_t, 1, 2 * H))
             else:
-                qkv = lin(xn1, Wqkv)
+                qkv = ops.gemm(xn1, Wqkv)
                 ops.rope_(qkv, cos_t, sin_t, 1, NH, D)
             cache.k[l][:, t].copy_(qkv[:, H:2 * H])
             cache.v[l][:, t].copy_(qkv[:, 2 * H:])
             attn = ops.attn_decode(qkv[:, :H].contiguous(), cache.k[l], cache.v[l], cache.lens, NH, D)
-            x_mid = lin(attn, Wo, residual=x)
+            x_mid = ops.gemm(attn, Wo, residual=x)
             xn2 = ops.rmsnorm_fwd(x_mid, flat.pview(pfx + "post_attention_layernorm.weight"), eps, rstd=rstd)
-            gu = lin(xn2, Wgu)
+            gu = ops.gemm(xn2, Wgu)
             act = ops.swiglu_fwd(gu)
-            x = lin(act, Wd, residual=x_mid)
+            x = ops.gemm(act, Wd, residual=x_mid)
         hn = ops.rmsnorm_fwd(x, flat.pview("model.norm.weight"), eps, rstd=rstd)
         ldv = (V + 63) // 64 * 64
         logits_buf = torch.empty((B, ldv), device=dev, dtype=BF16)
-        lin(hn, flat.pview("lm_head.weight", (V, H)), out=logits_buf, N=V)
+        ops.gemm(hn, flat.pview("lm_head.weight", (V, H)), out=logits_buf, N=V)
         cache.length = t + 1
         return logits_buf.view(B, 1, ldv)[:, :, :V]
 

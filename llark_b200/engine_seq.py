@@ -4,9 +4,21 @@ the same kernels with other numbers -- and returns fp32 logits for the rows that
 subclasses this and says how tokens become the residual stream (`_embed`), what its layers do to it (`_run_layers`) and
 how wanted rows become logits (`_logits`); slot handling, the step descriptor, validation and the order of things are
 here. The engine is host-side orchestration only, like LlamaEngine: every FLOP is a C-ABI call."""
+import numpy as np
 import torch
 
 F32 = torch.float32
+
+
+def _flat(tokens):
+    """The token ids of all requests in one integer array."""
+    try:
+        parts = [np.array(t, dtype=np.int64) for t in tokens]
+        if all(p.ndim == 1 for p in parts):
+            return np.concatenate(parts)
+    except (TypeError, ValueError, OverflowError, RuntimeError):
+        pass  # ids that numpy does not take as they are
+    return np.array([int(t) for ts in tokens for t in ts], dtype=object)
 
 
 class LayerListEngine:
@@ -43,29 +55,34 @@ class LayerListEngine:
         one of each). Returns fp32 logits [n_wanted, vocab] in the order of the requests and of `want` (None when nothing
         is wanted). The caches advance by the step's tokens."""
         lens = [len(t) for t in tokens]
-        st = cache.layout(slots, lens)
+        cache.check(slots)
+        if not lens or min(lens) <= 0:
+            raise ValueError("a step needs at least one token for every request in it")
         if self.max_positions is not None:
             for s, n in zip(slots, lens):
                 if cache.length[s] + n > self.max_positions:
                     raise ValueError("a request grows past max_positions")
         cache.reserve_positions(max(cache.length[s] + n for s, n in zip(slots, lens)))  # per-position stores grow first
-        flat = [int(t) for ts in tokens for t in ts]
-        if flat and (min(flat) < 0 or max(flat) >= self.cfg.vocab):
+        flat = _flat(tokens)
+        if flat.min() < 0 or flat.max() >= self.cfg.vocab:
             raise ValueError("token id outside the vocabulary")
-        ids = torch.tensor(flat, dtype=torch.int32).to(self.device, non_blocking=True)
         if want is None:
             want = [[n - 1] for n in lens]
-        for b, w in enumerate(want):
-            if any(k < 0 or k >= lens[b] for k in w):
-                raise ValueError("a wanted place lies outside the request's tokens")
-        rows = [st.cu_host[b] + int(k) for b, w in enumerate(want) for k in w]
+        rows, first = [], 0
+        for n, w in zip(lens, want):
+            for k in w:
+                if k < 0 or k >= n:
+                    raise ValueError("a wanted place lies outside the request's tokens")
+                rows.append(first + int(k))
+            first += n
+        st = cache.layout(slots, lens, extra=(flat, rows))
+        ids, idx = st.extra
         x = self._embed(ids, st)
         residuals = [] if return_residuals else None
         x = self._run_layers(cache, x, st, residuals)
         cache.advance(slots, lens)
         logits = None
         if rows:
-            idx = torch.tensor(rows, dtype=torch.int32).to(self.device, non_blocking=True)
             logits = self._logits(x, idx)
         if return_residuals:
             return logits, residuals

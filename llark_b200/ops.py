@@ -32,11 +32,15 @@ def init():
 
 
 def _p(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
+
+
+_raw_stream, _device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The handle of the current device's current stream (torch.cuda.current_stream() asks for much more on its way: 15 us)."""
+    return _raw_stream(_device())
 
 
 def _req(t, dtype=None):
@@ -108,7 +112,8 @@ def gemm(a, b, *, a_mn=False, b_mn=False, M=None, N=None, K=None, out=None, out_
         rc = lib().llark_gemm_ex(_p(a), int(a_mn), lda, _p(b), int(b_mn), ldb, _p(out), ldc, int(c_fp32), _p(bias),
                                  int(bias_fp32), _p(residual), ldr, M, N, K, int(in_fp32), max_ctas, ctypes.byref(ep),
                                  _stream())
-    check(rc, f"llark_gemm(M={M},N={N},K={K})")
+    if rc:
+        check(rc, f"llark_gemm(M={M},N={N},K={K})")
     if prof is not None:
         e1.record()
         prof.append((e0, e1, 2.0 * M * N * K, (M, N, K, int(a_mn), int(b_mn))))
@@ -502,8 +507,8 @@ def linear(a, w, bias=None, out_dtype=None, out=None, act=None, act_limit=0.0, a
         raise TypeError("linear: activation and weight dtypes differ")
     in_fp32 = _actf(a.dtype)
     M, K = a.shape
-    N = w.shape[0]
-    if w.shape[1] != K:
+    N, Kw = w.shape
+    if Kw != K:
         raise ValueError("linear: inner sizes differ")
     code = LINEAR_ACTS[act]
     paired = act in PAIRED_ACTS
@@ -514,23 +519,22 @@ def linear(a, w, bias=None, out_dtype=None, out=None, act=None, act_limit=0.0, a
     c_fp32 = _actf(out.dtype)
     if bias is not None:
         _req(bias, torch.float32)
-    vec = 4 if c_fp32 else 8
-    rows = (M <= LINEAR_ROWS_MAX and in_fp32) or (M <= LINEAR_FEW_MAX and not in_fp32 and K % 8 == 0 and a.stride(0) % 8 == 0
-                                                  and w.stride(0) % 8 == 0 and (a.data_ptr() | w.data_ptr()) % 16 == 0)
-    tc = (not rows and not in_fp32 and not (c_fp32 and paired) and K >= 64 and N >= 64 and K % 8 == 0 and a.stride(0) % 8 == 0
-          and w.stride(0) % 8 == 0 and out.stride(0) % vec == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
-          and out.data_ptr() % 16 == 0)
+    lda, ldw, ldc, pa, pw, pc = a.stride(0), w.stride(0), out.stride(0), a.data_ptr(), w.data_ptr(), out.data_ptr()
+    pieces = not (K | lda | ldw) % 8 and not (pa | pw) % 16  # rows in 16-byte pieces
+    rows = (M <= LINEAR_FEW_MAX and pieces) if not in_fp32 else M <= LINEAR_ROWS_MAX
+    tc = (not rows and not in_fp32 and not (c_fp32 and paired) and K >= 64 and N >= 64 and pieces and not ldc % (4 if c_fp32 else 8)
+          and not pc % 16)
     if rows or (M <= LINEAR_ROWS_MAX and not tc):
         LINEAR_STATS["rows"] += 1
-        check(lib().llark_linear_rows(_p(a), a.stride(0), _p(w), w.stride(0), _p(out), out.stride(0), c_fp32, _p(bias),
-                                      M, N, K, in_fp32, code, float(act_limit), float(act_slope), _stream()), "linear_rows")
+        check(lib().llark_linear_rows(pa, lda, pw, ldw, pc, ldc, c_fp32, _p(bias), M, N, K, in_fp32, code, float(act_limit),
+                                      float(act_slope), _stream()), "linear_rows")
     elif tc:
         LINEAR_STATS["tcgen05"] += 1
         gemm(a, w, bias=bias, out=out, M=M, N=N, K=K, act=act, act_limit=act_limit, act_slope=act_slope)
     else:
         LINEAR_STATS["simt"] += 1
-        check(lib().llark_linear_simt(_p(a), a.stride(0), _p(w), w.stride(0), _p(out), out.stride(0), c_fp32, _p(bias),
-                                      M, N, K, in_fp32, code, float(act_limit), float(act_slope), _stream()), "linear_simt")
+        check(lib().llark_linear_simt(pa, lda, pw, ldw, pc, ldc, c_fp32, _p(bias), M, N, K, in_fp32, code, float(act_limit),
+                                      float(act_slope), _stream()), "linear_simt")
     return out
 
 

@@ -14,37 +14,44 @@ kept in place.
 Sized for one B200: a ring is min(window, max_positions) entries per slot whatever the sequence length; a recurrent
 state is heads x dim x vdim fp32 per slot.
 """
+import numpy as np
 import torch
 
 
 class StepLayout:
     """One packed step on the device: request b brings lens[b] tokens that start at position pos0[b] of its sequence and
-    owns slot slots[b]. tok_seq[t] = request of row t; cu[b] = first row of request b. One pinned host buffer, one copy."""
+    owns slot slots[b]. tok_seq[t] = request of row t; cu[b] = first row of request b. One pinned host buffer, one copy, which
+    takes the integers of `extra` along (self.extra: their int32 tensors on the device)."""
 
-    def __init__(self, lens, pos0, slots, device):
+    def __init__(self, lens, pos0, slots, device, extra=()):
         n_seq = len(lens)
         n_tok = int(sum(lens))
         if n_seq == 0 or min(lens) <= 0:
             raise ValueError("a step needs at least one token for every request in it")
-        host = torch.empty(n_tok + 4 * n_seq + 1, dtype=torch.int32, pin_memory=torch.device(device).type == "cuda")
+        sizes = [len(e) for e in extra]
+        host = torch.empty(n_tok + 4 * n_seq + 1 + sum(sizes), dtype=torch.int32, pin_memory=torch.device(device).type == "cuda")
+        a = host.numpy()
         cu = [0]
         for n in lens:
             cu.append(cu[-1] + int(n))
-        seq = []
-        for b, n in enumerate(lens):
-            seq.extend([b] * int(n))
-        host[:n_tok] = torch.tensor(seq, dtype=torch.int32)
-        host[n_tok:n_tok + n_seq + 1] = torch.tensor(cu, dtype=torch.int32)
-        host[n_tok + n_seq + 1:n_tok + 2 * n_seq + 1] = torch.tensor([int(p) for p in pos0], dtype=torch.int32)
-        host[n_tok + 2 * n_seq + 1:n_tok + 3 * n_seq + 1] = torch.tensor([int(s) for s in slots], dtype=torch.int32)
-        host[n_tok + 3 * n_seq + 1:] = torch.tensor([int(n) for n in lens], dtype=torch.int32)
+        a[:n_tok] = np.arange(n_seq) if n_tok == n_seq else np.repeat(np.arange(n_seq), lens)
+        at = n_tok + 4 * n_seq + 1
+        a[n_tok:at] = cu + [int(p) for p in pos0] + [int(s) for s in slots] + [int(n) for n in lens]
+        for e, n in zip(extra, sizes):
+            a[at:at + n] = e
+            at += n
         dev = host.to(device, non_blocking=True)
+        at = n_tok + 4 * n_seq + 1
+        self.extra = []
+        for n in sizes:
+            self.extra.append(dev[at:at + n])
+            at += n
         self._host = host  # keeps the pinned buffer alive until the copy has run
         self.tok_seq = dev[:n_tok]
         self.cu = dev[n_tok:n_tok + n_seq + 1]
         self.pos0 = dev[n_tok + n_seq + 1:n_tok + 2 * n_seq + 1]
         self.slot = dev[n_tok + 2 * n_seq + 1:n_tok + 3 * n_seq + 1]
-        self.lens_dev = dev[n_tok + 3 * n_seq + 1:]
+        self.lens_dev = dev[n_tok + 3 * n_seq + 1:n_tok + 4 * n_seq + 1]
         self.device, self.slots_host, self._chunks = device, [int(s) for s in slots], {}
         self.tables = {}  # what ops computed once for this step (rotary cosines and sines by frequencies)
         self.n_tok, self.n_seq = n_tok, n_seq
@@ -189,14 +196,17 @@ class StateCache:
     def tokens_held(self):
         return sum(self.length.values())
 
-    def layout(self, slots, lens):
-        """StepLayout for requests `slots` bringing `lens` new tokens each; positions continue where each stopped."""
+    def check(self, slots):
         for s in slots:
             if s not in self.length:
                 raise KeyError(f"slot {s} is not in use")
         if len(set(slots)) != len(slots):
             raise ValueError("a request can appear once in a step")
-        return StepLayout(lens, [self.length[s] for s in slots], slots, self.device)
+
+    def layout(self, slots, lens, extra=()):
+        """StepLayout for requests `slots` bringing `lens` new tokens each; positions continue where each stopped."""
+        self.check(slots)
+        return StepLayout(lens, [self.length[s] for s in slots], slots, self.device, extra)
 
     def advance(self, slots, lens):
         for s, n in zip(slots, lens):
