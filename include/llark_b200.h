@@ -60,12 +60,14 @@ int llark_gemm(const void* A, int a_mn_major, long long lda, const void* B, int 
  *                         z = acc + bias, rounded once
  *   LLARK_EPI_CLAMP_GLU   the same with C[:, c] = g * sigmoid(f1 * g) * (u + 1), g = min(z[:, 2c], f0), u = z[:, 2c + 1]
  *                         clamped to -f0 .. f0 */
+/*   LLARK_EPI_SWIGLU      few rows only (M <= 64, bf16): the first half of B's rows are gates, the second ups, C bf16 [M, N / 2] =
+ *                         silu(gate) * up with every step rounded as llark_gemm and llark_swiglu_fwd round it */
 /*   LLARK_EPI_SEGMENTS    not an epilogue: the rows of A / C come in runs that each multiply their own block of B (stacked
  *                         [i1, N, K]); a = device int triples (block, first row, rows <= 256), i0 = their number (an upper
  *                         bound when b points at a device word with the real number), ld = LLARK_EPI_NONE,
  *                         LLARK_EPI_RELU2 or LLARK_EPI_CLAMP_GLU. Used by llark_gemm_segments. */
 enum { LLARK_EPI_NONE = 0, LLARK_EPI_QUICK_GELU = 1, LLARK_EPI_ROPE = 2, LLARK_EPI_SWIGLU_BWD = 3, LLARK_EPI_SEGMENTS = 4,
-       LLARK_EPI_RELU2 = 5, LLARK_EPI_RELU_GLU = 6, LLARK_EPI_CLAMP_GLU = 7 };
+       LLARK_EPI_RELU2 = 5, LLARK_EPI_RELU_GLU = 6, LLARK_EPI_CLAMP_GLU = 7, LLARK_EPI_SWIGLU = 8 };
 typedef struct LlarkGemmEpilogue {
     int kind;
     const void* a;
@@ -165,6 +167,10 @@ int llark_gemv(const void* A, long long lda, const void* W, long long ldw, void*
  * valid cached positions per row including the new token (<= s_max <= 4096), out [B, n_heads*128]. */
 int llark_attn_decode(const void* q, const void* k_cache, const void* v_cache, const int* lens, void* out, int B,
                       int s_max, int n_heads, int head_dim, float scale, cudaStream_t stream);
+/* The same for rows that all stand at position pos, straight from the packed projection: qkv [B, ld] = q | k | v (RoPE applied). The
+ * new key and value are taken from there and stored as entry pos of k_cache / v_cache [B, s_max, n_heads*128] by the same launch. */
+int llark_attn_decode_packed(const void* qkv, long long ld, void* k_cache, void* v_cache, int pos, void* out, int B, int s_max,
+                             int n_heads, int head_dim, float scale, cudaStream_t stream);
 long long llark_attn_bwd_workspace(int B, int S, int n_heads);
 int llark_attn_bwd(const void* qkv, const unsigned char* key_mask, const void* out, const void* dout, const float* lse,
                    void* dqkv, int B, int S, int n_heads, int head_dim, float scale, void* workspace,

@@ -38,7 +38,7 @@ SYMBOLS = [
     "llark_last_cuda_error", "llark_gemm", "llark_gemm_ex", "llark_gemm_clear_cache", "llark_gemm_set_mode", "llark_gemm_get_mode", "llark_splice_scan", "llark_embed_splice_fwd",
     "llark_embed_splice_bwd", "llark_cast_f32_to_bf16", "llark_cast_bf16_to_f32", "llark_rmsnorm_fwd",
     "llark_rmsnorm_bwd_workspace", "llark_rmsnorm_bwd", "llark_rope", "llark_swiglu_fwd", "llark_swiglu_bwd",
-    "llark_attn_fwd", "llark_attn_decode", "llark_gemv", "llark_attn_alibi_fwd", "llark_attn_alibi_bwd", "llark_ln_fwd",
+    "llark_attn_fwd", "llark_attn_decode", "llark_attn_decode_packed", "llark_gemv", "llark_attn_alibi_fwd", "llark_attn_alibi_bwd", "llark_ln_fwd",
     "llark_ln_bwd_workspace", "llark_ln_bwd", "llark_gelu_fwd", "llark_gelu_bwd", "llark_attn_bwd_workspace", "llark_attn_bwd", "llark_ce_fwd", "llark_ce_bwd",
     "llark_sumsq_workspace", "llark_grad_sumsq", "llark_adamw_step", "llark_comm_unique_id", "llark_comm_init",
     "llark_comm_destroy", "llark_grad_bucket_allreduce", "llark_jb_conv_down", "llark_jb_resblock",
@@ -58,7 +58,7 @@ class GemmEpilogue(ctypes.Structure):
                 ("i0", ctypes.c_int), ("i1", ctypes.c_int), ("f0", ctypes.c_float), ("f1", ctypes.c_float)]
 
 
-EPI_NONE, EPI_QUICK_GELU, EPI_ROPE, EPI_SWIGLU_BWD, EPI_RELU2, EPI_RELU_GLU, EPI_CLAMP_GLU = 0, 1, 2, 3, 5, 6, 7
+EPI_NONE, EPI_QUICK_GELU, EPI_ROPE, EPI_SWIGLU_BWD, EPI_RELU2, EPI_RELU_GLU, EPI_CLAMP_GLU, EPI_SWIGLU = 0, 1, 2, 3, 5, 6, 7, 8
 
 
 class LlarkError(RuntimeError):
@@ -102,6 +102,7 @@ def lib():
             "llark_swiglu_bwd": ([P, P, P, LL, I, P], I),
             "llark_attn_fwd": ([P, P, P, P, I, I, I, I, F, P], I),
             "llark_attn_decode": ([P, P, P, P, P, I, I, I, I, F, P], I),
+            "llark_attn_decode_packed": ([P, LL, P, P, I, P, I, I, I, I, F, P], I),
             "llark_gemv": ([P, LL, P, LL, P, LL, P, P, LL, I, I, I, P], I),
             "llark_attn_alibi_fwd": ([P, P, P, P, P, I, I, I, I, F, P], I),
             "llark_attn_alibi_bwd": ([P, P, P, P, P, P, P, I, I, I, I, F, P, P], I),

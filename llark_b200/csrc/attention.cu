@@ -660,6 +660,25 @@ extern "C" int llark_attn_decode(const void* q, const void* k_cache, const void*
     return check_launch2();
 }
 
+extern "C" int llark_attn_decode_packed(const void* qkv, long long ld, void* k_cache, void* v_cache, int pos, void* out, int B,
+                                        int s_max, int n_heads, int head_dim, float scale, cudaStream_t st) {
+    if (head_dim != HD || B <= 0 || n_heads <= 0 || pos < 0 || pos >= s_max || !qkv || !k_cache || !v_cache || !out || ld % 8 ||
+        ld < 3LL * n_heads * HD || !attnstep::fits(B, n_heads, n_heads, HD, qkv, k_cache, v_cache))
+        return LLARK_EINVAL;
+    attnstep::Args a = {};
+    a.k = a.k_new = (__nv_bfloat16*)k_cache, a.v = a.v_new = (__nv_bfloat16*)v_cache;
+    a.packed = (const __nv_bfloat16*)qkv, a.packed_ld = ld, a.n_keys = pos + 1;
+    a.out = (__nv_bfloat16*)out, a.out_ld = (long long)n_heads * HD;
+    a.B = B, a.H = a.G = n_heads, a.D = HD;
+    a.cap = s_max, a.scale = scale, a.out_scale = 1.f;
+    cudaError_t e = attnstep::launch(a, st);
+    if (e != cudaSuccess) {
+        g_last_cuda_error = (int)e;
+        return LLARK_ECUDA;
+    }
+    return LLARK_OK;
+}
+
 extern "C" int llark_attn_fwd(const void* qkv, const unsigned char* key_mask, void* out, float* lse, int B, int S,
                               int n_heads, int head_dim, float scale, cudaStream_t st) {
     if (head_dim != HD || B <= 0 || S <= 0 || n_heads <= 0) return LLARK_EINVAL;

@@ -53,6 +53,9 @@ attn_step_kernel(const Args p, int cs) {
     if (p.lens) {
         nkeys = p.lens[b] < p.cap ? p.lens[b] : p.cap;
         base = (long long)b * p.cap;
+    } else if (p.packed) {
+        nkeys = p.n_keys;
+        base = (long long)b * p.cap;
     } else {
         const int r = p.tok_seq[b];
         pos = (long long)p.pos0[r] + (b - p.cu[r]);
@@ -64,12 +67,22 @@ attn_step_kernel(const Args p, int cs) {
     const long long ld = (long long)p.G * D;
     const bf16_t* kb = p.k + base * ld + kvh * D;
     const bf16_t* vb = p.v + base * ld + kvh * D;
+    const bf16_t* qrow = p.packed ? p.packed + b * p.packed_ld + h0 * D : p.q + ((long long)b * p.H + h0) * D;
+    if (p.packed && rank == cs - 1) {  // the CTA that reads the last key stores the new one first (every query head has a key head)
+        if (threadIdx.x < D / 4) {
+            const int i = threadIdx.x % (D / 8) * 8;
+            const bool second = threadIdx.x >= D / 8;
+            *reinterpret_cast<uint4*>((second ? p.v_new : p.k_new) + (base + nkeys - 1) * ld + kvh * D + i) =
+                *reinterpret_cast<const uint4*>(qrow + (second ? 2 : 1) * p.H * D + i);
+        }
+        __syncthreads();
+    }
     // ---- queries: head g of the group, the pieces that this thread's key pieces meet
     uint4 qf[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
         qf[c] = make_uint4(0, 0, 0, 0);
-        if (g < HG) qf[c] = *reinterpret_cast<const uint4*>(p.q + ((long long)b * p.H + h0 + g) * D + c * 32 + t * 8);
+        if (g < HG) qf[c] = *reinterpret_cast<const uint4*>(qrow + g * D + c * 32 + t * 8);
     }
     // this thread's two heads (columns 2 t, 2 t + 1 of the scores)
     float sc[2] = {0.f, 0.f};

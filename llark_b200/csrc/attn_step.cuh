@@ -14,6 +14,13 @@ struct Args {
     // r = tok_seq[b] at position p = pos0[r] + b - cu[r], sees lo .. p with lo = max(0, p - window + 1), or the start of p's block
     // of `chunk` positions, and position j is entry slot[r] * cap + j % cap.
     const int *lens, *tok_seq, *cu, *pos0, *slot;
+    // packed given (with neither lens nor tok_seq; G = H): row b of packed [B, packed_ld] holds q | k | v of the new token, which is
+    // entry n_keys - 1 of every row's cap entries: its key and value are stored there (k_new, v_new are k and v, to be written)
+    // before they are read. q is then not used.
+    const __nv_bfloat16* packed;
+    long long packed_ld;
+    __nv_bfloat16 *k_new, *v_new;
+    int n_keys;
     int cap, window, chunk;
     const float* scale_h;  // [H], or NULL: scale
     float scale, softcap, out_scale;

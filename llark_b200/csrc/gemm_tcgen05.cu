@@ -1236,6 +1236,11 @@ extern "C" int llark_gemm_ex(const void* A, int a_mn_major, long long lda, const
             case LLARK_EPI_RELU2:
                 if (R || a_mn_major || b_mn_major || in_fp32) return LLARK_EINVAL;
                 break;
+            case LLARK_EPI_SWIGLU:
+                if (R || bias || c_fp32 || (N % 2) || ldc < N / 2 || M > skinny::kMaxRows || a_mn_major || b_mn_major || in_fp32 || max_ctas ||
+                    !skinny::fits(A, lda, B, ldb, K))
+                    return LLARK_EINVAL;
+                break;
             case LLARK_EPI_RELU_GLU:
             case LLARK_EPI_CLAMP_GLU:
                 if (R || a_mn_major || b_mn_major || in_fp32 || c_fp32 || (N % 2) || ldc < N / 2) return LLARK_EINVAL;
@@ -1258,7 +1263,7 @@ extern "C" int llark_gemm_ex(const void* A, int a_mn_major, long long lda, const
     // Few rows: 256-row tiles would be mostly padding and, for the widths of one layer, occupy 16 to 86 of the 148 SMs; the
     // product is a stream of B instead.
     if (M <= skinny::kMaxRows && !a_mn_major && !b_mn_major && !in_fp32 && max_ctas == 0 &&
-        (!ep || ep->kind == LLARK_EPI_NONE || ep->kind == LLARK_EPI_ROPE) && skinny::fits(A, lda, B, ldb, K)) {
+        (!ep || ep->kind == LLARK_EPI_NONE || ep->kind == LLARK_EPI_ROPE || ep->kind == LLARK_EPI_SWIGLU) && skinny::fits(A, lda, B, ldb, K)) {
         skinny::Args a = {};
         a.A = (const __nv_bfloat16*)A, a.lda = lda, a.W = (const __nv_bfloat16*)B, a.ldw = ldb;
         a.C = C, a.ldc = ldc, a.c_fp32 = c_fp32, a.bias = bias, a.bias_fp32 = bias_fp32, a.R = R, a.ldr = ldr;
@@ -1268,6 +1273,7 @@ extern "C" int llark_gemm_ex(const void* A, int a_mn_major, long long lda, const
             a.rope_cos = (const __nv_bfloat16*)ep->a, a.rope_sin = (const __nv_bfloat16*)ep->b;
             a.rope_S = ep->i0, a.rope_cols = ep->i1;
         }
+        if (ep && ep->kind == LLARK_EPI_SWIGLU) a.act = skinny::kActSwiglu;
         cudaError_t e = skinny::launch(a, stream);
         if (e != cudaSuccess) {
             g_last_cuda_error = (int)e;

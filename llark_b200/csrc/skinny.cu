@@ -38,6 +38,9 @@ __device__ __forceinline__ void mma16(float (&c)[4], const uint32_t (&a)[4], uin
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// gate rows in the first half of W, up rows in the second
+__host__ __device__ __forceinline__ bool gate_up(const Args& p) { return p.act == kActSiluGlu || p.act == kActSwiglu; }
+
 // byte offset of 16-byte piece c of row r in a slice
 __device__ __forceinline__ uint32_t piece(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
 
@@ -95,7 +98,7 @@ __device__ __forceinline__ void store4(bf16_t* C, const float (&v)[4], bool vec,
 // u + ROWS / 2.
 template <typename TC, bool GROUPED, int ROWS, int PITCH>
 __device__ __forceinline__ void epilogue(const Args& p, const float* red, int M, int row0, int base, int cs, int rank) {
-    const bool adjacent = p.act == kActReluGlu || p.act == kActClampGlu, halves = p.act == kActSiluGlu, rope = p.act == kActRope;
+    const bool adjacent = p.act == kActReluGlu || p.act == kActClampGlu, halves = gate_up(p), rope = p.act == kActRope;
     const bool two = adjacent || halves || rope;
     const int quads = (two ? ROWS / 8 : ROWS / 4) / cs, q0 = rank * quads;
     const int n_out = adjacent || halves ? p.N >> 1 : p.N;
@@ -178,6 +181,9 @@ __device__ __forceinline__ void epilogue(const Args& p, const float* red, int M,
         for (int e = 0; e < 4; ++e) {
             if (p.act == kActReluGlu) {
                 x[e] = fmaxf(x[e], 0.f) * y[e];
+            } else if (p.act == kActSwiglu) {  // the rounding steps of the product and of the op behind it
+                const float gr = bf16_round(x[e]);
+                x[e] = bf16_round(__fdividef(gr, 1.f + __expf(-gr))) * bf16_round(y[e]);
             } else if (p.act == kActSiluGlu) {
                 x[e] = x[e] * (1.0f / (1.0f + expf(-x[e]))) * y[e];
             } else {
@@ -195,7 +201,7 @@ template <int ROWS>
 __device__ __forceinline__ void tile_rows(const Args& p, int tile, int& base, int& gap) {
     base = tile * ROWS;
     gap = 0;
-    if (p.act == kActSiluGlu) {
+    if (gate_up(p)) {
         base = tile * (ROWS / 2);
         gap = (p.N >> 1) - ROWS / 2;
     } else if (p.act == kActRope && ROWS == 64) {
@@ -205,7 +211,7 @@ __device__ __forceinline__ void tile_rows(const Args& p, int tile, int& base, in
 }
 template <int ROWS>
 __device__ __forceinline__ bool row_live(const Args& p, int base, int gap, int i) {
-    return p.act == kActSiluGlu ? base + (i & (ROWS / 2 - 1)) < (p.N >> 1) : base + i + (i >= ROWS / 2 ? gap : 0) < p.N;
+    return gate_up(p) ? base + (i & (ROWS / 2 - 1)) < (p.N >> 1) : base + i + (i >= ROWS / 2 ? gap : 0) < p.N;
 }
 
 // ------------------------------------------------------------------------------------------------ up to eight tokens
@@ -455,7 +461,7 @@ cudaError_t launch(const Args& a, cudaStream_t st) {
     // times as exact. Routed experts have 0 to 64 tokens per tile, known only on the device.
     const bool tc = grouped || a.M > 8;
     const int rows = tc ? TN : BN;
-    const int tiles = a.act == kActSiluGlu ? (a.N / 2 + rows / 2 - 1) / (rows / 2) : (a.N + rows - 1) / rows;
+    const int tiles = gate_up(a) ? (a.N / 2 + rows / 2 - 1) / (rows / 2) : (a.N + rows - 1) / rows;
     // Cut along K until the grid holds as many CTAs as are resident at once (four or two for each of the 148 SMs), as long as a
     // CTA keeps four slices of K.
     const int nch = (a.K + BK - 1) / BK;

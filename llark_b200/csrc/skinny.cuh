@@ -8,7 +8,7 @@ namespace skinny {
 
 constexpr int kMaxRows = 64;
 
-enum { kActNone = 0, kActRelu2, kActReluGlu, kActClampGlu, kActSiluGlu, kActRope };
+enum { kActNone = 0, kActRelu2, kActReluGlu, kActClampGlu, kActSiluGlu, kActRope, kActSwiglu };
 
 struct Args {
     const __nv_bfloat16 *A, *W;
@@ -20,7 +20,7 @@ struct Args {
     int bias_fp32;
     const void* R;     // residual of C's type, or NULL
     long long ldr;
-    int M, N, K;       // N: rows of W (kActSiluGlu: gate rows, then as many up rows: N counts both)
+    int M, N, K;       // N: rows of W (kActSiluGlu, kActSwiglu: gate rows, then as many up rows: N counts both)
     int act;
     float limit, slope;
     // kActRope: columns below rope_cols are rotated per 128-wide head, position = row % rope_S

@@ -488,6 +488,7 @@ class LlamaEngine:
         cos, sin = self._tables(cache.s_max, dev)
         cos_t, sin_t = cos[t:], sin[t:]  # row 0 of these views is position t: with S = 1 every row reads it
         cache.lens.fill_(t + 1)
+        few = B <= ops.LINEAR_FEW_MAX and H % 8 == 0 and I % 8 == 0
         rstd = torch.empty(B, device=dev, dtype=torch.float32)
         for l in range(L):
             pfx = f"model.layers.{l}."
@@ -501,13 +502,10 @@ class LlamaEngine:
             else:
                 qkv = ops.gemm(xn1, Wqkv)
                 ops.rope_(qkv, cos_t, sin_t, 1, NH, D)
-            cache.k[l][:, t].copy_(qkv[:, H:2 * H])
-            cache.v[l][:, t].copy_(qkv[:, 2 * H:])
-            attn = ops.attn_decode(qkv[:, :H].contiguous(), cache.k[l], cache.v[l], cache.lens, NH, D)
+            attn = ops.attn_decode_packed(qkv, cache.k[l], cache.v[l], t, NH, D)  # stores the new keys and values too
             x_mid = ops.gemm(attn, Wo, residual=x)
             xn2 = ops.rmsnorm_fwd(x_mid, flat.pview(pfx + "post_attention_layernorm.weight"), eps, rstd=rstd)
-            gu = ops.gemm(xn2, Wgu)
-            act = ops.swiglu_fwd(gu)
+            act = ops.gemm(xn2, Wgu, swiglu=True) if few else ops.swiglu_fwd(ops.gemm(xn2, Wgu))
             x = ops.gemm(act, Wd, residual=x_mid)
         hn = ops.rmsnorm_fwd(x, flat.pview("model.norm.weight"), eps, rstd=rstd)
         ldv = (V + 63) // 64 * 64

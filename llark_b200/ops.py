@@ -9,8 +9,8 @@ import math
 
 import torch
 
-from ._lib import (EPI_CLAMP_GLU, EPI_NONE, EPI_QUICK_GELU, EPI_RELU2, EPI_RELU_GLU, EPI_ROPE, EPI_SWIGLU_BWD, GemmEpilogue, check,
-                   lib)
+from ._lib import (EPI_CLAMP_GLU, EPI_NONE, EPI_QUICK_GELU, EPI_RELU2, EPI_RELU_GLU, EPI_ROPE, EPI_SWIGLU, EPI_SWIGLU_BWD,
+                   GemmEpilogue, check, lib)
 
 BF16 = torch.bfloat16
 
@@ -53,13 +53,14 @@ def _req(t, dtype=None):
 
 def gemm(a, b, *, a_mn=False, b_mn=False, M=None, N=None, K=None, out=None, out_dtype=None, bias=None,
          residual=None, lda=None, ldb=None, ldc=None, ldr=None, max_ctas=0, quick_gelu=False, rope=None,
-         swiglu_bwd=None, act=None, act_limit=0.0, act_slope=0.0):
+         swiglu_bwd=None, act=None, act_limit=0.0, act_slope=0.0, swiglu=False):
     """C[M,N] = A[M,K] @ B[N,K]^T (+bias) (+residual), optionally with one fused epilogue (llark_gemm_ex):
 
     quick_gelu=True            C = quick_gelu(acc + bias)
     rope=(cos, sin, S, cols)   columns [0, cols) rotated per 128-wide head, position = row % S (fused-QKV projection)
     swiglu_bwd=gu              acc is d(act) [M, I]; `out` must be the dgu buffer [M, 2I]: out = (dgate | dup)
     act="relu2" | "relu_glu" | "clamp_glu"   see linear()
+    swiglu=True                few rows (M <= LINEAR_FEW_MAX, bf16): b = gate rows, then up rows; C [M, N / 2] = swiglu_fwd(A @ b^T)
 
     a: [M,K] (a_mn=False) or [K,M] (a_mn=True); b: [N,K] (b_mn=False) or [K,N] (b_mn=True); row-major with
     leading dimension = last-dim stride unless lda/ldb given. bf16 inputs use kind::f16, fp32 inputs kind::tf32.
@@ -79,7 +80,7 @@ def gemm(a, b, *, a_mn=False, b_mn=False, M=None, N=None, K=None, out=None, out_
     lda = lda if lda is not None else a.stride(0)
     ldb = ldb if ldb is not None else b.stride(0)
     if out is None:
-        out = torch.empty((M, N), device=a.device, dtype=out_dtype or (torch.float32 if in_fp32 else BF16))
+        out = torch.empty((M, N // 2 if swiglu else N), device=a.device, dtype=out_dtype or (torch.float32 if in_fp32 else BF16))
     ldc = ldc if ldc is not None else out.stride(0)
     c_fp32 = out.dtype == torch.float32
     if residual is not None:
@@ -100,6 +101,8 @@ def gemm(a, b, *, a_mn=False, b_mn=False, M=None, N=None, K=None, out=None, out_
     elif rope is not None:
         cos_t, sin_t, S_rope, cols = rope
         ep = GemmEpilogue(EPI_ROPE, cos_t.data_ptr(), sin_t.data_ptr(), 0, int(S_rope), int(cols), 0.0, 0.0)
+    elif swiglu:
+        ep = GemmEpilogue(EPI_SWIGLU, None, None, 0, 0, 0, 0.0, 0.0)
     elif swiglu_bwd is not None:
         ep = GemmEpilogue(EPI_SWIGLU_BWD, swiglu_bwd.data_ptr(), None, swiglu_bwd.stride(0), 0, 0, 0.0, 0.0)
     elif act is not None:
@@ -209,6 +212,16 @@ def attn_decode(q, k_cache, v_cache, lens, n_heads, head_dim, out=None):
     out = out if out is not None else torch.empty((B, n_heads * head_dim), device=q.device, dtype=BF16)
     check(lib().llark_attn_decode(_p(q), _p(k_cache), _p(v_cache), _p(lens), _p(out), B, s_max, n_heads, head_dim,
                                   1.0 / math.sqrt(head_dim), _stream()), "attn_decode")
+    return out
+
+
+def attn_decode_packed(qkv, k_cache, v_cache, pos, n_heads, head_dim, out=None):
+    """attn_decode for rows that all stand at position `pos`, from the packed projection qkv [B, 3H] (q | k | v): the new keys and
+    values are stored in the caches [B, s_max, H] by the same launch."""
+    B, s_max = k_cache.shape[0], k_cache.shape[1]
+    out = out if out is not None else torch.empty((B, n_heads * head_dim), device=qkv.device, dtype=BF16)
+    check(lib().llark_attn_decode_packed(_p(qkv), qkv.stride(0), _p(k_cache), _p(v_cache), int(pos), _p(out), B, s_max, n_heads,
+                                         head_dim, 1.0 / math.sqrt(head_dim), _stream()), "attn_decode_packed")
     return out
 
 

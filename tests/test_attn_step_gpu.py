@@ -73,3 +73,20 @@ def test_cache_rows_off_16_byte_boundaries_and_empty_rows():
     got, want = ops.attn_decode(q, k, v, lens, NH, 128), ops.attn_decode(q.clone(), k, v, lens, NH, 128)
     assert want[0].abs().max().item() == 0
     assert ((got - want).float().norm() / want.float().norm()).item() < 2.0 ** -7
+
+
+@pytest.mark.parametrize("B,S,NH,pos", [(1, 64, 2, 0), (3, 300, 4, 16), (2, 2000, 2, 1777), (40, 128, 16, 127)])
+def test_packed_projection_is_that_of_the_stores(B, S, NH, pos):
+    """The form that takes the new key and value from the packed projection stores them and gives what the stored ones give."""
+    from llark_b200 import ops
+
+    torch.manual_seed(pos + B)
+    H = NH * 128
+    qkv = torch.randn(B, 3 * H + 8, device="cuda").to(BF16)[:, :3 * H]
+    k, v = (torch.randn(B, S, H, device="cuda").to(BF16) for _ in range(2))
+    want_k, want_v = k.clone(), v.clone()
+    want_k[:, pos], want_v[:, pos] = qkv[:, H:2 * H], qkv[:, 2 * H:]
+    got = ops.attn_decode_packed(qkv, k, v, pos, NH, 128)
+    assert torch.equal(k, want_k) and torch.equal(v, want_v)
+    lens = torch.full((B,), pos + 1, device="cuda", dtype=torch.int32)
+    assert torch.equal(got, ops.attn_decode(qkv[:, :H].contiguous(), want_k, want_v, lens, NH, 128))

@@ -80,3 +80,14 @@ def test_routed_experts(T, C, ff, E, top, kind):
                 h = torch.relu(u) ** 2
             want[t, k] = wd[e].to(F64) @ h
     assert _rel(got, want) < 2.0 ** -8  # the units are rounded to eight bits between the two products
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 704, 256), (8, 1024, 512), (9, 208, 72), (40, 2816, 1024)])
+def test_gate_and_up_in_the_epilogue_are_those_of_the_op(M, N, K):
+    from llark_b200 import ops
+
+    torch.manual_seed(M + N)
+    x, w = (torch.randn(M, K, device="cuda") * 0.5).to(BF16), (torch.randn(N, K, device="cuda") * 0.2).to(BF16)
+    got = ops.gemm(x, w, swiglu=True)
+    # the halves' tiles cut K as the plain product's do, up to how many CTAs share a row: the sums may differ in their last bits
+    assert _rel(got, ops.swiglu_fwd(ops.gemm(x, w)).to(F64)) < 2.0 ** -8
