@@ -11,6 +11,15 @@
 #include <stdlib.h>
 
 namespace llark {
+namespace jbconv {  // jb_conv_tc.cu
+int resblock(const float* x, const float* w1, const float* b1, const float* w2, const float* b2, float* y, int N, int T, int dil,
+             cudaStream_t st);
+bool takes_down(int c_in, int c_out);
+int down(const float* x, const float* w, const float* b, float* y, int N, int c_in, int T, cudaStream_t st);
+bool takes_k3(int c_in, int c_out);
+int k3(const float* x, const float* w, const float* b, float* y, int N, int T, cudaStream_t st);
+}  // namespace jbconv
+
 
 extern thread_local int g_last_cuda_error;
 static inline int jb_check() {
@@ -218,51 +227,95 @@ conv_k3_kernel(const float* __restrict__ x, const float* __restrict__ w, const f
 }
 
 // ---------------------------------------------------------------------------------------------- VQ nearest code
-// One thread per (n,t); x vector in registers, codebook streamed through shared memory (broadcast reads).
-// dist = (|x|^2 - 2 x.k) + |k|^2, first minimum wins.
-__global__ void __launch_bounds__(128)
+// dist = (|x|^2 - 2 x.k) + |k|^2 in fp32, every sum in the order of the channels; first minimum wins. A lane holds two vectors (all 64
+// channels in registers), the eight warps of a CTA share 64 vectors and take an eighth of the codes each, streamed through shared
+// memory (one broadcast read of four channels feeds eight FMAs); the warps' best are merged in the codes' order. FMA-bound: 32768
+// vectors x 2048 codes 587 us with a thread per vector walking all codes (one warp per scheduler), see the launcher for now.
+constexpr int VQ_E = 64, VQ_CHUNK = 16, VQ_W = 8;
+__global__ void __launch_bounds__(VQ_W * 32)
 vq_encode_kernel(const float* __restrict__ x, const float* __restrict__ cb, long long* __restrict__ codes, int T,
                  int n_codes) {
-    constexpr int E = 64, CHUNK = 128;
-    __shared__ float scb[CHUNK * E];
-    __shared__ float skk[CHUNK];
-    const int n = blockIdx.y;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    float xv[E];
-    float xx = 0.f;
+    __shared__ __align__(16) float scb[VQ_W][VQ_CHUNK][VQ_E];
+    __shared__ float skk[VQ_W][VQ_CHUNK];
+    const int n = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t0 = blockIdx.x * 64 + lane;  // this lane's vectors: t0 and t0 + 32
+    float xv[2][VQ_E], xx[2] = {0.f, 0.f};
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-        xv[e] = (t < T) ? x[((long long)n * E + e) * T + t] : 0.f;
-        xx = fmaf(xv[e], xv[e], xx);
-    }
-    float best = INFINITY;
-    int best_j = 0;
-    for (int c0 = 0; c0 < n_codes; c0 += CHUNK) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < CHUNK * E; i += blockDim.x) {
-            const int j = c0 + i / E;
-            scb[i] = j < n_codes ? cb[(long long)c0 * E + i] : 0.f;
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int e = 0; e < VQ_E; ++e) {
+            const int t = t0 + 32 * u;
+            xv[u][e] = t < T ? x[((long long)n * VQ_E + e) * T + t] : 0.f;
+            xx[u] = fmaf(xv[u][e], xv[u][e], xx[u]);
         }
-        __syncthreads();
-        if (threadIdx.x < CHUNK) {
+    const int per = (n_codes + VQ_W - 1) / VQ_W, lo = warp * per, hi = lo + per < n_codes ? lo + per : n_codes;
+    const bool vec = (reinterpret_cast<uintptr_t>(cb) & 15) == 0;
+    float best[2] = {INFINITY, INFINITY};
+    int best_j[2] = {0, 0};
+    for (int c0 = lo; c0 < hi; c0 += VQ_CHUNK) {  // each warp its own codes: no barrier of the block
+        const int lim = hi - c0 < VQ_CHUNK ? hi - c0 : VQ_CHUNK;
+        __syncwarp();
+        if (vec)
+            for (int i = lane; i < lim * (VQ_E / 4); i += 32)
+                reinterpret_cast<float4*>(&scb[warp][0][0])[i] = reinterpret_cast<const float4*>(cb + (long long)c0 * VQ_E)[i];
+        else
+            for (int i = lane; i < lim * VQ_E; i += 32) (&scb[warp][0][0])[i] = cb[(long long)c0 * VQ_E + i];
+        __syncwarp();
+        if (lane < lim) {
             float kk = 0.f;
-            for (int e = 0; e < E; ++e) kk = fmaf(scb[threadIdx.x * E + e], scb[threadIdx.x * E + e], kk);
-            skk[threadIdx.x] = kk;
-        }
-        __syncthreads();
-        const int lim = min(CHUNK, n_codes - c0);
-        for (int j = 0; j < lim; ++j) {
-            float dot = 0.f;
 #pragma unroll
-            for (int e = 0; e < E; ++e) dot = fmaf(xv[e], scb[j * E + e], dot);
-            const float dist = (xx - 2.f * dot) + skk[j];
-            if (dist < best) {
-                best = dist;
-                best_j = c0 + j;
+            for (int e0 = 0; e0 < VQ_E; e0 += 4) {
+                const float4 k = *reinterpret_cast<const float4*>(&scb[warp][lane][e0]);
+                kk = fmaf(k.x, k.x, kk);
+                kk = fmaf(k.y, k.y, kk);
+                kk = fmaf(k.z, k.z, kk);
+                kk = fmaf(k.w, k.w, kk);
+            }
+            skk[warp][lane] = kk;
+        }
+        __syncwarp();
+        for (int j = 0; j < lim; ++j) {
+            float dot[2] = {0.f, 0.f};
+#pragma unroll
+            for (int e0 = 0; e0 < VQ_E; e0 += 4) {
+                const float4 k = *reinterpret_cast<const float4*>(&scb[warp][j][e0]);
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    dot[u] = fmaf(xv[u][e0], k.x, dot[u]);
+                    dot[u] = fmaf(xv[u][e0 + 1], k.y, dot[u]);
+                    dot[u] = fmaf(xv[u][e0 + 2], k.z, dot[u]);
+                    dot[u] = fmaf(xv[u][e0 + 3], k.w, dot[u]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float dist = (xx[u] - 2.f * dot[u]) + skk[warp][j];
+                if (dist < best[u]) {
+                    best[u] = dist;
+                    best_j[u] = c0 + j;
+                }
             }
         }
     }
-    if (t < T) codes[(long long)n * T + t] = best_j;
+    __syncthreads();  // the codes are no longer read: their place takes the warps' best
+    float* sd = &scb[0][0][0];
+    int* sj = reinterpret_cast<int*>(sd + VQ_W * 64);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        sd[warp * 64 + 32 * u + lane] = best[u];
+        sj[warp * 64 + 32 * u + lane] = best_j[u];
+    }
+    __syncthreads();
+    if (threadIdx.x < 64 && blockIdx.x * 64 + threadIdx.x < T) {
+        float d = sd[threadIdx.x];
+        int bj = sj[threadIdx.x];
+        for (int w = 1; w < VQ_W; ++w)  // later codes win only when they are nearer
+            if (sd[w * 64 + threadIdx.x] < d) {
+                d = sd[w * 64 + threadIdx.x];
+                bj = sj[w * 64 + threadIdx.x];
+            }
+        codes[(long long)n * T + blockIdx.x * 64 + threadIdx.x] = bj;
+    }
 }
 
 // ---------------------------------------------------------------------------------------------- LayerNorm
@@ -462,186 +515,6 @@ __device__ __forceinline__ void ja_load_rows(float* dst, const float* __restrict
         }
     }
 }
-// ---------------------------------------------------------------------------------------------- fused res block on tensor cores
-// The same ResConv1DBlock  y = x + W2 . relu(W1 (*dil d, k = 3) relu(x) + b1) + b2  (32 channels) as resblock_kernel, with
-// both convolutions as implicit GEMMs on mma.sync m16n8k8 TF32:  D[co, t] += A[co, k] . B[k, t],
-//   conv1: k = tap * 32 + ci (K = 96, 12 k-steps),  B[k, t] = relu(x)[ci, t + (tap - 1) d]   (shifted views of ONE smem tile)
-//   conv2: k = ci            (K = 32,  4 k-steps),  B[k, t] = relu(h)[ci, t]
-// and fp32 accuracy kept by the 3xTF32 split: every operand is hi + lo with hi = tf32(v), lo = tf32(v - hi), and
-// acc += A_lo.B_hi + A_hi.B_lo + A_hi.B_hi (the dropped lo.lo term is ~2^-22 relative). The SIMT kernel runs at 20 TFLOP/s
-// (27 % of the FP32 pipe, FMA / LDS-issue bound, profiles/r2f_prof_jukebox_hbm.md); the tensor cores take the FMAs away.
-// CTA = 256 threads = 8 warps over a 256-step time tile; warp w owns time steps [32 w, 32 w + 32) (4 n-tiles of 8) and all
-// 32 output channels (2 m-tiles of 16). Shared memory:
-//   sx  relu(x) tile [32][LDX], LDX = in_w rounded up to 8 mod 32 so the B-fragment reads (4 rows x 8 columns per
-//       instruction) touch 32 different banks;
-//   sh  relu(h) / staging tile [32][LDH = 264], each warp touches only its own 32 columns (1x1 conv: no halo) -> __syncwarp;
-//   weights pre-split and stored FRAGMENT-MAJOR: [k-step][m-tile][lane][a0..a3 hi, a0..a3 lo], so a thread fetches the hi and
-//       lo A fragments of one (k-step, m-tile) with two conflict-free LDS.128.
-constexpr int RTC_TT = 256;
-constexpr int RTC_LDH = 264;
-__device__ __forceinline__ void split_tf32(float v, uint32_t& hi, uint32_t& lo) {
-    hi = to_tf32(v);
-    lo = to_tf32(v - __uint_as_float(hi));
-}
-// w global [32 co][32 ci][KT]; frag [(ks * 2 + mt) * 32 + lane][8]; k = tap * 32 + ci
-template <int KT>
-__device__ __forceinline__ void load_weight_frags(float* frag, const float* __restrict__ w) {
-    constexpr int KS = KT * 4;  // k-steps of 8
-    for (int i = threadIdx.x; i < KS * 2 * 32 * 4; i += blockDim.x) {
-        const int r = i & 3, lane = (i >> 2) & 31, mt = (i >> 7) & 1, ks = i >> 8;
-        const int g = lane >> 2, t4 = lane & 3;
-        const int co = mt * 16 + g + (r & 1) * 8;
-        const int k = ks * 8 + t4 + (r >> 1) * 4;
-        const int tap = k >> 5, ci = k & 31;
-        const float v = w[(co * 32 + ci) * KT + tap];
-        uint32_t hi, lo;
-        split_tf32(v, hi, lo);
-        float* dst = frag + (((ks * 2 + mt) * 32 + lane) << 3);
-        dst[r] = __uint_as_float(hi);
-        dst[4 + r] = __uint_as_float(lo);
-    }
-}
-__global__ void __launch_bounds__(256, 2)
-resblock_tc_kernel(const float* __restrict__ x, const float* __restrict__ w1, const float* __restrict__ b1,
-                   const float* __restrict__ w2, const float* __restrict__ b2, float* __restrict__ y, int T, int d,
-                   int ldx) {
-    extern __shared__ __align__(16) float sm[];
-    constexpr int C = 32;
-    const int n = blockIdx.y;
-    const int t0 = blockIdx.x * RTC_TT;
-    const int in_w = RTC_TT + 2 * d;
-    float* f1 = sm;                       // conv1 weight fragments: 12 * 2 * 32 * 8
-    float* f2 = f1 + 12 * 2 * 32 * 8;     // conv2 weight fragments:  4 * 2 * 32 * 8
-    float* sh = f2 + 4 * 2 * 32 * 8;      // [C][RTC_LDH]
-    float* sx = sh + C * RTC_LDH;         // [C][ldx]
-    const float* xn = x + (long long)n * C * T;
-    // relu(x) tile, columns t0 - d .. t0 + 255 + d (zero outside [0, T)); eight independent loads per thread
-    for (int j = threadIdx.x; j < in_w; j += blockDim.x) {
-        const int ti = t0 - d + j;
-        const bool ok = ti >= 0 && ti < T;
-        const float* src = xn + (ok ? ti : 0);
-        for (int ci = 0; ci < C; ci += 8) {
-            float v[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = ok ? src[(long long)(ci + u) * T] : 0.f;
-#pragma unroll
-            for (int u = 0; u < 8; ++u) sx[(ci + u) * ldx + j] = fmaxf(v[u], 0.f);
-        }
-    }
-    load_weight_frags<3>(f1, w1);
-    load_weight_frags<1>(f2, w2);
-    __syncthreads();
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane >> 2, t4 = lane & 3;
-    const int tw = warp * 32;  // this warp's first time step inside the tile
-    float acc[2][4][4];
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt) {
-        const float blo = b1[mt * 16 + g], bhi = b1[mt * 16 + g + 8];
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            acc[mt][nt][0] = acc[mt][nt][1] = blo;
-            acc[mt][nt][2] = acc[mt][nt][3] = bhi;
-        }
-    }
-    // ---- conv1: 12 k-steps (tap-major), B from shifted columns of sx
-#pragma unroll 1
-    for (int ks = 0; ks < 12; ++ks) {
-        const int tap = ks >> 2, ci0 = (ks & 3) * 8;
-        uint32_t ah[2][4], al[2][4];
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
-            const float4* fp = reinterpret_cast<const float4*>(f1 + (((ks * 2 + mt) * 32 + lane) << 3));
-            const float4 h = fp[0], l = fp[1];
-            ah[mt][0] = __float_as_uint(h.x); ah[mt][1] = __float_as_uint(h.y);
-            ah[mt][2] = __float_as_uint(h.z); ah[mt][3] = __float_as_uint(h.w);
-            al[mt][0] = __float_as_uint(l.x); al[mt][1] = __float_as_uint(l.y);
-            al[mt][2] = __float_as_uint(l.z); al[mt][3] = __float_as_uint(l.w);
-        }
-        const float* r0 = sx + (ci0 + t4) * ldx + tw + g + tap * d;
-        const float* r1 = r0 + 4 * ldx;
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            uint32_t bh0, bl0, bh1, bl1;
-            split_tf32(r0[nt * 8], bh0, bl0);
-            split_tf32(r1[nt * 8], bh1, bl1);
-#pragma unroll
-            for (int mt = 0; mt < 2; ++mt) {
-                mma_tf32(acc[mt][nt], al[mt], bh0, bh1);
-                mma_tf32(acc[mt][nt], ah[mt], bl0, bl1);
-                mma_tf32(acc[mt][nt], ah[mt], bh0, bh1);
-            }
-        }
-    }
-    // ---- relu(h) -> this warp's 32 columns of sh (accumulator layout: rows g / g + 8, columns 2 t4, 2 t4 + 1)
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            float* p0 = sh + (mt * 16 + g) * RTC_LDH + tw + nt * 8 + 2 * t4;
-            *reinterpret_cast<float2*>(p0) = make_float2(fmaxf(acc[mt][nt][0], 0.f), fmaxf(acc[mt][nt][1], 0.f));
-            *reinterpret_cast<float2*>(p0 + 8 * RTC_LDH) = make_float2(fmaxf(acc[mt][nt][2], 0.f), fmaxf(acc[mt][nt][3], 0.f));
-        }
-    __syncwarp();
-    // ---- conv2 (1x1): 4 k-steps, B from sh
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt) {
-        const float blo = b2[mt * 16 + g], bhi = b2[mt * 16 + g + 8];
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            acc[mt][nt][0] = acc[mt][nt][1] = blo;
-            acc[mt][nt][2] = acc[mt][nt][3] = bhi;
-        }
-    }
-#pragma unroll 1
-    for (int ks = 0; ks < 4; ++ks) {
-        uint32_t ah[2][4], al[2][4];
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
-            const float4* fp = reinterpret_cast<const float4*>(f2 + (((ks * 2 + mt) * 32 + lane) << 3));
-            const float4 h = fp[0], l = fp[1];
-            ah[mt][0] = __float_as_uint(h.x); ah[mt][1] = __float_as_uint(h.y);
-            ah[mt][2] = __float_as_uint(h.z); ah[mt][3] = __float_as_uint(h.w);
-            al[mt][0] = __float_as_uint(l.x); al[mt][1] = __float_as_uint(l.y);
-            al[mt][2] = __float_as_uint(l.z); al[mt][3] = __float_as_uint(l.w);
-        }
-        const float* r0 = sh + (ks * 8 + t4) * RTC_LDH + tw + g;
-        const float* r1 = r0 + 4 * RTC_LDH;
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            uint32_t bh0, bl0, bh1, bl1;
-            split_tf32(r0[nt * 8], bh0, bl0);
-            split_tf32(r1[nt * 8], bh1, bl1);
-#pragma unroll
-            for (int mt = 0; mt < 2; ++mt) {
-                mma_tf32(acc[mt][nt], al[mt], bh0, bh1);
-                mma_tf32(acc[mt][nt], ah[mt], bl0, bl1);
-                mma_tf32(acc[mt][nt], ah[mt], bh0, bh1);
-            }
-        }
-    }
-    __syncwarp();  // every lane has finished reading relu(h) before the tile is reused as the output staging area
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            float* p0 = sh + (mt * 16 + g) * RTC_LDH + tw + nt * 8 + 2 * t4;
-            *reinterpret_cast<float2*>(p0) = make_float2(acc[mt][nt][0], acc[mt][nt][1]);
-            *reinterpret_cast<float2*>(p0 + 8 * RTC_LDH) = make_float2(acc[mt][nt][2], acc[mt][nt][3]);
-        }
-    __syncwarp();
-    // ---- y = x + (.): one channel row of this warp's 32 time steps per instruction (128 contiguous bytes)
-    const int t = t0 + tw + lane;
-    if (t < T) {
-#pragma unroll 8
-        for (int co = 0; co < C; ++co) {
-            const long long off = ((long long)n * C + co) * T + t;
-            y[off] = x[off] + sh[co * RTC_LDH + tw + lane];
-        }
-    }
-}
-
 template <int NKT>  // key tiles of 8 (8 -> 64 keys, 16 -> 128 keys)
 __global__ void __launch_bounds__(256)
 jb_sparse_attn_tc_kernel(const float* __restrict__ qkv, void* __restrict__ out, int out_bf16, int T, int heads, int dh,
@@ -858,7 +731,8 @@ using namespace llark;
 extern "C" int llark_jb_conv_down(const float* x, const float* w, const float* bias, float* y, int N, int c_in,
                                   int c_out, int T, cudaStream_t st) {
     if (N <= 0 || T <= 0 || (T & 1) || c_in <= 0 || (c_out != 32 && c_out != 64)) return LLARK_EINVAL;
-    int rc;
+    if (jbconv::takes_down(c_in, c_out)) return jbconv::down(x, w, bias, y, N, c_in, T, st);
+    int rc;  // one channel in (the waveform), or other widths: memory-bound or small
     if (c_out == 32) {
         constexpr int TILE = DownCfg<32>::Tile::TILE_T;
         const int smem = (c_in * (2 * TILE + 2) + c_out * c_in * 4) * (int)sizeof(float);
@@ -882,16 +756,7 @@ extern "C" int llark_jb_resblock(const float* x, const float* w1, const float* b
     if (N <= 0 || T <= 0 || dilation < 1 || dilation > 243) return LLARK_EINVAL;
     const char* tc_env = getenv("LLARK_JB_CONV_TC");  // "0" selects the fp32 SIMT kernel (read per call: tests toggle it)
     const int use_tc = (tc_env && tc_env[0] == '0') ? 0 : 1;
-    if (use_tc && dilation <= 81) {
-        const int in_w = RTC_TT + 2 * dilation;
-        const int ldx = ((in_w + 23) / 32) * 32 + 8;  // >= in_w and == 8 (mod 32): conflict-free B-fragment reads
-        const int smem_tc = ((12 + 4) * 2 * 32 * 8 + 32 * RTC_LDH + 32 * ldx) * (int)sizeof(float);
-        int rc_tc = set_dyn_smem((const void*)resblock_tc_kernel, smem_tc);
-        if (rc_tc) return rc_tc;
-        dim3 grid_tc((T + RTC_TT - 1) / RTC_TT, N);
-        resblock_tc_kernel<<<grid_tc, 256, smem_tc, st>>>(x, w1, b1, w2, b2, y, T, dilation, ldx);
-        return jb_check();
-    }
+    if (use_tc) return jbconv::resblock(x, w1, b1, w2, b2, y, N, T, dilation, st);
     const int smem = (32 * (RES_TT + 2 * dilation) + 32 * RES_TT + 32 * 32 * 3 + 32 * 32) * (int)sizeof(float);
     int rc = set_dyn_smem((const void*)resblock_kernel, smem);
     if (rc) return rc;
@@ -903,6 +768,7 @@ extern "C" int llark_jb_resblock(const float* x, const float* w1, const float* b
 extern "C" int llark_jb_conv_k3(const float* x, const float* w, const float* bias, float* y, int N, int c_in, int c_out,
                                 int T, cudaStream_t st) {
     if (N <= 0 || T <= 0 || c_in <= 0 || (c_out != 32 && c_out != 64)) return LLARK_EINVAL;
+    if (jbconv::takes_k3(c_in, c_out)) return jbconv::k3(x, w, bias, y, N, T, st);
     int rc;
     if (c_out == 64) {
         constexpr int TILE = K3Cfg<64>::Tile::TILE_T;
@@ -925,8 +791,8 @@ extern "C" int llark_jb_conv_k3(const float* x, const float* w, const float* bia
 extern "C" int llark_jb_vq_encode(const float* x, const float* codebook, long long* codes, int N, int T, int n_codes,
                                   cudaStream_t st) {
     if (N <= 0 || T <= 0 || n_codes <= 0) return LLARK_EINVAL;
-    dim3 grid((T + 127) / 128, N);
-    vq_encode_kernel<<<grid, 128, 0, st>>>(x, codebook, codes, T, n_codes);
+    dim3 grid((T + 63) / 64, N);
+    vq_encode_kernel<<<grid, VQ_W * 32, 0, st>>>(x, codebook, codes, T, n_codes);
     return jb_check();
 }
 

@@ -212,3 +212,50 @@ def test_resblock_tensor_core_kernel_matches_simt_and_fp64(d):
     check_close(f"resblock_tc_vs_fp64:d{d}", _rel(tc, ref), 2e-6)
     check_close(f"resblock_simt_vs_fp64:d{d}", _rel(simt, ref), 2e-6)
     check_close(f"resblock_tc_vs_simt:d{d}", _rel(tc, simt), 2e-6)
+
+
+@pytest.mark.parametrize("T", [2, 126, 128, 130, 1000])
+@pytest.mark.parametrize("kind,c_in", [("down", 1), ("down", 32), ("down", 64), ("k3", 32), ("res1", 32), ("res27", 32)])
+def test_convolutions_at_the_edges_of_their_tiles_match_fp64(kind, c_in, T):
+    """The tcgen05 convolutions (tiles of 128 time steps, several per CTA and clip) against fp64 conv1d: fewer steps than a tile, one
+    more than a tile, halos that cross clip ends. Split operands keep 22 bits and chains are 12 products long: 1e-6 of the result."""
+    import torch.nn.functional as F
+
+    from llark_b200 import ops
+
+    g = torch.Generator().manual_seed(T + c_in)
+    N = 3
+    x = torch.randn(N, c_in, T, generator=g)
+    xd = x.double()
+    if kind == "down":
+        w, b = torch.randn(32, c_in, 4, generator=g) / math.sqrt(4 * c_in), torch.randn(32, generator=g) * 0.1
+        got, ref = ops.jb_conv_down(x.cuda(), w.cuda(), b.cuda()), F.conv1d(xd, w.double(), b.double(), stride=2, padding=1)
+    elif kind == "k3":
+        w, b = torch.randn(64, 32, 3, generator=g) / math.sqrt(96), torch.randn(64, generator=g) * 0.1
+        got, ref = ops.jb_conv_k3(x.cuda(), w.cuda(), b.cuda()), F.conv1d(xd, w.double(), b.double(), padding=1)
+    else:
+        d = int(kind[3:])
+        w1, b1 = torch.randn(32, 32, 3, generator=g) / math.sqrt(96), torch.randn(32, generator=g) * 0.1
+        w2, b2 = torch.randn(32, 32, 1, generator=g) / math.sqrt(32), torch.randn(32, generator=g) * 0.1
+        got = ops.jb_resblock(*(t.cuda() for t in (x, w1, b1, w2, b2)), d)
+        h = F.conv1d(F.relu(xd), w1.double(), b1.double(), padding=d, dilation=d)
+        ref = xd + F.conv1d(F.relu(h), w2.double(), b2.double())
+    assert _rel(got.cpu(), ref) < 1e-6
+
+
+@pytest.mark.parametrize("T,n_codes", [(1, 5), (64, 2048), (65, 2047), (200, 37)])
+def test_nearest_code_in_every_slice_of_the_codebook(T, n_codes):
+    """Codes are shared out over eight warps: the same fp32 distances as one walk over all of them, the first minimum wins."""
+    from llark_b200 import ops
+
+    g = torch.Generator().manual_seed(T)
+    x, cb = torch.randn(2, 64, T, generator=g), torch.randn(n_codes, 64, generator=g)
+    cb[n_codes // 2] = cb[0]  # a tie across slices
+    x[0, :, 0] = cb[0]
+    codes = ops.jb_vq_encode(x.cuda(), cb.cuda()).cpu()
+    flat = x.permute(0, 2, 1).reshape(-1, 64).double()
+    dist = (flat.pow(2).sum(1, keepdim=True) - 2 * flat @ cb.double().t() + cb.double().pow(2).sum(1)[None])
+    best = dist.min(1).values
+    got = dist.gather(1, codes.view(-1, 1)).squeeze(1)
+    assert ((got - best) <= 1e-4 * best.clamp_min(1.0)).all()  # fp32 sums of 64 terms
+    assert codes[0, 0].item() == 0  # the first of two equal ones
