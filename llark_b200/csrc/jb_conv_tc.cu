@@ -1,33 +1,41 @@
 // The Jukebox encoder's convolutions on tcgen05: fp32 in and out, every product as three TF32 products of split operands.
 //
 // A convolution over time with few channels is a product with the time steps as rows: D[t, co] = sum over taps and channels of
-// x[ci, t * stride + tap * dilation - pad] w[co, ci, tap]. A thread owns a time step: it reads the 32 channels of a tap (coalesced over
-// the threads), splits them (x = hi + lo, hi what TF32 holds) and writes them as one 128-byte row of the A operand (128-byte swizzle),
-// and later finds its sums in its own TMEM lane, so that neither the layout change nor the epilogue needs another pass through shared
-// memory. Sums: hi hi in one accumulator, hi lo + lo hi in another (the tensor cores cut instead of rounding: short chains, 4e-7 of the
-// terms' norm). A CTA walks tiles of 128 time steps with the weights resident (split once); the next tap's values are on their way
-// while a tap's products run, and two CTAs share an SM.
+// x[ci, t * stride + tap * dilation - pad] w[co, ci, tap]. A thread owns a time step: it reads its 32 channels (coalesced over the
+// threads), splits them once (x = hi + lo, hi what TF32 holds) and writes them as one 128-byte row of the A operand (128-byte swizzle);
+// a tap is the same rows read from another first row, stride 2 keeps even and odd steps apart. The thread later finds its sums in its
+// own TMEM lane, so that neither the layout change nor the epilogue needs another pass through shared memory. The weights stay in
+// shared memory, split once, hi rows and lo rows behind one another: one product of the hi part with both (hi hi and hi lo side by side
+// in TMEM), one of the lo part with the hi rows. hi hi has accumulators of its own, one for the even taps, one for the odd ones: the
+// tensor cores cut instead of rounding, so chains are kept short (error of a res block against 64 bits 8e-8 of its second product;
+// 64 channels in, stride 2: 2.8e-7, with one chain 5.2e-7).
+//
+// A CTA is two or three groups of four warps, each with tiles of 128 steps, rows of A, accumulators and a barrier of its own; the next
+// tile's values are requested as soon as this one's rows are written.
 //
 //   res block   y = x + W2 relu(W1 (*dilation d, 3 taps) relu(x) + b1) + b2, both convolutions of a tile in one visit: the second's A
 //               operand is the first's result, written by the thread that owns the row
 //   others      taps 4 stride 2 (32 or 64 channels in, 32 out), taps 3 (32 in, 64 out)
 //
-// What bounds it: the instructions that split and write the operands, then memory (a res block reads and writes every value once).
-// Measured on a B200, 4 clips x 524288 steps x 32 channels: see the launchers.
+// What bounds it: the latency of load, split, product and read-back of a tile, hidden only by the other groups (a res block reads and
+// writes every value once; the tensor pipe works a quarter of the time). Measured on a B200, 4 clips x 524288 steps x 32 channels, a
+// res block: 257 us for dilations up to 64 and 346 at 81, with mma.sync 413 and 685. Three groups of four warps and not more: 168
+// registers a thread hold a step's 32 channels, the next step's and the sums; two groups with the input staged by cp.async: 325.
+//
 #include "common.cuh"
 
 namespace llark {
 extern thread_local int g_last_cuda_error;
 namespace jbconv {
 
-constexpr int TT = 128;                 // time steps per tile = threads = TMEM lanes
-constexpr int kHalf = TT * 128;         // hi or lo part of a 32-channel slice of A: 16 KB
-constexpr int kBuf = 2 * kHalf;
+constexpr int TT = 128;        // time steps per tile = threads of a group = TMEM lanes
+constexpr int kMaxDil = 81;    // two groups' rows fit into shared memory up to 81; three groups' up to 64
+constexpr int kMaxDil3 = 64;   // halo rows: one for every thread
 
 struct Args {
     const float *x, *w1, *b1, *w2, *b2;
     float* y;
-    int T, To, dil, tiles_per_clip, tiles;  // input and output steps per clip
+    int T, To, dil, rows, tiles_per_clip, tiles;  // input and output steps per clip; rows of A in a region
 };
 
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {  // 128-byte rows, 8-row groups of 1024 bytes, 128-byte swizzle
@@ -38,146 +46,210 @@ __device__ __forceinline__ uint32_t idesc_tf32(int n) {  // fp32 sums, both oper
 }
 __device__ __forceinline__ void split(float v, float& hi, float& lo) {
     hi = __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u);  // rounded to nearest: |v - hi| <= 2^-12 |v|
-    lo = __uint_as_float(__float_as_uint(v - hi) & 0xffffe000u);         // the difference is exact; cut at 2^-22 |v|
+    lo = __uint_as_float((__float_as_uint(v - hi) + 0x1000u) & 0xffffe000u);  // the difference is exact: |v - hi - lo| <= 2^-24 |v|
 }
-// 32 values as row r of a slice, split into its two parts
+// 32 values as row r of a region, split into its two parts, lo_at bytes apart
 template <bool RELU>
-__device__ __forceinline__ void put_row(unsigned char* buf, int r, const float (&v)[32]) {
+__device__ __forceinline__ void put_row(unsigned char* region, int lo_at, int r, const float (&v)[32]) {
+    unsigned char* row = region + r * 128;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
         float hi[4], lo[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) split(RELU ? fmaxf(v[4 * q + e], 0.f) : v[4 * q + e], hi[e], lo[e]);
-        unsigned char* p = buf + r * 128 + ((q ^ (r & 7)) << 4);
+        unsigned char* p = row + ((q ^ (r & 7)) << 4);
         *reinterpret_cast<float4*>(p) = make_float4(hi[0], hi[1], hi[2], hi[3]);
-        *reinterpret_cast<float4*>(p + kHalf) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+        *reinterpret_cast<float4*>(p + lo_at) = make_float4(lo[0], lo[1], lo[2], lo[3]);
     }
 }
-// weights [COUT][NCI * 32][TAPS] -> per (tap, 32 channels): hi rows [COUT][32], then lo rows
+// weights [COUT][NCI * 32][TAPS] -> per (32 channels, tap): hi rows [COUT][32], then lo rows; odd taps the other way round
 template <int TAPS, int NCI, int COUT>
 __device__ __forceinline__ void put_weights(unsigned char* dst, const float* __restrict__ w) {
-    for (int i = threadIdx.x; i < TAPS * NCI * COUT * 32; i += TT) {
-        const int ci = i & 31, co = (i >> 5) % COUT, kb = i / (32 * COUT), tap = kb / NCI, cb = kb % NCI;
+    for (int i = threadIdx.x; i < TAPS * NCI * COUT * 32; i += blockDim.x) {
+        const int ci = i & 31, co = (i >> 5) % COUT, kb = i / (32 * COUT), tap = kb % TAPS, cb = kb / TAPS;
         float hi, lo;
         split(w[((long long)co * (NCI * 32) + cb * 32 + ci) * TAPS + tap], hi, lo);
         unsigned char* p = dst + kb * (2 * COUT * 128) + co * 128 + (((ci >> 2) ^ (co & 7)) << 4) + (ci & 3) * 4;
-        *reinterpret_cast<float*>(p) = hi;
-        *reinterpret_cast<float*>(p + COUT * 128) = lo;
+        *reinterpret_cast<float*>(p) = tap & 1 ? lo : hi;
+        *reinterpret_cast<float*>(p + COUT * 128) = tap & 1 ? hi : lo;
     }
 }
-// one slice of 32 channels: hi hi into column d_hh, the two mixed products into column d_x
-template <int COUT>
-__device__ __forceinline__ void products(uint32_t a, uint32_t w, uint32_t d_hh, uint32_t d_x, bool first) {
-    const uint32_t id = idesc_tf32(COUT);
-    const uint64_t ah = smem_desc(a), al = smem_desc(a + kHalf), wh = smem_desc(w), wl = smem_desc(w + COUT * 128);
+// 32 channels of a tap. SIDE 0: hi hi into COUT columns from d on, hi lo + lo hi into the COUT columns behind them; SIDE 1: the weights'
+// lo rows come first, hi hi goes into the COUT columns behind the shared ones. first: hi hi begins a chain; first_lo: the shared one.
+template <int COUT, int SIDE>
+__device__ __forceinline__ void products(uint32_t a, int lo_at, uint32_t w, uint32_t d, bool first, bool first_lo) {
+    const uint64_t ah = smem_desc(a), al = smem_desc(a + lo_at), wd = smem_desc(w), wh = smem_desc(w + (SIDE ? COUT * 128 : 0)),
+                   wl = smem_desc(w + (SIDE ? 0 : COUT * 128));
+    const uint32_t both = d + (SIDE ? COUT : 0), hh = d + (SIDE ? 2 * COUT : 0), mid = d + COUT;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const uint64_t o = (uint64_t)(2 * k);  // 8 channels = 32 bytes
-        umma_tf32(d_hh, ah + o, wh + o, id, !(first && k == 0));
-        umma_tf32(d_x, al + o, wh + o, id, !(first && k == 0));
-        umma_tf32(d_x, ah + o, wl + o, id, 1);
+        const bool f = first && k == 0, fl = first_lo && k == 0;
+        if (f == fl) {
+            umma_tf32(both, ah + o, wd + o, idesc_tf32(2 * COUT), !f);
+        } else {
+            umma_tf32(hh, ah + o, wh + o, idesc_tf32(COUT), !f);
+            umma_tf32(mid, ah + o, wl + o, idesc_tf32(COUT), !fl);
+        }
+        umma_tf32(mid, al + o, wh + o, idesc_tf32(COUT), 1);
     }
 }
 
-// shared memory: two slices of A | W1 | W2 (res block); 1024-byte aligned
-template <int TAPS, int NCI, int COUT, bool RES> constexpr int smem_bytes() {
-    return 2 * kBuf + TAPS * NCI * 2 * COUT * 128 + (RES ? 2 * 32 * 128 : 0) + 1024;
-}
-
-template <int TAPS, int STRIDE, int NCI, int COUT, bool RES>
-__global__ void __launch_bounds__(TT, 2)
+// A tile's input rows: stride 1: one region, row r is step t0 - dil + r; stride 2: even steps (row r is step 2 (t0 + r)), then odd ones
+// (row r is step 2 (t0 + r) - 1). Shared memory, 1024-byte aligned: W1 | W2 (res block) | per group: the regions, hi rows then lo rows.
+template <int TAPS, int STRIDE, int NCI, int COUT, bool RES, int NG>
+__global__ void __launch_bounds__(NG * TT, 1)
 conv_kernel(const Args p) {
     extern __shared__ unsigned char raw[];
-    __shared__ uint64_t bar[2];
+    __shared__ uint64_t bars[NG];
     __shared__ uint32_t tmem_base;
     __shared__ float sb[COUT + 32];
-    constexpr int KB = TAPS * NCI, CIN = NCI * 32;
-    unsigned char* sm = raw + ((1024u - (smem_u32(raw) & 1023u)) & 1023u);
-    unsigned char* sw1 = sm + 2 * kBuf;
-    unsigned char* sw2 = sw1 + KB * 2 * COUT * 128;
-    const int tid = threadIdx.x, warp = tid >> 5;
+    constexpr int CIN = NCI * 32, kGroup = RES ? 160 : 3 * COUT, kCols = NG * kGroup > 256 ? 512 : 256;
+    const int grp = threadIdx.x >> 7, tid = threadIdx.x & 127, warp = (threadIdx.x >> 5) & 3;
+    const int lo_at = p.rows * 128, region = 2 * lo_at;
+    unsigned char* sw1 = raw + ((1024u - (smem_u32(raw) & 1023u)) & 1023u);
+    unsigned char* sw2 = sw1 + TAPS * NCI * 2 * COUT * 128;
+    unsigned char* sa = sw2 + (RES ? 2 * 32 * 128 : 0) + grp * (STRIDE * region);
+    uint64_t* bar = &bars[grp];
     if (tid == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
+        mbar_init(bar, 1);
         mbar_fence_init();
     }
-    if (warp == 0) {
-        tmem_alloc(&tmem_base, 128);
+    if (threadIdx.x < 32) {
+        tmem_alloc(&tmem_base, kCols);
         tmem_relinquish();
     }
     put_weights<TAPS, NCI, COUT>(sw1, p.w1);
     if (RES) put_weights<1, 1, 32>(sw2, p.w2);
-    for (int i = tid; i < COUT; i += TT) sb[i] = p.b1[i];
-    if (RES && tid < 32) sb[COUT + tid] = p.b2[tid];
+    for (int i = threadIdx.x; i < COUT; i += NG * TT) sb[i] = p.b1[i];
+    if (RES && threadIdx.x < 32) sb[COUT + threadIdx.x] = p.b2[threadIdx.x];
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_base, lane0 = tmem + ((uint32_t)(warp * 32) << 16);
-    // columns: first convolution hi hi at 0, mixed at 64; second at 32 and 96
-    float v[32], xc[RES ? 32 : 1];
-    auto load = [&](int tile, int kb) {
-        const int clip = tile / p.tiles_per_clip, t = (tile - clip * p.tiles_per_clip) * TT + tid;
-        const int tap = kb / NCI, cb = kb % NCI;
-        const int at = STRIDE == 1 ? t + (tap - TAPS / 2) * p.dil : STRIDE * t + tap - 1;
-        const float* src = p.x + ((long long)clip * CIN + cb * 32) * p.T + at;
-        const bool in = at >= 0 && at < p.T && t < p.To;
-#pragma unroll
-        for (int c = 0; c < 32; ++c) v[c] = in ? src[(long long)c * p.T] : 0.f;
+    // a group's columns: hi hi of the even taps, the mixed products, hi hi of the odd taps; the second convolution's (res block) from 96 on
+    const uint32_t tmem = tmem_base + grp * kGroup, lane0 = tmem + ((uint32_t)(warp * 32) << 16);
+    auto group_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory"); };
+    auto where = [&](int tile, int& clip, int& t0) {
+        clip = tile / p.tiles_per_clip;
+        t0 = (tile - clip * p.tiles_per_clip) * TT;
     };
-    int g = 0;  // groups of products so far: group g works on slice g & 1 and reports on barrier g & 1
-    auto wait_group = [&](int n) { mbar_wait(&bar[n & 1], (uint32_t)((n >> 1) & 1)); };
-    if ((int)blockIdx.x < p.tiles) load(blockIdx.x, 0);
-    for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {
+    const int n_halo = STRIDE == 1 ? 2 * p.dil : 2;
+    const bool pairs = STRIDE == 2 && (reinterpret_cast<uintptr_t>(p.x) & 7) == 0;  // T is even
+    float v[STRIDE][32], hv[32], xc[RES ? 32 : 1];
+    auto load_halo = [&](int tile, int cb, int i) {
+        int clip, t0;
+        where(tile, clip, t0);
+        const float* base = p.x + ((long long)clip * CIN + cb * 32) * p.T;
+        const int at = STRIDE == 1 ? (i < p.dil ? t0 - p.dil + i : t0 + TT + i - p.dil) : (i == 0 ? 2 * t0 - 1 : 2 * (t0 + TT));
+        const bool in = at >= 0 && at < p.T;
 #pragma unroll
-        for (int kb = 0; kb < KB; ++kb) {
-            unsigned char* buf = sm + (g & 1) * kBuf;
-            if (g >= 2) wait_group(g - 2);
-            put_row<RES>(buf, tid, v);
-            if (RES && kb == 1)
+        for (int c = 0; c < 32; ++c) hv[c] = in ? base[(long long)c * p.T + at] : 0.f;
+    };
+    auto load = [&](int tile, int cb) {
+        int clip, t0;
+        where(tile, clip, t0);
+        const float* base = p.x + ((long long)clip * CIN + cb * 32) * p.T;
+        const float* src = base + STRIDE * (t0 + tid);
+        const bool in = t0 + tid < p.To;
+        if (STRIDE == 2 && pairs) {
 #pragma unroll
-                for (int c = 0; c < 32; ++c) xc[RES ? c : 0] = v[c];  // the residual: this thread's own step
-            if (kb + 1 < KB)
-                load(tile, kb + 1);
-            else if (tile + (int)gridDim.x < p.tiles)
-                load(tile + gridDim.x, 0);
+            for (int c = 0; c < 32; ++c) {
+                const float2 f = in ? *reinterpret_cast<const float2*>(src + (long long)c * p.T) : make_float2(0.f, 0.f);
+                v[0][c] = f.x;
+                v[STRIDE - 1][c] = f.y;
+            }
+        } else {
+#pragma unroll
+            for (int s = 0; s < STRIDE; ++s)
+#pragma unroll
+                for (int c = 0; c < 32; ++c) v[s][c] = in ? src[(long long)c * p.T + s] : 0.f;
+        }
+        if (tid < n_halo) load_halo(tile, cb, tid);
+    };
+    int n = 0;  // product groups issued so far, each waited for before its rows are written again
+    auto wait_last = [&]() { mbar_wait(bar, (uint32_t)((n - 1) & 1)); };
+    auto read_sums = [&](int c0, float (&h)[32]) {  // 32 channels of the first convolution's three sums
+        uint32_t a[32], b[32];
+        tmem_ld_32x32b_x32(lane0 + c0, a);
+        tmem_ld_32x32b_x32(lane0 + 2 * COUT + c0, b);
+        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < 32; ++c) h[c] = __uint_as_float(a[c]) + __uint_as_float(b[c]);
+        tmem_ld_32x32b_x32(lane0 + COUT + c0, a);
+        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < 32; ++c) h[c] += __uint_as_float(a[c]);
+    };
+    const int first = blockIdx.x * NG + grp, step = gridDim.x * NG;
+    if (first < p.tiles) load(first, 0);
+    for (int tile = first; tile < p.tiles; tile += step) {
+#pragma unroll
+        for (int cb = 0; cb < NCI; ++cb) {
+            if (cb) wait_last();
+            if (STRIDE == 1) {
+                put_row<RES>(sa, lo_at, tid + p.dil, v[0]);
+                if (tid < n_halo) put_row<RES>(sa, lo_at, tid < p.dil ? tid : TT + tid, hv);
+                if (RES && NG == 2 && tid + TT < n_halo) {  // more than 128 halo rows: the rest is read now
+                    load_halo(tile, cb, tid + TT);
+                    put_row<RES>(sa, lo_at, TT + TT + tid, hv);
+                }
+            } else {
+                put_row<RES>(sa, lo_at, tid, v[0]);
+                put_row<RES>(sa + region, lo_at, tid + 1, v[STRIDE - 1]);
+                if (tid < 2) put_row<RES>(sa + (tid == 0 ? region : 0), lo_at, tid == 0 ? 0 : TT, hv);
+            }
+            if (RES)
+#pragma unroll
+                for (int c = 0; c < 32; ++c) xc[RES ? c : 0] = v[0][c];  // the residual: this thread's own step
+            if (cb + 1 < NCI)
+                load(tile, cb + 1);
+            else if (tile + step < p.tiles)
+                load(tile + step, 0);
             fence_proxy_async_smem();
             tc_fence_before();
-            __syncthreads();  // the slice is written, and (first of a tile) the sums of the tile before have been read
+            group_sync();  // the rows are written, and the sums of the tile before have been read
             if (tid == 0) {
                 tc_fence_after();
-                products<COUT>(smem_u32(buf), smem_u32(sw1) + kb * 2 * COUT * 128, tmem, tmem + 64, kb == 0);
-                umma_commit(&bar[g & 1]);
+                const uint32_t a = smem_u32(sa), w = smem_u32(sw1) + cb * TAPS * 2 * COUT * 128;
+#pragma unroll
+                for (int tap = 0; tap < TAPS; ++tap) {
+                    const uint32_t rows = STRIDE == 1 ? a + tap * p.dil * 128 : a + (tap & 1 ? 0 : region) + (tap >> 1) * 128;
+                    if (tap & 1)
+                        products<COUT, 1>(rows, lo_at, w + tap * 2 * COUT * 128, tmem, cb == 0 && tap == 1, false);
+                    else
+                        products<COUT, 0>(rows, lo_at, w + tap * 2 * COUT * 128, tmem, cb == 0 && tap == 0, cb == 0 && tap == 0);
+                }
+                umma_commit(bar);
             }
-            ++g;
+            ++n;
         }
-        const int clip = tile / p.tiles_per_clip, t = (tile - clip * p.tiles_per_clip) * TT + tid;
-        wait_group(g - 1);
+        int clip, t0;
+        where(tile, clip, t0);
+        const int t = t0 + tid;
+        wait_last();
         tc_fence_after();
         float* out = p.y + (long long)clip * COUT * p.To + t;
         if constexpr (RES) {
-            uint32_t a[32], b[32];
-            tmem_ld_32x32b_x32(lane0, a);
-            tmem_ld_32x32b_x32(lane0 + 64, b);
-            tmem_ld_wait();
             float h[32];
+            read_sums(0, h);
 #pragma unroll
-            for (int c = 0; c < 32; ++c) h[c] = (__uint_as_float(a[c]) + __uint_as_float(b[c])) + sb[c];
-            unsigned char* buf = sm + (g & 1) * kBuf;  // free: group g - 1 and all before it are done
-            put_row<true>(buf, tid, h);
+            for (int c = 0; c < 32; ++c) h[c] += sb[c];
+            put_row<true>(sa, lo_at, tid, h);
             fence_proxy_async_smem();
             tc_fence_before();
-            __syncthreads();
+            group_sync();
             if (tid == 0) {
                 tc_fence_after();
-                products<32>(smem_u32(buf), smem_u32(sw2), tmem + 32, tmem + 96, true);
-                umma_commit(&bar[g & 1]);
+                products<32, 0>(smem_u32(sa), lo_at, smem_u32(sw2), tmem + 96, true, true);
+                umma_commit(bar);
             }
-            ++g;
-            wait_group(g - 1);
+            ++n;
+            wait_last();
             tc_fence_after();
-            tmem_ld_32x32b_x32(lane0 + 32, a);
-            tmem_ld_32x32b_x32(lane0 + 96, b);
+            uint32_t a[32], b[32];
+            tmem_ld_32x32b_x32(lane0 + 96, a);
+            tmem_ld_32x32b_x32(lane0 + 128, b);
             tmem_ld_wait();
             if (t < p.To)
 #pragma unroll
@@ -186,32 +258,32 @@ conv_kernel(const Args p) {
         } else {
 #pragma unroll
             for (int c0 = 0; c0 < COUT; c0 += 32) {
-                uint32_t a[32], b[32];
-                tmem_ld_32x32b_x32(lane0 + c0, a);
-                tmem_ld_32x32b_x32(lane0 + 64 + c0, b);
-                tmem_ld_wait();
+                float h[32];
+                read_sums(c0, h);
                 if (t < p.To)
 #pragma unroll
                     for (int c = 0; c < 32; ++c)
-                        out[(long long)(c0 + c) * p.To] = (__uint_as_float(a[c]) + __uint_as_float(b[c])) + sb[c0 + c];
+                        out[(long long)(c0 + c) * p.To] = h[c] + sb[c0 + c];
             }
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, 128);
+    if (threadIdx.x < 32) tmem_dealloc(tmem_base, kCols);
 }
 
-template <int TAPS, int STRIDE, int NCI, int COUT, bool RES>
+template <int TAPS, int STRIDE, int NCI, int COUT, bool RES, int NG>
 static int launch(Args a, int N, cudaStream_t st) {
-    constexpr int smem = smem_bytes<TAPS, NCI, COUT, RES>();
+    a.rows = STRIDE == 1 ? (TT + 2 * a.dil + 7) & ~7 : TT + 8;
+    const int smem = 1024 + TAPS * NCI * 2 * COUT * 128 + (RES ? 2 * 32 * 128 : 0) + NG * STRIDE * 2 * a.rows * 128;
     a.tiles_per_clip = (a.To + TT - 1) / TT;
     if ((long long)a.tiles_per_clip * N > 0x7fffffff) return LLARK_EINVAL;
     a.tiles = a.tiles_per_clip * N;
-    const int grid = a.tiles < 296 ? a.tiles : 296;  // two CTAs on each of the 148 SMs
-    cudaError_t e = cudaFuncSetAttribute(conv_kernel<TAPS, STRIDE, NCI, COUT, RES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const int grid = a.tiles < 148 * NG ? (a.tiles + NG - 1) / NG : 148;
+    auto kernel = conv_kernel<TAPS, STRIDE, NCI, COUT, RES, NG>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) {
-        conv_kernel<TAPS, STRIDE, NCI, COUT, RES><<<grid, TT, smem, st>>>(a);
+        kernel<<<grid, NG * TT, smem, st>>>(a);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) {
@@ -221,18 +293,20 @@ static int launch(Args a, int N, cudaStream_t st) {
     return LLARK_OK;
 }
 
+bool takes_resblock(int dil) { return dil <= kMaxDil; }
 int resblock(const float* x, const float* w1, const float* b1, const float* w2, const float* b2, float* y, int N, int T, int dil,
              cudaStream_t st) {
-    return launch<3, 1, 1, 32, true>(Args{x, w1, b1, w2, b2, y, T, T, dil, 0, 0}, N, st);
+    const Args a{x, w1, b1, w2, b2, y, T, T, dil, 0, 0, 0};
+    return dil <= kMaxDil3 ? launch<3, 1, 1, 32, true, 3>(a, N, st) : launch<3, 1, 1, 32, true, 2>(a, N, st);
 }
 bool takes_down(int c_in, int c_out) { return (c_in == 32 || c_in == 64) && c_out == 32; }
 int down(const float* x, const float* w, const float* b, float* y, int N, int c_in, int T, cudaStream_t st) {
-    const Args a{x, w, b, nullptr, nullptr, y, T, T / 2, 1, 0, 0};
-    return c_in == 32 ? launch<4, 2, 1, 32, false>(a, N, st) : launch<4, 2, 2, 32, false>(a, N, st);
+    const Args a{x, w, b, nullptr, nullptr, y, T, T / 2, 1, 0, 0, 0};
+    return c_in == 32 ? launch<4, 2, 1, 32, false, 2>(a, N, st) : launch<4, 2, 2, 32, false, 2>(a, N, st);
 }
 bool takes_k3(int c_in, int c_out) { return c_in == 32 && c_out == 64; }
 int k3(const float* x, const float* w, const float* b, float* y, int N, int T, cudaStream_t st) {
-    return launch<3, 1, 1, 64, false>(Args{x, w, b, nullptr, nullptr, y, T, T, 1, 0, 0}, N, st);
+    return launch<3, 1, 1, 64, false, 2>(Args{x, w, b, nullptr, nullptr, y, T, T, 1, 0, 0, 0}, N, st);
 }
 
 }  // namespace jbconv

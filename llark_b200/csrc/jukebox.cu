@@ -12,6 +12,7 @@
 
 namespace llark {
 namespace jbconv {  // jb_conv_tc.cu
+bool takes_resblock(int dil);
 int resblock(const float* x, const float* w1, const float* b1, const float* w2, const float* b2, float* y, int N, int T, int dil,
              cudaStream_t st);
 bool takes_down(int c_in, int c_out);
@@ -230,7 +231,7 @@ conv_k3_kernel(const float* __restrict__ x, const float* __restrict__ w, const f
 // dist = (|x|^2 - 2 x.k) + |k|^2 in fp32, every sum in the order of the channels; first minimum wins. A lane holds two vectors (all 64
 // channels in registers), the eight warps of a CTA share 64 vectors and take an eighth of the codes each, streamed through shared
 // memory (one broadcast read of four channels feeds eight FMAs); the warps' best are merged in the codes' order. FMA-bound: 32768
-// vectors x 2048 codes 587 us with a thread per vector walking all codes (one warp per scheduler), see the launcher for now.
+// vectors x 2048 codes 436 us; 587 with a thread per vector walking all codes (one warp per scheduler), 465 with two codes at a time.
 constexpr int VQ_E = 64, VQ_CHUNK = 16, VQ_W = 8;
 __global__ void __launch_bounds__(VQ_W * 32)
 vq_encode_kernel(const float* __restrict__ x, const float* __restrict__ cb, long long* __restrict__ codes, int T,
@@ -756,7 +757,7 @@ extern "C" int llark_jb_resblock(const float* x, const float* w1, const float* b
     if (N <= 0 || T <= 0 || dilation < 1 || dilation > 243) return LLARK_EINVAL;
     const char* tc_env = getenv("LLARK_JB_CONV_TC");  // "0" selects the fp32 SIMT kernel (read per call: tests toggle it)
     const int use_tc = (tc_env && tc_env[0] == '0') ? 0 : 1;
-    if (use_tc) return jbconv::resblock(x, w1, b1, w2, b2, y, N, T, dilation, st);
+    if (use_tc && jbconv::takes_resblock(dilation)) return jbconv::resblock(x, w1, b1, w2, b2, y, N, T, dilation, st);
     const int smem = (32 * (RES_TT + 2 * dilation) + 32 * RES_TT + 32 * 32 * 3 + 32 * 32) * (int)sizeof(float);
     int rc = set_dyn_smem((const void*)resblock_kernel, smem);
     if (rc) return rc;

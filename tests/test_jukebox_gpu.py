@@ -215,7 +215,7 @@ def test_resblock_tensor_core_kernel_matches_simt_and_fp64(d):
 
 
 @pytest.mark.parametrize("T", [2, 126, 128, 130, 1000])
-@pytest.mark.parametrize("kind,c_in", [("down", 1), ("down", 32), ("down", 64), ("k3", 32), ("res1", 32), ("res27", 32)])
+@pytest.mark.parametrize("kind,c_in", [("down", 1), ("down", 32), ("down", 64), ("k3", 32), ("res1", 32), ("res27", 32), ("res64", 32), ("res81", 32)])
 def test_convolutions_at_the_edges_of_their_tiles_match_fp64(kind, c_in, T):
     """The tcgen05 convolutions (tiles of 128 time steps, several per CTA and clip) against fp64 conv1d: fewer steps than a tile, one
     more than a tile, halos that cross clip ends. Split operands keep 22 bits and chains are 12 products long: 1e-6 of the result."""
