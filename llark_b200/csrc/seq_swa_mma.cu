@@ -7,12 +7,18 @@
 // step) and from ring entry j % cap of the request's slot otherwise. Q, K and V tiles sit in shared memory row-major and
 // reach the registers through ldmatrix (V through ldmatrix.trans); the row pitch (+8 elements) keeps those
 // conflict-free. K / V tiles are double-buffered: the next tile is in flight (cp.async) while this one is multiplied. Per-head score scale (softmax scale x temperature) and the optional sigmoid output gate are applied
-// in registers. The SIMT kernel of seq_mixers.cu remains the path for single-token steps, fp32 and head
-// sizes that are not multiples of 16.
+// in registers. Prompts with heads of 128, no soft cap and no rotated values are taken by seq_swa_tc.cu (tcgen05). The SIMT
+// kernel of seq_mixers.cu remains the path for fp32 and head sizes that are not multiples of 16.
 #include "common.cuh"
 
 namespace llark {
 extern thread_local int g_last_cuda_error;
+namespace swatc {  // seq_swa_tc.cu
+bool takes(int D, int max_len, float softcap, const float* vfreq, const void* out, long long out_ld);
+int launch(const void* qn, const void* kn, const void* vv, const void* kring, const void* vring, const float* gate, long long gate_ld,
+           const float* scale_h, void* out, const int* cu, const int* pos0, const int* slot, int n_seq, int max_len, int H, int G,
+           int window, int cap, const float* sink, int gate_per_head, int chunk, long long out_ld, float out_scale, cudaStream_t st);
+}  // namespace swatc
 namespace swamma {
 
 typedef __nv_bfloat16 bf16_t;
@@ -356,6 +362,9 @@ extern "C" int llark_seq_swa_attn_mma(const void* qn, const void* kn, const void
         return LLARK_EINVAL;
     if (gate && !gate_per_head && (gate_ld % 2)) return LLARK_EINVAL;
     if (vfreq && !v_interleaved && D != 64 && D != 128 && D != 256) return LLARK_EINVAL;
+    if (swatc::takes(D, max_len, softcap, vfreq, out, out_ld))
+        return swatc::launch(qn, kn, vv, kring, vring, gate, gate_ld, scale_h, out, cu, pos0, slot, n_seq, max_len, H, G, window, cap,
+                             sink, gate_per_head, chunk, out_ld, out_scale, st);
     if (D <= 64)
         return swamma::launch<64>(qn, kn, vv, kring, vring, gate, gate_ld, scale_h, out, cu, pos0, slot, n_seq, max_len, H,
                                   G, D, window, cap, sink, gate_per_head, chunk, softcap, vfreq, v_interleaved, out_ld, out_scale, st);
