@@ -445,6 +445,14 @@ __device__ __forceinline__ void mma_pv_128x128(uint32_t tD, uint32_t a_addr, uin
         umma_f16(tD, ad + (uint64_t)(k * 2), bd + (uint64_t)(k * 128), idesc, accumulate || k != 0);
 }
 __device__ __forceinline__ void compute_group_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+// bits 0 .. n - 1
+__device__ __forceinline__ uint32_t first_columns(int n) { return n >= 32 ? 0xffffffffu : n <= 0 ? 0u : (1u << n) - 1u; }
+// The exponents of columns that are not seen become -inf, so that ex2 gives 0: a select per column, where a condition around ex2 was a
+// branch per column (17 instructions per score in the dQ kernel).
+__device__ __forceinline__ void mask_columns(float (&v)[32], uint32_t seen) {
+#pragma unroll
+    for (int c = 0; c < 32; ++c) v[c] = (seen >> c) & 1u ? v[c] : -INFINITY;
+}
 // 32 fp32 values -> 32 bf16 -> four 16-byte units (g*4 .. g*4+3) of row r of a 128-byte-row, XOR-swizzled tile
 __device__ __forceinline__ void store_half_row(uint8_t* tile, int r, int g, const float (&v)[32]) {
     uint8_t* row = tile + r * 128;
@@ -667,6 +675,9 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
         const bool row_ok = qi < S;
         const float lse2 = row_ok ? lse[((long long)b * NH + h) * S + qi] * LOG2E : INFINITY;
         const float dsum = row_ok ? Dsum[((long long)b * NH + h) * S + qi] : 0.f;
+#ifdef LLARK_ATC_ALIBI
+        const float slope2 = alibi_slopes[h] * LOG2E;
+#endif
         for (int j = 0; j < n_kv; ++j) {
             const int sb = j & 1;
             mbar_wait(&sdp_full[sb], (uint32_t)(j >> 1) & 1);
@@ -684,16 +695,15 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
             const bool plain = (kbase + 31 <= q0 + quad * 32) && mw == 0xffffffffu;  // warp-uniform
             float ds[32];
 #pragma unroll
-            for (int c = 0; c < 32; ++c) {
-                const bool ok = plain || (kbase + c <= qi && ((mw >> c) & 1u));
+            for (int c = 0; c < 32; ++c)
 #ifdef LLARK_ATC_ALIBI
-                const float p = ok ? ex2(fmaf(__uint_as_float(sv[c]), scale_log2,
-                                             fmaf(alibi_slopes[h] * LOG2E, (float)(kbase + c - (S - 1)), -lse2))) : 0.f;
+                ds[c] = fmaf(__uint_as_float(sv[c]), scale_log2, fmaf(slope2, (float)(kbase + c - (S - 1)), -lse2));
 #else
-                const float p = ok ? ex2(fmaf(__uint_as_float(sv[c]), scale_log2, -lse2)) : 0.f;
+                ds[c] = fmaf(__uint_as_float(sv[c]), scale_log2, -lse2);
 #endif
-                ds[c] = p * (__uint_as_float(dv[c]) - dsum);
-            }
+            if (!plain) mask_columns(ds, mw & first_columns(qi - kbase + 1));
+#pragma unroll
+            for (int c = 0; c < 32; ++c) ds[c] = ex2(ds[c]) * (__uint_as_float(dv[c]) - dsum);
             if (j >= 2) {
                 mbar_wait(&dq_done[j & 1], (uint32_t)((j >> 1) - 1) & 1);  // tile j-2 retired: buffer j & 1 is free
                 tc_fence_after();
@@ -862,6 +872,10 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
         const int ct = threadIdx.x - 64;     // 0..255 inside the compute group
         const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
         const bool kvalid = key < S && (!mask || mask[(long long)b * S + key] != 0);
+        const bool all_valid = __all_sync(0xffffffffu, kvalid);
+#ifdef LLARK_ATC_ALIBI
+        const float slope2 = alibi_slopes[h] * LOG2E;
+#endif
         const float* lse_bh = lse + ((long long)b * NH + h) * S;
         const float* d_bh = Dsum + ((long long)b * NH + h) * S;
         // lse*log2e (threads 0-63) / D (threads 64-127) of the streamed queries, fetched one tile ahead so the global
@@ -891,19 +905,30 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
             if (lane == 0) mbar_arrive(&sdp_empty[sb]);
 
             const int qc0 = qb + g * 32;  // query of column 0 of this half row
-            const bool plain = qc0 >= k0 + quad * 32 + 31;  // warp-uniform: every query of the half row sees every key
+            const bool plain = all_valid && qc0 >= k0 + quad * 32 + 31;  // warp-uniform: every query of the half row sees every key
             float pt[32], ds[32];
 #pragma unroll
-            for (int c = 0; c < 32; ++c) {
-                const bool ok = kvalid && (plain || qc0 + c >= key);
+            for (int c = 0; c < 32; c += 4) {
+                const float4 l = *reinterpret_cast<const float4*>(rv + g * 32 + c);
+                const float ls[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
 #ifdef LLARK_ATC_ALIBI
-                const float p = ok ? ex2(fmaf(__uint_as_float(sv[c]), scale_log2,
-                                             fmaf(alibi_slopes[h] * LOG2E, (float)(key - (S - 1)), -rv[g * 32 + c]))) : 0.f;
+                    pt[c + e] = fmaf(__uint_as_float(sv[c + e]), scale_log2, fmaf(slope2, (float)(key - (S - 1)), -ls[e]));
 #else
-                const float p = ok ? ex2(fmaf(__uint_as_float(sv[c]), scale_log2, -rv[g * 32 + c])) : 0.f;
+                    pt[c + e] = fmaf(__uint_as_float(sv[c + e]), scale_log2, -ls[e]);
 #endif
-                pt[c] = p;
-                ds[c] = p * (__uint_as_float(dv[c]) - rv[64 + g * 32 + c]);
+            }
+            if (!plain) mask_columns(pt, kvalid ? ~first_columns(key - qc0) : 0u);
+#pragma unroll
+            for (int c = 0; c < 32; c += 4) {
+                const float4 d = *reinterpret_cast<const float4*>(rv + 64 + g * 32 + c);
+                const float dd[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    pt[c + e] = ex2(pt[c + e]);
+                    ds[c + e] = pt[c + e] * (__uint_as_float(dv[c + e]) - dd[e]);
+                }
             }
             if (t >= 2) {
                 mbar_wait(&pds_done[t & 1], (uint32_t)((t >> 1) - 1) & 1);  // tile t-2 retired: buffers t & 1 free
