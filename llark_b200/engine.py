@@ -198,13 +198,12 @@ class _StepFn(torch.autograd.Function):
             loss, logits = engine._forward(batch, need_grad=True)
         ctx.engine = engine
         ctx.mark_non_differentiable(logits)
-        ctx.set_materialize_grads(False)  # no zeros of the logits' size for a gradient that nobody reads
         return loss, logits
 
     @staticmethod
     def backward(ctx, dloss, _dlogits):
         with _Nvtx("llark.backward"):
-            ctx.engine._backward(torch.zeros((), device=ctx.engine.flat.params.device) if dloss is None else dloss)
+            ctx.engine._backward(dloss)
         return None, None, None
 
 
