@@ -7,9 +7,12 @@ OBJ := $(patsubst llark_b200/csrc/%.cu,build/%.o,$(SRC))
 LIB := llark_b200/libllark_b200.so
 
 # the subset a native checkpoint of a layer-list decoder needs: GEMM core, decode linears, generation-path ops
-SERVE_OBJ := build/gemm_tcgen05.o build/gemv.o build/skinny.o build/attn_step.o build/seq_ops.o build/seq_mixers.o build/seq_swa_mma.o build/seq_delta.o \
-             build/seq_latent.o build/seq_moe.o build/seq_decay.o build/seq_chunk.o
+SERVE_OBJ := build/gemm_tcgen05.o build/gemv.o build/skinny.o build/attn_step.o build/seq_ops.o build/seq_mixers.o build/seq_swa_mma.o \
+             build/seq_swa_tc.o build/seq_delta.o build/seq_latent.o build/seq_moe.o build/seq_decay.o build/seq_chunk.o
 LIB_SERVE := llark_b200/libllark_serve.so
+
+# a shared link accepts what it cannot resolve, and the library then fails to load: make that an error of the build
+LDFLAGS := -shared -Xlinker --no-undefined
 
 all: $(LIB)
 serve: $(LIB_SERVE)
@@ -26,10 +29,10 @@ build/attn_step.o build/attention.o build/seq_mixers.o: llark_b200/csrc/attn_ste
 build/attention_tc_alibi.o: llark_b200/csrc/attention_tc.cu
 
 $(LIB): $(OBJ)
-	$(NVCC) $(ARCH) -shared -o $@ $(OBJ) -lnccl
+	$(NVCC) $(ARCH) $(LDFLAGS) -o $@ $(OBJ) -lnccl
 
 $(LIB_SERVE): $(SERVE_OBJ)
-	$(NVCC) $(ARCH) -shared -o $@ $(SERVE_OBJ)
+	$(NVCC) $(ARCH) $(LDFLAGS) -o $@ $(SERVE_OBJ)
 
 clean:
 	rm -rf build $(LIB) $(LIB_SERVE)

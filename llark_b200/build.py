@@ -19,8 +19,10 @@ def _sources_newer_than(lib, names):
     return any(os.path.exists(p) and os.path.getmtime(p) > t for p in paths)
 
 
-SERVE_SOURCES = ("gemm_tcgen05.cu", "gemv.cu", "seq_ops.cu", "seq_mixers.cu", "seq_swa_mma.cu", "seq_delta.cu",
-                 "seq_latent.cu", "seq_moe.cu", "seq_decay.cu", "common.cuh")
+# what the Makefile's SERVE_OBJ is compiled from, headers included
+SERVE_SOURCES = ("gemm_tcgen05.cu", "gemv.cu", "skinny.cu", "attn_step.cu", "seq_ops.cu", "seq_mixers.cu", "seq_swa_mma.cu",
+                 "seq_swa_tc.cu", "seq_delta.cu", "seq_latent.cu", "seq_moe.cu", "seq_decay.cu", "seq_chunk.cu", "common.cuh",
+                 "skinny.cuh", "attn_step.cuh")
 
 
 def ensure_built(verbose=False):
