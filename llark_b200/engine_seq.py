@@ -68,13 +68,14 @@ class LayerListEngine:
             raise ValueError("token id outside the vocabulary")
         if want is None:
             want = [[n - 1] for n in lens]
-        rows, first = [], 0
-        for n, w in zip(lens, want):
+        rows, first = [], [0]
+        for n in lens:
+            first.append(first[-1] + n)
+        for b, w in enumerate(want):
             for k in w:
-                if k < 0 or k >= n:
+                if k < 0 or k >= lens[b]:  # IndexError for a request that is not in the step
                     raise ValueError("a wanted place lies outside the request's tokens")
-                rows.append(first + int(k))
-            first += n
+                rows.append(first[b] + int(k))
         st = cache.layout(slots, lens, extra=(flat, rows))
         ids, idx = st.extra
         x = self._embed(ids, st)

@@ -1,0 +1,44 @@
+"""The step of a layer-list engine on the host: what it refuses, and that a refused step leaves the caches as they were. The layers are
+stand-ins; the step descriptor and the caches are the product's."""
+import types
+
+import pytest
+import torch
+
+
+def _engine():
+    from llark_b200.engine_seq import LayerListEngine
+    from llark_b200.state_cache import StateCache
+
+    class Rows(LayerListEngine):
+        """Logits = the token at the wanted place, and its row."""
+        cfg, device = types.SimpleNamespace(vocab=50), torch.device("cpu")
+
+        def _embed(self, ids, st):
+            return torch.stack([ids.float(), torch.arange(st.n_tok).float()], 1)
+
+        def _run_layers(self, cache, x, st, residuals):
+            return x
+
+        def _logits(self, x, rows):
+            return x[rows.long()]
+
+    cache = StateCache("cpu", n_slots=3)
+    cache.add_store((2,), torch.float32, True)
+    return Rows(), cache, [cache.alloc(), cache.alloc()]
+
+
+def test_wanted_places_in_the_order_of_the_requests():
+    eng, cache, slots = _engine()
+    out = eng.step(cache, slots, [[3, 4, 5], [6, 7]], want=[[2, 0], [1]])
+    assert out.tolist() == [[5.0, 2.0], [3.0, 0.0], [7.0, 4.0]]
+    assert eng.step(cache, slots, [[8], [9]], want=[[0]]).tolist() == [[8.0, 0.0]]
+    assert eng.step(cache, slots, [[8], [9]], want=[[], [0], []]).tolist() == [[9.0, 1.0]]
+
+
+@pytest.mark.parametrize("want,error", [([[0], [0], [0]], IndexError), ([[3], [0]], ValueError), ([[0], [-1]], ValueError)])
+def test_wanted_places_outside_the_step_are_refused(want, error):
+    eng, cache, slots = _engine()
+    with pytest.raises(error):
+        eng.step(cache, slots, [[3, 4, 5], [6, 7]], want=want)
+    assert [cache.length[s] for s in slots] == [0, 0]
