@@ -168,7 +168,8 @@ int llark_gemv(const void* A, long long lda, const void* W, long long ldw, void*
 int llark_attn_decode(const void* q, const void* k_cache, const void* v_cache, const int* lens, void* out, int B,
                       int s_max, int n_heads, int head_dim, float scale, cudaStream_t stream);
 /* The same for rows that all stand at position pos, straight from the packed projection: qkv [B, ld] = q | k | v (RoPE applied). The
- * new key and value are taken from there and stored as entry pos of k_cache / v_cache [B, s_max, n_heads*128] by the same launch. */
+ * new key and value are taken from there and stored as entry pos of k_cache / v_cache [B, s_max <= 4096, n_heads*128] by the same
+ * launch. */
 int llark_attn_decode_packed(const void* qkv, long long ld, void* k_cache, void* v_cache, int pos, void* out, int B, int s_max,
                              int n_heads, int head_dim, float scale, cudaStream_t stream);
 long long llark_attn_bwd_workspace(int B, int S, int n_heads);

@@ -662,7 +662,7 @@ extern "C" int llark_attn_decode(const void* q, const void* k_cache, const void*
 
 extern "C" int llark_attn_decode_packed(const void* qkv, long long ld, void* k_cache, void* v_cache, int pos, void* out, int B,
                                         int s_max, int n_heads, int head_dim, float scale, cudaStream_t st) {
-    if (head_dim != HD || B <= 0 || n_heads <= 0 || pos < 0 || pos >= s_max || !qkv || !k_cache || !v_cache || !out || ld % 8 ||
+    if (head_dim != HD || B <= 0 || n_heads <= 0 || pos < 0 || pos >= s_max || s_max > DEC_MAX_LEN || !qkv || !k_cache || !v_cache || !out || ld % 8 ||
         ld < 3LL * n_heads * HD || !attnstep::fits(B, n_heads, n_heads, HD, qkv, k_cache, v_cache))
         return LLARK_EINVAL;
     attnstep::Args a = {};

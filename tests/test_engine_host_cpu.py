@@ -380,3 +380,14 @@ def test_stand_in_ops_track_the_real_signatures():
         used -= {"GEMM_PROFILE"}
         assert used <= offered, (path, sorted(used - offered))
 
+
+
+def test_decode_attention_refuses_stores_of_more_than_4096_entries():
+    """Both forms of the decode attention; the arguments are checked before anything is launched."""
+    from llark_b200 import _lib
+
+    if not os.path.exists(_lib.LIB_PATH):
+        pytest.skip("the library has not been built")
+    c = _lib.lib()
+    assert c.llark_attn_decode(16, 16, 16, 16, 16, 1, 4097, 1, 128, 0.1, None) == -1
+    assert c.llark_attn_decode_packed(16, 384, 16, 16, 0, 16, 1, 4097, 1, 128, 0.1, None) == -1
