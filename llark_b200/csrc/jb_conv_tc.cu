@@ -21,7 +21,6 @@
 // writes every value once; the tensor pipe works a quarter of the time). Measured on a B200, 4 clips x 524288 steps x 32 channels, a
 // res block: 257 us for dilations up to 64 and 346 at 81, with mma.sync 413 and 685. Three groups of four warps and not more: 168
 // registers a thread hold a step's 32 channels, the next step's and the sums; two groups with the input staged by cp.async: 325.
-//
 #include "common.cuh"
 
 namespace llark {
@@ -29,8 +28,8 @@ extern thread_local int g_last_cuda_error;
 namespace jbconv {
 
 constexpr int TT = 128;        // time steps per tile = threads of a group = TMEM lanes
-constexpr int kMaxDil = 81;    // two groups' rows fit into shared memory up to 81; three groups' up to 64
-constexpr int kMaxDil3 = 64;   // halo rows: one for every thread
+constexpr int kMaxDil = 81;    // two groups: the largest power of three whose halo rows (at most 256) two passes of 128 threads cover
+constexpr int kMaxDil3 = 64;   // three groups: halo rows one for every thread, and the end of shared memory
 
 struct Args {
     const float *x, *w1, *b1, *w2, *b2;
@@ -44,9 +43,13 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {  // 128-byte rows
 __device__ __forceinline__ uint32_t idesc_tf32(int n) {  // fp32 sums, both operands TF32 and K-major, M = 128
     return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TT >> 4) << 24);
 }
+// The leading part is rounded on its bits. The NaN of the GPU's own arithmetic (0x7fffffff) becomes -0 there, so the other part has to
+// keep it, and is not rounded on its bits: the tensor cores cut the 13 bits that TF32 lacks, and times 1 + 2^-11.5 before that cut an
+// error is 0.65 units of the last place at most and 0 on average (cvt.rna.tf32 for both parts is as exact and 6 % slower: 3471 us for the
+// encoder of 4 clips against 3263).
 __device__ __forceinline__ void split(float v, float& hi, float& lo) {
-    hi = __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u);  // rounded to nearest: |v - hi| <= 2^-12 |v|
-    lo = __uint_as_float((__float_as_uint(v - hi) + 0x1000u) & 0xffffe000u);  // the difference is exact: |v - hi - lo| <= 2^-24 |v|
+    hi = __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u);  // |v - hi| <= 2^-11 |v|
+    lo = (v - hi) * 1.00034527f;                                          // the difference is exact: |v - hi - lo| < 2^-21 |v|
 }
 // 32 values as row r of a region, split into its two parts, lo_at bytes apart
 template <bool RELU>
@@ -92,6 +95,23 @@ __device__ __forceinline__ void products(uint32_t a, int lo_at, uint32_t w, uint
             umma_tf32(mid, ah + o, wl + o, idesc_tf32(COUT), !fl);
         }
         umma_tf32(mid, al + o, wh + o, idesc_tf32(COUT), 1);
+    }
+}
+
+// One step's sums of 32 output channels by FMAs, bias first, channels outside, taps inside: for steps whose split products are not
+// finite. An infinite value, or one that rounds to infinity, has a low part that is NaN, and infinity times a low part is another
+// infinity or NaN: what belongs there is what the FMAs give. Nothing but such values gets here.
+template <int TAPS, int STRIDE, int CIN>
+__device__ __noinline__ void step_by_fma(const float* x, const float* w, const float* b, int T, int t, float (&h)[32]) {
+#pragma unroll 1
+    for (int c = 0; c < 32; ++c) {
+        float acc = b[c];
+#pragma unroll 1
+        for (int i = 0; i < CIN * TAPS; ++i) {
+            const int ci = i / TAPS, at = STRIDE * t + (i % TAPS) - 1;
+            acc = fmaf(w[(long long)c * CIN * TAPS + i], at >= 0 && at < T ? x[(long long)ci * T + at] : 0.f, acc);
+        }
+        h[c] = acc;
     }
 }
 
@@ -258,12 +278,22 @@ conv_kernel(const Args p) {
         } else {
 #pragma unroll
             for (int c0 = 0; c0 < COUT; c0 += 32) {
-                float h[32];
+                float h[32], odd = 0.f;
                 read_sums(c0, h);
+#pragma unroll
+                for (int c = 0; c < 32; ++c) {
+                    h[c] += sb[c0 + c];
+                    odd = fmaf(h[c], 0.f, odd);  // NaN as soon as one of them is not finite
+                }
+                if (odd != 0.f && t < p.To) {
+                    float f[32];
+                    step_by_fma<TAPS, STRIDE, CIN>(p.x + (long long)clip * CIN * p.T, p.w1 + c0 * CIN * TAPS, p.b1 + c0, p.T, t, f);
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) h[c] = f[c];
+                }
                 if (t < p.To)
 #pragma unroll
-                    for (int c = 0; c < 32; ++c)
-                        out[(long long)(c0 + c) * p.To] = h[c] + sb[c0 + c];
+                    for (int c = 0; c < 32; ++c) out[(long long)(c0 + c) * p.To] = h[c];
             }
         }
     }
@@ -281,7 +311,9 @@ static int launch(Args a, int N, cudaStream_t st) {
     a.tiles = a.tiles_per_clip * N;
     const int grid = a.tiles < 148 * NG ? (a.tiles + NG - 1) / NG : 148;
     auto kernel = conv_kernel<TAPS, STRIDE, NCI, COUT, RES, NG>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    // the limit is the function's, and another thread may launch it with another dilation: always the largest size
+    const int most_rows = RES ? (TT + 2 * (NG == 3 ? kMaxDil3 : kMaxDil) + 7) & ~7 : a.rows;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem + NG * STRIDE * 2 * (most_rows - a.rows) * 128);
     if (e == cudaSuccess) {
         kernel<<<grid, NG * TT, smem, st>>>(a);
         e = cudaGetLastError();

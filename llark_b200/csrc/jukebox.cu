@@ -746,10 +746,16 @@ static int set_dyn_smem(const void* fn, int bytes) {
 
 using namespace llark;
 
+// LLARK_JB_CONV_TC=0 selects the fp32 FMA kernels for every convolution of the encoder (read per call: tests toggle it)
+static bool use_conv_tc() {
+    const char* e = getenv("LLARK_JB_CONV_TC");
+    return !(e && e[0] == '0');
+}
+
 extern "C" int llark_jb_conv_down(const float* x, const float* w, const float* bias, float* y, int N, int c_in,
                                   int c_out, int T, cudaStream_t st) {
     if (N <= 0 || T <= 0 || (T & 1) || c_in <= 0 || (c_out != 32 && c_out != 64)) return LLARK_EINVAL;
-    if (jbconv::takes_down(c_in, c_out)) return jbconv::down(x, w, bias, y, N, c_in, T, st);
+    if (use_conv_tc() && jbconv::takes_down(c_in, c_out)) return jbconv::down(x, w, bias, y, N, c_in, T, st);
     int rc;  // one channel in (the waveform), or other widths: memory-bound or small
     if (c_out == 32) {
         constexpr int TILE = DownCfg<32>::Tile::TILE_T;
@@ -772,9 +778,7 @@ extern "C" int llark_jb_conv_down(const float* x, const float* w, const float* b
 extern "C" int llark_jb_resblock(const float* x, const float* w1, const float* b1, const float* w2, const float* b2,
                                  float* y, int N, int T, int dilation, cudaStream_t st) {
     if (N <= 0 || T <= 0 || dilation < 1 || dilation > 243) return LLARK_EINVAL;
-    const char* tc_env = getenv("LLARK_JB_CONV_TC");  // "0" selects the fp32 SIMT kernel (read per call: tests toggle it)
-    const int use_tc = (tc_env && tc_env[0] == '0') ? 0 : 1;
-    if (use_tc && jbconv::takes_resblock(dilation)) return jbconv::resblock(x, w1, b1, w2, b2, y, N, T, dilation, st);
+    if (use_conv_tc() && jbconv::takes_resblock(dilation)) return jbconv::resblock(x, w1, b1, w2, b2, y, N, T, dilation, st);
     const int smem = (32 * (RES_TT + 2 * dilation) + 32 * RES_TT + 32 * 32 * 3 + 32 * 32) * (int)sizeof(float);
     int rc = set_dyn_smem((const void*)resblock_kernel, smem);
     if (rc) return rc;
@@ -786,7 +790,7 @@ extern "C" int llark_jb_resblock(const float* x, const float* w1, const float* b
 extern "C" int llark_jb_conv_k3(const float* x, const float* w, const float* bias, float* y, int N, int c_in, int c_out,
                                 int T, cudaStream_t st) {
     if (N <= 0 || T <= 0 || c_in <= 0 || (c_out != 32 && c_out != 64)) return LLARK_EINVAL;
-    if (jbconv::takes_k3(c_in, c_out)) return jbconv::k3(x, w, bias, y, N, T, st);
+    if (use_conv_tc() && jbconv::takes_k3(c_in, c_out)) return jbconv::k3(x, w, bias, y, N, T, st);
     int rc;
     if (c_out == 64) {
         constexpr int TILE = K3Cfg<64>::Tile::TILE_T;

@@ -186,7 +186,7 @@ def test_label_conditioning_on_gpu_matches_oracle_and_feeds_the_prior():
 
 @pytest.mark.parametrize("d", [1, 3, 9, 27])
 def test_resblock_tensor_core_kernel_matches_simt_and_fp64(d):
-    """The 3xTF32 mma.sync res-block (default) against the fp32 SIMT kernel (LLARK_JB_CONV_TC=0) and an fp64 conv1d
+    """The split-TF32 res-block (default) against the fp32 SIMT kernel (LLARK_JB_CONV_TC=0) and an fp64 conv1d
     reference: both must sit at fp32 rounding level (the 3x split keeps ~22 mantissa bits), on a time length that is not a
     multiple of the 256-step tile and with the dilation's halo crossing tile borders."""
     import torch.nn.functional as F
@@ -241,6 +241,64 @@ def test_convolutions_at_the_edges_of_their_tiles_match_fp64(kind, c_in, T):
         h = F.conv1d(F.relu(xd), w1.double(), b1.double(), padding=d, dilation=d)
         ref = xd + F.conv1d(F.relu(h), w2.double(), b2.double())
     assert _rel(got.cpu(), ref) < 1e-6
+
+
+def _by_fma(fn, *args):
+    """fn with the FMA kernels of the encoder's convolutions."""
+    os.environ["LLARK_JB_CONV_TC"] = "0"
+    try:
+        return fn(*args)
+    finally:
+        os.environ.pop("LLARK_JB_CONV_TC", None)
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf"), 3.4e38, -3.4027e38])
+@pytest.mark.parametrize("kind,c_in", [("down", 32), ("down", 64), ("k3", 32)])
+def test_values_that_do_not_split_come_out_where_conv1d_puts_them(kind, c_in, bad):
+    """NaN, infinities and numbers whose leading part rounds to infinity: exactly the steps that see them differ, as sums of products
+    have it; a NaN of the GPU's own arithmetic (0x7fffffff) too. All other steps keep their split products (1e-6, as above)."""
+    import torch.nn.functional as F
+
+    from llark_b200 import ops
+
+    g = torch.Generator().manual_seed(c_in)
+    T, c_out, taps = 300, 64 if kind == "k3" else 32, 3 if kind == "k3" else 4
+    x = torch.randn(2, c_in, T, generator=g)
+    w = torch.randn(c_out, c_in, taps, generator=g) / (taps * c_in)
+    w[0, 5] = 0.0  # 0 times infinity
+    b = torch.randn(c_out, generator=g) * 0.1
+    x[0, 5, 0], x[0, 7, 131], x[1, c_in - 1, T - 1] = bad, bad, bad
+    xc = x.cuda()
+    if bad != bad:
+        xc[0, 7, 131] = (torch.full((1,), float("inf"), device="cuda") - float("inf"))[0]
+    op = ops.jb_conv_k3 if kind == "k3" else ops.jb_conv_down
+    got = op(xc, w.cuda(), b.cuda()).cpu()
+    ref = F.conv1d(x.double(), w.double(), b.double(), stride=1 if kind == "k3" else 2, padding=1).float()
+    assert torch.equal(got.isnan(), ref.isnan()) and torch.equal(got.isinf(), ref.isinf())
+    assert torch.equal(got[got.isinf()], ref[ref.isinf()])
+    ok = ref.isfinite()
+    big = ok & (ref.abs() > 1e30)
+    assert big.any() == (abs(bad) < float("inf"))
+    # fp32 sums of at most 256 products
+    assert ((got[ok].double() - ref[ok].double()).abs() <= 256 * 2.0 ** -24 * F.conv1d(
+        x.nan_to_num(0, 0, 0).abs().double(), w.abs().double(), b.abs().double(), stride=1 if kind == "k3" else 2, padding=1)[ok]).all()
+    if abs(bad) > 3.402e38:  # rounds to infinity: these steps are sums of FMAs
+        assert torch.equal(_by_fma(op, xc, w.cuda(), b.cuda()).cpu()[big], got[big])
+
+
+def test_a_nan_sample_stays_nan_through_the_encoder():
+    """From the second level on the activations' NaN is the one the GPU's arithmetic gives; relu(NaN) is 0 in the res blocks (fmaxf), so
+    the latents that see it through the residual sums are NaN, with either kind of kernel."""
+    jo, ocfg, cfg = _cfgs()
+    from llark_b200.jukebox.model import JukeboxVQVAE
+
+    m = JukeboxVQVAE(cfg, jo.init_vqvae_params(ocfg, seed=0))
+    audio = torch.rand(1, 1, ocfg.sample_length, generator=torch.Generator().manual_seed(5)) * 2 - 1
+    audio[0, 0, ocfg.sample_length // 2] = float("nan")
+    got = m.encode_top_latents(audio.cuda())
+    want = _by_fma(m.encode_top_latents, audio.cuda())
+    assert want.isnan().any() and not want.isnan().all()
+    assert torch.equal(got.isnan(), want.isnan())
 
 
 @pytest.mark.parametrize("T,n_codes", [(1, 5), (64, 2048), (65, 2047), (200, 37)])
