@@ -188,6 +188,10 @@ def _op_work(name, a, k, out, ctx):
         q, lens_ctx = a[0], ctx["context"]
         B, H = q.shape
         return 2 * B * lens_ctx * H * 2 + 2 * _nbytes(q), 4.0 * B * lens_ctx * H
+    if name == "attn_decode_packed":
+        qkv, pos = a[0], a[3]
+        B, H = qkv.shape[0], qkv.shape[1] // 3
+        return 2 * B * (pos + 1) * H * 2 + _nbytes(qkv) + _nbytes(out), 4.0 * B * (pos + 1) * H
     if name == "seq_glr_scan":
         src, state, st, H, D, E = a[0], a[5], a[6], a[7], a[8], a[9]
         return _nbytes(src) + 2 * st.n_seq * H * D * E * 4 + st.n_tok * H * E * 4, 5.0 * st.n_tok * H * D * E
@@ -198,6 +202,10 @@ def _op_work(name, a, k, out, ctx):
         vec, v, state, st, H, D, E = a[0], a[1], a[2], a[3], a[4], a[5], a[6]
         per = 9.0 if k.get("correct", True) else 5.0  # without the correction: decay, write and read-out only
         return (_nbytes(vec) + st.n_tok * H * E * 8 + 2 * st.n_seq * H * D * E * 4), per * st.n_tok * H * D * E
+    if name == "seq_delta_rule":  # from the projections: q, k, values, decays and mixes in, o out, the state once in and out
+        rule, st, H, D, E = a[0], a[7], a[8], a[10], a[11]
+        per = 5.0 if rule == 3 else 9.0
+        return (sum(_nbytes(x) for x in a[1:6]) + st.n_tok * H * E * 4 + 2 * st.n_seq * H * D * E * 4), per * st.n_tok * H * D * E
     if name == "seq_moe_experts":
         x, ids, wup, wd = a[0], a[1], a[2], a[3]
         n_ent, (n_exp, n_up, C), ff = ids.numel(), wup.shape, wd.shape[2]
@@ -256,11 +264,11 @@ def op_table(records, ctx, peaks):
 
 KELUTAR_OPS = ["linear", "seq_embed", "seq_short_conv", "seq_add_rmsnorm", "seq_rmsnorm_rows", "seq_relu2",
                "seq_qk_headnorm", "seq_swa_attn", "seq_kv_ring_write", "seq_glr_scan", "seq_head_rmsnorm"]
-LLAMA_OPS = ["gemm", "gemv", "rmsnorm_fwd", "rope_", "attn_fwd", "attn_decode", "swiglu_fwd", "embed_splice_fwd"]
+LLAMA_OPS = ["gemm", "rmsnorm_fwd", "rope_", "attn_fwd", "attn_decode_packed", "swiglu_fwd", "embed_splice_fwd"]
 
 
 GOLAVIK_OPS = ["linear", "linear_w32", "seq_embed", "seq_short_conv", "seq_group_rmsnorm", "seq_residual_combine",
-               "seq_conv_act", "seq_delta_prep", "seq_delta_scan", "seq_head_norm_gate", "seq_latent_prep",
+               "seq_conv_act", "seq_delta_prep", "seq_delta_scan", "seq_delta_rule", "seq_head_norm_gate", "seq_latent_prep",
                "seq_head_linear", "seq_swa_attn", "seq_kv_ring_write", "seq_moe_route", "seq_moe_experts", "seq_tanh"]
 
 # (name, width, layers, heads, head dim, window, experts, top, expert ff, latent rank, rotated size, vocab): layers repeat
@@ -412,7 +420,7 @@ def run_golavik(args, peaks, peaks_kind, emit):
 
 
 GUBULORN_OPS = ["linear", "linear_w32", "seq_embed", "seq_post_norm", "seq_rmsnorm_rows", "seq_conv_act", "seq_delta_prep",
-                "seq_delta_scan", "seq_head_norm_gate", "seq_skip_gate_group_norm", "seq_qkv_headnorm", "seq_swa_attn",
+                "seq_delta_scan", "seq_delta_rule", "seq_head_norm_gate", "seq_skip_gate_group_norm", "seq_qkv_headnorm", "seq_swa_attn",
                 "seq_kv_ring_write", "seq_moe_route", "seq_moe_experts", "seq_glu_clamped", "seq_logit_cap_"]
 
 # (name, width, layers, heads, head dim, experts, pass-through experts, top, expert ff, state-space heads, state size,

@@ -18,7 +18,7 @@ import os
 import torch
 
 from . import ops
-from .ops import LINEAR_FEW_MAX, attn_decode_packed
+from .ops import LINEAR_FEW_MAX
 
 BF16 = torch.bfloat16
 _ALIGN = 128  # elements (256 B): keeps every view 16-byte aligned for TMA and fused views gap-free
@@ -489,8 +489,7 @@ class LlamaEngine:
         cos, sin = self._tables(cache.s_max, dev)
         cos_t, sin_t = cos[t:], sin[t:]  # row 0 of these views is position t: with S = 1 every row reads it
         cache.lens.fill_(t + 1)
-        # the fused forms (gate times up in the product, keys and values stored by the attention) exist on the device only
-        few = x.is_cuda and B <= LINEAR_FEW_MAX and H % 8 == 0 and I % 8 == 0
+        few = B <= LINEAR_FEW_MAX and H % 8 == 0 and I % 8 == 0  # gate times up in the product's epilogue
         rstd = torch.empty(B, device=dev, dtype=torch.float32)
         for l in range(L):
             pfx = f"model.layers.{l}."
@@ -504,12 +503,7 @@ class LlamaEngine:
             else:
                 qkv = ops.gemm(xn1, Wqkv)
                 ops.rope_(qkv, cos_t, sin_t, 1, NH, D)
-            if x.is_cuda:
-                attn = attn_decode_packed(qkv, cache.k[l], cache.v[l], t, NH, D)
-            else:
-                cache.k[l][:, t].copy_(qkv[:, H:2 * H])
-                cache.v[l][:, t].copy_(qkv[:, 2 * H:])
-                attn = ops.attn_decode(qkv[:, :H].contiguous(), cache.k[l], cache.v[l], cache.lens, NH, D)
+            attn = ops.attn_decode_packed(qkv, cache.k[l], cache.v[l], t, NH, D)
             x_mid = ops.gemm(attn, Wo, residual=x)
             xn2 = ops.rmsnorm_fwd(x_mid, flat.pview(pfx + "post_attention_layernorm.weight"), eps, rstd=rstd)
             act = ops.gemm(xn2, Wgu, swiglu=True) if few else ops.swiglu_fwd(ops.gemm(xn2, Wgu))

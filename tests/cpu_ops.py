@@ -136,6 +136,13 @@ def attn_decode(q, k_cache, v_cache, lens, n_heads, head_dim, out=None):
     return res
 
 
+def attn_decode_packed(qkv, k_cache, v_cache, pos, n_heads, head_dim, out=None):
+    B, H = k_cache.shape[0], k_cache.shape[2]
+    k_cache[:, pos].copy_(qkv[:, H:2 * H])
+    v_cache[:, pos].copy_(qkv[:, 2 * H:])
+    return attn_decode(qkv[:, :H], k_cache, v_cache, torch.full((B,), pos + 1), n_heads, head_dim)
+
+
 def swiglu_fwd(gu, act=None):
     I = gu.shape[1] // 2
     g, u = gu[:, :I].float(), gu[:, I:].float()
@@ -167,7 +174,9 @@ _gemm_fwd = gemm
 
 
 def gemm(a, b, **kw):  # noqa: F811
-    """Adds the SwiGLU-backward epilogue and residual-into-out accumulation to the forward stand-in."""
+    """Adds the SwiGLU epilogues and residual-into-out accumulation to the forward stand-in."""
+    if kw.pop("swiglu", False):
+        return swiglu_fwd(_gemm_fwd(a, b, **kw))
     gu = kw.pop("swiglu_bwd", None)
     if gu is None:
         return _gemm_fwd(a, b, **kw)

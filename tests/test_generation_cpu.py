@@ -78,3 +78,27 @@ def test_greedy_loop_batch_padding_and_limits():
     assert torch.equal(greedy_generate(step, ids, 0, eos_token_id=[9]), ids)
     with pytest.raises(ValueError):
         greedy_generate(step, ids[0], 2)
+
+
+def test_every_op_of_the_generation_path_is_in_its_table_of_times():
+    """The benchmark's per-op tables wrap ops by name: an op that a mixer, an engine or the Llama decode step calls and no list names
+    would be missing from its model's table, time and all."""
+    import ast
+
+    from llark_b200 import bench_generation as bench, ops
+
+    def called(tree):
+        return {n.func.attr for n in ast.walk(tree) if isinstance(n, ast.Call) and isinstance(n.func, ast.Attribute)
+                and isinstance(n.func.value, ast.Name) and n.func.value.id == "ops"}
+
+    def parse(path):
+        return ast.parse(open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "llark_b200", path)).read())
+
+    lists = {k: v for k, v in vars(bench).items() if k.endswith("_OPS")}
+    assert all(hasattr(ops, n) for names in lists.values() for n in names)
+    named = {n for names in lists.values() for n in names}
+    host = {"decay_powers"}  # a table made once, when the weights are laid out
+    assert called(parse("mixers.py")) <= named | host
+    decode = next(f for f in ast.walk(parse("engine.py")) if isinstance(f, ast.FunctionDef) and f.name == "decode_step")
+    assert called(decode) <= set(bench.LLAMA_OPS)
+    assert "attn_decode_packed" in called(decode)
