@@ -156,7 +156,7 @@ attn_step_kernel(const Args p, int cs) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int x = e & 1;
-            const float pr = m[x] == -INFINITY ? 0.f : exp2f(s[e] - m[x]);
+            const float pr = exp2f(s[e] - (m[x] == -INFINITY ? 0.f : m[x]));  // 0 for -inf, NaN stays
             l[x] += pr;
             if (2 * t + x < HG) sp[warp][2 * t + x][g + (e >> 1) * 8] = pr;
         }

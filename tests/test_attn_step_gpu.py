@@ -90,3 +90,39 @@ def test_packed_projection_is_that_of_the_stores(B, S, NH, pos):
     assert torch.equal(k, want_k) and torch.equal(v, want_v)
     lens = torch.full((B,), pos + 1, device="cuda", dtype=torch.int32)
     assert torch.equal(got, ops.attn_decode(qkv[:, :H].contiguous(), want_k, want_v, lens, NH, 128))
+
+
+@pytest.mark.parametrize("D,H,G", [(128, 4, 1), (64, 4, 4), (256, 4, 2)])
+def test_scores_that_are_not_numbers_reach_the_result(D, H, G):
+    """A query that is NaN beside a sink, and sixteen keys that are NaN, all that one warp takes at a time: NaN for the heads that read
+    them; scores of minus infinity weigh nothing; other requests and heads as without."""
+    from llark_b200 import ops
+
+    torch.manual_seed(D)
+    n, cap, nan, inf, dev = 4, 200, float("nan"), float("inf"), "cuda"
+    ints = lambda v: torch.tensor(v, device=dev, dtype=torch.int32)  # noqa: E731
+    st = types.SimpleNamespace(n_tok=n, n_seq=n, max_len=1, tok_seq=ints(range(n)), cu=ints(range(n + 1)), pos0=ints([70] * n), slot=ints(range(n)))
+    q, k, v = (torch.randn(*s, device=dev).to(BF16) for s in ((n, H, D), (n, cap, G, D), (n, cap, G, D)))
+    scale, sink = torch.full((H,), 0.1, device=dev), torch.randn(H, device=dev)
+
+    def run(q, k):
+        return ops.seq_swa_attn(q.view(n, H * D), None, None, k.view(n, cap, G * D), v.view(n, cap, G * D), None, 0, scale, st, H, G, D, D, cap,
+                                cap, from_ring_only=True, sink=sink).view(n, H, D)
+
+    want = run(q, k)
+    q2, k2 = q.clone(), k.clone()
+    q2[0, 1, 3] = nan
+    k2[1, 16:32, 0, :] = nan
+    q2[3, :, 0], k2[3, :, :, 0] = 1.0, 0.0
+    k2[3, :50, :, 0] = -inf
+    got = run(q2, k2)
+    heads = torch.arange(H, device=dev)
+    assert torch.equal(got[0].isnan().all(1), heads == 1) and torch.equal(got[0].isnan().any(1), heads == 1)
+    assert torch.equal(got[1].isnan().all(1), heads < H // G) and torch.equal(got[1].isnan().any(1), heads < H // G)
+    keep = torch.ones(n, H, dtype=torch.bool, device=dev)
+    keep[0, 1], keep[1, :H // G], keep[3] = False, False, False
+    assert torch.equal(got[keep], want[keep])
+    s = torch.einsum("hd,jhd->hj", q2[3].to(F64), k2[3, 50:71].repeat_interleave(H // G, 1).to(F64)) * 0.1
+    w = torch.softmax(torch.cat([s, sink.to(F64)[:, None]], 1), 1)[:, :-1]
+    ref = torch.einsum("hj,jhd->hd", w, v[3, 50:71].repeat_interleave(H // G, 1).to(F64))
+    assert ((got[3].to(F64) - ref).norm() / ref.norm()).item() < 2.0 ** -8
