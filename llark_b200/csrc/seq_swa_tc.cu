@@ -66,8 +66,30 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 
+// 32 channels of one query's weighted sum of values by FMAs, over the keys lo .. hi that it sees (counted as in the kernel; m: its
+// largest score): for rows in whose key tiles a value is infinite or NaN, since the products multiply what a row does not see by 0, and
+// that is NaN. Only a row whose own scores are finite gets here.
+__device__ __noinline__ void sum_by_fma(const Args& a, const bf16_t* q, int row0, int n_ring, int ring0, long long ring_base, int g, int lo,
+                                        int hi, float sc, float m, int c0, float (&o)[32]) {
+#pragma unroll 1
+    for (int e = 0; e < 32; ++e) o[e] = 0.f;
+#pragma unroll 1
+    for (int k = lo; k <= hi; ++k) {
+        const bool old = k < n_ring;
+        const int e = ring0 + k;
+        const long long at = ((old ? ring_base + (e >= a.cap ? e - a.cap : e) : (long long)row0 + k - n_ring) * a.G + g) * HD;
+        const bf16_t *kr = (old ? a.kring : a.kn) + at, *vr = (old ? a.vring : a.vv) + at + c0;
+        float s = 0.f;
+#pragma unroll 1
+        for (int c = 0; c < HD; ++c) s = fmaf(__bfloat162float(q[c]), __bfloat162float(kr[c]), s);
+        const float p = ex2(s * sc - m);
+#pragma unroll 1
+        for (int c = 0; c < 32; ++c) o[c] = fmaf(p, __bfloat162float(vr[c]), o[c]);
+    }
+}
+
 __global__ void __launch_bounds__(kThreads, 2)
-swa_tc_kernel(const Args a) {
+swa_tc_kernel(const __grid_constant__ Args a) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ uint64_t bars[2 * kSlots + 6];
     __shared__ uint32_t tmem_slot;
@@ -281,6 +303,16 @@ swa_tc_kernel(const Args a) {
             uint32_t o[32];
             tmem_ld_32x32b_x32(lane0 + 128 + c * 32, o);
             tmem_ld_wait();
+            float odd = 0.f;  // NaN as soon as one of them is not finite
+#pragma unroll
+            for (int e = 0; e < 32; ++e) odd = fmaf(__uint_as_float(o[e]), 0.f, odd);
+            if (ok && odd != 0.f && l < INFINITY) {
+                float f[32];
+                sum_by_fma(a, a.qn + (trow * a.H + h) * HD, row0, n_ring, (int)(k_lo % a.cap), (long long)a.slot[b] * a.cap, g, lo, hi, sc, m,
+                           c * 32, f);
+#pragma unroll
+                for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(f[e]);
+            }
             if (ok) {
                 if (a.gate && !a.gate_per_head) {
                     const float* gp = a.gate + trow * a.gate_ld + h * HD + c * 32;

@@ -62,3 +62,40 @@ def test_against_64_bits(H, G, lens, pos, cap, window, chunk, extra):
         err = (o[a:a + ln].view(ln, H, D).to(F64) - want).abs()
         assert (err <= 1.05 * bound).all(), (b, (err / bound).max().item())
     assert out is None or wide[:, :8].abs().max().item() == 0
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("pos,window,chunk", [(0, 1 << 30, 0), (90, 100, 0), (64, 1 << 30, 128)])
+def test_values_that_are_not_finite_reach_the_rows_that_see_them_only(pos, window, chunk, bad):
+    """A value row that is infinite or NaN, of the step and of the ring: queries in front of it and behind its window, in the same tile of
+    the products, are as without it."""
+    from llark_b200 import ops
+    from llark_b200.state_cache import StepLayout
+
+    torch.manual_seed(pos)
+    H, G, D, n, cap, dev = 2, 1, 128, 300, 512, "cuda"
+    st = StepLayout([n], [pos], [0], dev)
+    q, k, v = (torch.randn(n, x * D, device=dev).to(BF16) for x in (H, G, G))
+    kring, vring = (torch.randn(1, cap, G * D, device=dev).to(BF16) for _ in range(2))
+    scale = torch.full((H,), 0.1, device=dev)
+
+    def run(v, vring):
+        return ops.seq_swa_attn(q, k, v, kring, vring, None, 0, scale, st, H, G, D, D, window, cap, from_ring_only=False, chunk=chunk).view(n, H, D)
+
+    want = run(v, vring)
+    v2, vring2 = v.clone(), vring.clone()
+    at = [pos + 37, pos + 200] + ([pos - 8] if pos else [])  # positions; channels 5, 40 and 70
+    v2[37, 5], v2[200, 40] = bad, -bad
+    if pos:
+        vring2[0, pos - 8, 70] = bad
+    got = run(v2, vring2)
+    qp = torch.arange(pos, pos + n, device=dev)
+    hit = torch.zeros(n, D, dtype=torch.bool, device=dev)
+    for p, c in zip(at, (5, 40, 70)):
+        hit[:, c] = (qp >= p) & ((qp // chunk == p // chunk) if chunk else (qp - p < window))
+    hit = hit[:, None].expand(n, H, D)
+    assert not got[hit].isfinite().any() and got[~hit].isfinite().all()
+    if bad == float("inf"):
+        assert got[hit].isinf().all()
+    # beside them either the products' result or, in tiles that hold one, sums of FMAs: P is rounded to eight bits in the former
+    assert ((got[~hit].float() - want[~hit].float()).norm() / want[~hit].float().norm()).item() < 2.0 ** -7
