@@ -295,7 +295,8 @@ skinny_kernel(const Args p, int cs) {
 // ------------------------------------------------------------------------------------------------ more tokens
 // From nine tokens on the fragments of A that every warp of the kernel above reads again fill the shared-memory pipe (64 tokens:
 // 2.3x the memory time). Here the same slices go to tcgen05.mma: 128 weight rows are its M side, up to NTOK tokens its N side, the
-// sums lie in NTOK columns of TMEM.
+// sums lie in NTOK columns of TMEM. CH: every CH slices the products start from zero, in one of two sets of columns, and are added up
+// in registers while the next ones are multiplied (CH 0: one chain over K, 2 to 9e-6 of the result where fp32 FMAs give 1e-7).
 constexpr int TN = 128, TRP = TN + 4;
 template <int NTOK> constexpr int kStages = NTOK <= 16 ? 6 : NTOK <= 32 ? 5 : 4;  // 108, 100, 96 KB: two CTAs per SM
 
@@ -303,12 +304,20 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {  // 8-row groups 
     return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
-template <int NTOK, typename TC, bool GROUPED>
+__device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr));
+}
+
+template <int NTOK, typename TC, bool GROUPED, int CH>
 __global__ void __launch_bounds__(kThreads)
 skinny_tc_kernel(const Args p, int cs) {
     extern __shared__ unsigned char smraw_[];
     constexpr int kStage = TN * 128 + NTOK * 128, S = kStages<NTOK>;
-    constexpr int kCols = NTOK < 32 ? 32 : NTOK;
+    constexpr int kCols = CH ? 2 * NTOK : NTOK < 32 ? 32 : NTOK;
     __shared__ uint64_t done[S];
     __shared__ uint32_t tmem_base;
     unsigned char* smraw = smraw_ + ((1024u - (smem_u32(smraw_) & 1023u)) & 1023u);
@@ -377,38 +386,55 @@ skinny_tc_kernel(const Args p, int cs) {
     const uint32_t tmem = tmem_base;
     // fp32 sums, bf16 operands, both K-major, M = 128, N = m_pad
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(m_pad >> 3) << 17) | ((uint32_t)(TN >> 4) << 24);
+    auto set = [](int it) { return CH ? it / (CH ? CH : 1) % 2 * NTOK : 0; };  // the columns of a slice's products
+    float sum[NTOK];  // of weight row warp * 32 + lane
+#pragma unroll
+    for (int j = 0; j < NTOK; ++j) sum[j] = 0.f;
+    auto add = [&](int it) {  // the sums up to slice `it`, whose products have been waited for
+        tc_fence_after();
+        constexpr int NL = NTOK < 32 ? NTOK : 32;
+#pragma unroll
+        for (int c0 = 0; c0 < NTOK; c0 += NL) {
+            if (c0 >= m_pad) break;  // the same for everybody
+            uint32_t v[NL];
+            const uint32_t at = tmem + ((uint32_t)(warp * 32) << 16) + set(it) + c0;
+            if constexpr (NL == 16)
+                tmem_ld_32x32b_x16(at, v);
+            else
+                tmem_ld_32x32b_x32(at, v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < NL; ++j) sum[c0 + j] += __uint_as_float(v[j]);  // columns from m_pad on hold nothing and are not used
+        }
+        tc_fence_before();
+    };
     int st = 0, st_in = S - 1;
     for (int it = 0; it < n; ++it) {
         asm volatile("cp.async.wait_group %0;" ::"n"(S - 2) : "memory");
         fence_proxy_async_smem();
-        __syncthreads();  // slice `it` is there, written by everybody
+        __syncthreads();  // slice `it` is there, written by everybody; everybody has taken the sums before those of slice it - 1
         if (threadIdx.x == 0) {
+            tc_fence_after();
             const uint64_t wd = smem_desc(sm + st * kStage), ad = smem_desc(sm + st * kStage + TN * 128);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) umma_f16(tmem, wd + (uint64_t)(k * 2), ad + (uint64_t)(k * 2), idesc, (it | k) != 0);
+            for (int k = 0; k < 4; ++k)
+                umma_f16(tmem + set(it), wd + (uint64_t)(k * 2), ad + (uint64_t)(k * 2), idesc, (CH ? it % (CH ? CH : 1) : it) != 0 || k != 0);
             umma_commit(&done[st]);
         }
-        if (it + S - 1 < n) {
-            if (it) mbar_wait(&done[st_in], (uint32_t)(((it - 1) / S) & 1));  // the slice before, whose place this one takes
-            issue(it + S - 1, st_in);
-        }
+        if (it) mbar_wait(&done[st_in], (uint32_t)(((it - 1) / S) & 1));  // the slice before: its place is free, its sums are there
+        if (it + S - 1 < n) issue(it + S - 1, st_in);
         asm volatile("cp.async.commit_group;" ::: "memory");
+        if (CH && it && it % (CH ? CH : 1) == 0) add(it - 1);
         if (++st == S) st = 0;
         if (++st_in == S) st_in = 0;
     }
     mbar_wait(&done[(n - 1) % S], (uint32_t)(((n - 1) / S) & 1));
-    tc_fence_after();
+    add(n - 1);
     // ---- partial sums to shared memory, [token][row]: the slices are no longer read
     float* red = reinterpret_cast<float*>(smraw);
-    for (int c0 = 0; c0 < m_pad; c0 += 32) {
-        uint32_t v[32];
-        tmem_ld_32x32b_x32(tmem + ((uint32_t)(warp * 32) << 16) + c0, v);
-        tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 32; ++j)
-            if (c0 + j < m_pad) red[(c0 + j) * TRP + warp * 32 + lane] = __uint_as_float(v[j]);
-    }
-    tc_fence_before();
+    for (int j = 0; j < NTOK; ++j)
+        if (j < m_pad) red[j * TRP + warp * 32 + lane] = sum[j];
     if (cs > 1)
         cluster_sync_all();
     else
@@ -449,10 +475,10 @@ static cudaError_t go_mma(const Args& a, int cs, int tiles, cudaStream_t st) {
     static std::atomic<unsigned long long> allowed{0};
     return go(skinny_kernel<TC>, allowed, kStagesMma * kStageMma, a, cs, tiles, st);
 }
-template <int NTOK, typename TC, bool GROUPED>
+template <int NTOK, typename TC, bool GROUPED, int CH>
 static cudaError_t go_tc(const Args& a, int cs, int tiles, cudaStream_t st) {
     static std::atomic<unsigned long long> allowed{0};
-    return go(skinny_tc_kernel<NTOK, TC, GROUPED>, allowed, kStages<NTOK> * (TN * 128 + NTOK * 128) + 1024, a, cs, tiles, st);
+    return go(skinny_tc_kernel<NTOK, TC, GROUPED, CH>, allowed, kStages<NTOK> * (TN * 128 + NTOK * 128) + 1024, a, cs, tiles, st);
 }
 
 cudaError_t launch(const Args& a, cudaStream_t st) {
@@ -468,12 +494,20 @@ cudaError_t launch(const Args& a, cudaStream_t st) {
     const long long most = tc ? 296 : 592;
     int cs = 1;
     while (cs < 8 && (long long)tiles * (grouped ? a.max_tiles : 1) * cs * 2 <= most && nch / (cs * 2) >= 4) cs *= 2;
-#define LLARK_SKINNY(N_, GR_) (a.c_fp32 ? go_tc<N_, float, GR_>(a, cs, tiles, st) : go_tc<N_, bf16_t, GR_>(a, cs, tiles, st))
+#define LLARK_SKINNY(N_, GR_, CH_) (a.c_fp32 ? go_tc<N_, float, GR_, CH_>(a, cs, tiles, st) : go_tc<N_, bf16_t, GR_, CH_>(a, cs, tiles, st))
     if (!tc) return a.c_fp32 ? go_mma<float>(a, cs, tiles, st) : go_mma<bf16_t>(a, cs, tiles, st);
-    if (grouped) return LLARK_SKINNY(64, true);
-    if (a.M <= 16) return LLARK_SKINNY(16, false);
-    if (a.M <= 32) return LLARK_SKINNY(32, false);
-    return LLARK_SKINNY(64, false);
+    if (grouped) return LLARK_SKINNY(64, true, 1);
+    // Short chains for what fp32 FMAs computed before: narrow products and paired activations with an fp32 result. The others took the
+    // tcgen05 core, whose one chain over K errs by 4 to 12e-6; cut over a cluster theirs are shorter (0.5 to 1.4e-6), and 6 % faster than
+    // short ones (a decode step of 32 rows 549 us against 582).
+    if (a.N < 64 || (a.c_fp32 && (a.act == kActReluGlu || a.act == kActClampGlu))) {
+        if (a.M <= 16) return LLARK_SKINNY(16, false, 1);
+        if (a.M <= 32) return LLARK_SKINNY(32, false, 1);
+        return LLARK_SKINNY(64, false, 1);
+    }
+    if (a.M <= 16) return LLARK_SKINNY(16, false, 0);
+    if (a.M <= 32) return LLARK_SKINNY(32, false, 0);
+    return LLARK_SKINNY(64, false, 0);
 #undef LLARK_SKINNY
 }
 

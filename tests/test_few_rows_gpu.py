@@ -23,10 +23,11 @@ def test_products_and_epilogues(M, N, K):
     z = x.to(F64) @ w.to(F64).t()
     # fp32 results: products of bf16 numbers are exact, so only the order and the cut of K fp32 additions shows: at most
     # K * 2^-24 relative to the terms' norm, sqrt(K) of it in practice; the tensor cores' truncating adders measure 2e-6
+    taken = ops.LINEAR_STATS["rows"]
     assert _rel(ops.linear(x, w, bias=b, out_dtype=F32), z + b.to(F64)) < (5e-7 if M <= 8 else 5e-6)
     # bf16 results: one rounding to eight bits, at most 2^-8 of a value
     assert _rel(ops.linear(x, w, act="relu2"), torch.relu(z) ** 2) < 2.0 ** -8
-    assert ops.LINEAR_STATS["rows"] > 0
+    assert ops.LINEAR_STATS["rows"] == taken + 2
     if N % 2 == 0:
         v = z + b.to(F64)
         assert _rel(ops.linear(x, w, bias=b, act="relu_glu"), torch.relu(v[:, 0::2]) * v[:, 1::2]) < 2.0 ** -8
@@ -91,3 +92,42 @@ def test_gate_and_up_in_the_epilogue_are_those_of_the_op(M, N, K):
     got = ops.gemm(x, w, swiglu=True)
     # the halves' tiles cut K as the plain product's do, up to how many CTAs share a row: the sums may differ in their last bits
     assert _rel(got, ops.swiglu_fwd(ops.gemm(x, w)).to(F64)) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("M", [9, 16, 17, 33, 64])
+@pytest.mark.parametrize("N,K", [(40, 4096), (56, 72), (24, 11008)])
+def test_narrow_products_and_paired_fp32_results_are_as_exact_as_fmas(M, N, K):
+    """Rows above eight: chains of one slice of K in the tensor cores' truncating adders, everything else in fp32. An fp32 FMA chain of
+    these lengths measures 4e-7 to 1.1e-6, short chains 1 to 1.3e-7, one chain over K 2e-7 to 1.4e-6: 2^-22."""
+    from llark_b200 import ops
+
+    torch.manual_seed(M + N)
+    x, w = torch.randn(M, K, device="cuda").to(BF16), torch.randn(N, K, device="cuda").to(BF16)
+    z = x.to(F64) @ w.to(F64).t()
+    assert _rel(ops.linear(x, w, out_dtype=F32), z) < 2.0 ** -22
+    wide = torch.randn(8 * N, K, device="cuda").to(BF16)
+    u = x.to(F64) @ wide.to(F64).t()
+    assert _rel(ops.linear(x, wide, act="relu_glu", out_dtype=F32), torch.relu(u[:, 0::2]) * u[:, 1::2]) < 2.0 ** -21  # a product of two
+
+
+@pytest.mark.parametrize("T,C,ff,E,top", [(1, 128, 1024, 32, 4), (32, 256, 2048, 8, 4), (100, 72, 4096, 8, 4), (500, 64, 8192, 4, 2)])
+def test_the_experts_second_product_is_as_exact_as_fmas(T, C, ff, E, top):
+    """llark_seq_moe_down alone, whose sums are handed on in fp32: FMAs measured 0.7e-7 to 1e-6, short chains 1 to 2.2e-7, one chain over K
+    1 to 9e-6: 2^-21."""
+    from llark_b200 import ops
+    from llark_b200._lib import lib
+
+    torch.manual_seed(T)
+    n, L, p = T * top, lib(), ops._p
+    ids = torch.stack([torch.randperm(E, device="cuda")[:top] for _ in range(T)]).to(torch.int32)
+    most = (n + L.llark_seq_moe_tile_rows() - 1) // L.llark_seq_moe_tile_rows() + E
+    perm, pos, tiles, meta, seg = (torch.zeros(k, device="cuda", dtype=torch.int32) for k in (n, n, 3 * most, 2, E + 1))
+    assert L.llark_seq_moe_sort(p(ids), n, E, E, p(perm), p(pos), p(tiles), p(meta), p(seg), None, ops._stream()) == 0
+    act, wd = torch.randn(n, ff, device="cuda").to(BF16), torch.randn(E, C, ff, device="cuda").to(BF16)
+    z = torch.empty(n, C, device="cuda")
+    assert L.llark_seq_moe_down(p(act), p(wd), p(z), p(tiles), p(meta), most, n, C, ff, 0, ops._stream()) == 0
+    want, e = torch.empty(n, C, device="cuda", dtype=F64), ids.view(-1).long()
+    for k in range(E):
+        at = pos.long()[(e == k).nonzero().view(-1)]
+        want[at] = act[at].to(F64) @ wd[k].to(F64).t()
+    assert _rel(z, want) < 2.0 ** -21
