@@ -587,7 +587,15 @@ static void launch_rows(const T* A, long long lda, const int* perm, int top, con
         grouped_rows_kernel<T, TC, MODE, 8><<<grid, 256, 0, st>>>(A, lda, perm, top, W, C, N, tiles, meta, N, K, vec_ok, up);
 }
 
-// bf16 rows in 16-byte pieces, whatever their number: the few-rows product of skinny.cu over the tile list
+// bf16 rows in 16-byte pieces: the few-rows product of skinny.cu over the tile list, unless there is hardly a row per expert. A block
+// of launch_rows then streams an expert's weights as fast and needs no tile of 128 rows. Up + down, us, rows / tiles: 32 experts of
+// 2048 x 1024, 4 per token: 1 token 24 / 42, 4 tokens 42 / 46, 6 tokens 58 / 47; 64 of 4096 x 1024, 6 per token: 4 tokens 113 / 139, 8
+// tokens 201 / 217, 12 tokens 255 / 235; 8 of 1024 x 4096, 2 per token: 1 token 23 / 33, 3 tokens 41 / 48, 6 tokens 58 / 52; 128 of
+// 2048 x 768, 8 per token: 1 token 35 / 40, 3 tokens 62 / 55, 8 tokens 113 / 116, 12 tokens 145 / 126.
+static bool takes_tiles(int n_ent, int max_tiles) {
+    const int n_exp = max_tiles - (n_ent + kTileRows - 1) / kTileRows;
+    return n_ent > kRowsRouteMaxEntries || (n_ent > 6 && 2 * n_ent > n_exp);
+}
 static int launch_few(const void* A, long long lda, const int* perm, int top, const void* W, void* C, long long ldc, int c_fp32,
                       const int* tiles, const int* meta, int max_tiles, int n_rows, int K, int mode, UpArgs up, cudaStream_t st) {
     skinny::Args a = {};
@@ -610,7 +618,7 @@ template <typename T, int MODE>
 static int launch_up(const void* x, long long ldx, const int* perm, int top, const void* w, void* act, const int* tiles,
                      const int* meta, int max_tiles, int n_ent, int ff, int K, UpArgs up, cudaStream_t st) {
     constexpr bool dual = MODE == kSiluGlu || MODE == kClampGlu;
-    if (sizeof(T) == 2 && skinny::fits(x, ldx, w, K, K))
+    if (sizeof(T) == 2 && takes_tiles(n_ent, max_tiles) && skinny::fits(x, ldx, w, K, K))
         return launch_few(x, ldx, perm, top, w, act, ff, 0, tiles, meta, max_tiles, dual ? 2 * ff : ff, K, MODE, up, st);
     if (n_ent <= kRowsRouteMaxEntries) {  // a handful of rows per expert: stream the weights once
         const int vec = 16 / (int)sizeof(T);
@@ -643,7 +651,7 @@ extern "C" int llark_seq_moe_up(const void* x, long long ldx, const int* perm, i
 extern "C" int llark_seq_moe_down(const void* act, const void* w_down, float* z, const int* tiles, const int* meta,
                                   int max_tiles, int n_ent, int C, int ff, int act_fp32, cudaStream_t st) {
     if (max_tiles <= 0 || ff <= 0 || C <= 0 || !act || !w_down || !z || !tiles || !meta) return LLARK_EINVAL;
-    if (!act_fp32 && skinny::fits(act, ff, w_down, ff, ff))
+    if (!act_fp32 && takes_tiles(n_ent, max_tiles) && skinny::fits(act, ff, w_down, ff, ff))
         return launch_few(act, ff, nullptr, 1, w_down, z, C, 1, tiles, meta, max_tiles, C, ff, kPlain, UpArgs{}, st);
     if (n_ent <= kRowsRouteMaxEntries) {
         const int esz = act_fp32 ? 4 : 2, vec = 16 / esz;
