@@ -497,10 +497,11 @@ cudaError_t launch(const Args& a, cudaStream_t st) {
 #define LLARK_SKINNY(N_, GR_, CH_) (a.c_fp32 ? go_tc<N_, float, GR_, CH_>(a, cs, tiles, st) : go_tc<N_, bf16_t, GR_, CH_>(a, cs, tiles, st))
     if (!tc) return a.c_fp32 ? go_mma<float>(a, cs, tiles, st) : go_mma<bf16_t>(a, cs, tiles, st);
     if (grouped) return LLARK_SKINNY(64, true, 1);
-    // Short chains for what fp32 FMAs computed before: narrow products and paired activations with an fp32 result. The others took the
-    // tcgen05 core, whose one chain over K errs by 4 to 12e-6; cut over a cluster theirs are shorter (0.5 to 1.4e-6), and 6 % faster than
+    // Short chains for what fp32 FMAs computed before: narrow products, paired activations with an fp32 result and results off 16-byte
+    // boundaries. The others took the tcgen05 core, whose one chain over K errs by 4 to 12e-6; cut over a cluster theirs are shorter (0.5 to 1.4e-6), and 6 % faster than
     // short ones (a decode step of 32 rows 549 us against 582).
-    if (a.N < 64 || (a.c_fp32 && (a.act == kActReluGlu || a.act == kActClampGlu))) {
+    if (a.N < 64 || (a.c_fp32 && (a.act == kActReluGlu || a.act == kActClampGlu)) || a.ldc % (a.c_fp32 ? 4 : 8) ||
+        (reinterpret_cast<uintptr_t>(a.C) & 15)) {
         if (a.M <= 16) return LLARK_SKINNY(16, false, 1);
         if (a.M <= 32) return LLARK_SKINNY(32, false, 1);
         return LLARK_SKINNY(64, false, 1);
