@@ -1,7 +1,8 @@
 // Skinny linear layer for the single-token decode step of the generation path:
 //   C[M, N] = A[M, K] . W[N, K]^T (+ bias[N]) (+ R[M, N]),  M <= 8 rows, bf16 in / out, fp32 accumulation.
 // With M = batch (1 for the reference's inference scripts) the op is a pure stream of the weight matrix (N * K * 2 bytes,
-// 13.5 GB per token over a 7B model): the few-rows product of skinny.cu.
+// 13.5 GB per token over a 7B model): the few-rows product of skinny.cu. The engines reach it through llark_gemm_ex; this entry is kept for
+// programs that call the C interface.
 #include "skinny.cuh"
 
 namespace llark {

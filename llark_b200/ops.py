@@ -244,8 +244,8 @@ def attn_bwd(qkv, key_mask, out, dout, lse, B, S, n_heads, head_dim, dqkv=None, 
 
 
 def gemv(x, w, bias=None, residual=None, out=None, N=None):
-    """y[M, N] = x[M, K] @ w[N, K]^T (+ bias) (+ residual) for M <= 8 rows: the weight-streaming kernel of the decode step
-    (csrc/gemv.cu). `out` may be wider than N (padded logits buffer)."""
+    """y[M, N] = x[M, K] @ w[N, K]^T (+ bias) (+ residual) for M <= 8 rows (llark_gemv of the C interface; the
+    engines' products with few rows go through gemm and linear). `out` may be wider than N (padded logits buffer)."""
     M, K = x.shape
     N = int(N) if N is not None else w.shape[0]
     out = out if out is not None else torch.empty((M, N), device=x.device, dtype=BF16)
