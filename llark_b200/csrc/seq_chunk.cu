@@ -559,13 +559,14 @@ static int run(PrepArgs a, ScanArgs s, int n_seq, int max_len, cudaStream_t st) 
     const long long heads = (long long)n_seq * a.H;
     int cols = 32;
     while (cols < 64 && s.E % (2 * cols) == 0 && heads * (s.E / cols) > 148 * 4) cols *= 2;
-    const int threads = cols * 4, smem = (2 * Layout<D, CORRECT>::stage(cols) + 4 * threads * 4) * (int)sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(chunk_scan_kernel<D, CORRECT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    auto bytes = [](int c) { return (2 * Layout<D, CORRECT>::stage(c) + 4 * (c * 4) * 4) * (int)sizeof(float); };
+    // the limit is the function's, and another thread may launch it with the other width: always the larger size
+    cudaError_t e = cudaFuncSetAttribute(chunk_scan_kernel<D, CORRECT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes(64));
     for (int c0 = 0; c0 * C < max_len && e == cudaSuccess; c0 += a.chunks) {
         const int left = (max_len + C - 1) / C - c0, nc = left < a.chunks ? left : a.chunks;
         a.c0 = s.c0 = c0;
         chunk_prep_kernel<D, SRC><<<dim3(nc, (a.H + 3) / 4, n_seq), 128, 0, st>>>(a);
-        chunk_scan_kernel<D, CORRECT><<<dim3(s.E / cols, a.H, n_seq), threads, smem, st>>>(s);
+        chunk_scan_kernel<D, CORRECT><<<dim3(s.E / cols, a.H, n_seq), cols * 4, bytes(cols), st>>>(s);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) {
