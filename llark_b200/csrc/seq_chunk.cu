@@ -100,7 +100,7 @@ struct PrepArgs {
     float unit_eps;
     float* ws;                       // [n_seq, chunks, H] blocks
     const int* cu;
-    int H, G, c0, chunks;
+    int H, G, c0, chunks, src;
 };
 
 template <int D, int SRC>
@@ -329,6 +329,7 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool live) 
 }
 
 struct ScanArgs {
+    PrepArgs prep;     // for the blocks that the products cannot take
     const float* ws;
     const float* v;    // value of token row r, head h, channel e at v[r * v_ld + h * E + e]
     long long v_ld;
@@ -344,15 +345,106 @@ template <int D, bool CORRECT> struct Layout {
     __host__ __device__ static constexpr int stage(int cols) { return V + C * (cols + 8); }
 };
 
+// A block with an infinity or a NaN in it, or in the state: its tokens one after another, by FMAs, so that nothing reaches the tokens in
+// front of it (0 times infinity above the diagonal would) and infinities stay what they are (their low part is NaN). Two warps, half of
+// the rows of 16 columns each, as in the walk below: st is this thread's first entry of the state (the walk keeps it in registers and
+// puts it there for this), V are the block's values from this column group on, xu the group's exchange buffer (128 floats a warp). Inlined:
+// with a call in it the walk was given 128 registers and took 342 us instead of 301 (HGRN2, 4 requests of 333 to 2048 tokens).
+struct Outputs { float mine[4], give[4]; };  // of the walk: four outputs of this warp's tokens, four of the other's
 template <int D, bool CORRECT>
-__global__ void __launch_bounds__(256)
-chunk_scan_kernel(const ScanArgs p) {
+__device__ __forceinline__ Outputs block_by_tokens(const PrepArgs& p, int h, long long row0, int cnt, int half, const float* V, int VS,
+                                                   float* xu, int barrier, float* st, int E) {
+    constexpr int NT = D / 16;
+    Outputs out = {};
+    const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3, hd = half * (D / 2);
+    const bool wide = p.src == kChannel || p.src == kGlr;
+    const int kh = p.src == kGlr ? h : h / (p.H / p.G);
+    const float rate = p.src == kGlr ? 0.f : expf(p.rate_log[h]);
+#pragma unroll 1
+    for (int t = 0; t < cnt; ++t) {
+        const float* q = p.q + (row0 + t) * p.q_ld + (long long)kh * D;
+        const float* k = p.src == kGlr ? nullptr : p.k + (row0 + t) * p.k_ld + (long long)kh * D;
+        const float* dec = p.dec + (row0 + t) * p.dec_ld + (wide ? (long long)h * D : h);
+        float fq = 1.f, fk = 1.f, beta = 1.f, decay = 1.f, step = 0.f;
+        if (CORRECT) {
+            float sq = 0.f, sk = 0.f;
+#pragma unroll 1
+            for (int d = lane; d < D; d += 32) {
+                sq = fmaf(q[d], q[d], sq);
+                sk = fmaf(k[d], k[d], sk);
+            }
+            fq = 1.0f / sqrtf(warp_sum(sq) + p.unit_eps) / sqrtf((float)D);
+            fk = 1.0f / sqrtf(warp_sum(sk) + p.unit_eps);
+            beta = sigmoidf_(p.mix[(row0 + t) * p.mix_ld + h]);
+        }
+        if (!wide) {
+            step = softplusf_(dec[0] + p.bias[h]);
+            decay = expf(-rate * step);
+        }
+        float z[2 * NT], pp[2 * NT], dd[2 * NT], qq[2 * NT];  // of rows hd + 8 nt + 2 t4, + 1
+#pragma unroll 1
+        for (int i = 0; i < 2 * NT; ++i) {
+            const int d = hd + 8 * (i >> 1) + 2 * t4 + (i & 1);
+            dd[i] = decay;
+            z[i] = 0.f;
+            if (p.src == kGlr) {
+                const float low = p.bias ? p.bias[h * D + d] : 0.f;
+                qq[i] = q[d] * sigmoidf_(q[d]);
+                dd[i] = low + (1.0f - low) * sigmoidf_(dec[d]);
+                pp[i] = 1.0f - dd[i];
+            } else if (p.src == kState) {
+                qq[i] = q[d];
+                pp[i] = k[d] * step;
+            } else {
+                if (wide) dd[i] = expf(-rate * softplusf_(dec[d] + p.bias[h * D + d]));
+                qq[i] = q[d] * fq;
+                z[i] = k[d] * fk * dd[i];
+                pp[i] = beta * (k[d] * fk);
+            }
+        }
+        float u[2] = {V[t * VS + g], V[t * VS + g + 8]}, o[2] = {0.f, 0.f};
+        if (CORRECT) {
+#pragma unroll 1
+            for (int c = 0; c < 2; ++c) {
+                float a = 0.f;
+#pragma unroll 1
+                for (int i = 0; i < 2 * NT; ++i) a = fmaf(st[(long long)(8 * (i >> 1) + (i & 1)) * E + 8 * c], z[i], a);
+                a += __shfl_xor_sync(0xffffffffu, a, 1);
+                a += __shfl_xor_sync(0xffffffffu, a, 2);
+                if (t4 == 0) xu[half * 128 + g + 8 * c] = a;
+            }
+            asm volatile("bar.sync %0, 64;" ::"r"(barrier) : "memory");
+            for (int c = 0; c < 2; ++c) u[c] -= xu[g + 8 * c] + xu[128 + g + 8 * c];
+            asm volatile("bar.sync %0, 64;" ::"r"(barrier) : "memory");  // both have read them
+        }
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c) {
+#pragma unroll 1
+            for (int i = 0; i < 2 * NT; ++i) {
+                float& s = st[(long long)(8 * (i >> 1) + (i & 1)) * E + 8 * c];
+                s = fmaf(dd[i], s, pp[i] * u[c]);
+                o[c] = fmaf(s, qq[i], o[c]);
+            }
+            o[c] += __shfl_xor_sync(0xffffffffu, o[c], 1);
+            o[c] += __shfl_xor_sync(0xffffffffu, o[c], 2);
+#pragma unroll
+            for (int e = 0; e < 4; ++e)  // constant indexes: registers
+                if (t4 == (t & 7) >> 1 && e == (t & 1) + 2 * c) (t >> 3 == half ? out.mine[e] : out.give[e]) = o[c];
+        }
+    }
+    return out;
+}
+
+// Columns of S per CTA: 32 or 64, four threads each. Without the correction two CTAs of 64 columns fit on an SM with 128 registers a
+// thread (16 requests of 512 tokens, 32 heads: HGRN2 740 us, 859 with 174 registers and one CTA); with it they would spill.
+template <int D, bool CORRECT, int COLS>
+__global__ void __launch_bounds__(COLS * 4, !CORRECT && COLS == 64 ? 2 : 1)
+chunk_scan_kernel(const __grid_constant__ ScanArgs p) {
     constexpr int NT = D / 16;  // groups of eight rows of S that a warp keeps: half of them
     typedef Layout<D, CORRECT> Y;
     constexpr int M = CORRECT ? 2 : 1;  // Q alone, or Q and Z
     extern __shared__ __align__(16) float sm[];
-    const int cols = (blockDim.x >> 6) * 16, VS = cols + 8;
-    const int stage_floats = Y::stage(cols);
+    constexpr int cols = COLS, VS = cols + 8, stage_floats = Y::stage(cols);
     const int h = blockIdx.y, b = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
     const int half = warp & 1, e0 = blockIdx.x * cols, wc = (warp >> 1) * 16;
@@ -368,11 +460,12 @@ chunk_scan_kernel(const ScanArgs p) {
     const float* wsb = p.ws + ((long long)b * p.chunks * p.H + h) * block_floats(D, CORRECT);
     const long long ws_step = (long long)p.H * block_floats(D, CORRECT);
     float S[NT][4];  // rows g, g + 8 (columns of S) x entries d = hd + 8 nt + 2 t4, + 1
+    auto each_entry = [&](auto&& f) {
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
+        for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) S[nt][c] = st[(long long)(8 * nt + 2 * t4 + (c & 1)) * p.E + g + (c >> 1) * 8];
-
+            for (int c = 0; c < 4; ++c) f(S[nt][c], st + (long long)(8 * nt + 2 * t4 + (c & 1)) * p.E + g + (c >> 1) * 8);
+    };
     auto fetch = [&](int k, float* dst) {
         const float* s = wsb + k * ws_step;
         auto rows = [&](float* to, int pitch) {  // 16 rows of D
@@ -413,13 +506,35 @@ chunk_scan_kernel(const ScanArgs p) {
             if (r0 + t < n) op[(long long)t * p.H * p.E + (c >> 1) * 8] = mine[c] + other[c];
         }
     };
+    // Whether a block's results were finite is known at the barrier behind it, off the chain that the walk waits for. If they were not, the
+    // walk begins again (the state in memory is still that in front of it) and goes token by token from that block on.
+    int slow = nblk;
+    bool odd = false;
+again:
     fetch(0, sm);
+    each_entry([&](float& s, float* at) { s = *at; });
     for (int k = 0; k < nblk; ++k) {
         const float* x = sm + (k & 1) * stage_floats;
         asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();  // this block is here, and everybody is done with the one before
+        if (__syncthreads_or(odd)) {  // this block is here, and everybody is done with the one before
+            slow = k - 1;
+            odd = false;
+            goto again;
+        }
         if (k + 1 < nblk) fetch(k + 1, sm + ((k + 1) & 1) * stage_floats);
         if (k) finish(k - 1);
+        if (k >= slow) {
+            const int r0 = (p.c0 + k) * C;
+            each_entry([&](float& s, float* at) { *at = s; });
+            const Outputs out = block_by_tokens<D, CORRECT>(p.prep, h, row_b + r0, n - r0 < C ? n - r0 : C, half, x + Y::V + wc, VS,
+                                                            reinterpret_cast<float*>(xu + (warp & ~1) * 64), 1 + (warp >> 1),
+                                                            st + 2 * t4 * p.E + g, p.E);
+            each_entry([&](float& s, float* at) { s = *at; });
+#pragma unroll
+            for (int c = 0; c < 4; ++c) mine[c] = out.mine[c];
+            xo[(k & 1) * blockDim.x + warp * 32 + lane] = make_float4(out.give[0], out.give[1], out.give[2], out.give[3]);
+            continue;
+        }
         // ---- this warp's rows of S^T Q^T (and S^T Z^T)
         constexpr int NC = NT / 2;  // leading products in chains of two, the small ones in a chain of their own
         float hh[M][2][NC][4] = {}, xx[M][2][4] = {};
@@ -482,28 +597,32 @@ chunk_scan_kernel(const ScanArgs p) {
         for (int j = 0; j < 2; ++j)
 #pragma unroll
             for (int c = 0; c < 4; ++c) part[j][c] = total(0, j, c);
-        {
-            float give[4];
+        float give[4], all[4] = {};  // all: finite only if everything that follows from this block's numbers is
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                mine[c] = (half ? part[1][c] : part[0][c]) + vv[0][c];
-                give[c] = half ? part[0][c] : part[1][c];
-            }
-            xo[(k & 1) * blockDim.x + warp * 32 + lane] = make_float4(give[0], give[1], give[2], give[3]);
+        for (int c = 0; c < 4; ++c) {
+            mine[c] = (half ? part[1][c] : part[0][c]) + vv[0][c];
+            give[c] = half ? part[0][c] : part[1][c];
+            all[0] += mine[c];
+            all[1] += give[c];
         }
         // ---- S <- b S + P^T U
         FragA au[2];
+        float u[2][4];
         if (CORRECT) {
-            float u[2][4];
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     u[j][c] = -total(M - 1, j, c);
                     if (j == half) u[j][c] += vv[M - 1][c];
+                    all[2 + j] += u[j][c];
                 }
                 xu[(warp * 2 + j) * 32 + lane] = make_float4(u[j][0], u[j][1], u[j][2], u[j][3]);
             }
+        }
+        xo[(k & 1) * blockDim.x + warp * 32 + lane] = make_float4(give[0], give[1], give[2], give[3]);
+        odd = !(fabsf((all[0] + all[1]) + (all[2] + all[3])) < INFINITY);
+        if (CORRECT) {
             asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp >> 1)) : "memory");  // the two warps of these columns
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
@@ -541,12 +660,13 @@ chunk_scan_kernel(const ScanArgs p) {
             }
         }
     }
-    __syncthreads();
+    if (__syncthreads_or(odd)) {
+        slow = nblk - 1;
+        odd = false;
+        goto again;
+    }
     finish(nblk - 1);
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) st[(long long)(8 * nt + 2 * t4 + (c & 1)) * p.E + g + (c >> 1) * 8] = S[nt][c];
+    each_entry([&](float& s, float* at) { *at = s; });
 }
 
 // ------------------------------------------------------------------------------------------------ host
@@ -560,13 +680,13 @@ static int run(PrepArgs a, ScanArgs s, int n_seq, int max_len, cudaStream_t st) 
     int cols = 32;
     while (cols < 64 && s.E % (2 * cols) == 0 && heads * (s.E / cols) > 148 * 4) cols *= 2;
     auto bytes = [](int c) { return (2 * Layout<D, CORRECT>::stage(c) + 4 * (c * 4) * 4) * (int)sizeof(float); };
-    // the limit is the function's, and another thread may launch it with the other width: always the larger size
-    cudaError_t e = cudaFuncSetAttribute(chunk_scan_kernel<D, CORRECT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes(64));
+    auto scan = cols == 32 ? chunk_scan_kernel<D, CORRECT, 32> : chunk_scan_kernel<D, CORRECT, 64>;
+    cudaError_t e = cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes(cols));  // of this kernel always the same
     for (int c0 = 0; c0 * C < max_len && e == cudaSuccess; c0 += a.chunks) {
         const int left = (max_len + C - 1) / C - c0, nc = left < a.chunks ? left : a.chunks;
         a.c0 = s.c0 = c0;
         chunk_prep_kernel<D, SRC><<<dim3(nc, (a.H + 3) / 4, n_seq), 128, 0, st>>>(a);
-        chunk_scan_kernel<D, CORRECT><<<dim3(s.E / cols, a.H, n_seq), cols * 4, bytes(cols), st>>>(s);
+        scan<<<dim3(s.E / cols, a.H, n_seq), cols * 4, bytes(cols), st>>>(s);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) {
@@ -593,8 +713,8 @@ extern "C" int llark_seq_glr_chunks(const float* src, long long ld, int q_off, i
     if (bad_sizes(n_seq, max_len, H, D, E, chunks) || !src || !state || !o || !ws || !cu || !slot || ld % 4 || q_off % 4 || f_off % 4 ||
         v_off % 4 || !chunk::aligned16(src) || !chunk::aligned16(ws))
         return LLARK_EINVAL;
-    const chunk::PrepArgs a = {src + q_off, nullptr, src + f_off, nullptr, ld, 0, ld, 0, lower, nullptr, 0.f, ws, cu, H, H, 0, chunks};
-    const chunk::ScanArgs s = {ws, src + v_off, ld, state, o, cu, slot, H, E, 0, chunks};
+    const chunk::PrepArgs a = {src + q_off, nullptr, src + f_off, nullptr, ld, 0, ld, 0, lower, nullptr, 0.f, ws, cu, H, H, 0, chunks, chunk::kGlr};
+    const chunk::ScanArgs s = {a, ws, src + v_off, ld, state, o, cu, slot, H, E, 0, chunks};
     return D == 64 ? chunk::run<64, chunk::kGlr>(a, s, n_seq, max_len, st) : chunk::run<128, chunk::kGlr>(a, s, n_seq, max_len, st);
 }
 
@@ -608,8 +728,9 @@ extern "C" int llark_seq_delta_chunks(int rule, const float* q, long long q_ld, 
         !chunk::aligned16(q) || !chunk::aligned16(k) || !chunk::aligned16(v) || !chunk::aligned16(ws) ||
         (rule == 0 && (dec_ld % 4 || !chunk::aligned16(dec))))
         return LLARK_EINVAL;
-    const chunk::PrepArgs a = {q, k, dec, mix, q_ld, k_ld, dec_ld, mix_ld, dec_bias, rate_log, unit_eps, ws, cu, H, G, 0, chunks};
-    const chunk::ScanArgs s = {ws, v, v_ld, state, o, cu, slot, H, E, 0, chunks};
+    const int kind = rule == 0 ? chunk::kChannel : rule == 2 ? chunk::kScalar : chunk::kState;
+    const chunk::PrepArgs a = {q, k, dec, mix, q_ld, k_ld, dec_ld, mix_ld, dec_bias, rate_log, unit_eps, ws, cu, H, G, 0, chunks, kind};
+    const chunk::ScanArgs s = {a, ws, v, v_ld, state, o, cu, slot, H, E, 0, chunks};
 #define LLARK_CHUNKS(SRC_) (D == 64 ? chunk::run<64, SRC_>(a, s, n_seq, max_len, st) : chunk::run<128, SRC_>(a, s, n_seq, max_len, st))
     return rule == 0 ? LLARK_CHUNKS(chunk::kChannel) : rule == 2 ? LLARK_CHUNKS(chunk::kScalar) : LLARK_CHUNKS(chunk::kState);
 #undef LLARK_CHUNKS

@@ -90,3 +90,47 @@ def test_against_64_bits(kind, lens, H, D, E, bytes_, monkeypatch):
             assert eo < max(2 * rel(old.view(n, H, E)[at], want), 1e-6) and es < max(2 * rel(old_state[slots[b]], S), 1e-6)
     rest = [s for s in range(len(lens) + 1) if s not in slots]
     assert torch.equal(state[rest], S0[rest])  # nobody else's state was touched
+
+
+@pytest.mark.parametrize("kind", ["hgrn2", "scalar", "channel", "state"])
+@pytest.mark.parametrize("what,value", [("v", float("nan")), ("v", float("inf")), ("k", float("nan")), ("q", -float("inf")),
+                                        ("d", float("nan")), ("state", float("inf"))])
+def test_numbers_that_are_not_finite_stay_behind_their_token(kind, what, value, monkeypatch):
+    """An infinity or a NaN in one token of a block: nothing changes in front of it, and behind it results are those of the token-by-token
+    kernels, infinite or NaN where they are."""
+    from llark_b200 import ops
+
+    torch.manual_seed(7)
+    lens, H, D, E, dev = [40, 21], 2, 64, 32, "cuda"
+    n, st = sum(lens), _layout(lens, [1, 0])
+    S0 = torch.randn(2, H, D, E, device=dev)
+    t, h = 27, 1  # token 11 of the first request's second block
+    if what == "state":
+        S0[1, h, 3, 9] = value
+    if kind == "hgrn2":
+        src = torch.randn(n, 2 * H * D + H * E, device=dev)
+        at = {"v": 2 * H * D + h * E + 9, "k": None, "q": h * D + 3, "d": H * D + h * D + 3, "state": None}[what]
+        if what == "k":
+            pytest.skip("HGRN2 has no keys of its own")
+        if at is not None:
+            src[t, at] = value
+        run = lambda s: ops.seq_glr_scan(src, 0, H * D, 2 * H * D, None, s, st, H, D, E)  # noqa: E731
+    else:
+        rule = {"scalar": ops.DELTA_GATED_SCALAR, "channel": ops.DELTA_GATED, "state": ops.DELTA_STATE_SPACE}[kind]
+        q, k, v = (torch.randn(n, H * x, device=dev) for x in (D, D, E))
+        dec, mix = torch.randn(n, H * D if kind == "channel" else H, device=dev), torch.randn(n, H, device=dev)
+        bias, rate = torch.zeros(dec.shape[1], device=dev), torch.zeros(H, device=dev)
+        if what != "state":
+            {"v": v, "k": k, "q": q, "d": dec}[what][t, {"v": h * E + 9, "d": h * D + 3 if kind == "channel" else h}.get(what, h * D + 3)] = value
+        run = lambda s: ops.seq_delta_rule(rule, q, k, v, dec, None if kind == "state" else mix, s, st, H, H, D, E, dec_bias=bias,  # noqa: E731
+                                           rate_log=rate)
+    s1, s2 = S0.clone(), S0.clone()
+    o1 = run(s1)
+    monkeypatch.setattr(ops, "SCAN_BLOCK_MIN_LEN", 1 << 30)
+    o2 = run(s2)
+    for a, b in ((o1, o2), (s1, s2)):
+        assert not b.isfinite().all() or what == "q"
+        assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
+        assert torch.equal(a[a.isinf()], b[b.isinf()])
+        ok = b.isfinite()
+        assert ((a[ok] - b[ok]).norm() / b[ok].norm()).item() < 2e-6  # as above
