@@ -411,16 +411,19 @@ int llark_seq_glr_combine(const float* state, float* chunk_state, const float* c
                           const int* slot, int n_seq, int H, int D, int E, cudaStream_t stream);
 /* The same recurrences of prompts on the tensor cores, 16 tokens at a time (D 64 or 128, E a multiple of 32, every row and offset a
  * multiple of 16 bytes): _glr_chunks on the projection's columns as llark_seq_glr_scan; _delta_chunks on what llark_seq_delta_prep
- * reads, rules 0, 2 and 3 of it. state [slots, H, D, E] is read and written back. ws: n_seq * chunks * H blocks of
- * llark_seq_chunk_block_bytes (correct = 0 for HGRN2 and rule 3); any chunks >= 1 does, longer requests are walked in more passes. */
+ * reads, rules 0, 2 and 3 of it. state [slots, H, D, E] is read and written back. A call walks n_requests requests over consecutive
+ * blocks of 16 tokens, n_blocks in all: requests [n_requests, 4] = (request, its first block in the list, how many, the first one's place
+ * in the request), blocks [n_blocks, 2] = (request, place in it); on the device, a request's blocks one after another in the list. Long
+ * prompts take several calls. ws: n_blocks * H blocks of llark_seq_chunk_block_bytes (correct = 0 for HGRN2 and rule 3). */
 long long llark_seq_chunk_block_bytes(int D, int correct);
 int llark_seq_glr_chunks(const float* src, long long ld, int q_off, int f_off, int v_off, const float* lower, float* state, float* o,
-                         float* ws, int chunks, const int* cu, const int* slot, int n_seq, int max_len, int H, int D, int E,
-                         cudaStream_t stream);
+                         float* ws, const int* blocks, int n_blocks, const int* requests, int n_requests, const int* cu,
+                         const int* slot, int H, int D, int E, cudaStream_t stream);
 int llark_seq_delta_chunks(int rule, const float* q, long long q_ld, const float* k, long long k_ld, const float* dec, long long dec_ld,
                            const float* dec_bias, const float* rate_log, const float* mix, long long mix_ld, float unit_eps,
-                           const float* v, long long v_ld, float* state, float* o, float* ws, int chunks, const int* cu,
-                           const int* slot, int n_seq, int max_len, int H, int G, int D, int E, cudaStream_t stream);
+                           const float* v, long long v_ld, float* state, float* o, float* ws, const int* blocks, int n_blocks,
+                           const int* requests, int n_requests, const int* cu, const int* slot, int H, int G, int D, int E,
+                           cudaStream_t stream);
 int llark_seq_head_rmsnorm(const float* x, const float* w, void* out, long long n_rows, int E, float eps, int act_fp32,
                            cudaStream_t stream);
 

@@ -169,8 +169,8 @@ def lib():
             "llark_seq_decay_chunks": ([P, LL, I, I, I, P, I, I, F, I, P, I, P, P, P, P, P, P, P, I, I, I, I, P], I),
             "llark_seq_decay_combine": ([P, P, P, I, P, P, P, I, I, I, I, P], I),
             "llark_seq_chunk_block_bytes": ([I, I], LL),
-            "llark_seq_glr_chunks": ([P, LL, I, I, I, P, P, P, P, I, P, P, I, I, I, I, I, P], I),
-            "llark_seq_delta_chunks": ([I, P, LL, P, LL, P, LL, P, P, P, LL, F, P, LL, P, P, P, I, P, P, I, I, I, I, I, I, P], I),
+            "llark_seq_glr_chunks": ([P, LL, I, I, I, P, P, P, P, P, I, P, I, P, P, I, I, I, P], I),
+            "llark_seq_delta_chunks": ([I, P, LL, P, LL, P, LL, P, P, P, LL, F, P, LL, P, P, P, P, I, P, I, P, P, I, I, I, I, P], I),
             "llark_seq_kv_ring_write": ([P, P, P, P, P, P, P, P, I, I, I, I, I, P], I),
             "llark_seq_glr_scan": ([P, LL, I, I, I, P, P, P, P, P, P, P, P, P, I, I, I, I, P], I),
             "llark_seq_glr_combine": ([P, P, P, P, P, I, I, I, I, P], I),

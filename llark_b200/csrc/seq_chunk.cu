@@ -98,9 +98,9 @@ struct PrepArgs {
     long long q_ld, k_ld, dec_ld, mix_ld;
     const float *bias, *rate_log;    // of the decay; kGlr: bias = the lower bound (or NULL), no rate
     float unit_eps;
-    float* ws;                       // [n_seq, chunks, H] blocks
-    const int* cu;
-    int H, G, c0, chunks, src;
+    float* ws;                       // [blocks of this pass, H]
+    const int *blocks, *cu;          // (request, block of it) of every block of the pass
+    int H, G, src;
 };
 
 template <int D, int SRC>
@@ -110,13 +110,12 @@ chunk_prep_kernel(const PrepArgs p) {
     constexpr bool CORRECT = SRC == kChannel || SRC == kScalar;
     __shared__ float flat_[4][CORRECT ? 256 : 160], sT_[4][CORRECT ? C * C : 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h = blockIdx.y * 4 + warp, b = blockIdx.z, c = p.c0 + blockIdx.x;
-    const int row_b = p.cu[b], left = p.cu[b + 1] - row_b - c * C;
-    if (h >= p.H || left <= 0) return;  // no barrier of the block below
-    const int cnt = left < C ? left : C;
+    const int h = blockIdx.y * 4 + warp, b = p.blocks[2 * blockIdx.x], c = p.blocks[2 * blockIdx.x + 1];
+    if (h >= p.H) return;  // no barrier of the block below
+    const int row_b = p.cu[b], left = p.cu[b + 1] - row_b - c * C, cnt = left < C ? left : C;
     const long long row0 = row_b + c * C;
     float* flat = flat_[warp];
-    float* out = p.ws + (((long long)b * p.chunks + blockIdx.x) * p.H + h) * block_floats(D, CORRECT);
+    float* out = p.ws + ((long long)blockIdx.x * p.H + h) * block_floats(D, CORRECT);
     float* oZ = out;
     float* oQ = out + (CORRECT ? C * D : 0);
     float* oP = oQ + C * D;
@@ -334,8 +333,8 @@ struct ScanArgs {
     const float* v;    // value of token row r, head h, channel e at v[r * v_ld + h * E + e]
     long long v_ld;
     float *state, *o;  // [slots, H, D, E], [n_tok, H * E]
-    const int *cu, *slot;
-    int H, E, c0, chunks;
+    const int *requests, *cu, *slot;  // (request, its first block in ws, how many, the first one's place in the request) of the pass
+    int H, E;
 };
 
 // shared memory of a stage, in floats: Z [16][D + 8] | Q [16][D + 8] | P [16][PP] | b [D] | T [16][20] | A' [16][20] | V [16][cols + 8]
@@ -445,19 +444,17 @@ chunk_scan_kernel(const __grid_constant__ ScanArgs p) {
     constexpr int M = CORRECT ? 2 : 1;  // Q alone, or Q and Z
     extern __shared__ __align__(16) float sm[];
     constexpr int cols = COLS, VS = cols + 8, stage_floats = Y::stage(cols);
-    const int h = blockIdx.y, b = blockIdx.z;
+    const int* rq = p.requests + 4 * blockIdx.z;
+    const int h = blockIdx.y, b = rq[0], nblk = rq[2], c0 = rq[3];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
     const int half = warp & 1, e0 = blockIdx.x * cols, wc = (warp >> 1) * 16;
     const int row_b = p.cu[b], n = p.cu[b + 1] - row_b;
-    int nblk = (n + C - 1) / C - p.c0;
-    if (nblk <= 0) return;
-    if (nblk > p.chunks) nblk = p.chunks;
     const int hd = half * (D / 2);
     // partial results that the two warps of a column group hand each other: [2][warps][32] float4 of outputs, [warps][2][32] of U
     float4* xo = reinterpret_cast<float4*>(sm + 2 * stage_floats);
     float4* xu = xo + 2 * blockDim.x;
     float* st = p.state + ((long long)p.slot[b] * p.H + h) * (long long)D * p.E + (long long)hd * p.E + e0 + wc;
-    const float* wsb = p.ws + ((long long)b * p.chunks * p.H + h) * block_floats(D, CORRECT);
+    const float* wsb = p.ws + ((long long)rq[1] * p.H + h) * block_floats(D, CORRECT);
     const long long ws_step = (long long)p.H * block_floats(D, CORRECT);
     float S[NT][4];  // rows g, g + 8 (columns of S) x entries d = hd + 8 nt + 2 t4, + 1
     auto each_entry = [&](auto&& f) {
@@ -484,7 +481,7 @@ chunk_scan_kernel(const __grid_constant__ ScanArgs p) {
         s += D;
         if (CORRECT) square(dst + Y::T);
         square(dst + Y::A);
-        const int r0 = (p.c0 + k) * C, q = cols / 4;
+        const int r0 = (c0 + k) * C, q = cols / 4;
         for (int i = threadIdx.x; i < C * q; i += blockDim.x) {
             const int t = i / q, e = (i % q) * 4;
             const bool live = r0 + t < n;
@@ -496,7 +493,7 @@ chunk_scan_kernel(const __grid_constant__ ScanArgs p) {
     // is then there without a wait of its own). Rows g, g + 8 are channels, columns 2 t4, 2 t4 + 1 tokens.
     float mine[4];
     auto finish = [&](int k) {
-        const int r0 = (p.c0 + k) * C + 8 * half;
+        const int r0 = (c0 + k) * C + 8 * half;
         const float4 o4 = xo[(k & 1) * blockDim.x + (warp ^ 1) * 32 + lane];
         const float other[4] = {o4.x, o4.y, o4.z, o4.w};
         float* op = p.o + (long long)(row_b + r0) * p.H * p.E + (long long)h * p.E + e0 + wc + g;
@@ -524,7 +521,7 @@ again:
         if (k + 1 < nblk) fetch(k + 1, sm + ((k + 1) & 1) * stage_floats);
         if (k) finish(k - 1);
         if (k >= slow) {
-            const int r0 = (p.c0 + k) * C;
+            const int r0 = (c0 + k) * C;
             each_entry([&](float& s, float* at) { *at = s; });
             const Outputs out = block_by_tokens<D, CORRECT>(p.prep, h, row_b + r0, n - r0 < C ? n - r0 : C, half, x + Y::V + wc, VS,
                                                             reinterpret_cast<float*>(xu + (warp & ~1) * 64), 1 + (warp >> 1),
@@ -673,20 +670,18 @@ again:
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 template <int D, int SRC>
-static int run(PrepArgs a, ScanArgs s, int n_seq, int max_len, cudaStream_t st) {
+static int run(PrepArgs a, ScanArgs s, int n_blocks, int n_requests, cudaStream_t st) {
     constexpr bool CORRECT = SRC == kChannel || SRC == kScalar;
     // columns of S per CTA: few heads and requests are spread over the SMs, many share the blocks' operands
-    const long long heads = (long long)n_seq * a.H;
+    const long long heads = (long long)n_requests * a.H;
     int cols = 32;
     while (cols < 64 && s.E % (2 * cols) == 0 && heads * (s.E / cols) > 148 * 4) cols *= 2;
     auto bytes = [](int c) { return (2 * Layout<D, CORRECT>::stage(c) + 4 * (c * 4) * 4) * (int)sizeof(float); };
     auto scan = cols == 32 ? chunk_scan_kernel<D, CORRECT, 32> : chunk_scan_kernel<D, CORRECT, 64>;
     cudaError_t e = cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes(cols));  // of this kernel always the same
-    for (int c0 = 0; c0 * C < max_len && e == cudaSuccess; c0 += a.chunks) {
-        const int left = (max_len + C - 1) / C - c0, nc = left < a.chunks ? left : a.chunks;
-        a.c0 = s.c0 = c0;
-        chunk_prep_kernel<D, SRC><<<dim3(nc, (a.H + 3) / 4, n_seq), 128, 0, st>>>(a);
-        scan<<<dim3(s.E / cols, a.H, n_seq), cols * 4, bytes(cols), st>>>(s);
+    if (e == cudaSuccess) {
+        chunk_prep_kernel<D, SRC><<<dim3(n_blocks, (a.H + 3) / 4), 128, 0, st>>>(a);
+        scan<<<dim3(s.E / cols, a.H, n_requests), cols * 4, bytes(cols), st>>>(s);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) {
@@ -703,35 +698,39 @@ using namespace llark;
 
 extern "C" long long llark_seq_chunk_block_bytes(int D, int correct) { return 4LL * chunk::block_floats(D, correct != 0); }
 
-static bool bad_sizes(int n_seq, int max_len, int H, int D, int E, int chunks) {
-    return n_seq <= 0 || n_seq > 65535 || max_len <= 0 || H <= 0 || H > 65535 || (D != 64 && D != 128) || E <= 0 || E % 32 || chunks <= 0;
+static bool bad_sizes(int n_blocks, int n_requests, int H, int D, int E) {
+    return n_blocks <= 0 || n_requests <= 0 || n_requests > 65535 || H <= 0 || H > 65535 || (D != 64 && D != 128) || E <= 0 || E % 32;
 }
 
 extern "C" int llark_seq_glr_chunks(const float* src, long long ld, int q_off, int f_off, int v_off, const float* lower, float* state,
-                                    float* o, float* ws, int chunks, const int* cu, const int* slot, int n_seq, int max_len, int H,
-                                    int D, int E, cudaStream_t st) {
-    if (bad_sizes(n_seq, max_len, H, D, E, chunks) || !src || !state || !o || !ws || !cu || !slot || ld % 4 || q_off % 4 || f_off % 4 ||
-        v_off % 4 || !chunk::aligned16(src) || !chunk::aligned16(ws))
+                                    float* o, float* ws, const int* blocks, int n_blocks, const int* requests, int n_requests,
+                                    const int* cu, const int* slot, int H, int D, int E, cudaStream_t st) {
+    if (bad_sizes(n_blocks, n_requests, H, D, E) || !src || !state || !o || !ws || !blocks || !requests || !cu || !slot || ld % 4 ||
+        q_off % 4 || f_off % 4 || v_off % 4 || !chunk::aligned16(src) || !chunk::aligned16(ws))
         return LLARK_EINVAL;
-    const chunk::PrepArgs a = {src + q_off, nullptr, src + f_off, nullptr, ld, 0, ld, 0, lower, nullptr, 0.f, ws, cu, H, H, 0, chunks, chunk::kGlr};
-    const chunk::ScanArgs s = {a, ws, src + v_off, ld, state, o, cu, slot, H, E, 0, chunks};
-    return D == 64 ? chunk::run<64, chunk::kGlr>(a, s, n_seq, max_len, st) : chunk::run<128, chunk::kGlr>(a, s, n_seq, max_len, st);
+    const chunk::PrepArgs a = {src + q_off, nullptr, src + f_off, nullptr, ld,  0,  ld, 0, lower,
+                               nullptr,     0.f,     ws,          blocks,  cu, H, H,  chunk::kGlr};
+    const chunk::ScanArgs s = {a, ws, src + v_off, ld, state, o, requests, cu, slot, H, E};
+    return D == 64 ? chunk::run<64, chunk::kGlr>(a, s, n_blocks, n_requests, st)
+                   : chunk::run<128, chunk::kGlr>(a, s, n_blocks, n_requests, st);
 }
 
 extern "C" int llark_seq_delta_chunks(int rule, const float* q, long long q_ld, const float* k, long long k_ld, const float* dec,
                                       long long dec_ld, const float* dec_bias, const float* rate_log, const float* mix,
                                       long long mix_ld, float unit_eps, const float* v, long long v_ld, float* state, float* o,
-                                      float* ws, int chunks, const int* cu, const int* slot, int n_seq, int max_len, int H, int G,
-                                      int D, int E, cudaStream_t st) {
-    if (bad_sizes(n_seq, max_len, H, D, E, chunks) || (rule != 0 && rule != 2 && rule != 3) || G <= 0 || H % G || !q || !k || !dec ||
-        !dec_bias || !rate_log || (!mix && rule != 3) || !v || !state || !o || !ws || !cu || !slot || q_ld % 4 || k_ld % 4 || v_ld % 4 ||
-        !chunk::aligned16(q) || !chunk::aligned16(k) || !chunk::aligned16(v) || !chunk::aligned16(ws) ||
+                                      float* ws, const int* blocks, int n_blocks, const int* requests, int n_requests, const int* cu,
+                                      const int* slot, int H, int G, int D, int E, cudaStream_t st) {
+    if (bad_sizes(n_blocks, n_requests, H, D, E) || (rule != 0 && rule != 2 && rule != 3) || G <= 0 || H % G || !q || !k || !dec ||
+        !dec_bias || !rate_log || (!mix && rule != 3) || !v || !state || !o || !ws || !blocks || !requests || !cu || !slot || q_ld % 4 ||
+        k_ld % 4 || v_ld % 4 || !chunk::aligned16(q) || !chunk::aligned16(k) || !chunk::aligned16(v) || !chunk::aligned16(ws) ||
         (rule == 0 && (dec_ld % 4 || !chunk::aligned16(dec))))
         return LLARK_EINVAL;
     const int kind = rule == 0 ? chunk::kChannel : rule == 2 ? chunk::kScalar : chunk::kState;
-    const chunk::PrepArgs a = {q, k, dec, mix, q_ld, k_ld, dec_ld, mix_ld, dec_bias, rate_log, unit_eps, ws, cu, H, G, 0, chunks, kind};
-    const chunk::ScanArgs s = {a, ws, v, v_ld, state, o, cu, slot, H, E, 0, chunks};
-#define LLARK_CHUNKS(SRC_) (D == 64 ? chunk::run<64, SRC_>(a, s, n_seq, max_len, st) : chunk::run<128, SRC_>(a, s, n_seq, max_len, st))
+    const chunk::PrepArgs a = {q,        k,        dec, mix,    q_ld, k_ld, dec_ld, mix_ld, dec_bias,
+                               rate_log, unit_eps, ws,  blocks, cu,   H,    G,      kind};
+    const chunk::ScanArgs s = {a, ws, v, v_ld, state, o, requests, cu, slot, H, E};
+#define LLARK_CHUNKS(SRC_) \
+    (D == 64 ? chunk::run<64, SRC_>(a, s, n_blocks, n_requests, st) : chunk::run<128, SRC_>(a, s, n_blocks, n_requests, st))
     return rule == 0 ? LLARK_CHUNKS(chunk::kChannel) : rule == 2 ? LLARK_CHUNKS(chunk::kScalar) : LLARK_CHUNKS(chunk::kState);
 #undef LLARK_CHUNKS
 }

@@ -7,6 +7,7 @@ extension or without a GPU these raise.
 import ctypes
 import math
 
+import numpy as np
 import torch
 
 from ._lib import (EPI_CLAMP_GLU, EPI_NONE, EPI_QUICK_GELU, EPI_RELU2, EPI_RELU_GLU, EPI_ROPE, EPI_SWIGLU, EPI_SWIGLU_BWD,
@@ -795,14 +796,49 @@ SCAN_BLOCK_MIN_LEN = 16
 SCAN_BLOCK_BYTES = 96 << 20
 
 
+def scan_passes(st, most):
+    """The block walk's calls for a step: [(requests [n, 4], blocks [m, 2])] on the device (llark_seq_glr_chunks). A pass takes up to as
+    many blocks of 16 tokens from every request that has some left as `most` blocks in all allow (one each at least); requests that
+    have ended take no part in it. The longest come first."""
+    left = (np.diff(st.cu_host) + 15) // 16
+    done, ints, passes = 0, [], []
+    while left.any():
+        act = np.argsort(-left, kind="stable")[:np.count_nonzero(left)]
+        lo, hi = 1, int(left.max())
+        while lo < hi:  # the largest number of blocks a request that stays within `most`
+            mid = (lo + hi + 1) // 2
+            lo, hi = (mid, hi) if np.minimum(left, mid).sum() <= most else (lo, mid - 1)
+        n = np.minimum(left[act], lo)
+        first = np.cumsum(n) - n
+        m = int(n.sum())
+        blocks = np.stack([np.repeat(act, n), np.arange(m) - np.repeat(first - done, n)], 1)
+        requests = np.stack([act, first, n, np.full(len(act), done)], 1)
+        ints += [requests.ravel(), blocks.ravel()]
+        passes.append((len(act), m))
+        left = np.maximum(left - lo, 0)
+        done += lo
+    host = torch.from_numpy(np.concatenate(ints).astype(np.int32))
+    if torch.device(st.device).type == "cuda":
+        host = host.pin_memory()
+    dev, at, out = host.to(st.device, non_blocking=True), 0, []
+    for n, m in passes:
+        out.append((dev[at:at + 4 * n].view(n, 4), dev[at + 4 * n:at + 4 * n + 2 * m].view(m, 2)))
+        at += 4 * n + 2 * m
+    return out, host  # the pinned buffer lives as long as the step does
+
+
 def _scan_blocks(st, H, D, E, correct, tensors, offsets=()):
-    """(workspace, blocks of a request it holds) when the block walk takes these sizes and pointers, else None."""
-    if (st.max_len < SCAN_BLOCK_MIN_LEN or D not in (64, 128) or E % 32 or any(x % 4 for x in offsets)
+    """(workspace, passes) when the block walk takes these sizes and pointers, else None."""
+    if (st.max_len < SCAN_BLOCK_MIN_LEN or D not in (64, 128) or E % 32 or st.n_seq > 65535 or any(x % 4 for x in offsets)
             or any(t.data_ptr() % 16 or t.stride(0) % 4 for t in tensors)):
         return None
-    per = lib().llark_seq_chunk_block_bytes(D, int(correct)) * H * st.n_seq
-    n = max(1, min((st.max_len + 15) // 16, SCAN_BLOCK_BYTES // per))
-    return torch.empty(n * per, device=st.device, dtype=torch.uint8), n
+    per = lib().llark_seq_chunk_block_bytes(D, int(correct)) * H
+    most = max(1, SCAN_BLOCK_BYTES // per)
+    tables = getattr(st, "tables", {})  # the layers of a step share them
+    if ("scan", most) not in tables:
+        tables["scan", most] = scan_passes(st, most)
+    passes = tables["scan", most][0]
+    return torch.empty(max(b.shape[0] for _, b in passes) * per, device=st.device, dtype=torch.uint8), passes
 
 
 def seq_glr_scan(src, q_off, f_off, v_off, lower, state, st, H, D, E):
@@ -814,9 +850,11 @@ def seq_glr_scan(src, q_off, f_off, v_off, lower, state, st, H, D, E):
     L = lib()
     blocks = _scan_blocks(st, H, D, E, False, (src,), (q_off, f_off, v_off))
     if blocks is not None:
-        ws, n = blocks
-        check(L.llark_seq_glr_chunks(_p(src), src.stride(0), q_off, f_off, v_off, _p(lower), _p(state), _p(o), _p(ws), n, _p(st.cu),
-                                     _p(st.slot), st.n_seq, st.max_len, H, D, E, _stream()), "seq_glr_chunks")
+        ws, passes = blocks
+        for requests, blk in passes:
+            check(L.llark_seq_glr_chunks(_p(src), src.stride(0), q_off, f_off, v_off, _p(lower), _p(state), _p(o), _p(ws), _p(blk),
+                                         blk.shape[0], _p(requests), requests.shape[0], _p(st.cu), _p(st.slot), H, D, E, _stream()),
+                  "seq_glr_chunks")
         return o
     if st.max_len < GLR_CHUNK_MIN_LEN:
         check(L.llark_seq_glr_scan(_p(src), src.stride(0), q_off, f_off, v_off, _p(lower), _p(state), _p(state), None,
@@ -1012,12 +1050,13 @@ def seq_delta_rule(rule, q, k, v, dec, mix, state, st, H, G, D, E, dec_bias=None
     _req(q, torch.float32), _req(k, torch.float32), _req(v, torch.float32), _req(dec, torch.float32), _req(state, torch.float32)
     if mix is not None:
         _req(mix, torch.float32)
-    ws, n = blocks
+    ws, passes = blocks
     o = torch.empty((st.n_tok, H * E), device=v.device, dtype=torch.float32)
-    check(lib().llark_seq_delta_chunks(int(rule), _p(q), q.stride(0), _p(k), k.stride(0), _p(dec), dec.stride(0), _p(dec_bias),
-                                       _p(rate_log), _p(mix), mix.stride(0) if mix is not None else 0, float(unit_eps), _p(v),
-                                       v.stride(0), _p(state), _p(o), _p(ws), n, _p(st.cu), _p(st.slot), st.n_seq, st.max_len, H, G,
-                                       D, E, _stream()), "seq_delta_chunks")
+    for requests, blk in passes:
+        check(lib().llark_seq_delta_chunks(int(rule), _p(q), q.stride(0), _p(k), k.stride(0), _p(dec), dec.stride(0), _p(dec_bias),
+                                           _p(rate_log), _p(mix), mix.stride(0) if mix is not None else 0, float(unit_eps), _p(v),
+                                           v.stride(0), _p(state), _p(o), _p(ws), _p(blk), blk.shape[0], _p(requests),
+                                           requests.shape[0], _p(st.cu), _p(st.slot), H, G, D, E, _stream()), "seq_delta_chunks")
     return o
 
 
