@@ -414,8 +414,10 @@ int llark_seq_glr_combine(const float* state, float* chunk_state, const float* c
  * reads, rules 0, 2 and 3 of it. state [slots, H, D, E] is read and written back. A call walks n_requests requests over consecutive
  * blocks of 16 tokens, n_blocks in all: requests [n_requests, 4] = (request, its first block in the list, how many, the first one's place
  * in the request), blocks [n_blocks, 2] = (request, place in it); on the device, a request's blocks one after another in the list. Long
- * prompts take several calls. ws: n_blocks * H blocks of llark_seq_chunk_block_bytes (correct = 0 for HGRN2 and rule 3). */
+ * prompts take several calls. ws: n_blocks * H blocks of llark_seq_chunk_block_bytes (correct = 0 for HGRN2 and rule 3).
+ * _chunk_plan writes both lists for the requests that have more than `done` blocks, up to `each` of every one. */
 long long llark_seq_chunk_block_bytes(int D, int correct);
+int llark_seq_chunk_plan(const int* cu, int n_seq, int done, int each, int* requests, int* blocks, cudaStream_t stream);
 int llark_seq_glr_chunks(const float* src, long long ld, int q_off, int f_off, int v_off, const float* lower, float* state, float* o,
                          float* ws, const int* blocks, int n_blocks, const int* requests, int n_requests, const int* cu,
                          const int* slot, int H, int D, int E, cudaStream_t stream);

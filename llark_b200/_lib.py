@@ -28,7 +28,7 @@ SEQ_SYMBOLS = [
     "llark_seq_qkv_headnorm", "llark_seq_skip_gate_group_norm", "llark_seq_post_norm", "llark_seq_glu_clamped",
     "llark_seq_logit_cap", "llark_seq_moe_route_bias", "llark_seq_qkv_rotary", "llark_seq_gated_norm_add",
     "llark_seq_tanh_norm", "llark_seq_tanh_norm_add", "llark_seq_moe_route_top", "llark_seq_layer_norm_add",
-    "llark_seq_rotary_table", "llark_seq_chunk_block_bytes", "llark_seq_glr_chunks", "llark_seq_delta_chunks", "llark_seq_decay_rows", "llark_seq_decay_chunks", "llark_seq_decay_combine",
+    "llark_seq_rotary_table", "llark_seq_chunk_block_bytes", "llark_seq_chunk_plan", "llark_seq_glr_chunks", "llark_seq_delta_chunks", "llark_seq_decay_rows", "llark_seq_decay_chunks", "llark_seq_decay_combine",
 ]
 # what libllark_serve.so (`make serve`: GEMM core + decode linears + the ops above) exports
 SERVE_SYMBOLS = SEQ_SYMBOLS + ["llark_last_cuda_error", "llark_init", "llark_gemm", "llark_gemm_ex", "llark_gemv",
@@ -169,6 +169,7 @@ def lib():
             "llark_seq_decay_chunks": ([P, LL, I, I, I, P, I, I, F, I, P, I, P, P, P, P, P, P, P, I, I, I, I, P], I),
             "llark_seq_decay_combine": ([P, P, P, I, P, P, P, I, I, I, I, P], I),
             "llark_seq_chunk_block_bytes": ([I, I], LL),
+            "llark_seq_chunk_plan": ([P, I, I, I, P, P, P], I),
             "llark_seq_glr_chunks": ([P, LL, I, I, I, P, P, P, P, P, I, P, I, P, P, I, I, I, P], I),
             "llark_seq_delta_chunks": ([I, P, LL, P, LL, P, LL, P, P, P, LL, F, P, LL, P, P, P, P, I, P, I, P, P, I, I, I, I, P], I),
             "llark_seq_kv_ring_write": ([P, P, P, P, P, P, P, P, I, I, I, I, I, P], I),

@@ -666,6 +666,41 @@ again:
     each_entry([&](float& s, float* at) { *at = s; });
 }
 
+// ------------------------------------------------------------------------------------------------ the plan
+// One CTA: which requests have more than `done` blocks, where their blocks of this pass begin (a running sum over the requests), and the
+// list of blocks. A few us, once per step.
+constexpr int kPlanThreads = 1024;
+__global__ void __launch_bounds__(kPlanThreads)
+chunk_plan_kernel(const int* __restrict__ cu, int n_seq, int done, int each, int* __restrict__ requests, int* __restrict__ blocks) {
+    __shared__ int2 sums[32];  // requests, blocks of a warp
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int r0 = 0, b0 = 0;
+    for (int at = 0; at < n_seq; at += kPlanThreads) {
+        const int b = at + threadIdx.x;
+        int n = b < n_seq ? (cu[b + 1] - cu[b] + C - 1) / C - done : 0;
+        n = n < 0 ? 0 : n > each ? each : n;
+        int r = n > 0, f = n;  // up to this request, it included
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, r, o), y = __shfl_up_sync(0xffffffffu, f, o);
+            if (lane >= o) r += x, f += y;
+        }
+        if (lane == 31) sums[warp] = make_int2(r, f);
+        __syncthreads();
+        for (int w = 0; w < warp; ++w) r += sums[w].x, f += sums[w].y;
+        if (n > 0) {
+            int* q = requests + 4 * (r0 + r - 1);
+            q[0] = b, q[1] = b0 + f - n, q[2] = n, q[3] = done;
+            for (int i = 0; i < n; ++i) {
+                int* e = blocks + 2 * (b0 + f - n + i);
+                e[0] = b, e[1] = done + i;
+            }
+        }
+        for (int w = 0; w < kPlanThreads / 32; ++w) r0 += sums[w].x, b0 += sums[w].y;
+        __syncthreads();
+    }
+}
+
 // ------------------------------------------------------------------------------------------------ host
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
@@ -697,6 +732,17 @@ static int run(PrepArgs a, ScanArgs s, int n_blocks, int n_requests, cudaStream_
 using namespace llark;
 
 extern "C" long long llark_seq_chunk_block_bytes(int D, int correct) { return 4LL * chunk::block_floats(D, correct != 0); }
+
+extern "C" int llark_seq_chunk_plan(const int* cu, int n_seq, int done, int each, int* requests, int* blocks, cudaStream_t st) {
+    if (!cu || n_seq <= 0 || done < 0 || each <= 0 || !requests || !blocks) return LLARK_EINVAL;
+    chunk::chunk_plan_kernel<<<1, chunk::kPlanThreads, 0, st>>>(cu, n_seq, done, each, requests, blocks);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+        g_last_cuda_error = (int)e;
+        return LLARK_ECUDA;
+    }
+    return LLARK_OK;
+}
 
 static bool bad_sizes(int n_blocks, int n_requests, int H, int D, int E) {
     return n_blocks <= 0 || n_requests <= 0 || n_requests > 65535 || H <= 0 || H > 65535 || (D != 64 && D != 128) || E <= 0 || E % 32;

@@ -796,35 +796,37 @@ SCAN_BLOCK_MIN_LEN = 16
 SCAN_BLOCK_BYTES = 96 << 20
 
 
-def scan_passes(st, most):
-    """The block walk's calls for a step: [(requests [n, 4], blocks [m, 2])] on the device (llark_seq_glr_chunks). A pass takes up to as
-    many blocks of 16 tokens from every request that has some left as `most` blocks in all allow (one each at least); requests that
-    have ended take no part in it. The longest come first."""
-    left = (np.diff(st.cu_host) + 15) // 16
-    done, ints, passes = 0, [], []
+def scan_passes(cu_host, most):
+    """The block walk's passes over a step: [(blocks done before it, blocks it takes of a request at most, requests that have some left,
+    blocks in all)]. A pass takes as many as `most` blocks in all allow (one per request at least)."""
+    left = (np.diff(cu_host) + 15) // 16
+    done, out = 0, []
     while left.any():
-        act = np.argsort(-left, kind="stable")[:np.count_nonzero(left)]
         lo, hi = 1, int(left.max())
         while lo < hi:  # the largest number of blocks a request that stays within `most`
             mid = (lo + hi + 1) // 2
             lo, hi = (mid, hi) if np.minimum(left, mid).sum() <= most else (lo, mid - 1)
-        n = np.minimum(left[act], lo)
-        first = np.cumsum(n) - n
-        m = int(n.sum())
-        blocks = np.stack([np.repeat(act, n), np.arange(m) - np.repeat(first - done, n)], 1)
-        requests = np.stack([act, first, n, np.full(len(act), done)], 1)
-        ints += [requests.ravel(), blocks.ravel()]
-        passes.append((len(act), m))
+        out.append((done, lo, int(np.count_nonzero(left)), int(np.minimum(left, lo).sum())))
         left = np.maximum(left - lo, 0)
         done += lo
-    host = torch.from_numpy(np.concatenate(ints).astype(np.int32))
-    if torch.device(st.device).type == "cuda":
-        host = host.pin_memory()
-    dev, at, out = host.to(st.device, non_blocking=True), 0, []
-    for n, m in passes:
-        out.append((dev[at:at + 4 * n].view(n, 4), dev[at + 4 * n:at + 4 * n + 2 * m].view(m, 2)))
-        at += 4 * n + 2 * m
-    return out, host  # the pinned buffer lives as long as the step does
+    return out
+
+
+def _scan_tables(st, most):
+    """[(requests [n, 4], blocks [m, 2])] of each pass (llark_seq_glr_chunks), written by the device: no copy, and nothing that a stream
+    capture does not take. The layers of a step share them, but what a capture writes exists only in its replays."""
+    tables = None if torch.cuda.is_current_stream_capturing() else getattr(st, "tables", None)
+    if tables is not None and ("scan", most) in tables:
+        return tables["scan", most]
+    out = []
+    for done, each, n, m in scan_passes(st.cu_host, most):
+        t = torch.empty(4 * n + 2 * m, device=st.device, dtype=torch.int32)
+        requests, blocks = t[:4 * n].view(n, 4), t[4 * n:].view(m, 2)
+        check(lib().llark_seq_chunk_plan(_p(st.cu), st.n_seq, done, each, _p(requests), _p(blocks), _stream()), "seq_chunk_plan")
+        out.append((requests, blocks))
+    if tables is not None:
+        tables["scan", most] = out
+    return out
 
 
 def _scan_blocks(st, H, D, E, correct, tensors, offsets=()):
@@ -833,11 +835,7 @@ def _scan_blocks(st, H, D, E, correct, tensors, offsets=()):
             or any(t.data_ptr() % 16 or t.stride(0) % 4 for t in tensors)):
         return None
     per = lib().llark_seq_chunk_block_bytes(D, int(correct)) * H
-    most = max(1, SCAN_BLOCK_BYTES // per)
-    tables = getattr(st, "tables", {})  # the layers of a step share them
-    if ("scan", most) not in tables:
-        tables["scan", most] = scan_passes(st, most)
-    passes = tables["scan", most][0]
+    passes = _scan_tables(st, max(1, SCAN_BLOCK_BYTES // per))
     return torch.empty(max(b.shape[0] for _, b in passes) * per, device=st.device, dtype=torch.uint8), passes
 
 

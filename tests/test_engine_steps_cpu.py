@@ -46,24 +46,18 @@ def test_wanted_places_outside_the_step_are_refused(want, error):
 
 @pytest.mark.parametrize("lens,most", [([16], 1), ([1, 17, 40], 100), ([2048] + [1] * 31, 64), ([200, 70, 3, 64], 5), ([5] * 40 + [300], 8)])
 def test_passes_of_the_block_walk(lens, most):
-    """Every block of 16 tokens once, a request's in their order, and no more at a time than asked for (one per request at least)."""
+    """Every block of 16 tokens once, and no more at a time than asked for (one per request at least)."""
     from llark_b200 import ops
     from llark_b200.state_cache import StepLayout
 
     st = StepLayout(lens, [0] * len(lens), list(range(len(lens))), "cpu")
-    todo = [-(-n // 16) for n in lens]
-    done = [0] * len(lens)
-    passes, _ = ops.scan_passes(st, most)
-    for requests, blocks in passes:
-        alive = [b for b in range(len(lens)) if done[b] < todo[b]]
-        assert sorted(requests[:, 0].tolist()) == alive  # nobody who has ended
-        assert blocks.shape[0] <= max(most, len(alive))
-        at = 0
-        for b, first, n, c in requests.tolist():
-            assert (first, c) == (at, done[b]) and n > 0
-            assert blocks[at:at + n].tolist() == [[b, c + i] for i in range(n)]
-            at, done[b] = at + n, done[b] + n
-        assert at == blocks.shape[0]
-    assert done == todo
+    left, at = [-(-n // 16) for n in lens], 0
+    passes = ops.scan_passes(st.cu_host, most)
+    for done, each, n, m in passes:
+        take = [min(x, each) for x in left]
+        assert (done, n, m) == (at, sum(x > 0 for x in left), sum(take)) and n > 0
+        assert m <= max(most, n) and (each == max(left) or sum(min(x, each + 1) for x in left) > most)
+        left, at = [x - t for x, t in zip(left, take)], at + each
+    assert not any(left)
     if lens[0] == 2048:  # one long prompt beside single tokens: not a pass per block of it
         assert len(passes) <= 3

@@ -134,3 +134,20 @@ def test_numbers_that_are_not_finite_stay_behind_their_token(kind, what, value, 
         assert torch.equal(a[a.isinf()], b[b.isinf()])
         ok = b.isfinite()
         assert ((a[ok] - b[ok]).norm() / b[ok].norm()).item() < 2e-6  # as above
+
+
+@pytest.mark.parametrize("lens,most", [([40], 9), ([1, 17, 300, 2], 8), ([1] * 1500 + [500] + [30] * 700, 2400)])
+def test_the_plan_of_a_pass(lens, most):
+    """The device's lists against the step: more requests than one sweep of the kernel takes, requests that end in an earlier pass."""
+    from llark_b200 import ops
+
+    st = _layout(lens, list(range(len(lens))))
+    blocks = [-(-n // 16) for n in lens]
+    for (done, each, n, m), (requests, table) in zip(ops.scan_passes(st.cu_host, most), ops._scan_tables(st, most)):
+        want_r, want_b = [], []
+        for b, x in enumerate(blocks):
+            k = min(max(x - done, 0), each)
+            if k:
+                want_r.append([b, len(want_b), k, done])
+                want_b += [[b, done + i] for i in range(k)]
+        assert requests.tolist() == want_r and table.tolist() == want_b and (n, m) == (len(want_r), len(want_b))
