@@ -791,7 +791,7 @@ def seq_kv_ring_write(kn, vv, kring, vring, st, cap):
 GLR_CHUNK = 256        # rows per work item when a long prompt is scanned in chunks
 GLR_CHUNK_MIN_LEN = 512  # shortest longest-request of a step that is scanned in chunks
 # Steps whose longest request brings this many tokens take the tensor-core walk of csrc/seq_chunk.cu (blocks of 16 tokens) where its
-# sizes allow; its workspace holds up to SCAN_BLOCK_BYTES (less than L2, so that the walk finds there what was prepared)
+# sizes allow and walk_pays(); its workspace holds up to SCAN_BLOCK_BYTES (less than L2, so that the walk finds there what was prepared)
 SCAN_BLOCK_MIN_LEN = 16
 SCAN_BLOCK_BYTES = 96 << 20
 
@@ -829,10 +829,28 @@ def _scan_tables(st, most):
     return out
 
 
-def _scan_blocks(st, H, D, E, correct, tensors, offsets=()):
-    """(workspace, passes) when the block walk takes these sizes and pointers, else None."""
+# What the walk costs more than the token-by-token scan before the first token, per head and block beyond the first of a request, and
+# per head and request, and what it saves per head and further token, and per token of the longest request (us, heads of 128)
+WALK_COST = {"hgrn2": (15, 0.045, 0.022, 0.0045, 0.79), "channel": (17, 0.09, 0.0, 0.006, 0.27), "scalar": (6, 0.06, 0.0, 0.006, 0.27),
+             "state": (0, 0.05, 0.0, 0.006, 0.2)}
+
+
+def walk_pays(kind, H, longest, n_seq, n_tok, n_blocks):
+    """Whether the block walk is ahead of the scan for a step. It takes a block of 16 for a request's single token too, and a decay per
+    channel makes its preparation long. Measured on a B200, us, scan / walk, heads of 128: one request, 16 heads, of 16 / 24 / 32 / 64
+    tokens: HGRN2 22 / 27, 30 / 26, 38 / 28, 68 / 32; a decay per channel 24 / 36, 26 / 36, 30 / 38, 46 / 44; a decay per head 25 / 26,
+    25 / 26, 28 / 26, 43 / 34. 32 heads, 32 / 64 tokens beside 31 single ones: HGRN2 61 / 77, 91 / 80; per channel 117 / 134, 134 / 136; per
+    head 117 / 111, 133 / 114; 32 requests of 16: 118 / 87, 177 / 144, 170 / 117; 2048 tokens beside 31: 754 / 381, 1417 / 525, 1393 / 432."""
+    fixed, block, request, token, chain = WALK_COST[kind]
+    return fixed + H * (block * (n_blocks - n_seq) + request * n_seq - token * (n_tok - n_seq)) < chain * longest
+
+
+def _scan_blocks(kind, st, H, D, E, correct, tensors, offsets=()):
+    """(workspace, passes) when the block walk takes this step, these sizes and pointers, else None."""
     if (st.max_len < SCAN_BLOCK_MIN_LEN or D not in (64, 128) or E % 32 or st.n_seq > 65535 or any(x % 4 for x in offsets)
             or any(t.data_ptr() % 16 or t.stride(0) % 4 for t in tensors)):
+        return None
+    if not walk_pays(kind, H, st.max_len, st.n_seq, st.n_tok, int(((np.diff(st.cu_host) + 15) // 16).sum())):
         return None
     per = lib().llark_seq_chunk_block_bytes(D, int(correct)) * H
     passes = _scan_tables(st, max(1, SCAN_BLOCK_BYTES // per))
@@ -846,7 +864,7 @@ def seq_glr_scan(src, q_off, f_off, v_off, lower, state, st, H, D, E):
     _req(src, torch.float32), _req(state, torch.float32)
     o = torch.empty((st.n_tok, H * E), device=src.device, dtype=torch.float32)
     L = lib()
-    blocks = _scan_blocks(st, H, D, E, False, (src,), (q_off, f_off, v_off))
+    blocks = _scan_blocks("hgrn2", st, H, D, E, False, (src,), (q_off, f_off, v_off))
     if blocks is not None:
         ws, passes = blocks
         for requests, blk in passes:
@@ -1041,7 +1059,8 @@ def seq_delta_rule(rule, q, k, v, dec, mix, state, st, H, G, D, E, dec_bias=None
     correct = rule != DELTA_STATE_SPACE
     blocks = None
     if rule != DELTA_GENERALIZED:
-        blocks = _scan_blocks(st, H, D, E, correct, (q, k, v) + ((dec,) if rule == DELTA_GATED else ()))
+        kind = {DELTA_GATED: "channel", DELTA_GATED_SCALAR: "scalar", DELTA_STATE_SPACE: "state"}[rule]
+        blocks = _scan_blocks(kind, st, H, D, E, correct, (q, k, v) + ((dec,) if rule == DELTA_GATED else ()))
     if blocks is None:
         vec = seq_delta_prep(rule, q, k, dec, mix, H, G, D, dec_bias=dec_bias, rate_log=rate_log, unit_eps=unit_eps)
         return seq_delta_scan(vec, v, state, st, H, D, E, correct=correct)

@@ -61,3 +61,15 @@ def test_passes_of_the_block_walk(lens, most):
     assert not any(left)
     if lens[0] == 2048:  # one long prompt beside single tokens: not a pass per block of it
         assert len(passes) <= 3
+
+
+@pytest.mark.parametrize("H,lens,kinds", [
+    (16, [16], {"scalar": False, "channel": False, "hgrn2": False}), (16, [24], {"hgrn2": True, "channel": False}),
+    (32, [64], {"hgrn2": True, "channel": True, "scalar": True, "state": True}),
+    (32, [32] + [1] * 31, {"hgrn2": False, "channel": False, "state": True}), (32, [64] + [1] * 127, {"hgrn2": False}),
+    (32, [16] * 32, {"hgrn2": True, "channel": True, "scalar": True}), (32, [2048] + [1] * 127, {"hgrn2": True, "channel": True, "scalar": True})])
+def test_the_walk_is_taken_where_it_was_faster(H, lens, kinds):
+    from llark_b200 import ops
+
+    for kind, want in kinds.items():
+        assert ops.walk_pays(kind, H, max(lens), len(lens), sum(lens), sum(-(-n // 16) for n in lens)) == want, kind
