@@ -175,7 +175,8 @@ class GatedLinearRecurrence:
     def forward(self, hc, st, cache):
         w = self.w
         qfv = ops.linear(hc, w.w_qfv, bias=w.b_qfv, out_dtype=F32)
-        o_raw = ops.seq_glr_scan(qfv, w.q_off, w.f_off, w.v_off, w.lower, cache.view(self.h_state), st, w.H, w.D, w.E)
+        o_raw = ops.seq_glr_scan(qfv, w.q_off, w.f_off, w.v_off, w.lower, cache.view(self.h_state), st, w.H, w.D, w.E,
+                                 full_fp32=self.act == F32)
         o = ops.seq_head_rmsnorm(o_raw, w.norm, w.E, self.eps, self.act)
         return ops.linear(o, w.w_o, out_dtype=F32)
 
@@ -402,7 +403,8 @@ class GatedDeltaRule:
         gate = ops.linear(low[:, w.ra:], w.g2, out_dtype=F32)
         cv = ops.seq_conv_act(pin[:, :w.n_conv], w.conv, cache.view(self.h_carry), st, silu=True)
         o = ops.seq_delta_rule(ops.DELTA_GATED, cv[:, :GD], cv[:, GD:2 * GD], cv[:, 2 * GD:], dec, pin[:, w.b_off:],
-                               cache.view(self.h_state), st, w.H, w.G, w.D, w.E, dec_bias=w.dt_bias, rate_log=w.rate_log)
+                               cache.view(self.h_state), st, w.H, w.G, w.D, w.E, dec_bias=w.dt_bias, rate_log=w.rate_log,
+                               full_fp32=self.act == F32)
         on = ops.seq_head_norm_gate(o, w.norm, w.H, w.E, self.eps, self.act, gate=gate)
         return ops.linear(on, w.w_o, out_dtype=F32)
 
@@ -487,7 +489,7 @@ class ScalarGatedDeltaRule(_OneBranch):
         cv = ops.seq_conv_act(pin[:, :w.n_conv], w.conv, cache.view(self.h_carry), st, silu=True)
         o = ops.seq_delta_rule(ops.DELTA_GATED_SCALAR, cv[:, :GD], cv[:, GD:2 * GD], cv[:, 2 * GD:], pin[:, w.a_off:w.a_off + w.H],
                                pin[:, w.b_off:w.b_off + w.H], cache.view(self.h_state), st, w.H, w.G, w.D, w.E, dec_bias=w.dt_bias,
-                               rate_log=w.rate_log)
+                               rate_log=w.rate_log, full_fp32=self.act == F32)
         on = ops.seq_head_norm_gate(o, w.norm, w.H, w.E, self.eps, self.act, gate=pin[:, w.g_off:w.n_in], gate_silu=True)
         return ops.linear(on, w.w_o, out_dtype=F32)
 
@@ -873,7 +875,7 @@ class StateSpaceDuality(_OneBranch):
                               bias=w.conv_b)
         xs, write, read = cv[:, :inner], cv[:, inner:inner + GN], cv[:, inner + GN:]
         o = ops.seq_delta_rule(ops.DELTA_STATE_SPACE, read, write, xs, step, None, cache.view(self.h_state), st, w.H, w.G, w.N, w.E,
-                               dec_bias=w.dt_bias, rate_log=w.rate_log)
+                               dec_bias=w.dt_bias, rate_log=w.rate_log, full_fp32=self.act == F32)
         y = ops.seq_skip_gate_group_norm(o, xs, w.skip, gate, w.norm, w.H, w.E, w.NG, self.eps, self.act)
         return ops.linear(y, w.w_o, out_dtype=F32)
 

@@ -857,14 +857,15 @@ def _scan_blocks(kind, st, H, D, E, correct, tensors, offsets=()):
     return torch.empty(max(b.shape[0] for _, b in passes) * per, device=st.device, dtype=torch.uint8), passes
 
 
-def seq_glr_scan(src, q_off, f_off, v_off, lower, state, st, H, D, E):
+def seq_glr_scan(src, q_off, f_off, v_off, lower, state, st, H, D, E, full_fp32=False):
     """src fp32 [n_tok, ld] -> o_raw fp32 [n_tok, H*E]; state fp32 [slots, H, D, E] read and written back. Steps with a
     long request run in three passes over chunks of GLR_CHUNK rows (local states from zero; combine; outputs), which
-    gives the scan as many independent work items as there are chunks."""
+    gives the scan as many independent work items as there are chunks. From SCAN_BLOCK_MIN_LEN tokens on the block walk takes a step,
+    whose products are three TF32 products each; full_fp32: never."""
     _req(src, torch.float32), _req(state, torch.float32)
     o = torch.empty((st.n_tok, H * E), device=src.device, dtype=torch.float32)
     L = lib()
-    blocks = _scan_blocks("hgrn2", st, H, D, E, False, (src,), (q_off, f_off, v_off))
+    blocks = None if full_fp32 else _scan_blocks("hgrn2", st, H, D, E, False, (src,), (q_off, f_off, v_off))
     if blocks is not None:
         ws, passes = blocks
         for requests, blk in passes:
@@ -1053,12 +1054,12 @@ def seq_delta_scan(vec, v, state, st, H, D, E, correct=True):
     return o
 
 
-def seq_delta_rule(rule, q, k, v, dec, mix, state, st, H, G, D, E, dec_bias=None, rate_log=None, unit_eps=1e-6):
+def seq_delta_rule(rule, q, k, v, dec, mix, state, st, H, G, D, E, dec_bias=None, rate_log=None, unit_eps=1e-6, full_fp32=False):
     """seq_delta_prep and seq_delta_scan in one: o fp32 [n_tok, H*E] from the projections, state updated. Prompts of every rule but
-    DELTA_GENERALIZED take the block walk, which prepares what it needs itself."""
+    DELTA_GENERALIZED take the block walk (as seq_glr_scan), which prepares what it needs itself."""
     correct = rule != DELTA_STATE_SPACE
     blocks = None
-    if rule != DELTA_GENERALIZED:
+    if rule != DELTA_GENERALIZED and not full_fp32:
         kind = {DELTA_GATED: "channel", DELTA_GATED_SCALAR: "scalar", DELTA_STATE_SPACE: "state"}[rule]
         blocks = _scan_blocks(kind, st, H, D, E, correct, (q, k, v) + ((dec,) if rule == DELTA_GATED else ()))
     if blocks is None:

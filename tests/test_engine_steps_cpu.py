@@ -73,3 +73,17 @@ def test_the_walk_is_taken_where_it_was_faster(H, lens, kinds):
 
     for kind, want in kinds.items():
         assert ops.walk_pays(kind, H, max(lens), len(lens), sum(lens), sum(-(-n // 16) for n in lens)) == want, kind
+
+
+def test_fp32_mode_asks_every_recurrence_for_fp32():
+    """dtype=torch.float32 means no TF32: each scan that has a form on the tensor cores is told."""
+    import ast
+    import os
+
+    from llark_b200 import mixers
+
+    calls = [n for n in ast.walk(ast.parse(open(os.path.abspath(mixers.__file__)).read())) if isinstance(n, ast.Call)
+             and getattr(n.func, "attr", "") in ("seq_glr_scan", "seq_delta_rule", "seq_decay_scan")]
+    assert len(calls) == 5
+    for c in calls:
+        assert [ast.unparse(k.value) for k in c.keywords if k.arg == "full_fp32"] == ["self.act == F32"], ast.unparse(c)

@@ -159,3 +159,31 @@ def test_the_plan_of_a_pass(lens, most):
                 want_r.append([b, len(want_b), k, done])
                 want_b += [[b, done + i] for i in range(k)]
         assert requests.tolist() == want_r and table.tolist() == want_b and (n, m) == (len(want_r), len(want_b))
+
+
+@pytest.mark.parametrize("kind", ["hgrn2", "scalar", "channel", "state"])
+def test_full_fp32_is_the_token_by_token_scan(kind, monkeypatch):
+    from llark_b200 import ops
+
+    torch.manual_seed(3)
+    lens, H, D, E, dev = [40, 3], 2, 64, 32, "cuda"
+    n, st = sum(lens), _layout(lens, [0, 1])
+    S0, x = torch.randn(2, H, D, E, device=dev), torch.randn(n, 3 * H * D + 2 * H, device=dev)
+    one = torch.ones(H * D, device=dev)
+
+    def run(**kw):
+        s = S0.clone()
+        if kind == "hgrn2":
+            return ops.seq_glr_scan(x, 0, H * D, 2 * H * D, None, s, st, H, D, E, **kw), s
+        rule = {"scalar": ops.DELTA_GATED_SCALAR, "channel": ops.DELTA_GATED, "state": ops.DELTA_STATE_SPACE}[kind]
+        wide = kind == "channel"
+        dec, bias = (x[:, H * D:2 * H * D].contiguous(), one) if wide else (x[:, -H:], one[:H])
+        return ops.seq_delta_rule(rule, x[:, :H * D].contiguous(), x[:, H * D:2 * H * D].contiguous(), x[:, 2 * H * D:2 * H * D + H * E].contiguous(),
+                                  dec, None if kind == "state" else x[:, -2 * H:-H], s, st, H, H, D, E, dec_bias=bias, rate_log=one[:H], **kw), s
+
+    got = run(full_fp32=True)
+    walk = run()
+    monkeypatch.setattr(ops, "SCAN_BLOCK_MIN_LEN", 1 << 30)
+    want = run()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    assert not torch.equal(walk[0], want[0])  # the other form, at fp32 accuracy
