@@ -36,7 +36,7 @@ def _p(t):
     return t.data_ptr() if t is not None else None
 
 
-_raw_stream, _device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+_raw_stream, _device = (getattr(torch._C, n, None) for n in ("_cuda_getCurrentRawStream", "_cuda_getDevice"))  # None: no CUDA in torch
 
 
 def _stream():

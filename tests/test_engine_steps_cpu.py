@@ -87,3 +87,19 @@ def test_fp32_mode_asks_every_recurrence_for_fp32():
     assert len(calls) == 5
     for c in calls:
         assert [ast.unparse(k.value) for k in c.keywords if k.arg == "full_fp32"] == ["self.act == F32"], ast.unparse(c)
+
+
+def test_ops_import_on_a_torch_without_cuda():
+    """The host side (layouts, passes, checks) is used and tested where torch has no CUDA; only a call needs the device."""
+    import os
+    import subprocess
+    import sys
+
+    code = ("import torch\n"
+            "for n in ('_cuda_getCurrentRawStream', '_cuda_getDevice'):\n"
+            "    if hasattr(torch._C, n): delattr(torch._C, n)\n"
+            "import llark_b200.ops as ops\n"
+            "assert ops.scan_passes([0, 5, 40], 4)\n")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-1000:]
