@@ -116,7 +116,7 @@ class FlatBuckets:
 
     def pview(self, name, shape=None, span=1):
         """View of `span` consecutive parameters starting at `name` (fused q|k|v, gate|up)."""
-        key = (name, shape, span)
+        key = (name, shape if shape is None else tuple(shape), span)
         t = self._views.get(key)
         if t is None:
             t = self._views[key] = self._pview(name, shape, span)

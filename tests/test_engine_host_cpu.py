@@ -391,3 +391,13 @@ def test_decode_attention_refuses_stores_of_more_than_4096_entries():
     c = _lib.lib()
     assert c.llark_attn_decode(16, 16, 16, 16, 16, 1, 4097, 1, 128, 0.1, None) == -1
     assert c.llark_attn_decode_packed(16, 384, 16, 16, 0, 16, 1, 4097, 1, 128, 0.1, None) == -1
+
+
+def test_parameter_views_take_any_shape_that_view_takes():
+    from llark_b200.engine import FlatBuckets
+
+    p = torch.nn.Parameter(torch.arange(6.0).view(2, 3).to(BF16))
+    flat = FlatBuckets([("w", p)], "cpu")
+    for shape in (None, (3, 2), [3, 2], torch.Size([2, 3])):
+        v = flat.pview("w", shape)
+        assert v.data_ptr() == flat.params.data_ptr() and list(v.shape) == list(shape or [6])
