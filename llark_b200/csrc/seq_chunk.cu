@@ -23,9 +23,10 @@
 //                       zero and is added with an FMA.
 //
 // The token-by-token kernels (seq_mixers.cu, seq_delta.cu) walk a chain of shared-memory reads and FMAs per token and stay for short
-// steps, other sizes and the general rule. What bounds this: one chain of blocks per head and 16 columns, in which a warp issues some
-// 750 instructions per block (100 of them products at 8 cycles each). With one warp for all rows the walk took 1.6 times as long: one
-// warp per scheduler waits for its own results two thirds of the time.
+// steps, other sizes, the general rule and fp32 mode. What bounds this: one chain of blocks per head and 16 columns, in which a warp waits
+// for its own results most of the time. With one warp for all rows the walk took 1.6 times as long. Measured on a B200, heads of 128, us,
+// scan / here: HGRN2, 16 heads, 2048 + 1500 + 700 + 333 tokens 691 / 272; delta rule, 1777 + 1700 + 1500 tokens, a decay per head 1119 /
+// 410; 1000 + 600 tokens, a decay per channel 533 / 199, state space 425 / 112.
 #include "common.cuh"
 
 #include <utility>
@@ -296,7 +297,7 @@ chunk_prep_kernel(const PrepArgs p) {
 
 // ------------------------------------------------------------------------------------------------ the walk
 // x = hi + lo + (what neither holds, < 2^-21 |x|): hi rounded to TF32 on its bits, so that the rest has either sign; the tensor cores cut
-// lo to TF32 themselves. With hi cut as well every part errs the same way and the products with it: outputs 4.5e-7 off against 1.2e-7,
+// lo to TF32 themselves. With hi cut as well every part errs the same way and the products with it: outputs 4.5e-7 off against 1.1e-7,
 // where FMAs token by token are 0.7 to 1.6e-7 off (2048 tokens, heads of 128).
 __device__ __forceinline__ void split(float x, uint32_t& hi, uint32_t& lo) {
     hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
@@ -307,6 +308,9 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], 
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
+// The sum of the leading products and that of the small ones. The adders cut, so that a chain of one or two products comes out 2^-25 too
+// small on average, and every state with it (3.3e-8 for HGRN2, 6e-8 for the delta rule): that much is added.
+__device__ __forceinline__ float whole(float lead, float small) { return lead + fmaf(lead, 0x1p-25f, small); }
 struct FragA {
     uint32_t hi[4], lo[4];
     __device__ __forceinline__ void set(float x0, float x1, float x2, float x3) {
@@ -434,10 +438,12 @@ __device__ __forceinline__ Outputs block_by_tokens(const PrepArgs& p, int h, lon
     return out;
 }
 
-// Columns of S per CTA: 32 or 64, four threads each. Without the correction two CTAs of 64 columns fit on an SM with 128 registers a
-// thread (16 requests of 512 tokens, 32 heads: HGRN2 740 us, 859 with 174 registers and one CTA); with it they would spill.
-template <int D, bool CORRECT, int COLS>
-__global__ void __launch_bounds__(COLS * 4, !CORRECT && COLS == 64 ? 2 : 1)
+// Columns of S per CTA: 32 or 64, four threads each. PER_SM: CTAs that the registers have to leave room for. Without the correction two of
+// 64 columns fit with 128 registers a thread (16 requests of 512 tokens, 32 heads: HGRN2 740 us, 859 with 174 registers and one CTA); with
+// it they would spill. With it three of 32 columns fit with 168 registers, and are ahead once there are more than two for every SM (3
+// requests of 2048 tokens, 32 heads 961 -> 786 us; 3 of 1500 to 1777, 16 heads 409 -> 425).
+template <int D, bool CORRECT, int COLS, int PER_SM>
+__global__ void __launch_bounds__(COLS * 4, PER_SM)
 chunk_scan_kernel(const __grid_constant__ ScanArgs p) {
     constexpr int NT = D / 16;  // groups of eight rows of S that a warp keeps: half of them
     typedef Layout<D, CORRECT> Y;
@@ -539,7 +545,7 @@ again:
             float a = hh[m][j][0][c];
 #pragma unroll
             for (int i = 1; i < NC; ++i) a += hh[m][j][i][c];
-            return a + xx[m][j][c];
+            return whole(a, xx[m][j][c]);
         };
 #pragma unroll
         for (int kk = 0; kk < NT; ++kk) {
@@ -588,7 +594,7 @@ again:
 #pragma unroll
         for (int m = 0; m < M; ++m)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) vv[m][c] += vx[m][c];
+            for (int c = 0; c < 4; ++c) vv[m][c] = whole(vv[m][c], vx[m][c]);
         float part[2][4];
 #pragma unroll
         for (int j = 0; j < 2; ++j)
@@ -650,10 +656,10 @@ again:
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const float2 bb = *reinterpret_cast<const float2*>(x + Y::B + hd + 8 * (n0 + i) + 2 * t4);
-                S[n0 + i][0] = fmaf(S[n0 + i][0], bb.x, (acc[0][i][0] + acc[1][i][0]) + ax[i][0]);
-                S[n0 + i][1] = fmaf(S[n0 + i][1], bb.y, (acc[0][i][1] + acc[1][i][1]) + ax[i][1]);
-                S[n0 + i][2] = fmaf(S[n0 + i][2], bb.x, (acc[0][i][2] + acc[1][i][2]) + ax[i][2]);
-                S[n0 + i][3] = fmaf(S[n0 + i][3], bb.y, (acc[0][i][3] + acc[1][i][3]) + ax[i][3]);
+                S[n0 + i][0] = fmaf(S[n0 + i][0], bb.x, whole(acc[0][i][0] + acc[1][i][0], ax[i][0]));
+                S[n0 + i][1] = fmaf(S[n0 + i][1], bb.y, whole(acc[0][i][1] + acc[1][i][1], ax[i][1]));
+                S[n0 + i][2] = fmaf(S[n0 + i][2], bb.x, whole(acc[0][i][2] + acc[1][i][2], ax[i][2]));
+                S[n0 + i][3] = fmaf(S[n0 + i][3], bb.y, whole(acc[0][i][3] + acc[1][i][3], ax[i][3]));
             }
         }
     }
@@ -712,7 +718,9 @@ static int run(PrepArgs a, ScanArgs s, int n_blocks, int n_requests, cudaStream_
     int cols = 32;
     while (cols < 64 && s.E % (2 * cols) == 0 && heads * (s.E / cols) > 148 * 4) cols *= 2;
     auto bytes = [](int c) { return (2 * Layout<D, CORRECT>::stage(c) + 4 * (c * 4) * 4) * (int)sizeof(float); };
-    auto scan = cols == 32 ? chunk_scan_kernel<D, CORRECT, 32> : chunk_scan_kernel<D, CORRECT, 64>;
+    auto scan = cols == 32 ? chunk_scan_kernel<D, CORRECT, 32, 1> : chunk_scan_kernel<D, CORRECT, 64, CORRECT ? 1 : 2>;
+    if constexpr (CORRECT)
+        if (cols == 32 && heads * (s.E / cols) > 148 * 2) scan = chunk_scan_kernel<D, CORRECT, 32, 3>;
     cudaError_t e = cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes(cols));  // of this kernel always the same
     if (e == cudaSuccess) {
         chunk_prep_kernel<D, SRC><<<dim3(n_blocks, (a.H + 3) / 4), 128, 0, st>>>(a);

@@ -101,6 +101,49 @@ def test_against_64_bits(kind, lens, H, D, E, bytes_, monkeypatch):
 
 
 @pytest.mark.parametrize("kind", ["hgrn2", "scalar", "channel", "state"])
+def test_as_exact_as_fp32_sums(kind):
+    """Decays, keys and values as a layer's projections give them, 300 tokens: the split operands are rounded and the chains in the
+    truncating adders are two products long. Measured 1.2 to 1.6e-7 of the outputs, the token-by-token FMAs 0.7 to 1.4e-7, operands that
+    are cut 4.5e-7: 2^-22."""
+    from llark_b200 import ops
+
+    torch.manual_seed(11)
+    lens, H, D, E, dev = [300, 100], 4, 128, 128, "cuda"
+    n, st = sum(lens), _layout(lens, [0, 1])
+    state = torch.zeros(2, H, D, E, device=dev)
+    q, k, v = (torch.nn.functional.silu(torch.randn(n, H * D, device=dev)) for _ in range(3))
+    z = None
+    if kind == "hgrn2":
+        src, lower = torch.randn(n, 3 * H * D, device=dev), torch.rand(H * D, device=dev) * 0.9
+        src[:, H * D:2 * H * D] += 1.0
+        o = ops.seq_glr_scan(src, 0, H * D, 2 * H * D, lower, state, st, H, D, E)
+        s, lo = src.to(F64), lower.to(F64)
+        q = torch.nn.functional.silu(s[:, :H * D]).view(n, H, D)
+        d = (lo + (1 - lo) * torch.sigmoid(s[:, H * D:2 * H * D])).view(n, H, D)
+        p, v = 1 - d, s[:, 2 * H * D:].reshape(n, H, E)
+    else:
+        rule = {"scalar": ops.DELTA_GATED_SCALAR, "channel": ops.DELTA_GATED, "state": ops.DELTA_STATE_SPACE}[kind]
+        if kind == "state":
+            q, k = q / 11, k / 11
+        dec, mix = torch.randn(n, H * D if kind == "channel" else H, device=dev), torch.randn(n, H, device=dev)
+        rate, bias = torch.randn(H, device=dev) * 0.5 - 1, torch.randn(dec.shape[1], device=dev) - 1
+        o = ops.seq_delta_rule(rule, q, k, v, dec, None if kind == "state" else mix, state, st, H, H, D, E, dec_bias=bias, rate_log=rate)
+        q, k, v = (t.to(F64).view(n, H, D) for t in (q, k, v))
+        step = torch.nn.functional.softplus(dec.to(F64) + bias.to(F64))
+        step = step.view(n, H, D) if kind == "channel" else step[:, :, None]
+        d = torch.exp(-torch.exp(rate.to(F64))[:, None] * step).expand(n, H, D)
+        if kind == "state":
+            p = step * k
+        else:
+            q, k = (t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6) for t in (q, k))
+            q, z, p = q / D ** 0.5, k * d, torch.sigmoid(mix.to(F64))[:, :, None] * k
+    for b, ln in enumerate(lens):
+        at = slice(st.cu_host[b], st.cu_host[b] + ln)
+        want, _ = _walk(q[at], d[at], z[at] if z is not None else None, p[at], v[at], torch.zeros(H, D, E, device=dev, dtype=F64), z is not None)
+        assert ((o.view(n, H, E)[at].to(F64) - want).norm() / want.norm()).item() < 2.0 ** -22
+
+
+@pytest.mark.parametrize("kind", ["hgrn2", "scalar", "channel", "state"])
 @pytest.mark.parametrize("what,value", [("v", float("nan")), ("v", float("inf")), ("k", float("nan")), ("q", -float("inf")),
                                         ("d", float("nan")), ("state", float("inf"))])
 def test_numbers_that_are_not_finite_stay_behind_their_token(kind, what, value, monkeypatch):
