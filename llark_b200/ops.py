@@ -799,8 +799,10 @@ SCAN_BLOCK_BYTES = 96 << 20
 def scan_passes(cu_host, most):
     """The block walk's passes over a step: [(blocks done before it, blocks it takes of a request at most, requests that have some left,
     blocks in all)]. A pass takes as many as `most` blocks in all allow (one per request at least)."""
-    left = (np.diff(cu_host) + 15) // 16
-    done, out = 0, []
+    left = [(b - a + 15) // 16 for a, b in zip(cu_host, cu_host[1:])]
+    if sum(left) <= most:
+        return [(0, max(left), len(left), sum(left))]
+    left, done, out = np.array(left), 0, []
     while left.any():
         lo, hi = 1, int(left.max())
         while lo < hi:  # the largest number of blocks a request that stays within `most`
@@ -850,7 +852,10 @@ def _scan_blocks(kind, st, H, D, E, correct, tensors, offsets=()):
     if (st.max_len < SCAN_BLOCK_MIN_LEN or D not in (64, 128) or E % 32 or st.n_seq > 65535 or any(x % 4 for x in offsets)
             or any(t.data_ptr() % 16 or t.stride(0) % 4 for t in tensors)):
         return None
-    if not walk_pays(kind, H, st.max_len, st.n_seq, st.n_tok, int(((np.diff(st.cu_host) + 15) // 16).sum())):
+    tables = getattr(st, "tables", {})  # the layers of a step ask for the same
+    if "blocks" not in tables:
+        tables["blocks"] = sum((b - a + 15) // 16 for a, b in zip(st.cu_host, st.cu_host[1:]))
+    if not walk_pays(kind, H, st.max_len, st.n_seq, st.n_tok, tables["blocks"]):
         return None
     per = lib().llark_seq_chunk_block_bytes(D, int(correct)) * H
     passes = _scan_tables(st, max(1, SCAN_BLOCK_BYTES // per))
