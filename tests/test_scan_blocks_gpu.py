@@ -101,14 +101,15 @@ def test_against_64_bits(kind, lens, H, D, E, bytes_, monkeypatch):
 
 
 @pytest.mark.parametrize("kind", ["hgrn2", "scalar", "channel", "state"])
-def test_as_exact_as_fp32_sums(kind):
-    """Decays, keys and values as a layer's projections give them, 300 tokens: the split operands are rounded and the chains in the
-    truncating adders are two products long. Measured 1.2 to 1.6e-7 of the outputs, the token-by-token FMAs 0.7 to 1.4e-7, operands that
+@pytest.mark.parametrize("lens,H", [([300, 100], 4), ([70, 33], 40), ([70, 33], 80)])  # up to two CTAs per SM, more, 64 columns per CTA
+def test_as_exact_as_fp32_sums(kind, lens, H):
+    """Decays, keys and values as a layer's projections give them: the split operands are rounded and the chains in the truncating adders
+    are two products long. Measured 1.2 to 1.6e-7 of the outputs, the token-by-token FMAs 0.7 to 1.4e-7, operands that
     are cut 4.5e-7: 2^-22."""
     from llark_b200 import ops
 
     torch.manual_seed(11)
-    lens, H, D, E, dev = [300, 100], 4, 128, 128, "cuda"
+    D, E, dev = 128, 128, "cuda"
     n, st = sum(lens), _layout(lens, [0, 1])
     state = torch.zeros(2, H, D, E, device=dev)
     q, k, v = (torch.nn.functional.silu(torch.randn(n, H * D, device=dev)) for _ in range(3))
