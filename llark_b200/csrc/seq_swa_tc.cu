@@ -66,26 +66,46 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 
-// 32 channels of one query's weighted sum of values by FMAs, over the keys lo .. hi that it sees (counted as in the kernel; m: its
+// A query's weighted sum of values by FMAs, four channels a lane, over the keys lo .. hi that it sees (counted as in the kernel; m: its
 // largest score): for rows in whose key tiles a value is infinite or NaN, since the products multiply what a row does not see by 0, and
-// that is NaN. Only a row whose own scores are finite gets here.
-__device__ __noinline__ void sum_by_fma(const Args& a, const bf16_t* q, int row0, int n_ring, int ring0, long long ring_base, int g, int lo,
-                                        int hi, float sc, float m, int c0, float (&o)[32]) {
-#pragma unroll 1
-    for (int e = 0; e < 32; ++e) o[e] = 0.f;
-#pragma unroll 1
-    for (int k = lo; k <= hi; ++k) {
+// that is NaN. Only rows whose own scores are finite get here, a warp at a time: a lane scores a key, then all take its value.
+__device__ __noinline__ float4 sum_by_fma(const Args& a, const bf16_t* q, int row0, int n_ring, int ring0, long long ring_base, int g, int lo,
+                                          int hi, float sc, float m) {
+    const int lane = threadIdx.x & 31;
+    auto row = [&](const bf16_t* own, const bf16_t* ring, int k) {
         const bool old = k < n_ring;
         const int e = ring0 + k;
-        const long long at = ((old ? ring_base + (e >= a.cap ? e - a.cap : e) : (long long)row0 + k - n_ring) * a.G + g) * HD;
-        const bf16_t *kr = (old ? a.kring : a.kn) + at, *vr = (old ? a.vring : a.vv) + at + c0;
-        float s = 0.f;
+        return (old ? ring : own) + ((old ? ring_base + (e >= a.cap ? e - a.cap : e) : (long long)row0 + k - n_ring) * a.G + g) * HD;
+    };
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
-        for (int c = 0; c < HD; ++c) s = fmaf(__bfloat162float(q[c]), __bfloat162float(kr[c]), s);
-        const float p = ex2(s * sc - m);
-#pragma unroll 1
-        for (int c = 0; c < 32; ++c) o[c] = fmaf(p, __bfloat162float(vr[c]), o[c]);
+    for (int k0 = lo; k0 <= hi; k0 += 32) {
+        float p = 0.f;
+        if (k0 + lane <= hi) {
+            const uint4 *qr = reinterpret_cast<const uint4*>(q), *kr = reinterpret_cast<const uint4*>(row(a.kn, a.kring, k0 + lane));
+            float s = 0.f;
+#pragma unroll 4
+            for (int c = 0; c < HD / 8; ++c) {
+                const uint4 x = qr[c], y = kr[c];
+                const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float2 u = unpack_bf16x2(xs[e]), v = unpack_bf16x2(ys[e]);
+                    s = fmaf(u.y, v.y, fmaf(u.x, v.x, s));
+                }
+            }
+            p = ex2(s * sc - m);
+        }
+#pragma unroll 4
+        for (int j = 0; j < 32; ++j) {
+            if (k0 + j > hi) break;  // the same for the whole warp
+            const float pj = __shfl_sync(0xffffffffu, p, j);
+            const uint2 v = *reinterpret_cast<const uint2*>(row(a.vv, a.vring, k0 + j) + 4 * lane);
+            const float2 v0 = unpack_bf16x2(v.x), v1 = unpack_bf16x2(v.y);
+            o = make_float4(fmaf(pj, v0.x, o.x), fmaf(pj, v0.y, o.y), fmaf(pj, v1.x, o.z), fmaf(pj, v1.y, o.w));
+        }
     }
+    return o;
 }
 
 __global__ void __launch_bounds__(kThreads, 2)
@@ -298,21 +318,14 @@ swa_tc_kernel(const __grid_constant__ Args a) {
         // a sink adds exp(sink_h) to the denominator; a row of the prompt has seen its own key: m is finite
         float inv = a.out_scale / (a.sink ? l + exp2f(a.sink[h] * kLog2e - m) : l);
         if (a.gate && a.gate_per_head) inv *= 1.0f / (1.0f + expf(-a.gate[trow * a.gate_ld + h]));
+        float odd = 0.f;  // NaN as soon as a sum is not finite
 #pragma unroll 1
         for (int c = 0; c < HD / 32; ++c) {
             uint32_t o[32];
             tmem_ld_32x32b_x32(lane0 + 128 + c * 32, o);
             tmem_ld_wait();
-            float odd = 0.f;  // NaN as soon as one of them is not finite
 #pragma unroll
             for (int e = 0; e < 32; ++e) odd = fmaf(__uint_as_float(o[e]), 0.f, odd);
-            if (ok && odd != 0.f && l < INFINITY) {
-                float f[32];
-                sum_by_fma(a, a.qn + (trow * a.H + h) * HD, row0, n_ring, (int)(k_lo % a.cap), (long long)a.slot[b] * a.cap, g, lo, hi, sc, m,
-                           c * 32, f);
-#pragma unroll
-                for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(f[e]);
-            }
             if (ok) {
                 if (a.gate && !a.gate_per_head) {
                     const float* gp = a.gate + trow * a.gate_ld + h * HD + c * 32;
@@ -332,6 +345,21 @@ swa_tc_kernel(const __grid_constant__ Args a) {
             __syncwarp();
         }
         tc_fence_before();
+        for (uint32_t rows = __ballot_sync(0xffffffffu, ok && odd != 0.f && l < INFINITY); rows; rows &= rows - 1) {
+            const int from = __ffs(rows) - 1;
+            const long long t = row0 + qt0 + quad * 32 + from;
+            const float4 s = sum_by_fma(a, a.qn + (t * a.H + h) * HD, row0, n_ring, (int)(k_lo % a.cap), (long long)a.slot[b] * a.cap, g,
+                                        __shfl_sync(0xffffffffu, lo, from), __shfl_sync(0xffffffffu, hi, from), sc,
+                                        __shfl_sync(0xffffffffu, m, from));
+            const float f = __shfl_sync(0xffffffffu, inv, from);
+            float r[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (a.gate && !a.gate_per_head) r[e] *= 1.0f / (1.0f + expf(-a.gate[t * a.gate_ld + h * HD + 4 * lane + e]));
+                r[e] *= f;
+            }
+            *reinterpret_cast<uint2*>(a.out + t * a.out_ld + h * HD + 4 * lane) = make_uint2(pack_bf16x2(r[0], r[1]), pack_bf16x2(r[2], r[3]));
+        }
     }
     __syncthreads();
     if (warp == 2) {
