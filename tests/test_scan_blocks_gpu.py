@@ -231,3 +231,28 @@ def test_full_fp32_is_the_token_by_token_scan(kind, monkeypatch):
     want = run()
     assert all(torch.equal(a, b) for a, b in zip(got, want))
     assert not torch.equal(walk[0], want[0])  # the other form, at fp32 accuracy
+
+
+def test_a_capture_writes_its_own_lists():
+    """A step that a stream capture meets first, replayed, and the same step launched directly afterwards: the lists of the capture exist
+    in its replays only and must not be kept with the step."""
+    from llark_b200 import ops
+    from llark_b200.state_cache import StepLayout
+
+    torch.manual_seed(5)
+    H, D, E, lens = 2, 64, 32, [50, 20]
+    src, S0 = torch.randn(sum(lens), 3 * H * D, device="cuda"), torch.randn(2, H, D, E, device="cuda")
+    run = lambda st, s: ops.seq_glr_scan(src, 0, H * D, 2 * H * D, None, s, st, H, D, E)  # noqa: E731
+    want_s = S0.clone()
+    want = run(StepLayout(lens, [0, 0], [0, 1], "cuda"), want_s)
+    st, state = StepLayout(lens, [0, 0], [0, 1], "cuda"), S0.clone()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        got = run(st, state)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want) and torch.equal(state, want_s)
+    again = S0.clone()
+    assert torch.equal(run(st, again), want) and torch.equal(again, want_s)
+    del graph
