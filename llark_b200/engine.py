@@ -488,7 +488,7 @@ class LlamaEngine:
         ops.embed_splice_fwd(ids, table, None, None, None, None, x.view(B, 1, H))
         cos, sin = self._tables(cache.s_max, dev)
         cos_t, sin_t = cos[t:], sin[t:]  # row 0 of these views is position t: with S = 1 every row reads it
-        cache.lens.fill_(t + 1)
+        cache.lens.fill_(t + 1)  # the cache's own record, which attn_decode reads; the form below takes t
         few = B <= LINEAR_FEW_MAX and H % 8 == 0 and I % 8 == 0  # gate times up in the product's epilogue
         rstd = torch.empty(B, device=dev, dtype=torch.float32)
         for l in range(L):
