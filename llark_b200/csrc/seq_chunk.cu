@@ -26,7 +26,7 @@
 // steps, other sizes, the general rule and fp32 mode. What bounds this: one chain of blocks per head and 16 columns, in which a warp waits
 // for its own results most of the time. With one warp for all rows the walk took 1.6 times as long. Measured on a B200, heads of 128, us,
 // scan / here: HGRN2, 16 heads, 2048 + 1500 + 700 + 333 tokens 691 / 272; delta rule, 1777 + 1700 + 1500 tokens, a decay per head 1119 /
-// 410; 1000 + 600 tokens, a decay per channel 533 / 199, state space 425 / 112.
+// 416; 1000 + 600 tokens, a decay per channel 533 / 199, state space 425 / 112.
 #include "common.cuh"
 
 #include <utility>
@@ -351,13 +351,13 @@ template <int D, bool CORRECT> struct Layout {
 
 // A block with an infinity or a NaN in it, or in the state: its tokens one after another, by FMAs, so that nothing reaches the tokens in
 // front of it (0 times infinity above the diagonal would) and infinities stay what they are (their low part is NaN). Two warps, half of
-// the rows of 16 columns each, as in the walk below: st is this thread's first entry of the state (the walk keeps it in registers and
-// puts it there for this), V are the block's values from this column group on, xu the group's exchange buffer (128 floats a warp). Inlined:
+// the rows of 16 columns each, as in the walk below: S are this thread's entries of the state, laid out as there, V the block's values from
+// this column group on, xu the group's exchange buffer (128 floats a warp). Inlined:
 // with a call in it the walk was given 128 registers and took 342 us instead of 301 (HGRN2, 4 requests of 333 to 2048 tokens).
 struct Outputs { float mine[4], give[4]; };  // of the walk: four outputs of this warp's tokens, four of the other's
 template <int D, bool CORRECT>
 __device__ __forceinline__ Outputs block_by_tokens(const PrepArgs& p, int h, long long row0, int cnt, int half, const float* V, int VS,
-                                                   float* xu, int barrier, float* st, int E) {
+                                                   float* xu, int barrier, float (&S)[D / 16][4]) {
     constexpr int NT = D / 16;
     Outputs out = {};
     const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3, hd = half * (D / 2);
@@ -412,7 +412,7 @@ __device__ __forceinline__ Outputs block_by_tokens(const PrepArgs& p, int h, lon
             for (int c = 0; c < 2; ++c) {
                 float a = 0.f;
 #pragma unroll 1
-                for (int i = 0; i < 2 * NT; ++i) a = fmaf(st[(long long)(8 * (i >> 1) + (i & 1)) * E + 8 * c], z[i], a);
+                for (int i = 0; i < 2 * NT; ++i) a = fmaf(S[i >> 1][(i & 1) + 2 * c], z[i], a);
                 a += __shfl_xor_sync(0xffffffffu, a, 1);
                 a += __shfl_xor_sync(0xffffffffu, a, 2);
                 if (t4 == 0) xu[half * 128 + g + 8 * c] = a;
@@ -425,7 +425,7 @@ __device__ __forceinline__ Outputs block_by_tokens(const PrepArgs& p, int h, lon
         for (int c = 0; c < 2; ++c) {
 #pragma unroll 1
             for (int i = 0; i < 2 * NT; ++i) {
-                float& s = st[(long long)(8 * (i >> 1) + (i & 1)) * E + 8 * c];
+                float& s = S[i >> 1][(i & 1) + 2 * c];
                 s = fmaf(dd[i], s, pp[i] * u[c]);
                 o[c] = fmaf(s, qq[i], o[c]);
             }
@@ -511,32 +511,47 @@ chunk_scan_kernel(const __grid_constant__ ScanArgs p) {
         }
     };
     // Whether a block's results were finite is known at the barrier behind it, off the chain that the walk waits for. If they were not, the
-    // walk begins again (the state in memory is still that in front of it) and goes token by token from that block on.
+    // walk begins again (the state in memory is still that in front of it) and goes token by token from that block on, until every entry of
+    // the state is NaN: the products give what follows then (a request whose hidden states are NaN: one block, and not 10 us for every
+    // token of it).
     int slow = nblk;
-    bool odd = false;
+    bool odd = false, lost = false;
 again:
     fetch(0, sm);
     each_entry([&](float& s, float* at) { s = *at; });
     for (int k = 0; k < nblk; ++k) {
         const float* x = sm + (k & 1) * stage_floats;
         asm volatile("cp.async.wait_group 0;" ::: "memory");
-        if (__syncthreads_or(odd)) {  // this block is here, and everybody is done with the one before
-            slow = k - 1;
-            odd = false;
-            goto again;
+        const bool flag = __syncthreads_or(odd);  // this block is here, and everybody is done with the one before
+        if (slow == nblk) {
+            if (flag) {
+                slow = k - 1;
+                odd = false;
+                goto again;
+            }
+        } else if (k > slow && !flag) {
+            lost = true;
         }
         if (k + 1 < nblk) fetch(k + 1, sm + ((k + 1) & 1) * stage_floats);
         if (k) finish(k - 1);
-        if (k >= slow) {
+        if (k >= slow && !lost) {
             const int r0 = (c0 + k) * C;
-            each_entry([&](float& s, float* at) { *at = s; });
+            float kept[NT][4];  // indexed at run time, so not S itself
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) kept[nt][c] = S[nt][c];
             const Outputs out = block_by_tokens<D, CORRECT>(p.prep, h, row_b + r0, n - r0 < C ? n - r0 : C, half, x + Y::V + wc, VS,
-                                                            reinterpret_cast<float*>(xu + (warp & ~1) * 64), 1 + (warp >> 1),
-                                                            st + 2 * t4 * p.E + g, p.E);
-            each_entry([&](float& s, float* at) { s = *at; });
+                                                            reinterpret_cast<float*>(xu + (warp & ~1) * 64), 1 + (warp >> 1), kept);
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) S[nt][c] = kept[nt][c];
 #pragma unroll
             for (int c = 0; c < 4; ++c) mine[c] = out.mine[c];
             xo[(k & 1) * blockDim.x + warp * 32 + lane] = make_float4(out.give[0], out.give[1], out.give[2], out.give[3]);
+            odd = false;
+            each_entry([&](float& s, float*) { odd |= s == s; });  // something that is not NaN
             continue;
         }
         // ---- this warp's rows of S^T Q^T (and S^T Z^T)
@@ -625,7 +640,7 @@ again:
             }
         }
         xo[(k & 1) * blockDim.x + warp * 32 + lane] = make_float4(give[0], give[1], give[2], give[3]);
-        odd = !(fabsf((all[0] + all[1]) + (all[2] + all[3])) < INFINITY);
+        odd = slow == nblk && !(fabsf((all[0] + all[1]) + (all[2] + all[3])) < INFINITY);
         if (CORRECT) {
             asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp >> 1)) : "memory");  // the two warps of these columns
 #pragma unroll
@@ -664,7 +679,7 @@ again:
             }
         }
     }
-    if (__syncthreads_or(odd)) {
+    if (__syncthreads_or(odd) && slow == nblk) {
         slow = nblk - 1;
         odd = false;
         goto again;

@@ -256,3 +256,37 @@ def test_a_capture_writes_its_own_lists():
     again = S0.clone()
     assert torch.equal(run(st, again), want) and torch.equal(again, want_s)
     del graph
+
+
+@pytest.mark.parametrize("kind", ["hgrn2", "scalar", "state"])
+def test_a_request_that_is_nan_from_a_token_on(kind, monkeypatch):
+    """Every projection NaN from a token in the middle of a block on, over several blocks and passes: NaN from there, nothing before, and the
+    other request as alone."""
+    from llark_b200 import ops
+
+    torch.manual_seed(2)
+    lens, H, D, E, dev, bad = [150, 60], 2, 64, 32, "cuda", 37
+    n, st = sum(lens), _layout(lens, [1, 0])
+    src, mix, one = torch.randn(n, 3 * H * D, device=dev), torch.randn(n, H, device=dev), torch.ones(H, device=dev)
+    S0 = torch.randn(2, H, D, E, device=dev)
+    monkeypatch.setattr(ops, "SCAN_BLOCK_BYTES", 6 * H * ops.lib().llark_seq_chunk_block_bytes(D, 1))
+
+    def run():
+        s = S0.clone()
+        if kind == "hgrn2":
+            return ops.seq_glr_scan(src, 0, H * D, 2 * H * D, None, s, st, H, D, E), s
+        rule = ops.DELTA_GATED_SCALAR if kind == "scalar" else ops.DELTA_STATE_SPACE
+        return ops.seq_delta_rule(rule, src[:, :H * D], src[:, H * D:2 * H * D], src[:, 2 * H * D:], mix, None if kind == "state" else mix, s, st,
+                                  H, H, D, E, dec_bias=one, rate_log=one), s
+
+    want_o, want_s = run()
+    assert want_o.isfinite().all() and want_s.isfinite().all()
+    src[bad:lens[0]], mix[bad:lens[0]] = float("nan"), float("nan")
+    got_o, got_s = run()
+    assert got_o[bad:lens[0]].isnan().all() and got_s[1].isnan().all()
+    keep = torch.ones(n, dtype=torch.bool, device=dev)
+    keep[bad:lens[0]] = False
+    assert torch.equal(got_s[0], want_s[0]) and torch.equal(got_o[lens[0]:], want_o[lens[0]:])
+    # the block of the first bad token is summed by FMAs, everything in front of it by the same products
+    assert torch.equal(got_o[:bad // 16 * 16], want_o[:bad // 16 * 16])
+    assert ((got_o[keep] - want_o[keep]).norm() / want_o[keep].norm()).item() < 2e-6
