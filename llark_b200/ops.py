@@ -815,17 +815,18 @@ def scan_passes(cu_host, most):
 
 
 def _scan_tables(st, most):
-    """[(requests [n, 4], blocks [m, 2])] of each pass (llark_seq_glr_chunks), written by the device: no copy, and nothing that a stream
-    capture does not take. The layers of a step share them, but what a capture writes exists only in its replays."""
+    """[(lists, requests, blocks)] of each pass: int32 [4 requests + 2 blocks] as llark_seq_glr_chunks takes them, written by the device: no
+    copy, and nothing that a stream capture does not take. The layers of a step share them, but what a capture writes exists only in
+    its replays."""
     tables = None if torch.cuda.is_current_stream_capturing() else getattr(st, "tables", None)
     if tables is not None and ("scan", most) in tables:
         return tables["scan", most]
     out = []
     for done, each, n, m in scan_passes(st.cu_host, most):
         t = torch.empty(4 * n + 2 * m, device=st.device, dtype=torch.int32)
-        requests, blocks = t[:4 * n].view(n, 4), t[4 * n:].view(m, 2)
-        check(lib().llark_seq_chunk_plan(_p(st.cu), st.n_seq, done, each, _p(requests), _p(blocks), _stream()), "seq_chunk_plan")
-        out.append((requests, blocks))
+        at = t.data_ptr()
+        check(lib().llark_seq_chunk_plan(_p(st.cu), st.n_seq, done, each, at, at + 16 * n, _stream()), "seq_chunk_plan")
+        out.append((t, n, m))
     if tables is not None:
         tables["scan", most] = out
     return out
@@ -859,7 +860,7 @@ def _scan_blocks(kind, st, H, D, E, correct, tensors, offsets=()):
         return None
     per = lib().llark_seq_chunk_block_bytes(D, int(correct)) * H
     passes = _scan_tables(st, max(1, SCAN_BLOCK_BYTES // per))
-    return torch.empty(max(b.shape[0] for _, b in passes) * per, device=st.device, dtype=torch.uint8), passes
+    return torch.empty(max(m for _, _, m in passes) * per, device=st.device, dtype=torch.uint8), passes
 
 
 def seq_glr_scan(src, q_off, f_off, v_off, lower, state, st, H, D, E, full_fp32=False):
@@ -873,10 +874,10 @@ def seq_glr_scan(src, q_off, f_off, v_off, lower, state, st, H, D, E, full_fp32=
     blocks = None if full_fp32 else _scan_blocks("hgrn2", st, H, D, E, False, (src,), (q_off, f_off, v_off))
     if blocks is not None:
         ws, passes = blocks
-        for requests, blk in passes:
-            check(L.llark_seq_glr_chunks(_p(src), src.stride(0), q_off, f_off, v_off, _p(lower), _p(state), _p(o), _p(ws), _p(blk),
-                                         blk.shape[0], _p(requests), requests.shape[0], _p(st.cu), _p(st.slot), H, D, E, _stream()),
-                  "seq_glr_chunks")
+        for t, n, m in passes:
+            at = t.data_ptr()
+            check(L.llark_seq_glr_chunks(_p(src), src.stride(0), q_off, f_off, v_off, _p(lower), _p(state), _p(o), _p(ws), at + 16 * n, m,
+                                         at, n, _p(st.cu), _p(st.slot), H, D, E, _stream()), "seq_glr_chunks")
         return o
     if st.max_len < GLR_CHUNK_MIN_LEN:
         check(L.llark_seq_glr_scan(_p(src), src.stride(0), q_off, f_off, v_off, _p(lower), _p(state), _p(state), None,
@@ -1075,11 +1076,12 @@ def seq_delta_rule(rule, q, k, v, dec, mix, state, st, H, G, D, E, dec_bias=None
         _req(mix, torch.float32)
     ws, passes = blocks
     o = torch.empty((st.n_tok, H * E), device=v.device, dtype=torch.float32)
-    for requests, blk in passes:
+    for t, n, m in passes:
+        at = t.data_ptr()
         check(lib().llark_seq_delta_chunks(int(rule), _p(q), q.stride(0), _p(k), k.stride(0), _p(dec), dec.stride(0), _p(dec_bias),
                                            _p(rate_log), _p(mix), mix.stride(0) if mix is not None else 0, float(unit_eps), _p(v),
-                                           v.stride(0), _p(state), _p(o), _p(ws), _p(blk), blk.shape[0], _p(requests),
-                                           requests.shape[0], _p(st.cu), _p(st.slot), H, G, D, E, _stream()), "seq_delta_chunks")
+                                           v.stride(0), _p(state), _p(o), _p(ws), at + 16 * n, m, at, n, _p(st.cu), _p(st.slot), H, G,
+                                           D, E, _stream()), "seq_delta_chunks")
     return o
 
 

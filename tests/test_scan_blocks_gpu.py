@@ -195,7 +195,9 @@ def test_the_plan_of_a_pass(lens, most):
 
     st = _layout(lens, list(range(len(lens))))
     blocks = [-(-n // 16) for n in lens]
-    for (done, each, n, m), (requests, table) in zip(ops.scan_passes(st.cu_host, most), ops._scan_tables(st, most)):
+    for (done, each, n, m), (lists, n_, m_) in zip(ops.scan_passes(st.cu_host, most), ops._scan_tables(st, most)):
+        requests, table = lists[:4 * n].view(n, 4), lists[4 * n:].view(m, 2)
+        assert (n_, m_) == (n, m)
         want_r, want_b = [], []
         for b, x in enumerate(blocks):
             k = min(max(x - done, 0), each)
