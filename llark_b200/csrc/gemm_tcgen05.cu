@@ -34,12 +34,12 @@ constexpr int kThreads = 256;
 constexpr int A_STAGE_BYTES = BLOCK_M * BLOCK_KB;  // 16 KB
 constexpr int B_STAGE_BYTES = BLOCK_N * BLOCK_KB;  // 32 KB
 constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
-// Epilogue staging: every epilogue warp owns a [32 rows][32 + 4 pad fp32] patch of shared memory through which a 32-column
+// Epilogue staging: every epilogue warp owns a [32 rows][32 fp32] patch of shared memory through which a 32-column
 // accumulator chunk is transposed from "one row per thread" (what tcgen05.ld delivers) to "a quarter-warp per row", so
 // that the residual loads and the C stores of a warp instruction cover whole 128 B (fp32) / 64 B (bf16) row segments
 // instead of 32 different rows (see epilogue_tile_staged).
-constexpr int EPI_LD = 36;                        // floats per staged row; 36 = 32 + 4 keeps float4 rows conflict-free
-constexpr int EPI_WARP_BYTES = 32 * EPI_LD * 4;   // 4608 B per epilogue warp
+// Rows are 128 bytes, their 16-byte pieces exchanged by the row (128-byte swizzle), so that neither side has bank conflicts.
+constexpr int EPI_WARP_BYTES = 32 * 128;  // 4096 B per epilogue warp
 constexpr int EPI_STAGE_BYTES = 4 * EPI_WARP_BYTES;
 constexpr int SMEM_BYTES = kStages * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ + EPI_STAGE_BYTES;
 
@@ -63,7 +63,9 @@ struct GemmParams {
     // gate | up halves N apart; C receives dgate at column c and dup at column N + c), 5 squared ReLU, 6 gated ReLU (weight
     // rows alternate gate, up: C column c = relu(acc column 2c) * acc column 2c + 1; C has N / 2 columns), 7 the same with the
     // clamped gated unit (epi_f0 = limit, epi_f1 = slope)
-    int staged;      // 1 = staged (coalesced) epilogue, 0 = direct row-per-thread stores (see epilogue_dispatch)
+    int staged;      // 2 = through shared memory and TMA (CTA-pair kernel: epi_tma), 1 = staged (coalesced) epilogue,
+                     // 0 = direct row-per-thread stores (see epilogue_dispatch)
+    int stages;      // CTA-pair kernel: operand stages; what they leave of kSlots2 stages are the epilogue warps' patches
     int group_m;     // m-blocks per rasterisation group (tile_coord): sized on the host so a group's A panel stays in L2
     int epi;
     const void* epi_a;
@@ -245,15 +247,16 @@ __device__ __forceinline__ void epilogue_store_chunk(const GemmParams& p, long l
 // epilogue_store_chunk, or -- for the q and k columns of a fused-RoPE QKV projection -- pairs of chunks 64 columns
 // apart rotated as HF apply_rotary_pos_emb does in bf16: x = bf16(acc) (the Linear output),
 // out = bf16(bf16(x*cos) + bf16(rotate_half(x)*sin)), identical to llark_rope applied after an unfused GEMM.
+// [c_lo, c_hi): the 32-column chunks of the tile that this warp has (all eight, or four of them: whole heads of 128)
 template <int EPI>
 __device__ __forceinline__ void epilogue_tile(const GemmParams& p, long long row, bool row_ok, int ncol0,
-                                              uint32_t taddr) {
+                                              uint32_t taddr, int c_lo, int c_hi) {
     if (EPI == 2 && ncol0 < p.epi_i1) {
         const int spos = (int)(row % p.epi_i0);
         const __nv_bfloat16* cs = reinterpret_cast<const __nv_bfloat16*>(p.epi_a) + (long long)spos * 128;
         const __nv_bfloat16* sn = reinterpret_cast<const __nv_bfloat16*>(p.epi_b) + (long long)spos * 128;
 #pragma unroll 1
-        for (int hc = 0; hc < 4; ++hc) {
+        for (int hc = c_lo / 2; hc < c_hi / 2; ++hc) {
             const int clo = (hc >> 1) * 128 + (hc & 1) * 32;  // tile-local column of the low-half chunk
             if (ncol0 + clo >= p.N) break;                    // warp-uniform (N % 128 == 0 is checked on the host)
             uint32_t lo[32], hi[32];
@@ -284,7 +287,7 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, long long row
         return;
     }
 #pragma unroll 1
-    for (int c = 0; c < BLOCK_N / 32; ++c) {
+    for (int c = c_lo; c < c_hi; ++c) {
         const int col0 = ncol0 + c * 32;
         if (col0 >= p.N) break;  // warp-uniform
         uint32_t v[32];
@@ -307,11 +310,11 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, long long row
 // is the one that writes C[row, col], so C may alias R (in-place accumulation).
 template <int EPI>
 __device__ __forceinline__ void epi_staged_f32(const GemmParams& p, long long row0, int ncol0, uint32_t taddr, float* stg,
-                                               int lane) {
+                                               int lane, int c_lo, int c_hi) {
     const int rsub = lane >> 3, cq = (lane & 7) * 4;
     float* const C = reinterpret_cast<float*>(p.C);
     const float* const R = reinterpret_cast<const float*>(p.R);
-    const int nchunks = min(BLOCK_N / 32, (p.N - ncol0 + 31) / 32);  // warp-uniform
+    const int nchunks = min(c_hi, (p.N - ncol0 + 31) / 32);  // warp-uniform
     float4 rc[8], rn[8];
     auto load_res = [&](int col0, float4 (&r)[8]) {
         const int col = col0 + cq;
@@ -331,17 +334,17 @@ __device__ __forceinline__ void epi_staged_f32(const GemmParams& p, long long ro
             }
         }
     };
-    if (R) load_res(ncol0, rc);
+    if (R) load_res(ncol0 + c_lo * 32, rc);
 #pragma unroll 1
-    for (int c = 0; c < nchunks; ++c) {
+    for (int c = c_lo; c < nchunks; ++c) {
         const int col0 = ncol0 + c * 32;
         uint32_t v[32];
         tmem_ld_32x32b_x32(taddr + c * 32, v);
         tmem_ld_wait();
-        float* srow = stg + lane * EPI_LD;
+        float* srow = stg + lane * 32;
 #pragma unroll
         for (int j = 0; j < 8; ++j)
-            *reinterpret_cast<float4*>(srow + 4 * j) =
+            *reinterpret_cast<float4*>(srow + 4 * (j ^ (lane & 7))) =
                 make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]),
                             __uint_as_float(v[4 * j + 3]));
         __syncwarp();
@@ -360,7 +363,7 @@ __device__ __forceinline__ void epi_staged_f32(const GemmParams& p, long long ro
         for (int i = 0; i < 8; ++i) {
             const int r = i * 4 + rsub;
             const long long row = row0 + r;
-            const float4 a = *reinterpret_cast<const float4*>(stg + r * EPI_LD + cq);
+            const float4 a = *reinterpret_cast<const float4*>(stg + r * 32 + (cq ^ (4 * (r & 7))));
             if (row >= p.M || nc <= 0) continue;
             float f[4] = {a.x + b[0], a.y + b[1], a.z + b[2], a.w + b[3]};
             if constexpr (EPI == 1) {
@@ -387,14 +390,14 @@ __device__ __forceinline__ void epi_staged_f32(const GemmParams& p, long long ro
 
 template <int EPI>
 __device__ __forceinline__ void epi_staged_bf16(const GemmParams& p, long long row0, int ncol0, uint32_t taddr, float* stg,
-                                                int lane) {
+                                                int lane, int c_lo, int c_hi) {
     const int rsub = lane >> 2, cq = (lane & 3) * 8;
     __nv_bfloat16* const C = reinterpret_cast<__nv_bfloat16*>(p.C);
     // operand streamed alongside the accumulator: the residual R, or (EPI 3) gu = gate | up of the SwiGLU backward
     const __nv_bfloat16* const X = EPI == 3 ? reinterpret_cast<const __nv_bfloat16*>(p.epi_a)
                                             : reinterpret_cast<const __nv_bfloat16*>(p.R);
     const long long ldx = EPI == 3 ? p.epi_ld : p.ldr;
-    const int nchunks = min(BLOCK_N / 32, (p.N - ncol0 + 31) / 32);  // warp-uniform
+    const int nchunks = min(c_hi, (p.N - ncol0 + 31) / 32);  // warp-uniform
     uint4 xc[4], xn[4], uc[4], un[4];  // uc / un: the `up` half (EPI 3 only)
     auto load_x = [&](int col0, uint4 (&x)[4], uint4 (&u)[4]) {
         const int col = col0 + cq;
@@ -417,17 +420,17 @@ __device__ __forceinline__ void epi_staged_bf16(const GemmParams& p, long long r
             }
         }
     };
-    if (X) load_x(ncol0, xc, uc);
+    if (X) load_x(ncol0 + c_lo * 32, xc, uc);
 #pragma unroll 1
-    for (int c = 0; c < nchunks; ++c) {
+    for (int c = c_lo; c < nchunks; ++c) {
         const int col0 = ncol0 + c * 32;
         uint32_t v[32];
         tmem_ld_32x32b_x32(taddr + c * 32, v);
         tmem_ld_wait();
-        float* srow = stg + lane * EPI_LD;
+        float* srow = stg + lane * 32;
 #pragma unroll
         for (int j = 0; j < 8; ++j)
-            *reinterpret_cast<float4*>(srow + 4 * j) =
+            *reinterpret_cast<float4*>(srow + 4 * (j ^ (lane & 7))) =
                 make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]),
                             __uint_as_float(v[4 * j + 3]));
         __syncwarp();
@@ -448,8 +451,8 @@ __device__ __forceinline__ void epi_staged_bf16(const GemmParams& p, long long r
         for (int i = 0; i < 4; ++i) {
             const int r = i * 8 + rsub;
             const long long row = row0 + r;
-            const float4 a0 = *reinterpret_cast<const float4*>(stg + r * EPI_LD + cq);
-            const float4 a1 = *reinterpret_cast<const float4*>(stg + r * EPI_LD + cq + 4);
+            const float4 a0 = *reinterpret_cast<const float4*>(stg + r * 32 + (cq ^ (4 * (r & 7))));
+            const float4 a1 = *reinterpret_cast<const float4*>(stg + r * 32 + ((cq + 4) ^ (4 * (r & 7))));
             if (row >= p.M || nc <= 0) continue;
             float f[8] = {a0.x + b[0], a0.y + b[1], a0.z + b[2], a0.w + b[3],
                           a1.x + b[4], a1.y + b[5], a1.z + b[6], a1.w + b[7]};
@@ -503,23 +506,188 @@ __device__ __forceinline__ void epi_staged_bf16(const GemmParams& p, long long r
 
 // Epilogue of one 128 x 256 accumulator tile for the warp owning TMEM lanes [32 ew, 32 ew + 32): rows row0 .. row0 + 31.
 // The RoPE columns of a fused-QKV projection keep the row-per-thread path (rotation partners are 64 columns apart).
-// p.staged (chosen on the host, llark_gemm_ex) selects the staged path where the epilogue is the longer leg: a residual
-// with an fp32 tile or a short K, and the SwiGLU backward. Plain output at long K stays direct: its epilogue already hides
-// behind the next tile's MMAs, and the staging patch's extra 256 KB of shared-memory traffic per tile slows the operand
-// pipeline by 3-8 % (profiles/r2c_epilogue_ab.md, profiles/r2k_epilogue_probe.md).
-template <int EPI>
+// p.staged == 1 (chosen on the host, llark_gemm_ex) selects the staged path where the epilogue is the longer leg: the SwiGLU
+// backward and, in the single-CTA kernel, a residual with an fp32 tile or a short K. Plain output at long K stays direct there: its
+// epilogue already hides behind the next tile's MMAs, and the staging patch's extra 256 KB of shared-memory traffic per tile slows
+// the operand pipeline by 3-8 % (profiles/r2c_epilogue_ab.md, profiles/r2k_epilogue_probe.md).
+template <int EPI, bool STAGED>
 __device__ __forceinline__ void epilogue_dispatch(const GemmParams& p, long long row0, long long m_end, int lane, int ncol0,
-                                                  uint32_t taddr, float* stg) {
-    if ((EPI == 2 && ncol0 < p.epi_i1) || EPI == 5 || EPI == 6 || EPI == 7 || !p.staged) {
+                                                  uint32_t taddr, float* stg, int c_lo, int c_hi) {
+    if (!STAGED || (EPI == 2 && ncol0 < p.epi_i1) || EPI == 5 || EPI == 6 || EPI == 7 || p.staged != 1) {
         const long long row = row0 + lane;
-        epilogue_tile<EPI>(p, row, row < m_end, ncol0, taddr);
+        epilogue_tile<EPI>(p, row, row < m_end, ncol0, taddr, c_lo, c_hi);
         return;
     }
-    if constexpr (EPI != 5 && EPI != 6) {  // these two have no staged form
+    if constexpr (STAGED && EPI != 5 && EPI != 6 && EPI != 7) {  // these have no staged form
         if (p.c_fp32) {
-            if constexpr (EPI == 0 || EPI == 1) epi_staged_f32<EPI>(p, row0, ncol0, taddr, stg, lane);
+            if constexpr (EPI == 0 || EPI == 1) epi_staged_f32<EPI>(p, row0, ncol0, taddr, stg, lane, c_lo, c_hi);
         } else {
-            epi_staged_bf16<EPI>(p, row0, ncol0, taddr, stg, lane);
+            epi_staged_bf16<EPI>(p, row0, ncol0, taddr, stg, lane, c_lo, c_hi);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// Epilogue of the CTA-pair kernel through TMA. A warp's share of a tile, 32 rows x 128 columns, goes out in pieces of 32
+// rows x 128 bytes: the accumulators of a row are its own thread's, which writes them into the warp's patch (128-byte
+// swizzle), and one TMA store takes the piece to C, cut off at the edges of C. A residual comes in the same way, into the
+// patch that its sums leave by, one piece ahead and the first of a tile while the tile is still being multiplied. The
+// arithmetic of an element is that of epilogue_store_chunk, and R's element is read before C's is written: C may be R.
+//
+// What it is bound by: nothing of its own at long K (it hides behind the next tile's products); with a short K the bytes of
+// R that are under way, here 32 KB to 64 KB per SM where four warps with loads to registers had 16 KB. Measured on a B200, us before -> now:
+// M 16384, N 4800, K 1200, fp32 with a residual 316 -> 204; K 4800, fp32 with a residual 609 -> 595, bf16 with quick-GELU 617 -> 544; M 6100,
+// N 6144, K 2048, fp32 163 -> 134; M 8192, bf16: N 12288, K 4096 559 -> 555, N 4096, K 4096 with a residual 203 -> 198, N 32000 1438 -> 1428.
+// Eight warps with direct stores: slower than four in all of these by 1 to 2 % (569 us where TMA takes 555).
+__device__ __forceinline__ void load_bias32(const GemmParams& p, int col0, float (&b)[32]) {
+    if (col0 + 32 <= p.N && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) {  // the same addresses for the whole warp
+        if (p.bias_fp32) {
+            const float4* src = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.bias) + col0);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float4 t = src[j];
+                b[4 * j] = t.x; b[4 * j + 1] = t.y; b[4 * j + 2] = t.z; b[4 * j + 3] = t.w;
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float t[8];
+                ld8_bf16(reinterpret_cast<const __nv_bfloat16*>(p.bias) + col0 + 8 * j, t);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) b[8 * j + e] = t[e];
+            }
+        }
+        return;
+    }
+#pragma unroll
+    for (int e = 0; e < 32; ++e) {
+        const int col = col0 + e;
+        b[e] = col >= p.N ? 0.f
+                          : (p.bias_fp32 ? reinterpret_cast<const float*>(p.bias)[col]
+                                         : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[col]));
+    }
+}
+// 32 sums of a row: bias and activation
+template <int EPI>
+__device__ __forceinline__ void epi_values(const GemmParams& p, int col0, const uint32_t (&v)[32], float (&f)[32]) {
+#pragma unroll
+    for (int e = 0; e < 32; ++e) f[e] = __uint_as_float(v[e]);
+    if (p.bias) {
+        float b[32];
+        load_bias32(p, col0, b);
+#pragma unroll
+        for (int e = 0; e < 32; ++e) f[e] += b[e];
+    }
+    if constexpr (EPI == 1) {
+#pragma unroll
+        for (int e = 0; e < 32; ++e) f[e] = f[e] / (1.f + __expf(-1.702f * f[e]));
+    } else if constexpr (EPI == 5) {
+#pragma unroll
+        for (int e = 0; e < 32; ++e) {
+            const float r = fmaxf(f[e], 0.f);
+            f[e] = r * r;
+        }
+    }
+}
+struct EpiPatch {  // an epilogue warp's patches and how far it is: piece g lies in patch g % 2 (with one patch: always in it)
+    uint8_t* at;
+    uint64_t* bar;  // [2] the residual's piece has arrived
+    int n;          // patches: 2, or 1 where the operand stages take the room
+    uint32_t g;
+};
+__device__ __forceinline__ uint8_t* patch_of(const EpiPatch& e, uint32_t g) { return e.at + (e.n == 2 ? (g & 1u) * EPI_WARP_BYTES : 0u); }
+// lane 0: ask for the residual of piece g, whose patch is free once the piece before the last has been stored
+__device__ __forceinline__ void ask_residual(const EpiPatch& e, uint32_t g, const CUtensorMap* rmap, int col, int row) {
+    tma_store_wait_read<0>();
+    uint64_t* bar = &e.bar[g & 1u];
+    mbar_arrive_expect_tx(bar, EPI_WARP_BYTES);
+    tma_load_2d(patch_of(e, g), rmap, bar, col, row);
+}
+// Pieces of this warp in a tile: columns [col_lo, col_lo + 128) of N, rows from row0 on. A row of C that ends inside 16 bytes
+// is cut off behind them by TMA (the bytes beside C were overwritten): its last columns are left to epi_rest.
+__device__ __forceinline__ int epi_pieces(const GemmParams& p, long long row0, int col_lo) {
+    if (row0 >= p.M || col_lo >= p.N) return 0;
+    const int w = p.c_fp32 ? 32 : 64, last = p.N % (p.c_fp32 ? 4 : 8) ? p.N / w : (p.N + w - 1) / w;
+    return min(128 / w, last - col_lo / w);
+}
+template <int EPI>
+__device__ __forceinline__ void epi_rest(const GemmParams& p, long long row, int col_lo, int pieces, uint32_t taddr) {
+    const int end = min(col_lo + 128, p.N);
+#pragma unroll 1
+    for (int col = col_lo + pieces * (p.c_fp32 ? 32 : 64); col < end; col += 32) {
+        uint32_t v[32];
+        tmem_ld_32x32b_x32(taddr + (col - col_lo), v);
+        tmem_ld_wait();
+        if (row < p.M) epilogue_store_chunk<EPI>(p, row, col, v);
+    }
+}
+template <int EPI>
+__device__ __forceinline__ void epi_tma(const GemmParams& p, const CUtensorMap* cmap, const CUtensorMap* rmap, int row0, int col_lo,
+                                        int pieces, uint32_t taddr, EpiPatch& e, int lane) {
+    const int w = p.c_fp32 ? 32 : 64;
+    const bool res = p.R != nullptr;
+#pragma unroll 1
+    for (int c = 0; c < pieces; ++c, ++e.g) {
+        uint8_t* const patch = patch_of(e, e.g);
+        const int col0 = col_lo + c * w;
+        if (res) {
+            if (lane == 0 && c + 1 < pieces) ask_residual(e, e.g + 1, rmap, col0 + w, row0);
+            mbar_wait(&e.bar[e.g & 1u], (e.g >> 1) & 1u);
+        } else {
+            if (lane == 0) {
+                if (e.n == 2)
+                    tma_store_wait_read<1>();
+                else
+                    tma_store_wait_read<0>();
+            }
+            __syncwarp();
+        }
+        uint8_t* const row = patch + lane * 128;
+        const int sw = lane & 7;
+        if (p.c_fp32) {
+            uint32_t v[32];
+            float f[32];
+            tmem_ld_32x32b_x32(taddr + c * 32, v);
+            tmem_ld_wait();
+            epi_values<EPI>(p, col0, v, f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                float4* q = reinterpret_cast<float4*>(row + ((j ^ sw) << 4));
+                if (res) {
+                    const float4 r = *q;
+                    f[4 * j] += r.x; f[4 * j + 1] += r.y; f[4 * j + 2] += r.z; f[4 * j + 3] += r.w;
+                }
+                *q = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
+            }
+        } else {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint32_t v[32];
+                float f[32];
+                tmem_ld_32x32b_x32(taddr + c * 64 + h * 32, v);
+                tmem_ld_wait();
+                epi_values<EPI>(p, col0 + h * 32, v, f);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    __nv_bfloat16* q = reinterpret_cast<__nv_bfloat16*>(row + (((h * 4 + j) ^ sw) << 4));
+                    float o[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) o[i] = f[8 * j + i];
+                    if (res) {
+                        float r[8];
+                        ld8_bf16(q, r);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) o[i] += r[i];
+                    }
+                    st8_bf16(q, o);
+                }
+            }
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+            tma_store_2d(cmap, patch, col0, row0);
+            tma_store_commit();
         }
     }
 }
@@ -663,8 +831,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
             mbar_wait(&tmem_full[as], aphase);
             tc_fence_after();
             const long long row0 = (long long)tc.m_blk * BLOCK_M + ew * 32;
-            epilogue_dispatch<EPI>(p, row0, p.M, lane, tc.n_blk * BLOCK_N, tmem_base + ((uint32_t)(ew * 32) << 16) + as * BLOCK_N,
-                                   epi_stage + ew * (EPI_WARP_BYTES / 4));
+            epilogue_dispatch<EPI, true>(p, row0, p.M, lane, tc.n_blk * BLOCK_N, tmem_base + ((uint32_t)(ew * 32) << 16) + as * BLOCK_N,
+                                   epi_stage + ew * (EPI_WARP_BYTES / 4), 0, BLOCK_N / 32);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&tmem_empty[as]);
@@ -685,29 +853,35 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
 // (rank 0) issues tcgen05.mma.cta_group::2 (M = 256, N = 256) which reads both CTAs' operands, and each CTA's
 // TMEM receives its 128 accumulator rows x 256 columns. Per SM the shared-memory traffic drops from
 // 96 (TMA writes) + 96 (UMMA reads) B/clk to 64 + 64 B/clk, which is what lets the tensor pipe stay busy.
-constexpr int kStages2 = 6;
+constexpr int kThreads2 = 384;   // warps 0-3 as above, 4-11 epilogue: two per 32 rows, 128 columns each
+constexpr int kEpiWarps2 = 8;
+constexpr int kSlots2 = 7;       // 32 KB slots of shared memory: operand stages, the epilogue warps' patches behind them
+constexpr int kMaxStages2 = 6;   // six stages and a patch per warp, or five and two (GemmParams::stages)
 constexpr int kSched = 4;  // depth of the tile-index ring of the dynamic scheduler
 constexpr int B2_STAGE_BYTES = 128 * BLOCK_KB;  // this CTA's half of B: 16 KB
 constexpr int STAGE2_BYTES = A_STAGE_BYTES + B2_STAGE_BYTES;  // 32 KB per CTA per stage
-constexpr int SMEM2_BYTES = kStages2 * STAGE2_BYTES + 1024 + 512 + EPI_STAGE_BYTES;
+constexpr int SMEM2_BYTES = kSlots2 * STAGE2_BYTES + 1024 + 512;
+static_assert(kEpiWarps2 * EPI_WARP_BYTES == STAGE2_BYTES, "one patch per epilogue warp fills a slot");
 
 template <int A_MN, int B_MN, int TF32, int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads2, 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-             const GemmParams p) {
+             const __grid_constant__ CUtensorMap tma_c, const __grid_constant__ CUtensorMap tma_r, const GemmParams p) {
     constexpr int kElemBytes = TF32 ? 4 : 2;  // operand element size is a property of the instantiation
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kStages2 * STAGE2_BYTES);
-    uint64_t* empty_bar = full_bar + kStages2;
-    uint64_t* tmem_full = empty_bar + kStages2;
+    const int stages = p.stages;
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kSlots2 * STAGE2_BYTES);
+    uint64_t* empty_bar = full_bar + kMaxStages2;
+    uint64_t* tmem_full = empty_bar + kMaxStages2;
     uint64_t* tmem_empty = tmem_full + kAccStages;
     uint64_t* sched_full = tmem_empty + kAccStages;   // [kSched] tile index published (one arrive per CTA)
-    uint64_t* sched_empty = sched_full + kSched;      // [kSched] leader's: all 13 consumers of the pair have read it
-    uint32_t* sched_tile = reinterpret_cast<uint32_t*>(sched_empty + kSched);  // [kSched]
+    uint64_t* sched_empty = sched_full + kSched;      // [kSched] leader's: all consumers of the pair have read it
+    uint64_t* res_bar = sched_empty + kSched;         // [epilogue warps][2]
+    uint32_t* sched_tile = reinterpret_cast<uint32_t*>(res_bar + 2 * kEpiWarps2);  // [kSched]
     uint32_t* tmem_base_slot = sched_tile + kSched;
-    float* epi_stage = reinterpret_cast<float*>(smem + kStages2 * STAGE2_BYTES + 512);
+    uint8_t* epi_stage = smem + stages * STAGE2_BYTES;
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -723,20 +897,23 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
     if (warp == 0 && lane == 0) {
         tma_prefetch_desc(&tma_a);
         tma_prefetch_desc(&tma_b);
+        if (p.staged == 2) tma_prefetch_desc(&tma_c);
+        if (p.staged == 2 && p.R) tma_prefetch_desc(&tma_r);
     }
     if (warp == 1 && lane == 0) {
-        for (int i = 0; i < kStages2; ++i) {
+        for (int i = 0; i < stages; ++i) {
             mbar_init(&full_bar[i], 1);   // leader: one arrive.expect_tx covering both CTAs' bytes
             mbar_init(&empty_bar[i], 1);  // one multicast tcgen05.commit arrive per CTA
         }
         for (int i = 0; i < kAccStages; ++i) {
             mbar_init(&tmem_full[i], 1);
-            mbar_init(&tmem_empty[i], 8);  // 4 epilogue warps x 2 CTAs arrive on the leader's barrier
+            mbar_init(&tmem_empty[i], 2 * kEpiWarps2);  // the epilogue warps of both CTAs arrive on the leader's barrier
         }
         for (int i = 0; i < kSched; ++i) {
             mbar_init(&sched_full[i], 1);
-            mbar_init(&sched_empty[i], 13);  // leader: A/B producers, MMA, 4 epilogue warps; peer: the same minus MMA
+            mbar_init(&sched_empty[i], 5 + 2 * kEpiWarps2);  // A/B producers and epilogue warps of both CTAs, the leader's MMA
         }
+        for (int i = 0; i < 2 * kEpiWarps2; ++i) mbar_init(&res_bar[i], 1);
         mbar_fence_init();
         fence_proxy_async_smem();
     }
@@ -861,7 +1038,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
                         }
                     }
                 }
-                if (++stage == kStages2) {
+                if (++stage == stages) {
                     stage = 0;
                     phase ^= 1;
                 }
@@ -913,7 +1090,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
                         umma_f16_2sm(tmem_d, ad, bd, idesc, (kb | k) != 0);
                 }
                 umma_commit_2sm(&empty_bar[stage], 3);  // frees the slot in BOTH CTAs
-                if (++stage == kStages2) {
+                if (++stage == stages) {
                     stage = 0;
                     phase ^= 1;
                 }
@@ -922,24 +1099,37 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
         }
     } else if (warp >= 4) {
         // ===================== epilogue (both CTAs, own 128 rows) =====================
-        const int ew = warp - 4;
+        const int ew = warp & 3, half = (warp - 4) >> 2;  // TMEM lanes 32 ew .. are open to warps with this warp % 4
         int it = 0;
         const uint32_t leader_empty0 = mapa_shared(smem_u32(&tmem_empty[0]), 0);
+        const int n_patches = kSlots2 - stages;
+        EpiPatch patch = {epi_stage + (warp - 4) * n_patches * EPI_WARP_BYTES, res_bar + 2 * (warp - 4), n_patches, 0u};
         for (int tile = next_tile(true); tile >= 0; tile = next_tile(true), ++it) {
             const TileCoord tc = tile_coord(tile, num_m_blocks, p.num_n_blocks, p.group_m);
             const int as = it & 1;
             const uint32_t aphase = (it >> 1) & 1;
-            mbar_wait(&tmem_full[as], aphase);
-            tc_fence_after();
             const long long mbase = p.seg_tiles ? p.seg_tiles[3 * tc.m_blk + 1] : (long long)tc.m_blk * 256;
             const long long m_end = p.seg_tiles ? mbase + p.seg_tiles[3 * tc.m_blk + 2] : (long long)p.M;
             const long long row0 = mbase + (long long)rank * 128 + ew * 32;
-            epilogue_dispatch<EPI>(p, row0, m_end, lane, tc.n_blk * BLOCK_N, tmem_base + ((uint32_t)(ew * 32) << 16) + as * BLOCK_N,
-                                   epi_stage + ew * (EPI_WARP_BYTES / 4));
+            const int ncol0 = tc.n_blk * BLOCK_N;
+            const uint32_t acc = tmem_base + ((uint32_t)(ew * 32) << 16) + as * BLOCK_N;
+            if ((EPI == 0 || EPI == 1 || EPI == 2 || EPI == 5) && p.staged == 2 && !(EPI == 2 && ncol0 < p.epi_i1)) {
+                const int pieces = epi_pieces(p, row0, ncol0 + half * 128);
+                if (p.R && pieces && lane == 0) ask_residual(patch, patch.g, &tma_r, ncol0 + half * 128, (int)row0);
+                mbar_wait(&tmem_full[as], aphase);
+                tc_fence_after();
+                epi_tma<EPI>(p, &tma_c, &tma_r, (int)row0, ncol0 + half * 128, pieces, acc + half * 128, patch, lane);
+                epi_rest<EPI>(p, row0 + lane, ncol0 + half * 128, pieces, acc + half * 128);
+            } else {
+                mbar_wait(&tmem_full[as], aphase);
+                tc_fence_after();
+                epilogue_dispatch<EPI, EPI == 3>(p, row0, m_end, lane, ncol0, acc, reinterpret_cast<float*>(patch.at), half * 4, half * 4 + 4);
+            }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_remote(leader_empty0 + (uint32_t)as * 8u);
         }
+        if (lane == 0) tma_store_wait_all();
     }
 
     tc_fence_before();
@@ -1132,8 +1322,12 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams
     return LLARK_OK;
 }
 
+struct GemmMaps {  // of C and R, where the epilogue goes through TMA
+    CUtensorMap c, r;
+};
+
 template <int A_MN, int B_MN, int TF32, int EPI = 0>
-static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int max_ctas, cudaStream_t stream) {
+static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const GemmMaps& m, const GemmParams& p, int max_ctas, cudaStream_t stream) {
     static bool attr_set = false;
     auto kfn = gemm2_kernel<A_MN, B_MN, TF32, EPI>;
     if (!attr_set) {
@@ -1149,7 +1343,7 @@ static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParam
     if (tiles < clusters) clusters = tiles;
     if (max_ctas > 1 && clusters > max_ctas / 2) clusters = max_ctas / 2;
     if (clusters < 1) clusters = 1;
-    kfn<<<clusters * 2, kThreads, SMEM2_BYTES, stream>>>(ta, tb, p);
+    kfn<<<clusters * 2, kThreads2, SMEM2_BYTES, stream>>>(ta, tb, m.c, m.r, p);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         g_last_cuda_error = (int)e;
@@ -1339,12 +1533,12 @@ extern "C" int llark_gemm_ex(const void* A, int a_mn_major, long long lda, const
     p.seg_count = segs ? static_cast<const int*>(ep->b) : nullptr;
     if (segs) p.num_m_blocks = ep->i0;
     {
-        static int mode = -1;  // LLARK_GEMM_EPILOGUE = auto (default) | staged | direct
+        static int mode = -1;  // LLARK_GEMM_EPILOGUE = auto (default) | staged (single-CTA kernel) | direct
         if (mode < 0) {
             const char* e = getenv("LLARK_GEMM_EPILOGUE");
             mode = (e && e[0] == 's') ? 1 : ((e && e[0] == 'd') ? 2 : 0);
         }
-        // auto: staged where the isolated-GEMM probe (tools/gemm_epilogue_probe.py, profiles/r2k_epilogue_probe.md) and
+        // auto, single-CTA kernel: staged where the isolated-GEMM probe (tools/gemm_epilogue_probe.py, profiles/r2k_epilogue_probe.md) and
         // the in-step A/B (profiles/r2c_epilogue_ab.md) measured it faster -- the SwiGLU backward; any residual with an fp32
         // tile (K = 1200: 17.8 vs 21.6 us per tile, K = 4800: 35.8 vs 36.2) or with a short K (bf16, K = 1200: 12.8 vs 16.5);
         // fp32 tiles without a residual only when K is short (K = 4800: direct 32.4 vs staged 35.1). Otherwise direct.
@@ -1352,6 +1546,19 @@ extern "C" int llark_gemm_ex(const void* A, int a_mn_major, long long lda, const
         const bool want = p.epi == LLARK_EPI_SWIGLU_BWD || (R != nullptr && (c_fp32 || short_k)) ||
                           (c_fp32 && R == nullptr && short_k);
         p.staged = segs ? 0 : (mode == 1 ? 1 : (mode == 2 ? 0 : (want ? 1 : 0)));
+        // The CTA pair's epilogue goes through TMA wherever an element of C depends on nothing but its own sum, bias and
+        // residual; rows in runs end inside a tile, where a piece of 32 rows must not write, and keep the direct stores.
+        if (two_cta && !segs && mode == 0 &&
+            (p.epi == LLARK_EPI_NONE || p.epi == LLARK_EPI_QUICK_GELU || p.epi == LLARK_EPI_ROPE || p.epi == LLARK_EPI_RELU2))
+            p.staged = 2;
+        p.stages = p.staged == 2 && R ? kMaxStages2 - 1 : kMaxStages2;
+    }
+    GemmMaps cr = {};
+    if (p.staged == 2) {
+        const int ceb = c_fp32 ? 4 : 2;
+        rc = get_tensor_map(&cr.c, C, N, M, ldc, 128 / ceb, 32, ceb);
+        if (rc == LLARK_OK && R) rc = get_tensor_map(&cr.r, R, N, M, ldr, 128 / ceb, 32, ceb);
+        if (rc != LLARK_OK) return rc;
     }
     {
         // Rasterisation group: tiles sweep n inside groups of `group_m` m-blocks, so a group's A panel
@@ -1392,38 +1599,38 @@ extern "C" int llark_gemm_ex(const void* A, int a_mn_major, long long lda, const
     if (p.epi != LLARK_EPI_NONE) {
         // fused epilogues exist for the operand layouts their call sites use (validated above for everything else)
         if (p.epi == LLARK_EPI_QUICK_GELU && sel == 0) {
-            if (two_cta) return in_fp32 ? launch2<0, 0, 1, 1>(ta, tb, p, max_ctas, stream)
-                                        : launch2<0, 0, 0, 1>(ta, tb, p, max_ctas, stream);
+            if (two_cta) return in_fp32 ? launch2<0, 0, 1, 1>(ta, tb, cr, p, max_ctas, stream)
+                                        : launch2<0, 0, 0, 1>(ta, tb, cr, p, max_ctas, stream);
             return in_fp32 ? launch<0, 0, 1, 1>(ta, tb, p, max_ctas, stream)
                            : launch<0, 0, 0, 1>(ta, tb, p, max_ctas, stream);
         }
         if (p.epi == LLARK_EPI_ROPE && sel == 0 && !in_fp32)
-            return two_cta ? launch2<0, 0, 0, 2>(ta, tb, p, max_ctas, stream)
+            return two_cta ? launch2<0, 0, 0, 2>(ta, tb, cr, p, max_ctas, stream)
                            : launch<0, 0, 0, 2>(ta, tb, p, max_ctas, stream);
         if (p.epi == LLARK_EPI_SWIGLU_BWD && sel == 1 && !in_fp32)
-            return two_cta ? launch2<0, 1, 0, 3>(ta, tb, p, max_ctas, stream)
+            return two_cta ? launch2<0, 1, 0, 3>(ta, tb, cr, p, max_ctas, stream)
                            : launch<0, 1, 0, 3>(ta, tb, p, max_ctas, stream);
         if (p.epi == LLARK_EPI_RELU2 && sel == 0 && !in_fp32)
-            return two_cta ? launch2<0, 0, 0, 5>(ta, tb, p, max_ctas, stream)
+            return two_cta ? launch2<0, 0, 0, 5>(ta, tb, cr, p, max_ctas, stream)
                            : launch<0, 0, 0, 5>(ta, tb, p, max_ctas, stream);
         if (p.epi == LLARK_EPI_RELU_GLU && sel == 0 && !in_fp32)
-            return two_cta ? launch2<0, 0, 0, 6>(ta, tb, p, max_ctas, stream)
+            return two_cta ? launch2<0, 0, 0, 6>(ta, tb, cr, p, max_ctas, stream)
                            : launch<0, 0, 0, 6>(ta, tb, p, max_ctas, stream);
         if (p.epi == LLARK_EPI_CLAMP_GLU && sel == 0 && !in_fp32)
-            return two_cta ? launch2<0, 0, 0, 7>(ta, tb, p, max_ctas, stream)
+            return two_cta ? launch2<0, 0, 0, 7>(ta, tb, cr, p, max_ctas, stream)
                            : launch<0, 0, 0, 7>(ta, tb, p, max_ctas, stream);
         return LLARK_EINVAL;
     }
     if (two_cta) {
         if (!in_fp32) {
             switch (sel) {
-                case 0: return launch2<0, 0, 0>(ta, tb, p, max_ctas, stream);
-                case 1: return launch2<0, 1, 0>(ta, tb, p, max_ctas, stream);
-                case 2: return launch2<1, 0, 0>(ta, tb, p, max_ctas, stream);
-                default: return launch2<1, 1, 0>(ta, tb, p, max_ctas, stream);
+                case 0: return launch2<0, 0, 0>(ta, tb, cr, p, max_ctas, stream);
+                case 1: return launch2<0, 1, 0>(ta, tb, cr, p, max_ctas, stream);
+                case 2: return launch2<1, 0, 0>(ta, tb, cr, p, max_ctas, stream);
+                default: return launch2<1, 1, 0>(ta, tb, cr, p, max_ctas, stream);
             }
         }
-        return launch2<0, 0, 1>(ta, tb, p, max_ctas, stream);
+        return launch2<0, 0, 1>(ta, tb, cr, p, max_ctas, stream);
     }
     if (!in_fp32) {
         switch (sel) {

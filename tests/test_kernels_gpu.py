@@ -123,6 +123,30 @@ def test_gemm_bias_residual_and_fp32_out(gemm_mode):
     assert _rel(out32, a.float() @ b.float().t()) < 1e-5
 
 
+@pytest.mark.parametrize("M,N,K", [(65, 8, 64), (129, 36, 192), (257, 132, 72), (300, 260, 640), (1500, 1030, 128)])
+@pytest.mark.parametrize("dt", [torch.float32, BF16])
+def test_gemm_output_pieces_end_at_the_edges(M, N, K, dt):
+    """Rows and columns that end inside a piece of 32 rows x 128 bytes, every combination of bias and residual, in place too:
+    against 64 bits (fp32 sums: 2^-20 of the result, a bf16 result 2^-8) and nothing written beside C."""
+    ops = _ops()
+    torch.manual_seed(M + N + K)
+    a, b = (torch.randn(M, K, device="cuda")).to(BF16), (torch.randn(N, K, device="cuda")).to(BF16)
+    z = a.double() @ b.double().t()
+    bias, ld = torch.randn(N + 1, device="cuda")[1:], (N + 7) // 8 * 8 + 8  # a bias off 16-byte boundaries
+    res = torch.randn(M + 2, ld, device="cuda").to(dt)
+    tol = 2.0 ** -20 if dt == torch.float32 else 2.0 ** -8
+    for with_bias in (False, True):
+        for with_res, in_place in ((False, False), (True, False), (True, True)):
+            buf = res.clone() if in_place else torch.full((M + 2, ld), 7.0, device="cuda", dtype=dt)
+            was = buf.clone()
+            ops.gemm(a, b, out=buf[1:M + 1], N=N, bias=bias if with_bias else None,
+                     residual=(buf if in_place else res)[1:M + 1, :N] if with_res else None)
+            want = z + (bias.double() if with_bias else 0) + (res[1:M + 1, :N].double() if with_res else 0)
+            assert ((buf[1:M + 1, :N].double() - want).norm() / want.norm()).item() < tol
+            buf[1:M + 1, :N] = was[1:M + 1, :N]
+            assert torch.equal(buf, was)
+
+
 def test_gemm_tf32_mn_major_rejected():
     ops = _ops()
     from llark_b200._lib import LlarkError
