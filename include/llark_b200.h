@@ -229,6 +229,11 @@ int llark_jb_conv_down(const float* x, const float* w, const float* bias, float*
 /* Fused ResConv1DBlock: y = x + W2 * relu(W1 (*dil) relu(x) + b1) + b2, width 32 channels. x,y [N,32,T]. */
 int llark_jb_resblock(const float* x, const float* w1, const float* b1, const float* w2, const float* b2, float* y,
                       int N, int T, int dilation, cudaStream_t stream);
+/* The first n of a run of such blocks that one visit takes (0: none, they go one by one), and that visit. weights: w1, b1, w2, b2 of
+ * block 0, then of block 1, ... (device pointers in a host array); n of llark_jb_resblocks is at most llark_jb_resblocks_length. */
+int llark_jb_resblocks_length(const int* dilations, int n);
+int llark_jb_resblocks(const float* x, const float* const* weights, const int* dilations, int n, float* y, int N, int T,
+                       cudaStream_t stream);
 /* Conv1d(c_in -> c_out, k=3, s=1, p=1) + bias (block output projection 32 -> 64). */
 int llark_jb_conv_k3(const float* x, const float* w, const float* bias, float* y, int N, int c_in, int c_out, int T,
                      cudaStream_t stream);

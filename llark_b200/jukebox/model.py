@@ -21,6 +21,7 @@ from types import SimpleNamespace
 import torch
 
 from llark_b200 import ops
+from llark_b200.ops import jb_resblocks
 
 BF16 = torch.bfloat16
 
@@ -91,16 +92,19 @@ class JukeboxVQVAE:
         self.sample_length = cfg.sample_length
 
     def encode_top_latents(self, x):
-        """x fp32 [N,1,T] -> fp32 [N,64,T/128] (time-tiled fused res-blocks, one HBM pass per block)."""
+        """x fp32 [N,1,T] -> fp32 [N,64,T/128] (the res blocks of a level in one HBM pass)."""
         cfg, w = self.cfg, self.w
         h = x
         for b, down_t in enumerate(cfg.downs_t):
             for i in range(down_t):
                 h = ops.jb_conv_down(h, w[f"enc.{b}.down.{i}.w"], w[f"enc.{b}.down.{i}.b"])
-                for d in range(cfg.depth):
-                    h = ops.jb_resblock(h, w[f"enc.{b}.res.{i}.{d}.w1"], w[f"enc.{b}.res.{i}.{d}.b1"],
-                                        w[f"enc.{b}.res.{i}.{d}.w2"], w[f"enc.{b}.res.{i}.{d}.b2"],
-                                        cfg.dilation_growth_rate ** d)
+                blocks = [tuple(w[f"enc.{b}.res.{i}.{d}.{n}"] for n in ("w1", "b1", "w2", "b2")) for d in range(cfg.depth)]
+                dilations = [cfg.dilation_growth_rate ** d for d in range(cfg.depth)]
+                if h.is_cuda:
+                    h = jb_resblocks(h, blocks, dilations)
+                else:
+                    for blk, dil in zip(blocks, dilations):
+                        h = ops.jb_resblock(h, *blk, dil)
             h = ops.jb_conv_k3(h, w[f"enc.{b}.proj.w"], w[f"enc.{b}.proj.b"])
         return h
 

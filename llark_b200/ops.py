@@ -344,6 +344,25 @@ def jb_resblock(x, w1, b1, w2, b2, dilation):
     return y
 
 
+def jb_resblocks(x, blocks, dilations):
+    """jb_resblock after jb_resblock: blocks = [(w1, b1, w2, b2), ...]; as many of them in one visit as fit."""
+    N, C, T = x.shape
+    at = 0
+    while at < len(blocks):
+        left = (ctypes.c_int * (len(blocks) - at))(*dilations[at:])
+        n = lib().llark_jb_resblocks_length(left, len(left))
+        if n == 0:  # not this one
+            x = jb_resblock(x, *blocks[at], dilations[at])
+            at += 1
+            continue
+        w = (ctypes.c_void_p * (4 * n))(*[_p(t) for b in blocks[at:at + n] for t in b])
+        y = torch.empty_like(x)
+        check(lib().llark_jb_resblocks(_p(x), w, left, n, _p(y), N, T, _stream()), "jb_resblocks")
+        x = y
+        at += n
+    return x
+
+
 def jb_conv_k3(x, w, b):
     N, c_in, T = x.shape
     c_out = w.shape[0]

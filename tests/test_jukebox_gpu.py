@@ -243,6 +243,32 @@ def test_convolutions_at_the_edges_of_their_tiles_match_fp64(kind, c_in, T):
     assert _rel(got.cpu(), ref) < 1e-6
 
 
+@pytest.mark.parametrize("T", [2, 431, 432, 433, 1000])
+@pytest.mark.parametrize("dils", [(1, 3, 9, 27), (27, 9, 3, 1), (32, 32, 32), (2, 5), (1, 3, 9, 27, 81), (40, 1, 1)])
+def test_res_blocks_in_one_visit_match_fp64(dils, T):
+    """Runs of res blocks against fp64 conv1d block after block: shorter than a window's results, one step more, windows that begin and
+    end at the clip's ends, runs whose last block goes alone. Split operands keep 24 bits: 1e-6 of the result, as block by block."""
+    import torch.nn.functional as F
+
+    from llark_b200 import ops
+
+    g = torch.Generator().manual_seed(T + len(dils))
+    x = torch.randn(3, 32, T, generator=g)
+    blocks, ref = [], x.double()
+    for d in dils:
+        w1, b1 = torch.randn(32, 32, 3, generator=g) / math.sqrt(96), torch.randn(32, generator=g) * 0.1
+        w2, b2 = torch.randn(32, 32, 1, generator=g) / math.sqrt(32), torch.randn(32, generator=g) * 0.1
+        blocks.append((w1.cuda(), b1.cuda(), w2.cuda(), b2.cuda()))
+        h = F.conv1d(F.relu(ref), w1.double(), b1.double(), padding=d, dilation=d)
+        ref = ref + F.conv1d(F.relu(h), w2.double(), b2.double())
+    got = ops.jb_resblocks(x.cuda(), blocks, dils)
+    one = x.cuda()
+    for b, d in zip(blocks, dils):
+        one = ops.jb_resblock(one, *b, d)
+    assert _rel(got.cpu(), ref) < 1e-6
+    assert _rel(got.cpu(), ref) < 1.2 * _rel(one.cpu(), ref) + 1e-8
+
+
 def _by_fma(fn, *args):
     """fn with the FMA kernels of the encoder's convolutions."""
     os.environ["LLARK_JB_CONV_TC"] = "0"
