@@ -22,7 +22,9 @@ int down(const float* x, const float* w, const float* b, float* y, int N, int c_
 bool takes_k3(int c_in, int c_out);
 int k3(const float* x, const float* w, const float* b, float* y, int N, int T, cudaStream_t st);
 }  // namespace jbconv
-
+namespace jbvq {  // jb_vq_tc.cu
+int encode(const float* x, const float* cb, long long* codes, int N, int T, int n_codes, cudaStream_t st);
+}
 
 extern thread_local int g_last_cuda_error;
 static inline int jb_check() {
@@ -226,98 +228,6 @@ conv_k3_kernel(const float* __restrict__ x, const float* __restrict__ w, const f
 #pragma unroll
             for (int c = 0; c < Tile::CPT; ++c) y[((long long)n * COUT + cg * Tile::CPT + c) * T + t] = acc[k][c];
         }
-    }
-}
-
-// ---------------------------------------------------------------------------------------------- VQ nearest code
-// dist = (|x|^2 - 2 x.k) + |k|^2 in fp32, every sum in the order of the channels; first minimum wins. A lane holds two vectors (all 64
-// channels in registers), the eight warps of a CTA share 64 vectors and take an eighth of the codes each, streamed through shared
-// memory (one broadcast read of four channels feeds eight FMAs); the warps' best are merged in the codes' order. FMA-bound: 32768
-// vectors x 2048 codes 436 us; 587 with a thread per vector walking all codes (one warp per scheduler), 465 with two codes at a time.
-constexpr int VQ_E = 64, VQ_CHUNK = 16, VQ_W = 8;
-__global__ void __launch_bounds__(VQ_W * 32)
-vq_encode_kernel(const float* __restrict__ x, const float* __restrict__ cb, long long* __restrict__ codes, int T,
-                 int n_codes) {
-    __shared__ __align__(16) float scb[VQ_W][VQ_CHUNK][VQ_E];
-    __shared__ float skk[VQ_W][VQ_CHUNK];
-    const int n = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t0 = blockIdx.x * 64 + lane;  // this lane's vectors: t0 and t0 + 32
-    float xv[2][VQ_E], xx[2] = {0.f, 0.f};
-#pragma unroll
-    for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int e = 0; e < VQ_E; ++e) {
-            const int t = t0 + 32 * u;
-            xv[u][e] = t < T ? x[((long long)n * VQ_E + e) * T + t] : 0.f;
-            xx[u] = fmaf(xv[u][e], xv[u][e], xx[u]);
-        }
-    const int per = (n_codes + VQ_W - 1) / VQ_W, lo = warp * per, hi = lo + per < n_codes ? lo + per : n_codes;
-    const bool vec = (reinterpret_cast<uintptr_t>(cb) & 15) == 0;
-    float best[2] = {INFINITY, INFINITY};
-    int best_j[2] = {0, 0};
-    for (int c0 = lo; c0 < hi; c0 += VQ_CHUNK) {  // each warp its own codes: no barrier of the block
-        const int lim = hi - c0 < VQ_CHUNK ? hi - c0 : VQ_CHUNK;
-        __syncwarp();
-        if (vec)
-            for (int i = lane; i < lim * (VQ_E / 4); i += 32)
-                reinterpret_cast<float4*>(&scb[warp][0][0])[i] = reinterpret_cast<const float4*>(cb + (long long)c0 * VQ_E)[i];
-        else
-            for (int i = lane; i < lim * VQ_E; i += 32) (&scb[warp][0][0])[i] = cb[(long long)c0 * VQ_E + i];
-        __syncwarp();
-        if (lane < lim) {
-            float kk = 0.f;
-#pragma unroll
-            for (int e0 = 0; e0 < VQ_E; e0 += 4) {
-                const float4 k = *reinterpret_cast<const float4*>(&scb[warp][lane][e0]);
-                kk = fmaf(k.x, k.x, kk);
-                kk = fmaf(k.y, k.y, kk);
-                kk = fmaf(k.z, k.z, kk);
-                kk = fmaf(k.w, k.w, kk);
-            }
-            skk[warp][lane] = kk;
-        }
-        __syncwarp();
-        for (int j = 0; j < lim; ++j) {
-            float dot[2] = {0.f, 0.f};
-#pragma unroll
-            for (int e0 = 0; e0 < VQ_E; e0 += 4) {
-                const float4 k = *reinterpret_cast<const float4*>(&scb[warp][j][e0]);
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    dot[u] = fmaf(xv[u][e0], k.x, dot[u]);
-                    dot[u] = fmaf(xv[u][e0 + 1], k.y, dot[u]);
-                    dot[u] = fmaf(xv[u][e0 + 2], k.z, dot[u]);
-                    dot[u] = fmaf(xv[u][e0 + 3], k.w, dot[u]);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const float dist = (xx[u] - 2.f * dot[u]) + skk[warp][j];
-                if (dist < best[u]) {
-                    best[u] = dist;
-                    best_j[u] = c0 + j;
-                }
-            }
-        }
-    }
-    __syncthreads();  // the codes are no longer read: their place takes the warps' best
-    float* sd = &scb[0][0][0];
-    int* sj = reinterpret_cast<int*>(sd + VQ_W * 64);
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-        sd[warp * 64 + 32 * u + lane] = best[u];
-        sj[warp * 64 + 32 * u + lane] = best_j[u];
-    }
-    __syncthreads();
-    if (threadIdx.x < 64 && blockIdx.x * 64 + threadIdx.x < T) {
-        float d = sd[threadIdx.x];
-        int bj = sj[threadIdx.x];
-        for (int w = 1; w < VQ_W; ++w)  // later codes win only when they are nearer
-            if (sd[w * 64 + threadIdx.x] < d) {
-                d = sd[w * 64 + threadIdx.x];
-                bj = sj[w * 64 + threadIdx.x];
-            }
-        codes[(long long)n * T + blockIdx.x * 64 + threadIdx.x] = bj;
     }
 }
 
@@ -829,9 +739,7 @@ extern "C" int llark_jb_conv_k3(const float* x, const float* w, const float* bia
 extern "C" int llark_jb_vq_encode(const float* x, const float* codebook, long long* codes, int N, int T, int n_codes,
                                   cudaStream_t st) {
     if (N <= 0 || T <= 0 || n_codes <= 0) return LLARK_EINVAL;
-    dim3 grid((T + 63) / 64, N);
-    vq_encode_kernel<<<grid, VQ_W * 32, 0, st>>>(x, codebook, codes, T, n_codes);
-    return jb_check();
+    return jbvq::encode(x, codebook, codes, N, T, n_codes, st);
 }
 
 extern "C" int llark_layernorm_fwd(const float* x, const float* gamma, const float* beta, void* y, int y_bf16,

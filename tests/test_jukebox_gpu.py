@@ -327,6 +327,47 @@ def test_a_nan_sample_stays_nan_through_the_encoder():
     assert torch.equal(got.isnan(), want.isnan())
 
 
+@pytest.mark.parametrize("T,n_codes", [(1, 1), (129, 256), (130, 257), (300, 2048), (128, 1000)])
+@pytest.mark.parametrize("kind", ["spread", "crowded", "equal", "not finite"])
+def test_nearest_code_is_that_of_the_walk_over_all_codes(T, n_codes, kind):
+    """The candidates that tensor cores leave against fp32 walks over all codes, FMA after FMA in the order of the channels (restated in
+    64 bits, rounded to fp32 after every step; where that rounds twice the two nearest may change places, which 64 bits then show):
+    codes far apart, codes closer together than bf16 tells them apart (lists overflow), equal codes, numbers that are not finite."""
+    from llark_b200 import ops
+
+    g = torch.Generator().manual_seed(T + n_codes)
+    x, cb = torch.randn(2, 64, T, generator=g), torch.randn(n_codes, 64, generator=g)
+    if kind == "crowded":
+        cb = cb[:1] + 1e-3 * cb
+    if kind == "equal":
+        cb = cb[torch.arange(n_codes) % 3 if n_codes >= 3 else torch.zeros(n_codes, dtype=torch.long)]
+    if kind == "not finite":
+        cb[n_codes // 2, 3] = float("inf")
+        cb[n_codes // 3, 5] = float("nan")
+        cb[n_codes // 4] = 1e25  # |k|^2 overflows
+        x[0, 1, 0], x[1, 2, T - 1], x[1, 0, T // 2] = float("nan"), float("inf"), 1e25
+    codes = ops.jb_vq_encode(x.cuda(), cb.cuda()).cpu()
+    flat = x.permute(0, 2, 1).reshape(-1, 64)
+
+    def fma(a, b, c):
+        return (a.double() * b.double() + c.double()).float()
+
+    xx, dot, kk = torch.zeros(len(flat)), torch.zeros(len(flat), n_codes), torch.zeros(n_codes)
+    for e in range(64):
+        xx, kk = fma(flat[:, e], flat[:, e], xx), fma(cb[:, e], cb[:, e], kk)
+        dot = fma(flat[:, e, None], cb[None, :, e], dot)
+    dist = (xx[:, None] - 2 * dot) + kk[None]
+    dist = torch.where(dist < float("inf"), dist, torch.full_like(dist, float("inf")))
+    best, want = dist.min(1).values, (dist == dist.min(1).values[:, None]).int().argmax(1)
+    got = codes.view(-1)
+    same = (got == want) | (best == float("inf")) & (got == 0)
+    if kind in ("equal", "not finite"):
+        assert same.all()
+    else:  # an ulp of a rounding done twice
+        off = dist.gather(1, got[:, None])[:, 0] - best
+        assert (same | (off <= 2.0 ** -20 * (xx + kk.max()))).all() and same.float().mean() > 0.9
+
+
 @pytest.mark.parametrize("T,n_codes", [(1, 5), (64, 2048), (65, 2047), (200, 37)])
 def test_nearest_code_in_every_slice_of_the_codebook(T, n_codes):
     """Codes are shared out over eight warps: the same fp32 distances as one walk over all of them, the first minimum wins."""
