@@ -408,29 +408,38 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const unsigned ch
 
 
 // =====================================================================================================================
-// BACKWARD on tcgen05. Two kernels with the forward kernel's structure and exactly its two MMA forms
-//   "KK": D[128 x 64]  = A[128 rows, K-major, d in 2 chunks] . B[64 rows, K-major]^T            (8 x K16)
-//   "PV": D[128 x 128] += A[128 rows x 64, K-major, written by threads] . B[64 K-rows x 128, MN-major]  (4 x K16)
+// BACKWARD on tcgen05. Two kernels with two MMA forms
+//   "KK": D[128 x N]    = A[128 rows, K-major, d in 2 chunks] . B[N rows, K-major]^T  (8 x K16)
+//   "PV": D[128 x 128] += A[128 rows x 64, written by threads] . B[64 K-rows x 128, MN-major]  (4 x K16)
 // so no operand is ever transposed in memory:
-//   dQ kernel   (CTA = 128 queries, streams 64-key tiles):  S = Q K^T, dP = dO V^T (KK); dS = P o (dP - D);
-//                                                           dQ += dS K (PV, K_j read MN-major)
-//   dK/dV kernel (CTA = 128 keys, streams 64-query tiles):  S^T = K Q^T, dP^T = V dO^T (KK); P^T, dS^T;
-//                                                           dV += P^T dO, dK += dS^T Q (PV, dO_i / Q_i read MN-major)
+//   dQ kernel    (CTA = 128 queries, streams 128-key tiles):  S = Q K^T, dP = dO V^T (KK); dS = P o (dP - D);
+//                                                             dQ += dS K (PV, dS in TMEM, K_j read MN-major)
+//   dK/dV kernel (CTA = 128 keys, streams 64-query tiles):    S^T = K Q^T, dP^T = V dO^T (KK); P^T, dS^T;
+//                                                             dV += P^T dO, dK += dS^T Q (PV, dO_i / Q_i read MN-major)
 // P is recomputed from the saved LSE (p = exp2(s*scale*log2e - lse*log2e)), D = rowsum(dO o O) comes from
-// attn_bwd_prep_kernel (attention.cu). 320 threads: warp 0 = TMA producer, warp 1 = TMEM allocator + MMA issuer,
-// warps 2-9 = two compute warpgroups that split the 64 columns of every S / dP row (no row reductions are needed in
-// the backward pass, so the split is free). S and dP are double-buffered in TMEM: the KK MMAs of tile t+1 run while
-// the compute warps work on tile t. One CTA per SM (145-162 KB of shared memory, all 512 TMEM columns).
-constexpr int kBwdThreads = 320;
-constexpr int RING_SLOTS = 6;   // three streamed tiles in flight: with 4 the load of tile j+2 could only be requested after
+// attn_bwd_prep_kernel (attention.cu). 608 threads, one CTA per SM: warp 0 = TMA producer, warp 1 = TMEM allocator + issuer of the KK
+// MMAs, warps 2-17 compute (no row reductions are needed in the backward pass, so the columns of a row are split freely), warp 18
+// = issuer of the PV MMAs.
+//
+// What bounds it: in the dQ kernel the MMAs, some 2050 cycles a tile of 128 keys (an MMA of 128 rows takes 54 to 84 cycles at N = 64 and
+// 72 at 128, and 300 more after the tensor pipe ran dry), and 5000 cycles a CTA before its first and after its last; in the dK/dV kernel
+// shared memory, which its A operands, P^T and dS^T pass through (TMEM is full). Measured on a B200, 4 x 32 heads x 2048 tokens, us:
+// dQ 352 -> 228, dK/dV 442 -> 364. Of the dQ kernel's, tiles of 128 with every load a tile ahead 283 (with four slots, where the load of K_j+2
+// waits for tile j's last MMA, 352 as before), two issuers 245, sixteen compute warps 241; of the dK/dV kernel's, two issuers 434, sixteen
+// compute warps that take tiles in turn 405; the rest by first loads that do not wait for TMEM and results that leave through TMA.
+constexpr int kBwdThreads = 64 + 512 + 32;
+constexpr int RING_SLOTS = 6;   // dK/dV: three streamed tiles in flight: with 4 the load of tile j+2 could only be requested after
                                 // tile j's last MMA retired, and its latency sat on the critical path of every tile
+constexpr int K_SLOTS = 3, V_SLOTS = 2;  // dQ: the same; V_j is done with one step before K_j
+constexpr int TILE_BYTES = BQ * HD * 2;  // 128 streamed rows: 32 KB
 __device__ __forceinline__ int ring_slot(int it) { return it % RING_SLOTS; }
 __device__ __forceinline__ uint32_t ring_phase(int it) { return (uint32_t)(it / RING_SLOTS) & 1u; }
 
-__device__ __forceinline__ void mma_kk_128x64(uint32_t tD, uint32_t a_addr, uint32_t a_chunk_bytes, uint32_t b_addr,
-                                              uint32_t b_chunk_bytes, uint32_t idesc) {
-    const uint64_t a0 = make_desc(a_addr, 0, 1024), a1 = make_desc(a_addr + a_chunk_bytes, 0, 1024);
-    const uint64_t b0 = make_desc(b_addr, 0, 1024), b1 = make_desc(b_addr + b_chunk_bytes, 0, 1024);
+// N: 64 or 128 rows of B in two chunks of N * 128 bytes
+template <int N>
+__device__ __forceinline__ void mma_kk(uint32_t tD, uint32_t a_addr, uint32_t b_addr, uint32_t idesc) {
+    const uint64_t a0 = make_desc(a_addr, 0, 1024), a1 = make_desc(a_addr + BQ * 128, 0, 1024);
+    const uint64_t b0 = make_desc(b_addr, 0, 1024), b1 = make_desc(b_addr + N * 128, 0, 1024);
 #pragma unroll
     for (int k = 0; k < 8; ++k)
         umma_f16(tD, (k < 4 ? a0 : a1) + (uint64_t)((k & 3) * 2), (k < 4 ? b0 : b1) + (uint64_t)((k & 3) * 2), idesc,
@@ -444,7 +453,47 @@ __device__ __forceinline__ void mma_pv_128x128(uint32_t tD, uint32_t a_addr, uin
     for (int k = 0; k < 4; ++k)
         umma_f16(tD, ad + (uint64_t)(k * 2), bd + (uint64_t)(k * 128), idesc, accumulate || k != 0);
 }
-__device__ __forceinline__ void compute_group_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+// the same with A (bf16, two columns of K in one) in TMEM; b_addr: 64 of the rows of a 128-row tile
+__device__ __forceinline__ void mma_pv_tmem(uint32_t tD, uint32_t tA, uint32_t b_addr, uint32_t idesc, bool accumulate) {
+    const uint64_t bd = make_desc(b_addr, BQ * 128, 1024);  // MN-major: the two 64-wide N chunks are 16 KB apart
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        asm volatile(
+            "{\n"
+            ".reg .pred p;\n"
+            "setp.ne.b32 p, %4, 0;\n"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+            "}\n" ::"r"(tD),
+            "r"(tA + 8 * k), "l"(bd + (uint64_t)(k * 128)), "r"(idesc), "r"((uint32_t)(accumulate || k != 0))
+            : "memory");
+}
+// a 128-row tile of 128 columns: two column chunks of 128 bytes, boxes of 64 rows
+__device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int col, int row) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int rh = 0; rh < 2; ++rh) tma_load_2d(dst + c * (BQ * 128) + rh * (64 * 128), tm, bar, col + c * 64, row + rh * 64);
+}
+__device__ __forceinline__ void store_tile(const uint8_t* src, const CUtensorMap* tm, int col, int row) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int rh = 0; rh < 2; ++rh) tma_store_2d(tm, src + c * (BQ * 128) + rh * (64 * 128), col + c * 64, row + rh * 64);
+}
+// 32 fp32 values -> 32 bf16 -> 16 columns of this thread's TMEM lane
+__device__ __forceinline__ void tmem_st_bf16(uint32_t taddr, const float (&v)[32]) {
+    uint32_t u[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) u[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+        "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]), "r"(u[8]), "r"(u[9]), "r"(u[10]),
+        "r"(u[11]), "r"(u[12]), "r"(u[13]), "r"(u[14]), "r"(u[15])
+        : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
+__device__ __forceinline__ void compute_sync(int half) { asm volatile("bar.sync %0, 256;" ::"r"(2 + half) : "memory"); }  // eight warps
 // bits 0 .. n - 1
 __device__ __forceinline__ uint32_t first_columns(int n) { return n >= 32 ? 0xffffffffu : n <= 0 ? 0u : (1u << n) - 1u; }
 // The exponents of columns that are not seen become -inf, so that ex2 gives 0: a select per column, where a condition around ex2 was a
@@ -466,10 +515,18 @@ __device__ __forceinline__ void store_half_row(uint8_t* tile, int r, int g, cons
         *reinterpret_cast<uint4*>(row + (((g * 4 + u) ^ (r & 7)) << 4)) = w;
     }
 }
-// 64 fp32 accumulator columns of this thread's TMEM lane -> scaled bf16 -> 128 contiguous bytes in global memory
-__device__ __forceinline__ void store_acc_64(uint32_t taddr, __nv_bfloat16* dst, float mul, bool ok) {
+// Where the 16-byte units of a thread's 64 bf16 results go: 128 contiguous bytes in global memory, or (sw >= 0: the row % 8) a row of a
+// 128-byte-swizzled tile in shared memory, which TMA takes to global memory: 16 bytes of 32 rows at a time, written from
+// registers, took 2000 cycles a CTA.
+struct RowOut {
+    void* row;
+    int sw;
+    __device__ __forceinline__ uint4* unit(int u) const { return reinterpret_cast<uint4*>(row) + (sw >= 0 ? u ^ sw : u); }
+};
+// 64 fp32 accumulator columns of this thread's TMEM lane -> scaled bf16 (those 32 of them from c_lo to c_hi)
+__device__ __forceinline__ void store_acc_64(uint32_t taddr, RowOut dst, float mul, bool ok, int c_lo = 0, int c_hi = 2) {
 #pragma unroll 1
-    for (int c = 0; c < 2; ++c) {
+    for (int c = c_lo; c < c_hi; ++c) {
         uint32_t ov[32];
         tmem_ld_32x32b_x32(taddr + c * 32, ov);
         tmem_ld_wait();
@@ -481,7 +538,7 @@ __device__ __forceinline__ void store_acc_64(uint32_t taddr, __nv_bfloat16* dst,
                 o.y = pack_bf16x2(__uint_as_float(ov[8 * u + 2]) * mul, __uint_as_float(ov[8 * u + 3]) * mul);
                 o.z = pack_bf16x2(__uint_as_float(ov[8 * u + 4]) * mul, __uint_as_float(ov[8 * u + 5]) * mul);
                 o.w = pack_bf16x2(__uint_as_float(ov[8 * u + 6]) * mul, __uint_as_float(ov[8 * u + 7]) * mul);
-                *reinterpret_cast<uint4*>(dst + c * 32 + u * 8) = o;
+                *dst.unit(c * 4 + u) = o;
             }
         }
     }
@@ -495,10 +552,10 @@ __device__ __forceinline__ void store_acc_64(uint32_t taddr, __nv_bfloat16* dst,
 //   half 1:  o[d + 64] = bf16(x[d + 64] * cos[d + 64]) + bf16(-x[d] * sin[d])        with x = bf16(acc * mul),
 // the rounding points of rope_kernel (llama_ops.cu) on the bf16 values the unfused path would have stored: bit-identical.
 // cs / sn: this row's 128 cos / sin values (bf16, position = row % S).
-__device__ __forceinline__ void store_acc_64_irope(uint32_t taddr_row, int g, __nv_bfloat16* dst, float mul, bool ok,
-                                                   const __nv_bfloat16* cs, const __nv_bfloat16* sn) {
+__device__ __forceinline__ void store_acc_64_irope(uint32_t taddr_row, int g, RowOut dst, float mul, bool ok,
+                                                   const __nv_bfloat16* cs, const __nv_bfloat16* sn, int c_lo = 0, int c_hi = 2) {
 #pragma unroll 1
-    for (int c = 0; c < 2; ++c) {
+    for (int c = c_lo; c < c_hi; ++c) {
         uint32_t own[32], oth[32];
         tmem_ld_32x32b_x32(taddr_row + g * 64 + c * 32, own);
         tmem_ld_32x32b_x32(taddr_row + (1 - g) * 64 + c * 32, oth);
@@ -526,7 +583,7 @@ __device__ __forceinline__ void store_acc_64_irope(uint32_t taddr_row, int g, __
                     }
                     ow[e2] = pack_bf16x2(r[0], r[1]);
                 }
-                *reinterpret_cast<uint4*>(dst + d0 + u * 8) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+                *dst.unit(c * 4 + u) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
             }
         }
     }
@@ -535,13 +592,13 @@ __device__ __forceinline__ void store_acc_64_irope(uint32_t taddr_row, int g, __
 // ---------------------------------------------------------------------------------------------------- dQ
 constexpr int DQ_OFF_DO = Q_BYTES;
 constexpr int DQ_OFF_RING = 2 * Q_BYTES;
-constexpr int DQ_OFF_DS = DQ_OFF_RING + RING_SLOTS * KV_BYTES;
-constexpr int DQ_OFF_BAR = DQ_OFF_DS + 2 * P_BYTES;  // dS is double-buffered
+constexpr int DQ_OFF_BAR = DQ_OFF_RING + (K_SLOTS + V_SLOTS) * TILE_BYTES;
 constexpr int DQ_OFF_MASK = DQ_OFF_BAR + 256;
 constexpr int DQ_SMEM_BYTES = DQ_OFF_MASK + (MAX_S / 32) * 4 + 1024;
 
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
+                      const __grid_constant__ CUtensorMap tm_out,
                       const unsigned char* __restrict__ mask, const float* __restrict__ lse,
                       const float* __restrict__ Dsum, __nv_bfloat16* __restrict__ dqkv, int S, int NH, float scale,
                       float scale_log2, const __nv_bfloat16* __restrict__ rope_cos,
@@ -550,17 +607,20 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sQ = smem;
     uint8_t* sdO = smem + DQ_OFF_DO;
-    uint8_t* sRing = smem + DQ_OFF_RING;
-    uint8_t* sdS = smem + DQ_OFF_DS;
+    uint8_t* sKt = smem + DQ_OFF_RING;
+    uint8_t* sVt = sKt + K_SLOTS * TILE_BYTES;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + DQ_OFF_BAR);
     uint64_t* q_full = bars;                       // [1]  Q and dO tiles landed
-    uint64_t* ring_full = bars + 1;                // [RING_SLOTS]
-    uint64_t* ring_empty = ring_full + RING_SLOTS; // [RING_SLOTS]
-    uint64_t* sdp_full = ring_empty + RING_SLOTS;  // [2]  S and dP of tile j are in TMEM
-    uint64_t* sdp_empty = sdp_full + 2;            // [2]  8 compute warps have read them
-    uint64_t* ds_full = sdp_empty + 2;             // [2]  dS tile j written to shared-memory buffer j & 1
-    uint64_t* dq_done = ds_full + 2;               // [2]  dQ += dS_j K_j retired (buffer j & 1 free again)
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(dq_done + 2);
+    uint64_t* k_full = bars + 1;                   // [K_SLOTS]
+    uint64_t* k_empty = k_full + K_SLOTS;          // [K_SLOTS]
+    uint64_t* v_full = k_empty + K_SLOTS;          // [V_SLOTS]
+    uint64_t* v_empty = v_full + V_SLOTS;          // [V_SLOTS]
+    uint64_t* sdp_full = v_empty + V_SLOTS;        // [1]  S and dP of tile j are in TMEM
+    uint64_t* sdp_empty = sdp_full + 1;            // [1]  the compute warps have read them
+    uint64_t* ds_full = sdp_empty + 1;             // [2]  half h of dS of tile j is in TMEM
+    uint64_t* dq_done = ds_full + 2;               // [2]  dQ += dS_j K_j of half h retired (its columns are free again)
+    uint64_t* dq_all = dq_done + 2;                // [1]  every MMA retired
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(dq_all + 1);
     uint32_t* maskw = reinterpret_cast<uint32_t*>(smem + DQ_OFF_MASK);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -568,26 +628,27 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
     const int h = blockIdx.y, b = blockIdx.z;
     const int q0 = qt * BQ;
     const int n_key_tiles = (S + BK - 1) / BK;
-    const int n_kv = min(n_key_tiles, (q0 + BQ) / BK);
+    const int n_half = min(n_key_tiles, (q0 + BQ) / BK);  // halves of 64 keys in all
+    const int n_kv = (n_half + 1) / 2;
 
     if (warp == 0 && lane == 0) {
         tma_prefetch_desc(&tm_qkv);
         tma_prefetch_desc(&tm_do);
         mbar_init(q_full, 1);
-        for (int i = 0; i < RING_SLOTS; ++i) {
-            mbar_init(&ring_full[i], 1);
-            mbar_init(&ring_empty[i], 1);
-        }
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(&sdp_full[i], 1);
-            mbar_init(&sdp_empty[i], 8);
-        }
+        for (int i = 0; i < 2 * (K_SLOTS + V_SLOTS); ++i) mbar_init(&k_full[i], 1);
+        mbar_init(sdp_full, 1);
+        mbar_init(sdp_empty, 16);
         for (int i = 0; i < 2; ++i) {
             mbar_init(&ds_full[i], 8);
             mbar_init(&dq_done[i], 1);
         }
+        mbar_init(dq_all, 1);
         mbar_fence_init();
         fence_proxy_async_smem();
+        // on their way while TMEM is allocated
+        mbar_arrive_expect_tx(q_full, 2 * Q_BYTES);
+        load_tile(sQ, &tm_qkv, q_full, h * HD, b * S + q0);
+        load_tile(sdO, &tm_do, q_full, h * HD, b * S + q0);
     }
     if (warp == 1) {
         tmem_alloc(tmem_slot, 512);
@@ -596,81 +657,73 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;  // S[2] @ 0,64   dP[2] @ 128,192   dQ @ 256..383
+    const uint32_t tmem_base = *tmem_slot;  // S @ 0   dP @ 128   dQ @ 256   dS (bf16) @ 384, 416
 
     if (warp == 0) {
         if (lane == 0) {
             const int row0 = b * S;
-            const int cq = h * HD, ck = NH * HD + h * HD, cv = 2 * NH * HD + h * HD;
-            mbar_arrive_expect_tx(q_full, 2 * Q_BYTES);
-            for (int c = 0; c < 2; ++c)
-                for (int rh = 0; rh < 2; ++rh) {
-                    tma_load_2d(sQ + c * (BQ * 128) + rh * (64 * 128), &tm_qkv, q_full, cq + c * 64, row0 + q0 + rh * 64);
-                    tma_load_2d(sdO + c * (BQ * 128) + rh * (64 * 128), &tm_do, q_full, cq + c * 64, row0 + q0 + rh * 64);
-                }
+            const int ck = NH * HD + h * HD, cv = 2 * NH * HD + h * HD;
             for (int j = 0; j < n_kv; ++j) {
-#pragma unroll
-                for (int kv = 0; kv < 2; ++kv) {
-                    const int it = 2 * j + kv, slot = ring_slot(it);
-                    mbar_wait(&ring_empty[slot], ring_phase(it) ^ 1);
-                    uint8_t* dst = sRing + slot * KV_BYTES;
-                    mbar_arrive_expect_tx(&ring_full[slot], KV_BYTES);
-                    const int col = kv ? cv : ck;
-                    tma_load_2d(dst, &tm_qkv, &ring_full[slot], col, row0 + j * BK);
-                    tma_load_2d(dst + BK * 128, &tm_qkv, &ring_full[slot], col + 64, row0 + j * BK);
-                }
+                const int ks = j % K_SLOTS, vs = j % V_SLOTS;
+                mbar_wait(&k_empty[ks], ((uint32_t)(j / K_SLOTS) & 1) ^ 1);
+                mbar_arrive_expect_tx(&k_full[ks], TILE_BYTES);
+                load_tile(sKt + ks * TILE_BYTES, &tm_qkv, &k_full[ks], ck, row0 + j * BQ);
+                mbar_wait(&v_empty[vs], ((uint32_t)(j / V_SLOTS) & 1) ^ 1);
+                mbar_arrive_expect_tx(&v_full[vs], TILE_BYTES);
+                load_tile(sVt + vs * TILE_BYTES, &tm_qkv, &v_full[vs], cv, row0 + j * BQ);
             }
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            const uint32_t idesc_kk = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BK >> 3) << 17) |
+            const uint32_t idesc_kk = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BQ >> 3) << 17) |
                                       ((uint32_t)(BQ >> 4) << 24);
+            mbar_wait(q_full, 0);
+            for (int j = 0; j < n_kv; ++j) {
+                const int ks = j % K_SLOTS, vs = j % V_SLOTS;
+                mbar_wait(sdp_empty, ((uint32_t)j & 1) ^ 1);
+                mbar_wait(&k_full[ks], (uint32_t)(j / K_SLOTS) & 1);
+                tc_fence_after();
+                mma_kk<BQ>(tmem_base, smem_u32(sQ), smem_u32(sKt + ks * TILE_BYTES), idesc_kk);
+                mbar_wait(&v_full[vs], (uint32_t)(j / V_SLOTS) & 1);
+                tc_fence_after();
+                mma_kk<BQ>(tmem_base + 128, smem_u32(sdO), smem_u32(sVt + vs * TILE_BYTES), idesc_kk);
+                umma_commit(&v_empty[vs]);  // V_j is not needed again
+                umma_commit(sdp_full);
+            }
+        }
+    } else if (warp == kBwdThreads / 32 - 1) {
+        if (lane == 0) {  // a warp of its own: the tensor pipe has one kind of products while the other's operands are waited for
             const uint32_t idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) |
                                       ((uint32_t)(BQ >> 4) << 24);
-            auto issue_sdp = [&](int j) {
-                const int sb = j & 1;
-                const int itk = 2 * j, itv = 2 * j + 1;
-                mbar_wait(&sdp_empty[sb], ((uint32_t)(j >> 1) & 1) ^ 1);
-                mbar_wait(&ring_full[ring_slot(itk)], ring_phase(itk));
-                tc_fence_after();
-                mma_kk_128x64(tmem_base + sb * BK, smem_u32(sQ), BQ * 128, smem_u32(sRing + ring_slot(itk) * KV_BYTES),
-                              BK * 128, idesc_kk);
-                mbar_wait(&ring_full[ring_slot(itv)], ring_phase(itv));
-                tc_fence_after();
-                mma_kk_128x64(tmem_base + 128 + sb * BK, smem_u32(sdO), BQ * 128,
-                              smem_u32(sRing + ring_slot(itv) * KV_BYTES), BK * 128, idesc_kk);
-                umma_commit(&ring_empty[ring_slot(itv)]);  // V_j is not needed again
-                umma_commit(&sdp_full[sb]);
-            };
-            mbar_wait(q_full, 0);
-            issue_sdp(0);
             for (int j = 0; j < n_kv; ++j) {
-                if (j + 1 < n_kv) issue_sdp(j + 1);
-                mbar_wait(&ds_full[j & 1], (uint32_t)(j >> 1) & 1);
-                tc_fence_after();
-                const int itk = 2 * j;
-                mma_pv_128x128(tmem_base + 256, smem_u32(sdS + (j & 1) * P_BYTES),
-                               smem_u32(sRing + ring_slot(itk) * KV_BYTES), idesc_pv, j != 0);
-                umma_commit(&ring_empty[ring_slot(itk)]);
-                umma_commit(&dq_done[j & 1]);
+                const int ks = j % K_SLOTS;
+                for (int hf = 0; hf < 2 && 2 * j + hf < n_half; ++hf) {
+                    mbar_wait(&ds_full[hf], (uint32_t)j & 1);
+                    tc_fence_after();
+                    mma_pv_tmem(tmem_base + 256, tmem_base + 384 + hf * 32, smem_u32(sKt + ks * TILE_BYTES + hf * (64 * 128)), idesc_pv,
+                                j + hf != 0);
+                    umma_commit(&dq_done[hf]);
+                }
+                umma_commit(&k_empty[ks]);
             }
+            umma_commit(dq_all);
         }
     } else {
         const int cw = warp - 2;
-        const int g = cw >> 2;       // column half of every S / dP row this warpgroup handles
+        const int hf = cw >> 3, g = (cw >> 2) & 1;  // this warpgroup has columns 64 hf + 32 g .. + 31 of every tile
         const int quad = warp & 3;
         const int r_in = quad * 32 + lane;
         const int qi = q0 + r_in;
         const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
         {
             const int nwords = n_key_tiles * 2;
-            for (int w = cw; w < nwords; w += 8) {
+            for (int w = cw; w < nwords; w += 16) {
                 const int key = w * 32 + lane;
                 const bool ok = key < S && (!mask || mask[(long long)b * S + key] != 0);
                 const uint32_t bits = __ballot_sync(0xffffffffu, ok);
                 if (lane == 0) maskw[w] = bits;
             }
-            compute_group_sync();
+            compute_sync();
         }
         const bool row_ok = qi < S;
         const float lse2 = row_ok ? lse[((long long)b * NH + h) * S + qi] * LOG2E : INFINITY;
@@ -679,19 +732,18 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
         const float slope2 = alibi_slopes[h] * LOG2E;
 #endif
         for (int j = 0; j < n_kv; ++j) {
-            const int sb = j & 1;
-            mbar_wait(&sdp_full[sb], (uint32_t)(j >> 1) & 1);
+            mbar_wait(sdp_full, (uint32_t)j & 1);
             tc_fence_after();
             uint32_t sv[32], dv[32];
-            tmem_ld_32x32b_x32(lane_base + sb * BK + g * 32, sv);
-            tmem_ld_32x32b_x32(lane_base + 128 + sb * BK + g * 32, dv);
+            tmem_ld_32x32b_x32(lane_base + hf * 64 + g * 32, sv);
+            tmem_ld_32x32b_x32(lane_base + 128 + hf * 64 + g * 32, dv);
             tmem_ld_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sdp_empty[sb]);
-
-            const int kbase = j * BK + g * 32;
-            const uint32_t mw = maskw[2 * j + g];
+            if (lane == 0) mbar_arrive(sdp_empty);
+            if (2 * j + hf >= n_half) break;  // past the last half
+            const int kbase = j * BQ + hf * 64 + g * 32;
+            const uint32_t mw = maskw[4 * j + 2 * hf + g];
             const bool plain = (kbase + 31 <= q0 + quad * 32) && mw == 0xffffffffu;  // warp-uniform
             float ds[32];
 #pragma unroll
@@ -704,24 +756,34 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
             if (!plain) mask_columns(ds, mw & first_columns(qi - kbase + 1));
 #pragma unroll
             for (int c = 0; c < 32; ++c) ds[c] = ex2(ds[c]) * (__uint_as_float(dv[c]) - dsum);
-            if (j >= 2) {
-                mbar_wait(&dq_done[j & 1], (uint32_t)((j >> 1) - 1) & 1);  // tile j-2 retired: buffer j & 1 is free
+            if (j > 0) {
+                mbar_wait(&dq_done[hf], (uint32_t)(j - 1) & 1);  // this half of tile j-1 retired: its columns are free
                 tc_fence_after();
             }
-            store_half_row(sdS + (j & 1) * P_BYTES, r_in, g, ds);
-            fence_proxy_async_smem();
+            tmem_st_bf16(lane_base + 384 + hf * 32 + g * 16, ds);
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&ds_full[j & 1]);
+            if (lane == 0) mbar_arrive(&ds_full[hf]);
         }
-        mbar_wait(&dq_done[(n_kv - 1) & 1], (uint32_t)((n_kv - 1) >> 1) & 1);  // MMAs retire in order
+        mbar_wait(dq_all, 0);  // a warp follows the phases of its own half only
         tc_fence_after();
-        __nv_bfloat16* dqp = dqkv + ((long long)b * S + qi) * (3LL * NH * HD) + (long long)h * HD + g * 64;
+        const bool whole = q0 + BQ <= S;  // a tile that ends at a sample's end must not write the next one's rows
+        RowOut out = {dqkv + ((long long)b * S + qi) * (3LL * NH * HD) + (long long)h * HD + g * 64, -1};
+        if (whole) out = {sQ + g * (BQ * 128) + r_in * 128, r_in & 7};  // Q has been read
         if (rope_cos)  // inverse RoPE of dq fused into the store (position = query index)
-            store_acc_64_irope(lane_base + 256, g, dqp, scale, row_ok, rope_cos + (long long)(row_ok ? qi : 0) * HD,
-                               rope_sin + (long long)(row_ok ? qi : 0) * HD);
+            store_acc_64_irope(lane_base + 256, g, out, scale, row_ok, rope_cos + (long long)(row_ok ? qi : 0) * HD,
+                               rope_sin + (long long)(row_ok ? qi : 0) * HD, hf, hf + 1);
         else
-            store_acc_64(lane_base + 256 + g * 64, dqp, scale, row_ok);
+            store_acc_64(lane_base + 256 + g * 64, out, scale, row_ok, hf, hf + 1);
+        if (whole) {
+            fence_proxy_async_smem();
+            compute_sync();
+            if (threadIdx.x == 64) {
+                store_tile(sQ, &tm_out, h * HD, b * S + q0);
+                tma_store_commit();
+                tma_store_wait_all();
+            }
+        }
         tc_fence_before();
     }
 
@@ -740,11 +802,13 @@ constexpr int KV_OFF_RING = 2 * Q_BYTES;          // Q_i / dO_i tiles of 64 quer
 constexpr int KV_OFF_PT = KV_OFF_RING + RING_SLOTS * KV_BYTES;
 constexpr int KV_OFF_DST = KV_OFF_PT + 2 * P_BYTES;   // P^T and dS^T are double-buffered
 constexpr int KV_OFF_BAR = KV_OFF_DST + 2 * P_BYTES;
-constexpr int KV_OFF_ROWV = KV_OFF_BAR + 256;     // float [2][2][64]: lse*log2e and D of the streamed queries
+constexpr int KV_OFF_ROWV = KV_OFF_BAR + 256;     // float [2][2][64]: lse*log2e and D of the queries of tile t, by t & 1
 constexpr int KV_SMEM_BYTES = KV_OFF_ROWV + 2 * 2 * 64 * 4 + 1024;
+static_assert(KV_SMEM_BYTES <= 232448 && DQ_SMEM_BYTES <= 232448, "shared memory of a CTA");
 
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
+                        const __grid_constant__ CUtensorMap tm_out,
                         const unsigned char* __restrict__ mask, const float* __restrict__ lse,
                         const float* __restrict__ Dsum, __nv_bfloat16* __restrict__ dqkv, int S, int NH, float scale,
                         float scale_log2, const __nv_bfloat16* __restrict__ rope_cos,
@@ -764,7 +828,8 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
     uint64_t* sdp_empty = sdp_full + 2;            // [2]
     uint64_t* pds_full = sdp_empty + 2;            // [2]  P^T and dS^T of tile t written to buffers t & 1
     uint64_t* pds_done = pds_full + 2;             // [2]  dV / dK MMAs of tile t retired (buffers t & 1 free)
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pds_done + 2);
+    uint64_t* kv_all = pds_done + 2;               // [1]  every MMA retired
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(kv_all + 1);
     float* rowv = reinterpret_cast<float*>(smem + KV_OFF_ROWV);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -791,8 +856,13 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
             mbar_init(&pds_full[i], 8);
             mbar_init(&pds_done[i], 1);
         }
+        mbar_init(kv_all, 1);
         mbar_fence_init();
         fence_proxy_async_smem();
+        // on their way while TMEM is allocated
+        mbar_arrive_expect_tx(kv_full, 2 * Q_BYTES);
+        load_tile(sK, &tm_qkv, kv_full, NH * HD + h * HD, b * S + k0);
+        load_tile(sV, &tm_qkv, kv_full, 2 * NH * HD + h * HD, b * S + k0);
     }
     if (warp == 1) {
         tmem_alloc(tmem_slot, 512);
@@ -806,13 +876,7 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
     if (warp == 0) {
         if (lane == 0) {
             const int row0 = b * S;
-            const int cq = h * HD, ck = NH * HD + h * HD, cv = 2 * NH * HD + h * HD;
-            mbar_arrive_expect_tx(kv_full, 2 * Q_BYTES);
-            for (int c = 0; c < 2; ++c)
-                for (int rh = 0; rh < 2; ++rh) {
-                    tma_load_2d(sK + c * (BQ * 128) + rh * (64 * 128), &tm_qkv, kv_full, ck + c * 64, row0 + k0 + rh * 64);
-                    tma_load_2d(sV + c * (BQ * 128) + rh * (64 * 128), &tm_qkv, kv_full, cv + c * 64, row0 + k0 + rh * 64);
-                }
+            const int cq = h * HD;
             for (int t = 0; t < n_it; ++t) {
                 const int qrow = row0 + (t0 + t) * BK;
 #pragma unroll
@@ -831,26 +895,25 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
         if (lane == 0) {
             const uint32_t idesc_kk = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BK >> 3) << 17) |
                                       ((uint32_t)(BQ >> 4) << 24);
-            const uint32_t idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) |
-                                      ((uint32_t)(BQ >> 4) << 24);
-            auto issue_sdp = [&](int t) {
+            mbar_wait(kv_full, 0);
+            for (int t = 0; t < n_it; ++t) {
                 const int sb = t & 1;
                 const int itq = 2 * t, itd = 2 * t + 1;
                 mbar_wait(&sdp_empty[sb], ((uint32_t)(t >> 1) & 1) ^ 1);
                 mbar_wait(&ring_full[ring_slot(itq)], ring_phase(itq));
                 tc_fence_after();
-                mma_kk_128x64(tmem_base + sb * BK, smem_u32(sK), BQ * 128, smem_u32(sRing + ring_slot(itq) * KV_BYTES),
-                              BK * 128, idesc_kk);
+                mma_kk<BK>(tmem_base + sb * BK, smem_u32(sK), smem_u32(sRing + ring_slot(itq) * KV_BYTES), idesc_kk);
                 mbar_wait(&ring_full[ring_slot(itd)], ring_phase(itd));
                 tc_fence_after();
-                mma_kk_128x64(tmem_base + 128 + sb * BK, smem_u32(sV), BQ * 128,
-                              smem_u32(sRing + ring_slot(itd) * KV_BYTES), BK * 128, idesc_kk);
+                mma_kk<BK>(tmem_base + 128 + sb * BK, smem_u32(sV), smem_u32(sRing + ring_slot(itd) * KV_BYTES), idesc_kk);
                 umma_commit(&sdp_full[sb]);
-            };
-            mbar_wait(kv_full, 0);
-            issue_sdp(0);
+            }
+        }
+    } else if (warp == kBwdThreads / 32 - 1) {
+        if (lane == 0) {
+            const uint32_t idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) |
+                                      ((uint32_t)(BQ >> 4) << 24);
             for (int t = 0; t < n_it; ++t) {
-                if (t + 1 < n_it) issue_sdp(t + 1);
                 mbar_wait(&pds_full[t & 1], (uint32_t)(t >> 1) & 1);
                 tc_fence_after();
                 const int itq = 2 * t, itd = 2 * t + 1;
@@ -862,14 +925,15 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
                 umma_commit(&ring_empty[ring_slot(itq)]);
                 umma_commit(&pds_done[t & 1]);
             }
+            umma_commit(kv_all);
         }
     } else {
         const int cw = warp - 2;
-        const int g = cw >> 2;
+        const int sb = cw >> 3, g = (cw >> 2) & 1;  // this warpgroup has columns 32 g .. + 31 of every tile t with t & 1 == sb
         const int quad = warp & 3;
         const int r_in = quad * 32 + lane;   // key row inside the tile == TMEM lane
         const int key = k0 + r_in;
-        const int ct = threadIdx.x - 64;     // 0..255 inside the compute group
+        const int ct = (threadIdx.x - 64) & 255;  // inside the eight warps of these tiles
         const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
         const bool kvalid = key < S && (!mask || mask[(long long)b * S + key] != 0);
         const bool all_valid = __all_sync(0xffffffffu, kvalid);
@@ -886,14 +950,14 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
             if (ct < 64) return q < S ? lse_bh[q] * LOG2E : INFINITY;  // +inf => p = 0 past the sequence end
             return q < S ? d_bh[q] : 0.f;
         };
-        float rowv_next = fetch_rowv(0);
-        for (int t = 0; t < n_it; ++t) {
-            const int sb = t & 1;
+        float* const rv = rowv + sb * 128;
+        float rowv_next = fetch_rowv(sb);
+        for (int t = sb; t < n_it; t += 2) {
             const int qb = (t0 + t) * BK;  // first query of the streamed tile
-            float* rv = rowv + sb * 128;
+            compute_sync(sb);  // tile t-2's values have been read
             if (ct < 128) rv[ct] = rowv_next;
-            rowv_next = fetch_rowv(t + 1);
-            compute_group_sync();  // also orders tile t-2's readers of this buffer before the writes above (see t-1)
+            rowv_next = fetch_rowv(t + 2);
+            compute_sync(sb);
             mbar_wait(&sdp_full[sb], (uint32_t)(t >> 1) & 1);
             tc_fence_after();
             uint32_t sv[32], dv[32];
@@ -941,17 +1005,30 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
             __syncwarp();
             if (lane == 0) mbar_arrive(&pds_full[t & 1]);
         }
-        mbar_wait(&pds_done[(n_it - 1) & 1], (uint32_t)((n_it - 1) >> 1) & 1);  // MMAs retire in order
+        mbar_wait(kv_all, 0);  // a warp follows the phases of its own tiles only
         tc_fence_after();
-        __nv_bfloat16* dkp = dqkv + ((long long)b * S + key) * (3LL * NH * HD) + (long long)NH * HD + (long long)h * HD +
-                             g * 64;
-        __nv_bfloat16* dvp = dkp + (long long)NH * HD;
-        store_acc_64(lane_base + 256 + g * 64, dvp, 1.f, key < S);
-        if (rope_cos)  // inverse RoPE of dk fused into the store (position = key index)
-            store_acc_64_irope(lane_base + 384, g, dkp, scale, key < S, rope_cos + (long long)(key < S ? key : 0) * HD,
+        // eight warps store dV, eight dK; through the K and V tiles, which have been read
+        const bool whole = k0 + BQ <= S;  // a tile that ends at a sample's end must not write the next one's rows
+        const int col = (sb == 0 ? 2 : 1) * NH * HD + h * HD;
+        uint8_t* const tile = sb == 0 ? sV : sK;
+        RowOut out = {dqkv + ((long long)b * S + key) * (3LL * NH * HD) + col + g * 64, -1};
+        if (whole) out = {tile + g * (BQ * 128) + r_in * 128, r_in & 7};
+        if (sb == 0)
+            store_acc_64(lane_base + 256 + g * 64, out, 1.f, key < S);
+        else if (rope_cos)  // inverse RoPE of dk fused into the store (position = key index)
+            store_acc_64_irope(lane_base + 384, g, out, scale, key < S, rope_cos + (long long)(key < S ? key : 0) * HD,
                                rope_sin + (long long)(key < S ? key : 0) * HD);
         else
-            store_acc_64(lane_base + 384 + g * 64, dkp, scale, key < S);
+            store_acc_64(lane_base + 384 + g * 64, out, scale, key < S);
+        if (whole) {
+            fence_proxy_async_smem();
+            compute_sync(sb);
+            if (ct == 0) {
+                store_tile(tile, &tm_out, col, b * S + k0);
+                tma_store_commit();
+                tma_store_wait_all();
+            }
+        }
         tc_fence_before();
     }
 
@@ -1009,6 +1086,9 @@ int LLARK_ATC_BWD_LAUNCH(const void* qkv, const unsigned char* key_mask, const v
     if (rc) return rc;
     rc = tensor_map_2d(&td, dout, ldo, (long long)B * S, ldo, 64, 64, 2);
     if (rc) return rc;
+    CUtensorMap to;
+    rc = tensor_map_2d(&to, dqkv, ld, (long long)B * S, ld, 64, 64, 2);
+    if (rc) return rc;
     static bool attr_set = false;
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(attn_bwd_dq_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1022,11 +1102,11 @@ int LLARK_ATC_BWD_LAUNCH(const void* qkv, const unsigned char* key_mask, const v
         attr_set = true;
     }
     dim3 grid((S + BQ - 1) / BQ, n_heads, B);
-    attn_bwd_dkdv_tc_kernel<<<grid, kBwdThreads, KV_SMEM_BYTES, st>>>(tq, td, key_mask, lse, Dsum, (__nv_bfloat16*)dqkv,
+    attn_bwd_dkdv_tc_kernel<<<grid, kBwdThreads, KV_SMEM_BYTES, st>>>(tq, td, to, key_mask, lse, Dsum, (__nv_bfloat16*)dqkv,
                                                                       S, n_heads, scale, scale * LOG2E,
                                                                       (const __nv_bfloat16*)rope_cos,
                                                                       (const __nv_bfloat16*)rope_sin LLARK_ATC_SLOPES_ARG);
-    attn_bwd_dq_tc_kernel<<<grid, kBwdThreads, DQ_SMEM_BYTES, st>>>(tq, td, key_mask, lse, Dsum, (__nv_bfloat16*)dqkv, S,
+    attn_bwd_dq_tc_kernel<<<grid, kBwdThreads, DQ_SMEM_BYTES, st>>>(tq, td, to, key_mask, lse, Dsum, (__nv_bfloat16*)dqkv, S,
                                                                     n_heads, scale, scale * LOG2E,
                                                                     (const __nv_bfloat16*)rope_cos,
                                                                     (const __nv_bfloat16*)rope_sin LLARK_ATC_SLOPES_ARG);

@@ -367,6 +367,36 @@ def test_attention_fwd_bwd(B, S, NH, pad):
         assert _rel(got[:, :, i], g[:, :, i]) < 1.5e-2, name
 
 
+@pytest.mark.parametrize("S", [1, 63, 65, 127, 128, 129, 191, 193, 321, 384])
+def test_attention_bwd_tiles_end_inside_and_between_samples(S):
+    """One half of a tile of keys, one row of the next, whole tiles only: gradients of the middle one of three samples against autograd in
+    64 bits of the same bf16 inputs. dS and P pass through bf16 (2^-9 each, two roundings a product), as the bounds above have it. The
+    samples beside it get the same gradients whatever their neighbours hold: no tile reads or writes over its sample's end."""
+    ops = _ops()
+    torch.manual_seed(S)
+    B, NH, D = 3, 2, 128
+    qkv = torch.randn(B * S, 3 * NH * D, device="cuda").to(BF16)
+    dout = (0.1 * torch.randn(B * S, NH * D, device="cuda")).to(BF16)
+    out, lse = ops.attn_fwd(qkv, None, B, S, NH, D)
+    got = ops.attn_bwd(qkv, None, out, dout, lse, B, S, NH, D)
+    x = qkv.view(B, S, 3, NH, D)[1].double().requires_grad_(True)
+    sc = torch.einsum("thd,shd->hts", x[:, 0], x[:, 1]) / math.sqrt(D)
+    seen = torch.ones(S, S, device="cuda", dtype=torch.bool).tril()
+    o = torch.einsum("hts,shd->thd", torch.softmax(sc.masked_fill(~seen, -math.inf), -1), x[:, 2])
+    want, = torch.autograd.grad(o, x, dout.view(B, S, NH, D)[1].double())
+    mid = got.view(B, S, 3, NH, D)[1]
+    for i, name in enumerate("qkv"):
+        if S > 1 or name == "v":  # one key: p = 1, and dq = dk = 0
+            assert _rel(mid[:, i], want[:, i]) < 1.5e-2, name
+        else:
+            assert mid[:, i].float().abs().max() < 1e-2
+    for b in range(B):
+        one = slice(b * S, (b + 1) * S)
+        alone = ops.attn_bwd(qkv[one].contiguous(), None, out[one].contiguous(), dout[one].contiguous(),
+                             lse.view(B, -1)[b].contiguous(), 1, S, NH, D)
+        assert torch.equal(alone, got[one])
+
+
 @pytest.mark.parametrize("B,S,NH,pad", [(2, 512, 4, True), (1, 200, 2, False), (1, 4160, 1, True)])
 def test_attention_bwd_with_fused_inverse_rope_is_bit_identical(B, S, NH, pad):
     """llark_attn_bwd_rope == llark_attn_bwd followed by llark_rope(inverse=1), bit for bit: on the tcgen05 kernels (rotation
