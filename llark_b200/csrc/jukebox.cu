@@ -397,8 +397,10 @@ jb_sparse_attn_kernel(const float* __restrict__ qkv, float* __restrict__ out, in
 //   O = P V    with P taken straight from the S accumulators: the m16n8k8 A fragment wants key slots (t, t+4) where the
 //              accumulator holds keys (2t, 2t+1), so the k index of the P.V product is permuted consistently -- slot t
 //              reads V row 8j+2t, slot t+4 reads V row 8j+2t+1 -- and no shuffle is needed.
-// K and V rows are gathered (stride 1 or `blk`) into shared memory once per CTA; while S is computed the V tile
-// replaces the Q staging tile. Operands are rounded to TF32 (cvt.rna) when the fragments are formed. Causal key tiles
+// K and V rows are gathered (stride 1 or `blk`) into shared memory by cp.async, all of them under way at once, and Q goes to its
+// fragments; S waits for K alone. It is bound by these loads: with eight granules of 8 bytes a thread in flight through registers, and V
+// after Q in one buffer, 16384 tokens x 8 heads took 239 us (64 rows) and 302 us (128 rows); now 119
+// and 179. Operands are rounded to TF32 (cvt.rna) when the fragments are formed. Causal key tiles
 // above the diagonal are skipped. Output fp32 or bf16 (fused cast for the bf16 prior).
 constexpr int JA_LD = 156;   // shared-memory row pitch (floats): 156 mod 32 = 28 -> conflict-free fragment loads
 constexpr int JA_KS = 19;    // k-steps of 8 covering head channels (<= 152)
@@ -413,28 +415,25 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], 
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// rows x dh floats gathered from global (row r at base + (pos0 + r*stride)*rs) into smem [rows][JA_LD], pad columns zero
-__device__ __forceinline__ void ja_load_rows(float* dst, const float* __restrict__ base, long long pos0, int stride,
-                                             long long rs, int rows, int dh) {
-    constexpr int pairs = JA_LD / 2;  // float2 granules per row (dh is even, rows are 8-byte aligned)
-    const int total = rows * pairs;
-    // eight independent loads in flight per thread before the first shared-memory store
-    for (int i0 = threadIdx.x; i0 < total; i0 += 8 * blockDim.x) {
-        float2 v[8];
+// rows x dh floats gathered from global (row r at base + (pos0 + r*stride)*rs) into smem [rows][JA_LD], pad columns zero: every granule of
+// 8 bytes (dh is even, rows are 8-byte aligned) is asked for at once, none passes through a register
+__device__ __forceinline__ void ja_ask_rows(float* dst, const float* __restrict__ base, long long pos0, int stride,
+                                            long long rs, int rows, int dh) {
+    const int lane = threadIdx.x & 31;
+    const float* src = base + (pos0 + (long long)(threadIdx.x >> 5) * stride) * rs;
+    const long long step = (long long)(blockDim.x >> 5) * stride * rs;
+    for (int r = threadIdx.x >> 5; r < rows; r += blockDim.x >> 5, src += step) {  // a warp per row
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int i = i0 + u * blockDim.x;
-            const int r = i / pairs, c = (i % pairs) * 2;
-            v[u] = make_float2(0.f, 0.f);
-            if (i < total && c < dh) v[u] = *reinterpret_cast<const float2*>(base + (pos0 + (long long)r * stride) * rs + c);
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int i = i0 + u * blockDim.x;
-            const int r = i / pairs, c = (i % pairs) * 2;
-            if (i < total) *reinterpret_cast<float2*>(dst + r * JA_LD + c) = v[u];
+        for (int k = 0; k < (JA_LD / 2 + 31) / 32; ++k) {
+            const int c = 2 * (lane + 32 * k);
+            float* to = dst + r * JA_LD + c;
+            if (c < dh)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(to)), "l"(src + c) : "memory");
+            else if (c < JA_LD)
+                *reinterpret_cast<float2*>(to) = make_float2(0.f, 0.f);
         }
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
 }
 template <int NKT>  // key tiles of 8 (8 -> 64 keys, 16 -> 128 keys)
 __global__ void __launch_bounds__(256)
@@ -443,7 +442,7 @@ jb_sparse_attn_tc_kernel(const float* __restrict__ qkv, void* __restrict__ out, 
     extern __shared__ __align__(16) float sm[];
     constexpr int NK = NKT * 8;
     float* sK = sm;                 // [NK][JA_LD]
-    float* sV = sm + NK * JA_LD;    // [NK][JA_LD]  (first holds the Q tile)
+    float* sV = sm + NK * JA_LD;    // [NK][JA_LD]
     const int g = blockIdx.x, h = blockIdx.y, n = blockIdx.z;
     int qstride, q0, k0;
     bool causal, has_keys = true;
@@ -465,19 +464,23 @@ jb_sparse_attn_tc_kernel(const float* __restrict__ qkv, void* __restrict__ out, 
         }
         return;
     }
-    ja_load_rows(sK, base + (long long)heads * dh, k0, qstride, rs, NK, dh);
-    ja_load_rows(sV, base, q0, qstride, rs, NK, dh);  // Q staged in the V buffer
-    __syncthreads();
+    ja_ask_rows(sK, base + (long long)heads * dh, k0, qstride, rs, NK, dh);
+    ja_ask_rows(sV, base + 2LL * heads * dh, k0, qstride, rs, NK, dh);
     uint32_t qa[JA_KS][4];
+    {
+        const float* q = base + (q0 + (long long)r0 * qstride) * rs;
+        const float* q8 = q + 8LL * qstride * rs;
 #pragma unroll
-    for (int ks = 0; ks < JA_KS; ++ks) {
-        qa[ks][0] = to_tf32(sV[r0 * JA_LD + ks * 8 + t4]);
-        qa[ks][1] = to_tf32(sV[(r0 + 8) * JA_LD + ks * 8 + t4]);
-        qa[ks][2] = to_tf32(sV[r0 * JA_LD + ks * 8 + t4 + 4]);
-        qa[ks][3] = to_tf32(sV[(r0 + 8) * JA_LD + ks * 8 + t4 + 4]);
+        for (int ks = 0; ks < JA_KS; ++ks) {
+            const int c = ks * 8 + t4;
+            qa[ks][0] = to_tf32(c < dh ? q[c] : 0.f);
+            qa[ks][1] = to_tf32(c < dh ? q8[c] : 0.f);
+            qa[ks][2] = to_tf32(c + 4 < dh ? q[c + 4] : 0.f);
+            qa[ks][3] = to_tf32(c + 4 < dh ? q8[c + 4] : 0.f);
+        }
     }
-    __syncthreads();  // every warp holds its Q fragments: the buffer may now receive V
-    ja_load_rows(sV, base + 2LL * heads * dh, k0, qstride, rs, NK, dh);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();  // K is there
     // key tiles this warp needs: causal rows 16w .. 16w+15 see keys <= 16w+15
     const int nt_end = causal ? min(NKT, 2 * warp + 2) : NKT;
     float sc[NKT][4];
@@ -523,7 +526,8 @@ jb_sparse_attn_tc_kernel(const float* __restrict__ qkv, void* __restrict__ out, 
         sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 1);
         sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 2);
     }
-    __syncthreads();  // V tile complete in shared memory
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();  // V is there
     float oacc[JA_KS][4];
 #pragma unroll
     for (int nn = 0; nn < JA_KS; ++nn) oacc[nn][0] = oacc[nn][1] = oacc[nn][2] = oacc[nn][3] = 0.f;
