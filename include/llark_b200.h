@@ -172,6 +172,16 @@ int llark_attn_decode(const void* q, const void* k_cache, const void* v_cache, c
  * launch. */
 int llark_attn_decode_packed(const void* qkv, long long ld, void* k_cache, void* v_cache, int pos, void* out, int B, int s_max,
                              int n_heads, int head_dim, float scale, cudaStream_t stream);
+/* The decoder layers of a step of B <= 64 rows (one token each, all at position `pos`), heads of 128: x [B, H] bf16 goes through them in
+ * place; per layer the weights (gate_up: gate rows, then up rows) and its caches [B, s_max, H], which get the new keys and values.
+ * cos_row / sin_row: 128 values of position `pos`. scratch: llark_decode_scratch bytes, rstd: B floats. */
+typedef struct LlarkDecodeLayer {
+    const void *norm1, *qkv, *o, *norm2, *gate_up, *down;
+    void *k, *v;
+} LlarkDecodeLayer;
+long long llark_decode_scratch(int B, int H, int I);
+int llark_decode_layers(const LlarkDecodeLayer* layers, int n_layers, void* x, void* scratch, const void* cos_row, const void* sin_row,
+                        int pos, int B, int s_max, int H, int I, int n_heads, float eps, float* rstd, cudaStream_t stream);
 long long llark_attn_bwd_workspace(int B, int S, int n_heads);
 int llark_attn_bwd(const void* qkv, const unsigned char* key_mask, const void* out, const void* dout, const float* lse,
                    void* dqkv, int B, int S, int n_heads, int head_dim, float scale, void* workspace,

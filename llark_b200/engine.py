@@ -18,7 +18,7 @@ import os
 import torch
 
 from . import ops
-from .ops import LINEAR_FEW_MAX
+from .ops import LINEAR_FEW_MAX, DecodeLayer, decode_layers
 
 BF16 = torch.bfloat16
 _ALIGN = 128  # elements (256 B): keeps every view 16-byte aligned for TMA and fused views gap-free
@@ -73,7 +73,7 @@ class FlatBuckets:
             view = self.params[o:o + k].view(p.shape)
             view.copy_(p.data)  # converts when cast_to_bf16 admitted another storage dtype
             p.data = view
-        self._views = {}  # fused views asked for before: (name, shape, span) -> view of params
+        self._views = {}  # fused views asked for before: (name, shape, span) -> view of params; "decode": decode_table()
         self._order = None  # the parameters in module order, as is_same() saw them last
         self.grads_attached = False
         # set by the fused optimizer step: the bucket's contents have been consumed, so the next backward
@@ -136,6 +136,23 @@ class FlatBuckets:
                 raise RuntimeError(f"parameters after {name} are not contiguous in the flat bucket")
             tot += kj
         return self.params[o:o + tot].view(shape)
+
+    def decode_table(self, n_layers, H, I, keys, values):
+        """The layers' weights (addresses in this bucket, found once) and caches as decode_layers() takes them."""
+        plan = self._views.get("decode")
+        if plan is None:
+            plan = (DecodeLayer * n_layers)()
+            for l, row in enumerate(plan):
+                pfx = f"model.layers.{l}."
+                for field, name, shape, span in (("norm1", "input_layernorm", None, 1), ("qkv", "self_attn.q_proj", (3 * H, H), 3),
+                                                 ("o", "self_attn.o_proj", (H, H), 1), ("norm2", "post_attention_layernorm", None, 1),
+                                                 ("gate_up", "mlp.gate_proj", (2 * I, H), 2), ("down", "mlp.down_proj", (H, I), 1)):
+                    setattr(row, field, self.pview(f"{pfx}{name}.weight", shape, span=span).data_ptr())
+            self._views["decode"] = plan
+        table = type(plan).from_buffer_copy(plan)  # a step's own: another thread may be in another step
+        for row, k, v in zip(table, keys, values):
+            row.k, row.v = k.data_ptr(), v.data_ptr()
+        return table
 
     def gview(self, name, shape=None, span=1):
         o, k = self.offsets[name]
@@ -491,7 +508,10 @@ class LlamaEngine:
         cache.lens.fill_(t + 1)  # the cache's own record, which attn_decode reads; the form below takes t
         few = B <= LINEAR_FEW_MAX and H % 8 == 0 and I % 8 == 0  # gate times up in the product's epilogue
         rstd = torch.empty(B, device=dev, dtype=torch.float32)
-        for l in range(L):
+        native = few and x.is_cuda and self.fuse_epilogues and D == 128 and ops.GEMM_PROFILE is None
+        if native:  # the loop below, its launches issued by one call
+            decode_layers(flat.decode_table(L, H, I, cache.k, cache.v), x, cos_t, sin_t, t, cache.s_max, I, NH, eps, rstd)
+        for l in range(0 if native else L):
             pfx = f"model.layers.{l}."
             Wqkv = flat.pview(pfx + "self_attn.q_proj.weight", (3 * H, H), span=3)
             Wo = flat.pview(pfx + "self_attn.o_proj.weight", (H, H))

@@ -226,6 +226,22 @@ def attn_decode_packed(qkv, k_cache, v_cache, pos, n_heads, head_dim, out=None):
     return out
 
 
+class DecodeLayer(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_void_p) for n in ("norm1", "qkv", "o", "norm2", "gate_up", "down", "k", "v")]
+
+
+def decode_layers(layers, x, cos, sin, pos, s_max, inner, n_heads, eps, rstd):
+    """layers: array of DecodeLayer; x bf16 [B, H] goes through them in place, one token per row at position `pos`; cos / sin: views of the
+    rotary tables whose first row is that position."""
+    if not _INITED:
+        init()
+    B, H = x.shape
+    L = lib()
+    scratch = torch.empty(L.llark_decode_scratch(B, H, inner), device=x.device, dtype=torch.uint8)
+    check(L.llark_decode_layers(layers, len(layers), _p(x), _p(scratch), _p(cos), _p(sin), int(pos), B, s_max, H, inner, n_heads,
+                                float(eps), _p(rstd), _stream()), "decode_layers")
+
+
 def attn_bwd(qkv, key_mask, out, dout, lse, B, S, n_heads, head_dim, dqkv=None, workspace=None, rope=None):
     """dqkv = (dq | dk | dv). rope=(cos, sin) (bf16 [>= S, head_dim]): the inverse rotary embedding of the dq | dk heads is
     fused into the backward kernels (llark_attn_bwd_rope), bit-identical to attn_bwd followed by rope_(inverse=True)."""

@@ -126,3 +126,30 @@ def test_scores_that_are_not_numbers_reach_the_result(D, H, G):
     w = torch.softmax(torch.cat([s, sink.to(F64)[:, None]], 1), 1)[:, :-1]
     ref = torch.einsum("hj,jhd->hd", w, v[3, 50:71].repeat_interleave(H // G, 1).to(F64))
     assert ((got[3].to(F64) - ref).norm() / ref.norm()).item() < 2.0 ** -8
+
+
+@pytest.mark.parametrize("B,H,I,pos", [(1, 256, 512, 0), (9, 256, 520, 5), (33, 512, 1000, 17), (64, 256, 264, 31)])
+def test_layers_of_a_decode_step_in_one_call(B, H, I, pos):
+    """The layers issued by one call against the single ops of the same step: the same launches, so the same bits, in x and in the caches."""
+    from llark_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(B + H)
+    r = lambda *s, std=1.0: (std * torch.randn(*s, device="cuda", generator=g)).to(torch.bfloat16)  # noqa: E731
+    L, NH, s_max = 3, H // 128, 40
+    cos, sin = r(s_max, 128), r(s_max, 128)
+    w = [dict(norm1=r(H), qkv=r(3 * H, H, std=H ** -0.5), o=r(H, H, std=H ** -0.5), norm2=r(H), gate_up=r(2 * I, H, std=H ** -0.5),
+              down=r(H, I, std=I ** -0.5), k=r(B, s_max, H), v=r(B, s_max, H)) for _ in range(L)]
+    x0 = r(B, H)
+    rstd = torch.empty(B, device="cuda", dtype=torch.float32)
+    caches = [(a["k"].clone(), a["v"].clone()) for a in w]
+    x = x0
+    for a, (k, v) in zip(w, caches):
+        qkv = ops.gemm(ops.rmsnorm_fwd(x, a["norm1"], 1e-5, rstd=rstd), a["qkv"], rope=(cos[pos:], sin[pos:], 1, 2 * H))
+        mid = ops.gemm(ops.attn_decode_packed(qkv, k, v, pos, NH, 128), a["o"], residual=x)
+        act = ops.gemm(ops.rmsnorm_fwd(mid, a["norm2"], 1e-5, rstd=rstd), a["gate_up"], swiglu=True)
+        x = ops.gemm(act, a["down"], residual=mid)
+    table = (ops.DecodeLayer * L)(*[ops.DecodeLayer(**{n: t.data_ptr() for n, t in a.items()}) for a in w])
+    got = x0.clone()
+    ops.decode_layers(table, got, cos[pos:], sin[pos:], pos, s_max, I, NH, 1e-5, rstd)
+    assert torch.equal(got, x)
+    assert all(torch.equal(a["k"], k) and torch.equal(a["v"], v) for a, (k, v) in zip(w, caches))
