@@ -13,8 +13,9 @@
 // A CTA is two or three groups of four warps, each with tiles of 128 steps, rows of A, accumulators and a barrier of its own; the next
 // tile's values are requested as soon as this one's rows are written.
 //
-//   res block   (dilations from 33 on; up to 32 jb_chain_tc.cu is ahead, 184 to 201 us at the size below) y = x + W2 relu(W1 (*dilation d, 3 taps) relu(x) + b1) + b2, both convolutions of a tile in one visit: the second's A
-//               operand is the first's result, written by the thread that owns the row
+//   res block   y = x + W2 relu(W1 (*dilation d, 3 taps) relu(x) + b1) + b2, both convolutions of a tile in one visit: the second's A
+//               operand is the first's result, written by the thread that owns the row. For dilations from 33 on: up to 32
+//               jb_chain_tc.cu is ahead (184 to 201 us at the size below)
 //   others      taps 4 stride 2 (32 or 64 channels in, 32 out), taps 3 (32 in, 64 out)
 //
 // What bounds it: the latency of load, split, product and read-back of a tile, hidden only by the other groups (a res block reads and
