@@ -138,21 +138,15 @@ class FlatBuckets:
         return self.params[o:o + tot].view(shape)
 
     def decode_table(self, n_layers, H, I, keys, values):
-        """The layers' weights (addresses in this bucket, found once) and caches as decode_layers() takes them."""
-        plan = self._views.get("decode")
-        if plan is None:
-            plan = (DecodeLayer * n_layers)()
-            for l, row in enumerate(plan):
-                pfx = f"model.layers.{l}."
-                for field, name, shape, span in (("norm1", "input_layernorm", None, 1), ("qkv", "self_attn.q_proj", (3 * H, H), 3),
-                                                 ("o", "self_attn.o_proj", (H, H), 1), ("norm2", "post_attention_layernorm", None, 1),
-                                                 ("gate_up", "mlp.gate_proj", (2 * I, H), 2), ("down", "mlp.down_proj", (H, I), 1)):
-                    setattr(row, field, self.pview(f"{pfx}{name}.weight", shape, span=span).data_ptr())
-            self._views["decode"] = plan
-        table = type(plan).from_buffer_copy(plan)  # a step's own: another thread may be in another step
-        for row, k, v in zip(table, keys, values):
-            row.k, row.v = k.data_ptr(), v.data_ptr()
-        return table
+        """The layers' weights and caches as decode_layers() takes them. What is kept are the views: a copy of this bucket has its own."""
+        rows = self._views.get("decode")
+        if rows is None:
+            names = (("input_layernorm", None, 1), ("self_attn.q_proj", (3 * H, H), 3), ("self_attn.o_proj", (H, H), 1),
+                     ("post_attention_layernorm", None, 1), ("mlp.gate_proj", (2 * I, H), 2), ("mlp.down_proj", (H, I), 1))
+            rows = self._views["decode"] = [[self.pview(f"model.layers.{l}.{n}.weight", shape, span=span) for n, shape, span in names]
+                                            for l in range(n_layers)]
+        return (DecodeLayer * n_layers)(*[DecodeLayer(*[t.data_ptr() for t in row], k.data_ptr(), v.data_ptr())
+                                          for row, k, v in zip(rows, keys, values)])
 
     def gview(self, name, shape=None, span=1):
         o, k = self.offsets[name]
