@@ -13,6 +13,10 @@
 //
 // A CTA has 256 vectors (two row tiles of A) and goes through the codebook in tiles of 128 codes: four threads make one row of B of the
 // next tile while the tensor cores multiply; two threads share a vector's sums, 64 columns each.
+//
+// What bounds it: a tile's chain of conversion, products and sums' reading, and the candidates' walks at the end. Measured on a B200, 32768
+// vectors, us, walk over all codes / here: 2048 codes 425 / 97, a hundred times closer together 420 / 90, 512 codes 103 / 32. With one
+// bf16 part each (bound 2^-7 |x| |k|, so that more is walked) 169, and 949 where codes are close.
 #include "common.cuh"
 #include <math.h>
 
