@@ -538,7 +538,7 @@ __device__ __forceinline__ void epilogue_dispatch(const GemmParams& p, long long
 // R that are under way, here 32 KB to 64 KB per SM where four warps with loads to registers had 16 KB. Measured on a B200, us before -> now:
 // M 16384, N 4800, K 1200, fp32 with a residual 316 -> 204; K 4800, fp32 with a residual 609 -> 595, bf16 with quick-GELU 617 -> 544; M 6100,
 // N 6144, K 2048, fp32 163 -> 134; M 8192, bf16: N 12288, K 4096 559 -> 555, N 4096, K 4096 with a residual 203 -> 198, N 32000 1438 -> 1428.
-// Eight warps with direct stores: slower than four in all of these by 1 to 2 % (569 us where TMA takes 555).
+// (These are from before the issuer slept, see there.) Eight warps with direct stores: slower than four in all of these by 1 to 2 %.
 __device__ __forceinline__ void load_bias32(const GemmParams& p, int col0, float (&b)[32]) {
     if (col0 + 32 <= p.N && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) {  // the same addresses for the whole warp
         if (p.bias_fp32) {
@@ -853,8 +853,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
 // (rank 0) issues tcgen05.mma.cta_group::2 (M = 256, N = 256) which reads both CTAs' operands, and each CTA's
 // TMEM receives its 128 accumulator rows x 256 columns. Per SM the shared-memory traffic drops from
 // 96 (TMA writes) + 96 (UMMA reads) B/clk to 64 + 64 B/clk, which is what lets the tensor pipe stay busy.
-constexpr int kThreads2 = 384;   // warps 0-3 as above, 4-11 epilogue: two per 32 rows, 128 columns each
-constexpr int kEpiWarps2 = 8;
+constexpr int kEpiWarps2 = 8;    // two per 32 rows of a tile, 128 columns each
+// Four with 256 columns each for the gated pairs (EPI 6, 7), which have no TMA form: eight / four, B200, us: ReLU pairs M 300, N 2048, K 1024
+// 16.0 / 14.4, M 8192, N 8192, K 2048 230 / 219; clamped pairs 232 / 224.
+template <int EPI>
+constexpr int epi_warps = EPI == 6 || EPI == 7 ? 4 : kEpiWarps2;
+template <int EPI>
+constexpr int kThreads2 = (4 + epi_warps<EPI>) * 32;  // warps 0-3 as above, epilogue
 constexpr int kSlots2 = 7;       // 32 KB slots of shared memory: operand stages, the epilogue warps' patches behind them
 constexpr int kMaxStages2 = 6;   // six stages and a patch per warp, or five and two (GemmParams::stages)
 constexpr int kSched = 4;  // depth of the tile-index ring of the dynamic scheduler
@@ -864,7 +869,7 @@ constexpr int SMEM2_BYTES = kSlots2 * STAGE2_BYTES + 1024 + 512;
 static_assert(kEpiWarps2 * EPI_WARP_BYTES == STAGE2_BYTES, "one patch per epilogue warp fills a slot");
 
 template <int A_MN, int B_MN, int TF32, int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads2, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads2<EPI>, 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
              const __grid_constant__ CUtensorMap tma_c, const __grid_constant__ CUtensorMap tma_r, const GemmParams p) {
     constexpr int kElemBytes = TF32 ? 4 : 2;  // operand element size is a property of the instantiation
@@ -907,11 +912,11 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
         }
         for (int i = 0; i < kAccStages; ++i) {
             mbar_init(&tmem_full[i], 1);
-            mbar_init(&tmem_empty[i], 2 * kEpiWarps2);  // the epilogue warps of both CTAs arrive on the leader's barrier
+            mbar_init(&tmem_empty[i], 2 * epi_warps<EPI>);  // the epilogue warps of both CTAs arrive on the leader's barrier
         }
         for (int i = 0; i < kSched; ++i) {
             mbar_init(&sched_full[i], 1);
-            mbar_init(&sched_empty[i], 5 + 2 * kEpiWarps2);  // A/B producers and epilogue warps of both CTAs, the leader's MMA
+            mbar_init(&sched_empty[i], 5 + 2 * epi_warps<EPI>);  // A/B producers and epilogue warps of both CTAs, the leader's MMA
         }
         for (int i = 0; i < 2 * kEpiWarps2; ++i) mbar_init(&res_bar[i], 1);
         mbar_fence_init();
@@ -1102,7 +1107,9 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
         }
     } else if (warp >= 4) {
         // ===================== epilogue (both CTAs, own 128 rows) =====================
-        const int ew = warp & 3, half = (warp - 4) >> 2;  // TMEM lanes 32 ew .. are open to warps with this warp % 4
+        const int ew = warp & 3;  // TMEM lanes 32 ew .. are open to warps with this warp % 4
+        constexpr int span = BLOCK_N * 4 / epi_warps<EPI>;  // columns of a warp
+        const int lo = ((warp - 4) >> 2) * span;
         int it = 0;
         const uint32_t leader_empty0 = mapa_shared(smem_u32(&tmem_empty[0]), 0);
         const int n_patches = kSlots2 - stages;
@@ -1117,16 +1124,16 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
             const int ncol0 = tc.n_blk * BLOCK_N;
             const uint32_t acc = tmem_base + ((uint32_t)(ew * 32) << 16) + as * BLOCK_N;
             if ((EPI == 0 || EPI == 1 || EPI == 2 || EPI == 5) && p.staged == 2 && !(EPI == 2 && ncol0 < p.epi_i1)) {
-                const int pieces = epi_pieces(p, row0, ncol0 + half * 128);
-                if (p.R && pieces && lane == 0) ask_residual(patch, patch.g, &tma_r, ncol0 + half * 128, (int)row0);
+                const int pieces = epi_pieces(p, row0, ncol0 + lo);
+                if (p.R && pieces && lane == 0) ask_residual(patch, patch.g, &tma_r, ncol0 + lo, (int)row0);
                 mbar_wait(&tmem_full[as], aphase);
                 tc_fence_after();
-                epi_tma<EPI>(p, &tma_c, &tma_r, (int)row0, ncol0 + half * 128, pieces, acc + half * 128, patch, lane);
-                epi_rest<EPI>(p, row0 + lane, ncol0 + half * 128, pieces, acc + half * 128);
+                epi_tma<EPI>(p, &tma_c, &tma_r, (int)row0, ncol0 + lo, pieces, acc + lo, patch, lane);
+                epi_rest<EPI>(p, row0 + lane, ncol0 + lo, pieces, acc + lo);
             } else {
                 mbar_wait(&tmem_full[as], aphase);
                 tc_fence_after();
-                epilogue_dispatch<EPI, EPI == 3>(p, row0, m_end, lane, ncol0, acc, reinterpret_cast<float*>(patch.at), half * 4, half * 4 + 4);
+                epilogue_dispatch<EPI, EPI == 3>(p, row0, m_end, lane, ncol0, acc, reinterpret_cast<float*>(patch.at), lo / 32, (lo + span) / 32);
             }
             tc_fence_before();
             __syncwarp();
@@ -1346,7 +1353,7 @@ static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const GemmMaps&
     if (tiles < clusters) clusters = tiles;
     if (max_ctas > 1 && clusters > max_ctas / 2) clusters = max_ctas / 2;
     if (clusters < 1) clusters = 1;
-    kfn<<<clusters * 2, kThreads2, SMEM2_BYTES, stream>>>(ta, tb, m.c, m.r, p);
+    kfn<<<clusters * 2, kThreads2<EPI>, SMEM2_BYTES, stream>>>(ta, tb, m.c, m.r, p);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         g_last_cuda_error = (int)e;
