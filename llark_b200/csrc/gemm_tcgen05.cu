@@ -604,21 +604,22 @@ __device__ __forceinline__ void ask_residual(const EpiPatch& e, uint32_t g, cons
     tma_load_2d(patch_of(e, g), rmap, bar, col, row);
 }
 // Pieces of this warp in a tile: columns [col_lo, col_lo + 128) of N, rows from row0 on. A row of C that ends inside 16 bytes
-// is cut off behind them by TMA (the bytes beside C were overwritten): its last columns are left to epi_rest.
-__device__ __forceinline__ int epi_pieces(const GemmParams& p, long long row0, int col_lo) {
-    if (row0 >= p.M || col_lo >= p.N) return 0;
+// is cut off behind them by TMA (the bytes beside C were overwritten): its last columns are left to epi_rest. So are 32 rows
+// in which a run of rows ends: the next run's are another tile's.
+__device__ __forceinline__ int epi_pieces(const GemmParams& p, long long row0, long long m_end, int col_lo) {
+    if (row0 >= m_end || col_lo >= p.N || (p.seg_tiles && row0 + 32 > m_end)) return 0;
     const int w = p.c_fp32 ? 32 : 64, last = p.N % (p.c_fp32 ? 4 : 8) ? p.N / w : (p.N + w - 1) / w;
     return min(128 / w, last - col_lo / w);
 }
 template <int EPI>
-__device__ __forceinline__ void epi_rest(const GemmParams& p, long long row, int col_lo, int pieces, uint32_t taddr) {
+__device__ __forceinline__ void epi_rest(const GemmParams& p, long long row, long long m_end, int col_lo, int pieces, uint32_t taddr) {
     const int end = min(col_lo + 128, p.N);
 #pragma unroll 1
     for (int col = col_lo + pieces * (p.c_fp32 ? 32 : 64); col < end; col += 32) {
         uint32_t v[32];
         tmem_ld_32x32b_x32(taddr + (col - col_lo), v);
         tmem_ld_wait();
-        if (row < p.M) epilogue_store_chunk<EPI>(p, row, col, v);
+        if (row < m_end) epilogue_store_chunk<EPI>(p, row, col, v);
     }
 }
 template <int EPI>
@@ -1124,12 +1125,12 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
             const int ncol0 = tc.n_blk * BLOCK_N;
             const uint32_t acc = tmem_base + ((uint32_t)(ew * 32) << 16) + as * BLOCK_N;
             if ((EPI == 0 || EPI == 1 || EPI == 2 || EPI == 5) && p.staged == 2 && !(EPI == 2 && ncol0 < p.epi_i1)) {
-                const int pieces = epi_pieces(p, row0, ncol0 + lo);
+                const int pieces = epi_pieces(p, row0, m_end, ncol0 + lo);
                 if (p.R && pieces && lane == 0) ask_residual(patch, patch.g, &tma_r, ncol0 + lo, (int)row0);
                 mbar_wait(&tmem_full[as], aphase);
                 tc_fence_after();
                 epi_tma<EPI>(p, &tma_c, &tma_r, (int)row0, ncol0 + lo, pieces, acc + lo, patch, lane);
-                epi_rest<EPI>(p, row0 + lane, ncol0 + lo, pieces, acc + lo);
+                epi_rest<EPI>(p, row0 + lane, m_end, ncol0 + lo, pieces, acc + lo);
             } else {
                 mbar_wait(&tmem_full[as], aphase);
                 tc_fence_after();
@@ -1557,8 +1558,9 @@ extern "C" int llark_gemm_ex(const void* A, int a_mn_major, long long lda, const
                           (c_fp32 && R == nullptr && short_k);
         p.staged = segs ? 0 : (mode == 1 ? 1 : (mode == 2 ? 0 : (want ? 1 : 0)));
         // The CTA pair's epilogue goes through TMA wherever an element of C depends on nothing but its own sum, bias and
-        // residual; rows in runs end inside a tile, where a piece of 32 rows must not write, and keep the direct stores.
-        if (two_cta && !segs && mode == 0 &&
+        // residual; rows in runs as well (direct stores / TMA, B200, us, all kernels of the layer: 6000 rows over 64 experts of 1024 x 512,
+        // ReLU squared 98 / 88; 16384 over 32 of 2048 x 1024 253 / 211, 24576 over 64 of 4096 x 1024 707 / 578).
+        if (two_cta && mode == 0 &&
             (p.epi == LLARK_EPI_NONE || p.epi == LLARK_EPI_QUICK_GELU || p.epi == LLARK_EPI_ROPE || p.epi == LLARK_EPI_RELU2))
             p.staged = 2;
         p.stages = p.staged == 2 && R ? kMaxStages2 - 1 : kMaxStages2;

@@ -147,6 +147,42 @@ def test_gemm_output_pieces_end_at_the_edges(M, N, K, dt):
             assert torch.equal(buf, was)
 
 
+@pytest.mark.parametrize("N,K", [(8, 64), (36, 72), (130, 192), (512, 1024)])
+@pytest.mark.parametrize("epi", ["none", "relu2"])
+@pytest.mark.parametrize("dt", [torch.float32, BF16])
+def test_gemm_of_runs_of_rows_ends_with_its_runs(N, K, epi, dt):
+    """Runs that end inside, at and one row behind 32 rows and 256 rows, an empty one, rows between runs that belong to none: against 64
+    bits (the tensor cores cut each of the K / 16 sums of a product below 2^-23 of what is there, eight of them at least; squares double it; a
+    bf16 result 2^-8), and nothing written beside the runs or beside C."""
+    ops = _ops()
+    from llark_b200._lib import EPI_NONE, EPI_RELU2, check, lib
+
+    torch.manual_seed(N + K)
+    runs = [(0, 1), (1, 31), (3, 32), (2, 33), (4, 0), (5, 256), (6, 257), (7, 95)]  # (weights, rows)
+    ops.init()
+    tiles, row, spans = [], 5, []
+    for w, n in runs:
+        spans.append((w, row, n))
+        tiles += [(w, row + i, min(256, n - i)) for i in range(0, n, 256)]
+        row += n + (3 if w == 2 else 0)  # three rows of nobody
+    M, ld = row + 7, (N + 7) // 8 * 8 + 8
+    a, b = torch.randn(M, K, device="cuda").to(BF16), torch.randn(8, N, K, device="cuda").to(BF16)
+    dev = torch.tensor(tiles, device="cuda", dtype=torch.int32).flatten().contiguous()
+    count = torch.tensor([len(tiles)], device="cuda", dtype=torch.int32)
+    buf = torch.full((M, ld), 7.0, device="cuda", dtype=dt)
+    check(lib().llark_gemm_segments(a.data_ptr(), K, b.data_ptr(), buf.data_ptr(), ld, int(dt == torch.float32), None, 8, dev.data_ptr(),
+                                    len(tiles), count.data_ptr(), M, N, K, EPI_RELU2 if epi == "relu2" else EPI_NONE, 0.0, 0.0,
+                                    torch.cuda.current_stream().cuda_stream), "gemm_segments")
+    tol = max(K / 16, 8) * 2.0 ** -23 * (2 if epi == "relu2" else 1) if dt == torch.float32 else 2.0 ** -8
+    for w, r, n in spans:
+        if n:
+            z = a[r:r + n].double() @ b[w].double().t()
+            want = z.clamp_min(0).square() if epi == "relu2" else z
+            assert ((buf[r:r + n, :N].double() - want).norm() / want.norm()).item() < tol, (w, n)
+            buf[r:r + n, :N] = 7.0
+    assert (buf == 7.0).all()
+
+
 def test_gemm_tf32_mn_major_rejected():
     ops = _ops()
     from llark_b200._lib import LlarkError
