@@ -7,6 +7,7 @@
 //   that the product lacks three times 2^-18 |x| |k| (Cauchy-Schwarz), the sum of 192 products on the tensor cores is off by less than
 //   2^-16 |x| |k|, the walk's sum of 64 by 2^-18, and the three fp32 roundings of dist by 2^-24 (|x| + |k|)^2 each.
 //   Every code whose s - eps is not above the least s + eps is walked.
+// From 1e18 on (|x| or a code's |k|) sums may pass the largest number, and the bound says nothing: all codes are walked.
 // Codes whose |k|^2 is not finite have a dist that is not below anything, and are no candidates; a vector whose |x|^2 is not finite has
 // none below infinity and keeps code 0. Candidates are noted in runs of 32 codes, twelve runs a thread; if that overflows even after runs have
 // been struck off, the thread walks all codes of its half.
@@ -187,6 +188,7 @@ vq_kernel(const float* __restrict__ x, const float* __restrict__ cb, long long* 
         const float kn = sqrtf(__uint_as_float(*const_cast<volatile uint32_t*>(&most_kk))) * 1.0001f;
         if (tile + 1 < tiles) make_tile(tile + 1);
         const float eps = 1.220703125e-4f * xn * kn + 4.76837158203125e-7f * (xn + kn) * (xn + kn) + 1e-30f;
+        if (!(xn < 1e18f && kn < 1e18f)) runs.all = true;
         mbar_wait(&bar[buf], (tile >> 1) & 1);
         tc_fence_after();
 #pragma unroll 1
@@ -208,7 +210,9 @@ vq_kernel(const float* __restrict__ x, const float* __restrict__ cb, long long* 
                 uint32_t mask = 0u;
 #pragma unroll
                 for (int i = 0; i < 32; ++i) mask |= s[i] - eps <= least ? 1u << i : 0u;
-                note(runs, m - eps, mask, tile * 4 + half * 2 + (c >> 5), least);
+                const int run = tile * 4 + half * 2 + (c >> 5), real = n_codes - 32 * run;  // behind the last code: none
+                if (real < 32) mask &= (1u << max(real, 0)) - 1u;
+                note(runs, m - eps, mask, run, least);
             }
         }
         tc_fence_before();
