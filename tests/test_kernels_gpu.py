@@ -147,6 +147,23 @@ def test_gemm_output_pieces_end_at_the_edges(M, N, K, dt):
             assert torch.equal(buf, was)
 
 
+@pytest.mark.parametrize("M", [40, 300])
+@pytest.mark.parametrize("pitch", [0, 8, 64])
+@pytest.mark.parametrize("dt", [torch.float32, BF16])
+def test_gemm_residual_whose_rows_overlap(M, pitch, dt):
+    """A residual's row may begin before the last one's end: one row for all of them, or a sliding view. Few rows (the weights' stream) and
+    many (tiles), against 64 bits with the bounds above."""
+    ops = _ops()
+    torch.manual_seed(M + pitch)
+    N, K = 136, 128
+    a, b = torch.randn(M, K, device="cuda").to(BF16), torch.randn(N, K, device="cuda").to(BF16)
+    store = torch.randn(M * 64 + N, device="cuda").to(dt)
+    res = store.as_strided((M, N), (pitch, 1))
+    got = ops.gemm(a, b, out_dtype=dt, residual=res)
+    want = a.double() @ b.double().t() + res.double()
+    assert ((got.double() - want).norm() / want.norm()).item() < (2.0 ** -20 if dt == torch.float32 else 2.0 ** -8)
+
+
 @pytest.mark.parametrize("N,K", [(8, 64), (36, 72), (130, 192), (512, 1024)])
 @pytest.mark.parametrize("epi", ["none", "relu2"])
 @pytest.mark.parametrize("dt", [torch.float32, BF16])
