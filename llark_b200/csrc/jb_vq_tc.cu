@@ -9,15 +9,21 @@
 //   Every code whose s - eps is not above the least s + eps is walked.
 // From 1e18 on (|x| or a code's |k|) sums may pass the largest number, and the bound says nothing: all codes are walked.
 // Codes whose |k|^2 is not finite have a dist that is not below anything, and are no candidates; a vector whose |x|^2 is not finite has
-// none below infinity and keeps code 0. Candidates are noted in runs of 32 codes, twelve runs a thread; if that overflows even after runs have
-// been struck off, the thread walks all codes of its half.
+// none below infinity and keeps code 0. Candidates are noted in runs of 32 codes, twelve runs a thread.
 //
-// A CTA has 256 vectors (two row tiles of A) and goes through the codebook in tiles of 128 codes: four threads make one row of B of the
-// next tile while the tensor cores multiply; two threads share a vector's sums, 64 columns each.
+// A CTA has 256 vectors (two row tiles of A), or 128 where there are then no more CTAs than SMs, and goes through the codebook in tiles of 128
+// codes: four threads make one row of B of the next tile while the tensor cores multiply; two or four threads share a vector's sums. As
+// soon as a list overflows even after runs have been struck off, or where in the end a vector has more candidates than one in sixteen codes
+// (each costs its thread a microsecond, alone), the CTA walks all codes for its vectors (walk_all): with codes that are close or equal that is
+// what has to be done anyway. Vectors are counted through, whatever their clips' lengths.
 //
-// What bounds it: a tile's chain of conversion, products and sums' reading, and the candidates' walks at the end. Measured on a B200, 32768
-// vectors, us, walk over all codes / here: 2048 codes 425 / 97, a hundred times closer together 420 / 90, 512 codes 103 / 32. With one
-// bf16 part each (bound 2^-7 |x| |k|, so that more is walked) 169, and 949 where codes are close.
+// With no more than a CTA of 64 vectors an SM, or up to 256 codes, walk_all is all there is (walk_kernel): no slower than a walk of one lane per
+// two vectors for any data, where candidates would be faster for codes apart and slower for codes together.
+//
+// What bounds it: a tile's chain of conversion, products and sums' reading, and the candidates' walks at the end; walk_all: shared memory, 64
+// FMAs for four 16-byte reads. Measured on a B200, 2048 codes, us, codes apart / a third of them equal; in brackets the walk of one lane per two
+// vectors: 64 to 8192 vectors 84 / 84 (107), 16384 62 / 175 (210), 24576 89 / 260 (312), 32768 91 / 260 (415); 512 codes, 16384 vectors 23 / 51
+// (55), 32768 31 / 82 (100). The walk of 8192 vectors by CTAs of 128: 62 / 165. Of 64 codes and less the walk's staging is seen: 10 (8).
 #include "common.cuh"
 #include <math.h>
 
@@ -25,10 +31,150 @@ namespace llark {
 extern thread_local int g_last_cuda_error;
 namespace jbvq {
 
-constexpr int kE = 64, kRows = 256, kThreads = 2 * kRows, kTile = 128, kList = 12;
-constexpr int kPartA = kRows * 128, kPartB = kTile * 128;  // bytes of a part: 64 bf16 a row
-constexpr int kListBytes = kList * kThreads * 12;          // per run: s - eps of its least, which of the 32, number of the run
-constexpr int kSmem = 1024 + 2 * kPartA + 2 * 2 * kPartB + kListBytes;
+// x [N, 64, T] and the codes in shared memory, channel by channel; a thread has 8 vectors x 8 codes of a tile
+template <int ROWS, int THREADS>
+struct Walk {
+    static constexpr int kGroups = ROWS / 8, kShares = THREADS / kGroups, kCodes = 8 * kShares, kPitch = kCodes + 4;
+    static constexpr int kTileFloats = 64 * kPitch;
+    static constexpr int kBytes = (64 * ROWS + 2 * kTileFloats) * 4;
+    static_assert(kShares >= 8 && kGroups % 4 == 0 && 2 * kTileFloats >= 2 * ROWS * kShares, "");
+};
+// All codes for ROWS vectors from number v0 on (of N T): dist as above, every sum in the order of the channels. The thread's vectors and codes are two
+// runs of four each, half a tile apart: a quarter-warp reads 128 bytes side by side.
+template <int ROWS, int THREADS>
+__device__ __forceinline__ void walk_all(float* sx, float* sk, float* skk, float* sxx, const float* __restrict__ x,
+                         const float* __restrict__ cb, long long* __restrict__ codes, int v0, int vectors, int T, int n_codes) {
+    using W = Walk<ROWS, THREADS>;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int vg = (warp % (W::kGroups / 4)) * 4 + (lane >> 3), cg = (warp / (W::kGroups / 4)) * 8 + (lane & 7);
+    auto ask = [&](int tile) {  // 4 codes x 8 channels a warp: sectors of 32 bytes there, all banks here
+        float* dst = sk + (tile & 1) * W::kTileFloats;
+        for (int i = warp; i < 8 * (W::kCodes / 4); i += THREADS / 32) {
+            const int e = (i & 7) * 8 + (lane >> 2), r = (i >> 3) * 4 + (lane & 3), j = tile * W::kCodes + r;
+            if (j < n_codes)  // what lies behind the last code is multiplied and never taken
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst + e * W::kPitch + r)), "l"(cb + (long long)j * 64 + e)
+                             : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    {
+        static_assert(THREADS % ROWS == 0, "");
+        const int v = v0 + tid % ROWS, n = v / T;
+        const float* src = x + (long long)n * 64 * T + (v - n * T);
+        for (int e = tid / ROWS; e < 64; e += THREADS / ROWS) {
+            float* to = sx + e * ROWS + tid % ROWS;
+            if (v < vectors)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(to)), "l"(src + (long long)e * T) : "memory");
+            else
+                *to = 0.f;
+        }
+    }
+    ask(0);
+    float best[8];
+    int code[8];
+#pragma unroll
+    for (int v = 0; v < 8; ++v) best[v] = INFINITY, code[v] = 0;
+    const int tiles = (n_codes + W::kCodes - 1) / W::kCodes;
+    for (int tile = 0; tile < tiles; ++tile) {
+        const float* k0 = sk + (tile & 1) * W::kTileFloats;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();  // this tile is there, and the one before has been read
+        if (tile + 1 < tiles) ask(tile + 1);
+        if (tid < W::kCodes) {
+            float kk = 0.f;
+#pragma unroll 16
+            for (int e = 0; e < 64; ++e) kk = fmaf(k0[e * W::kPitch + tid], k0[e * W::kPitch + tid], kk);
+            skk[(tile & 1) * W::kCodes + tid] = kk;
+        }
+        if (tile == 0 && tid >= THREADS - ROWS) {
+            const int v = tid - (THREADS - ROWS);
+            float xx = 0.f;
+#pragma unroll 16
+            for (int e = 0; e < 64; ++e) xx = fmaf(sx[e * ROWS + v], sx[e * ROWS + v], xx);
+            sxx[v] = xx;
+        }
+        float dot[8][8];
+#pragma unroll
+        for (int v = 0; v < 8; ++v)
+#pragma unroll
+            for (int c = 0; c < 8; ++c) dot[v][c] = 0.f;
+        const float *px = sx + vg * 4, *pk = k0 + cg * 4;
+        const int left = n_codes - tile * W::kCodes;
+        if ((cg & ~7) * 4 < left)  // the warp's first code
+#pragma unroll 2
+        for (int e = 0; e < 64; ++e, px += ROWS, pk += W::kPitch) {
+            const float4 xa = *reinterpret_cast<const float4*>(px), xb = *reinterpret_cast<const float4*>(px + ROWS / 2);
+            const float4 ka = *reinterpret_cast<const float4*>(pk), kb = *reinterpret_cast<const float4*>(pk + W::kCodes / 2);
+            const float xv[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w}, kv[8] = {ka.x, ka.y, ka.z, ka.w, kb.x, kb.y, kb.z, kb.w};
+#pragma unroll
+            for (int v = 0; v < 8; ++v)
+#pragma unroll
+                for (int c = 0; c < 8; ++c) dot[v][c] = fmaf(xv[v], kv[c], dot[v][c]);
+        }
+        __syncthreads();  // |k|^2 of this tile, |x|^2
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            const int r = (c >> 2) * (W::kCodes / 2) + cg * 4 + (c & 3), j = tile * W::kCodes + r;
+            const float kk = skk[(tile & 1) * W::kCodes + r];
+#pragma unroll
+            for (int v = 0; v < 8; ++v) {
+                const float dist = (sxx[(v >> 2) * (ROWS / 2) + vg * 4 + (v & 3)] - 2.f * dot[v][c]) + kk;
+                if (j < n_codes && dist < best[v]) {
+                    best[v] = dist;
+                    code[v] = j;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    float* sd = sk;  // [share][vector]
+    int* sj = reinterpret_cast<int*>(sk + ROWS * W::kShares);
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+        const int at = cg * ROWS + (v >> 2) * (ROWS / 2) + vg * 4 + (v & 3);
+        sd[at] = best[v];
+        sj[at] = code[v];
+    }
+    __syncthreads();
+    if (tid < ROWS && v0 + tid < vectors) {
+        float d = INFINITY;
+        int j = 0;
+        for (int c = 0; c < W::kShares; ++c) {  // the shares' codes are not in order: equal ones, the first
+            const float dc = sd[c * ROWS + tid];
+            const int jc = sj[c * ROWS + tid];
+            if (dc < d || (dc == d && d < INFINITY && jc < j)) d = dc, j = jc;
+        }
+        codes[v0 + tid] = j;
+    }
+}
+
+constexpr int kWalkRows = 64, kWalkThreads = 128;
+__global__ void __launch_bounds__(kWalkThreads, 3)
+walk_kernel(const float* __restrict__ x, const float* __restrict__ cb, long long* __restrict__ codes, int vectors, int T, int n_codes) {
+    using W = Walk<kWalkRows, kWalkThreads>;
+    extern __shared__ __align__(16) unsigned char raw[];
+    __shared__ float skk[2 * W::kCodes], sxx[kWalkRows];
+    float* sx = reinterpret_cast<float*>(raw);
+    walk_all<kWalkRows, kWalkThreads>(sx, sx + 64 * kWalkRows, skk, sxx, x, cb, codes, blockIdx.x * kWalkRows, vectors, T, n_codes);
+}
+
+// in vq_kernel: called, so that its registers are not the sums' and candidates'
+template <int ROWS, int THREADS>
+__device__ __noinline__ void walk_all_called(float* sx, float* sk, float* skk, float* sxx,
+                                             const float* __restrict__ x, const float* __restrict__ cb, long long* __restrict__ codes,
+                                             int v0, int vectors, int T, int n_codes) {
+    walk_all<ROWS, THREADS>(sx, sk, skk, sxx, x, cb, codes, v0, vectors, T, n_codes);
+}
+
+constexpr int kE = 64, kThreads = 512, kTile = 128, kList = 12;
+constexpr int kPartB = kTile * 128;                // bytes of a part: 64 bf16 a row
+constexpr int kListBytes = kList * kThreads * 12;  // per run: s - eps of its least, which of the 32, number of the run
+template <int ROWS>  // 128 or 256 vectors, 4 or 2 threads each
+struct Shape {
+    static constexpr int kPartA = ROWS * 128, kParts = kThreads / ROWS, kCols = kTile / kParts;
+    static constexpr int kLists = 1024 + 2 * kPartA + 2 * 2 * kPartB + kListBytes, kWalk = 1024 + Walk<ROWS, kThreads>::kBytes;
+    static constexpr int kSmem = kLists > kWalk ? kLists : kWalk;  // walk_all takes the place of rows and lists
+};
 
 __device__ __forceinline__ uint64_t desc(uint32_t addr) {  // 128-byte rows, 8-row groups of 1024 bytes, 128-byte swizzle
     return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
@@ -62,7 +208,7 @@ struct Runs {  // a thread's noted runs, ascending
     uint32_t* mask;
     int* run;
     int n;
-    bool all;  // too many: walk everything
+    bool all;  // too many: all codes are walked
 };
 __device__ __noinline__ void note(Runs& r, float low, uint32_t mask, int run, float least) {
     if (r.all) return;
@@ -89,20 +235,23 @@ __device__ __noinline__ void note(Runs& r, float low, uint32_t mask, int run, fl
     ++r.n;
 }
 
+template <int ROWS>
 __global__ void __launch_bounds__(kThreads, 1)
-vq_kernel(const float* __restrict__ x, const float* __restrict__ cb, long long* __restrict__ codes, int T, int n_codes) {
+vq_kernel(const float* __restrict__ x, const float* __restrict__ cb, long long* __restrict__ codes, int vectors, int T, int n_codes) {
+    using S = Shape<ROWS>;
+    constexpr int kPartA = S::kPartA, kParts = S::kParts, kCols = S::kCols;
     extern __shared__ unsigned char raw[];
-    __shared__ __align__(16) float skk[2][kTile];  // read four at a time
+    __shared__ __align__(16) float skk[2 * Walk<ROWS, kThreads>::kCodes];  // of two tiles; read four at a time
     __shared__ uint64_t bar[2];
     __shared__ uint32_t tmem_base, most_kk;  // most_kk: bits of the largest finite |k|^2 of the tiles made so far
-    __shared__ float s_least[2][kRows], s_dist[kRows];
-    __shared__ int s_code[kRows];
+    __shared__ float s_least[kParts][ROWS], s_dist[kParts][ROWS];
+    __shared__ int s_code[kParts][ROWS];
     unsigned char* sa = raw + ((1024u - (smem_u32(raw) & 1023u)) & 1023u);
     unsigned char* sb = sa + 2 * kPartA;
     unsigned char* sl = sb + 2 * 2 * kPartB;
-    const int tid = threadIdx.x, row = tid & (kRows - 1), half = tid / kRows, warp = tid >> 5, lane = tid & 31;
-    const int n = blockIdx.y, t = blockIdx.x * kRows + row;
-    const bool vec = (reinterpret_cast<uintptr_t>(cb) & 15) == 0, in = t < T;
+    const int tid = threadIdx.x, row = tid & (ROWS - 1), part = tid / ROWS, warp = tid >> 5, lane = tid & 31;
+    const int v0 = blockIdx.x * ROWS, number = v0 + row, n = number / T;  // this thread's vector
+    const bool vec = (reinterpret_cast<uintptr_t>(cb) & 15) == 0, in = number < vectors;
     if (tid == 0) {
         mbar_init(&bar[0], 1);
         mbar_init(&bar[1], 1);
@@ -113,7 +262,7 @@ vq_kernel(const float* __restrict__ x, const float* __restrict__ cb, long long* 
         tmem_alloc(&tmem_base, 512);
         tmem_relinquish();
     }
-    const float* const xs = x + (long long)n * kE * T + t;
+    const float* const xs = x + (long long)n * kE * T + (number - n * T);
     float xx = 0.f;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
@@ -123,13 +272,13 @@ vq_kernel(const float* __restrict__ x, const float* __restrict__ cb, long long* 
             v[e] = in ? xs[(long long)(8 * q + e) * T] : 0.f;
             xx = fmaf(v[e], v[e], xx);
         }
-        if ((q >> 2) == half) put8(sa, kPartA, row, q, v);  // the two threads of a vector write half of its row each
+        if (q * kParts / 8 == part) put8(sa, kPartA, row, q, v);  // the threads of a vector write a share of its row each
     }
     const float xn = sqrtf(xx) * 1.0001f;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_base, lane0 = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (row >> 7) * kTile + half * 64;
+    const uint32_t tmem = tmem_base, lane0 = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (row >> 7) * kTile + part * kCols;
     const int tiles = (n_codes + kTile - 1) / kTile;
 
     auto make_tile = [&](int tile) {  // a quarter of a code: 16 channels
@@ -150,7 +299,7 @@ vq_kernel(const float* __restrict__ x, const float* __restrict__ cb, long long* 
         put8(sb + buf * 2 * kPartB, kPartB, r, 2 * seg, v[0]);
         put8(sb + buf * 2 * kPartB, kPartB, r, 2 * seg + 1, v[1]);
         if (!real) kk = INFINITY;
-        if (seg == 0) skk[buf][r] = kk;
+        if (seg == 0) skk[buf * kTile + r] = kk;
         const uint32_t most = __reduce_max_sync(0xffffffffu, __float_as_uint(kk < INFINITY ? kk : 0.f));
         if (lane == 0) atomicMax(&most_kk, most);
         fence_proxy_async_smem();
@@ -158,7 +307,7 @@ vq_kernel(const float* __restrict__ x, const float* __restrict__ cb, long long* 
     auto multiply = [&](int tile) {  // one thread
         const uint32_t b = smem_u32(sb) + (tile & 1) * 2 * kPartB;
 #pragma unroll
-        for (int rt = 0; rt < 2; ++rt) {
+        for (int rt = 0; rt < ROWS / 128; ++rt) {
             const uint32_t a = smem_u32(sa) + rt * 128 * 128, d = tmem + (tile & 1) * 256 + rt * kTile;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
@@ -177,6 +326,7 @@ vq_kernel(const float* __restrict__ x, const float* __restrict__ cb, long long* 
                  reinterpret_cast<int*>(list + 2 * kList * kThreads) + tid, 0, false};
     make_tile(0);
     __syncthreads();
+    bool many = false;
     for (int tile = 0; tile < tiles; ++tile) {
         const int buf = tile & 1;
         if (tid == 0) {
@@ -192,12 +342,12 @@ vq_kernel(const float* __restrict__ x, const float* __restrict__ cb, long long* 
         mbar_wait(&bar[buf], (tile >> 1) & 1);
         tc_fence_after();
 #pragma unroll 1
-        for (int c = 0; c < 64; c += 32) {
+        for (int c = 0; c < kCols; c += 32) {
             uint32_t u[32];
             tmem_ld_32x32b_x32(lane0 + buf * 256 + c, u);
             tmem_ld_wait();
             float s[32], m = INFINITY;
-            const float4* kk = reinterpret_cast<const float4*>(&skk[buf][half * 64 + c]);
+            const float4* kk = reinterpret_cast<const float4*>(&skk[buf * kTile + part * kCols + c]);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const float4 k4 = kk[i];
@@ -210,17 +360,30 @@ vq_kernel(const float* __restrict__ x, const float* __restrict__ cb, long long* 
                 uint32_t mask = 0u;
 #pragma unroll
                 for (int i = 0; i < 32; ++i) mask |= s[i] - eps <= least ? 1u << i : 0u;
-                const int run = tile * 4 + half * 2 + (c >> 5), real = n_codes - 32 * run;  // behind the last code: none
+                const int run = tile * 4 + ((part * kCols + c) >> 5), real = n_codes - 32 * run;  // behind the last code: none
                 if (real < 32) mask &= (1u << max(real, 0)) - 1u;
                 note(runs, m - eps, mask, run, least);
             }
         }
         tc_fence_before();
-        __syncthreads();  // sums read, next tile's rows written
+        if (__syncthreads_or(live && runs.all)) {  // sums read, next tile's rows written
+            many = true;
+            break;
+        }
     }
-    s_least[half][row] = least;
+    s_least[part][row] = least;
     __syncthreads();
-    least = fminf(least, s_least[half ^ 1][row]);
+#pragma unroll
+    for (int i = 0; i < kParts; ++i) least = fminf(least, s_least[i][row]);
+    int candidates = 0;
+    for (int i = 0; i < runs.n; ++i)
+        if (runs.low[i * kThreads] <= least) candidates += __popc(runs.mask[i * kThreads]);
+    if (__syncthreads_or(many || (live && candidates > n_codes / 16 + 4))) {
+        if (warp == 0) tmem_dealloc(tmem, 512);
+        float* sx = reinterpret_cast<float*>(sa);
+        walk_all_called<ROWS, kThreads>(sx, sx + kE * ROWS, skk, s_dist[0], x, cb, codes, v0, vectors, T, n_codes);
+        return;
+    }
     float best = INFINITY;
     int code = 0;
     if (live) {
@@ -246,46 +409,57 @@ vq_kernel(const float* __restrict__ x, const float* __restrict__ cb, long long* 
                 code = j;
             }
         };
-        int i = 0, next = half * 64;  // runs noted: the next one; all codes: the next one of this half of every tile
+        int i = 0, base = 0;
         uint32_t mask = 0u;
-        int base = 0;
-        for (;;) {  // one place that walks, however the next code is found
-            int j;
-            if (runs.all) {
-                if (next >= n_codes) break;
-                j = next;
-                next += (next & 63) == 63 ? 65 : 1;
-            } else {
-                while (mask == 0u && i < runs.n) {
-                    if (runs.low[i * kThreads] <= least) mask = runs.mask[i * kThreads], base = 32 * runs.run[i * kThreads];
-                    ++i;
-                }
-                if (mask == 0u) break;
-                j = base + __ffs(mask) - 1;
-                mask &= mask - 1u;
+        for (;;) {  // one place that walks, whichever run the next candidate is of
+            while (mask == 0u && i < runs.n) {
+                if (runs.low[i * kThreads] <= least) mask = runs.mask[i * kThreads], base = 32 * runs.run[i * kThreads];
+                ++i;
             }
-            walk(j);
+            if (mask == 0u) break;
+            walk(base + __ffs(mask) - 1);
+            mask &= mask - 1u;
         }
     }
-    if (half) {
-        s_dist[row] = best;
-        s_code[row] = code;
+    if (part) {
+        s_dist[part][row] = best;
+        s_code[part][row] = code;
     }
     __syncthreads();
-    if (!half && in) {
-        const float d = s_dist[row];
-        const int j = s_code[row];
-        if (d < best || (d == best && d < INFINITY && j < code)) code = j;
-        codes[(long long)n * T + t] = code;
+    if (part == 0 && in) {
+#pragma unroll
+        for (int i = 1; i < kParts; ++i) {
+            const float d = s_dist[i][row];
+            const int j = s_code[i][row];
+            if (d < best || (d == best && d < INFINITY && j < code)) best = d, code = j;
+        }
+        codes[number] = code;
     }
     if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
+template <int ROWS>
+static cudaError_t launch(const float* x, const float* cb, long long* codes, int vectors, int T, int n_codes, cudaStream_t st) {
+    const cudaError_t e = cudaFuncSetAttribute(vq_kernel<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<ROWS>::kSmem);
+    if (e != cudaSuccess) return e;
+    vq_kernel<ROWS><<<(vectors + ROWS - 1) / ROWS, kThreads, Shape<ROWS>::kSmem, st>>>(x, cb, codes, vectors, T, n_codes);
+    return cudaGetLastError();
+}
+
 int encode(const float* x, const float* cb, long long* codes, int N, int T, int n_codes, cudaStream_t st) {
-    cudaError_t e = cudaFuncSetAttribute(vq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
-    if (e == cudaSuccess) {
-        vq_kernel<<<dim3((T + kRows - 1) / kRows, N), kThreads, kSmem, st>>>(x, cb, codes, T, n_codes);
-        e = cudaGetLastError();
+    if ((long long)N * T > 0x7fffffff - 256) return LLARK_EINVAL;  // 550 GB of vectors
+    const int vectors = N * T;
+    using W = Walk<kWalkRows, kWalkThreads>;
+    cudaError_t e;
+    if (vectors <= 148 * kWalkRows || n_codes <= 256) {
+        e = cudaFuncSetAttribute(walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, W::kBytes);
+        if (e == cudaSuccess) {
+            const int smem = n_codes > W::kCodes ? W::kBytes : W::kBytes - W::kTileFloats * 4;  // one tile has no next
+            walk_kernel<<<(vectors + kWalkRows - 1) / kWalkRows, kWalkThreads, smem, st>>>(x, cb, codes, vectors, T, n_codes);
+            e = cudaGetLastError();
+        }
+    } else {
+        e = vectors <= 148 * 128 ? launch<128>(x, cb, codes, vectors, T, n_codes, st) : launch<256>(x, cb, codes, vectors, T, n_codes, st);
     }
     if (e != cudaSuccess) {
         g_last_cuda_error = (int)e;
