@@ -293,37 +293,36 @@ layernorm_kernel(const float* __restrict__ x, const float* __restrict__ gamma, c
 }
 
 // ---------------------------------------------------------------------------------------------- prior input embedding
-// A block has a time step of all clips: its two additive rows are read once, and the clips' token rows are under way together. Bound by
-// memory: 2 clips x 8192 steps x 4800 (two additive tables of 157 MB, 315 MB written) 119 us, with a block per clip and step 160.
+// A block has a time step of up to K clips: its two additive rows are read once for them, and their token rows are under way together. Bound
+// by memory: 2 clips x 8192 steps x 4800 (two additive tables of 157 MB, 315 MB written) 124 us with K = 2, 166 with K = 1. K = 1 for one
+// clip, and where the tables stay in L2 anyway and blocks matter more: 64 clips x 16 steps 9 us (43 with all clips in a block).
+template <int K>
 __global__ void __launch_bounds__(256)
 jb_embed_kernel(const long long* __restrict__ codes, const float* __restrict__ emb,
                                 const float* __restrict__ y_cond, const float* __restrict__ pos_emb,
                                 const float* __restrict__ x_cond, float* __restrict__ out, int N, int T, int W) {
-    const int t = blockIdx.x;
+    const int t = blockIdx.x, n0 = blockIdx.y * K;
     const float* pe = pos_emb + (long long)t * W;
     const float* xc = x_cond + (long long)t * W;
-    constexpr int kClips = 4;
-    for (int n0 = 0; n0 < N; n0 += kClips) {
-        const float* src[kClips];
+    const float* src[K];
 #pragma unroll
-        for (int k = 0; k < kClips; ++k) {
-            const int n = min(n0 + k, N - 1);
-            src[k] = t == 0 ? y_cond : emb + codes[(long long)n * T + t - 1] * W;
-        }
-        for (int i = threadIdx.x * 4; i < W; i += blockDim.x * 4) {
-            const float4 b = *reinterpret_cast<const float4*>(pe + i);
-            const float4 c = *reinterpret_cast<const float4*>(xc + i);
-            float4 a[kClips];
+    for (int k = 0; k < K; ++k) {
+        const int n = min(n0 + k, N - 1);
+        src[k] = t == 0 ? y_cond : emb + codes[(long long)n * T + t - 1] * W;
+    }
+    for (int i = threadIdx.x * 4; i < W; i += blockDim.x * 4) {
+        const float4 b = *reinterpret_cast<const float4*>(pe + i);
+        const float4 c = *reinterpret_cast<const float4*>(xc + i);
+        float4 a[K];
 #pragma unroll
-            for (int k = 0; k < kClips; ++k)
-                if (n0 + k < N) a[k] = *reinterpret_cast<const float4*>(src[k] + i);
-            // reference order: (x_emb + pos_emb) + x_cond
+        for (int k = 0; k < K; ++k)
+            if (K == 1 || n0 + k < N) a[k] = *reinterpret_cast<const float4*>(src[k] + i);
+        // reference order: (x_emb + pos_emb) + x_cond
 #pragma unroll
-            for (int k = 0; k < kClips; ++k)
-                if (n0 + k < N)
-                    *reinterpret_cast<float4*>(out + ((long long)(n0 + k) * T + t) * W + i) = make_float4(
-                        (a[k].x + b.x) + c.x, (a[k].y + b.y) + c.y, (a[k].z + b.z) + c.z, (a[k].w + b.w) + c.w);
-        }
+        for (int k = 0; k < K; ++k)
+            if (K == 1 || n0 + k < N)
+                *reinterpret_cast<float4*>(out + ((long long)(n0 + k) * T + t) * W + i) = make_float4(
+                    (a[k].x + b.x) + c.x, (a[k].y + b.y) + c.y, (a[k].z + b.z) + c.z, (a[k].w + b.w) + c.w);
     }
 }
 
@@ -776,7 +775,11 @@ extern "C" int llark_jb_embed_tokens(const long long* codes, const float* emb, c
                                      const float* pos_emb, const float* x_cond, float* out, int N, int T, int W,
                                      cudaStream_t st) {
     if (N <= 0 || T <= 0 || (W & 3)) return LLARK_EINVAL;
-    jb_embed_kernel<<<T, 256, 0, st>>>(codes, emb, y_cond, pos_emb, x_cond, out, N, T, W);
+    const bool in_l2 = (long long)T * W * 8 <= 64LL << 20;
+    const int k = N == 1 || in_l2 ? 1 : N == 2 ? 2 : 4;
+    const dim3 grid(T, (N + k - 1) / k);
+    auto* kernel = k == 1 ? jb_embed_kernel<1> : k == 2 ? jb_embed_kernel<2> : jb_embed_kernel<4>;
+    kernel<<<grid, 256, 0, st>>>(codes, emb, y_cond, pos_emb, x_cond, out, N, T, W);
     return jb_check();
 }
 
