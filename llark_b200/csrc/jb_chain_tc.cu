@@ -21,9 +21,15 @@
 // new rows for the neighbours' products, and the groups' first products are issued one group after another, so that the first reads its
 // sums back and splits while the others' products run.
 //
+// An infinite number, or one whose first part rounds to infinity, leaves NaN in its other parts and so in all 32 sums of the rows that see it: the
+// first channel's sums of either convolution tell; weights and biases from 2^60 on are told by their staging. The windows that had some
+// are walked again in the end, block after block by FMAs in the order of the FMA kernel (relu(NaN) is 0 as there). Nothing but such numbers
+// gets there. What it cannot tell: single products beyond the largest number, of both signs in one sum, are NaN and not the first one's
+// infinity. (A look at all 32 channels for large numbers: 678 us where this takes 633.)
+//
 // What bounds it: a product of 128 rows takes 50 to 60 cycles whatever its N up to 96 (its A operand's 4 KB from shared memory; from TMEM
 // 85), 28 of them a group and block, and some 800 instructions a warp and block between them; 8700 cycles a block and window. Measured
-// on a B200, 4 clips x 524288 steps, dilations 1, 3, 9, 27: 664 us where four launches of one block took 1075; one block alone 184 to 201
+// on a B200, 4 clips x 524288 steps, dilations 1, 3, 9, 27: 633 us where four launches of one block took 1075; one block alone 181 to 198
 // (257). Error of the encoder against 64 bits 2.2e-6 (2.9e-6). Tried: both convolutions from shared memory, all groups in step: 820;
 // hidden rows in TMEM, all groups in step: 772; two windows of 256 steps side by side: 999; parts cut instead of rounded: 669.
 #include "common.cuh"
@@ -65,6 +71,7 @@ __device__ __forceinline__ uint32_t part2(float& a, float& b) {
 __device__ __forceinline__ uint4 part8(float (&v)[8]) {
     return make_uint4(part2(v[0], v[1]), part2(v[2], v[3]), part2(v[4], v[5]), part2(v[6], v[7]));
 }
+__device__ __forceinline__ bool too_large(float v) { return !(fabsf(v) < 1152921504606846976.f); }  // 2^60, or NaN
 // eight channels (q: which eight) of row r
 __device__ __forceinline__ void put8(unsigned char* region, int r, int q, float (&v)[8]) {
     unsigned char* p = region + r * 64 + ((q ^ ((r >> 1) & 3)) << 4);
@@ -73,10 +80,12 @@ __device__ __forceinline__ void put8(unsigned char* region, int r, int q, float 
 }
 // weights [32][32][TAPS] -> per tap 96 rows: first parts, second parts, third parts
 template <int TAPS>
-__device__ __forceinline__ void put_taps(unsigned char* dst, const float* __restrict__ w) {
+__device__ __forceinline__ bool put_taps(unsigned char* dst, const float* __restrict__ w) {  // true: one is too large
+    bool odd = false;
     for (int i = threadIdx.x; i < TAPS * 32 * 32; i += blockDim.x) {
         const int ci = i & 31, co = (i >> 5) & 31, tap = i >> 10;
         float v = w[(co * 32 + ci) * TAPS + tap];
+        odd |= too_large(v);
 #pragma unroll
         for (int part = 0; part < 3; ++part) {
             const __nv_bfloat16 h = __float2bfloat16_rn(v);
@@ -85,6 +94,7 @@ __device__ __forceinline__ void put_taps(unsigned char* dst, const float* __rest
             *reinterpret_cast<__nv_bfloat16*>(dst + tap * kTapBytes + row * 64 + (((ci >> 3) ^ ((row >> 1) & 3)) << 4) + (ci & 7) * 2) = h;
         }
     }
+    return odd;
 }
 // one tap: A rows from byte address a on (first part), weights at w, sums at d
 __device__ __forceinline__ void tap_products(uint32_t a, uint32_t w, uint32_t d, bool first) {
@@ -138,11 +148,48 @@ __device__ __forceinline__ void bias8(const float* b, float (&u)[8]) {
     u[0] = u0.x, u[1] = u0.y, u[2] = u0.z, u[3] = u0.w, u[4] = u1.x, u[5] = u1.y, u[6] = u1.z, u[7] = u1.w;
 }
 
+// A window by FMAs: bias first, channels outside, taps inside. A thread has a step, rows: [32][kWin].
+__device__ __noinline__ void window_by_fma(const ChainArgs& p, float* rows, int win) {
+    const int clip = win / p.windows_per_clip, i = threadIdx.x;
+    const int t = (win - clip * p.windows_per_clip) * (kWin - 2 * p.halo) - p.halo + i;
+    const bool in = t >= 0 && t < p.T;
+    const long long at = (long long)clip * 32 * p.T + t;
+    __syncthreads();  // the window before has been read
+    for (int c = 0; c < 32; ++c) rows[c * kWin + i] = in ? p.x[at + (long long)c * p.T] : 0.f;
+#pragma unroll 1
+    for (int b = 0; b < p.blocks; ++b) {
+        __syncthreads();
+        float h[32], o[32];
+        for (int c = 0; c < 32; ++c) {
+            float acc = p.b1[b][c];
+            for (int k = 0; k < 96; ++k) {
+                const int j = i + (k % 3 - 1) * p.dil[b];
+                acc = fmaf(p.w1[b][c * 96 + k], j >= 0 && j < kWin ? fmaxf(rows[k / 3 * kWin + j], 0.f) : 0.f, acc);
+            }
+            h[c] = fmaxf(acc, 0.f);
+        }
+        for (int c = 0; c < 32; ++c) {
+            float acc = p.b2[b][c];
+            for (int k = 0; k < 32; ++k) acc = fmaf(p.w2[b][c * 32 + k], h[k], acc);
+            o[c] = rows[c * kWin + i] + acc;
+        }
+        __syncthreads();  // the neighbours have read this row
+        for (int c = 0; c < 32; ++c) rows[c * kWin + i] = in ? o[c] : 0.f;
+    }
+    if (in && i >= p.halo && i < kWin - p.halo)
+        for (int c = 0; c < 32; ++c) p.y[at + (long long)c * p.T] = rows[c * kWin + i];
+}
+
+// Which of a CTA's windows are walked again: a bit each, the last bit for all from there on.
+__device__ __forceinline__ int bit_of(int win) { return min((win - (int)blockIdx.x) / (int)gridDim.x, 32 * 32 - 1); }
+__device__ __forceinline__ void again(uint32_t* odd, int win) { atomicOr(&odd[bit_of(win) >> 5], 1u << (bit_of(win) & 31)); }
+
 __global__ void __launch_bounds__(kWin, 1)
 chain_kernel(const __grid_constant__ ChainArgs p) {
     extern __shared__ unsigned char raw[];
     __shared__ uint64_t ready[4], done1[4], done2[4], turn[4];  // per group: rows written; first products done; second products done; first products on their way
     __shared__ uint32_t tmem_base;
+    __shared__ uint32_t odd[32];
     unsigned char* sa = raw + ((1024u - (smem_u32(raw) & 1023u)) & 1023u);
     unsigned char* sw = sa + 3 * kPart;
     float* sb = reinterpret_cast<float*>(sw + kMost * kBlockBytes);  // [block][b1 | b2]
@@ -160,19 +207,24 @@ chain_kernel(const __grid_constant__ ChainArgs p) {
         tmem_alloc(&tmem_base, 512);
         tmem_relinquish();
     }
+    bool every = false;
     for (int b = 0; b < p.blocks; ++b) {
-        put_taps<3>(sw + b * kBlockBytes, p.w1[b]);
-        put_taps<1>(sw + b * kBlockBytes + 3 * kTapBytes, p.w2[b]);
+        every |= put_taps<3>(sw + b * kBlockBytes, p.w1[b]);
+        every |= put_taps<1>(sw + b * kBlockBytes + 3 * kTapBytes, p.w2[b]);
         if (threadIdx.x < 32) {
-            sb[b * 64 + threadIdx.x] = p.b1[b][threadIdx.x];
-            sb[b * 64 + 32 + threadIdx.x] = p.b2[b][threadIdx.x];
+            const float u1 = p.b1[b][threadIdx.x], u2 = p.b2[b][threadIdx.x];
+            sb[b * 64 + threadIdx.x] = u1;
+            sb[b * 64 + 32 + threadIdx.x] = u2;
+            every |= too_large(u1) || too_large(u2);
         }
     }
     for (int i = threadIdx.x; i < 3 * kPart / 16; i += kWin) reinterpret_cast<uint4*>(sa)[i] = make_uint4(0u, 0u, 0u, 0u);
     fence_proxy_async_smem();
     tc_fence_before();
-    __syncthreads();
+    const uint32_t odd_from_the_start = __syncthreads_or(every) ? 0xffffffffu : 0u;
     tc_fence_after();
+    if (threadIdx.x < 32) odd[threadIdx.x] = odd_from_the_start;
+    __syncthreads();
     const uint32_t tmem = tmem_base + g * 128, lane0 = tmem + ((uint32_t)(warp * 32) << 16);
     const int row = kSpare + threadIdx.x, stride = kWin - 2 * p.halo;
     auto where = [&](int win, int& clip, int& t) {
@@ -247,7 +299,11 @@ chain_kernel(const __grid_constant__ ChainArgs p) {
                 bias8(bias + 8 * q, u);
                 tmem_ld_wait();
 #pragma unroll
-                for (int e = 0; e < 8; ++e) v[e] = fmaxf((v[e] + s[8 * q + e]) + u[e], 0.f);
+                for (int e = 0; e < 8; ++e) {
+                    v[e] = (v[e] + s[8 * q + e]) + u[e];
+                    if (q == 0 && e == 0 && !(fabsf(v[0]) <= 3.402823466e38f)) again(odd, win);
+                    v[e] = fmaxf(v[e], 0.f);
+                }
 #pragma unroll
                 for (int part = 0; part < 3; ++part) tmem_st_x4(lane0 + kHidden + 16 * part + 4 * q, part8(v));
             }
@@ -270,7 +326,11 @@ chain_kernel(const __grid_constant__ ChainArgs p) {
                 bias8(bias + 32 + 8 * q, u);
                 tmem_ld_wait();
 #pragma unroll
-                for (int e = 0; e < 8; ++e) x[8 * q + e] += (c0[e] + c1[e]) + u[e];
+                for (int e = 0; e < 8; ++e) {
+                    const float o = (c0[e] + c1[e]) + u[e];
+                    if (q == 0 && e == 0 && !(fabsf(o) <= 3.402823466e38f)) again(odd, win);
+                    x[8 * q + e] += o;
+                }
             }
         }
         if (in && (int)threadIdx.x >= p.halo && (int)threadIdx.x < kWin - p.halo) {
@@ -282,6 +342,8 @@ chain_kernel(const __grid_constant__ ChainArgs p) {
     tc_fence_before();
     __syncthreads();
     if (threadIdx.x < 32) tmem_dealloc(tmem_base, 512);
+    for (int win = blockIdx.x; win < p.windows; win += gridDim.x)
+        if (odd[bit_of(win) >> 5] >> (bit_of(win) & 31) & 1u) window_by_fma(p, reinterpret_cast<float*>(sa), win);
 }
 
 int chain_length(const int* dil, int n) {

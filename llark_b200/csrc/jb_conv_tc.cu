@@ -15,7 +15,7 @@
 //
 //   res block   y = x + W2 relu(W1 (*dilation d, 3 taps) relu(x) + b1) + b2, both convolutions of a tile in one visit: the second's A
 //               operand is the first's result, written by the thread that owns the row. For dilations from 33 on: up to 32
-//               jb_chain_tc.cu is ahead (184 to 201 us at the size below)
+//               jb_chain_tc.cu is ahead (181 to 198 us at the size below)
 //   others      taps 4 stride 2 (32 or 64 channels in, 32 out), taps 3 (32 in, 64 out)
 //
 // What bounds it: the latency of load, split, product and read-back of a tile, hidden only by the other groups (a res block reads and
@@ -68,15 +68,19 @@ __device__ __forceinline__ void put_row(unsigned char* region, int lo_at, int r,
 }
 // weights [COUT][NCI * 32][TAPS] -> per (32 channels, tap): hi rows [COUT][32], then lo rows; odd taps the other way round
 template <int TAPS, int NCI, int COUT>
-__device__ __forceinline__ void put_weights(unsigned char* dst, const float* __restrict__ w) {
+__device__ __forceinline__ bool put_weights(unsigned char* dst, const float* __restrict__ w) {  // true: one is 2^60 or more, or NaN
+    bool large = false;
     for (int i = threadIdx.x; i < TAPS * NCI * COUT * 32; i += blockDim.x) {
         const int ci = i & 31, co = (i >> 5) % COUT, kb = i / (32 * COUT), tap = kb % TAPS, cb = kb / TAPS;
         float hi, lo;
-        split(w[((long long)co * (NCI * 32) + cb * 32 + ci) * TAPS + tap], hi, lo);
+        const float v = w[((long long)co * (NCI * 32) + cb * 32 + ci) * TAPS + tap];
+        large |= !(fabsf(v) < 1152921504606846976.f);
+        split(v, hi, lo);
         unsigned char* p = dst + kb * (2 * COUT * 128) + co * 128 + (((ci >> 2) ^ (co & 7)) << 4) + (ci & 3) * 4;
         *reinterpret_cast<float*>(p) = tap & 1 ? lo : hi;
         *reinterpret_cast<float*>(p + COUT * 128) = tap & 1 ? hi : lo;
     }
+    return large;
 }
 // 32 channels of a tap. SIDE 0: hi hi into COUT columns from d on, hi lo + lo hi into the COUT columns behind them; SIDE 1: the weights'
 // lo rows come first, hi hi goes into the COUT columns behind the shared ones. first: hi hi begins a chain; first_lo: the shared one.
@@ -116,6 +120,28 @@ __device__ __noinline__ void step_by_fma(const float* x, const float* w, const f
     }
 }
 
+// The same for a res block's step, all of it: relu(NaN) = 0 as everywhere in them.
+__device__ __noinline__ void res_step_by_fma(const Args& p, const float* x, int t, float (&o)[32]) {
+    float h[32];
+#pragma unroll 1
+    for (int c = 0; c < 32; ++c) {
+        float acc = p.b1[c];
+#pragma unroll 1
+        for (int i = 0; i < 96; ++i) {
+            const int at = t + (i % 3 - 1) * p.dil;
+            acc = fmaf(p.w1[c * 96 + i], at >= 0 && at < p.T ? fmaxf(x[(long long)(i / 3) * p.T + at], 0.f) : 0.f, acc);
+        }
+        h[c] = fmaxf(acc, 0.f);
+    }
+#pragma unroll 1
+    for (int c = 0; c < 32; ++c) {
+        float acc = p.b2[c];
+#pragma unroll 1
+        for (int i = 0; i < 32; ++i) acc = fmaf(p.w2[c * 32 + i], h[i], acc);
+        o[c] = x[(long long)c * p.T + t] + acc;
+    }
+}
+
 // A tile's input rows: stride 1: one region, row r is step t0 - dil + r; stride 2: even steps (row r is step 2 (t0 + r)), then odd ones
 // (row r is step 2 (t0 + r) - 1). Shared memory, 1024-byte aligned: W1 | W2 (res block) | per group: the regions, hi rows then lo rows.
 template <int TAPS, int STRIDE, int NCI, int COUT, bool RES, int NG>
@@ -140,13 +166,16 @@ conv_kernel(const Args p) {
         tmem_alloc(&tmem_base, kCols);
         tmem_relinquish();
     }
-    put_weights<TAPS, NCI, COUT>(sw1, p.w1);
-    if (RES) put_weights<1, 1, 32>(sw2, p.w2);
+    bool every = put_weights<TAPS, NCI, COUT>(sw1, p.w1);  // res block: all steps by FMAs
+    if (RES) every |= put_weights<1, 1, 32>(sw2, p.w2);
     for (int i = threadIdx.x; i < COUT; i += NG * TT) sb[i] = p.b1[i];
     if (RES && threadIdx.x < 32) sb[COUT + threadIdx.x] = p.b2[threadIdx.x];
     fence_proxy_async_smem();
     tc_fence_before();
-    __syncthreads();
+    if (RES)
+        every = __syncthreads_or(every);
+    else
+        __syncthreads();
     tc_fence_after();
     // a group's columns: hi hi of the even taps, the mixed products, hi hi of the odd taps; the second convolution's (res block) from 96 on
     const uint32_t tmem = tmem_base + grp * kGroup, lane0 = tmem + ((uint32_t)(warp * 32) << 16);
@@ -256,6 +285,7 @@ conv_kernel(const Args p) {
             read_sums(0, h);
 #pragma unroll
             for (int c = 0; c < 32; ++c) h[c] += sb[c];
+            const float first = h[0];  // a row that does not split leaves NaN in all channels, so one tells
             put_row<true>(sa, lo_at, tid, h);
             fence_proxy_async_smem();
             tc_fence_before();
@@ -272,10 +302,19 @@ conv_kernel(const Args p) {
             tmem_ld_32x32b_x32(lane0 + 96, a);
             tmem_ld_32x32b_x32(lane0 + 128, b);
             tmem_ld_wait();
-            if (t < p.To)
+            const float second = __uint_as_float(a[0]) + __uint_as_float(b[0]);
+            if (!(fabsf(first) <= 3.402823466e38f) || !(fabsf(second) <= 3.402823466e38f) || every) {
+                if (t < p.To) {
+                    float f[32];
+                    res_step_by_fma(p, p.x + (long long)clip * CIN * p.T, t, f);
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) out[(long long)c * p.To] = f[c];
+                }
+            } else if (t < p.To) {
 #pragma unroll
                 for (int c = 0; c < 32; ++c)
                     out[(long long)c * p.To] = xc[c] + ((__uint_as_float(a[c]) + __uint_as_float(b[c])) + sb[COUT + c]);
+            }
         } else {
 #pragma unroll
             for (int c0 = 0; c0 < COUT; c0 += 32) {

@@ -312,6 +312,37 @@ def test_values_that_do_not_split_come_out_where_conv1d_puts_them(kind, c_in, ba
         assert torch.equal(_by_fma(op, xc, w.cuda(), b.cuda()).cpu()[big], got[big])
 
 
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf"), 3.4e38, -3.4027e38, 2e25])
+@pytest.mark.parametrize("dils", [(1, 3, 9, 27), (27, 1), (3,), (40, 1), (81,)])
+@pytest.mark.parametrize("where", ["values", "weights", "bias"])
+def test_res_blocks_with_values_that_do_not_split(dils, where, bad):
+    """NaN, infinities and numbers whose sums may pass the largest one, among the values, the weights and the biases: the same steps are
+    infinite and NaN as with the FMA kernels, block after block (relu(NaN) is 0 in both), and all others differ by roundings: two ways of 128
+    products in a block, 1e-5 of what a step holds."""
+    from llark_b200 import ops
+
+    g = torch.Generator().manual_seed(len(dils))
+    T = 1200
+    x = torch.randn(2, 32, T, generator=g)
+    blocks = [[torch.randn(32, 32, 3, generator=g) / math.sqrt(96), torch.randn(32, generator=g) * 0.1,
+               torch.randn(32, 32, 1, generator=g) / math.sqrt(32), torch.randn(32, generator=g) * 0.1] for _ in dils]
+    if where == "values":
+        x[0, 5, 0], x[0, 7, 431], x[1, 31, T - 1] = bad, bad, bad
+    elif where == "weights":
+        blocks[0][0][3, 4, 1] = bad
+    else:
+        blocks[0][1][9] = bad
+    blocks, x = [tuple(t.cuda() for t in b) for b in blocks], x.cuda()
+    got, want = ops.jb_resblocks(x, blocks, dils), _by_fma(ops.jb_resblocks, x, blocks, dils)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    assert torch.equal(got[got.isinf()], want[want.isinf()])
+    ok = want.isfinite()
+    size = torch.where(ok, want.abs(), 0).amax(1, keepdim=True)  # of a step: its channels are sums of the same numbers
+    assert ((got - want).abs() <= 1e-5 * (1 + size))[ok].all()
+    if where == "values" and bad == float("inf"):
+        assert not want.isfinite()[0, :, 431 - dils[0]].all()  # the neighbours see it
+
+
 def test_a_nan_sample_stays_nan_through_the_encoder():
     """From the second level on the activations' NaN is the one the GPU's arithmetic gives; relu(NaN) is 0 in the res blocks (fmaxf), so
     the latents that see it through the residual sums are NaN, with either kind of kernel."""
