@@ -26,6 +26,10 @@ namespace llark {
 extern thread_local int g_last_cuda_error;
 int tensor_map_2d(CUtensorMap* out, const void* ptr, long long inner, long long outer, long long ld, int box_inner,
                   int box_outer, int elem_bytes);  // gemm_tcgen05.cu (cached cuTensorMapEncodeTiled, 128 B swizzle)
+// The same over samples: loads past a sample's end bring zeros and not the next sample's rows, whose numbers, if they are not finite, would be
+// NaN after the product with a probability of 0.
+int tensor_map_batches(CUtensorMap* out, const void* ptr, long long inner, long long outer, long long ld, int batches, int box_inner,
+                       int box_outer, int elem_bytes);
 
 // This file is also compiled a second time by attention_tc_alibi.cu with LLARK_ATC_ALIBI defined: same kernels with an
 // ALiBi bias slope_h * key added to the scaled scores (MPT variant, no RoPE involved). Without the macro the
@@ -157,19 +161,18 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const unsigned ch
     if (warp == 0) {
         if (lane == 0) {
             // ===================== TMA producer =====================
-            const int row0 = b * S;
             const int cq = h * HD, ck = NH * HD + h * HD, cv = 2 * NH * HD + h * HD;
             mbar_arrive_expect_tx(q_full, Q_BYTES);
             for (int c = 0; c < 2; ++c)
                 for (int rh = 0; rh < 2; ++rh)
-                    tma_load_2d(sQ + c * (BQ * 128) + rh * (64 * 128), &tm_qkv, q_full, cq + c * 64, row0 + q0 + rh * 64);
+                    tma_load_3d(sQ + c * (BQ * 128) + rh * (64 * 128), &tm_qkv, q_full, cq + c * 64, q0 + rh * 64, b);
             Ring r;
             auto load_tile = [&](int col, int j) {
                 mbar_wait(&kv_empty[r.slot], r.phase ^ 1);
                 uint8_t* dst = sKV + r.slot * KV_BYTES;
                 mbar_arrive_expect_tx(&kv_full[r.slot], KV_BYTES);
-                tma_load_2d(dst, &tm_qkv, &kv_full[r.slot], col, row0 + j * BK);
-                tma_load_2d(dst + BK * 128, &tm_qkv, &kv_full[r.slot], col + 64, row0 + j * BK);
+                tma_load_3d(dst, &tm_qkv, &kv_full[r.slot], col, j * BK, b);
+                tma_load_3d(dst + BK * 128, &tm_qkv, &kv_full[r.slot], col + 64, j * BK, b);
                 r.advance();
             };
             load_tile(ck, 0);
@@ -468,11 +471,11 @@ __device__ __forceinline__ void mma_pv_tmem(uint32_t tD, uint32_t tA, uint32_t b
             : "memory");
 }
 // a 128-row tile of 128 columns: two column chunks of 128 bytes, boxes of 64 rows
-__device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int col, int row) {
+__device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int col, int row, int b) {
 #pragma unroll
     for (int c = 0; c < 2; ++c)
 #pragma unroll
-        for (int rh = 0; rh < 2; ++rh) tma_load_2d(dst + c * (BQ * 128) + rh * (64 * 128), tm, bar, col + c * 64, row + rh * 64);
+        for (int rh = 0; rh < 2; ++rh) tma_load_3d(dst + c * (BQ * 128) + rh * (64 * 128), tm, bar, col + c * 64, row + rh * 64, b);
 }
 __device__ __forceinline__ void store_tile(const uint8_t* src, const CUtensorMap* tm, int col, int row) {
 #pragma unroll
@@ -647,8 +650,8 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
         fence_proxy_async_smem();
         // on their way while TMEM is allocated
         mbar_arrive_expect_tx(q_full, 2 * Q_BYTES);
-        load_tile(sQ, &tm_qkv, q_full, h * HD, b * S + q0);
-        load_tile(sdO, &tm_do, q_full, h * HD, b * S + q0);
+        load_tile(sQ, &tm_qkv, q_full, h * HD, q0, b);
+        load_tile(sdO, &tm_do, q_full, h * HD, q0, b);
     }
     if (warp == 1) {
         tmem_alloc(tmem_slot, 512);
@@ -661,16 +664,15 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
 
     if (warp == 0) {
         if (lane == 0) {
-            const int row0 = b * S;
             const int ck = NH * HD + h * HD, cv = 2 * NH * HD + h * HD;
             for (int j = 0; j < n_kv; ++j) {
                 const int ks = j % K_SLOTS, vs = j % V_SLOTS;
                 mbar_wait(&k_empty[ks], ((uint32_t)(j / K_SLOTS) & 1) ^ 1);
                 mbar_arrive_expect_tx(&k_full[ks], TILE_BYTES);
-                load_tile(sKt + ks * TILE_BYTES, &tm_qkv, &k_full[ks], ck, row0 + j * BQ);
+                load_tile(sKt + ks * TILE_BYTES, &tm_qkv, &k_full[ks], ck, j * BQ, b);
                 mbar_wait(&v_empty[vs], ((uint32_t)(j / V_SLOTS) & 1) ^ 1);
                 mbar_arrive_expect_tx(&v_full[vs], TILE_BYTES);
-                load_tile(sVt + vs * TILE_BYTES, &tm_qkv, &v_full[vs], cv, row0 + j * BQ);
+                load_tile(sVt + vs * TILE_BYTES, &tm_qkv, &v_full[vs], cv, j * BQ, b);
             }
         }
     } else if (warp == 1) {
@@ -861,8 +863,8 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
         fence_proxy_async_smem();
         // on their way while TMEM is allocated
         mbar_arrive_expect_tx(kv_full, 2 * Q_BYTES);
-        load_tile(sK, &tm_qkv, kv_full, NH * HD + h * HD, b * S + k0);
-        load_tile(sV, &tm_qkv, kv_full, 2 * NH * HD + h * HD, b * S + k0);
+        load_tile(sK, &tm_qkv, kv_full, NH * HD + h * HD, k0, b);
+        load_tile(sV, &tm_qkv, kv_full, 2 * NH * HD + h * HD, k0, b);
     }
     if (warp == 1) {
         tmem_alloc(tmem_slot, 512);
@@ -875,10 +877,9 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
 
     if (warp == 0) {
         if (lane == 0) {
-            const int row0 = b * S;
             const int cq = h * HD;
             for (int t = 0; t < n_it; ++t) {
-                const int qrow = row0 + (t0 + t) * BK;
+                const int qrow = (t0 + t) * BK;
 #pragma unroll
                 for (int which = 0; which < 2; ++which) {  // 0: Q_t, 1: dO_t
                     const int it = 2 * t + which, slot = ring_slot(it);
@@ -886,8 +887,8 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
                     uint8_t* dst = sRing + slot * KV_BYTES;
                     mbar_arrive_expect_tx(&ring_full[slot], KV_BYTES);
                     const CUtensorMap* tm = which ? &tm_do : &tm_qkv;
-                    tma_load_2d(dst, tm, &ring_full[slot], cq, qrow);
-                    tma_load_2d(dst + BK * 128, tm, &ring_full[slot], cq + 64, qrow);
+                    tma_load_3d(dst, tm, &ring_full[slot], cq, qrow, b);
+                    tma_load_3d(dst + BK * 128, tm, &ring_full[slot], cq + 64, qrow, b);
                 }
             }
         }
@@ -1051,7 +1052,7 @@ int LLARK_ATC_FWD_LAUNCH(const void* qkv, const unsigned char* key_mask, void* o
     if (S > MAX_S || (long long)B * S > 0x7fffffffLL) return LLARK_EINVAL;
     CUtensorMap tm;
     const long long ld = 3LL * n_heads * HD;
-    int rc = tensor_map_2d(&tm, qkv, ld, (long long)B * S, ld, 64, 64, 2);
+    int rc = tensor_map_batches(&tm, qkv, ld, S, ld, B, 64, 64, 2);
     if (rc) return rc;
     static bool attr_set = false;
     if (!attr_set) {
@@ -1082,9 +1083,9 @@ int LLARK_ATC_BWD_LAUNCH(const void* qkv, const unsigned char* key_mask, const v
     if ((long long)B * S > 0x7fffffffLL || S > MAX_S) return LLARK_EINVAL;
     CUtensorMap tq, td;
     const long long ld = 3LL * n_heads * HD, ldo = (long long)n_heads * HD;
-    int rc = tensor_map_2d(&tq, qkv, ld, (long long)B * S, ld, 64, 64, 2);
+    int rc = tensor_map_batches(&tq, qkv, ld, S, ld, B, 64, 64, 2);
     if (rc) return rc;
-    rc = tensor_map_2d(&td, dout, ldo, (long long)B * S, ldo, 64, 64, 2);
+    rc = tensor_map_batches(&td, dout, ldo, S, ldo, B, 64, 64, 2);
     if (rc) return rc;
     CUtensorMap to;
     rc = tensor_map_2d(&to, dqkv, ld, (long long)B * S, ld, 64, 64, 2);

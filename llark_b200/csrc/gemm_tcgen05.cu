@@ -1183,7 +1183,7 @@ static int ensure_driver() {
 struct MapKey {
     const void* ptr;
     long long inner, outer, ld;
-    int box_inner, box_outer, elem;
+    int box_inner, box_outer, elem, batches;
     bool operator==(const MapKey& o) const { return memcmp(this, &o, sizeof(MapKey)) == 0; }
 };
 struct MapKeyHash {
@@ -1196,13 +1196,15 @@ struct MapKeyHash {
 };
 static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> g_map_cache;
 
-// 2-D tensor map over a row-major [outer][ld] array of which [outer][inner] is valid; 128 B swizzle.
+// 2-D tensor map over a row-major [outer][ld] array of which [outer][inner] is valid; 128 B swizzle. batches > 0: 3-D, that many of
+// them behind one another, boxes of one batch.
 static int get_tensor_map(CUtensorMap* out, const void* ptr, long long inner, long long outer, long long ld,
-                          int box_inner, int box_outer, int elem_bytes) {
+                          int box_inner, int box_outer, int elem_bytes, int batches = 0) {
     MapKey key;
     memset(&key, 0, sizeof(key));
     key.ptr = ptr; key.inner = inner; key.outer = outer; key.ld = ld;
     key.box_inner = box_inner; key.box_outer = box_outer; key.elem = elem_bytes;
+    key.batches = batches;
     {
         std::lock_guard<std::mutex> lk(g_mu);
         auto itf = g_map_cache.find(key);
@@ -1212,11 +1214,12 @@ static int get_tensor_map(CUtensorMap* out, const void* ptr, long long inner, lo
         }
     }
     if ((reinterpret_cast<uintptr_t>(ptr) & 15) != 0 || ((ld * elem_bytes) & 15) != 0) return LLARK_EINVAL;
-    cuuint64_t gdim[2] = {(cuuint64_t)inner, (cuuint64_t)outer};
-    cuuint64_t gstride[1] = {(cuuint64_t)(ld * elem_bytes)};
-    cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_outer};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = g_encode(out, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
+    cuuint64_t gdim[3] = {(cuuint64_t)inner, (cuuint64_t)outer, (cuuint64_t)batches};
+    cuuint64_t gstride[2] = {(cuuint64_t)(ld * elem_bytes), (cuuint64_t)(outer * ld * elem_bytes)};
+    cuuint32_t box[3] = {(cuuint32_t)box_inner, (cuuint32_t)box_outer, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = g_encode(out, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+                          batches ? 3 : 2,
                           const_cast<void*>(ptr), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1236,6 +1239,13 @@ int tensor_map_2d(CUtensorMap* out, const void* ptr, long long inner, long long 
     int rc = ensure_driver();
     if (rc) return rc;
     return get_tensor_map(out, ptr, inner, outer, ld, box_inner, box_outer, elem_bytes);
+}
+
+int tensor_map_batches(CUtensorMap* out, const void* ptr, long long inner, long long outer, long long ld, int batches, int box_inner,
+                       int box_outer, int elem_bytes) {
+    int rc = ensure_driver();
+    if (rc) return rc;
+    return get_tensor_map(out, ptr, inner, outer, ld, box_inner, box_outer, elem_bytes, batches);
 }
 
 // 4-D tensor map over a row-major [K][ld] array ([K][MN] valid, MN contiguous) that delivers a whole MN-major

@@ -423,8 +423,8 @@ def test_attention_fwd_bwd(B, S, NH, pad):
 @pytest.mark.parametrize("S", [1, 63, 65, 127, 128, 129, 191, 193, 321, 384])
 def test_attention_bwd_tiles_end_inside_and_between_samples(S):
     """One half of a tile of keys, one row of the next, whole tiles only: gradients of the middle one of three samples against autograd in
-    64 bits of the same bf16 inputs. dS and P pass through bf16 (2^-9 each, two roundings a product), as the bounds above have it. The
-    samples beside it get the same gradients whatever their neighbours hold: no tile reads or writes over its sample's end."""
+    64 bits of the same bf16 inputs. dS and P pass through bf16 (2^-9 each, two roundings a product), as the bounds above have it. Each
+    sample gets the gradients that it gets alone: no tile writes over its sample's end."""
     ops = _ops()
     torch.manual_seed(S)
     B, NH, D = 3, 2, 128
@@ -448,6 +448,27 @@ def test_attention_bwd_tiles_end_inside_and_between_samples(S):
         alone = ops.attn_bwd(qkv[one].contiguous(), None, out[one].contiguous(), dout[one].contiguous(),
                              lse.view(B, -1)[b].contiguous(), 1, S, NH, D)
         assert torch.equal(alone, got[one])
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("S,alibi", [(S, a) for S in (1, 63, 65, 100, 129, 191, 193, 330) for a in (False, True)] + [(4100, False)])
+def test_attention_of_a_sample_whose_neighbours_are_not_finite(S, alibi, bad):
+    """Tiles reach past a sample's end: what lies there is the next sample's and must not get in, not as 0 times NaN either."""
+    ops = _ops()
+    torch.manual_seed(S)
+    B, NH, D = 3, 1, 128
+    qkv = torch.randn(B * S, 3 * NH * D, device="cuda").to(BF16)
+    dout = (0.1 * torch.randn(B * S, NH * D, device="cuda")).to(BF16)
+    slopes = (torch.tensor([0.5], device="cuda"),) if alibi else ()
+    fwd, bwd = (ops.attn_alibi_fwd, ops.attn_alibi_bwd) if alibi else (ops.attn_fwd, ops.attn_bwd)
+    mid = slice(S, 2 * S)
+    want, wlse = fwd(qkv[mid].contiguous(), None, 1, S, NH, D, *slopes)
+    dwant = bwd(qkv[mid].contiguous(), None, want, dout[mid].contiguous(), wlse, 1, S, NH, D, *slopes)
+    qkv[:S], qkv[2 * S:], dout[:S], dout[2 * S:] = bad, bad, bad, bad
+    out, lse = fwd(qkv, None, B, S, NH, D, *slopes)
+    assert torch.equal(out[mid], want) and torch.equal(lse[1], wlse[0])
+    dgot = bwd(qkv, None, out, dout, lse, B, S, NH, D, *slopes)
+    assert torch.equal(dgot[mid], dwant) and want.isfinite().all() and dwant.isfinite().all()
 
 
 @pytest.mark.parametrize("B,S,NH,pad", [(2, 512, 4, True), (1, 200, 2, False), (1, 4160, 1, True)])
