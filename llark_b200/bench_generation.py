@@ -264,7 +264,7 @@ def op_table(records, ctx, peaks):
 
 KELUTAR_OPS = ["linear", "seq_embed", "seq_short_conv", "seq_add_rmsnorm", "seq_rmsnorm_rows", "seq_relu2",
                "seq_qk_headnorm", "seq_swa_attn", "seq_kv_ring_write", "seq_glr_scan", "seq_head_rmsnorm"]
-LLAMA_OPS = ["gemm", "rmsnorm_fwd", "rope_", "attn_fwd", "attn_decode_packed", "swiglu_fwd", "embed_splice_fwd"]
+LLAMA_OPS = ["gemm", "rmsnorm_fwd", "rope_", "attn_fwd", "attn_decode_packed", "swiglu_fwd", "embed_splice_fwd", "decode_layers"]
 
 
 GOLAVIK_OPS = ["linear", "linear_w32", "seq_embed", "seq_short_conv", "seq_group_rmsnorm", "seq_residual_combine",

@@ -18,7 +18,7 @@ import os
 import torch
 
 from . import ops
-from .ops import LINEAR_FEW_MAX, DecodeLayer, decode_layers
+from .ops import LINEAR_FEW_MAX, DecodeLayer
 
 BF16 = torch.bfloat16
 _ALIGN = 128  # elements (256 B): keeps every view 16-byte aligned for TMA and fused views gap-free
@@ -502,9 +502,9 @@ class LlamaEngine:
         cache.lens.fill_(t + 1)  # the cache's own record, which attn_decode reads; the form below takes t
         few = B <= LINEAR_FEW_MAX and H % 8 == 0 and I % 8 == 0  # gate times up in the product's epilogue
         rstd = torch.empty(B, device=dev, dtype=torch.float32)
-        native = few and x.is_cuda and self.fuse_epilogues and D == 128 and ops.GEMM_PROFILE is None
+        native = few and self.fuse_epilogues and D == 128 and ops.GEMM_PROFILE is None
         if native:  # the loop below, its launches issued by one call
-            decode_layers(flat.decode_table(L, H, I, cache.k, cache.v), x, cos_t, sin_t, t, cache.s_max, I, NH, eps, rstd)
+            ops.decode_layers(flat.decode_table(L, H, I, cache.k, cache.v), x, cos_t, sin_t, t, cache.s_max, I, NH, eps, rstd)
         for l in range(0 if native else L):
             pfx = f"model.layers.{l}."
             Wqkv = flat.pview(pfx + "self_attn.q_proj.weight", (3 * H, H), span=3)

@@ -21,7 +21,6 @@ from types import SimpleNamespace
 import torch
 
 from llark_b200 import ops
-from llark_b200.ops import jb_resblocks
 
 BF16 = torch.bfloat16
 
@@ -100,11 +99,7 @@ class JukeboxVQVAE:
                 h = ops.jb_conv_down(h, w[f"enc.{b}.down.{i}.w"], w[f"enc.{b}.down.{i}.b"])
                 blocks = [tuple(w[f"enc.{b}.res.{i}.{d}.{n}"] for n in ("w1", "b1", "w2", "b2")) for d in range(cfg.depth)]
                 dilations = [cfg.dilation_growth_rate ** d for d in range(cfg.depth)]
-                if h.is_cuda:
-                    h = jb_resblocks(h, blocks, dilations)
-                else:
-                    for blk, dil in zip(blocks, dilations):
-                        h = ops.jb_resblock(h, *blk, dil)
+                h = ops.jb_resblocks(h, blocks, dilations)
             h = ops.jb_conv_k3(h, w[f"enc.{b}.proj.w"], w[f"enc.{b}.proj.b"])
         return h
 

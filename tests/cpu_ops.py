@@ -4,6 +4,7 @@ flat-bucket views, the order of the launches, splice bookkeeping, the KV-cache i
 trick of the decode step -- can be exercised by the CPU test suite, which has no GPU. The product never imports this
 module (tests/test_dist_cpu.py::test_no_cpu_fallback); the CUDA kernels themselves are tested in the `-m gpu` suite.
 Arithmetic: fp32 math on bf16 tensors, rounded to bf16 where the kernels round."""
+import ctypes
 import math
 
 import torch
@@ -141,6 +142,21 @@ def attn_decode_packed(qkv, k_cache, v_cache, pos, n_heads, head_dim, out=None):
     k_cache[:, pos].copy_(qkv[:, H:2 * H])
     v_cache[:, pos].copy_(qkv[:, 2 * H:])
     return attn_decode(qkv[:, :H], k_cache, v_cache, torch.full((B,), pos + 1), n_heads, head_dim)
+
+
+def _at(address, *shape):
+    n = 2 * math.prod(shape)
+    return torch.frombuffer((ctypes.c_char * n).from_address(address), dtype=BF16).view(shape)
+
+
+def decode_layers(layers, x, cos, sin, pos, s_max, inner, n_heads, eps, rstd):
+    B, H = x.shape
+    for w in layers:
+        qkv = gemm(rmsnorm_fwd(x, _at(w.norm1, H), eps, rstd=rstd), _at(w.qkv, 3 * H, H), rope=(cos, sin, 1, 2 * H))
+        k, v = _at(w.k, B, s_max, H), _at(w.v, B, s_max, H)
+        mid = gemm(attn_decode_packed(qkv, k, v, pos, n_heads, H // n_heads), _at(w.o, H, H), residual=x)
+        act = swiglu_fwd(gemm(rmsnorm_fwd(mid, _at(w.norm2, H), eps, rstd=rstd), _at(w.gate_up, 2 * inner, H)))
+        x.copy_(gemm(act, _at(w.down, H, inner), residual=mid))
 
 
 def swiglu_fwd(gu, act=None):
@@ -329,6 +345,12 @@ def jb_conv_down(x, w, b):
 def jb_resblock(x, w1, b1, w2, b2, dilation):
     h = _F.conv1d(torch.relu(x), w1, b1, padding=dilation, dilation=dilation)
     return x + _F.conv1d(torch.relu(h), w2, b2)
+
+
+def jb_resblocks(x, blocks, dilations):
+    for b, d in zip(blocks, dilations):
+        x = jb_resblock(x, *b, d)
+    return x
 
 
 def jb_conv_k3(x, w, b):
