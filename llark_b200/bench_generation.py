@@ -119,13 +119,16 @@ class OpTimer:
     """Wraps the named functions of llark_b200.ops with CUDA-event brackets while active. Bytes and FLOPs are counted at the
     call, so that the records keep no tensor alive (a step that outgrows the allocator's pool would be timed with it)."""
 
-    def __init__(self, names, ctx=None):
+    def __init__(self, names, ctx=None, engine=None):
+        """engine: its decode steps go op by op meanwhile, and not by one call for all layers."""
         from llark_b200 import ops
 
-        self.ctx = ctx or {}
+        self.ctx, self.engine = ctx or {}, engine
         self.ops, self.names, self.saved, self.records, self.depth = ops, names, {}, [], 0
 
     def __enter__(self):
+        if self.engine is not None:
+            self.engine.fuse_calls = False
         for n in self.names:
             f = getattr(self.ops, n)
             self.saved[n] = f
@@ -151,6 +154,8 @@ class OpTimer:
     def __exit__(self, *exc):
         for n, f in self.saved.items():
             setattr(self.ops, n, f)
+        if self.engine is not None:
+            self.engine.fuse_calls = True
         torch.cuda.synchronize()
 
 
@@ -960,7 +965,7 @@ def bench_size(name, width, layers, heads, dim, window, ff, vocab, peaks, steps,
         out["decode"]["llama_b%d_ms" % B] = round(ms, 3)
         if B == decode_batches[-1] or B == 8:
             for _ in range(2):
-                with OpTimer(LLAMA_OPS, {"context": context}) as t:
+                with OpTimer(LLAMA_OPS, {"context": context}, le) as t:
                     l_step()
             out["decode"]["llama_b%d_ops" % B] = op_table(t.records, {"context": context}, peaks)
     del lm, le, lc

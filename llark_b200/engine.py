@@ -236,6 +236,7 @@ class LlamaEngine:
         # RoPE and SwiGLU-backward fused into GEMM epilogues (llark_gemm_ex); LLARK_FUSE_EPILOGUES=0 keeps the
         # separate llark_rope / llark_swiglu_bwd kernels (same results bit for bit)
         self.fuse_epilogues = os.environ.get("LLARK_FUSE_EPILOGUES", "1") != "0"
+        self.fuse_calls = True  # a decode step's layers issued by one call; False: op by op, to time the ops
         # Activation recompute (the reference's --gradient_checkpointing True, m2t/models/llamav2.py:241,255-257):
         # "auto" = only when the model's gradient_checkpointing flag is set AND the saved activations of the step would
         # not fit comfortably in free HBM (a 7B step at S=512, B=16 keeps 35 GB and does not need it); "1" / "0" force it.
@@ -502,7 +503,7 @@ class LlamaEngine:
         cache.lens.fill_(t + 1)  # the cache's own record, which attn_decode reads; the form below takes t
         few = B <= LINEAR_FEW_MAX and H % 8 == 0 and I % 8 == 0  # gate times up in the product's epilogue
         rstd = torch.empty(B, device=dev, dtype=torch.float32)
-        native = few and self.fuse_epilogues and D == 128 and ops.GEMM_PROFILE is None
+        native = few and self.fuse_epilogues and self.fuse_calls and D == 128 and ops.GEMM_PROFILE is None
         if native:  # the loop below, its launches issued by one call
             ops.decode_layers(flat.decode_table(L, H, I, cache.k, cache.v), x, cos_t, sin_t, t, cache.s_max, I, NH, eps, rstd)
         for l in range(0 if native else L):

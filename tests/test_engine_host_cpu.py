@@ -100,6 +100,41 @@ def test_generate_cacheless_and_kv_cache_agree(cpu_engine, monkeypatch):
         model._engine.prefill(torch.zeros((1, 300), dtype=torch.int64), None, cache)
 
 
+def test_decode_step_by_one_call_and_op_by_op(cpu_engine, monkeypatch):
+    """The layers issued by one call and the ops one by one, which is what the generation benchmark's tables of ops time: the same logits and
+    caches, every op of every layer in the table."""
+    import collections
+
+    import cpu_ops
+    from llark_b200 import bench_generation as bench
+    from oracle.make_golden_generation import gen_inputs
+
+    cfg, params, ids, enc = gen_inputs()
+    model = _build(cfg, params)
+    out = model(input_ids=ids, audio_encodings=enc, use_cache=True)
+    engine, cache, nxt = model._engine, out.past_key_values, ids[:, -1:]
+    at = cache.length
+    called = collections.Counter()
+    real = cpu_ops.decode_layers
+    monkeypatch.setattr(cpu_ops, "decode_layers", lambda *a: called.update(["decode_layers"]) or real(*a))
+    one = engine.decode_step(nxt, cache)
+    keys = [k[:, at].clone() for k in cache.k]
+    assert called["decode_layers"] == 1 and len(keys) == cfg.num_layers
+    cache.length = at
+    event = type("Event", (), {"__init__": lambda self, **k: None, "record": lambda self: None})
+    monkeypatch.setattr(torch.cuda, "Event", event)
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda: None)
+    monkeypatch.setattr(cpu_ops, "gemm", lambda a, b, _f=cpu_ops.gemm, swiglu=False, **k: cpu_ops.swiglu_fwd(_f(a, b, **k)) if swiglu else _f(a, b, **k))
+    monkeypatch.setattr(bench, "_op_work", lambda *a: (0, 0.0))
+    timer = bench.OpTimer(["gemm", "rmsnorm_fwd", "attn_decode_packed", "decode_layers"], engine=engine)
+    timer.ops = cpu_ops
+    with timer:
+        two = engine.decode_step(nxt, cache)
+    table, L = collections.Counter(r[0] for r in timer.records), cfg.num_layers
+    assert table == {"gemm": 4 * L + 1, "rmsnorm_fwd": 2 * L + 1, "attn_decode_packed": L} and engine.fuse_calls
+    assert torch.equal(one, two) and all(torch.equal(k[:, at], w) for k, w in zip(cache.k, keys))
+
+
 def test_engine_backward_and_optimizer_host_logic(cpu_engine, monkeypatch):
     """Manual backward into the flat gradient bucket (views, overwrite-after-step vs accumulate, frozen lm_head, detached
     text rows) and the fused optimizer's bookkeeping, against the oracle's autograd gradients."""
