@@ -494,6 +494,8 @@ class LlamaEngine:
         t = cache.length
         if t >= cache.s_max:
             raise ValueError("KV cache is full")
+        if B != cache.B:
+            raise ValueError(f"{B} rows for a KV cache of {cache.B}")
         ids = last_ids.to(torch.int64).contiguous()
         table = flat.pview("model.embed_tokens.weight", (V, H))
         x = torch.empty((B, H), device=dev, dtype=BF16)

@@ -102,7 +102,7 @@ def test_generate_cacheless_and_kv_cache_agree(cpu_engine, monkeypatch):
 
 def test_decode_step_by_one_call_and_op_by_op(cpu_engine, monkeypatch):
     """The layers issued by one call and the ops one by one, which is what the generation benchmark's tables of ops time: the same logits and
-    caches, every op of every layer in the table."""
+    caches, every op of every layer in the table. Rows that the cache was not made for are refused before anything is written."""
     import collections
 
     import cpu_ops
@@ -133,6 +133,11 @@ def test_decode_step_by_one_call_and_op_by_op(cpu_engine, monkeypatch):
     table, L = collections.Counter(r[0] for r in timer.records), cfg.num_layers
     assert table == {"gemm": 4 * L + 1, "rmsnorm_fwd": 2 * L + 1, "attn_decode_packed": L} and engine.fuse_calls
     assert torch.equal(one, two) and all(torch.equal(k[:, at], w) for k, w in zip(cache.k, keys))
+    before = [k[:, : at + 1].clone() for k in cache.k]
+    cache.length = at
+    with pytest.raises(ValueError):
+        engine.decode_step(nxt.repeat(2, 1), cache)
+    assert cache.length == at and all(torch.equal(k[:, : at + 1], w) for k, w in zip(cache.k, before))
 
 
 def test_engine_backward_and_optimizer_host_logic(cpu_engine, monkeypatch):
