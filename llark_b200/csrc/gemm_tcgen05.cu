@@ -509,7 +509,7 @@ __device__ __forceinline__ void epi_staged_bf16(const GemmParams& p, long long r
 // p.staged == 1 (chosen on the host, llark_gemm_ex) selects the staged path where the epilogue is the longer leg: the SwiGLU
 // backward and, in the single-CTA kernel, a residual with an fp32 tile or a short K. Plain output at long K stays direct there: its
 // epilogue already hides behind the next tile's MMAs, and the staging patch's extra 256 KB of shared-memory traffic per tile slows
-// the operand pipeline by 3-8 % (profiles/r2c_epilogue_ab.md, profiles/r2k_epilogue_probe.md).
+// the operand pipeline by 3-8 % (in a training step and alone).
 template <int EPI, bool STAGED>
 __device__ __forceinline__ void epilogue_dispatch(const GemmParams& p, long long row0, long long m_end, int lane, int ncol0,
                                                   uint32_t taddr, float* stg, int c_lo, int c_hi) {
@@ -987,8 +987,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
         // ===================== TMA producers (both CTAs) =====================
         const bool do_a = warp == 0, do_b = split_prod ? (warp == 3) : true;
         // Everything that does not change per stage is computed out here: TMA issue from these two threads paces the
-        // MN-major kinds (profiles/r1_gemm_mn_major_investigation.md), and a build whose stage loop carried two integer
-        // divisions and a mapa lost 11 % on dgrad / wgrad (1403 -> 1248 TFLOP/s, same box, profiles/r1_session2_summary.md).
+        // MN-major kinds, and a build whose stage loop carried two integer divisions and a mapa lost 11 % on dgrad / wgrad
+        // (1403 -> 1248 TFLOP/s, one after the other on one GPU).
         const int mn_per_box = 128 / kElemBytes;
         const int box_bytes = elems_per_row * 128;
         const uint32_t bar0 = mapa_shared(smem_u32(&full_bar[0]), 0);  // the leader's full barriers
@@ -1554,13 +1554,13 @@ extern "C" int llark_gemm_ex(const void* A, int a_mn_major, long long lda, const
     p.seg_count = segs ? static_cast<const int*>(ep->b) : nullptr;
     if (segs) p.num_m_blocks = ep->i0;
     {
-        static int mode = -1;  // LLARK_GEMM_EPILOGUE = auto (default) | staged (single-CTA kernel) | direct
+        static int mode = -1;  // LLARK_GEMM_EPILOGUE = auto (default) | staged (through shared memory wherever there is such a form) | direct
         if (mode < 0) {
             const char* e = getenv("LLARK_GEMM_EPILOGUE");
             mode = (e && e[0] == 's') ? 1 : ((e && e[0] == 'd') ? 2 : 0);
         }
-        // auto, single-CTA kernel: staged where the isolated-GEMM probe (tools/gemm_epilogue_probe.py, profiles/r2k_epilogue_probe.md) and
-        // the in-step A/B (profiles/r2c_epilogue_ab.md) measured it faster -- the SwiGLU backward; any residual with an fp32
+        // auto, single-CTA kernel: staged where a product alone (tools/gemm_epilogue_probe.py) and whole steps measured it faster --
+        // the SwiGLU backward (in the CTA pair too); any residual with an fp32
         // tile (K = 1200: 17.8 vs 21.6 us per tile, K = 4800: 35.8 vs 36.2) or with a short K (bf16, K = 1200: 12.8 vs 16.5);
         // fp32 tiles without a residual only when K is short (K = 4800: direct 32.4 vs staged 35.1). Otherwise direct.
         const bool short_k = (long long)K * eb < 2400LL * 2;  // fewer than ~2400 bf16-equivalent K elements
@@ -1570,7 +1570,7 @@ extern "C" int llark_gemm_ex(const void* A, int a_mn_major, long long lda, const
         // The CTA pair's epilogue goes through TMA wherever an element of C depends on nothing but its own sum, bias and
         // residual; rows in runs as well (direct stores / TMA, B200, us, all kernels of the layer: 6000 rows over 64 experts of 1024 x 512,
         // ReLU squared 98 / 88; 16384 over 32 of 2048 x 1024 253 / 211, 24576 over 64 of 4096 x 1024 707 / 578).
-        if (two_cta && mode == 0 &&
+        if (two_cta && mode != 2 &&
             (p.epi == LLARK_EPI_NONE || p.epi == LLARK_EPI_QUICK_GELU || p.epi == LLARK_EPI_ROPE || p.epi == LLARK_EPI_RELU2))
             p.staged = 2;
         p.stages = p.staged == 2 && R ? kMaxStages2 - 1 : kMaxStages2;
@@ -1586,7 +1586,7 @@ extern "C" int llark_gemm_ex(const void* A, int a_mn_major, long long lda, const
         // Rasterisation group: tiles sweep n inside groups of `group_m` m-blocks, so a group's A panel
         // (group_m x tile_m rows x K) is re-used across the sweep. ncu shows 3.5-4.4x the algorithmic DRAM bytes on the
         // K >= 11008 shapes with the fixed group of 16 (profiles/gemm_traffic.json); LLARK_GEMM_L2_MB=<MB> sizes the group so
-        // that panel fits that many MB of L2 instead. Measured (profiles/r2g_negative_results.md): 32 and 48 MB leave every
+        // that panel fits that many MB of L2 instead. Measured: 32 and 48 MB leave every
         // shape's in-step rate within +-1 % -- DRAM is at ~35 % of its bandwidth on these kernels either way -- so the default
         // stays the fixed 16 (0).
         static int l2_mb = -1;
