@@ -5,7 +5,7 @@
  * call. This header is what those call sites bind to instead: plain device pointers, sizes and a CUDA stream,
  * no torch types. Each entry point cites the reference call site (file:line under the reference root) whose
  * arithmetic it replaces. The Python mirror of the reference API lives in llark_b200/ and calls these through
- * ctypes (INTEGRATION.md shows the binding).
+ * ctypes (llark_b200/_lib.py shows the binding).
  *
  * Conventions: all pointers are DEVICE pointers owned by the caller unless stated; functions never allocate,
  * never free, never synchronise; they enqueue work on `stream` and return LLARK_OK (0) or a negative LLARK_E*.
@@ -231,7 +231,7 @@ int llark_grad_bucket_allreduce(void* comm, void* grads_bf16, long long n, cudaS
 
 /* ---------------------------------------------------------------------------------------------------------
  * Jukebox front end (jukebox/main.py:54-68 get_z, :101-110 get_final_activations, :113-130 windowed_average;
- * arithmetic of openai/jukebox@08efbbc, SURVEY Appendix A). All fp32 activations unless noted.
+ * arithmetic of openai/jukebox@08efbbc). All fp32 activations unless noted.
  */
 /* Strided down-conv Conv1d(c_in -> c_out, k=4, s=2, p=1) + bias. x [N, c_in, T] -> y [N, c_out, T/2]. */
 int llark_jb_conv_down(const float* x, const float* w, const float* bias, float* y, int N, int c_in, int c_out, int T,

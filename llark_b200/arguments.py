@@ -127,7 +127,7 @@ class TrainingArguments:
 
 def check_supported(training_args) -> None:
     """The regime of scripts/training/train_llark.sh is 16-bit full fine-tuning under DDP; the quantised / LoRA / FSDP
-    branches of m2t/train.py:65-88,166-167,185-234 are outside this library (DESIGN.md §7) and fail here, up front."""
+    branches of m2t/train.py:65-88,166-167,185-234 are outside this library and fail here, up front."""
     if getattr(training_args, "bits", 16) != 16:
         raise NotImplementedError(f"--bits {training_args.bits}: bitsandbytes quantisation is not part of llark_b200")
     if getattr(training_args, "lora_enable", False):

@@ -1,5 +1,5 @@
 """Data-parallel exchange step: ONE NCCL all-reduce of the flat bf16 gradient bucket per optimizer step
-(reference: HF Trainer + DDP, scripts/training/train_llark.sh:20-22,44; SURVEY §8(e)).
+(reference: HF Trainer + DDP, scripts/training/train_llark.sh:20-22,44).
 
 The communicator lives in libllark_b200.so (llark_comm_init / llark_grad_bucket_allreduce); torch.distributed is
 only the out-of-band channel that carries the 128-byte ncclUniqueId from rank 0 to the other ranks.
@@ -12,7 +12,7 @@ from ._lib import check, lib
 
 
 def shard_seeds(rank, world, n, base=0):
-    """Synthetic-data partition: rank r draws seeds {base + r, base + r + world, ...} (SURVEY §8(e))."""
+    """Synthetic-data partition: rank r draws seeds {base + r, base + r + world, ...}."""
     return [base + rank + i * world for i in range(n)]
 
 

@@ -1,6 +1,6 @@
 // Data-parallel exchange step of the LLark training path: ONE ncclAllReduce(sum, bf16) over the flat gradient
 // bucket per optimizer step (reference: HF Trainer + DDP under torch.distributed.launch,
-// scripts/training/train_llark.sh:20-22,44; SURVEY §2.3 k14, §8(e)). The 1/(world*accum) scale and the
+// scripts/training/train_llark.sh:20-22,44). The 1/(world*accum) scale and the
 // global-norm clip are fused into the AdamW kernel that consumes the reduced bucket (llama_ops.cu).
 // Large buckets are split into chunks so the caller can enqueue them on a comm stream while wgrad kernels of
 // earlier layers are still running.

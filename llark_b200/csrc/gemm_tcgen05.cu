@@ -2,7 +2,7 @@
 //
 //   C[M,N] = A[M,K] * B[N,K]^T (+ bias[N]) (+ R[M,N]),  fp32 accumulate in TMEM.
 //
-// Replaces every cuBLAS `addmm`/`Linear` call on the reference hot path (SURVEY §2.3 k3, k6, k8, k9):
+// Replaces every cuBLAS `addmm`/`Linear` call on the reference hot path:
 // reference call sites m2t/models/llamav2.py:133 (mm_projector), :224 (LlamaModel q/k/v/o/gate/up/down),
 // :312 (lm_head), their autograd dgrad/wgrad, and jukebox/main.py:108 (prior c_attn/c_proj/mlp).
 //

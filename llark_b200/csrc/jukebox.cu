@@ -1,11 +1,11 @@
 // Jukebox front end kernels (everything of the 5b VQ-VAE encoder + prior that is not a GEMM).
 // Reference call sites: jukebox/main.py:54-68 (get_z -> vqvae.encode), :101-110 (prior.forward, only_encode),
-// :113-130 (windowed_average). Arithmetic follows openai/jukebox@08efbbc as restated in SURVEY Appendix A
+// :113-130 (windowed_average). Arithmetic follows openai/jukebox@08efbbc
 // (the upstream source is not vendored; oracle/jukebox_oracle.py is the CPU restatement these are tested against).
 //
 // All activations fp32 (the reference runs the prior with fp16=False). The conv stack is written time-tiled with
 // all channels of a tile resident in shared memory, so each ResConv1DBlock is ONE pass over HBM
-// (read x, write x'): the per-res-block fusion SURVEY §8(d) counts 1.42 GB/clip against.
+// (read x, write x'), 1.42 GB a clip in all where each is fused by itself.
 #include "common.cuh"
 #include <math.h>
 #include <stdlib.h>
@@ -41,7 +41,7 @@ static inline int jb_check() {
 // TPT output positions tg*32*TPT + l + 32*k. Weights sit in shared memory transposed to [ci][tap][co] so a thread
 // fetches its CPT channels with CPT/4 broadcast LDS.128 per tap: per input channel that is TPT*KT scalar LDS +
 // KT*CPT/4 LDS.128 against TPT*KT*CPT FMAs (>= 4 FMAs per shared-memory wavefront; the first version issued one
-// LDS per FMA and was MIO-bound at 29 % FMA utilisation, profiles/r1h_jukebox_full.md). The accumulation order
+// LDS per FMA and was MIO-bound at 29 % FMA utilisation). The accumulation order
 // (bias, then ci ascending, taps ascending) is unchanged, so results are bit-identical to that version.
 template <int COUT, int KT, int STRIDE, int NCG, int TPT>
 struct ConvTile {
@@ -405,8 +405,7 @@ jb_sparse_attn_kernel(const float* __restrict__ qkv, float* __restrict__ out, in
 
 // ---------------------------------------------------------------------------------------------- factored attention, tensor cores
 // Same contract as jb_sparse_attn_kernel, on mma.sync m16n8k8 TF32 (fp32 accumulate): the SIMT kernel above issues one
-// shared-memory load per FMA and runs at ~6 TFLOP/s (4.7 ms per prior layer at batch 8, a third of the front end,
-// profiles/r1_session2_summary.md); here one CTA = one (group, head, n), each warp owns 16 query rows:
+// shared-memory load per FMA and runs at ~6 TFLOP/s (4.7 ms per prior layer at batch 8, a third of the front end); here one CTA = one (group, head, n), each warp owns 16 query rows:
 //   S = Q K^T  (Q fragments in registers, K from shared memory, 19 k-steps of 8 over the 150(+2 zero) channels),
 //   softmax in registers on the accumulator fragments (quad shuffles),
 //   O = P V    with P taken straight from the S accumulators: the m16n8k8 A fragment wants key slots (t, t+4) where the

@@ -1,8 +1,8 @@
 // HBM-bound kernels of the LLark/Llama training step (everything that is not a GEMM or attention):
 // embedding gather + audio splice, RMSNorm, RoPE, SwiGLU, shifted cross-entropy, gradient norm, AdamW.
-// All are coalesced 16-byte-vector streaming kernels; none touches tensor cores (HBM roof).
+// All are coalesced 16-byte-vector streaming kernels; none touches tensor cores.
 //
-// Reference call sites (file:line under /root/reference unless noted):
+// Reference call sites (file:line of the reference unless noted):
 //   embed gather + splice     m2t/models/llamav2.py:124,141-222
 //   RMSNorm / RoPE / SwiGLU   transformers LlamaRMSNorm / apply_rotary_pos_emb / LlamaMLP (reached at llamav2.py:224)
 //   shifted CE                m2t/models/llamav2.py:314-325
@@ -618,7 +618,7 @@ extern "C" int llark_embed_splice_bwd(const long long* ids, const void* dout, vo
 // H must be 8 * threads * VPT with threads a multiple of 32: pick (threads, VPT) for the supported widths.
 // small_cta: prefer the SMALLEST CTA (largest VPT). A row is then handled by e.g. 128 threads x 4 vectors instead of 512 x 1,
 // four times as many rows are resident per SM and four times the bytes are in flight: the one-row-per-CTA forward was
-// latency-bound at 59 % of the HBM peak with 512-thread CTAs (profiles/r2f_prof_misc_hbm.md).
+// latency-bound at 59 % of the HBM peak with 512-thread CTAs.
 static bool norm_cfg(int H, int* threads, int* vpt, bool small_cta = false) {
     for (int k = 1; k <= 4; ++k) {
         const int v = small_cta ? 5 - k : k;
@@ -656,7 +656,7 @@ extern "C" int llark_rmsnorm_bwd(const void* x, const void* w, const void* dy, c
                                  void* dx, void* dw, int accumulate_dw, long long rows, int H, void* workspace,
                                  cudaStream_t st) {
     int t, v;
-    // (measured, profiles/r2h_prof_opt_hbm.md: a two-rows-per-iteration variant on 128-thread CTAs ran at 2.5 TB/s against
+    // (measured: a two-rows-per-iteration variant on 128-thread CTAs ran at 2.5 TB/s against
     // 3.7-4.5 TB/s for this one-row, 512-thread form -- 255 registers left 8 warps per SM -- so the backward keeps it)
     if (rows <= 0 || !norm_cfg(H, &t, &v) || !workspace) return LLARK_EINVAL;
     const int nb = (int)(rows < 296 ? rows : 296);

@@ -1,11 +1,11 @@
-// HBM-bound kernels of the CLAP + MPT-1B variant (SURVEY §8(f) row 1) that the Llama path does not have:
+// HBM-bound kernels of the CLAP + MPT-1B variant that the Llama path does not have:
 //   bias-free LayerNorm forward / backward over bf16 rows with a row stride (so the q and k thirds of the packed qkv
 //   buffer are normalised in place of a copy): LPLayerNorm of m2t/llava/model/mpt/norm.py:26-52 (norm_1, norm_2, norm_f)
 //   and the q_ln / k_ln LayerNorms of attention.py:248-251,289-292 -- both are "fp32 statistics, one rounding of the
 //   output to bf16", so one kernel serves both;
 //   exact GELU forward / backward (blocks.py:14, nn.GELU(approximate="none")).
 // Wired through llark_b200.ops / engine_mpt.py; per-op parity against fp32 references and the whole engine step against the
-// pinned oracle run on a B200 in tests/test_mpt_gpu.py (round 2).
+// pinned oracle run on a B200 in tests/test_mpt_gpu.py.
 #include "common.cuh"
 #include <math.h>
 

@@ -9,7 +9,7 @@ Host-side orchestration only: every FLOP is a C-ABI call (llark_b200.ops -> libl
   * the forward/backward schedule of the decoder stack (manual backward: dgrad/wgrad GEMMs read weights and saved
     activations in place through MN-major UMMA descriptors, no transposes are materialised).
 
-Reference semantics reproduced (SURVEY §8, Appendix D): pure-bf16 weights/grads, loss = per-rank mean over
+Reference semantics reproduced: pure-bf16 weights/grads, loss = per-rank mean over
 non-ignored shifted tokens computed on bf16 logits, lm_head frozen when requires_grad is False, text-token
 embedding rows detached when `orig_embeds_params` is set (m2t/models/llamav2.py:176-198).
 """
@@ -25,7 +25,7 @@ _ALIGN = 128  # elements (256 B): keeps every view 16-byte aligned for TMA and f
 
 
 class _Nvtx:
-    """NVTX ranges around the phases of a step (LLARK_NVTX=1; SURVEY section 5 tracing): `llark.forward`, `llark.backward`,
+    """NVTX ranges around the phases of a step (LLARK_NVTX=1): `llark.forward`, `llark.backward`,
     `llark.layer_fwd[l]` / `llark.layer_bwd[l]`, and `llark.optimizer` (optim.py), so `ncu --nvtx --nvtx-include` and any
     timeline tool can cut a capture down to one phase or one layer. Off by default: two calls per range otherwise."""
     on = os.environ.get("LLARK_NVTX", "0") == "1"

@@ -1,8 +1,8 @@
-"""Execution schedule of the CLAP + MPT-1B variant (SURVEY §8(f) row 1, BASELINE configs[4]) on the engine's flat
+"""Execution schedule of the CLAP + MPT-1B variant on the engine's flat
 buckets: what m2t/models/mpt.py WrappedMPTForCausalLM + m2t/llava/model/mpt/{modeling_mpt,blocks,attention,norm}.py
 compute, as a manual forward / backward over C-ABI ops.
 
-STATUS: runs on the B200 since round 2 (tests/test_mpt_gpu.py in `pytest -m gpu`, tools/bench_mpt.py: 392 samples/s on one
+STATUS: runs on the B200 (tests/test_mpt_gpu.py in `pytest -m gpu`, tools/bench_mpt.py: 392 samples/s on one
 GPU, 757 on two). The schedule is verified on CPU against oracle/mpt_oracle.py (itself pinned to the reference's classes)
 with the test-only ops stand-in (tests/test_mpt_host_cpu.py). The ops only this variant calls -- `ln_fwd`, `ln_bwd`
 (bias-free LayerNorm, also over the q / k thirds of the packed qkv rows), `gelu_fwd`, `gelu_bwd` (csrc/mpt_ops.cu) and

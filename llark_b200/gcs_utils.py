@@ -1,5 +1,5 @@
 """Local-filesystem half of m2t/gcs_utils.py: the `.npy` embedding files the Jukebox front end writes and the training
-data builders read (SURVEY §8(f) row 3). `gs://` paths are the reference's Google Cloud Storage I/O, out of scope here:
+data builders read. `gs://` paths are the reference's Google Cloud Storage I/O, out of scope here:
 they raise NotImplementedError instead of importing google.cloud.
 
     list_files_with_extension   m2t/gcs_utils.py:162-172 (local branch)
@@ -15,7 +15,7 @@ import torch
 
 
 def _no_gcs(path):
-    raise NotImplementedError(f"{path}: Google Cloud Storage I/O is outside llark_b200's scope (DESIGN.md §7)")
+    raise NotImplementedError(f"{path}: Google Cloud Storage I/O is outside llark_b200's scope")
 
 
 def list_files_with_extension(input_dir: str, extension: str) -> Sequence[str]:

@@ -1,6 +1,6 @@
 """Batch inference from the command line, for use without a reference checkout (the reference's own
-scripts/inference/infer_from_webdataset.py and infer_from_encodings.py also run unchanged over llark_b200's modules,
-INTEGRATION.md §2). One entry point, two sources:
+scripts/inference/infer_from_webdataset.py and infer_from_encodings.py also run unchanged over llark_b200's modules).
+One entry point, two sources:
 
     python -m llark_b200.infer_cli --model_name_or_path <run dir> --ckpt-num 100000 --bf16 True \\
         --eval_data_path 'eval-{000000..000021}.tar' [--prompt "Describe the audio."] --outfile results.csv

@@ -143,7 +143,7 @@ def get_acts_from_file(fpath, hps, vqvae, top_prior, meanpool=True, pool_frames_
 
 
 def embed_batch(waveforms, vqvae, top_prior, pool_frames_per_second=10):
-    """Batched form of get_acts_from_file for waveforms already in memory (batch 8):
+    """Batched form of get_acts_from_file for waveforms already in memory:
     fp32 [N, n_samples] (already mono) -> device tensor fp32 [N, n_frames, W]. Peak normalisation, padding /
     truncation, encoding, prior and pooling follow the per-file function above."""
     cfg = top_prior.cfg

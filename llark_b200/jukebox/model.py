@@ -7,7 +7,7 @@ Only what the reference's call sites touch is provided:
     top_prior.raw_to_tokens, .labeller.get_batch_labels, .get_y, .get_cond           (jukebox/main.py:74-93)
     top_prior.prior.only_encode, top_prior.prior.forward(x, x_cond=, y_cond=, encoder_kv=None, fp16=False)
                                                                                       (jukebox/main.py:101-110)
-Architecture: SURVEY Appendix A (openai/jukebox@08efbbc, not vendored). Levels 0/1 of the VQ-VAE are dead work
+Architecture: openai/jukebox@08efbbc (not vendored). Levels 0/1 of the VQ-VAE are dead work
 in the reference (only zs[-1] is kept, :63) and are skipped: results are identical.
 
 Weights: no checkpoint exists offline; `state` dicts use the names of oracle/jukebox_oracle.py so parity tests can

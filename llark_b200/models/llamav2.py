@@ -2,7 +2,7 @@
 with the arithmetic executed by hand-written sm_100a kernels (llark_b200.engine -> C-ABI) instead of
 transformers/cuBLAS/ATen.
 
-Drop-in contract (SURVEY §8(b)): `WrappedLlamav2Config`, `WrappedLlamav2Model` (with `mm_projector`,
+Drop-in contract: `WrappedLlamav2Config`, `WrappedLlamav2Model` (with `mm_projector`,
 `audio_encoder_config`, `orig_embeds_params`, `initialize_adapter_modules`), `WrappedLlamav2ForCausalLM`
 (`get_model`, `forward(..., audio_encodings=)`, `initialize_audio_tokenizer`, `prepare_inputs_for_generation`),
 HF state_dict key names (`model.embed_tokens.weight`, `model.layers.{i}...`, `model.norm.weight`,
@@ -117,8 +117,8 @@ class WrappedLlamav2ForCausalLM(LlamaForCausalLM):
         **kwargs,
     ):
         """Same signature and return value as m2t/models/llamav2.py:259-337. Training / scoring / cache-less
-        generation. `past_key_values` / `use_cache=True` run the KV-cache path (prefill + one-token decode steps,
-        SURVEY §8(f) row 2; verified on a B200 against the cache-less loop, tests/test_model_gpu.py)."""
+        generation. `past_key_values` / `use_cache=True` run the KV-cache path (prefill + one-token decode steps;
+        verified on a B200 against the cache-less loop, tests/test_model_gpu.py)."""
         if os.environ.get("LLARK_VERIFY") == "fp32":
             # fp32 verification mode (north_star: fp32 logits within 1e-3 relative of the reference's fp32 run):
             # forward only, fp32 tensors end to end on the 3xTF32 tcgen05 path -- llark_b200/verify.py

@@ -1,9 +1,9 @@
-"""Mirror of m2t/models/mpt.py (the CLAP + MPT-1B variant, SURVEY §8(f) row 1): same class names, methods, attribute
+"""Mirror of m2t/models/mpt.py (the CLAP + MPT-1B variant): same class names, methods, attribute
 and state-dict key names (`transformer.wte.weight`, `transformer.blocks.{i}.{norm_1,attn.Wqkv,attn.q_ln,attn.k_ln,
 attn.out_proj,norm_2,ffn.up_proj,ffn.down_proj}.weight`, `transformer.norm_f.weight`, `transformer.mm_projector.*`),
 so `m2t/train.py` takes its `"mpt" in model_name_or_path` branch over it unchanged.
 
-STATUS: runs on the B200 since round 2. The modules hold parameters; `forward` runs llark_b200.engine_mpt.MPTEngine, whose
+STATUS: runs on the B200. The modules hold parameters; `forward` runs llark_b200.engine_mpt.MPTEngine, whose
 schedule is verified against oracle/mpt_oracle.py on CPU (tests/test_mpt_host_cpu.py) and on the GPU kernels
 (tests/test_mpt_gpu.py, part of `pytest -m gpu`). Supported configuration = what MPT-1B uses: multi-head attention with
 ALiBi and q/k LayerNorm, low-precision LayerNorm, no biases, tied embeddings, no logit scale, attn_impl irrelevant."""

@@ -3,7 +3,7 @@ AdamW, as ONE NCCL call and two HBM-bound kernels (sum of squares, fused AdamW) 
 
 Reference: HF Trainer step = DDP all-reduce + clip_grad_norm_(max_grad_norm=1.0) + torch.optim.AdamW on bf16
 parameters without master weights (m2t/arguments.py:84 optim="adamw_torch", m2t/train.py:101-103,
-scripts/training/train_llark.sh:28-36: lr 5e-5, wd 0). Algorithmic traffic: 7 passes x 2 B x n (SURVEY §8(d)).
+scripts/training/train_llark.sh:28-36: lr 5e-5, wd 0). Algorithmic traffic: 7 passes x 2 B x n.
 """
 import torch
 

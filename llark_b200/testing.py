@@ -37,7 +37,7 @@ def to_cuda(batch):
 
 
 # ---- measured parity errors: every tolerance check of the GPU parity tests goes through check_close, which records the
-# measured value next to its bound; tests/conftest.py writes the table to gpurun_out/parity_measured.txt at session end
+# measured value next to its bound; tests/conftest.py writes the table to a file at session end
 PARITY_LOG = []
 
 

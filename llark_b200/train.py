@@ -1,7 +1,7 @@
 """Training entry point: `python -m llark_b200.train <the flags of scripts/training/train_llark.sh>` (under torchrun for
 more than one GPU), or `train(model_args, data_args, training_args)` from Python. It walks the same sequence as
 m2t/train.py:53-278 for the regime that script uses -- 16-bit full fine-tuning, data parallel -- on llark_b200's own
-classes (the reference's train() also runs unchanged over them, INTEGRATION.md §2; this module is for use without a
+classes (the reference's train() also runs unchanged over them; this module is for use without a
 reference checkout):
 
     from_pretrained (MPT when "mpt" is in the name, else Llama-2)        m2t/train.py:62-76

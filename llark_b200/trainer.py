@@ -3,7 +3,7 @@
 `.save_state()`, `._save()`), mirrored from m2t/models/trainer.py:34-129.
 
 The reference subclasses transformers.Trainer (DDP + torch AdamW + autocast). On B200 the step is executed by the
-fused engine, so this is a self-contained loop with the reference's semantics (SURVEY §8 T1-T5):
+fused engine, so this is a self-contained loop with the reference's semantics:
   * micro-batch loss divided by gradient_accumulation_steps; gradients accumulate in the flat bf16 bucket;
   * every `gradient_accumulation_steps` micro-batches: ONE NCCL all-reduce of the bucket (world > 1), global-norm
     clip at max_grad_norm, bf16 AdamW (no master weights), cosine schedule with warm-up ratio;

@@ -3,9 +3,9 @@
 CPU/PyTorch restatement of the Jukebox "5b" front end as LLark uses it: VQ-VAE top-level (level 2) encoder ->
 nearest-code bottleneck -> prior embedding + 36 factored-attention transformer blocks (only_encode) -> 10 Hz
 mean-pool.  The arithmetic lives in openai/jukebox @ 08efbbc1d4ed1a3cef96e08a931944c8b4d63bb3
-(docker/jukebox-embed.dockerfile:50-51), which is NOT vendored under /root/reference and not installed; neither the
-source nor the weights are reachable offline.  This file restates the published architecture (SURVEY Appendix A,
-[UPSTREAM-RECALLED]) and anchors on the reference's own call sites:
+(docker/jukebox-embed.dockerfile:50-51), which the reference does NOT vendor and not installed; neither the
+source nor the weights are reachable offline.  This file restates the published architecture
+([UPSTREAM-RECALLED]) and anchors on the reference's own call sites:
 
     jukebox/main.py:29-45   load_audio_from_file   (mono mean, peak normalise)          -> normalize_audio
     jukebox/main.py:48-51   maybe_pad_audio_to_max_len                                     -> pad_or_truncate
@@ -16,8 +16,7 @@ source nor the weights are reachable offline.  This file restates the published 
     jukebox/main.py:133-173 get_acts_from_file                                              -> get_acts
 
 Only `windowed_average` / the frame arithmetic are pinned against the reference itself (tests/golden/pool_ref.pt,
-generated by importing jukebox/main.py in place).  The network restatement has no golden vectors from upstream:
-the judge caps its parity at "partial"; DESIGN.md says the same.
+generated by importing jukebox/main.py in place).  The network restatement has no golden vectors from upstream.
 """
 import math
 from dataclasses import dataclass
@@ -247,7 +246,7 @@ def prior_forward(codes, p, cfg):
 
 
 def get_acts(audio, vq_params, prior_params, cfg, meanpool=True, pool_frames_per_second=10):
-    """jukebox/main.py:133-173 for an in-memory waveform (decode/resample J1 happens outside; SURVEY §8(a))."""
+    """jukebox/main.py:133-173 for an in-memory waveform (decode/resample J1 happens outside)."""
     audio = normalize_audio(audio)
     input_len = audio.numel()
     latent_len = floor(cfg.n_ctx * input_len / cfg.sample_length)

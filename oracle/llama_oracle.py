@@ -45,7 +45,7 @@ class LlamaCfg:
 
 
 def param_names(cfg):
-    """Parameter names in the reference's state_dict order (SURVEY Appendix C probe)."""
+    """Parameter names in the reference's state_dict order."""
     names = ["model.embed_tokens.weight"]
     for i in range(cfg.num_layers):
         p = f"model.layers.{i}."
@@ -228,7 +228,7 @@ def forward(params, cfg, input_ids, attention_mask=None, labels=None, audio_enco
 
 
 def forward_backward(params, cfg, batch, detach_text=True, freeze_lm_head=True):
-    """Loss, logits and gradients (dict name -> grad or None) with the reference's trainable set (SURVEY §8 T2)."""
+    """Loss, logits and gradients (dict name -> grad or None) with the reference's trainable set."""
     ps = {}
     for n, t in params.items():
         t = t.detach().clone()

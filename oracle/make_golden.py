@@ -5,7 +5,7 @@
 
 The fixtures pin oracle/llama_oracle.py (and, through it, the CUDA path) to the reference:
   llama_tiny_ref.pt   WrappedLlamav2ForCausalLM (m2t/models/llamav2.py) forward/backward, fp32 and bf16, both
-                      splice paths (orig_embeds_params set / unset), frozen lm_head (SURVEY Appendix D 1,3)
+                      splice paths (orig_embeds_params set / unset), frozen lm_head
   pool_ref.pt         jukebox/main.py windowed_average (:113-130) on a seeded [T,4800] array, frame 34
   data_ref.pt         m2t/data_modules.py tokenise/mask/collate index work on a synthetic tokenizer
 """

@@ -1,5 +1,5 @@
 """ORACLE support (test infrastructure only): golden vectors for the on-disk formats and checkpoint formats either side
-of the hot path (SURVEY §8(f) rows 3 and 4), produced by the REFERENCE's own functions imported in place:
+of the hot path, produced by the REFERENCE's own functions imported in place:
 m2t/data_modules.py (_to_conversation_hf, repeat_shards, maybe_add_gcs_prefix, preprocess_multimodal, preprocess_for_lm,
 hf_preprocess_encodings, gen_from_msgpack_shards, read_jsonl_data), m2t/models/utils.py (load_sharded_checkpoint,
 load_sharded_mm_projector_weights), m2t/utils.py, m2t/gcs_utils.py (write_npy, read_audio_encoding).

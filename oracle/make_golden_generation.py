@@ -1,4 +1,4 @@
-"""ORACLE support (test infrastructure only): golden vectors for the generation plumbing (SURVEY §8(f) row 2) from the
+"""ORACLE support (test infrastructure only): golden vectors for the generation plumbing from the
 REFERENCE's own code imported in place: m2t/generate.py (KeywordsStoppingCriteria), m2t/conversation_utils.py,
 m2t/tokenizer.py (get_prompt_end_token_sequence), m2t/infer.py (infer_with_prompt up to the model.generate call), and
 greedy token sequences of the reference's WrappedLlamav2ForCausalLM.generate (transformers GenerationMixin) on the tiny

@@ -2,7 +2,7 @@
 WrappedMPTForCausalLM (m2t/models/mpt.py + m2t/llava/model/mpt/*, imported in place) on the seeded tiny model and batch
 of oracle/mpt_oracle.py, in fp32 and under bf16 autocast, with and without the detached-text splice.
 
-transformers 5.5 note (SURVEY Appendix C): PretrainedConfig no longer keeps two attributes MPTConfig relies on
+transformers 5.5 note: PretrainedConfig no longer keeps two attributes MPTConfig relies on
 (`use_cache`, `tie_word_embeddings`); they are set on the config OBJECT after construction (the reference's source is not
 touched), everything else runs as is with attn_impl="torch"."""
 import os

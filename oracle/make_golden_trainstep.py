@@ -1,6 +1,6 @@
 """ORACLE support (test infrastructure only): tests/golden/trainstep_ref.pt -- a short optimisation TRAJECTORY of the
-reference's own model class under the training regime of scripts/training/train_llark.sh, to pin SURVEY §8(a) rows
-T1-T3 (pure-bf16 weights and AdamW moments, micro-batch losses divided by the accumulation count, clip at 1.0 on the
+reference's own model class under the training regime of scripts/training/train_llark.sh, to pin the training step
+(pure-bf16 weights and AdamW moments, micro-batch losses divided by the accumulation count, clip at 1.0 on the
 accumulated gradient, torch.optim.AdamW, cosine schedule with warm-up stepped once per optimizer step).
 
     python oracle/make_golden_trainstep.py

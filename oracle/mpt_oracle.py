@@ -1,5 +1,5 @@
 """ORACLE (test infrastructure only; never imported by the product): CPU restatement, in plain PyTorch, of the
-reference's CLAP + MPT-1B variant of the hot path (SURVEY §8(f) row 1, BASELINE configs[4]) -- what
+reference's CLAP + MPT-1B variant of the hot path -- what
 `m2t/models/mpt.py` WrappedMPTForCausalLM computes on top of m2t/llava/model/mpt/{modeling_mpt,blocks,attention,norm}.py:
 
     embed (wte) + mm_projector + splice            m2t/models/mpt.py:104-236 (same splice rules as the Llama model)

@@ -1,5 +1,5 @@
 """ORACLE support (test infrastructure only): import shims so the reference's own Python classes load from
-/root/reference under this image's torch 2.11 / transformers 5.5 (SURVEY §8(c), Appendix C).
+/root/reference under this image's torch 2.11 / transformers 5.5.
 
 Only oracle/make_golden.py uses this, and only in the build container: /root/reference does not exist on the GPU box.
 Nothing is copied from the reference; its modules are imported in place.

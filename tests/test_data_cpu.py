@@ -1,6 +1,6 @@
 """CPU tests of the host-side index work (llark_b200/data_modules.py) against golden vectors produced by the
 REFERENCE's own m2t/data_modules.py functions (oracle/make_golden_data.py): bit-exact input_ids / labels /
-attention_mask, prompt construction, the masking quirks of SURVEY Appendix D.4-D.7."""
+attention_mask, prompt construction, the masking quirks of the reference."""
 import os
 import random
 import sys
@@ -103,7 +103,7 @@ def test_tar_shard_reader_and_make_data_module(tmp_path):
     k0 = {i["example_id"] for i in r0}
     k1 = {i["example_id"] for i in r1}
     assert k0 and k1 and not (k0 & k1)
-    # ADVICE r1 (medium): a training rank never starves -- with ONE shard and two ranks both ranks draw from it (wds
+    # a training rank never starves -- with ONE shard and two ranks both ranks draw from it (wds
     # resampled=True), the Q/A pairs of a clip are spread by the 100-element buffer, and shard weights follow
     # task_sample_probs; eval_data_subsample thins the evaluation stream
     import itertools

@@ -1,4 +1,4 @@
-"""World-size-2 (gloo, CPU) test of the HOST logic of the data-parallel step (SURVEY §8(e), T5): two ranks run
+"""World-size-2 (gloo, CPU) test of the HOST logic of the data-parallel step: two ranks run
 WrappedTrainer + LlarkAdamW over different micro-batches with gradient accumulation; the bucket slices the engine
 announces as final during backward (`grad_ready_hook`, reverse layer order) are all-reduced as they appear, step()
 reduces the remainder, scales by 1/world and applies clip + AdamW. Stand-ins (test infrastructure): tests/cpu_ops.py for

@@ -1,4 +1,4 @@
-"""CPU parity tests of the on-disk formats and checkpoint formats either side of the hot path (SURVEY §8(f) rows 3, 4):
+"""CPU parity tests of the on-disk formats and checkpoint formats either side of the hot path:
 llark_b200.data_modules / gcs_utils / models.utils / utils are fed the inputs of oracle/make_golden_formats.py and must
 reproduce, bit for bit, what the REFERENCE's own functions produced for them (tests/golden/formats_ref.pt)."""
 import os

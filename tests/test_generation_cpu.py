@@ -1,4 +1,4 @@
-"""CPU parity tests of the generation plumbing (SURVEY §8(f) row 2) against golden vectors from the REFERENCE's own
+"""CPU parity tests of the generation plumbing against golden vectors from the REFERENCE's own
 m2t/generate.py, m2t/conversation_utils.py, m2t/tokenizer.py, m2t/infer.py and WrappedLlamav2ForCausalLM.generate
 (tests/golden/generation_ref.pt, oracle/make_golden_generation.py). The decoding loop is driven here by the oracle's CPU
 forward (test infrastructure); tests/test_model_gpu.py drives the same loop with the CUDA engine."""

@@ -104,7 +104,7 @@ def test_infer_cli_over_embedding_folder(run_dir, tmp_path):
 
 
 def test_trainer_save_then_load_pretrained_model_keeps_the_projector(run_dir, tmp_path):
-    """ADVICE r1 (high): WrappedTrainer._save writes a single pytorch_model.bin; load_pretrained_model must bring the
+    """WrappedTrainer._save writes a single pytorch_model.bin; load_pretrained_model must bring the
     trained mm_projector back (upstream only reads it from shards) instead of a freshly initialised nn.Linear."""
     from types import SimpleNamespace
 

@@ -1,5 +1,5 @@
-"""Host logic of SURVEY §8(a) rows J4 (get_cond: label rows, RangeEmbedding bins, conditioning tensors) and J7 (load_model
-from upstream-format checkpoints: name map, "module." prefix, 36-of-72 non-strict load) on CPU, with tests/cpu_ops.py
+"""Host logic of get_cond (label rows, RangeEmbedding bins, conditioning tensors) and of load_model
+(upstream-format checkpoints: name map, "module." prefix, 36-of-72 non-strict load) on CPU, with tests/cpu_ops.py
 standing in for the CUDA ops. The checker is oracle/jukebox_oracle.py's restatement of upstream's LabelConditioner
 ([UPSTREAM-RECALLED], parity unpinned as for the rest of the Jukebox network)."""
 import os

@@ -2,8 +2,8 @@
 C-ABI) against (a) the golden vectors produced by the REFERENCE's own class and (b) the oracle restatement run on
 CPU on the same seeded inputs. Tolerances (stated per assert): the reference trains in bf16, so two bf16 pipelines
 are compared by relative Frobenius norm and the CUDA path's error against the fp32 reference must not exceed the bf16
-reference's own error by more than 50 %. Bounds are ~2x the errors measured on a B200 in round 2
-(profiles/r2_parity_measured.txt: logits 4.5e-3 - 1.4e-2, gradients 8e-3 - 1.8e-2, in-place accumulation 2.5e-3)."""
+reference's own error by more than 50 %. Bounds are ~2x the errors measured on a B200
+(logits 4.5e-3 - 1.4e-2, gradients 8e-3 - 1.8e-2, in-place accumulation 2.5e-3)."""
 import os
 
 import pytest

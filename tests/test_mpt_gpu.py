@@ -1,7 +1,6 @@
-"""GPU tests of the MPT variant's kernels (SURVEY §8(f) row 1): bias-free LayerNorm fwd/bwd, exact GELU fwd/bwd, the
+"""GPU tests of the MPT variant's kernels: bias-free LayerNorm fwd/bwd, exact GELU fwd/bwd, the
 ALiBi instantiation of the tcgen05 attention, and the whole MPTEngine step against oracle/mpt_oracle.py (which
-tests/test_mpt_oracle_cpu.py pins to the reference's WrappedMPTForCausalLM). First run on a B200 in round 2
-(profiles/r2a_staged_pytest.txt: all green)."""
+tests/test_mpt_oracle_cpu.py pins to the reference's WrappedMPTForCausalLM)."""
 import math
 import os
 import sys

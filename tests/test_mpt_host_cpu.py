@@ -1,4 +1,4 @@
-"""Host-logic tests of the CLAP + MPT-1B variant (SURVEY §8(f) row 1): llark_b200.models.mpt + llark_b200.engine_mpt run
+"""Host-logic tests of the CLAP + MPT-1B variant: llark_b200.models.mpt + llark_b200.engine_mpt run
 on CPU with tests/cpu_ops.py standing in for the CUDA ops (five of which do not exist as kernels yet) and are checked
 against oracle/mpt_oracle.py, which tests/test_mpt_oracle_cpu.py pins to the reference's own WrappedMPTForCausalLM.
 Pinned here: parameter / state-dict names, the manual backward of the MPT block (LayerNorms incl. the q / k ones, ALiBi
@@ -117,7 +117,7 @@ def test_mpt_config_envelope_and_errors(cpu_mpt):
 
 
 def test_mpt_backward_announces_block_gradients_for_the_overlapped_allreduce(cpu_mpt):
-    """Data-parallel overlap (SURVEY §8(e)): during backward the engine hands contiguous, final slices of the flat gradient
+    """Data-parallel overlap: during backward the engine hands contiguous, final slices of the flat gradient
     bucket to `grad_ready_hook` in reverse block order; together they cover exactly the blocks' parameters, and a slice's
     contents do not change afterwards (the optimizer all-reduces it on a side stream meanwhile)."""
     from oracle import mpt_oracle as mo

@@ -1,4 +1,4 @@
-"""Pins oracle/mpt_oracle.py (the CPU restatement of the CLAP + MPT-1B variant, SURVEY §8(f) row 1) to the REFERENCE's
+"""Pins oracle/mpt_oracle.py (the CPU restatement of the CLAP + MPT-1B variant) to the REFERENCE's
 own WrappedMPTForCausalLM: tests/golden/mpt_tiny_ref.pt holds its loss, logits and gradients on seeded inputs
 (oracle/make_golden_mpt.py). fp32: 1e-5 on loss / logits, 1e-4 on gradients; bf16 autocast: 2e-2 / 6e-2 (rounding-order
 noise of two bf16 pipelines). No product code is involved yet -- this is the oracle gate of that row."""

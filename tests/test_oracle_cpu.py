@@ -33,7 +33,7 @@ def test_oracle_fp32_matches_reference(gold, detach):
     for n, entry in ref["grads"].items():
         g = grads[n]
         if entry is None:
-            assert g is None, n  # frozen lm_head (SURVEY Appendix D.1)
+            assert g is None, n  # frozen lm_head
             continue
         assert abs(g.norm().item() - entry["norm"]) <= 1e-4 * max(entry["norm"], 1e-6), n
         if "full" in entry:

@@ -1,4 +1,4 @@
-"""Drop-in proof for the inference path (SURVEY §8(f) row 2) at the reference's own entry point: the REFERENCE's
+"""Drop-in proof for the inference path at the reference's own entry point: the REFERENCE's
 `scripts/inference/infer_from_webdataset.py::main()` is imported in place and run UNCHANGED over llark_b200's modules
 aliased under their `m2t.*` names -- `load_pretrained_model` on a sharded fp16-loaded checkpoint (projector from the
 shards), the tar-shard eval data module, `get_prompt_end_token_sequence`, `extract_prompt_tokens`,

@@ -1,6 +1,6 @@
-"""Drop-in proof at the reference's own entry point (BASELINE configs[0], the plumbing case): the REFERENCE's
-`m2t/train.py::train()` is imported in place from /root/reference and run UNCHANGED with the three module aliases of
-INTEGRATION.md §2 (m2t.models.llamav2, m2t.data_modules, m2t.models.trainer -> llark_b200), from
+"""Drop-in proof at the reference's own entry point (the plumbing case): the REFERENCE's
+`m2t/train.py::train()` is imported in place from /root/reference and run UNCHANGED with the three module aliases
+(m2t.models.llamav2, m2t.data_modules, m2t.models.trainer -> llark_b200), from
 `WrappedLlamav2ForCausalLM.from_pretrained` through tokenizer surgery, adapter initialisation, `make_data_module` over a
 webdataset-layout tar shard, `WrappedTrainer.train()` and `safe_save_model_for_hf_trainer`.
 
@@ -77,7 +77,7 @@ def test_reference_train_py_runs_unchanged_over_llark_b200(tmp_path, monkeypatch
     import llark_b200.trainer
 
     ref_shims.install()
-    # --- INTEGRATION.md §2: the three aliases, before m2t.train is imported
+    # --- the three aliases, before m2t.train is imported
     for name, mod in (("m2t.models.llamav2", llark_b200.models.llamav2), ("m2t.data_modules", llark_b200.data_modules),
                       ("m2t.models.trainer", llark_b200.trainer)):
         monkeypatch.setitem(sys.modules, name, mod)

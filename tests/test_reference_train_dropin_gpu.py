@@ -1,7 +1,7 @@
 """The reference's own `m2t/train.py::train()` run UNCHANGED on the CUDA engine (the GPU twin of
 tests/test_reference_train_dropin_cpu.py, which proves the same entry point over a CPU stand-in for the ops): imported
 from the verbatim copy of the reference that `__graft_entry__.build()` stages under the git-ignored baseline/_ref/
-(/root/reference does not exist on the GPU box), with the three module aliases of INTEGRATION.md section 2. Every kernel of
+(/root/reference does not exist on the GPU box), with the three module aliases. Every kernel of
 the training step runs through libllark_b200.so; nothing is patched but `sys.modules`. Skipped when the copy is absent."""
 import json
 import os

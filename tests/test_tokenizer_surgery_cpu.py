@@ -1,4 +1,4 @@
-"""SURVEY §8(a) row M3 / Appendix D.2 against the reference, side by side: the reference's own
+"""Tokenizer and embedding surgery against the reference, side by side: the reference's own
 `smart_tokenizer_and_embedding_resize` (m2t/utils.py:60-80) + `WrappedLlamav2ForCausalLM.initialize_audio_tokenizer`
 (m2t/models/llamav2.py:367-419), imported in place, and llark_b200's mirrors run on copies of the same tiny checkpoint
 and tokenizer with the same torch seed (transformers' resize draws the not-mean-initialised rows at random). Compared:

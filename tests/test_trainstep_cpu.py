@@ -1,4 +1,4 @@
-"""SURVEY §8(a) rows T1-T3 against the reference: tests/golden/trainstep_ref.pt is a 4-optimizer-step trajectory (grad
+"""The training step against the reference: tests/golden/trainstep_ref.pt is a 4-optimizer-step trajectory (grad
 accumulation 2, clip 1.0, torch.optim.AdamW on pure-bf16 weights, cosine schedule with warm-up) of the reference's own
 WrappedLlamav2ForCausalLM under the transformers-4.29.2 Trainer loop (oracle/make_golden_trainstep.py). Here
 llark_b200.trainer.WrappedTrainer + LlarkAdamW run the same batches on CPU with tests/cpu_ops.py standing in for the CUDA
