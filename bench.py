@@ -783,7 +783,7 @@ def main():
     achieved = gemm_flops / (gemm_ms / 1000.0) / 1e12 if gemm_ms > 0 else 0.0
     peak = pk.get("bf16_tflops_sustained", pk.get("bf16_tflops"))
     # DRAM traffic of the GEMM kernel: dram__bytes_read.sum + dram__bytes_write.sum per launch from the ncu pass over the
-    # bench's OWN shapes (tools/gpu/r2_evidence.sh -> profiles/gemm_traffic.json, keyed like gemm_by_shape); `traffic` is
+    # bench's OWN shapes (profiles/gemm_traffic.json, keyed like gemm_by_shape); `traffic` is
     # the launch-weighted mean over this step's launches, `traffic_by_shape` carries each shape next to its algorithmic bytes
     traffic, traffic_by_shape = None, None
     tpath = os.path.join(ROOT, "profiles", "gemm_traffic.json")

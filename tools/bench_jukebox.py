@@ -1,4 +1,4 @@
-"""BASELINE configs[1]: Jukebox front end only (see bench.jukebox_measure, which bench.py also folds into its JSON line
+"""Jukebox front end only (see bench.jukebox_measure, which bench.py also folds into its JSON line
 as `configs1_jukebox`).
 
     python tools/bench_jukebox.py [--precision tf32|bf16] [--batch 8] [--steps 3] [--depth 36]

@@ -1,8 +1,7 @@
-"""BASELINE configs[4] (SURVEY §8(f) row 1): CLAP + MPT-1B training step -- one [1, 512] CLAP embedding per sample
+"""CLAP + MPT-1B training step -- one [1, 512] CLAP embedding per sample
 spliced into a 256-token sequence, MPT-1B dims (m2t/llava/model/mpt/configuration_mpt.py:30-36: d_model 2048, 16 heads,
 24 layers, expansion 4, vocab 50368; ALiBi, q/k LayerNorm, no biases, tied head), bf16, fwd + bwd + clip + AdamW.
-First run on a B200 in round 2 (profiles/r2a_bench_mpt.json). Under torchrun it is the data-parallel step on N GPUs
-(configs[4] names 2 x B200): one rank per GPU, the flat-bucket NCCL all-reduce overlapped with backward as in bench.py.
+Under torchrun it is the data-parallel step on N GPUs: one rank per GPU, the flat-bucket NCCL all-reduce overlapped with backward as in bench.py.
 
     python tools/bench_mpt.py [--batch 32] [--steps 5] [--warmup 3] [--layers 24]
     python -m torch.distributed.run --nnodes=1 --nproc-per-node 2 --master-addr 127.0.0.1 --master-port 29517 \

@@ -2,9 +2,9 @@
 records every GEMM launch's (kind, M, N, K) IN LAUNCH ORDER to a JSON file. Run once plainly and once under
 `ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum -k regex:gemm` : the n-th GEMM row of
 the ncu CSV is the n-th entry of the JSON, which is how profiles/gemm_traffic.json gets per-shape DRAM traffic for the
-bench's OWN shapes (tools/gpu/r2_evidence.sh, tools/summarize_ncu.py gemm_traffic).
+bench's OWN shapes (tools/summarize_ncu.py gemm_traffic).
 
-    python tools/gemm_shape_trace.py --out gpurun_out/gemm_shapes.json [--batch 32] [--layers 2]
+    python tools/gemm_shape_trace.py --out gemm_shapes.json [--batch 32] [--layers 2]
 """
 import argparse
 import json

@@ -1,9 +1,9 @@
 """Summarise ncu outputs into small text files under profiles/ (run in the build container, no GPU needed).
 
-  python tools/summarize_ncu.py launches gpurun_out/r1a_launches.csv profiles/r1_launches_summary.md
-  python tools/summarize_ncu.py full gpurun_out/r1a_prof_gemm.ncu-rep profiles/r1_gemm_full.md
-  python tools/summarize_ncu.py gemm_traffic gpurun_out/r2e_gemm_dram.csv gpurun_out/r2e_gemm_shapes.json profiles/gemm_traffic.json
-  python tools/summarize_ncu.py hbm gpurun_out/r2e_prof_misc.ncu-rep profiles/r2e_hbm_kernels.md   (GB/s from dram bytes / duration)
+  python tools/summarize_ncu.py launches launches.csv launches_summary.md
+  python tools/summarize_ncu.py full prof_gemm.ncu-rep gemm_full.md
+  python tools/summarize_ncu.py gemm_traffic gemm_dram.csv gemm_shapes.json profiles/gemm_traffic.json
+  python tools/summarize_ncu.py hbm prof_misc.ncu-rep hbm_kernels.md   (GB/s from dram bytes / duration)
 """
 import json
 import csv
