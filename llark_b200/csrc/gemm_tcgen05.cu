@@ -536,9 +536,10 @@ __device__ __forceinline__ void epilogue_dispatch(const GemmParams& p, long long
 //
 // What it is bound by: nothing of its own at long K (it hides behind the next tile's products); with a short K the bytes of
 // R that are under way, here 32 KB to 64 KB per SM where four warps with loads to registers had 16 KB. Measured on a B200, us before -> now:
-// M 16384, N 4800, K 1200, fp32 with a residual 316 -> 204; K 4800, fp32 with a residual 609 -> 595, bf16 with quick-GELU 617 -> 544; M 6100,
-// N 6144, K 2048, fp32 163 -> 134; M 8192, bf16: N 12288, K 4096 559 -> 555, N 4096, K 4096 with a residual 203 -> 198, N 32000 1438 -> 1428.
-// (These are from before the issuer slept, see there.) Eight warps with direct stores: slower than four in all of these by 1 to 2 %.
+// M 16384, N 4800, K 1200, fp32 with a residual 328 -> 212; K 4800, fp32 with a residual 685 -> 645, bf16 with quick-GELU 794 -> 554; M 6100,
+// N 6144, K 2048, fp32 157 -> 134; M 8192, bf16: N 12288, K 4096 691 -> 616 (rotary columns direct), N 4096, K 4096 with a residual 246 -> 222,
+// N 32004 1735 -> 1631 (the issuer's sleep, see there, has its part in them). Long products of many tiles run against the power
+// cap and gain nothing from it: 36 of M 65536, N 3600, K 4800, fp32, in a step 65.5 ms here and 65.5 with direct stores.
 __device__ __forceinline__ void load_bias32(const GemmParams& p, int col0, float (&b)[32]) {
     if (col0 + 32 <= p.N && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) {  // the same addresses for the whole warp
         if (p.bias_fp32) {
@@ -855,7 +856,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
 // TMEM receives its 128 accumulator rows x 256 columns. Per SM the shared-memory traffic drops from
 // 96 (TMA writes) + 96 (UMMA reads) B/clk to 64 + 64 B/clk, which is what lets the tensor pipe stay busy.
 constexpr int kEpiWarps2 = 8;    // two per 32 rows of a tile, 128 columns each
-// Four with 256 columns each for the gated pairs (EPI 6, 7), which have no TMA form: eight / four, B200, us: ReLU pairs M 300, N 2048, K 1024
+// Four with 256 columns each for the gated pairs (EPI 6, 7), which have no TMA form and go out by direct stores: eight / four, B200, us: ReLU pairs M 300, N 2048, K 1024
 // 16.0 / 14.4, M 8192, N 8192, K 2048 230 / 219; clamped pairs 232 / 224.
 template <int EPI>
 constexpr int epi_warps = EPI == 6 || EPI == 7 ? 4 : kEpiWarps2;
