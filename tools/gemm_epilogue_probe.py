@@ -1,6 +1,7 @@
 """Where does the GEMM epilogue time go? Times C[M,N] = A[M,K] @ B[N,K]^T for the prior's c_proj shape (K = 1200, the
 epilogue-bound case) and a K = 4800 control with every output variant: bf16 / fp32 output, with / without a residual.
-Run once per epilogue mode (LLARK_GEMM_EPILOGUE=staged|direct is read once per process):
+Run once per epilogue mode (LLARK_GEMM_EPILOGUE=staged|direct is read once per process; on the CTA pair auto and staged are the same for
+these products, through TMA; LLARK_GEMM_2CTA=0 gives the single-CTA kernel, where all three differ):
 
     python tools/gemm_epilogue_probe.py            # auto
     LLARK_GEMM_EPILOGUE=direct python tools/gemm_epilogue_probe.py
