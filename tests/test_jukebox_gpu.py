@@ -115,6 +115,20 @@ def test_sparse_attention_tc_full_geometry(pattern):
     check_close("test_sparse_attention_tc_full_geometry:_rel_got_ref_", _rel(got, ref), 2e-3)
 
 
+@pytest.mark.parametrize("N", [1, 2, 3, 5, 9])
+@pytest.mark.parametrize("T,W", [(1, 4), (7, 260), (1800, 4800)])  # the last: additive tables beyond what stays in L2
+def test_prior_input_rows(N, T, W):
+    """One, two or four clips a block, the last block's clips short: (token + position) + condition, y_cond at step 0, the same bits."""
+    from llark_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(N + T)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    codes, emb = torch.randint(0, 40, (N, T), device="cuda", generator=g), r(40, W)
+    y, pos, xc = r(W), r(T, W), r(T, W)
+    rows = torch.cat([y.expand(N, 1, W), emb[codes[:, :-1]]], 1)
+    assert torch.equal(ops.jb_embed_tokens(codes, emb, y, pos, xc).view(N, T, W), (rows + pos) + xc)
+
+
 def test_pool_matches_reference_golden():
     from llark_b200.jukebox import main as jm
 
@@ -384,7 +398,8 @@ def _walk(x, cb):
     return (dist == dist.min(1, keepdim=True).values).int().argmax(1).view(x.shape[0], x.shape[2]), dist
 
 
-@pytest.mark.parametrize("T,n_codes", [(1, 1), (129, 256), (130, 257), (300, 2048), (128, 1000)])
+@pytest.mark.parametrize("T,n_codes", [(1, 1), (129, 256), (130, 257), (300, 2048), (128, 1000),  # walked as they are
+                                       (4800, 257), (4737, 2048), (9600, 300), (9473, 2047)])  # CTAs of 128 vectors, of 256
 @pytest.mark.parametrize("kind", ["spread", "crowded", "close pairs", "lengths apart", "equal", "not finite", "large"])
 def test_nearest_code_is_that_of_the_walk_over_all_codes(T, n_codes, kind):
     """The candidates that tensor cores leave against fp32 walks over all codes, which must name the same ones: codes far apart, codes
