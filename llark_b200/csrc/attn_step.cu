@@ -50,6 +50,7 @@ attn_step_kernel(const Args p, int cs) {
     const int kvh = h0 / (p.H / p.G);
     long long pos = 0, base;
     int nkeys, ring0 = 0;
+    if (p.one_wave) let_next_begin();
     if (p.lens) {
         nkeys = p.lens[b] < p.cap ? p.lens[b] : p.cap;
         base = (long long)b * p.cap;
@@ -273,10 +274,13 @@ attn_step_kernel(const Args p, int cs) {
 }
 
 template <int D, int HG>
-static cudaError_t go(const Args& a, cudaStream_t st) {
+static cudaError_t go(Args a, cudaStream_t st) {
     const long long ctas = (long long)(a.H / HG) * a.B;
     int cs = 1;  // cut along the keys until there are about four CTAs for each of the 148 SMs
     while (cs < 8 && ctas * cs * 2 <= 592) cs *= 2;
+    // Where all CTAs are resident at once the next kernel may come in while they end (a step of one row 242 -> 239 us); it would take room
+    // from CTAs that are still to come (32 rows 525 -> 545). Launched early itself, 1024 CTAs became slower, 540 -> 660.
+    a.one_wave = ctas * cs <= 592;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(a.H / HG * cs), (unsigned)a.B);
     cfg.blockDim = dim3(kThreads);

@@ -30,6 +30,7 @@ struct Args {
     int gate_per_head;
     const float* vfreq;    // [D / 2] or NULL: outputs are turned back by the query's position
     int v_interleaved;
+    int one_wave;          // set by launch()
 };
 
 // Whether launch() takes these operands: head sizes it is built for, rows in 16-byte pieces

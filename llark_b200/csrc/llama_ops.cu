@@ -189,6 +189,8 @@ __global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __
     __shared__ float red[32];
     const long long row = blockIdx.x;
     const __nv_bfloat16* xr = x + row * H;
+    let_next_begin();
+    wait_for_previous();
     float v[VPT][8];
     float ss = 0.f;
 #pragma unroll
@@ -633,19 +635,29 @@ static bool norm_cfg(int H, int* threads, int* vpt, bool small_cta = false) {
     return false;
 }
 
-extern "C" int llark_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, long long rows, int H, float eps,
-                                 cudaStream_t st) {
+// early: a decode step's few rows, between two products
+int llark::rmsnorm_rows(const void* x, const void* w, void* y, float* rstd, long long rows, int H, float eps, bool early, cudaStream_t st) {
     int t, v;
     if (rows <= 0 || !norm_cfg(H, &t, &v, rows >= 1024)) return LLARK_EINVAL;
     const __nv_bfloat16 *xp = (const __nv_bfloat16*)x, *wp = (const __nv_bfloat16*)w;
     __nv_bfloat16* yp = (__nv_bfloat16*)y;
+    auto go = [&](auto kernel) {
+        if (early)
+            (void)launch_early(kernel, dim3((unsigned)rows), dim3(t), 0, 1, st, xp, wp, yp, rstd, H, eps);
+        else
+            kernel<<<(unsigned)rows, t, 0, st>>>(xp, wp, yp, rstd, H, eps);
+    };
     switch (v) {
-        case 1: rmsnorm_fwd_kernel<1><<<(unsigned)rows, t, 0, st>>>(xp, wp, yp, rstd, H, eps); break;
-        case 2: rmsnorm_fwd_kernel<2><<<(unsigned)rows, t, 0, st>>>(xp, wp, yp, rstd, H, eps); break;
-        case 3: rmsnorm_fwd_kernel<3><<<(unsigned)rows, t, 0, st>>>(xp, wp, yp, rstd, H, eps); break;
-        default: rmsnorm_fwd_kernel<4><<<(unsigned)rows, t, 0, st>>>(xp, wp, yp, rstd, H, eps); break;
+        case 1: go(rmsnorm_fwd_kernel<1>); break;
+        case 2: go(rmsnorm_fwd_kernel<2>); break;
+        case 3: go(rmsnorm_fwd_kernel<3>); break;
+        default: go(rmsnorm_fwd_kernel<4>); break;
     }
     return check_launch();
+}
+extern "C" int llark_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, long long rows, int H, float eps,
+                                 cudaStream_t st) {
+    return rmsnorm_rows(x, w, y, rstd, rows, H, eps, rows <= 64, st);
 }
 
 extern "C" long long llark_rmsnorm_bwd_workspace(long long rows, int H) {

@@ -7,9 +7,15 @@
 // tokens ride on one read of a weight. A slice is kept as 128-byte rows whose 16-byte pieces are XORed with the row number: the
 // copies and ldmatrix are free of bank conflicts, and it is the 128-byte swizzle of tcgen05 operands.
 //
-// Measured on a B200, launches in a row on rotating weights (floor = the weights at 6.65 TB/s), against the 256-row tiles of the
-// tcgen05 GEMM core: N 4096 K 4096, 32 tokens 12.3 us (core 28.7, floor 5.0); N 22016 K 4096 40.1 (54.9, 27.1); N 4096 K 11008
-// 21.1 (61.0, 13.6); N 32004 K 4096 47.4 (56.3, 39.4); 64 tokens 14.1 / 46.0 / 23.5 / 51.5.
+// A decode step is a row of such products with short kernels between them, and each of them filled an empty chip and drained it again:
+// 202 us of products for 163 us of bytes in a step of two layers and the head, one row, and 268 us for the whole step. So a CTA starts
+// while the kernel in front of it ends (launch_early): its weights are under way, or on their way to L2, before the tokens are there.
+// The next kernel is let in at once: after half of the slices or with the last ones asked for the step took 2 to 3 us longer.
+// Measured, a step of 1 / 8 / 32 rows: 269 -> 236, 297 -> 270, 560 -> 525 us.
+//
+// Measured on a B200, launches in a row on rotating weights (floor = the weights at 6.55 TB/s), against the 256-row tiles of the
+// tcgen05 GEMM core: N 4096 K 4096, 32 tokens 10.7 us (core 28.7, floor 5.1); N 22016 K 4096 39.4 (54.9, 27.5); N 4096 K 11008
+// 19.3 (61.0, 13.8); N 32004 K 4096 45.9 (56.3, 40.0); 64 tokens 13.2 / 45.2 / 22.0 / 49.7; one token 7.7 / 30.2 / 16.3 / 41.6.
 #include "skinny.cuh"
 
 #include <atomic>
@@ -214,6 +220,16 @@ __device__ __forceinline__ bool row_live(const Args& p, int base, int gap, int i
     return gate_up(p) ? base + (i & (ROWS / 2 - 1)) < (p.N >> 1) : base + i + (i >= ROWS / 2 ? gap : 0) < p.N;
 }
 
+// The first SLICES slices of this CTA's weights, asked for in L2
+template <int ROWS, int SLICES>
+__device__ __forceinline__ void ahead(const Args& p, const bf16_t* W, int base, int gap, int c_lo, int n) {
+    for (int i = threadIdx.x; i < ROWS * SLICES; i += kThreads) {
+        const int r = i / SLICES, s = i % SLICES;
+        if (s < n && row_live<ROWS>(p, base, gap, r))
+            prefetch_l2(W + (long long)(base + r + (r >= ROWS / 2 ? gap : 0)) * p.ldw + (c_lo + s) * BK);
+    }
+}
+
 // ------------------------------------------------------------------------------------------------ up to eight tokens
 template <typename TC>
 __global__ void __launch_bounds__(kThreads, 4)
@@ -239,26 +255,52 @@ skinny_kernel(const Args p, int cs) {
     }
     const bool alive = pr < p.M;
     const bf16_t* asrc = p.A + (alive ? pr * p.lda : 0) + pc * 8;
-    auto issue = [&](int c, int stage) {
+    auto issue_w = [&](int c, int stage) {
         const int k = (c_lo + c) * BK;
         const bool in = k + pc * 8 < p.K;
-        const uint32_t w = sm + stage * kStageMma, a = w + BN * 128;
+        const uint32_t w = sm + stage * kStageMma;
 #pragma unroll
         for (int j = 0; j < 4; ++j) copy16(w + piece(pr + 16 * j, pc), wlive[j] && in ? wsrc[j] + k : p.W, wlive[j] && in);
-        if (pr < 8) copy16(a + piece(pr, pc), alive && in ? asrc + k : p.A, alive && in);
+    };
+    auto issue_a = [&](int c, int stage) {
+        const int k = (c_lo + c) * BK;
+        const bool in = alive && k + pc * 8 < p.K;
+        if (pr < 8) copy16(sm + stage * kStageMma + BN * 128 + piece(pr, pc), in ? asrc + k : p.A, in);
     };
     // The tensor cores cut what does not fit their accumulators instead of rounding it, so the products of a slice start from
     // zero and its sums are added up in registers: the error over K = 4096 is that of fp32 FMAs (1.2e-7; 1.0e-6 in one chain).
     float sum[4] = {0.f, 0.f, 0.f, 0.f};
+    let_next_begin();
+    if (!p.weights_there) {
+        ahead<BN, kStagesMma - 1>(p, p.W, base, gap, c_lo, n);
+        wait_for_previous();
+    }
+#pragma unroll
     for (int s = 0; s < kStagesMma - 1; ++s) {
-        if (s < n) issue(s, s);
+        if (s < n) issue_w(s, s);
         asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    if (p.weights_there) wait_for_previous();
+    if (pr < 8) {  // the tokens of the first slices, by loads: a copy of theirs would be done after all of the weights before it
+        uint4 v[kStagesMma - 1];
+#pragma unroll
+        for (int s = 0; s < kStagesMma - 1; ++s) {
+            const int k = (c_lo + s) * BK;
+            v[s] = make_uint4(0, 0, 0, 0);
+            if (s < n && alive && k + pc * 8 < p.K) v[s] = *reinterpret_cast<const uint4*>(asrc + k);
+        }
+#pragma unroll
+        for (int s = 0; s < kStagesMma - 1; ++s)
+            *reinterpret_cast<uint4*>(smraw + s * kStageMma + BN * 128 + piece(pr, pc)) = v[s];
     }
     int st = 0, st_in = kStagesMma - 1;
     for (int it = 0; it < n; ++it) {
         asm volatile("cp.async.wait_group %0;" ::"n"(kStagesMma - 2) : "memory");
         __syncthreads();  // slice `it` is there for everybody, and everybody is done with the one before
-        if (it + kStagesMma - 1 < n) issue(it + kStagesMma - 1, st_in);
+        if (it + kStagesMma - 1 < n) {
+            issue_w(it + kStagesMma - 1, st_in);
+            issue_a(it + kStagesMma - 1, st_in);
+        }
         asm volatile("cp.async.commit_group;" ::: "memory");
         const uint32_t w = sm + st * kStageMma, a = w + BN * 128;
         const int wr = warp * 16 + (lane & 15);
@@ -326,6 +368,7 @@ skinny_tc_kernel(const Args p, int cs) {
     int M = p.M, row0 = 0;
     const bf16_t* W = p.W;
     if (GROUPED) {
+        wait_for_previous();
         if ((int)blockIdx.y >= p.meta[0]) return;  // the whole cluster
         const int* t = p.tiles + 3 * blockIdx.y;
         W += (long long)t[0] * p.N * p.K;
@@ -366,23 +409,51 @@ skinny_tc_kernel(const Args p, int cs) {
         asrc[j] = p.A + r * p.lda + pc * 8;
     }
     const int m_pad = (M + 15) & ~15;  // tokens that are multiplied
-    auto issue = [&](int c, int stage) {
+    auto issue_w = [&](int c, int stage) {
         const int k = (c_lo + c) * BK;
         const bool in = k + pc * 8 < p.K;
-        const uint32_t w = sm + stage * kStage, a = w + TN * 128;
+        const uint32_t w = sm + stage * kStage;
 #pragma unroll
         for (int j = 0; j < 8; ++j) copy16(w + piece(pr + 16 * j, pc), wlive[j] && in ? wsrc[j] + k : p.W, wlive[j] && in);
-#pragma unroll
-        for (int j = 0; j < NA; ++j)
-            if (pr + 16 * j < m_pad) copy16(a + piece(pr + 16 * j, pc), alive[j] && in ? asrc[j] + k : p.A, alive[j] && in);
     };
+    auto issue_a = [&](int c, int stage) {
+        const int k = (c_lo + c) * BK;
+        const uint32_t a = sm + stage * kStage + TN * 128;
+#pragma unroll
+        for (int j = 0; j < NA; ++j) {
+            const bool in = alive[j] && k + pc * 8 < p.K;
+            if (pr + 16 * j < m_pad) copy16(a + piece(pr + 16 * j, pc), in ? asrc[j] + k : p.A, in);
+        }
+    };
+    const bool early = !GROUPED && p.weights_there;
+    if (!GROUPED && !early) ahead<TN, S - 1>(p, W, base, gap, c_lo, n);
+    tc_fence_before();
+    __syncthreads();  // TMEM is allocated
+    tc_fence_after();
+    let_next_begin();
+    if (!GROUPED && !early) wait_for_previous();
+#pragma unroll
     for (int s = 0; s < S - 1; ++s) {
-        if (s < n) issue(s, s);
+        if (s < n) issue_w(s, s);
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
+    if (early) wait_for_previous();
+    {  // the tokens of the first slices, by loads: a copy of theirs would be done after all of the weights before it
+        uint4 v[S - 1][NA];
+#pragma unroll
+        for (int s = 0; s < S - 1; ++s)
+#pragma unroll
+            for (int j = 0; j < NA; ++j) {
+                const int k = (c_lo + s) * BK;
+                v[s][j] = make_uint4(0, 0, 0, 0);
+                if (s < n && alive[j] && k + pc * 8 < p.K) v[s][j] = *reinterpret_cast<const uint4*>(asrc[j] + k);
+            }
+#pragma unroll
+        for (int s = 0; s < S - 1; ++s)
+#pragma unroll
+            for (int j = 0; j < NA; ++j)
+                *reinterpret_cast<uint4*>(smraw + s * kStage + TN * 128 + piece(pr + 16 * j, pc)) = v[s][j];
+    }
     const uint32_t tmem = tmem_base;
     // fp32 sums, bf16 operands, both K-major, M = 128, N = m_pad
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(m_pad >> 3) << 17) | ((uint32_t)(TN >> 4) << 24);
@@ -422,7 +493,10 @@ skinny_tc_kernel(const Args p, int cs) {
             umma_commit(&done[st]);
         }
         if (it) mbar_wait(&done[st_in], (uint32_t)(((it - 1) / S) & 1));  // the slice before: its place is free, its sums are there
-        if (it + S - 1 < n) issue(it + S - 1, st_in);
+        if (it + S - 1 < n) {
+            issue_w(it + S - 1, st_in);
+            issue_a(it + S - 1, st_in);
+        }
         asm volatile("cp.async.commit_group;" ::: "memory");
         if (CH && it && it % (CH ? CH : 1) == 0) add(it - 1);
         if (++st == S) st = 0;
@@ -456,19 +530,7 @@ static cudaError_t go(F kernel, std::atomic<unsigned long long>& allowed, int sm
         if (e != cudaSuccess) return e;
         if (dev < 64) allowed.fetch_or(1ull << dev, std::memory_order_relaxed);
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(tiles * cs), a.tiles ? (unsigned)a.max_tiles : 1u);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)cs;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = cs > 1 ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, a, cs);
+    return launch_early(kernel, dim3((unsigned)(tiles * cs), a.tiles ? (unsigned)a.max_tiles : 1u), dim3(kThreads), (size_t)smem, cs, st, a, cs);
 }
 template <typename TC>
 static cudaError_t go_mma(const Args& a, int cs, int tiles, cudaStream_t st) {

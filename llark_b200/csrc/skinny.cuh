@@ -32,6 +32,9 @@ struct Args {
     const int *tiles, *meta, *perm;
     int max_tiles, top;
     const float* in_wts;
+    // The weights were there before the kernel in front of this one began (launches of one call behind each other): they are
+    // fetched before that kernel has ended. Otherwise they are only asked for in L2, which a later write does no harm to.
+    int weights_there;
 };
 
 // Whether launch() takes these operands: 16-byte pieces of A and W

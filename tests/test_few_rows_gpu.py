@@ -131,3 +131,44 @@ def test_the_experts_second_product_is_as_exact_as_fmas(T, C, ff, E, top):
         at = pos.long()[(e == k).nonzero().view(-1)]
         want[at] = act[at].to(F64) @ wd[k].to(F64).t()
     assert _rel(z, want) < 2.0 ** -21
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 33, 64])
+def test_products_that_begin_early_see_what_was_written_before(M):
+    """Kernels launched behind each other without a wait: tokens, residuals and weights written by the launch in front, buffers written
+    again while the launch in front may still read them; eagerly and as a captured graph, against the same launches one at a time."""
+    from llark_b200 import ops
+
+    torch.manual_seed(M)
+    K = 1024
+    ws = [(torch.randn(K, K, device="cuda") * K ** -0.5).to(BF16) for _ in range(4)]
+    gamma = torch.ones(K, device="cuda", dtype=BF16)
+    w, x, y, n, rstd = ws[0].clone(), *(torch.empty(M, K, device="cuda", dtype=BF16) for _ in range(3)), torch.empty(M, device="cuda")
+    x0 = torch.randn(M, K, device="cuda").to(BF16)
+
+    def walk(wait):
+        x.copy_(x0)
+        wait()
+        for step in range(12):
+            w.copy_(ws[step % 4])  # the weights of the product right behind
+            wait()
+            ops.gemm(x, w, out=y)
+            wait()
+            ops.rmsnorm_fwd(y, gamma, 1e-5, y=n, rstd=rstd)
+            wait()
+            ops.gemm(n, ws[(step + 1) % 4], residual=x, out=y)  # y has been read
+            wait()
+            ops.gemm(y, ws[(step + 2) % 4], out=x)
+            wait()
+        return x.clone()
+
+    want = walk(torch.cuda.synchronize)
+    assert want.isfinite().all()
+    for _ in range(20):
+        assert torch.equal(walk(lambda: None), want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = walk(lambda: None)
+    for _ in range(5):
+        graph.replay()
+        assert torch.equal(got, want)
