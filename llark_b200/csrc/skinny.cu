@@ -1,26 +1,31 @@
 // Products with few rows (decode steps, routed experts of a few tokens): a stream of the weight matrix. See skinny.cuh.
 //
-// What bounds it is how many bytes of the weights are on their way. A CTA of four warps takes a tile of weight rows; its operands
-// come by cp.async through a ring of 64-wide slices of K (54 to 108 KB of it per CTA, four or two CTAs per SM), and matrices with
-// few rows are also cut along K over a cluster of up to eight CTAs, whose partial sums meet in distributed shared memory in a
-// fixed order (no atomics, no workspace). The weights are the M side of the products and the tokens the N side, so that up to 64
-// tokens ride on one read of a weight. A slice is kept as 128-byte rows whose 16-byte pieces are XORed with the row number: the
-// copies and ldmatrix are free of bank conflicts, and it is the 128-byte swizzle of tcgen05 operands.
+// What bounds it is how many bytes of the weights are on their way. A CTA takes a tile of weight rows; its operands come through a ring of
+// 64-wide slices of K (54 or 112 KB of it per CTA, four or two CTAs per SM), and matrices with few rows are also cut along K over a
+// cluster of up to eight CTAs, whose partial sums meet in distributed shared memory in a fixed order (no atomics, no workspace). The
+// weights are the M side of the products and the tokens the N side, so that up to 64 tokens ride on one read of a weight. A slice is kept
+// as 128-byte rows whose 16-byte pieces are XORed with the row number: cp.async and ldmatrix are free of bank conflicts, and it is the
+// 128-byte swizzle of TMA boxes and tcgen05 operands.
 //
 // A decode step is a row of such products with short kernels between them, and each of them filled an empty chip and drained it again:
 // 202 us of products for 163 us of bytes in a step of two layers and the head, one row, and 268 us for the whole step. So a CTA starts
 // while the kernel in front of it ends (launch_early): its weights are under way, or on their way to L2, before the tokens are there.
 // The next kernel is let in at once: after half of the slices or with the last ones asked for the step took 2 to 3 us longer.
-// Measured, a step of 1 / 8 / 32 rows: 269 -> 236, 297 -> 270, 560 -> 525 us.
+// Measured, a step of 1 / 8 / 32 rows: 269 -> 236, 297 -> 270, 560 -> 525 us (504 with the weights of 32 rows through TMA).
 //
 // Measured on a B200, launches in a row on rotating weights (floor = the weights at 6.55 TB/s), against the 256-row tiles of the
-// tcgen05 GEMM core: N 4096 K 4096, 32 tokens 10.7 us (core 28.7, floor 5.1); N 22016 K 4096 39.4 (54.9, 27.5); N 4096 K 11008
-// 19.3 (61.0, 13.8); N 32004 K 4096 45.9 (56.3, 40.0); 64 tokens 13.2 / 45.2 / 22.0 / 49.7; one token 7.7 / 30.2 / 16.3 / 41.6.
+// tcgen05 GEMM core: N 4096 K 4096, 32 tokens 11.1 us (core 28.7, floor 5.1); N 22016 K 4096 33.0 (54.9, 27.5); N 4096 K 11008
+// 19.3 (61.0, 13.8); N 32004 K 4096 43.3 (56.3, 40.0); 64 tokens 12.8 / 34.2 / 21.0 / 46.0; one token 7.7 / 30.2 / 16.3 / 41.6.
 #include "skinny.cuh"
+
+#include <cuda.h>
 
 #include <atomic>
 
 namespace llark {
+int tensor_map_2d(CUtensorMap* out, const void* ptr, long long inner, long long outer, long long ld, int box_inner, int box_outer,
+                  int elem_bytes);  // gemm_tcgen05.cu
+
 namespace skinny {
 
 typedef __nv_bfloat16 bf16_t;
@@ -99,21 +104,24 @@ __device__ __forceinline__ void store4(bf16_t* C, const float (&v)[4], bool vec,
             if (e < n) C[e] = __float2bfloat16_rn(v[e]);
 }
 
-// A tile's columns from the partial sums red [token][row] (ROWS weight rows, PITCH apart) of the cluster's CTAs; this CTA does its
-// share of them, four results at a time. The two rows that a paired activation or a rotation needs are 2 u and 2 u + 1, or u and
-// u + ROWS / 2.
-template <typename TC, bool GROUPED, int ROWS, int PITCH>
-__device__ __forceinline__ void epilogue(const Args& p, const float* red, int M, int row0, int base, int cs, int rank) {
-    const bool adjacent = p.act == kActReluGlu || p.act == kActClampGlu, halves = gate_up(p), rope = p.act == kActRope;
-    const bool two = adjacent || halves || rope;
-    const int quads = (two ? ROWS / 8 : ROWS / 4) / cs, q0 = rank * quads;
-    const int n_out = adjacent || halves ? p.N >> 1 : p.N;
+// A unit is a row of W, or the two rows that meet in the epilogue.
+__host__ __device__ __forceinline__ bool adjacent_rows(const Args& p) { return p.act == kActReluGlu || p.act == kActClampGlu; }
+__host__ __device__ __forceinline__ bool paired(const Args& p) { return adjacent_rows(p) || gate_up(p) || p.act == kActRope; }
+
+// The results of the `units` units from u0 on (both multiples of four), from the partial sums red [token][row] (rows PITCH apart) of the
+// cluster's CTAs; this CTA does its share of them, four at a time. The two rows of a unit are rows 2 u and 2 u + 1 of the tile, or u and
+// u + units.
+template <typename TC, bool GROUPED, int PITCH>
+__device__ __forceinline__ void epilogue(const Args& p, const float* red, int M, int row0, int u0, int units, int cs, int rank) {
+    const bool adjacent = adjacent_rows(p), rope = p.act == kActRope, two = paired(p);
+    const int quads = units >> 2, q0 = rank * quads / cs, nq = (rank + 1) * quads / cs - q0;
+    const int all = two ? p.N >> 1 : p.N;
     TC* C = static_cast<TC*>(p.C);
     const bool vec = p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(C) & (4 * sizeof(TC) - 1)) == 0;
     auto bias_at = [&](int c) { return p.bias_fp32 ? ldc_<float>(p.bias, c) : ldc_<bf16_t>(p.bias, c); };
-    for (int i = threadIdx.x; i < M * quads; i += kThreads) {
-        const int m = i / quads, u = 4 * (q0 + i % quads);
-        const int col = adjacent ? (base >> 1) + u : base + u, n = n_out - col;
+    for (int i = threadIdx.x; i < M * nq; i += kThreads) {
+        const int m = i / nq, u = 4 * (q0 + i % nq);
+        const int n = all - (u0 + u), col = rope ? ((u0 + u) >> 6) * 128 + ((u0 + u) & 63) : u0 + u;
         if (n <= 0) continue;
         TC* c = C + (long long)(GROUPED ? row0 + m : m) * p.ldc + col;
         float x[4], y[4];
@@ -152,7 +160,7 @@ __device__ __forceinline__ void epilogue(const Args& p, const float* red, int M,
                     }
         } else {
             total4(red, m * PITCH + u, cs, x);
-            total4(red, m * PITCH + u + ROWS / 2, cs, y);
+            total4(red, m * PITCH + u + units, cs, y);
         }
         if (rope) {  // out = bf16(bf16(x cos) + bf16(rotate_half(x) sin)), as the fused GEMM epilogue rounds
 #pragma unroll
@@ -330,7 +338,7 @@ skinny_kernel(const Args p, int cs) {
         cluster_sync_all();
     else
         __syncthreads();
-    epilogue<TC, false, BN, RP>(p, red, p.M, 0, base, cs, rank);
+    epilogue<TC, false, RP>(p, red, p.M, 0, tile * (paired(p) ? BN / 2 : BN), paired(p) ? BN / 2 : BN, cs, rank);
     if (cs > 1) cluster_sync_all();  // nobody leaves while its partial sums may still be read
 }
 
@@ -339,8 +347,17 @@ skinny_kernel(const Args p, int cs) {
 // 2.3x the memory time). Here the same slices go to tcgen05.mma: 128 weight rows are its M side, up to NTOK tokens its N side, the
 // sums lie in NTOK columns of TMEM. CH: every CH slices the products start from zero, in one of two sets of columns, and are added up
 // in registers while the next ones are multiplied (CH 0: one chain over K, 2 to 9e-6 of the result where fp32 FMAs give 1e-7).
+//
+// The weights come as TMA boxes that one thread requests. With cp.async a slice took 0.6 us of every warp's instructions and of waiting
+// for the products of the slice before, whatever its bytes, and two slices less were under way: N 22016 K 4096 39.4 -> 33.0 us with 32
+// tokens, 45.2 -> 34.2 with 64; N 12288 K 4096 23.6 -> 20.4, 27.0 -> 22.9; routed experts of 32 tokens 114 -> 111.
 constexpr int TN = 128, TRP = TN + 4;
-template <int NTOK> constexpr int kStages = NTOK <= 16 ? 6 : NTOK <= 32 ? 5 : 4;  // 108, 100, 96 KB: two CTAs per SM
+constexpr int kTcSmem = 112 * 1024, kMaxStages = 12;  // two CTAs per SM
+constexpr int kGroupedSmem = kTcSmem - 1024;
+// How W is cut: a tile of `units` units, `rows` rows of W (a multiple of eight), for the cs CTAs of a cluster
+struct Cut {
+    int units, rows, cs, stages;
+};
 
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {  // 8-row groups of 1024 bytes, 128-byte swizzle
     return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
@@ -354,210 +371,285 @@ __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&v)
         : "r"(taddr));
 }
 
+// Four warps for the sums and results, one that requests, one that multiplies, and two that copy tokens: where they are gathered, and up to
+// 32 of them, where the same few lines asked for by every CTA at once hold up the weights' boxes in the TMA (N 32004: 43.2 us, by boxes 44.6);
+// 64 tokens come as boxes, of which more slices are under way (N 22016: 41.6 us by copies, 37.5).
+__host__ __device__ constexpr bool copied(int ntok, bool grouped) { return grouped || ntok <= 32; }
+__host__ __device__ constexpr int tc_threads(bool copies) { return copies ? 256 : 192; }
+constexpr int kTokenLag = 3;     // slices of tokens on their way while the next is requested
+
 template <int NTOK, typename TC, bool GROUPED, int CH>
-__global__ void __launch_bounds__(kThreads)
-skinny_tc_kernel(const Args p, int cs) {
+__global__ void __launch_bounds__(tc_threads(copied(NTOK, GROUPED)), 2)
+skinny_tc_kernel(const Args p, const Cut cut, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap amap) {
     extern __shared__ unsigned char smraw_[];
-    constexpr int kStage = TN * 128 + NTOK * 128, S = kStages<NTOK>;
+    constexpr bool COPIES = copied(NTOK, GROUPED);
+    const int cs = cut.cs;
     constexpr int kCols = CH ? 2 * NTOK : NTOK < 32 ? 32 : NTOK;
-    __shared__ uint64_t done[S];
+    __shared__ uint64_t full[kMaxStages], empty[kMaxStages], ready[2], drained[2];
     __shared__ uint32_t tmem_base;
     unsigned char* smraw = smraw_ + ((1024u - (smem_u32(smraw_) & 1023u)) & 1023u);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = cs > 1 ? (int)(blockIdx.x % cs) : 0, tile = (int)blockIdx.x / cs;
-    int M = p.M, row0 = 0;
-    const bf16_t* W = p.W;
-    if (GROUPED) {
-        wait_for_previous();
-        if ((int)blockIdx.y >= p.meta[0]) return;  // the whole cluster
-        const int* t = p.tiles + 3 * blockIdx.y;
-        W += (long long)t[0] * p.N * p.K;
-        row0 = t[1];
-        M = t[2];
-    }
-    int base, gap;
-    tile_rows<TN>(p, tile, base, gap);
     if (threadIdx.x == 0) {
-        for (int i = 0; i < S; ++i) mbar_init(&done[i], 1);
+        for (int i = 0; i < kMaxStages; ++i) {
+            mbar_init(&full[i], COPIES ? 3 : 1);  // the request, and both warps of the tokens
+            mbar_init(&empty[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&ready[i], 1);
+            mbar_init(&drained[i], 4);
+        }
         mbar_fence_init();
     }
-    if (warp == 0) {
+    if (warp == 5) {
         tmem_alloc(&tmem_base, kCols);
         tmem_relinquish();
     }
     const uint32_t sm = smem_u32(smraw);
     const int nch = (p.K + BK - 1) / BK;
     const int c_lo = rank * nch / cs, n = (rank + 1) * nch / cs - c_lo;
-    const int pc = threadIdx.x & 7, pr = threadIdx.x >> 3;
-    const bf16_t* wsrc[8];
-    bool wlive[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int i = pr + 16 * j;
-        wlive[j] = row_live<TN>(p, base, gap, i);
-        wsrc[j] = W + (wlive[j] ? (long long)(base + i + (i >= TN / 2 ? gap : 0)) * p.ldw : 0) + pc * 8;
-    }
-    constexpr int NA = NTOK / 16;
-    const bf16_t* asrc[NA];
-    bool alive[NA];
-#pragma unroll
-    for (int j = 0; j < NA; ++j) {
-        const int m = pr + 16 * j;
-        alive[j] = m < M;
-        long long r = 0;
-        if (alive[j]) r = GROUPED ? (p.perm ? p.perm[row0 + m] / p.top : row0 + m) : m;
-        asrc[j] = p.A + r * p.lda + pc * 8;
-    }
-    const int m_pad = (M + 15) & ~15;  // tokens that are multiplied
-    auto issue_w = [&](int c, int stage) {
-        const int k = (c_lo + c) * BK;
-        const bool in = k + pc * 8 < p.K;
-        const uint32_t w = sm + stage * kStage;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) copy16(w + piece(pr + 16 * j, pc), wlive[j] && in ? wsrc[j] + k : p.W, wlive[j] && in);
-    };
-    auto issue_a = [&](int c, int stage) {
-        const int k = (c_lo + c) * BK;
-        const uint32_t a = sm + stage * kStage + TN * 128;
-#pragma unroll
-        for (int j = 0; j < NA; ++j) {
-            const bool in = alive[j] && k + pc * 8 < p.K;
-            if (pr + 16 * j < m_pad) copy16(a + piece(pr + 16 * j, pc), in ? asrc[j] + k : p.A, in);
-        }
-    };
-    const bool early = !GROUPED && p.weights_there;
-    if (!GROUPED && !early) ahead<TN, S - 1>(p, W, base, gap, c_lo, n);
     tc_fence_before();
     __syncthreads();  // TMEM is allocated
     tc_fence_after();
-    let_next_begin();
-    if (!GROUPED && !early) wait_for_previous();
-#pragma unroll
-    for (int s = 0; s < S - 1; ++s) {
-        if (s < n) issue_w(s, s);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    if (early) wait_for_previous();
-    {  // the tokens of the first slices, by loads: a copy of theirs would be done after all of the weights before it
-        uint4 v[S - 1][NA];
-#pragma unroll
-        for (int s = 0; s < S - 1; ++s)
-#pragma unroll
-            for (int j = 0; j < NA; ++j) {
-                const int k = (c_lo + s) * BK;
-                v[s][j] = make_uint4(0, 0, 0, 0);
-                if (s < n && alive[j] && k + pc * 8 < p.K) v[s][j] = *reinterpret_cast<const uint4*>(asrc[j] + k);
-            }
-#pragma unroll
-        for (int s = 0; s < S - 1; ++s)
-#pragma unroll
-            for (int j = 0; j < NA; ++j)
-                *reinterpret_cast<uint4*>(smraw + s * kStage + TN * 128 + piece(pr + 16 * j, pc)) = v[s][j];
-    }
     const uint32_t tmem = tmem_base;
-    // fp32 sums, bf16 operands, both K-major, M = 128, N = m_pad
-    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(m_pad >> 3) << 17) | ((uint32_t)(TN >> 4) << 24);
+    let_next_begin();
+    int M = p.M, row0 = 0, wrow = 0;
+    if (GROUPED) {
+        wait_for_previous();
+        if ((int)blockIdx.y >= p.meta[0]) {  // the whole cluster
+            if (warp == 5) tmem_dealloc(tmem, kCols);
+            return;
+        }
+        const int* t = p.tiles + 3 * blockIdx.y;
+        wrow = t[0] * p.N;
+        row0 = t[1];
+        M = t[2];
+    }
+    const int u0 = tile * cut.units;
+    wrow += p.act == kActRope ? (u0 >> 6) * 128 + (u0 & 63) : adjacent_rows(p) ? 2 * u0 : u0;
+    const int m_pad = (M + 15) & ~15;  // tokens that are multiplied
+    // of a stage, in bytes; with few tokens a routed tile has room for more stages than the worst case
+    const int kWeights = (GROUPED ? TN : cut.rows) * 128, kStage = kWeights + (GROUPED ? m_pad : NTOK) * 128;
+    const int S = GROUPED ? kGroupedSmem / kStage : cut.stages;
     auto set = [](int it) { return CH ? it / (CH ? CH : 1) % 2 * NTOK : 0; };  // the columns of a slice's products
     float sum[NTOK];  // of weight row warp * 32 + lane
+    if (warp < 4) {
+        wait_for_previous();  // for the residual, and before anything is written
 #pragma unroll
-    for (int j = 0; j < NTOK; ++j) sum[j] = 0.f;
-    auto add = [&](int it) {  // the sums up to slice `it`, whose products have been waited for
-        tc_fence_after();
-        constexpr int NL = NTOK < 32 ? NTOK : 32;
-#pragma unroll
-        for (int c0 = 0; c0 < NTOK; c0 += NL) {
-            if (c0 >= m_pad) break;  // the same for everybody
-            uint32_t v[NL];
-            const uint32_t at = tmem + ((uint32_t)(warp * 32) << 16) + set(it) + c0;
-            if constexpr (NL == 16)
-                tmem_ld_32x32b_x16(at, v);
-            else
-                tmem_ld_32x32b_x32(at, v);
-            tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < NL; ++j) sum[c0 + j] += __uint_as_float(v[j]);  // columns from m_pad on hold nothing and are not used
-        }
-        tc_fence_before();
-    };
-    int st = 0, st_in = S - 1;
-    for (int it = 0; it < n; ++it) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(S - 2) : "memory");
-        fence_proxy_async_smem();
-        __syncthreads();  // slice `it` is there, written by everybody; everybody has taken the sums before those of slice it - 1
-        if (threadIdx.x == 0) {
+        for (int j = 0; j < NTOK; ++j) sum[j] = 0.f;
+        const int chains = CH ? (n + (CH ? CH : 1) - 1) / (CH ? CH : 1) : 1;
+        for (int c = 0; c < chains; ++c) {
+            mbar_wait(&ready[c & 1], (uint32_t)((c >> 1) & 1));
             tc_fence_after();
-            const uint64_t wd = smem_desc(sm + st * kStage), ad = smem_desc(sm + st * kStage + TN * 128);
+            constexpr int NL = NTOK < 32 ? NTOK : 32;
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-                umma_f16(tmem + set(it), wd + (uint64_t)(k * 2), ad + (uint64_t)(k * 2), idesc, (CH ? it % (CH ? CH : 1) : it) != 0 || k != 0);
-            umma_commit(&done[st]);
+            for (int c0 = 0; c0 < NTOK; c0 += NL) {
+                if (c0 >= m_pad) break;  // the same for everybody
+                uint32_t v[NL];
+                const uint32_t at = tmem + ((uint32_t)(warp * 32) << 16) + (CH ? (c & 1) * NTOK : 0) + c0;
+                if constexpr (NL == 16)
+                    tmem_ld_32x32b_x16(at, v);
+                else
+                    tmem_ld_32x32b_x32(at, v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < NL; ++j) sum[c0 + j] += __uint_as_float(v[j]);  // columns from m_pad on hold nothing and are not used
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&drained[c & 1]);
         }
-        if (it) mbar_wait(&done[st_in], (uint32_t)(((it - 1) / S) & 1));  // the slice before: its place is free, its sums are there
-        if (it + S - 1 < n) {
-            issue_w(it + S - 1, st_in);
-            issue_a(it + S - 1, st_in);
+    } else if (warp == 4) {
+        if (lane == 0) {
+            const int other = gate_up(p) ? p.N >> 1 : p.act == kActRope && cut.units < 64 ? 64 : 0;  // where the units' other rows are
+            auto each = [&](int it, auto use) {  // the boxes of a slice
+                const int k = (c_lo + it) * BK;
+                use(k, wrow, 0);
+                if (other) use(k, wrow + other, kWeights / 2);
+            };
+            auto request = [&](int it, int st) {
+                mbar_arrive_expect_tx(&full[st], COPIES ? kWeights : kStage);
+                each(it, [&](int k, int row, int at) { tma_load_2d(smraw + st * kStage + at, &wmap, &full[st], k, row); });
+            };
+            if (!GROUPED && !p.weights_there) {
+                for (int it = 0; it < S && it < n; ++it) each(it, [&](int k, int row, int) { tma_prefetch_2d(&wmap, k, row); });
+                wait_for_previous();
+            }
+            const int first = n < S ? n : S;
+            for (int it = 0; it < first; ++it) request(it, it);
+            auto tokens = [&](int it, int st) {
+                if (!COPIES) tma_load_2d(smraw + st * kStage + kWeights, &amap, &full[st], (c_lo + it) * BK, 0);
+            };
+            if (!COPIES) {
+                if (p.weights_there) wait_for_previous();
+                for (int it = 0; it < first; ++it) tokens(it, it);
+            }
+            for (int it = S, st = 0, ph = 0; it < n; ++it) {
+                mbar_wait(&empty[st], ph);
+                request(it, st);
+                tokens(it, st);
+                if (++st == S) st = 0, ph ^= 1;
+            }
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        if (CH && it && it % (CH ? CH : 1) == 0) add(it - 1);
-        if (++st == S) st = 0;
-        if (++st_in == S) st_in = 0;
+    } else if (warp == 5) {
+        if (lane == 0) {
+            // fp32 sums, bf16 operands, both K-major, M = 128, N = m_pad
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(m_pad >> 3) << 17) | ((uint32_t)(TN >> 4) << 24);
+            for (int it = 0, st = 0, ph = 0; it < n; ++it) {
+                const int c = CH ? it / (CH ? CH : 1) : 0;
+                if (CH && c >= 2 && it % (CH ? CH : 1) == 0) mbar_wait(&drained[c & 1], (uint32_t)(((c >> 1) - 1) & 1));
+                mbar_wait(&full[st], ph);
+                tc_fence_after();
+                const uint64_t wd = smem_desc(sm + st * kStage), ad = smem_desc(sm + st * kStage + kWeights);
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    umma_f16(tmem + set(it), wd + (uint64_t)(k * 2), ad + (uint64_t)(k * 2), idesc, (CH ? it % (CH ? CH : 1) : it) != 0 || k != 0);
+                umma_commit(&empty[st]);
+                if (it == n - 1 || (CH && (it + 1) % (CH ? CH : 1) == 0)) umma_commit(&ready[c & 1]);
+                if (++st == S) st = 0, ph ^= 1;
+            }
+        }
+    } else if (COPIES) {
+        wait_for_previous();
+        const int pc = threadIdx.x & 7, pr = (threadIdx.x - 192) >> 3;
+        constexpr int NA = NTOK / 8;
+        const bf16_t* asrc[NA];
+        bool alive[NA];
+#pragma unroll
+        for (int j = 0; j < NA; ++j) {
+            const int m = pr + 8 * j;
+            alive[j] = m < M;
+            long long r = 0;
+            if (alive[j]) r = !GROUPED ? m : p.perm ? p.perm[row0 + m] / p.top : row0 + m;
+            asrc[j] = p.A + r * p.lda + pc * 8;
+        }
+        int st = 0, ph = 1, st_out = 0;
+        for (int it = 0; it < n + kTokenLag; ++it) {
+            if (it < n) {
+                if (it >= S) mbar_wait(&empty[st], ph);
+                const int k = (c_lo + it) * BK;
+                const uint32_t a = sm + st * kStage + kWeights;
+#pragma unroll
+                for (int j = 0; j < NA; ++j) {
+                    const bool in = alive[j] && k + pc * 8 < p.K;
+                    if (pr + 8 * j < m_pad) copy16(a + piece(pr + 8 * j, pc), in ? asrc[j] + k : p.A, in);
+                }
+                if (++st == S) st = 0, ph ^= 1;
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            if (it >= kTokenLag) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(kTokenLag) : "memory");
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full[st_out]);
+                if (++st_out == S) st_out = 0;
+            }
+        }
     }
-    mbar_wait(&done[(n - 1) % S], (uint32_t)(((n - 1) / S) & 1));
-    add(n - 1);
+    __syncwarp();
     // ---- partial sums to shared memory, [token][row]: the slices are no longer read
     float* red = reinterpret_cast<float*>(smraw);
+    if (warp < 4) {
 #pragma unroll
-    for (int j = 0; j < NTOK; ++j)
-        if (j < m_pad) red[j * TRP + warp * 32 + lane] = sum[j];
+        for (int j = 0; j < NTOK; ++j)
+            if (j < m_pad) red[j * TRP + warp * 32 + lane] = sum[j];
+    }
     if (cs > 1)
         cluster_sync_all();
     else
         __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, kCols);
-    epilogue<TC, GROUPED, TN, TRP>(p, red, M, row0, base, cs, rank);
+    if (warp == 5) tmem_dealloc(tmem, kCols);
+    if (warp < 4) epilogue<TC, GROUPED, TRP>(p, red, M, row0, u0, cut.units, cs, rank);
     if (cs > 1) cluster_sync_all();  // nobody leaves while its partial sums may still be read
 }
 
 // ------------------------------------------------------------------------------------------------ host
-template <typename F>
-static cudaError_t go(F kernel, std::atomic<unsigned long long>& allowed, int smem, const Args& a, int cs, int tiles,
-                      cudaStream_t st) {
+template <typename F, typename... X>
+static cudaError_t go(F kernel, std::atomic<unsigned long long>& allowed, int most, int smem, int threads, int tiles, int cs, cudaStream_t st,
+                      const Args& a, const X&... more) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev >= 64 || !(allowed.load(std::memory_order_relaxed) >> dev & 1)) {  // once per device
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         if (e != cudaSuccess) return e;
         if (dev < 64) allowed.fetch_or(1ull << dev, std::memory_order_relaxed);
     }
-    return launch_early(kernel, dim3((unsigned)(tiles * cs), a.tiles ? (unsigned)a.max_tiles : 1u), dim3(kThreads), (size_t)smem, cs, st, a, cs);
+    return launch_early(kernel, dim3((unsigned)(tiles * cs), a.tiles ? (unsigned)a.max_tiles : 1u), dim3(threads), (size_t)smem, cs, st, a, more...);
 }
 template <typename TC>
 static cudaError_t go_mma(const Args& a, int cs, int tiles, cudaStream_t st) {
     static std::atomic<unsigned long long> allowed{0};
-    return go(skinny_kernel<TC>, allowed, kStagesMma * kStageMma, a, cs, tiles, st);
+    return go(skinny_kernel<TC>, allowed, kStagesMma * kStageMma, kStagesMma * kStageMma, kThreads, tiles, cs, st, a, cs);
+}
+static int units_of(const Args& a) { return paired(a) ? a.N / 2 : a.N; }
+
+// Stages that fit beside what the products read behind the last one: they take 128 rows whatever the tile has
+static int stages(int rows, int ntok, int& smem) {
+    const int stage = (rows + ntok) * 128, tail = stage < TN * 128 ? TN * 128 - stage : 0;
+    int s = (kTcSmem - 1024 - tail) / stage;
+    if (s > kMaxStages) s = kMaxStages;
+    smem = s * stage + tail + 1024;
+    if (smem < ntok * TRP * 4 + 1024) smem = ntok * TRP * 4 + 1024;  // the partial sums
+    return s;
 }
 template <int NTOK, typename TC, bool GROUPED, int CH>
-static cudaError_t go_tc(const Args& a, int cs, int tiles, cudaStream_t st) {
+static cudaError_t go_tc(const Args& a, Cut cut, cudaStream_t st) {
     static std::atomic<unsigned long long> allowed{0};
-    return go(skinny_tc_kernel<NTOK, TC, GROUPED, CH>, allowed, kStages<NTOK> * (TN * 128 + NTOK * 128) + 1024, a, cs, tiles, st);
+    int smem;
+    cut.stages = stages(cut.rows, NTOK, smem);
+    if (GROUPED) smem = kTcSmem;
+    const bool boxes = gate_up(a) || (a.act == kActRope && cut.units < 64);  // two for a slice
+    CUtensorMap wmap;
+    if (tensor_map_2d(&wmap, a.W, a.K, GROUPED ? (long long)a.experts * a.N : a.N, a.ldw, BK, boxes ? cut.units : cut.rows, 2)) return cudaErrorInvalidValue;
+    CUtensorMap amap = wmap;
+    if (!copied(NTOK, GROUPED) && tensor_map_2d(&amap, a.A, a.K, a.M, a.lda, BK, NTOK, 2)) return cudaErrorInvalidValue;
+    return go(skinny_tc_kernel<NTOK, TC, GROUPED, CH>, allowed, kTcSmem, smem, tc_threads(copied(NTOK, GROUPED)), (units_of(a) + cut.units - 1) / cut.units, cut.cs, st, a,
+              cut, wmap, amap);
 }
 
 cudaError_t launch(const Args& a, cudaStream_t st) {
-    const bool grouped = a.tiles != nullptr;
-    // Up to eight tokens the mma.sync kernel: as fast as the other or faster (K = 2048, N = 2048: 5.4 against 6.7 us), and ten
+    const bool grouped = a.tiles != nullptr, two = paired(a);
+    const int nch = (a.K + BK - 1) / BK, all = units_of(a);
+    // Up to eight tokens the mma.sync kernel: as fast as the other or faster (K = 2048, N = 2048: 4.5 against 5.8 us), and ten
     // times as exact. Routed experts have 0 to 64 tokens per tile, known only on the device.
-    const bool tc = grouped || a.M > 8;
-    const int rows = tc ? TN : BN;
-    const int tiles = gate_up(a) ? (a.N / 2 + rows / 2 - 1) / (rows / 2) : (a.N + rows - 1) / rows;
-    // Cut along K until the grid holds as many CTAs as are resident at once (four or two for each of the 148 SMs), as long as a
-    // CTA keeps four slices of K.
-    const int nch = (a.K + BK - 1) / BK;
-    const long long most = tc ? 296 : 592;
-    int cs = 1;
-    while (cs < 8 && (long long)tiles * (grouped ? a.max_tiles : 1) * cs * 2 <= most && nch / (cs * 2) >= 4) cs *= 2;
-#define LLARK_SKINNY(N_, GR_, CH_) (a.c_fp32 ? go_tc<N_, float, GR_, CH_>(a, cs, tiles, st) : go_tc<N_, bf16_t, GR_, CH_>(a, cs, tiles, st))
-    if (!tc) return a.c_fp32 ? go_mma<float>(a, cs, tiles, st) : go_mma<bf16_t>(a, cs, tiles, st);
+    if (!grouped && a.M <= 8) {
+        // Cut along K until the grid holds as many CTAs as are resident at once (four for each of the 148 SMs), as long as a CTA keeps four
+        // slices of K.
+        const int units = two ? BN / 2 : BN, tiles = (all + units - 1) / units;
+        int cs = 1;
+        while (cs < 8 && tiles * cs * 2 <= 592 && nch / (cs * 2) >= 4) cs *= 2;
+        return a.c_fp32 ? go_mma<float>(a, cs, tiles, st) : go_mma<bf16_t>(a, cs, tiles, st);
+    }
+    const int most = two ? TN / 2 : TN;
+    Cut cut = {most, TN, 1, 0};
+    if (grouped) {  // the same with two CTAs for an SM
+        const int tiles = (all + most - 1) / most;
+        while (cut.cs < 8 && (long long)tiles * a.max_tiles * cut.cs * 2 <= 296 && nch / (cut.cs * 2) >= 4) cut.cs *= 2;
+    } else {
+        const int ntok = a.M <= 16 ? 16 : a.M <= 32 ? 32 : 64;
+        // The tiles and clusters with most of the weights under way, of those that are all resident at once (two CTAs for each of the 148 SMs; of
+        // clusters of four and eight 71 and 33 fit), as long as a CTA keeps four slices of K; larger tiles and smaller clusters unless others have a
+        // twentieth more. Tiles of less than 64 rows leave the tensor cores more products than the time of their bytes. 22016 rows of gate
+        // and up in 276 tiles of 80 instead of 172 of 128: 34.8 -> 32.7 us with 32 tokens, 37.5 -> 34.4 with 64. (Clusters of three: 12288
+        // rows in 288 CTAs instead of 192 20.8 -> 31.)
+        static const int sizes[] = {1, 2, 4, 8}, fit[] = {296, 148, 71, 33};
+        long long best = 0;
+        const long long bytes = 2LL * a.N * a.K / 128;
+        for (int i = 0; i < 4; ++i) {
+            if (sizes[i] > 1 && nch / sizes[i] < 4) break;
+            for (int rows = TN; rows >= 64; rows -= 8) {
+                const int units = two ? rows / 2 : rows;
+                if (units % 8 || (a.act == kActRope && units != 64 && units != 32)) continue;
+                const int tiles = (all + units - 1) / units;
+                int smem;
+                long long way = tiles <= fit[i] ? (long long)tiles * sizes[i] * stages(rows, ntok, smem) * rows : 0;
+                if (way > bytes) way = bytes;
+                if (way * 20 > best * 21) best = way, cut = {units, rows, sizes[i], 0};
+            }
+        }
+    }
+#define LLARK_SKINNY(N_, GR_, CH_) (a.c_fp32 ? go_tc<N_, float, GR_, CH_>(a, cut, st) : go_tc<N_, bf16_t, GR_, CH_>(a, cut, st))
     if (grouped) return LLARK_SKINNY(64, true, 1);
     // Short chains for what fp32 FMAs computed before: narrow products, paired activations with an fp32 result and results off 16-byte
     // boundaries. The others took the tcgen05 core, whose one chain over K errs by 4 to 12e-6; cut over a cluster theirs are shorter (0.5 to 1.4e-6), and 6 % faster than

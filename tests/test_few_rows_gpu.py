@@ -172,3 +172,21 @@ def test_products_that_begin_early_see_what_was_written_before(M):
     for _ in range(5):
         graph.replay()
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("M", [9, 32, 33, 64])
+@pytest.mark.parametrize("N,K", [(22016, 520), (9000, 1032), (2176, 4104)])
+def test_tiles_of_fewer_rows_and_clusters(M, N, K):
+    """Matrices that are cut into tiles of 64 to 128 rows and clusters of one to eight, the last tile and the last slice of K ragged."""
+    from llark_b200 import ops
+
+    torch.manual_seed(M + N)
+    x, w = torch.randn(M, K, device="cuda").to(BF16), (torch.randn(N, K, device="cuda") * K ** -0.5).to(BF16)
+    z = x.to(F64) @ w.to(F64).t()
+    # fp32 results: only the order and the cut of the sums shows, 5e-6 as above; bf16: one rounding, 2^-8 of a value; gate times up
+    # rounds its two sums, the gate's function and the result: four of 2^-9 each at most
+    assert _rel(ops.linear(x, w, out_dtype=F32), z) < 5e-6
+    assert _rel(ops.linear(x, w, act="relu_glu"), torch.relu(z[:, 0::2]) * z[:, 1::2]) < 2.0 ** -8
+    if N % 16 == 0:  # rows of the result on 16-byte boundaries
+        g, u = z[:, :N // 2], z[:, N // 2:]
+        assert _rel(ops.gemm(x, w, swiglu=True), torch.nn.functional.silu(g) * u) < 2.0 ** -7
