@@ -14,8 +14,15 @@ LIB_SERVE := llark_b200/libllark_serve.so
 # a shared link accepts what it cannot resolve, and the library then fails to load: make that an error of the build
 LDFLAGS := -shared -Xlinker --no-undefined
 
-all: $(LIB)
-serve: $(LIB_SERVE)
+# the entry points as Python functions (without Python's headers the package calls the library through ctypes)
+PYINC := $(shell python3 -c "import sysconfig; print(sysconfig.get_paths()['include'])" 2>/dev/null)
+CALLS := $(if $(wildcard $(PYINC)/Python.h),llark_b200/_calls.so)
+
+all: $(LIB) $(CALLS)
+serve: $(LIB_SERVE) $(CALLS)
+
+llark_b200/_calls.so: llark_b200/csrc/calls.cpp include/llark_b200.h
+	g++ -std=c++17 -O2 -shared -fPIC -I$(PYINC) -I$(dir $(NVCC))../include -o $@ $< -ldl
 
 build/%.o: llark_b200/csrc/%.cu llark_b200/csrc/common.cuh include/llark_b200.h
 	@mkdir -p build
@@ -35,5 +42,5 @@ $(LIB_SERVE): $(SERVE_OBJ)
 	$(NVCC) $(ARCH) $(LDFLAGS) -o $@ $(SERVE_OBJ)
 
 clean:
-	rm -rf build $(LIB) $(LIB_SERVE)
+	rm -rf build $(LIB) $(LIB_SERVE) llark_b200/_calls.so
 .PHONY: all serve clean

@@ -306,6 +306,13 @@ int llark_v32_ce_fwd(const float* logits, long long ldv, int V, const long long*
  * request b (cu[n_seq] = n_tok), pos0[b] = position of that row in its sequence, slot[b] = the request's row in every
  * state store. The residual stream, norms, scores, softmax and recurrent state are fp32; `act_fp32` selects the
  * activation / matrix dtype (0: bf16, 1: float = the all-fp32 mode). */
+
+/* The integers of a packed step on the device, out [n_tok + n_values] = tok_seq | values, from HOST memory that may be used again when the
+ * call returns: values = cu [n_seq + 1] | pos0 [n_seq] | slot [n_seq] | lengths [n_seq] | others; at most LLARK_STEP_INTS of them. Every
+ * request has a row. */
+#define LLARK_STEP_INTS 8000
+int llark_seq_step_ints(const int* values, int n_values, int n_seq, int n_tok, int* out, cudaStream_t stream);
+
 int llark_seq_embed(const int* ids, const int* tok_seq, const int* cu, const int* pos0, const void* table,
                     const void* pos_table, float scale, float* x, void* x_act, int n_tok, int C, int act_fp32,
                     cudaStream_t stream); /* x_act (optional): a copy of x in the activation dtype */

@@ -17,7 +17,7 @@ _ERR = {-1: "LLARK_EINVAL (bad shape/alignment/argument)", -2: "LLARK_ECUDA", -3
 
 # the generation path of layer-list decoders (csrc/seq_*.cu)
 SEQ_SYMBOLS = [
-    "llark_seq_embed", "llark_seq_short_conv", "llark_seq_conv_tail", "llark_seq_add_rmsnorm", "llark_seq_rmsnorm_rows",
+    "llark_seq_step_ints", "llark_seq_embed", "llark_seq_short_conv", "llark_seq_conv_tail", "llark_seq_add_rmsnorm", "llark_seq_rmsnorm_rows",
     "llark_seq_relu2", "llark_linear_rows", "llark_linear_simt", "llark_seq_qk_headnorm", "llark_seq_swa_attn",
     "llark_seq_swa_attn_mma",
     "llark_seq_kv_ring_write", "llark_seq_glr_scan", "llark_seq_glr_combine", "llark_seq_head_rmsnorm",
@@ -149,6 +149,7 @@ def lib():
             "llark_v32_swiglu_fwd": ([P, P, LL, I, P], I),
             "llark_v32_attn_fwd": ([P, P, P, I, I, I, I, F, P], I),
             "llark_v32_ce_fwd": ([P, LL, I, P, I, I, P, P, P], I),
+            "llark_seq_step_ints": ([P, I, I, I, P, P], I),
             "llark_seq_embed": ([P, P, P, P, P, P, F, P, P, I, I, I, P], I),
             "llark_seq_short_conv": ([P, P, P, P, P, P, P, I, I, I, I, I, P], I),
             "llark_seq_conv_tail": ([P, P, P, P, I, I, I, P], I),
@@ -211,6 +212,40 @@ def lib():
             fn.argtypes = argtypes
             fn.restype = restype
     return _lib
+
+
+_calls = None
+
+
+def calls():
+    """The entry points to call them often: lib()'s, those that launch something as native functions (csrc/calls.cpp) where the package has
+    them built; structures and arrays go in by ref()."""
+    global _calls
+    if _calls is None:
+        c = lib()
+        try:
+            from . import _calls as native
+        except ImportError:  # built without Python's headers
+            native = None
+        have = set(native.bind(os.path.abspath(c._name))) if native else set()
+        ns = _Calls()
+        for name in SYMBOLS:
+            if name in have:
+                setattr(ns, name, getattr(native, name))
+            elif hasattr(c, name):
+                setattr(ns, name, getattr(c, name))
+        ns.native = native is not None
+        _calls = ns
+    return _calls
+
+
+class _Calls:
+    pass
+
+
+def ref(x):
+    """A ctypes structure as an argument of calls()."""
+    return x if calls().native else ctypes.byref(x)
 
 
 def check(rc, what):

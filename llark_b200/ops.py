@@ -11,7 +11,7 @@ import numpy as np
 import torch
 
 from ._lib import (EPI_CLAMP_GLU, EPI_NONE, EPI_QUICK_GELU, EPI_RELU2, EPI_RELU_GLU, EPI_ROPE, EPI_SWIGLU, EPI_SWIGLU_BWD,
-                   GemmEpilogue, check, lib)
+                   GemmEpilogue, calls as lib, check, ref)
 
 BF16 = torch.bfloat16
 
@@ -114,7 +114,7 @@ def gemm(a, b, *, a_mn=False, b_mn=False, M=None, N=None, K=None, out=None, out_
                               int(bias_fp32), _p(residual), ldr, M, N, K, int(in_fp32), max_ctas, _stream())
     else:
         rc = lib().llark_gemm_ex(_p(a), int(a_mn), lda, _p(b), int(b_mn), ldb, _p(out), ldc, int(c_fp32), _p(bias),
-                                 int(bias_fp32), _p(residual), ldr, M, N, K, int(in_fp32), max_ctas, ctypes.byref(ep),
+                                 int(bias_fp32), _p(residual), ldr, M, N, K, int(in_fp32), max_ctas, ref(ep),
                                  _stream())
     if rc:
         check(rc, f"llark_gemm(M={M},N={N},K={K})")
@@ -584,6 +584,16 @@ def linear(a, w, bias=None, out_dtype=None, out=None, act=None, act_limit=0.0, a
         LINEAR_STATS["simt"] += 1
         check(lib().llark_linear_simt(pa, lda, pw, ldw, pc, ldc, c_fp32, _p(bias), M, N, K, in_fp32, code, float(act_limit),
                                       float(act_slope), _stream()), "linear_simt")
+    return out
+
+
+STEP_INTS = 8000  # LLARK_STEP_INTS
+
+
+def seq_step_ints(values, n_seq, n_tok, device):
+    """tok_seq | values on the device; values: array.array of C ints (cu | pos0 | slots | lens | others), free again on return."""
+    out = torch.empty(n_tok + len(values), device=device, dtype=torch.int32)
+    check(lib().llark_seq_step_ints(values.buffer_info()[0], len(values), n_seq, n_tok, out.data_ptr(), _stream()), "seq_step_ints")
     return out
 
 

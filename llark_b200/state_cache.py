@@ -14,49 +14,57 @@ kept in place.
 Sized for one B200: a ring is min(window, max_positions) entries per slot whatever the sequence length; a recurrent
 state is heads x dim x vdim fp32 per slot.
 """
+from array import array
+from itertools import accumulate
+
 import numpy as np
 import torch
+
+from . import ops
+
+
+def _current(device):
+    """Whether `device` is the GPU that the library launches on."""
+    d = device if isinstance(device, torch.device) else torch.device(device)
+    return d.type == "cuda" and (d.index is None or d.index == torch.cuda.current_device())
 
 
 class StepLayout:
     """One packed step on the device: request b brings lens[b] tokens that start at position pos0[b] of its sequence and
-    owns slot slots[b]. tok_seq[t] = request of row t; cu[b] = first row of request b. One pinned host buffer, one copy, which
-    takes the integers of `extra` along (self.extra: their int32 tensors on the device)."""
+    owns slot slots[b]. tok_seq[t] = request of row t; cu[b] = first row of request b. They and the integers of `extra`
+    (self.extra: their int32 tensors on the device) come with one launch, larger steps and other devices' with one copy."""
 
     def __init__(self, lens, pos0, slots, device, extra=()):
         n_seq = len(lens)
-        n_tok = int(sum(lens))
         if n_seq == 0 or min(lens) <= 0:
             raise ValueError("a step needs at least one token for every request in it")
+        self.lens, self.pos0_host, self.slots_host = [int(n) for n in lens], [int(p) for p in pos0], [int(s) for s in slots]
+        self.cu_host = cu = list(accumulate(self.lens, initial=0))
+        self.n_seq, self.n_tok, self.max_len = n_seq, cu[-1], max(self.lens)
+        self.device, self._chunks = device, {}
+        self.tables = {}  # what ops computed once for this step (rotary cosines and sines by frequencies)
         sizes = [len(e) for e in extra]
+        if 4 * n_seq + 1 + sum(sizes) <= ops.STEP_INTS and _current(device):
+            values = array("i", cu + self.pos0_host + self.slots_host + self.lens)
+            for e in extra:
+                values.extend(e.tolist() if isinstance(e, np.ndarray) else e)
+            dev = ops.seq_step_ints(values, n_seq, self.n_tok, device)
+        else:
+            dev = self._copied(sizes, extra)
+        self.tok_seq, self.cu, self.pos0, self.slot, self.lens_dev, *self.extra = dev.split([self.n_tok, n_seq + 1, n_seq, n_seq, n_seq] + sizes)
+
+    def _copied(self, sizes, extra):
+        n_seq, n_tok, device, lens, cu = self.n_seq, self.n_tok, self.device, self.lens, self.cu_host
         host = torch.empty(n_tok + 4 * n_seq + 1 + sum(sizes), dtype=torch.int32, pin_memory=torch.device(device).type == "cuda")
         a = host.numpy()
-        cu = [0]
-        for n in lens:
-            cu.append(cu[-1] + int(n))
         a[:n_tok] = np.arange(n_seq) if n_tok == n_seq else np.repeat(np.arange(n_seq), lens)
         at = n_tok + 4 * n_seq + 1
-        a[n_tok:at] = cu + [int(p) for p in pos0] + [int(s) for s in slots] + [int(n) for n in lens]
+        a[n_tok:at] = cu + self.pos0_host + self.slots_host + lens
         for e, n in zip(extra, sizes):
             a[at:at + n] = e
             at += n
-        dev = host.to(device, non_blocking=True)
-        at = n_tok + 4 * n_seq + 1
-        self.extra = []
-        for n in sizes:
-            self.extra.append(dev[at:at + n])
-            at += n
         self._host = host  # keeps the pinned buffer alive until the copy has run
-        self.tok_seq = dev[:n_tok]
-        self.cu = dev[n_tok:n_tok + n_seq + 1]
-        self.pos0 = dev[n_tok + n_seq + 1:n_tok + 2 * n_seq + 1]
-        self.slot = dev[n_tok + 2 * n_seq + 1:n_tok + 3 * n_seq + 1]
-        self.lens_dev = dev[n_tok + 3 * n_seq + 1:n_tok + 4 * n_seq + 1]
-        self.device, self.slots_host, self._chunks = device, [int(s) for s in slots], {}
-        self.tables = {}  # what ops computed once for this step (rotary cosines and sines by frequencies)
-        self.n_tok, self.n_seq = n_tok, n_seq
-        self.max_len = int(max(lens))
-        self.lens, self.cu_host, self.pos0_host = [int(n) for n in lens], cu, [int(p) for p in pos0]
+        return host.to(device, non_blocking=True)
 
 
 class _Chunks:
