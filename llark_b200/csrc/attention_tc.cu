@@ -8,7 +8,7 @@
 // each) so one CTA's softmax overlaps the other's MMAs:
 //   warp 0 (one lane) : TMA producer. Q tile once (4 boxes of 64 rows x 128 B), then the K / V tiles of 64 keys in the
 //                       order the MMA warp consumes them (K0, K1, V0, K2, V1, ...) through a 3-slot 16 KB ring.
-//   warp 1            : TMEM allocator; one lane issues tcgen05.mma:
+//   warp 1            : TMEM allocator; issues tcgen05.mma, the warp together (see warp_umma_f16):
 //                         S[j&1] (128 x 64 fp32, TMEM)  = Q (K-major smem) . K_j^T (K-major smem)       8 x K16
 //                         O      (128 x 128 fp32, TMEM) += P_j (K-major smem, bf16) . V_j (MN-major smem) 4 x K16
 //                       S is double-buffered so Q.K_{j+1}^T runs while the softmax warps work on S_j.
@@ -17,6 +17,11 @@
 //                       128-byte-swizzled K-major layout the UMMA descriptor expects. When a row's running max moved,
 //                       the O accumulator is rescaled in TMEM (tcgen05.ld / tcgen05.st) before P.V_j is issued.
 //                       Epilogue: O / l -> bf16, LSE (natural log, +inf for a fully masked row).
+// What bounds it: softmax and products of a tile in turn, two CTAs filling each other's gaps: without the products it would take 140 us of
+// 168 (4 x 32 heads x 2048 tokens), without the softmax 127. Measured, us, before -> now: 4 x 32 x 2048 183 -> 168 (right-padded samples
+// 202 -> 180), 1 x 32 x 2048 64 -> 47, 1 x 32 x 4096 178 -> 148, 16 x 32 x 512 88 -> 84: products issued by the warp, heads placed in groups
+// (place), pairs of numbers per instruction and a mask word per 32 keys in the softmax. Tried: two threads a row 196 against 183; tiles of
+// 128 keys with P in TMEM 175, the same with two query tiles a CTA that share the keys 181.
 #include "common.cuh"
 #include "../../include/llark_b200.h"
 #include <cuda.h>
@@ -53,6 +58,7 @@ constexpr int HD = 128;
 constexpr int BQ = 128;         // query rows per CTA
 constexpr int BK = 64;          // keys per tile
 constexpr int kThreads = 192;
+constexpr int kGroup = 32;      // heads whose tiles are handed out together
 constexpr int kSlots = 3;       // K/V ring
 constexpr int Q_BYTES = BQ * HD * 2;        // 32 KB: 2 d-chunks x 128 rows x 128 B
 constexpr int KV_BYTES = BK * HD * 2;       // 16 KB: 2 d-chunks x 64 rows x 128 B
@@ -94,6 +100,29 @@ __device__ __forceinline__ float ex2(float x) {
 }
 __device__ __forceinline__ void softmax_group_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
+// two numbers in one register pair: one instruction for both
+__device__ __forceinline__ uint64_t two(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void apart(uint64_t r, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
 struct Ring {
     int slot = 0;
     uint32_t phase = 0;
@@ -105,9 +134,20 @@ struct Ring {
     }
 };
 
+// Which tile, head and sample a CTA takes: heads in groups of kGroup, of a group the longest tiles of all heads first (rank 0), then the
+// next ones. What runs at a time shares its keys and values in L2, and the last CTAs are short: with one head's tiles behind another's a
+// quarter of the SMs' time went by behind their last CTA (1 x 32 heads x 2048: 64 -> 48 us, 4 x 32 x 2048: 183 -> 168).
+__device__ __forceinline__ void place(int n_tiles, int n_heads, int n_batch, int& rank, int& h, int& b) {
+    const int group = blockIdx.x / (kGroup * n_tiles), at = blockIdx.x % (kGroup * n_tiles);
+    const int size = min(kGroup, n_heads * n_batch - group * kGroup), head = group * kGroup + at % size;
+    rank = at / size;
+    h = head % n_heads;
+    b = head / n_heads;
+}
+
 __global__ void __launch_bounds__(kThreads, 2)
 attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const unsigned char* __restrict__ mask,
-                   __nv_bfloat16* __restrict__ O, float* __restrict__ lse_out, int S, int NH, float scale_log2
+                   __nv_bfloat16* __restrict__ O, float* __restrict__ lse_out, int S, int NH, int n_batch, float scale_log2
                    LLARK_ATC_SLOPES_PARAM) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -125,9 +165,10 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const unsigned ch
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 1);
     uint32_t* maskw = reinterpret_cast<uint32_t*>(smem + OFF_MASK);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int qt = gridDim.x - 1 - blockIdx.x;  // longest rows first
-    const int h = blockIdx.y, b = blockIdx.z;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    int rank, h, b;
+    place((S + BQ - 1) / BQ, NH, n_batch, rank, h, b);
+    const int qt = (S + BQ - 1) / BQ - 1 - rank;
     const int q0 = qt * BQ;
     const int n_key_tiles = (S + BK - 1) / BK;
     const int n_kv = min(n_key_tiles, (q0 + BQ) / BK);  // causal: keys <= q0 + 127
@@ -182,7 +223,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const unsigned ch
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             // ===================== MMA issuer =====================
             // instruction descriptors: F32 accumulate, bf16 operands; S: M128 N64, both K-major;
             // PV: M128 N128, A (P) K-major, B (V, stored [key][d]) MN-major
@@ -207,10 +248,10 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const unsigned ch
                 for (int k = 0; k < 8; ++k) {
                     const uint64_t ad = (k < 4 ? qdesc0 : qdesc1) + (uint64_t)((k & 3) * 2);
                     const uint64_t bd = (k < 4 ? kdesc0 : kdesc1) + (uint64_t)((k & 3) * 2);
-                    umma_f16(tS, ad, bd, idesc_s, k != 0);
+                    warp_umma_f16(tS, ad, bd, idesc_s, k != 0);
                 }
-                umma_commit(&kv_empty[r.slot]);
-                umma_commit(&s_full[sb]);
+                warp_umma_commit(&kv_empty[r.slot]);
+                warp_umma_commit(&s_full[sb]);
                 r.advance();
             };
             mbar_wait(q_full, 0);
@@ -223,9 +264,9 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const unsigned ch
                 const uint64_t vdesc = make_desc(smem_u32(sKV + r.slot * KV_BYTES), BK * 128, 1024);
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
-                    umma_f16(tmem_O, pdesc + (uint64_t)(k * 2), vdesc + (uint64_t)(k * 128), idesc_pv, (j | k) != 0);
-                umma_commit(&kv_empty[r.slot]);
-                umma_commit(pv_done);
+                    warp_umma_f16(tmem_O, pdesc + (uint64_t)(k * 2), vdesc + (uint64_t)(k * 128), idesc_pv, (j | k) != 0);
+                warp_umma_commit(&kv_empty[r.slot]);
+                warp_umma_commit(pv_done);
                 r.advance();
             }
         }
@@ -299,26 +340,23 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const unsigned ch
                 }
 #else
             // row max of the RAW scores (scale > 0, so the max commutes with the scaling); masked entries -> -inf
-            float rmax = -INFINITY;
-            if (plain) {
-#pragma unroll
-                for (int hh = 0; hh < 2; ++hh)
-#pragma unroll
-                    for (int c = 0; c < 32; ++c) rmax = fmaxf(rmax, __uint_as_float(sv[hh][c]));
-            } else {
+            if (!plain) {
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh) {
-                    const uint32_t mw = hh ? mw1 : mw0;
+                    const int last = qi - (k0 + hh * 32);  // the last of these keys that the row may see
+                    const uint32_t seen = (hh ? mw1 : mw0) & (last >= 31 ? 0xffffffffu : last < 0 ? 0u : (2u << last) - 1u);
 #pragma unroll
-                    for (int c = 0; c < 32; ++c) {
-                        const int key = k0 + hh * 32 + c;
-                        const bool ok = key <= qi && ((mw >> c) & 1u);
-                        const float v = ok ? __uint_as_float(sv[hh][c]) : -INFINITY;
-                        sv[hh][c] = __float_as_uint(v);
-                        rmax = fmaxf(rmax, v);
-                    }
+                    for (int c = 0; c < 32; ++c)
+                        if (!((seen >> c) & 1u)) sv[hh][c] = __float_as_uint(-INFINITY);
                 }
             }
+            float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh)
+#pragma unroll
+                for (int c = 0; c < 32; c += 2)
+                    top[(c >> 1) & 3] = max3(top[(c >> 1) & 3], __uint_as_float(sv[hh][c]), __uint_as_float(sv[hh][c + 1]));
+            const float rmax = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
             // Lazy rescaling: the reference maximum m_run only moves when the true maximum has grown by more than
             // 2^8 (probabilities then stay <= 256, exact enough in bf16 / fp32), so the TMEM round trip that rescales
             // O is rare after the first tile. O / l and LSE = m*ln2 + log(l) are invariant to the choice of m_run.
@@ -328,17 +366,23 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const unsigned ch
             const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
             const float alpha = ex2(m_run - m_use);
             m_run = m_new;
-            float psum = 0.f;
             uint32_t pk[32];  // 64 bf16 probabilities
+            uint64_t psum2[2] = {0, 0};
+            const uint64_t scale2 = two(scale_log2, scale_log2), shift2 = two(-m_use, -m_use);
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh)
 #pragma unroll
                 for (int c = 0; c < 32; c += 2) {
-                    const float p0 = ex2(fmaf(__uint_as_float(sv[hh][c]), scale_log2, -m_use));
-                    const float p1 = ex2(fmaf(__uint_as_float(sv[hh][c + 1]), scale_log2, -m_use));
-                    psum += p0 + p1;
+                    float p0, p1;
+                    apart(fma2(two(__uint_as_float(sv[hh][c]), __uint_as_float(sv[hh][c + 1])), scale2, shift2), p0, p1);
+                    p0 = ex2(p0);
+                    p1 = ex2(p1);
+                    psum2[(c >> 1) & 1] = add2(psum2[(c >> 1) & 1], two(p0, p1));
                     pk[hh * 16 + (c >> 1)] = pack_bf16x2(p0, p1);
                 }
+            float psum, psum1;
+            apart(add2(psum2[0], psum2[1]), psum, psum1);
+            psum += psum1;
 #endif
             l_run = l_run * alpha + psum;
 
@@ -427,7 +471,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const unsigned ch
 // What bounds it: in the dQ kernel the MMAs, some 2050 cycles a tile of 128 keys (an MMA of 128 rows takes 54 to 84 cycles at N = 64 and
 // 72 at 128, and 300 more after the tensor pipe ran dry), and 5000 cycles a CTA before its first and after its last; in the dK/dV kernel
 // shared memory, which its A operands, P^T and dS^T pass through (TMEM is full). Measured on a B200, 4 x 32 heads x 2048 tokens, us:
-// dQ 352 -> 228, dK/dV 442 -> 364. Of the dQ kernel's, tiles of 128 with every load a tile ahead 283 (with four slots, where the load of K_j+2
+// dQ 352 -> 228, dK/dV 442 -> 364; with products issued by whole warps 206 and 330. Of the dQ kernel's, tiles of 128 with every load a tile ahead 283 (with four slots, where the load of K_j+2
 // waits for tile j's last MMA, 352 as before), two issuers 245, sixteen compute warps 241; of the dK/dV kernel's, two issuers 434, sixteen
 // compute warps that take tiles in turn 405; the rest by first loads that do not wait for TMEM and results that leave through TMA.
 constexpr int kBwdThreads = 64 + 512 + 32;
@@ -445,7 +489,7 @@ __device__ __forceinline__ void mma_kk(uint32_t tD, uint32_t a_addr, uint32_t b_
     const uint64_t b0 = make_desc(b_addr, 0, 1024), b1 = make_desc(b_addr + N * 128, 0, 1024);
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-        umma_f16(tD, (k < 4 ? a0 : a1) + (uint64_t)((k & 3) * 2), (k < 4 ? b0 : b1) + (uint64_t)((k & 3) * 2), idesc,
+        warp_umma_f16(tD, (k < 4 ? a0 : a1) + (uint64_t)((k & 3) * 2), (k < 4 ? b0 : b1) + (uint64_t)((k & 3) * 2), idesc,
                  k != 0);
 }
 __device__ __forceinline__ void mma_pv_128x128(uint32_t tD, uint32_t a_addr, uint32_t b_addr, uint32_t idesc,
@@ -454,21 +498,14 @@ __device__ __forceinline__ void mma_pv_128x128(uint32_t tD, uint32_t a_addr, uin
     const uint64_t bd = make_desc(b_addr, BK * 128, 1024);  // MN-major: the two 64-wide N chunks are 8 KB apart
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-        umma_f16(tD, ad + (uint64_t)(k * 2), bd + (uint64_t)(k * 128), idesc, accumulate || k != 0);
+        warp_umma_f16(tD, ad + (uint64_t)(k * 2), bd + (uint64_t)(k * 128), idesc, accumulate || k != 0);
 }
 // the same with A (bf16, two columns of K in one) in TMEM; b_addr: 64 of the rows of a 128-row tile
 __device__ __forceinline__ void mma_pv_tmem(uint32_t tD, uint32_t tA, uint32_t b_addr, uint32_t idesc, bool accumulate) {
     const uint64_t bd = make_desc(b_addr, BQ * 128, 1024);  // MN-major: the two 64-wide N chunks are 16 KB apart
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-        asm volatile(
-            "{\n"
-            ".reg .pred p;\n"
-            "setp.ne.b32 p, %4, 0;\n"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
-            "}\n" ::"r"(tD),
-            "r"(tA + 8 * k), "l"(bd + (uint64_t)(k * 128)), "r"(idesc), "r"((uint32_t)(accumulate || k != 0))
-            : "memory");
+        warp_umma_f16_ts(tD, tA + 8 * k, bd + (uint64_t)(k * 128), idesc, accumulate || k != 0);
 }
 // a 128-row tile of 128 columns: two column chunks of 128 bytes, boxes of 64 rows
 __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int col, int row, int b) {
@@ -603,7 +640,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
                       const __grid_constant__ CUtensorMap tm_out,
                       const unsigned char* __restrict__ mask, const float* __restrict__ lse,
-                      const float* __restrict__ Dsum, __nv_bfloat16* __restrict__ dqkv, int S, int NH, float scale,
+                      const float* __restrict__ Dsum, __nv_bfloat16* __restrict__ dqkv, int S, int NH, int n_batch, float scale,
                       float scale_log2, const __nv_bfloat16* __restrict__ rope_cos,
                       const __nv_bfloat16* __restrict__ rope_sin LLARK_ATC_SLOPES_PARAM) {
     extern __shared__ uint8_t smem_raw[];
@@ -626,9 +663,10 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(dq_all + 1);
     uint32_t* maskw = reinterpret_cast<uint32_t*>(smem + DQ_OFF_MASK);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int qt = gridDim.x - 1 - blockIdx.x;
-    const int h = blockIdx.y, b = blockIdx.z;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    int rank, h, b;
+    place((S + BQ - 1) / BQ, NH, n_batch, rank, h, b);
+    const int qt = (S + BQ - 1) / BQ - 1 - rank;
     const int q0 = qt * BQ;
     const int n_key_tiles = (S + BK - 1) / BK;
     const int n_half = min(n_key_tiles, (q0 + BQ) / BK);  // halves of 64 keys in all
@@ -676,7 +714,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             const uint32_t idesc_kk = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BQ >> 3) << 17) |
                                       ((uint32_t)(BQ >> 4) << 24);
             mbar_wait(q_full, 0);
@@ -689,12 +727,12 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
                 mbar_wait(&v_full[vs], (uint32_t)(j / V_SLOTS) & 1);
                 tc_fence_after();
                 mma_kk<BQ>(tmem_base + 128, smem_u32(sdO), smem_u32(sVt + vs * TILE_BYTES), idesc_kk);
-                umma_commit(&v_empty[vs]);  // V_j is not needed again
-                umma_commit(sdp_full);
+                warp_umma_commit(&v_empty[vs]);  // V_j is not needed again
+                warp_umma_commit(sdp_full);
             }
         }
     } else if (warp == kBwdThreads / 32 - 1) {
-        if (lane == 0) {  // a warp of its own: the tensor pipe has one kind of products while the other's operands are waited for
+        {  // a warp of its own: the tensor pipe has one kind of products while the other's operands are waited for
             const uint32_t idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) |
                                       ((uint32_t)(BQ >> 4) << 24);
             for (int j = 0; j < n_kv; ++j) {
@@ -704,11 +742,11 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
                     tc_fence_after();
                     mma_pv_tmem(tmem_base + 256, tmem_base + 384 + hf * 32, smem_u32(sKt + ks * TILE_BYTES + hf * (64 * 128)), idesc_pv,
                                 j + hf != 0);
-                    umma_commit(&dq_done[hf]);
+                    warp_umma_commit(&dq_done[hf]);
                 }
-                umma_commit(&k_empty[ks]);
+                warp_umma_commit(&k_empty[ks]);
             }
-            umma_commit(dq_all);
+            warp_umma_commit(dq_all);
         }
     } else {
         const int cw = warp - 2;
@@ -812,7 +850,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
                         const __grid_constant__ CUtensorMap tm_out,
                         const unsigned char* __restrict__ mask, const float* __restrict__ lse,
-                        const float* __restrict__ Dsum, __nv_bfloat16* __restrict__ dqkv, int S, int NH, float scale,
+                        const float* __restrict__ Dsum, __nv_bfloat16* __restrict__ dqkv, int S, int NH, int n_batch, float scale,
                         float scale_log2, const __nv_bfloat16* __restrict__ rope_cos,
                         const __nv_bfloat16* __restrict__ rope_sin LLARK_ATC_SLOPES_PARAM) {
     extern __shared__ uint8_t smem_raw[];
@@ -834,9 +872,9 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(kv_all + 1);
     float* rowv = reinterpret_cast<float*>(smem + KV_OFF_ROWV);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kt = blockIdx.x;  // key tile 0 has the most query tiles and starts first
-    const int h = blockIdx.y, b = blockIdx.z;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    int kt, h, b;
+    place((S + BQ - 1) / BQ, NH, n_batch, kt, h, b);  // key tile 0 has the most query tiles
     const int k0 = kt * BQ;
     const int n_q_tiles = (S + BK - 1) / BK;
     const int t0 = k0 / BK;               // first 64-query tile that can see these keys
@@ -893,7 +931,7 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             const uint32_t idesc_kk = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BK >> 3) << 17) |
                                       ((uint32_t)(BQ >> 4) << 24);
             mbar_wait(kv_full, 0);
@@ -907,11 +945,11 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
                 mbar_wait(&ring_full[ring_slot(itd)], ring_phase(itd));
                 tc_fence_after();
                 mma_kk<BK>(tmem_base + 128 + sb * BK, smem_u32(sV), smem_u32(sRing + ring_slot(itd) * KV_BYTES), idesc_kk);
-                umma_commit(&sdp_full[sb]);
+                warp_umma_commit(&sdp_full[sb]);
             }
         }
     } else if (warp == kBwdThreads / 32 - 1) {
-        if (lane == 0) {
+        {
             const uint32_t idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) |
                                       ((uint32_t)(BQ >> 4) << 24);
             for (int t = 0; t < n_it; ++t) {
@@ -920,13 +958,13 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
                 const int itq = 2 * t, itd = 2 * t + 1;
                 mma_pv_128x128(tmem_base + 256, smem_u32(sPT + (t & 1) * P_BYTES),
                                smem_u32(sRing + ring_slot(itd) * KV_BYTES), idesc_pv, t != 0);
-                umma_commit(&ring_empty[ring_slot(itd)]);
+                warp_umma_commit(&ring_empty[ring_slot(itd)]);
                 mma_pv_128x128(tmem_base + 384, smem_u32(sdST + (t & 1) * P_BYTES),
                                smem_u32(sRing + ring_slot(itq) * KV_BYTES), idesc_pv, t != 0);
-                umma_commit(&ring_empty[ring_slot(itq)]);
-                umma_commit(&pds_done[t & 1]);
+                warp_umma_commit(&ring_empty[ring_slot(itq)]);
+                warp_umma_commit(&pds_done[t & 1]);
             }
-            umma_commit(kv_all);
+            warp_umma_commit(kv_all);
         }
     } else {
         const int cw = warp - 2;
@@ -1063,8 +1101,7 @@ int LLARK_ATC_FWD_LAUNCH(const void* qkv, const unsigned char* key_mask, void* o
         }
         attr_set = true;
     }
-    dim3 grid((S + BQ - 1) / BQ, n_heads, B);
-    attn_fwd_tc_kernel<<<grid, kThreads, SMEM_BYTES, st>>>(tm, key_mask, (__nv_bfloat16*)out, lse, S, n_heads,
+    attn_fwd_tc_kernel<<<(unsigned)((S + BQ - 1) / BQ * n_heads * B), kThreads, SMEM_BYTES, st>>>(tm, key_mask, (__nv_bfloat16*)out, lse, S, n_heads, B,
                                                            scale * LOG2E LLARK_ATC_SLOPES_ARG);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -1102,13 +1139,13 @@ int LLARK_ATC_BWD_LAUNCH(const void* qkv, const unsigned char* key_mask, const v
         }
         attr_set = true;
     }
-    dim3 grid((S + BQ - 1) / BQ, n_heads, B);
+    const unsigned grid = (unsigned)((S + BQ - 1) / BQ * n_heads * B);
     attn_bwd_dkdv_tc_kernel<<<grid, kBwdThreads, KV_SMEM_BYTES, st>>>(tq, td, to, key_mask, lse, Dsum, (__nv_bfloat16*)dqkv,
-                                                                      S, n_heads, scale, scale * LOG2E,
+                                                                      S, n_heads, B, scale, scale * LOG2E,
                                                                       (const __nv_bfloat16*)rope_cos,
                                                                       (const __nv_bfloat16*)rope_sin LLARK_ATC_SLOPES_ARG);
     attn_bwd_dq_tc_kernel<<<grid, kBwdThreads, DQ_SMEM_BYTES, st>>>(tq, td, to, key_mask, lse, Dsum, (__nv_bfloat16*)dqkv, S,
-                                                                    n_heads, scale, scale * LOG2E,
+                                                                    n_heads, B, scale, scale * LOG2E,
                                                                     (const __nv_bfloat16*)rope_cos,
                                                                     (const __nv_bfloat16*)rope_sin LLARK_ATC_SLOPES_ARG);
     cudaError_t e = cudaGetLastError();
