@@ -27,10 +27,10 @@
 // gets there. What it cannot tell: single products beyond the largest number, of both signs in one sum, are NaN and not the first one's
 // infinity. (A look at all 32 channels for large numbers: 678 us where this takes 633.)
 //
-// What bounds it: a product of 128 rows takes 50 to 60 cycles whatever its N up to 96 (its A operand's 4 KB from shared memory; from TMEM
-// 85), 28 of them a group and block, and some 800 instructions a warp and block between them; 8700 cycles a block and window. Measured
-// on a B200, 4 clips x 524288 steps, dilations 1, 3, 9, 27: 633 us where four launches of one block took 1075; one block alone 181 to 198
-// (257). Error of the encoder against 64 bits 2.2e-6 (2.9e-6). Tried: both convolutions from shared memory, all groups in step: 820;
+// What bounds it: 28 products a group and block, one behind another, and some 800 instructions a warp and block between them; 6500 cycles a
+// block and window. Measured on a B200, 4 clips x 524288 steps, dilations 1, 3, 9, 27: 477 us where four launches of one block took 1075;
+// one block alone 158 to 171 (257). Issued by one lane instead of a warp together a product took 50 to 85 cycles whatever its N, and the
+// four blocks 634 us. Error of the encoder against 64 bits 2.2e-6 (2.9e-6). Tried: both convolutions from shared memory, all groups in step: 820;
 // hidden rows in TMEM, all groups in step: 772; two windows of 256 steps side by side: 999; parts cut instead of rounded: 669.
 #include "common.cuh"
 
@@ -102,33 +102,23 @@ __device__ __forceinline__ void tap_products(uint32_t a, uint32_t w, uint32_t d,
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
         const uint64_t o = (uint64_t)(2 * k);  // 16 channels = 32 bytes
-        umma_f16(d, a1 + o, b + o, idesc_bf16(96), !(first && k == 0));
-        umma_f16(d + 32, a2 + o, b + o, idesc_bf16(64), 1);
-        umma_f16(d + 64, a3 + o, b + o, idesc_bf16(32), 1);
+        warp_umma_f16(d, a1 + o, b + o, idesc_bf16(96), !(first && k == 0));
+        warp_umma_f16(d + 32, a2 + o, b + o, idesc_bf16(64), 1);
+        warp_umma_f16(d + 64, a3 + o, b + o, idesc_bf16(32), 1);
     }
 }
 // the second convolution: A is this group's own rows, so they stay in TMEM (16 columns for each part from a on); c2's products go to c1
-__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
-        "}\n" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 __device__ __forceinline__ void second_products(uint32_t a, uint32_t w, uint32_t d) {
     const uint64_t b1 = desc64(w), b2 = desc64(w + 32 * 64), b3 = desc64(w + 64 * 64);
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
         const uint64_t o = (uint64_t)(2 * k);
         const uint32_t a1 = a + 8 * k;  // 16 channels = 8 columns
-        umma_f16_ts(d, a1, b1 + o, idesc_bf16(64), k != 0);
-        umma_f16_ts(d + 32, a1, b3 + o, idesc_bf16(32), 1);
-        umma_f16_ts(d + 32, a1 + 16, b1 + o, idesc_bf16(32), 1);
-        umma_f16_ts(d + 32, a1 + 16, b2 + o, idesc_bf16(32), 1);
-        umma_f16_ts(d + 32, a1 + 32, b1 + o, idesc_bf16(32), 1);
+        warp_umma_f16_ts(d, a1, b1 + o, idesc_bf16(64), k != 0);
+        warp_umma_f16_ts(d + 32, a1, b3 + o, idesc_bf16(32), 1);
+        warp_umma_f16_ts(d + 32, a1 + 16, b1 + o, idesc_bf16(32), 1);
+        warp_umma_f16_ts(d + 32, a1 + 16, b2 + o, idesc_bf16(32), 1);
+        warp_umma_f16_ts(d + 32, a1 + 32, b1 + o, idesc_bf16(32), 1);
     }
 }
 __device__ __forceinline__ void tmem_st_x4(uint32_t taddr, uint4 u) {
@@ -193,7 +183,7 @@ chain_kernel(const __grid_constant__ ChainArgs p) {
     unsigned char* sa = raw + ((1024u - (smem_u32(raw) & 1023u)) & 1023u);
     unsigned char* sw = sa + 3 * kPart;
     float* sb = reinterpret_cast<float*>(sw + kMost * kBlockBytes);  // [block][b1 | b2]
-    const int g = threadIdx.x >> 7, tid = threadIdx.x & 127, warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
+    const int g = __shfl_sync(0xffffffffu, threadIdx.x >> 7, 0), warp = __shfl_sync(0xffffffffu, (threadIdx.x >> 5) & 3, 0), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int i = 0; i < 4; ++i) {
             mbar_init(&ready[i], 4);
@@ -266,7 +256,7 @@ chain_kernel(const __grid_constant__ ChainArgs p) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&ready[g]);
-            if (tid == 0) {
+            if (warp == 0) {  // of the group, together
                 if (g > 0) mbar_wait(&ready[g - 1], par);
                 mbar_wait(&ready[g], par);
                 if (g < 3) mbar_wait(&ready[g + 1], par);
@@ -276,8 +266,9 @@ chain_kernel(const __grid_constant__ ChainArgs p) {
                 const int d = p.dil[b] * 64;
 #pragma unroll
                 for (int tap = 0; tap < 3; ++tap) tap_products(a + (tap - 1) * d, w + tap * kTapBytes, tmem, tap == 0);
-                umma_commit(&done1[g]);
-                mbar_arrive(&turn[g]);
+                warp_umma_commit(&done1[g]);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&turn[g]);
             }
             __syncwarp();
             mbar_wait(&done1[g], par);
@@ -310,10 +301,10 @@ chain_kernel(const __grid_constant__ ChainArgs p) {
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc_fence_before();
             asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");
-            if (tid == 0) {
+            if (warp == 0) {  // of the group, together
                 tc_fence_after();
                 second_products(tmem + kHidden, smem_u32(sw) + b * kBlockBytes + 3 * kTapBytes, tmem);
-                umma_commit(&done2[g]);
+                warp_umma_commit(&done2[g]);
             }
             __syncwarp();
             mbar_wait(&done2[g], par);

@@ -94,12 +94,12 @@ __device__ __forceinline__ void products(uint32_t a, int lo_at, uint32_t w, uint
         const uint64_t o = (uint64_t)(2 * k);  // 8 channels = 32 bytes
         const bool f = first && k == 0, fl = first_lo && k == 0;
         if (f == fl) {
-            umma_tf32(both, ah + o, wd + o, idesc_tf32(2 * COUT), !f);
+            warp_umma_tf32(both, ah + o, wd + o, idesc_tf32(2 * COUT), !f);
         } else {
-            umma_tf32(hh, ah + o, wh + o, idesc_tf32(COUT), !f);
-            umma_tf32(mid, ah + o, wl + o, idesc_tf32(COUT), !fl);
+            warp_umma_tf32(hh, ah + o, wh + o, idesc_tf32(COUT), !f);
+            warp_umma_tf32(mid, ah + o, wl + o, idesc_tf32(COUT), !fl);
         }
-        umma_tf32(mid, al + o, wh + o, idesc_tf32(COUT), 1);
+        warp_umma_tf32(mid, al + o, wh + o, idesc_tf32(COUT), 1);
     }
 }
 
@@ -152,7 +152,7 @@ conv_kernel(const Args p) {
     __shared__ uint32_t tmem_base;
     __shared__ float sb[COUT + 32];
     constexpr int CIN = NCI * 32, kGroup = RES ? 160 : 3 * COUT, kCols = NG * kGroup > 256 ? 512 : 256;
-    const int grp = threadIdx.x >> 7, tid = threadIdx.x & 127, warp = (threadIdx.x >> 5) & 3;
+    const int grp = __shfl_sync(0xffffffffu, threadIdx.x >> 7, 0), tid = threadIdx.x & 127, warp = __shfl_sync(0xffffffffu, (threadIdx.x >> 5) & 3, 0);
     const int lo_at = p.rows * 128, region = 2 * lo_at;
     unsigned char* sw1 = raw + ((1024u - (smem_u32(raw) & 1023u)) & 1023u);
     unsigned char* sw2 = sw1 + TAPS * NCI * 2 * COUT * 128;
@@ -259,7 +259,7 @@ conv_kernel(const Args p) {
             fence_proxy_async_smem();
             tc_fence_before();
             group_sync();  // the rows are written, and the sums of the tile before have been read
-            if (tid == 0) {
+            if (warp == 0) {  // of the group, together
                 tc_fence_after();
                 const uint32_t a = smem_u32(sa), w = smem_u32(sw1) + cb * TAPS * 2 * COUT * 128;
 #pragma unroll
@@ -270,7 +270,7 @@ conv_kernel(const Args p) {
                     else
                         products<COUT, 0>(rows, lo_at, w + tap * 2 * COUT * 128, tmem, cb == 0 && tap == 0, cb == 0 && tap == 0);
                 }
-                umma_commit(bar);
+                warp_umma_commit(bar);
             }
             ++n;
         }
@@ -290,10 +290,10 @@ conv_kernel(const Args p) {
             fence_proxy_async_smem();
             tc_fence_before();
             group_sync();
-            if (tid == 0) {
+            if (warp == 0) {  // of the group, together
                 tc_fence_after();
                 products<32, 0>(smem_u32(sa), lo_at, smem_u32(sw2), tmem + 96, true, true);
-                umma_commit(bar);
+                warp_umma_commit(bar);
             }
             ++n;
             wait_last();

@@ -249,7 +249,7 @@ vq_kernel(const float* __restrict__ x, const float* __restrict__ cb, long long* 
     unsigned char* sa = raw + ((1024u - (smem_u32(raw) & 1023u)) & 1023u);
     unsigned char* sb = sa + 2 * kPartA;
     unsigned char* sl = sb + 2 * 2 * kPartB;
-    const int tid = threadIdx.x, row = tid & (ROWS - 1), part = tid / ROWS, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, row = tid & (ROWS - 1), part = tid / ROWS, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int v0 = blockIdx.x * ROWS, number = v0 + row, n = number / T;  // this thread's vector
     const bool vec = (reinterpret_cast<uintptr_t>(cb) & 15) == 0, in = number < vectors;
     if (tid == 0) {
@@ -304,19 +304,19 @@ vq_kernel(const float* __restrict__ x, const float* __restrict__ cb, long long* 
         if (lane == 0) atomicMax(&most_kk, most);
         fence_proxy_async_smem();
     };
-    auto multiply = [&](int tile) {  // one thread
+    auto multiply = [&](int tile) {  // one warp
         const uint32_t b = smem_u32(sb) + (tile & 1) * 2 * kPartB;
 #pragma unroll
         for (int rt = 0; rt < ROWS / 128; ++rt) {
             const uint32_t a = smem_u32(sa) + rt * 128 * 128, d = tmem + (tile & 1) * 256 + rt * kTile;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                umma_f16(d, desc(a) + 2 * k, desc(b) + 2 * k, kIdesc, k != 0);
-                umma_f16(d, desc(a) + 2 * k, desc(b + kPartB) + 2 * k, kIdesc, 1);
-                umma_f16(d, desc(a + kPartA) + 2 * k, desc(b) + 2 * k, kIdesc, 1);
+                warp_umma_f16(d, desc(a) + 2 * k, desc(b) + 2 * k, kIdesc, k != 0);
+                warp_umma_f16(d, desc(a) + 2 * k, desc(b + kPartB) + 2 * k, kIdesc, 1);
+                warp_umma_f16(d, desc(a + kPartA) + 2 * k, desc(b) + 2 * k, kIdesc, 1);
             }
         }
-        umma_commit(&bar[tile & 1]);
+        warp_umma_commit(&bar[tile & 1]);
     };
 
     float least = INFINITY;  // smallest s + eps so far
@@ -329,7 +329,7 @@ vq_kernel(const float* __restrict__ x, const float* __restrict__ cb, long long* 
     bool many = false;
     for (int tile = 0; tile < tiles; ++tile) {
         const int buf = tile & 1;
-        if (tid == 0) {
+        if (warp == 0) {
             tc_fence_after();
             multiply(tile);
         }

@@ -13,7 +13,8 @@
 //
 // What bounds it: the exponentials (16 per SM and clock) and the softmax around them; V and K are read from L2 by every head of a group.
 // Measured on a B200, 4 prompts of 2048 tokens, 32 heads over 8, window 1024: 224 us (459 TFLOP/s of visible pairs), seq_swa_mma.cu 722;
-// window 128: 99 against 253; 32 portions of 96 tokens behind 2000: 257 against 498.
+// window 128: 99 against 253; 32 portions of 96 tokens behind 2000: 257 against 498. With the products issued by the warp together (see
+// warp_umma_f16), two numbers per instruction and a mask word for 32 keys, 4 prompts of 2048 to 1173 tokens: 184 -> 150.
 #include "common.cuh"
 
 namespace llark {
@@ -119,7 +120,7 @@ swa_tc_kernel(const __grid_constant__ Args a) {
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint64_t *kv_full = bars, *kv_empty = kv_full + kSlots, *s_full = kv_empty + kSlots, *s_empty = s_full + 2, *p_full = s_empty + 2,
              *pv_done = p_full + 1;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int i = 0; i < kSlots; ++i) {
             mbar_init(&kv_full[i], 2);
@@ -201,8 +202,8 @@ swa_tc_kernel(const __grid_constant__ Args a) {
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(&kv_full[(issued - 1) % kSlots]);
-    } else if (warp == 2) {
-        if (lane == 0) {
+    } else if (warp == 2) {  // together
+        {
             constexpr uint32_t kBase = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BQ >> 4) << 24);  // fp32 sums, bf16 operands
             const uint32_t idesc_s = kBase | ((uint32_t)(BK >> 3) << 17), idesc_pv = kBase | (1u << 16) | ((uint32_t)(HD >> 3) << 17);
             const uint64_t q = make_desc(smem_u32(smem), 0), pd = make_desc(smem_u32(smem + kOffP), 0);
@@ -215,10 +216,10 @@ swa_tc_kernel(const __grid_constant__ Args a) {
                 const uint64_t k = make_desc(smem_u32(smem + kOffKV + slot * kSlotBytes), 0);
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
-                    umma_f16(tmem + sb * BK, q + (i >> 2) * (BQ * 128 >> 4) + (i & 3) * 2, k + (i >> 2) * (BK * 128 >> 4) + (i & 3) * 2,
+                    warp_umma_f16(tmem + sb * BK, q + (i >> 2) * (BQ * 128 >> 4) + (i & 3) * 2, k + (i >> 2) * (BK * 128 >> 4) + (i & 3) * 2,
                              idesc_s, i != 0);
-                umma_commit(&kv_empty[slot]);
-                umma_commit(&s_full[sb]);
+                warp_umma_commit(&kv_empty[slot]);
+                warp_umma_commit(&s_full[sb]);
                 ++used;
             };
             issue_s(0);
@@ -230,9 +231,9 @@ swa_tc_kernel(const __grid_constant__ Args a) {
                 tc_fence_after();
                 const uint64_t v = make_desc(smem_u32(smem + kOffKV + slot * kSlotBytes), BK * 128);  // [key][channel]: MN-major
 #pragma unroll
-                for (int i = 0; i < 4; ++i) umma_f16(tmem_o, pd + i * 2, v + i * 128, idesc_pv, (j | i) != 0);
-                umma_commit(&kv_empty[slot]);
-                umma_commit(pv_done);
+                for (int i = 0; i < 4; ++i) warp_umma_f16(tmem_o, pd + i * 2, v + i * 128, idesc_pv, (j | i) != 0);
+                warp_umma_commit(&kv_empty[slot]);
+                warp_umma_commit(pv_done);
                 ++used;
             }
         }
@@ -259,33 +260,53 @@ swa_tc_kernel(const __grid_constant__ Args a) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&s_empty[sb]);
-            float top[2] = {-INFINITY, -INFINITY};
             const bool whole = k0 >= lo_all && k0 + BK - 1 <= hi_all;
+            const uint64_t sc2 = two(sc, sc);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+#pragma unroll
+                for (int c = 0; c < 32; c += 2) {
+                    float x, y;
+                    apart(mul2(two(__uint_as_float(s[e][c]), __uint_as_float(s[e][c + 1])), sc2), x, y);
+                    s[e][c] = __float_as_uint(x);
+                    s[e][c + 1] = __float_as_uint(y);
+                }
+                if (!whole) {
+                    const int from = lo - (k0 + e * 32), to = hi - (k0 + e * 32);  // the row sees these of the 32 keys
+                    uint32_t seen = to < 0 || from > 31 ? 0u : to >= 31 ? 0xffffffffu : (2u << to) - 1u;
+                    if (from > 0 && from < 32) seen &= 0xffffffffu << from;
+#pragma unroll
+                    for (int c = 0; c < 32; ++c)
+                        if (!((seen >> c) & 1u)) s[e][c] = __float_as_uint(-INFINITY);
+                }
+            }
+            float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
             for (int e = 0; e < 2; ++e)
 #pragma unroll
-                for (int c = 0; c < 32; ++c) {
-                    float v = __uint_as_float(s[e][c]) * sc;
-                    if (!whole) v = k0 + e * 32 + c >= lo && k0 + e * 32 + c <= hi ? v : -INFINITY;
-                    s[e][c] = __float_as_uint(v);
-                    top[c & 1] = fmaxf(top[c & 1], v);
-                }
-            const float cand = fmaxf(m, fmaxf(top[0], top[1]));
+                for (int c = 0; c < 32; c += 2)
+                    top[(c >> 1) & 3] = max3(top[(c >> 1) & 3], __uint_as_float(s[e][c]), __uint_as_float(s[e][c + 1]));
+            const float cand = fmaxf(m, fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])));
             const float use = cand == -INFINITY ? 0.f : cand;
             const float alpha = ex2(m - use);
             m = cand;
-            float sum[2] = {0.f, 0.f};
+            uint64_t sum[2] = {0, 0};
+            const uint64_t less = two(-use, -use);
             uint32_t pk[32];
 #pragma unroll
             for (int e = 0; e < 2; ++e)
 #pragma unroll
                 for (int c = 0; c < 32; c += 2) {
-                    const float x = ex2(__uint_as_float(s[e][c]) - use), y = ex2(__uint_as_float(s[e][c + 1]) - use);
-                    sum[0] += x;
-                    sum[1] += y;
+                    float x, y;
+                    apart(add2(two(__uint_as_float(s[e][c]), __uint_as_float(s[e][c + 1])), less), x, y);
+                    x = ex2(x);
+                    y = ex2(y);
+                    sum[(c >> 1) & 1] = add2(sum[(c >> 1) & 1], two(x, y));
                     pk[e * 16 + (c >> 1)] = pack_bf16x2(x, y);
                 }
-            l = l * alpha + (sum[0] + sum[1]);
+            float s0, s1;
+            apart(add2(sum[0], sum[1]), s0, s1);
+            l = l * alpha + (s0 + s1);
             if (j > 0) {
                 mbar_wait(pv_done, (uint32_t)(j - 1) & 1);  // P's rows are free, O holds the tiles before
                 tc_fence_after();
