@@ -244,6 +244,10 @@ int llark_jb_resblock(const float* x, const float* w1, const float* b1, const fl
 int llark_jb_resblocks_length(const int* dilations, int n);
 int llark_jb_resblocks(const float* x, const float* const* weights, const int* dilations, int n, float* y, int N, int T,
                        cudaStream_t stream);
+/* llark_jb_conv_down of a waveform [N, 1, T] to 32 channels (w [32, 1, 4]) and n of such blocks behind it in one visit: y [N, 32, T / 2]; the
+ * convolution's result is not stored. */
+int llark_jb_wave_resblocks(const float* wave, const float* w, const float* bias, const float* const* weights, const int* dilations, int n,
+                            float* y, int N, int T, cudaStream_t stream);
 /* Conv1d(c_in -> c_out, k=3, s=1, p=1) + bias (block output projection 32 -> 64). */
 int llark_jb_conv_k3(const float* x, const float* w, const float* bias, float* y, int N, int c_in, int c_out, int T,
                      cudaStream_t stream);

@@ -41,7 +41,7 @@ SYMBOLS = [
     "llark_attn_fwd", "llark_attn_decode", "llark_attn_decode_packed", "llark_gemv", "llark_attn_alibi_fwd", "llark_attn_alibi_bwd", "llark_ln_fwd",
     "llark_ln_bwd_workspace", "llark_ln_bwd", "llark_gelu_fwd", "llark_gelu_bwd", "llark_attn_bwd_workspace", "llark_attn_bwd", "llark_ce_fwd", "llark_ce_bwd",
     "llark_sumsq_workspace", "llark_grad_sumsq", "llark_adamw_step", "llark_comm_unique_id", "llark_comm_init",
-    "llark_comm_destroy", "llark_grad_bucket_allreduce", "llark_jb_conv_down", "llark_jb_resblock", "llark_jb_resblocks_length", "llark_jb_resblocks", "llark_decode_scratch", "llark_decode_layers",
+    "llark_comm_destroy", "llark_grad_bucket_allreduce", "llark_jb_conv_down", "llark_jb_resblock", "llark_jb_resblocks_length", "llark_jb_resblocks", "llark_jb_wave_resblocks", "llark_decode_scratch", "llark_decode_layers",
     "llark_jb_conv_k3", "llark_jb_vq_encode", "llark_layernorm_fwd", "llark_jb_embed_tokens", "llark_jb_sparse_attn",
     "llark_jb_sparse_attn_tc",
     "llark_quick_gelu", "llark_add3", "llark_jb_pool", "llark_jb_pool_batched", "llark_colsum",
@@ -128,6 +128,7 @@ def lib():
             "llark_decode_layers": ([P, I, P, P, P, P, I, I, I, I, I, I, F, P, P], I),
             "llark_jb_resblocks_length": ([P, I], I),
             "llark_jb_resblocks": ([P, P, P, I, P, I, I, P], I),
+            "llark_jb_wave_resblocks": ([P, P, P, P, P, I, P, I, I, P], I),
             "llark_jb_conv_k3": ([P, P, P, P, I, I, I, I, P], I),
             "llark_jb_vq_encode": ([P, P, P, I, I, I, P], I),
             "llark_layernorm_fwd": ([P, P, P, P, I, LL, I, F, P], I),

@@ -52,7 +52,25 @@ struct ChainArgs {
     float* y;
     int dil[kMost], blocks, halo;  // halo: sum of the dilations
     int T, windows_per_clip, windows;
+    // WAVE: the blocks' input is the strided convolution of a waveform x [clips, 2 T] (one channel, taps 4, pad 1), made where it is needed:
+    const float *w0, *b0;
 };
+
+// Channel by channel, bias first and the taps in order, as the FMA kernel of that convolution sums: v are samples 2 t - 1 .. 2 t + 2.
+struct Samples { float v[4]; };
+__device__ __forceinline__ Samples samples(const ChainArgs& p, int clip, int t) {
+    const float* wave = p.x + (long long)clip * 2 * p.T;
+    Samples s;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int i = 2 * t - 1 + k;
+        s.v[k] = i >= 0 && i < 2 * p.T ? wave[i] : 0.f;
+    }
+    return s;
+}
+__device__ __forceinline__ float strided(const Samples& s, float4 w, float b) {
+    return fmaf(w.w, s.v[3], fmaf(w.z, s.v[2], fmaf(w.y, s.v[1], fmaf(w.x, s.v[0], b))));
+}
 
 __device__ __forceinline__ uint64_t desc64(uint32_t addr) {  // 64-byte rows, 8-row groups of 512 bytes, 64-byte swizzle
     return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)(512 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)4 << 61);
@@ -139,13 +157,20 @@ __device__ __forceinline__ void bias8(const float* b, float (&u)[8]) {
 }
 
 // A window by FMAs: bias first, channels outside, taps inside. A thread has a step, rows: [32][kWin].
+template <bool WAVE>
 __device__ __noinline__ void window_by_fma(const ChainArgs& p, float* rows, int win) {
     const int clip = win / p.windows_per_clip, i = threadIdx.x;
     const int t = (win - clip * p.windows_per_clip) * (kWin - 2 * p.halo) - p.halo + i;
     const bool in = t >= 0 && t < p.T;
     const long long at = (long long)clip * 32 * p.T + t;
     __syncthreads();  // the window before has been read
-    for (int c = 0; c < 32; ++c) rows[c * kWin + i] = in ? p.x[at + (long long)c * p.T] : 0.f;
+    if (WAVE) {
+        const Samples s = in ? samples(p, clip, t) : Samples{};
+        for (int c = 0; c < 32; ++c)
+            rows[c * kWin + i] = in ? strided(s, make_float4(p.w0[4 * c], p.w0[4 * c + 1], p.w0[4 * c + 2], p.w0[4 * c + 3]), p.b0[c]) : 0.f;
+    } else {
+        for (int c = 0; c < 32; ++c) rows[c * kWin + i] = in ? p.x[at + (long long)c * p.T] : 0.f;
+    }
 #pragma unroll 1
     for (int b = 0; b < p.blocks; ++b) {
         __syncthreads();
@@ -174,12 +199,15 @@ __device__ __noinline__ void window_by_fma(const ChainArgs& p, float* rows, int 
 __device__ __forceinline__ int bit_of(int win) { return min((win - (int)blockIdx.x) / (int)gridDim.x, 32 * 32 - 1); }
 __device__ __forceinline__ void again(uint32_t* odd, int win) { atomicOr(&odd[bit_of(win) >> 5], 1u << (bit_of(win) & 31)); }
 
+template <bool WAVE>
 __global__ void __launch_bounds__(kWin, 1)
 chain_kernel(const __grid_constant__ ChainArgs p) {
     extern __shared__ unsigned char raw[];
     __shared__ uint64_t ready[4], done1[4], done2[4], turn[4];  // per group: rows written; first products done; second products done; first products on their way
     __shared__ uint32_t tmem_base;
     __shared__ uint32_t odd[32];
+    __shared__ float4 sw0[WAVE ? 32 : 1];
+    __shared__ float sb0[WAVE ? 32 : 1];
     unsigned char* sa = raw + ((1024u - (smem_u32(raw) & 1023u)) & 1023u);
     unsigned char* sw = sa + 3 * kPart;
     float* sb = reinterpret_cast<float*>(sw + kMost * kBlockBytes);  // [block][b1 | b2]
@@ -196,6 +224,11 @@ chain_kernel(const __grid_constant__ ChainArgs p) {
     if (threadIdx.x < 32) {
         tmem_alloc(&tmem_base, 512);
         tmem_relinquish();
+    }
+    if (WAVE && threadIdx.x < 32) {
+        const float* w = p.w0 + 4 * threadIdx.x;
+        sw0[threadIdx.x] = make_float4(w[0], w[1], w[2], w[3]);
+        sb0[threadIdx.x] = p.b0[threadIdx.x];
     }
     bool every = false;
     for (int b = 0; b < p.blocks; ++b) {
@@ -226,14 +259,22 @@ chain_kernel(const __grid_constant__ ChainArgs p) {
         int clip, t;
         where(win, clip, t);
         const bool in = t >= 0 && t < p.T;  // outside: zeros for every convolution
-        const float* src = p.x + (long long)clip * 32 * p.T + t;
         float x[32];
+        if (WAVE) {
+            const Samples s = in ? samples(p, clip, t) : Samples{};
 #pragma unroll
-        for (int c = 0; c < 32; ++c) x[c] = in ? src[(long long)c * p.T] : 0.f;
+            for (int c = 0; c < 32; ++c) x[c] = in ? strided(s, sw0[c], sb0[c]) : 0.f;
+        } else {
+            const float* src = p.x + (long long)clip * 32 * p.T + t;
+#pragma unroll
+            for (int c = 0; c < 32; ++c) x[c] = in ? src[(long long)c * p.T] : 0.f;
+        }
         if (win + (int)gridDim.x < p.windows) {  // the next window on its way to L2
             int nclip, nt;
             where(win + gridDim.x, nclip, nt);
-            if (nt >= 0 && nt < p.T && (lane & 7) == 0) {
+            if (WAVE) {
+                if (nt >= 0 && nt < p.T && (lane & 15) == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.x + (long long)nclip * 2 * p.T + 2 * nt));
+            } else if (nt >= 0 && nt < p.T && (lane & 7) == 0) {
                 const float* next = p.x + (long long)nclip * 32 * p.T + nt;
 #pragma unroll 4
                 for (int c = 0; c < 32; ++c) asm volatile("prefetch.global.L2 [%0];" ::"l"(next + (long long)c * p.T));
@@ -334,7 +375,7 @@ chain_kernel(const __grid_constant__ ChainArgs p) {
     __syncthreads();
     if (threadIdx.x < 32) tmem_dealloc(tmem_base, 512);
     for (int win = blockIdx.x; win < p.windows; win += gridDim.x)
-        if (odd[bit_of(win) >> 5] >> (bit_of(win) & 31) & 1u) window_by_fma(p, reinterpret_cast<float*>(sa), win);
+        if (odd[bit_of(win) >> 5] >> (bit_of(win) & 31) & 1u) window_by_fma<WAVE>(p, reinterpret_cast<float*>(sa), win);
 }
 
 int chain_length(const int* dil, int n) {
@@ -343,8 +384,10 @@ int chain_length(const int* dil, int n) {
     return k;
 }
 
-int chain(const float* x, const float* const* w, const int* dil, int n, float* y, int N, int T, cudaStream_t st) {
+// w0, b0: of the strided convolution in front, or NULL
+int chain(const float* x, const float* w0, const float* b0, const float* const* w, const int* dil, int n, float* y, int N, int T, cudaStream_t st) {
     ChainArgs a = {};
+    a.w0 = w0, a.b0 = b0;
     a.x = x, a.y = y, a.T = T, a.blocks = n;
     for (int b = 0; b < n; ++b) {
         a.w1[b] = w[4 * b], a.b1[b] = w[4 * b + 1], a.w2[b] = w[4 * b + 2], a.b2[b] = w[4 * b + 3];
@@ -355,9 +398,10 @@ int chain(const float* x, const float* const* w, const int* dil, int n, float* y
     a.windows_per_clip = (T + stride - 1) / stride;
     if ((long long)a.windows_per_clip * N > 0x7fffffff - 148) return LLARK_EINVAL;
     a.windows = a.windows_per_clip * N;
-    cudaError_t e = cudaFuncSetAttribute(chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemChain);
+    auto kernel = w0 ? chain_kernel<true> : chain_kernel<false>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemChain);
     if (e == cudaSuccess) {
-        chain_kernel<<<a.windows < 148 ? a.windows : 148, kWin, kSmemChain, st>>>(a);
+        kernel<<<a.windows < 148 ? a.windows : 148, kWin, kSmemChain, st>>>(a);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) {

@@ -16,7 +16,7 @@ bool takes_resblock(int dil);
 int resblock(const float* x, const float* w1, const float* b1, const float* w2, const float* b2, float* y, int N, int T, int dil,
              cudaStream_t st);
 int chain_length(const int* dil, int n);  // jb_chain_tc.cu
-int chain(const float* x, const float* const* w, const int* dil, int n, float* y, int N, int T, cudaStream_t st);
+int chain(const float* x, const float* w0, const float* b0, const float* const* w, const int* dil, int n, float* y, int N, int T, cudaStream_t st);
 bool takes_down(int c_in, int c_out);
 int down(const float* x, const float* w, const float* b, float* y, int N, int c_in, int T, cudaStream_t st);
 bool takes_k3(int c_in, int c_out);
@@ -710,7 +710,7 @@ extern "C" int llark_jb_resblock(const float* x, const float* w1, const float* b
     if (N <= 0 || T <= 0 || dilation < 1 || dilation > 243) return LLARK_EINVAL;
     if (use_conv_tc() && jbconv::chain_length(&dilation, 1) == 1) {  // up to dilation 32; 201 us against 257 at 27
         const float* const w[4] = {w1, b1, w2, b2};
-        return jbconv::chain(x, w, &dilation, 1, y, N, T, st);
+        return jbconv::chain(x, nullptr, nullptr, w, &dilation, 1, y, N, T, st);
     }
     if (use_conv_tc() && jbconv::takes_resblock(dilation)) return jbconv::resblock(x, w1, b1, w2, b2, y, N, T, dilation, st);
     const int smem = (32 * (RES_TT + 2 * dilation) + 32 * RES_TT + 32 * 32 * 3 + 32 * 32) * (int)sizeof(float);
@@ -728,7 +728,14 @@ extern "C" int llark_jb_resblocks_length(const int* dilations, int n) {
 extern "C" int llark_jb_resblocks(const float* x, const float* const* weights, const int* dilations, int n, float* y, int N, int T,
                                   cudaStream_t st) {
     if (N <= 0 || T <= 0 || n <= 0 || !x || !weights || !dilations || !y || jbconv::chain_length(dilations, n) != n) return LLARK_EINVAL;
-    return jbconv::chain(x, weights, dilations, n, y, N, T, st);
+    return jbconv::chain(x, nullptr, nullptr, weights, dilations, n, y, N, T, st);
+}
+
+extern "C" int llark_jb_wave_resblocks(const float* wave, const float* w, const float* bias, const float* const* weights, const int* dilations,
+                                       int n, float* y, int N, int T, cudaStream_t st) {
+    if (N <= 0 || T <= 0 || (T & 1) || n <= 0 || !wave || !w || !bias || !weights || !dilations || !y || jbconv::chain_length(dilations, n) != n)
+        return LLARK_EINVAL;
+    return jbconv::chain(wave, w, bias, weights, dilations, n, y, N, T / 2, st);
 }
 
 extern "C" int llark_jb_conv_k3(const float* x, const float* w, const float* bias, float* y, int N, int c_in, int c_out,

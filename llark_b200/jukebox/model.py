@@ -96,10 +96,13 @@ class JukeboxVQVAE:
         h = x
         for b, down_t in enumerate(cfg.downs_t):
             for i in range(down_t):
-                h = ops.jb_conv_down(h, w[f"enc.{b}.down.{i}.w"], w[f"enc.{b}.down.{i}.b"])
+                down = w[f"enc.{b}.down.{i}.w"], w[f"enc.{b}.down.{i}.b"]
                 blocks = [tuple(w[f"enc.{b}.res.{i}.{d}.{n}"] for n in ("w1", "b1", "w2", "b2")) for d in range(cfg.depth)]
                 dilations = [cfg.dilation_growth_rate ** d for d in range(cfg.depth)]
-                h = ops.jb_resblocks(h, blocks, dilations)
+                if h.is_cuda and h.shape[1] == 1:  # the waveform: its convolution in the blocks' visit
+                    h = ops.jb_resblocks(h, blocks, dilations, down=down)
+                else:
+                    h = ops.jb_resblocks(ops.jb_conv_down(h, *down), blocks, dilations)
             h = ops.jb_conv_k3(h, w[f"enc.{b}.proj.w"], w[f"enc.{b}.proj.b"])
         return h
 

@@ -360,13 +360,23 @@ def jb_resblock(x, w1, b1, w2, b2, dilation):
     return y
 
 
-def jb_resblocks(x, blocks, dilations):
-    """jb_resblock after jb_resblock: blocks = [(w1, b1, w2, b2), ...]; as many of them in one visit as fit."""
-    N, C, T = x.shape
+def jb_resblocks(x, blocks, dilations, down=None):
+    """jb_resblock after jb_resblock: blocks = [(w1, b1, w2, b2), ...]; as many of them in one visit as fit. down = (w, b): behind jb_conv_down,
+    of a waveform [N, 1, T] in the same visit."""
     at = 0
     while at < len(blocks):
         left = (ctypes.c_int * (len(blocks) - at))(*dilations[at:])
         n = lib().llark_jb_resblocks_length(left, len(left))
+        if at == 0 and down is not None:
+            N, c_in, T = x.shape
+            if n and c_in == 1 and T > 0 and T % 2 == 0 and down[0].shape[0] == 32:
+                w = (ctypes.c_void_p * (4 * n))(*[_p(t) for b in blocks[:n] for t in b])
+                y = torch.empty((N, 32, T // 2), device=x.device, dtype=torch.float32)
+                check(lib().llark_jb_wave_resblocks(_p(x), _p(down[0]), _p(down[1]), w, left, n, _p(y), N, T, _stream()), "jb_wave_resblocks")
+                x, at = y, n
+                continue
+            x = jb_conv_down(x, *down)
+        N, C, T = x.shape
         if n == 0:  # not this one
             x = jb_resblock(x, *blocks[at], dilations[at])
             at += 1
@@ -376,7 +386,7 @@ def jb_resblocks(x, blocks, dilations):
         check(lib().llark_jb_resblocks(_p(x), w, left, n, _p(y), N, T, _stream()), "jb_resblocks")
         x = y
         at += n
-    return x
+    return x if blocks or down is None else jb_conv_down(x, *down)
 
 
 def jb_conv_k3(x, w, b):
