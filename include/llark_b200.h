@@ -325,6 +325,17 @@ int llark_seq_embed(const int* ids, const int* tok_seq, const int* cu, const int
  * otherwise call llark_seq_conv_tail after it. */
 int llark_seq_short_conv(const float* h, const float* w, float* tail, const int* tok_seq, const int* cu, const int* slot,
                          void* y, int n_tok, int C, int taps, int inline_tail, int act_fp32, cudaStream_t stream);
+/* llark_seq_add_rmsnorm, and llark_seq_short_conv of its result for steps of one token per request (row b belongs to slot[b], the carry moves on):
+ * the same numbers in one launch. C a multiple of four, all rows on 16-byte boundaries. */
+int llark_seq_add_rmsnorm_conv(const float* x, const float* y, const float* w, float* x_out, const float* conv_w, float* tail, const int* slot,
+                               void* out, int rows, int C, int taps, float eps, int act_fp32, cudaStream_t stream);
+/* Zeros for `slot` in n stores (host array, at most LLARK_SLOT_STORES): layers blocks, layer_bytes apart, with slot_bytes for each slot. */
+typedef struct LlarkSlotStore {
+    void* base;
+    long long layer_bytes, slot_bytes, layers;
+} LlarkSlotStore;
+#define LLARK_SLOT_STORES 16
+int llark_seq_zero_slot(const LlarkSlotStore* stores, int n, int slot, cudaStream_t stream);
 int llark_seq_conv_tail(const float* h, float* tail, const int* cu, const int* slot, int n_seq, int C, int taps,
                         cudaStream_t stream);
 /* x_out = x + y / sqrt(mean(y^2) + eps) * w (row-wise; x_out may not alias x when other rows of x are still read by the
@@ -452,6 +463,10 @@ int llark_seq_delta_chunks(int rule, const float* q, long long q_ld, const float
                            const float* v, long long v_ld, float* state, float* o, float* ws, const int* blocks, int n_blocks,
                            const int* requests, int n_requests, const int* cu, const int* slot, int H, int G, int D, int E,
                            cudaStream_t stream);
+/* A step of one token per request (row b: slot[b]): llark_seq_glr_scan and llark_seq_head_rmsnorm of its outputs in one launch. E = 128, D 64 or 128;
+ * src and state on 16-byte boundaries, ld and v_off multiples of four. */
+int llark_seq_glr_step(const float* src, long long ld, int q_off, int f_off, int v_off, const float* lower, float* state, const float* norm, void* out,
+                       const int* slot, int n_seq, int H, int D, int E, float eps, int act_fp32, cudaStream_t stream);
 int llark_seq_head_rmsnorm(const float* x, const float* w, void* out, long long n_rows, int E, float eps, int act_fp32,
                            cudaStream_t stream);
 

@@ -221,6 +221,12 @@ def _op_work(name, a, k, out, ctx):
         x, w, y, N, K = a[0], a[2], a[3], k["N"], k["K"]
         M, H = x.shape[0], w.shape[0]
         return M * H * (K * x.element_size() + N * y.element_size()) + _nbytes(w), 2.0 * M * H * N * K
+    if name == "seq_glr_step":
+        src, st, H, D, E = a[0], a[6], a[7], a[8], a[9]
+        return _nbytes(src) + 2 * st.n_seq * H * D * E * 4 + _nbytes(out), 5.0 * st.n_tok * H * D * E
+    if name == "seq_add_rmsnorm_conv":  # x, y in, the stream and the convolution's result out, the carry in and out
+        taps = a[4].shape[1]
+        return _nbytes(a[0]) * (2 + 2 * (taps - 1)) + _nbytes(out), 0.0
     if name == "seq_short_conv":
         return _nbytes(a[0]) + _nbytes(out), 0.0
     if name == "seq_qk_headnorm":
@@ -268,7 +274,8 @@ def op_table(records, ctx, peaks):
 
 
 KELUTAR_OPS = ["linear", "seq_embed", "seq_short_conv", "seq_add_rmsnorm", "seq_rmsnorm_rows", "seq_relu2",
-               "seq_qk_headnorm", "seq_swa_attn", "seq_kv_ring_write", "seq_glr_scan", "seq_head_rmsnorm"]
+               "seq_qk_headnorm", "seq_swa_attn", "seq_kv_ring_write", "seq_glr_scan", "seq_head_rmsnorm", "seq_glr_step",
+               "seq_add_rmsnorm_conv"]
 LLAMA_OPS = ["gemm", "rmsnorm_fwd", "rope_", "attn_fwd", "attn_decode_packed", "swiglu_fwd", "embed_splice_fwd", "decode_layers"]
 
 

@@ -80,16 +80,22 @@ class KelutarEngine(LayerListEngine):
         return ops.seq_embed(ids, st, self.embed, self.pos, self.cfg.embedding_scale)
 
     def _run_layers(self, cache, x, st, residuals):
-        cfg = self.cfg
-        for entry in cache.layers:
+        cfg, layers = self.cfg, cache.layers
+        joined = st.max_len == 1 and cfg.width % 4 == 0 and x.data_ptr() % 16 == 0  # a layer's last norm and the next one's convolution in one launch
+        hc = None
+        for i, entry in enumerate(layers):
             pk = entry["pk"]
-            hc = ops.seq_short_conv(x, pk["canon"], cache.view(entry["tail"]), st, self.act)
-            y = entry["mixer"].forward(hc, st, cache)
-            if entry["ff"] is None:
-                x = ops.seq_add_rmsnorm(x, y, pk["norm1"], cfg.eps)
+            if hc is None:
+                hc = ops.seq_short_conv(x, pk["canon"], cache.view(entry["tail"]), st, self.act)
+            y, norm = entry["mixer"].forward(hc, st, cache), pk["norm1"]
+            if entry["ff"] is not None:
+                x, xa = ops.seq_add_rmsnorm(x, y, norm, cfg.eps, act=self.act)
+                y, norm = entry["ff"].forward(xa), pk["norm2"]
+            if joined and i + 1 < len(layers) and not (y.data_ptr() | norm.data_ptr()) % 16:
+                after = layers[i + 1]
+                x, hc = ops.seq_add_rmsnorm_conv(x, y, norm, cfg.eps, after["pk"]["canon"], cache.view(after["tail"]), st, self.act)
             else:
-                x, xa = ops.seq_add_rmsnorm(x, y, pk["norm1"], cfg.eps, act=self.act)
-                x = ops.seq_add_rmsnorm(x, entry["ff"].forward(xa), pk["norm2"], cfg.eps)
+                x, hc = ops.seq_add_rmsnorm(x, y, norm, cfg.eps), None
             if residuals is not None:
                 residuals.append(x)
         return x

@@ -165,6 +165,12 @@ class GatedLinearRecurrenceWeights:
                 raise ValueError(f"{pfx}: tensor of shape {tuple(t.shape)}, expected {shape}")
 
 
+def _glr_step_takes(src, v_off, state, st, D, E):
+    """Whether ops.seq_glr_step takes a step: one token per request, heads of 64 or 128 by 128, rows on 16-byte boundaries."""
+    return (st.max_len == 1 and D in (64, 128) and E == 128 and not (src.stride(0) | v_off) % 4 and not (src.data_ptr() | state.data_ptr()) % 16
+            and st.n_seq <= 65535)
+
+
 class GatedLinearRecurrence:
     Weights = GatedLinearRecurrenceWeights
 
@@ -175,9 +181,12 @@ class GatedLinearRecurrence:
     def forward(self, hc, st, cache):
         w = self.w
         qfv = ops.linear(hc, w.w_qfv, bias=w.b_qfv, out_dtype=F32)
-        o_raw = ops.seq_glr_scan(qfv, w.q_off, w.f_off, w.v_off, w.lower, cache.view(self.h_state), st, w.H, w.D, w.E,
-                                 full_fp32=self.act == F32)
-        o = ops.seq_head_rmsnorm(o_raw, w.norm, w.E, self.eps, self.act)
+        state = cache.view(self.h_state)
+        if _glr_step_takes(qfv, w.v_off, state, st, w.D, w.E):
+            o = ops.seq_glr_step(qfv, w.q_off, w.f_off, w.v_off, w.lower, state, st, w.H, w.D, w.E, w.norm, self.eps, self.act)
+        else:
+            o_raw = ops.seq_glr_scan(qfv, w.q_off, w.f_off, w.v_off, w.lower, state, st, w.H, w.D, w.E, full_fp32=self.act == F32)
+            o = ops.seq_head_rmsnorm(o_raw, w.norm, w.E, self.eps, self.act)
         return ops.linear(o, w.w_o, out_dtype=F32)
 
 

@@ -6,6 +6,7 @@ extension or without a GPU these raise.
 """
 import ctypes
 import math
+from array import array
 
 import numpy as np
 import torch
@@ -607,6 +608,12 @@ def seq_step_ints(values, n_seq, n_tok, device):
     return out
 
 
+def seq_zero_slot(stores, slot):
+    """stores: (address, bytes from layer to layer, bytes of a slot, layers) of each; zeros for the slot in all of them."""
+    a = array("q", [v for s in stores for v in s])
+    check(lib().llark_seq_zero_slot(a.buffer_info()[0], len(stores), slot, _stream()), "seq_zero_slot")
+
+
 def seq_embed(ids, st, table, pos_table, scale, copy=False):
     """ids int32 [n_tok] -> x fp32 [n_tok, C] = table[id] * scale + pos_table[position]; copy: (x, x in the table's dtype)."""
     _req(ids, torch.int32)
@@ -643,6 +650,16 @@ def seq_add_rmsnorm(x, y, w, eps, act=None):
     check(lib().llark_seq_add_rmsnorm(_p(x), _p(y), _p(w), _p(out), _p(xa), rows, C, float(eps),
                                       _actf(act) if act is not None else 0, _stream()), "seq_add_rmsnorm")
     return (out, xa) if act is not None else out
+
+
+def seq_add_rmsnorm_conv(x, y, w, eps, conv_w, tail, st, act):
+    """(seq_add_rmsnorm(x, y, w, eps), seq_short_conv of it) for a step of one token per request."""
+    _req(x, torch.float32), _req(y, torch.float32), _req(w, torch.float32), _req(conv_w, torch.float32)
+    rows, C = x.shape
+    out, h = torch.empty_like(x), torch.empty((rows, C), device=x.device, dtype=act)
+    check(lib().llark_seq_add_rmsnorm_conv(x.data_ptr(), y.data_ptr(), w.data_ptr(), out.data_ptr(), conv_w.data_ptr(), tail.data_ptr(), _p(st.slot),
+                                           h.data_ptr(), rows, C, conv_w.shape[1], float(eps), _actf(act), _stream()), "seq_add_rmsnorm_conv")
+    return out, h
 
 
 def seq_gated_norm_add(x, y, w, eps, gate=None, w_next=None, act=None):
@@ -951,6 +968,15 @@ def seq_glr_scan(src, q_off, f_off, v_off, lower, state, st, H, D, E, full_fp32=
                                _p(ch.row0), _p(ch.n), _p(ch.index), _p(ch.last_slot), ch.n_items, H, D, E, _stream()),
           "seq_glr_scan(outputs)")
     return o
+
+
+def seq_glr_step(src, q_off, f_off, v_off, lower, state, st, H, D, E, norm, eps, act):
+    """seq_head_rmsnorm(seq_glr_scan(..), norm) in `act` of a step of one token per request (heads of 64 or 128 by 128); state is updated."""
+    _req(src, torch.float32), _req(state, torch.float32), _req(norm, torch.float32)
+    out = torch.empty((st.n_tok, H * E), device=src.device, dtype=act)
+    check(lib().llark_seq_glr_step(src.data_ptr(), src.stride(0), q_off, f_off, v_off, _p(lower), state.data_ptr(), norm.data_ptr(), out.data_ptr(),
+                                   _p(st.slot), st.n_seq, H, D, E, float(eps), _actf(act), _stream()), "seq_glr_step")
+    return out
 
 
 # linear attention with a fixed decay per head (csrc/seq_decay.cu)

@@ -5,7 +5,7 @@ than a growing key / value list (a ring of the last `window` keys, a recurrent s
 convolution) and whose requests come and go with different lengths use this instead: every layer registers the stores
 it needs (`add_store`), a request owns one SLOT = one row of every store from `alloc()` to `release()`, and the kernels
 index the stores by slot. Stores of equal shape are stacked into one tensor [n_layers_of_that_kind, n_slots, ...], so
-starting a request zeroes each kind with one fill and a layer's view [n_slots, ...] stays contiguous. Stores grow by
+starting a request zeroes all kinds with one launch and a layer's view [n_slots, ...] stays contiguous. Stores grow by
 doubling when the slots run out. A store that holds one entry per POSITION of a request (the keys and values of an
 attention that looks back without a bound) is declared with per_position=True: its first axis is `positions` entries
 long for every such store of the cache and doubles (`reserve_positions`) before a step that would outgrow it, old entries
@@ -185,8 +185,11 @@ class StateCache:
         if not self._free:
             self._grow()
         slot = self._free.pop()
-        for key, t in self._tensors.items():
-            if key[2]:
+        zeroed = [t for key, t in self._tensors.items() if key[2]]
+        if zeroed and len(zeroed) <= 16 and _current(self.device) and all(t.element_size() * t.stride(1) % 4 == 0 and t.numel() for t in zeroed):
+            ops.seq_zero_slot([(t.data_ptr(), t.stride(0) * t.element_size(), t.stride(1) * t.element_size(), t.shape[0]) for t in zeroed], slot)
+        else:
+            for t in zeroed:
                 t[:, slot].zero_()
         self.length[slot] = 0
         self.allocs += 1
