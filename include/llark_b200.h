@@ -80,6 +80,11 @@ int llark_gemm_ex(const void* A, int a_mn_major, long long lda, const void* B, i
                   long long ldc, int c_fp32, const void* bias, int bias_fp32, const void* R, long long ldr, int M, int N,
                   int K, int in_fp32, int max_ctas, const LlarkGemmEpilogue* ep, cudaStream_t stream);
 void llark_gemm_clear_cache(void);
+/* A bf16 [M, K] @ W^T (+ bias), W [(H + G) * D + G * E, K]: q [M, H * D], k [M, G * D], v [M, G * E] in bf16, columns [0, n_rot) of q's and k's heads
+ * turned in pairs (2i, 2i + 1) by cs fp32 [M, n_rot / 2, 2] (cos, sin) before the one rounding. CTA-pair kernel only; D and n_rot multiples of
+ * 32, columns of q, of k and of all of 64, rows in 16-byte pieces. */
+int llark_linear_qkv_rotary(const void* A, long long lda, const void* W, long long ldw, const float* bias, const float* cs, int n_rot, void* q,
+                            void* k, void* v, int M, int K, int H, int G, int D, int E, cudaStream_t stream);
 /* Kernel variant: 1 = CTA-pair kernel (cta_group::2, 256x256 tile per 2-CTA cluster; default), 0 = single-CTA
  * kernel (128x256 tile). Default comes from the environment variable LLARK_GEMM_2CTA (unset or != "0" -> 1). */
 void llark_gemm_set_mode(int two_cta);

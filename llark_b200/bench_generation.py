@@ -233,6 +233,8 @@ def _op_work(name, a, k, out, ctx):
         return _nbytes(a[0]) * 2 // 3 + _nbytes(out), 0.0
     if name == "seq_qkv_rotary":  # reads the q | k | v columns of the fused projection, writes them in the activation dtype
         return 3 * _nbytes(out), 0.0
+    if name == "linear_qkv_rotary":
+        return _nbytes(a[0]) + _nbytes(a[1]) + _nbytes(out), 2.0 * a[0].shape[0] * a[1].numel()
     if name == "seq_kv_ring_write":
         return 2 * (_nbytes(a[0]) + _nbytes(a[1])), 0.0
     if name == "embed_splice_fwd":
@@ -553,7 +555,7 @@ def run_gubulorn(args, peaks, peaks_kind, emit):
           "sizes": results, "wall_s": round(time.time() - t0, 1)})
 
 
-TOKATAR_OPS = ["linear", "seq_embed", "seq_group_rmsnorm", "seq_gated_norm_add", "seq_relu2", "seq_qkv_rotary", "seq_swa_attn",
+TOKATAR_OPS = ["linear", "seq_embed", "seq_group_rmsnorm", "seq_gated_norm_add", "seq_relu2", "linear_qkv_rotary", "seq_qkv_rotary", "seq_swa_attn",
                "seq_kv_ring_write", "seq_latent_prep", "seq_head_linear"]
 
 # (name, width, layers, heads, key/value heads, head dim, block of positions, ff, latent rank, rotated size, vocab): layers
@@ -675,7 +677,7 @@ def run_tokatar(args, peaks, peaks_kind, emit):
           "sizes": results, "wall_s": round(time.time() - t0, 1)})
 
 
-MANAPEL_OPS = ["linear", "linear_w32", "seq_embed", "seq_tanh_norm", "seq_tanh_norm_add", "seq_qkv_rotary", "seq_swa_attn",
+MANAPEL_OPS = ["linear", "linear_w32", "seq_embed", "seq_tanh_norm", "seq_tanh_norm_add", "linear_qkv_rotary", "seq_qkv_rotary", "seq_swa_attn",
                "seq_kv_ring_write", "seq_moe_route_top", "seq_moe_experts"]
 
 # (name, width, layers, heads, key/value heads, head dim, dense ff, experts, top, expert ff, shared ff, vocab): the first layer
@@ -787,7 +789,7 @@ def run_manapel(args, peaks, peaks_kind, emit):
 
 
 BUVESUN_OPS = ["linear", "linear_w32", "seq_embed", "seq_layer_norm", "seq_layer_norm_add", "seq_rotary_table", "seq_decay_scan",
-               "seq_head_norm_gate", "seq_qkv_rotary", "seq_swa_attn", "seq_kv_ring_write", "seq_moe_route_top", "seq_moe_experts"]
+               "seq_head_norm_gate", "linear_qkv_rotary", "seq_qkv_rotary", "seq_swa_attn", "seq_kv_ring_write", "seq_moe_route_top", "seq_moe_experts"]
 
 # (name, width, layer runs, heads, key/value heads, head dim, window, experts, top, expert ff, shared ff, vocab): one retention
 # layer that runs in half of the places (a loop), parallel layers in the others, experts everywhere. Beside it: a Gubulorn

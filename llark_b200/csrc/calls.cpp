@@ -13,28 +13,28 @@
 #include "../../include/llark_b200.h"
 
 #define LLARK_CALLS(X) \
-    X(llark_gemm) X(llark_gemm_ex) X(llark_splice_scan) X(llark_embed_splice_fwd) X(llark_embed_splice_bwd) X(llark_cast_f32_to_bf16) \
-    X(llark_cast_bf16_to_f32) X(llark_rmsnorm_fwd) X(llark_rmsnorm_bwd) X(llark_rope) X(llark_swiglu_fwd) X(llark_swiglu_bwd) \
-    X(llark_attn_fwd) X(llark_attn_alibi_fwd) X(llark_attn_alibi_bwd) X(llark_ln_fwd) X(llark_ln_bwd) X(llark_gelu_fwd) \
-    X(llark_gelu_bwd) X(llark_gemv) X(llark_attn_decode) X(llark_attn_decode_packed) X(llark_decode_layers) X(llark_attn_bwd) \
-    X(llark_attn_bwd_rope) X(llark_colsum) X(llark_ce_fwd) X(llark_ce_bwd) X(llark_grad_sumsq) X(llark_adamw_step) X(llark_jb_conv_down) \
-    X(llark_jb_resblock) X(llark_jb_resblocks) X(llark_jb_wave_resblocks) X(llark_jb_conv_k3) X(llark_jb_vq_encode) \
-    X(llark_layernorm_fwd) X(llark_jb_embed_tokens) X(llark_jb_sparse_attn) X(llark_jb_sparse_attn_tc) X(llark_quick_gelu) X(llark_add3) \
-    X(llark_jb_pool) X(llark_jb_label_cond) X(llark_jb_pool_batched) X(llark_v32_split_tf32) X(llark_v32_embed_splice_fwd) \
-    X(llark_v32_rmsnorm_fwd) X(llark_v32_rope) X(llark_v32_swiglu_fwd) X(llark_v32_attn_fwd) X(llark_v32_ce_fwd) X(llark_seq_step_ints) \
-    X(llark_seq_embed) X(llark_seq_short_conv) X(llark_seq_add_rmsnorm_conv) X(llark_seq_zero_slot) X(llark_seq_conv_tail) \
-    X(llark_seq_add_rmsnorm) X(llark_seq_gated_norm_add) X(llark_seq_rmsnorm_rows) X(llark_seq_relu2) X(llark_seq_layer_norm_add) \
-    X(llark_seq_tanh_norm) X(llark_seq_tanh_norm_add) X(llark_linear_rows) X(llark_linear_simt) X(llark_seq_qk_headnorm) \
-    X(llark_seq_qkv_headnorm) X(llark_seq_qkv_rotary) X(llark_seq_swa_attn) X(llark_seq_swa_attn_mma) X(llark_seq_kv_ring_write) \
-    X(llark_seq_glr_scan) X(llark_seq_glr_combine) X(llark_seq_chunk_plan) X(llark_seq_glr_chunks) X(llark_seq_delta_chunks) \
-    X(llark_seq_glr_step) X(llark_seq_head_rmsnorm) X(llark_seq_rotary_table) X(llark_seq_decay_rows) X(llark_seq_decay_chunks) \
-    X(llark_seq_decay_combine) X(llark_linear_simt_w32) X(llark_seq_group_rmsnorm) X(llark_seq_residual_combine) X(llark_seq_conv_act) \
-    X(llark_seq_delta_prep) X(llark_seq_delta_scan) X(llark_seq_head_norm_gate) X(llark_seq_skip_gate_group_norm) X(llark_seq_post_norm) \
-    X(llark_seq_glu_clamped) X(llark_seq_logit_cap) X(llark_seq_latent_prep) X(llark_seq_head_linear) X(llark_seq_tanh) \
-    X(llark_gemm_segments) X(llark_seq_moe_route) X(llark_seq_moe_route_bias) X(llark_seq_moe_route_top) X(llark_seq_moe_sort) \
-    X(llark_seq_moe_gather) X(llark_seq_silu_mul) X(llark_seq_moe_up) X(llark_seq_moe_down) X(llark_rmsnorm_bwd_workspace) \
-    X(llark_ln_bwd_workspace) X(llark_decode_scratch) X(llark_attn_bwd_workspace) X(llark_jb_resblocks_length) \
-    X(llark_seq_chunk_block_bytes) X(llark_seq_moe_tile_rows)
+    X(llark_gemm) X(llark_gemm_ex) X(llark_linear_qkv_rotary) X(llark_splice_scan) X(llark_embed_splice_fwd) X(llark_embed_splice_bwd) \
+    X(llark_cast_f32_to_bf16) X(llark_cast_bf16_to_f32) X(llark_rmsnorm_fwd) X(llark_rmsnorm_bwd) X(llark_rope) X(llark_swiglu_fwd) \
+    X(llark_swiglu_bwd) X(llark_attn_fwd) X(llark_attn_alibi_fwd) X(llark_attn_alibi_bwd) X(llark_ln_fwd) X(llark_ln_bwd) \
+    X(llark_gelu_fwd) X(llark_gelu_bwd) X(llark_gemv) X(llark_attn_decode) X(llark_attn_decode_packed) X(llark_decode_layers) \
+    X(llark_attn_bwd) X(llark_attn_bwd_rope) X(llark_colsum) X(llark_ce_fwd) X(llark_ce_bwd) X(llark_grad_sumsq) X(llark_adamw_step) \
+    X(llark_jb_conv_down) X(llark_jb_resblock) X(llark_jb_resblocks) X(llark_jb_wave_resblocks) X(llark_jb_conv_k3) \
+    X(llark_jb_vq_encode) X(llark_layernorm_fwd) X(llark_jb_embed_tokens) X(llark_jb_sparse_attn) X(llark_jb_sparse_attn_tc) \
+    X(llark_quick_gelu) X(llark_add3) X(llark_jb_pool) X(llark_jb_label_cond) X(llark_jb_pool_batched) X(llark_v32_split_tf32) \
+    X(llark_v32_embed_splice_fwd) X(llark_v32_rmsnorm_fwd) X(llark_v32_rope) X(llark_v32_swiglu_fwd) X(llark_v32_attn_fwd) \
+    X(llark_v32_ce_fwd) X(llark_seq_step_ints) X(llark_seq_embed) X(llark_seq_short_conv) X(llark_seq_add_rmsnorm_conv) \
+    X(llark_seq_zero_slot) X(llark_seq_conv_tail) X(llark_seq_add_rmsnorm) X(llark_seq_gated_norm_add) X(llark_seq_rmsnorm_rows) \
+    X(llark_seq_relu2) X(llark_seq_layer_norm_add) X(llark_seq_tanh_norm) X(llark_seq_tanh_norm_add) X(llark_linear_rows) \
+    X(llark_linear_simt) X(llark_seq_qk_headnorm) X(llark_seq_qkv_headnorm) X(llark_seq_qkv_rotary) X(llark_seq_swa_attn) \
+    X(llark_seq_swa_attn_mma) X(llark_seq_kv_ring_write) X(llark_seq_glr_scan) X(llark_seq_glr_combine) X(llark_seq_chunk_plan) \
+    X(llark_seq_glr_chunks) X(llark_seq_delta_chunks) X(llark_seq_glr_step) X(llark_seq_head_rmsnorm) X(llark_seq_rotary_table) \
+    X(llark_seq_decay_rows) X(llark_seq_decay_chunks) X(llark_seq_decay_combine) X(llark_linear_simt_w32) X(llark_seq_group_rmsnorm) \
+    X(llark_seq_residual_combine) X(llark_seq_conv_act) X(llark_seq_delta_prep) X(llark_seq_delta_scan) X(llark_seq_head_norm_gate) \
+    X(llark_seq_skip_gate_group_norm) X(llark_seq_post_norm) X(llark_seq_glu_clamped) X(llark_seq_logit_cap) X(llark_seq_latent_prep) \
+    X(llark_seq_head_linear) X(llark_seq_tanh) X(llark_gemm_segments) X(llark_seq_moe_route) X(llark_seq_moe_route_bias) \
+    X(llark_seq_moe_route_top) X(llark_seq_moe_sort) X(llark_seq_moe_gather) X(llark_seq_silu_mul) X(llark_seq_moe_up) \
+    X(llark_seq_moe_down) X(llark_rmsnorm_bwd_workspace) X(llark_ln_bwd_workspace) X(llark_decode_scratch) X(llark_attn_bwd_workspace) \
+    X(llark_jb_resblocks_length) X(llark_seq_chunk_block_bytes) X(llark_seq_moe_tile_rows)
 
 namespace {
 

@@ -77,6 +77,9 @@ struct GemmParams {
     // of A / C and multiplies weight block seg_tiles[3i] of B (stacked [blocks, N, K]); nullptr: one matrix
     const int* seg_tiles;
     const int* seg_count;  // device word: how many entries of seg_tiles are real (num_m_blocks is then an upper bound)
+    // 9 (llark_linear_qkv_rotary): epi_a = fp32 (cos, sin) [M][epi_i1 / 2], heads of epi_i0 of which the first epi_i1 columns turn in pairs
+    // (2i, 2i + 1); columns [0, q_cols) of the product are q's, the next k_cols k's, the rest v's, a matrix each
+    int q_cols, k_cols;
 };
 
 __device__ __forceinline__ void ld8_bf16(const __nv_bfloat16* ptr, float (&f)[8]) {
@@ -590,6 +593,21 @@ __device__ __forceinline__ void epi_values(const GemmParams& p, int col0, const 
         }
     }
 }
+// 32 columns of q or k at column col0 of the product, turned by their row's position
+__device__ __forceinline__ void turn_pairs(const GemmParams& p, long long row, int col0, float (&f)[32]) {
+    const int c = col0 % p.epi_i0;
+    if (col0 >= p.q_cols + p.k_cols || c >= p.epi_i1 || row >= p.M) return;
+    const float4* cs = reinterpret_cast<const float4*>(static_cast<const float*>(p.epi_a) + row * p.epi_i1 + c);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const float4 t = __ldg(cs + j);
+        const float a = f[4 * j], b = f[4 * j + 1], d = f[4 * j + 2], e = f[4 * j + 3];
+        f[4 * j] = a * t.x - b * t.y;
+        f[4 * j + 1] = b * t.x + a * t.y;
+        f[4 * j + 2] = d * t.z - e * t.w;
+        f[4 * j + 3] = e * t.z + d * t.w;
+    }
+}
 struct EpiPatch {  // an epilogue warp's patches and how far it is: piece g lies in patch g % 2 (with one patch: always in it)
     uint8_t* at;
     uint64_t* bar;  // [2] the residual's piece has arrived
@@ -625,9 +643,9 @@ __device__ __forceinline__ void epi_rest(const GemmParams& p, long long row, lon
 }
 template <int EPI>
 __device__ __forceinline__ void epi_tma(const GemmParams& p, const CUtensorMap* cmap, const CUtensorMap* rmap, int row0, int col_lo,
-                                        int pieces, uint32_t taddr, EpiPatch& e, int lane) {
+                                        const CUtensorMap* vmap, int pieces, uint32_t taddr, EpiPatch& e, int lane) {
     const int w = p.c_fp32 ? 32 : 64;
-    const bool res = p.R != nullptr;
+    const bool res = EPI != 9 && p.R != nullptr;
 #pragma unroll 1
     for (int c = 0; c < pieces; ++c, ++e.g) {
         uint8_t* const patch = patch_of(e, e.g);
@@ -669,6 +687,7 @@ __device__ __forceinline__ void epi_tma(const GemmParams& p, const CUtensorMap* 
                 tmem_ld_32x32b_x32(taddr + c * 64 + h * 32, v);
                 tmem_ld_wait();
                 epi_values<EPI>(p, col0 + h * 32, v, f);
+                if constexpr (EPI == 9) turn_pairs(p, row0 + lane, col0 + h * 32, f);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     __nv_bfloat16* q = reinterpret_cast<__nv_bfloat16*>(row + (((h * 4 + j) ^ sw) << 4));
@@ -688,7 +707,12 @@ __device__ __forceinline__ void epi_tma(const GemmParams& p, const CUtensorMap* 
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
-            tma_store_2d(cmap, patch, col0, row0);
+            if (EPI == 9 && col0 >= p.q_cols + p.k_cols)
+                tma_store_2d(vmap, patch, col0 - p.q_cols - p.k_cols, row0);
+            else if (EPI == 9 && col0 >= p.q_cols)
+                tma_store_2d(rmap, patch, col0 - p.q_cols, row0);
+            else
+                tma_store_2d(cmap, patch, col0, row0);
             tma_store_commit();
         }
     }
@@ -873,7 +897,8 @@ static_assert(kEpiWarps2 * EPI_WARP_BYTES == STAGE2_BYTES, "one patch per epilog
 template <int A_MN, int B_MN, int TF32, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads2<EPI>, 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-             const __grid_constant__ CUtensorMap tma_c, const __grid_constant__ CUtensorMap tma_r, const GemmParams p) {
+             const __grid_constant__ CUtensorMap tma_c, const __grid_constant__ CUtensorMap tma_r, const __grid_constant__ CUtensorMap tma_v,
+             const GemmParams p) {  // q | k | v: tma_c, tma_r and tma_v are theirs
     constexpr int kElemBytes = TF32 ? 4 : 2;  // operand element size is a property of the instantiation
 
     extern __shared__ uint8_t smem_raw[];
@@ -905,7 +930,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
         tma_prefetch_desc(&tma_a);
         tma_prefetch_desc(&tma_b);
         if (p.staged == 2) tma_prefetch_desc(&tma_c);
-        if (p.staged == 2 && p.R) tma_prefetch_desc(&tma_r);
+        if (p.staged == 2 && (p.R || EPI == 9)) tma_prefetch_desc(&tma_r);
+        if (EPI == 9) tma_prefetch_desc(&tma_v);
     }
     if (warp == 1 && lane == 0) {
         for (int i = 0; i < stages; ++i) {
@@ -1125,12 +1151,12 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
             const long long row0 = mbase + (long long)rank * 128 + ew * 32;
             const int ncol0 = tc.n_blk * BLOCK_N;
             const uint32_t acc = tmem_base + ((uint32_t)(ew * 32) << 16) + as * BLOCK_N;
-            if ((EPI == 0 || EPI == 1 || EPI == 2 || EPI == 5) && p.staged == 2 && !(EPI == 2 && ncol0 < p.epi_i1)) {
+            if ((EPI == 0 || EPI == 1 || EPI == 2 || EPI == 5 || EPI == 9) && p.staged == 2 && !(EPI == 2 && ncol0 < p.epi_i1)) {
                 const int pieces = epi_pieces(p, row0, m_end, ncol0 + lo);
                 if (p.R && pieces && lane == 0) ask_residual(patch, patch.g, &tma_r, ncol0 + lo, (int)row0);
                 mbar_wait(&tmem_full[as], aphase);
                 tc_fence_after();
-                epi_tma<EPI>(p, &tma_c, &tma_r, (int)row0, ncol0 + lo, pieces, acc + lo, patch, lane);
+                epi_tma<EPI>(p, &tma_c, &tma_r, (int)row0, ncol0 + lo, &tma_v, pieces, acc + lo, patch, lane);
                 epi_rest<EPI>(p, row0 + lane, m_end, ncol0 + lo, pieces, acc + lo);
             } else {
                 mbar_wait(&tmem_full[as], aphase);
@@ -1345,7 +1371,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams
 }
 
 struct GemmMaps {  // of C and R, where the epilogue goes through TMA
-    CUtensorMap c, r;
+    CUtensorMap c, r, v;
 };
 
 template <int A_MN, int B_MN, int TF32, int EPI = 0>
@@ -1365,7 +1391,7 @@ static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const GemmMaps&
     if (tiles < clusters) clusters = tiles;
     if (max_ctas > 1 && clusters > max_ctas / 2) clusters = max_ctas / 2;
     if (clusters < 1) clusters = 1;
-    kfn<<<clusters * 2, kThreads2<EPI>, SMEM2_BYTES, stream>>>(ta, tb, m.c, m.r, p);
+    kfn<<<clusters * 2, kThreads2<EPI>, SMEM2_BYTES, stream>>>(ta, tb, m.c, m.r, m.v, p);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         g_last_cuda_error = (int)e;
@@ -1670,6 +1696,39 @@ extern "C" int llark_gemm_ex(const void* A, int a_mn_major, long long lda, const
             default: return launch<1, 1, 1>(ta, tb, p, max_ctas, stream);
         }
     }
+}
+
+// q, k and v of a window layer's prompts from one product: C of llark_gemm_ex in three matrices, bf16, the pairs (2i, 2i + 1) of q's and k's
+// heads turned in the epilogue, which hides behind the products of the next tile. What it saves is the product in fp32 and a kernel that reads
+// it: the whole layer, 6443 rows, K 4096, 32 + 8 + 8 heads of 128, of which product and rotation were 245 + 69 us: 608 us -> 546.
+extern "C" int llark_linear_qkv_rotary(const void* A, long long lda, const void* W, long long ldw, const float* bias, const float* cs, int n_rot,
+                                       void* q, void* k, void* v, int M, int K, int H, int G, int D, int E, cudaStream_t stream) {
+    const long long qc = (long long)H * D, kc = (long long)G * D, N = qc + kc + (long long)G * E;
+    if (M <= 0 || K <= 0 || H <= 0 || G <= 0 || D <= 0 || E <= 0 || !A || !W || !q || !k || !v || (n_rot && !cs) || n_rot < 0 || n_rot > D || n_rot % 32 ||
+        D % 32 || qc % 64 || kc % 64 || N % 64 || N > (1 << 30) || lda % 8 || ldw % 8 || !llark_gemm_get_mode() ||
+        ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(cs) | reinterpret_cast<uintptr_t>(q) |
+          reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15))
+        return LLARK_EINVAL;
+    int rc = ensure_driver();
+    CUtensorMap ta, tb;
+    GemmMaps m = {};
+    if (rc == LLARK_OK) rc = get_tensor_map(&ta, A, K, M, lda, 64, BLOCK_M, 2);
+    if (rc == LLARK_OK) rc = get_tensor_map(&tb, W, K, N, ldw, 64, 128, 2);
+    if (rc == LLARK_OK) rc = get_tensor_map(&m.c, q, qc, M, qc, 64, 32, 2);
+    if (rc == LLARK_OK) rc = get_tensor_map(&m.r, k, kc, M, kc, 64, 32, 2);
+    if (rc == LLARK_OK) rc = get_tensor_map(&m.v, v, N - qc - kc, M, N - qc - kc, 64, 32, 2);
+    if (rc != LLARK_OK) return rc;
+    GemmParams p = {};
+    p.M = M, p.N = (int)N, p.K = K;
+    p.bias = bias, p.bias_fp32 = 1;
+    p.num_m_blocks = (M + 255) / 256, p.num_n_blocks = (int)((N + BLOCK_N - 1) / BLOCK_N), p.num_k_blocks = (K + 63) / 64;
+    p.elem_bytes = 2;
+    p.tile_counter = next_tile_counter();
+    if (!p.tile_counter) return LLARK_ECUDA;
+    p.epi = 9, p.staged = 2, p.stages = kMaxStages2, p.group_m = 16;
+    p.epi_a = n_rot ? cs : nullptr, p.epi_i0 = D, p.epi_i1 = n_rot;
+    p.q_cols = (int)qc, p.k_cols = (int)kc;
+    return launch2<0, 0, 0, 9>(ta, tb, m, p, 0, stream);
 }
 
 // Tensor maps are cached by (pointer, shape): callers that free and re-allocate buffers at the same address

@@ -72,6 +72,7 @@ import math
 import torch
 
 from . import ops
+from .ops import linear_qkv_rotary_takes
 
 F32 = torch.float32
 
@@ -663,23 +664,33 @@ class RotaryAttention(_OneBranch):
 
     def forward(self, hc, st, cache):
         w = self.w
+        if self._turns_in_product(hc, st):
+            self.side = None
+            qkv = ops.linear_qkv_rotary(hc, w.w_in, st, w.H, w.G, w.D, w.E, bias=w.b_in, freq=w.qk_freq)
+            return ops.linear(self.attend(None, st, cache, qkv=qkv), w.w_o, out_dtype=F32)
         pin = ops.linear(hc, w.w_in, bias=w.b_in, out_dtype=F32)
         self.side = pin[:, :w.side_n] if w.side_n else None
         return ops.linear(self.attend(pin, st, cache), w.w_o, out_dtype=F32)
 
-    def attend(self, pin, st, cache, out=None, out_scale=1.0):
-        """The heads' outputs (times out_scale) from the fused projection pin; into `out` when given."""
+    def _turns_in_product(self, hc, st):
+        """Whether the product itself can turn q and k: nothing but q, k and v in it, nothing but their pairs' angles between it and them."""
+        w = self.w
+        return (w.interleaved and st.max_len > 1 and self.act == torch.bfloat16 and self.lender is None and not (w.side_n or w.gated or w.unit_heads)
+                and w.q_norm is None and w.v_freq is None
+                and linear_qkv_rotary_takes(hc, w.w_in, w.H, w.G, w.D, w.E, 2 * w.qk_freq.numel() if w.qk_freq is not None else 0))
+
+    def attend(self, pin, st, cache, out=None, out_scale=1.0, qkv=None):
+        """The heads' outputs (times out_scale) from the fused projection pin, or from q, k and v; into `out` when given."""
         w = self.w
         kring, vring = cache.view(self.h_k), cache.view(self.h_v)
         cap = self.ring if self.ring is not None else cache.positions
         single = st.max_len == 1
         own = self.lender is None
         write = single and own  # one token per request: its keys and values go straight into the stores
-        q, k, v = ops.seq_qkv_rotary(pin, w.q_off, w.k_off, w.v_off, w.H, w.G if own else 0, w.D, w.E, self.eps, self.act, st,
-                                     wq=w.q_norm, wk=w.k_norm, qk_freq=w.qk_freq, qk_interleaved=w.interleaved,
-                                     v_freq=w.v_freq if own else None, v_interleaved=w.interleaved,
-                                     kring=kring if write else None, vring=vring if write else None, cap=cap,
-                                     unit=w.unit_heads)
+        q, k, v = qkv if qkv is not None else ops.seq_qkv_rotary(
+            pin, w.q_off, w.k_off, w.v_off, w.H, w.G if own else 0, w.D, w.E, self.eps, self.act, st, wq=w.q_norm, wk=w.k_norm,
+            qk_freq=w.qk_freq, qk_interleaved=w.interleaved, v_freq=w.v_freq if own else None, v_interleaved=w.interleaved,
+            kring=kring if write else None, vring=vring if write else None, cap=cap, unit=w.unit_heads)
         if not own and not single:  # what this step brought to the lender (single tokens are in its stores already)
             k, v = self.lender.step_kv
         chunk = w.span if (w.span is not None and w.mask_kind == "chunk") else 0

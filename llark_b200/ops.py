@@ -1012,11 +1012,43 @@ def seq_rotary_table(freq, st):
     _req(freq, torch.float32)
     key = freq.data_ptr()
     if key not in st.tables:
-        cs = torch.empty((st.n_tok, freq.numel(), 2), device=freq.device, dtype=torch.float32)
-        check(lib().llark_seq_rotary_table(_p(freq), freq.numel(), _p(st.tok_seq), _p(st.cu), _p(st.pos0), _p(cs), st.n_tok,
-                                           _stream()), "seq_rotary_table")
-        st.tables[key] = cs
+        st.tables[key] = _rotary_table(freq, st)
     return st.tables[key]
+
+
+def _rotary_table(freq, st):
+    cs = torch.empty((st.n_tok, freq.numel(), 2), device=freq.device, dtype=torch.float32)
+    check(lib().llark_seq_rotary_table(_p(freq), freq.numel(), _p(st.tok_seq), _p(st.cu), _p(st.pos0), _p(cs), st.n_tok, _stream()),
+          "seq_rotary_table")
+    return cs
+
+
+def linear_qkv_rotary_takes(a, w, H, G, D, E, n_rot):
+    """Whether linear_qkv_rotary takes a and w: bf16, more rows than the row-wise product's, heads of a multiple of 32 of which a multiple of 32
+    entries turn, parts that end on 64 columns, rows in 16-byte pieces."""
+    return (a.is_cuda and a.dtype == w.dtype == BF16 and a.shape[0] > LINEAR_FEW_MAX and a.shape[1] == w.shape[1] >= 64 and G > 0
+            and w.shape[0] == (H + G) * D + G * E and not (D % 32 or n_rot % 32 or H * D % 64 or G * D % 64 or w.shape[0] % 64)
+            and not (a.stride(0) | w.stride(0)) % 8 and not (a.data_ptr() | w.data_ptr()) % 16 and a.stride(1) == w.stride(1) == 1
+            and bool(lib().llark_gemm_get_mode()))
+
+
+def linear_qkv_rotary(a, w, st, H, G, D, E, bias=None, freq=None):
+    """seq_qkv_rotary(linear(a, w, bias, out_dtype=float32), ..) of interleaved pairs without norms: q, k and v in bf16, from one launch. The
+    step's table of angles is kept with it, except in a capture: what that writes exists only in its replays."""
+    _req(a, BF16), _req(w, BF16)
+    if bias is not None:
+        _req(bias, torch.float32)
+    if not _INITED:
+        init()
+    n = a.shape[0]
+    cs = None
+    if freq is not None:
+        cs = _rotary_table(freq, st) if torch.cuda.is_current_stream_capturing() else seq_rotary_table(freq, st)
+    q, k, v = (torch.empty((n, c), device=a.device, dtype=BF16) for c in (H * D, G * D, G * E))
+    LINEAR_STATS["tcgen05"] += 1
+    check(lib().llark_linear_qkv_rotary(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), _p(bias), _p(cs), 2 * freq.numel() if cs is not None else 0,
+                                        q.data_ptr(), k.data_ptr(), v.data_ptr(), n, a.shape[1], H, G, D, E, _stream()), "linear_qkv_rotary")
+    return q, k, v
 
 
 def seq_decay_scan(src, q_off, k_off, v_off, powers, state, st, H, D, E, freq=None, interleaved=False, k_scale=1.0, silu=False,
