@@ -66,24 +66,41 @@ __global__ void conv_act_kernel(const float* __restrict__ src, long long ld, con
     }
 }
 
-// Prompts: a thread takes TB consecutive rows of V adjacent channels. Inside a request (nearly always) it requests all of them and
-// the TAPS-1 rows before at once and reads every input once; a run of rows in which a request starts or ends goes row by row.
-// Memory-bound: 5297 rows x 6144 channels 53 us (82 with one channel per thread and one row at a time; 40 us of traffic).
+// Prompts: a thread takes TB consecutive rows of V adjacent channels. It requests all of them and the TAPS-1 rows before at once and reads
+// every input once, before it knows of whose request they are (four channels: with the look-up first and the rows of a run of channels first,
+// 4572 rows x 6144 channels took 63 us, now 50; 34 us of traffic; sixteen rows a thread 57); a run of rows in which a request starts or ends, which is rare, goes row by row.
 template <int TAPS, int TB, int V>
 __global__ void __launch_bounds__(128)
 conv_act_rows_kernel(const float* __restrict__ src, long long ld, const float* __restrict__ w,
                      const float* __restrict__ carry, const int* __restrict__ tok_seq,
                      const int* __restrict__ cu, const int* __restrict__ slot, float* __restrict__ out,
                      int n_tok, int n_ch, int silu, const float* __restrict__ bias) {
-    const int c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
+    const int parts = (n_ch + 128 * V - 1) / (128 * V);  // blocks of the same rows are neighbours: whole rows are asked for at a time
+    const int c = ((int)(blockIdx.x % parts) * 128 + threadIdx.x) * V;
     if (c >= n_ch) return;
-    const int t0 = blockIdx.x * TB;
+    const int t0 = (int)(blockIdx.x / parts) * TB;
     float wr[V][TAPS], b0[V];
 #pragma unroll
-    for (int x = 0; x < V; ++x) {
+    for (int x = 0; x < V; ++x) b0[x] = bias ? bias[c + x] : 0.f;
+    float in[TB + TAPS - 1][V];
+    if constexpr (V == 4) {
 #pragma unroll
-        for (int j = 0; j < TAPS; ++j) wr[x][j] = w[(long long)(c + x) * TAPS + j];
-        b0[x] = bias ? bias[c + x] : 0.f;
+        for (int i = 0; i < TB + TAPS - 1; ++i) {
+            const float4 f = ld_ahead(src + (long long)min(max(t0 - (TAPS - 1) + i, 0), n_tok - 1) * ld + c);
+            in[i][0] = f.x, in[i][1] = f.y, in[i][2] = f.z, in[i][3] = f.w;
+        }
+    }
+    if (TAPS == 4 && V == 4 && (reinterpret_cast<uintptr_t>(w) & 15) == 0) {
+#pragma unroll
+        for (int x = 0; x < V; ++x) {
+            const float4 f = __ldg(reinterpret_cast<const float4*>(w) + c + x);
+            wr[x][0] = f.x, wr[x][1] = f.y, wr[x][2 % TAPS] = f.z, wr[x][3 % TAPS] = f.w;
+        }
+    } else {
+#pragma unroll
+        for (int x = 0; x < V; ++x)
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j) wr[x][j] = w[(long long)(c + x) * TAPS + j];
     }
     auto load = [&](const float* p, float (&v)[V]) {
         if constexpr (V == 4) {
@@ -105,9 +122,10 @@ conv_act_rows_kernel(const float* __restrict__ src, long long ld, const float* _
     };
     const int b = tok_seq[t0], local0 = t0 - cu[b];
     if (local0 >= TAPS - 1 && t0 + TB <= cu[b + 1]) {
-        float in[TB + TAPS - 1][V];
+        if constexpr (V != 4) {
 #pragma unroll
-        for (int i = 0; i < TB + TAPS - 1; ++i) load(src + (long long)(t0 - (TAPS - 1) + i) * ld + c, in[i]);
+            for (int i = 0; i < TB + TAPS - 1; ++i) load(src + (long long)(t0 - (TAPS - 1) + i) * ld + c, in[i]);
+        }
 #pragma unroll
         for (int i = 0; i < TB; ++i) {
             float acc[V];
@@ -592,7 +610,7 @@ extern "C" int llark_seq_conv_act(const float* src, long long ld, const float* w
         const bool vec = n_ch % 4 == 0 && ld % 4 == 0 &&
                          ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(carry)) & 15) == 0;
 #define LLARK_ROWS(T_, TB_, V_)                                                                                              \
-    conv_act_rows_kernel<T_, TB_, V_><<<dim3((n_tok + TB_ - 1) / TB_, (n_ch + 128 * V_ - 1) / (128 * V_)), 128, 0, st>>>(    \
+    conv_act_rows_kernel<T_, TB_, V_><<<(unsigned)((long long)((n_tok + TB_ - 1) / TB_) * ((n_ch + 128 * V_ - 1) / (128 * V_))), 128, 0, st>>>(    \
         src, ld, w, carry, tok_seq, cu, slot, out, n_tok, n_ch, silu, bias)
 #define LLARK_TAPS(TB_, V_)            \
     if (taps == 2) LLARK_ROWS(2, TB_, V_); \

@@ -146,9 +146,10 @@ __global__ void short_conv4_kernel(const float* __restrict__ h, const float* __r
     }
 }
 
-// Prompts: a CTA walks TB consecutive rows with the last TAPS-1 inputs of each 4-channel group in registers, so a row of
-// h and the taps are read once per CTA instead of once per output row (the per-row kernels above are bound by the number
-// of L1 requests, not by bytes). The window is rebuilt from h / the tail wherever a request starts inside the group.
+// Prompts: a thread takes TB consecutive rows of four channels and requests them and the TAPS-1 in front of them at once, before it knows of
+// whose request they are, so a row of h and the taps are read once instead of once per output row (the per-row kernels above are
+// bound by the number of L1 requests, not by bytes). Where a request starts or ends among the rows they go one by one, the window rebuilt
+// from h / the tail. With its tail's launch, 2048 channels, one row after another -> now: 952 rows 19.2 us -> 17.6, 6443 rows 29.2 -> 25.1.
 template <typename T> __device__ __forceinline__ void st4(T* p, float4 v);
 template <> __device__ __forceinline__ void st4<float>(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
 template <> __device__ __forceinline__ void st4<__nv_bfloat16>(__nv_bfloat16* p, float4 v) {
@@ -163,11 +164,31 @@ __global__ void short_conv4t_kernel(const float* __restrict__ h, const float* __
     const int t0 = blockIdx.x * TB;
     const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
     if (c >= C) return;
+    float4 in[TB + TAPS - 1];  // all rows at once, before it is known of whose request they are; row by row below where one starts or ends
+#pragma unroll
+    for (int i = 0; i < TB + TAPS - 1; ++i) in[i] = ld_ahead(h + (long long)min(max(t0 - (TAPS - 1) + i, 0), n_tok - 1) * C + c);
     float wr[4][TAPS];
 #pragma unroll
     for (int ch = 0; ch < 4; ++ch)
 #pragma unroll
         for (int j = 0; j < TAPS; ++j) wr[ch][j] = w[(long long)(c + ch) * TAPS + j];
+    const int b0 = tok_seq[t0];
+    if (t0 - cu[b0] >= TAPS - 1 && t0 + TB <= cu[b0 + 1]) {
+#pragma unroll
+        for (int i = 0; i < TB; ++i) {
+            const float4 cur = in[i + TAPS - 1];
+            float4 acc = make_float4(wr[0][TAPS - 1] * cur.x, wr[1][TAPS - 1] * cur.y, wr[2][TAPS - 1] * cur.z, wr[3][TAPS - 1] * cur.w);
+#pragma unroll
+            for (int j = 0; j < TAPS - 1; ++j) {
+                acc.x = fmaf(wr[0][j], in[i + j].x, acc.x);
+                acc.y = fmaf(wr[1][j], in[i + j].y, acc.y);
+                acc.z = fmaf(wr[2][j], in[i + j].z, acc.z);
+                acc.w = fmaf(wr[3][j], in[i + j].w, acc.w);
+            }
+            st4(y + (long long)(t0 + i) * C + c, make_float4(cur.x + acc.x, cur.y + acc.y, cur.z + acc.z, cur.w + acc.w));
+        }
+        return;
+    }
     float4 win[TAPS > 1 ? TAPS - 1 : 1];
     for (int i = 0; i < TB && t0 + i < n_tok; ++i) {
         const int t = t0 + i;
