@@ -15,12 +15,12 @@
 //
 //   res block   y = x + W2 relu(W1 (*dilation d, 3 taps) relu(x) + b1) + b2, both convolutions of a tile in one visit: the second's A
 //               operand is the first's result, written by the thread that owns the row. For dilations from 33 on: up to 32
-//               jb_chain_tc.cu is ahead (181 to 198 us at the size below)
+//               jb_chain_tc.cu is ahead (158 to 171 us at the size below)
 //   others      taps 4 stride 2 (32 or 64 channels in, 32 out), taps 3 (32 in, 64 out)
 //
 // What bounds it: the latency of load, split, product and read-back of a tile, hidden only by the other groups (a res block reads and
 // writes every value once; the tensor pipe works less than a fifth of the time). Measured on a B200, 4 clips x 524288 steps x 32 channels, a
-// res block: 257 us for dilations up to 64 and 346 at 81, with mma.sync 413 and 685. Three groups of four warps and not more: 168
+// res block: 232 us for dilations up to 64 and 323 at 81 (products issued by one lane 257 and 346), with mma.sync 413 and 685. Three groups of four warps and not more: 168
 // registers a thread hold a step's 32 channels, the next step's and the sums (20 of them spilled); two groups with the input staged by cp.async: 325.
 #include "common.cuh"
 
