@@ -319,7 +319,7 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
 
 // =============================================================================================== backward
 // Dsum[b,h,s] = sum_d dO[b,s,h,d] * O[b,s,h,d]; sixteen lanes per (b,s,h), four of them a warp, whose loads are all under way before the
-// first is used: bound by memory (8192 tokens x 32 heads, 134 MB: 32 us; a warp each, 8 bytes a lane, 49).
+// first is used: bound by memory (8192 tokens x 32 heads, 134 MB: 28 us; with divisions of 64 bits 32; a warp each, 8 bytes a lane, 49).
 constexpr int kPrepRows = 4;
 __global__ void attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __restrict__ dO,
                                      float* __restrict__ Dsum, long long B, int S, int NH) {
@@ -356,9 +356,15 @@ __global__ void attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ O, const 
         for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         const long long r = first + 2 * i;
         if ((lane & 15) == 0 && r < total) {
-            const int h = (int)(r % NH);
-            const long long bs = r / NH;
-            Dsum[(bs / S * NH + h) * S + bs % S] = s;
+            long long at;
+            if (total <= 0x7fffffff) {  // three divisions of 64 bits are some 200 instructions
+                const uint32_t bs = (uint32_t)r / (uint32_t)NH, h = (uint32_t)r - bs * NH, b = bs / (uint32_t)S;
+                at = ((long long)b * NH + h) * S + (bs - b * S);
+            } else {
+                const long long bs = r / NH;
+                at = (bs / S * NH + r % NH) * S + bs % S;
+            }
+            Dsum[at] = s;
         }
     }
 }
