@@ -1008,9 +1008,9 @@ def decay_powers(decay, device):
 
 def seq_rotary_table(freq, st):
     """(cos, sin) of position * frequency for every row of the step, fp32 [n_tok, n_freq, 2]; kept with the step for the other
-    layers (and heads, and passes) that rotate by the same tensor of frequencies."""
+    layers (and heads, and passes) on this stream that rotate by the same tensor of frequencies."""
     _req(freq, torch.float32)
-    key = freq.data_ptr()
+    key = freq.data_ptr(), _stream()
     if key not in st.tables:
         st.tables[key] = _rotary_table(freq, st)
     return st.tables[key]

@@ -53,3 +53,17 @@ def test_what_it_does_not_take():
         assert not takes(a, w, 2, 1, 64, 64, 64)
     finally:
         ops.lib().llark_gemm_set_mode(two)
+
+
+def test_a_stream_makes_its_own_table_of_angles():
+    from llark_b200 import ops
+    from llark_b200.state_cache import StepLayout
+
+    st, freq = StepLayout([3, 70], [0, 5], [0, 1], torch.device("cuda")), torch.rand(32, device="cuda")
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        there = ops.seq_rotary_table(freq, st)
+    here = ops.seq_rotary_table(freq, st)
+    torch.cuda.synchronize()
+    assert here is not there and here is ops.seq_rotary_table(freq, st) and torch.equal(here, there)
