@@ -575,6 +575,9 @@ int llark_seq_moe_route_bias(const float* logits, long long ld, const float* cor
 int llark_seq_moe_route_top(const float* logits, long long ld, int* ids, float* wts, int n_tok, int n_exp, int top,
                             int sigmoid_wts, cudaStream_t stream);
 int llark_seq_moe_tile_rows(void);
+/* How a product of 9 to 64 rows, or one of routed experts (max_tiles > 0, M is not used), is cut: out[7] = results of a tile, its rows of W,
+ * CTAs that share K, rows of a box of W, and the extents of W's tensor map (K, rows, experts or 0). act: that of csrc/skinny.cuh. */
+int llark_few_rows_plan(int M, int N, int K, int act, int max_tiles, long long* out);
 /* meta[0] = number of 64-row tiles; with tiles256: 256-row tiles for llark_gemm_segments, their number in meta[1];
  * experts >= n_real have no weights and get no tiles */
 int llark_seq_moe_sort(const int* ids, int n_ent, int n_exp, int n_real, int* perm, int* pos_of, int* tiles, int* meta,

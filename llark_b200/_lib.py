@@ -18,7 +18,7 @@ _ERR = {-1: "LLARK_EINVAL (bad shape/alignment/argument)", -2: "LLARK_ECUDA", -3
 # the generation path of layer-list decoders (csrc/seq_*.cu)
 SEQ_SYMBOLS = [
     "llark_linear_qkv_rotary", "llark_seq_step_ints", "llark_seq_glr_step", "llark_seq_add_rmsnorm_conv", "llark_seq_zero_slot", "llark_seq_embed", "llark_seq_short_conv", "llark_seq_conv_tail", "llark_seq_add_rmsnorm", "llark_seq_rmsnorm_rows",
-    "llark_seq_relu2", "llark_linear_rows", "llark_linear_simt", "llark_seq_qk_headnorm", "llark_seq_swa_attn",
+    "llark_seq_relu2", "llark_few_rows_plan", "llark_linear_rows", "llark_linear_simt", "llark_seq_qk_headnorm", "llark_seq_swa_attn",
     "llark_seq_swa_attn_mma",
     "llark_seq_kv_ring_write", "llark_seq_glr_scan", "llark_seq_glr_combine", "llark_seq_head_rmsnorm",
     "llark_linear_simt_w32", "llark_seq_group_rmsnorm", "llark_seq_residual_combine", "llark_seq_conv_act",
@@ -150,6 +150,7 @@ def lib():
             "llark_v32_swiglu_fwd": ([P, P, LL, I, P], I),
             "llark_v32_attn_fwd": ([P, P, P, I, I, I, I, F, P], I),
             "llark_v32_ce_fwd": ([P, LL, I, P, I, I, P, P, P], I),
+            "llark_few_rows_plan": ([I, I, I, I, I, P], I),
             "llark_seq_step_ints": ([P, I, I, I, P, P], I),
             "llark_linear_qkv_rotary": ([P, LL, P, LL, P, P, I, P, P, P, I, I, I, I, I, I, P], I),
             "llark_seq_glr_step": ([P, LL, I, I, I, P, P, P, P, P, I, I, I, I, F, I, P], I),

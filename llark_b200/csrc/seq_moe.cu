@@ -597,9 +597,8 @@ static bool takes_tiles(int n_ent, int max_tiles) {
     return n_ent > kRowsRouteMaxEntries || (n_ent > 6 && 2 * n_ent > n_exp);
 }
 static int launch_few(const void* A, long long lda, const int* perm, int top, const void* W, void* C, long long ldc, int c_fp32,
-                      const int* tiles, const int* meta, int max_tiles, int n_ent, int n_rows, int K, int mode, UpArgs up, cudaStream_t st) {
+                      const int* tiles, const int* meta, int max_tiles, int n_rows, int K, int mode, UpArgs up, cudaStream_t st) {
     skinny::Args a = {};
-    a.experts = max_tiles - (n_ent + kTileRows - 1) / kTileRows;
     a.A = (const bf16_t*)A, a.lda = lda, a.W = (const bf16_t*)W, a.ldw = K;
     a.C = C, a.ldc = ldc, a.c_fp32 = c_fp32;
     a.N = n_rows, a.K = K;
@@ -620,7 +619,7 @@ static int launch_up(const void* x, long long ldx, const int* perm, int top, con
                      const int* meta, int max_tiles, int n_ent, int ff, int K, UpArgs up, cudaStream_t st) {
     constexpr bool dual = MODE == kSiluGlu || MODE == kClampGlu;
     if (sizeof(T) == 2 && takes_tiles(n_ent, max_tiles) && skinny::fits(x, ldx, w, K, K))
-        return launch_few(x, ldx, perm, top, w, act, ff, 0, tiles, meta, max_tiles, n_ent, dual ? 2 * ff : ff, K, MODE, up, st);
+        return launch_few(x, ldx, perm, top, w, act, ff, 0, tiles, meta, max_tiles, dual ? 2 * ff : ff, K, MODE, up, st);
     if (n_ent <= kRowsRouteMaxEntries) {  // a handful of rows per expert: stream the weights once
         const int vec = 16 / (int)sizeof(T);
         const int vec_ok = (K % vec == 0) && (ldx % vec == 0) &&
@@ -653,7 +652,7 @@ extern "C" int llark_seq_moe_down(const void* act, const void* w_down, float* z,
                                   int max_tiles, int n_ent, int C, int ff, int act_fp32, cudaStream_t st) {
     if (max_tiles <= 0 || ff <= 0 || C <= 0 || !act || !w_down || !z || !tiles || !meta) return LLARK_EINVAL;
     if (!act_fp32 && takes_tiles(n_ent, max_tiles) && skinny::fits(act, ff, w_down, ff, ff))
-        return launch_few(act, ff, nullptr, 1, w_down, z, C, 1, tiles, meta, max_tiles, n_ent, C, ff, kPlain, UpArgs{}, st);
+        return launch_few(act, ff, nullptr, 1, w_down, z, C, 1, tiles, meta, max_tiles, C, ff, kPlain, UpArgs{}, st);
     if (n_ent <= kRowsRouteMaxEntries) {
         const int esz = act_fp32 ? 4 : 2, vec = 16 / esz;
         const int vec_ok = (ff % vec == 0) &&

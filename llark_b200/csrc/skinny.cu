@@ -25,6 +25,8 @@
 namespace llark {
 int tensor_map_2d(CUtensorMap* out, const void* ptr, long long inner, long long outer, long long ld, int box_inner, int box_outer,
                   int elem_bytes);  // gemm_tcgen05.cu
+int tensor_map_batches(CUtensorMap* out, const void* ptr, long long inner, long long outer, long long ld, int batches, int box_inner,
+                       int box_outer, int elem_bytes);
 
 namespace skinny {
 
@@ -414,7 +416,7 @@ skinny_tc_kernel(const Args p, const Cut cut, const __grid_constant__ CUtensorMa
     tc_fence_after();
     const uint32_t tmem = tmem_base;
     let_next_begin();
-    int M = p.M, row0 = 0, wrow = 0;
+    int M = p.M, row0 = 0, expert = 0;
     if (GROUPED) {
         wait_for_previous();
         if ((int)blockIdx.y >= p.meta[0]) {  // the whole cluster
@@ -422,12 +424,12 @@ skinny_tc_kernel(const Args p, const Cut cut, const __grid_constant__ CUtensorMa
             return;
         }
         const int* t = p.tiles + 3 * blockIdx.y;
-        wrow = t[0] * p.N;
+        expert = t[0];
         row0 = t[1];
         M = t[2];
     }
     const int u0 = tile * cut.units;
-    wrow += p.act == kActRope ? (u0 >> 6) * 128 + (u0 & 63) : adjacent_rows(p) ? 2 * u0 : u0;
+    const int wrow = p.act == kActRope ? (u0 >> 6) * 128 + (u0 & 63) : adjacent_rows(p) ? 2 * u0 : u0;
     const int m_pad = (M + 15) & ~15;  // tokens that are multiplied
     // of a stage, in bytes; with few tokens a routed tile has room for more stages than the worst case
     const int kWeights = (GROUPED ? TN : cut.rows) * 128, kStage = kWeights + (GROUPED ? m_pad : NTOK) * 128;
@@ -470,7 +472,12 @@ skinny_tc_kernel(const Args p, const Cut cut, const __grid_constant__ CUtensorMa
             };
             auto request = [&](int it, int st) {
                 mbar_arrive_expect_tx(&full[st], COPIES ? kWeights : kStage);
-                each(it, [&](int k, int row, int at) { tma_load_2d(smraw + st * kStage + at, &wmap, &full[st], k, row); });
+                each(it, [&](int k, int row, int at) {
+                    if (GROUPED)
+                        tma_load_3d(smraw + st * kStage + at, &wmap, &full[st], k, row, expert);
+                    else
+                        tma_load_2d(smraw + st * kStage + at, &wmap, &full[st], k, row);
+                });
             };
             if (!GROUPED && !p.weights_there) {
                 for (int it = 0; it < S && it < n; ++it) each(it, [&](int k, int row, int) { tma_prefetch_2d(&wmap, k, row); });
@@ -594,34 +601,37 @@ static int stages(int rows, int ntok, int& smem) {
     if (smem < ntok * TRP * 4 + 1024) smem = ntok * TRP * 4 + 1024;  // the partial sums
     return s;
 }
+// The weights as their tensor map has them: K by rows of W by experts. What a box reaches past an expert's last row is zeros and not read, the
+// last expert's as well; a tile's expert is one that there is, so the third extent need not be their number.
+struct Boxes {
+    long long inner, outer;
+    int experts, rows;  // rows of a box
+};
+static Boxes boxes_of(const Args& a, const Cut& cut) {
+    const bool halves = gate_up(a) || (a.act == kActRope && cut.units < 64);  // two boxes for a slice
+    return {a.K, a.N, a.tiles ? 65536 : 0, halves ? cut.units : cut.rows};
+}
 template <int NTOK, typename TC, bool GROUPED, int CH>
 static cudaError_t go_tc(const Args& a, Cut cut, cudaStream_t st) {
     static std::atomic<unsigned long long> allowed{0};
     int smem;
     cut.stages = stages(cut.rows, NTOK, smem);
     if (GROUPED) smem = kTcSmem;
-    const bool boxes = gate_up(a) || (a.act == kActRope && cut.units < 64);  // two for a slice
+    const Boxes b = boxes_of(a, cut);
     CUtensorMap wmap;
-    if (tensor_map_2d(&wmap, a.W, a.K, GROUPED ? (long long)a.experts * a.N : a.N, a.ldw, BK, boxes ? cut.units : cut.rows, 2)) return cudaErrorInvalidValue;
+    if (b.experts ? tensor_map_batches(&wmap, a.W, b.inner, b.outer, a.ldw, b.experts, BK, b.rows, 2)
+                  : tensor_map_2d(&wmap, a.W, b.inner, b.outer, a.ldw, BK, b.rows, 2))
+        return cudaErrorInvalidValue;
     CUtensorMap amap = wmap;
     if (!copied(NTOK, GROUPED) && tensor_map_2d(&amap, a.A, a.K, a.M, a.lda, BK, NTOK, 2)) return cudaErrorInvalidValue;
     return go(skinny_tc_kernel<NTOK, TC, GROUPED, CH>, allowed, kTcSmem, smem, tc_threads(copied(NTOK, GROUPED)), (units_of(a) + cut.units - 1) / cut.units, cut.cs, st, a,
               cut, wmap, amap);
 }
 
-cudaError_t launch(const Args& a, cudaStream_t st) {
+// How the products of more than eight rows and of routed experts are cut
+static Cut cut_of(const Args& a) {
     const bool grouped = a.tiles != nullptr, two = paired(a);
     const int nch = (a.K + BK - 1) / BK, all = units_of(a);
-    // Up to eight tokens the mma.sync kernel: as fast as the other or faster (K = 2048, N = 2048: 4.5 against 5.8 us), and ten
-    // times as exact. Routed experts have 0 to 64 tokens per tile, known only on the device.
-    if (!grouped && a.M <= 8) {
-        // Cut along K until the grid holds as many CTAs as are resident at once (four for each of the 148 SMs), as long as a CTA keeps four
-        // slices of K.
-        const int units = two ? BN / 2 : BN, tiles = (all + units - 1) / units;
-        int cs = 1;
-        while (cs < 8 && tiles * cs * 2 <= 592 && nch / (cs * 2) >= 4) cs *= 2;
-        return a.c_fp32 ? go_mma<float>(a, cs, tiles, st) : go_mma<bf16_t>(a, cs, tiles, st);
-    }
     const int most = two ? TN / 2 : TN;
     Cut cut = {most, TN, 1, 0};
     if (grouped) {  // the same with two CTAs for an SM
@@ -650,6 +660,23 @@ cudaError_t launch(const Args& a, cudaStream_t st) {
             }
         }
     }
+    return cut;
+}
+
+cudaError_t launch(const Args& a, cudaStream_t st) {
+    const bool grouped = a.tiles != nullptr, two = paired(a);
+    const int nch = (a.K + BK - 1) / BK, all = units_of(a);
+    // Up to eight tokens the mma.sync kernel: as fast as the other or faster (K = 2048, N = 2048: 4.5 against 5.8 us), and ten
+    // times as exact. Routed experts have 0 to 64 tokens per tile, known only on the device.
+    if (!grouped && a.M <= 8) {
+        // Cut along K until the grid holds as many CTAs as are resident at once (four for each of the 148 SMs), as long as a CTA keeps four
+        // slices of K.
+        const int units = two ? BN / 2 : BN, tiles = (all + units - 1) / units;
+        int cs = 1;
+        while (cs < 8 && tiles * cs * 2 <= 592 && nch / (cs * 2) >= 4) cs *= 2;
+        return a.c_fp32 ? go_mma<float>(a, cs, tiles, st) : go_mma<bf16_t>(a, cs, tiles, st);
+    }
+    const Cut cut = cut_of(a);
 #define LLARK_SKINNY(N_, GR_, CH_) (a.c_fp32 ? go_tc<N_, float, GR_, CH_>(a, cut, st) : go_tc<N_, bf16_t, GR_, CH_>(a, cut, st))
     if (grouped) return LLARK_SKINNY(64, true, 1);
     // Short chains for what fp32 FMAs computed before: narrow products, paired activations with an fp32 result and results off 16-byte
@@ -669,3 +696,16 @@ cudaError_t launch(const Args& a, cudaStream_t st) {
 
 }  // namespace skinny
 }  // namespace llark
+
+extern "C" int llark_few_rows_plan(int M, int N, int K, int act, int max_tiles, long long* out) {
+    using namespace llark::skinny;
+    if (N <= 0 || K <= 0 || !out || (max_tiles <= 0 && (M <= 8 || M > kMaxRows))) return LLARK_EINVAL;
+    static const int one = 0;
+    Args a = {};
+    a.M = M, a.N = N, a.K = K, a.act = act, a.max_tiles = max_tiles, a.tiles = max_tiles > 0 ? &one : nullptr;
+    const Cut c = cut_of(a);
+    const Boxes b = boxes_of(a, c);
+    const long long v[] = {c.units, c.rows, c.cs, b.rows, b.inner, b.outer, b.experts};
+    for (int i = 0; i < 7; ++i) out[i] = v[i];
+    return LLARK_OK;
+}

@@ -30,7 +30,7 @@ struct Args {
     // are perm[sorted row] / top (NULL: the sorted row itself), W holds one [N, K] block per expert, sums are multiplied by
     // in_wts[perm[sorted row]] when given. M is not used.
     const int *tiles, *meta, *perm;
-    int max_tiles, top, experts;
+    int max_tiles, top;
     const float* in_wts;
     // The weights were there before the kernel in front of this one began (launches of one call behind each other): they are
     // fetched before that kernel has ended. Otherwise they are only asked for in L2, which a later write does no harm to.
