@@ -628,26 +628,36 @@ static cudaError_t go_tc(const Args& a, Cut cut, cudaStream_t st) {
               cut, wmap, amap);
 }
 
+// Whether the products of every slice of K start from zero (CH = 1 of skinny_tc_kernel): what fp32 FMAs computed before the tensor cores did, narrow
+// products, paired activations with an fp32 result and results off 16-byte boundaries, and routed experts. The others are a chain over a CTA's
+// part of K, in adders that cut what does not fit, and 6 % faster (a decode step of 32 rows 549 us against 582).
+static bool short_chains(const Args& a) {
+    return a.tiles || a.N < 64 || (a.c_fp32 && (a.act == kActReluGlu || a.act == kActClampGlu)) || a.ldc % (a.c_fp32 ? 4 : 8) ||
+           (reinterpret_cast<uintptr_t>(a.C) & 15);
+}
+
 // How the products of more than eight rows and of routed experts are cut
 static Cut cut_of(const Args& a) {
     const bool grouped = a.tiles != nullptr, two = paired(a);
-    const int nch = (a.K + BK - 1) / BK, all = units_of(a);
-    const int most = two ? TN / 2 : TN;
+    const int nch = (a.K + BK - 1) / BK, all = units_of(a), most = two ? TN / 2 : TN;
+    // Tiles of 128 rows, cut along K until the grid holds two CTAs for each of the 148 SMs, as long as a CTA keeps four slices of K
     Cut cut = {most, TN, 1, 0};
-    if (grouped) {  // the same with two CTAs for an SM
-        const int tiles = (all + most - 1) / most;
-        while (cut.cs < 8 && (long long)tiles * a.max_tiles * cut.cs * 2 <= 296 && nch / (cut.cs * 2) >= 4) cut.cs *= 2;
-    } else {
+    const int tiles = (all + most - 1) / most;
+    while (cut.cs < 8 && (long long)tiles * (grouped ? a.max_tiles : 1) * cut.cs * 2 <= 296 && nch / (cut.cs * 2) >= 4) cut.cs *= 2;
+    if (!grouped) {
         const int ntok = a.M <= 16 ? 16 : a.M <= 32 ? 32 : 64;
         // The tiles and clusters with most of the weights under way, of those that are all resident at once (two CTAs for each of the 148 SMs; of
         // clusters of four and eight 71 and 33 fit), as long as a CTA keeps four slices of K; larger tiles and smaller clusters unless others have a
         // twentieth more. Tiles of less than 64 rows leave the tensor cores more products than the time of their bytes. 22016 rows of gate
         // and up in 276 tiles of 80 instead of 172 of 128: 34.8 -> 32.7 us with 32 tokens, 37.5 -> 34.4 with 64. (Clusters of three: 12288
-        // rows in 288 CTAs instead of 192 20.8 -> 31.)
+        // rows in 288 CTAs instead of 192 20.8 -> 31.) A chain over K is never cut over fewer CTAs than
+        // above: its error goes with its length, 2.3e-7 of the result over 256, 4.7e-7 over 512, 2.1e-6 over 2048.
         static const int sizes[] = {1, 2, 4, 8}, fit[] = {296, 148, 71, 33};
+        const int least = short_chains(a) ? 1 : cut.cs;
         long long best = 0;
         const long long bytes = 2LL * a.N * a.K / 128;
         for (int i = 0; i < 4; ++i) {
+            if (sizes[i] < least) continue;
             if (sizes[i] > 1 && nch / sizes[i] < 4) break;
             for (int rows = TN; rows >= 64; rows -= 8) {
                 const int units = two ? rows / 2 : rows;
@@ -679,11 +689,7 @@ cudaError_t launch(const Args& a, cudaStream_t st) {
     const Cut cut = cut_of(a);
 #define LLARK_SKINNY(N_, GR_, CH_) (a.c_fp32 ? go_tc<N_, float, GR_, CH_>(a, cut, st) : go_tc<N_, bf16_t, GR_, CH_>(a, cut, st))
     if (grouped) return LLARK_SKINNY(64, true, 1);
-    // Short chains for what fp32 FMAs computed before: narrow products, paired activations with an fp32 result and results off 16-byte
-    // boundaries. The others took the tcgen05 core, whose one chain over K errs by 4 to 12e-6; cut over a cluster theirs are shorter (0.5 to 1.4e-6), and 6 % faster than
-    // short ones (a decode step of 32 rows 549 us against 582).
-    if (a.N < 64 || (a.c_fp32 && (a.act == kActReluGlu || a.act == kActClampGlu)) || a.ldc % (a.c_fp32 ? 4 : 8) ||
-        (reinterpret_cast<uintptr_t>(a.C) & 15)) {
+    if (short_chains(a)) {
         if (a.M <= 16) return LLARK_SKINNY(16, false, 1);
         if (a.M <= 32) return LLARK_SKINNY(32, false, 1);
         return LLARK_SKINNY(64, false, 1);

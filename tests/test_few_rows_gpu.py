@@ -190,3 +190,16 @@ def test_tiles_of_fewer_rows_and_clusters(M, N, K):
     if N % 16 == 0:  # rows of the result on 16-byte boundaries
         g, u = z[:, :N // 2], z[:, N // 2:]
         assert _rel(ops.gemm(x, w, swiglu=True), torch.nn.functional.silu(g) * u) < 2.0 ** -7
+
+
+@pytest.mark.parametrize("M", [9, 32, 33])
+@pytest.mark.parametrize("N,K", [(1024, 512), (6144, 1024), (2048, 2048), (4224, 2048), (2560, 2560)])
+def test_chains_over_k_are_short(M, N, K):
+    """A chain of n products of 16 channels in the tensor cores' adders, which cut, loses about n / 4 of 2^-24 (2.3e-7 over 256 channels, 4.7e-7 over
+    512); these sizes are cut into chains of 256 or 320. Half as much again is allowed; a chain twice as long is not."""
+    from llark_b200 import ops
+
+    torch.manual_seed(M + N)
+    x, w = torch.randn(M, K, device="cuda").to(BF16), (torch.randn(N, K, device="cuda") * K ** -0.5).to(BF16)
+    chain = 320 if K == 2560 else 256
+    assert _rel(ops.linear(x, w, out_dtype=F32), x.to(F64) @ w.to(F64).t()) < 1.5 * chain / 16 / 4 * 2.0 ** -24

@@ -41,3 +41,16 @@ def test_boxes_of_routed_experts_end_with_the_experts_that_have_weights(ff, K, a
                         assert not at or at[-1] < real * N
                         seen.update(at)
                 assert set(range(expert * N, (expert + 1) * N)) <= seen
+
+
+@pytest.mark.parametrize("M", [9, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("act", [NONE, SILU_GLU])
+def test_chains_over_k_are_no_longer_than_those_of_whole_tiles(M, act):
+    """The sums of a CTA's part of K are one chain in adders that cut instead of rounding: never longer than with tiles of 128 rows in as many CTAs
+    as are resident at once (two for each of 148 SMs, clusters of up to eight, four slices of 64 or more for each)."""
+    for N in (64, 1000, 1024, 2048, 2560, 3072, 4096, 4224, 4608, 6144, 8192, 12288, 22016, 32004):
+        for K in (64, 504, 512, 1024, 1536, 2048, 2560, 4096, 5120, 11008):
+            slices, tiles, cs = (K + 63) // 64, (N + 127) // 128, 1
+            while cs < 8 and tiles * cs * 2 <= 296 and slices // (cs * 2) >= 4:
+                cs *= 2
+            assert -(-slices // _plan(M, N, K, act)["cs"]) <= -(-slices // cs), (N, K)
