@@ -24,13 +24,10 @@ serve: $(LIB_SERVE) $(CALLS)
 llark_b200/_calls.so: llark_b200/csrc/calls.cpp include/llark_b200.h
 	g++ -std=c++17 -O2 -shared -fPIC -I$(PYINC) -I$(dir $(NVCC))../include -o $@ $< -ldl
 
-build/%.o: llark_b200/csrc/%.cu llark_b200/csrc/common.cuh include/llark_b200.h
+# all headers are behind all objects: a list for each was found short of one
+build/%.o: llark_b200/csrc/%.cu $(wildcard llark_b200/csrc/*.cuh) include/llark_b200.h
 	@mkdir -p build
 	$(NVCC) $(NVFLAGS) -c $< -o $@ 2> build/$*.ptxas.log || (cat build/$*.ptxas.log; exit 1)
-
-build/skinny.o build/gemv.o build/gemm_tcgen05.o build/seq_ops.o build/seq_moe.o: llark_b200/csrc/skinny.cuh
-
-build/attn_step.o build/attention.o build/seq_mixers.o: llark_b200/csrc/attn_step.cuh
 
 # the ALiBi instantiation #includes the attention source: rebuild it when that changes
 build/attention_tc_alibi.o: llark_b200/csrc/attention_tc.cu
