@@ -14,15 +14,20 @@ LIB_SERVE := llark_b200/libllark_serve.so
 # a shared link accepts what it cannot resolve, and the library then fails to load: make that an error of the build
 LDFLAGS := -shared -Xlinker --no-undefined
 
-# the entry points as Python functions (without Python's headers the package calls the library through ctypes)
-PYINC := $(shell python3 -c "import sysconfig; print(sysconfig.get_paths()['include'])" 2>/dev/null)
-CALLS := $(if $(wildcard $(PYINC)/Python.h),llark_b200/_calls.so)
+# the entry points as Python functions, for the interpreter PYTHON and under its name for extension modules, so that no other one takes them
+# (without Python's headers the package calls the library through ctypes)
+PYTHON ?= python3
+PY := $(shell $(PYTHON) -c "import sysconfig as s; print(s.get_paths()['include'], s.get_config_var('EXT_SUFFIX'))" 2>/dev/null)
+CALLS := $(if $(wildcard $(firstword $(PY))/Python.h),llark_b200/_calls$(lastword $(PY)))
 
 all: $(LIB) $(CALLS)
 serve: $(LIB_SERVE) $(CALLS)
 
-llark_b200/_calls.so: llark_b200/csrc/calls.cpp include/llark_b200.h
-	g++ -std=c++17 -O2 -shared -fPIC -I$(PYINC) -I$(dir $(NVCC))../include -o $@ $< -ldl
+ifneq ($(CALLS),)
+$(CALLS): llark_b200/csrc/calls.cpp include/llark_b200.h
+	@rm -f llark_b200/_calls.so
+	g++ -std=c++17 -O2 -shared -fPIC -I$(firstword $(PY)) -I$(dir $(shell command -v $(NVCC)))../include -o $@ $< -ldl
+endif
 
 # all headers are behind all objects: a list for each was found short of one
 build/%.o: llark_b200/csrc/%.cu $(wildcard llark_b200/csrc/*.cuh) include/llark_b200.h
@@ -39,5 +44,5 @@ $(LIB_SERVE): $(SERVE_OBJ)
 	$(NVCC) $(ARCH) $(LDFLAGS) -o $@ $(SERVE_OBJ)
 
 clean:
-	rm -rf build $(LIB) $(LIB_SERVE) llark_b200/_calls.so
+	rm -rf build $(LIB) $(LIB_SERVE) $(wildcard llark_b200/_calls*.so)
 .PHONY: all serve clean
