@@ -1,12 +1,14 @@
 // The library's entry points as Python functions. A ctypes call converts each of its 10 to 31 arguments through Python objects: 3 to 5 us
 // beside 2 to 3 of the launch itself, and a step of a small decoder makes a hundred and fifty of them. Here every argument is read by its C type, known
-// from the prototype. Arguments are taken as the ctypes signatures of _lib.py take them: None or an address for a pointer (or an object with
-// a buffer: a ctypes structure or array), integers cut to their type, any number for a float. The interpreter lock is given up meanwhile.
+// from the prototype. Arguments are taken as the ctypes signatures of _lib.py take them: None, an address, or a ctypes array, structure or
+// pointer for a pointer (nothing else that has a buffer: an array of the host must not reach a kernel), integers cut to their type, any number
+// for a float. The interpreter lock is given up meanwhile.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <cuda_runtime.h>
 #include <dlfcn.h>
 
+#include <initializer_list>
 #include <tuple>
 #include <utility>
 
@@ -38,6 +40,8 @@
 
 namespace {
 
+PyObject *kinds_in_place, *kinds_of_pointer;  // ctypes' arrays and structures; its pointers
+
 template <typename T> bool get(PyObject* o, T*& v) {
     if (o == Py_None) {
         v = nullptr;
@@ -48,13 +52,15 @@ template <typename T> bool get(PyObject* o, T*& v) {
         v = reinterpret_cast<T*>(x);
         return x != (unsigned long long)-1 || !PyErr_Occurred();
     }
+    const int array = PyObject_IsInstance(o, kinds_in_place), pointer = array ? 0 : PyObject_IsInstance(o, kinds_of_pointer);
+    if (array < 0 || pointer < 0) return false;
     Py_buffer b;
-    if (PyObject_GetBuffer(o, &b, PyBUF_SIMPLE)) {
+    if ((!array && !pointer) || PyObject_GetBuffer(o, &b, PyBUF_SIMPLE)) {
         PyErr_Clear();
         PyErr_Format(PyExc_TypeError, "an address, None or a ctypes object expected, not %s", Py_TYPE(o)->tp_name);
         return false;
     }
-    v = reinterpret_cast<T*>(b.buf);  // the caller holds the object
+    v = array ? reinterpret_cast<T*>(b.buf) : *static_cast<T**>(b.buf);  // the caller holds the object
     PyBuffer_Release(&b);
     return true;
 }
@@ -116,6 +122,18 @@ LLARK_CALLS(X)
 PyObject* bind(PyObject*, PyObject* path) {  // the entry points of the (loaded) library at `path`; returns the names that it has
     const char* p = PyUnicode_AsUTF8(path);
     if (!p) return nullptr;
+    if (!kinds_in_place) {
+        PyObject* m = PyImport_ImportModule("_ctypes");
+        PyObject* c = m ? PyImport_ImportModule("ctypes") : nullptr;
+        PyObject *array = nullptr, *structure = nullptr, *pointer = nullptr, *address = nullptr;
+        if (c && (array = PyObject_GetAttrString(m, "Array")) && (structure = PyObject_GetAttrString(m, "Structure")) &&
+            (pointer = PyObject_GetAttrString(m, "_Pointer")) && (address = PyObject_GetAttrString(c, "c_void_p"))) {
+            kinds_of_pointer = PyTuple_Pack(2, pointer, address);
+            if (kinds_of_pointer) kinds_in_place = PyTuple_Pack(2, array, structure);
+        }
+        for (PyObject* o : {m, c, array, structure, pointer, address}) Py_XDECREF(o);
+        if (!kinds_in_place) return nullptr;
+    }
     void* lib = dlopen(p, RTLD_NOW | RTLD_LOCAL);
     if (!lib) {
         PyErr_SetString(PyExc_OSError, dlerror());

@@ -41,3 +41,27 @@ def test_native_calls_take_what_ctypes_takes():
     for bad in ((1.5,) + (0,) * 15, (0, 1.5) + (0,) * 14, (0,) * 13 + ("x", 0, 0), (0,) * 15, (torch.zeros(1),) + (0,) * 15):
         with pytest.raises(TypeError):
             n.llark_linear_rows(*bad)
+
+
+def test_native_calls_take_no_host_array_for_a_pointer():
+    """What ctypes refuses for an address (an array of the host would reach a kernel as one) is refused; its own arrays and pointers are taken."""
+    import array
+    import ctypes
+
+    import numpy as np
+
+    from llark_b200 import _lib
+
+    if not os.path.exists(_lib.LIB_PATH):
+        pytest.skip("the library has not been built")
+    native = pytest.importorskip("llark_b200._calls")
+    _lib.calls()
+    host = np.array([1, 3, 9], dtype=np.int32)
+    own = (ctypes.c_int * 3)(1, 3, 9)
+    for bad in (host, host[0], host.tobytes(), bytearray(12), memoryview(own), array.array("i", [1, 3, 9]), "1", ctypes.c_int(1), ctypes.byref(own), object()):
+        with pytest.raises(TypeError):
+            native.llark_jb_resblocks_length(bad, 3)
+    want = _lib.lib().llark_jb_resblocks_length(own, 3)
+    assert want == 3
+    for good in (own, host.ctypes.data, ctypes.cast(own, ctypes.c_void_p), ctypes.cast(own, ctypes.POINTER(ctypes.c_int))):
+        assert native.llark_jb_resblocks_length(good, 3) == want
