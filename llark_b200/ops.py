@@ -886,22 +886,31 @@ def scan_passes(cu_host, most):
     return out
 
 
+def _kept(st, key, make):
+    """What make() writes once for the layers of a step, with the step and for this stream: another stream's writing need not have ended. Not in a
+    capture: what that writes exists only in its replays."""
+    tables = getattr(st, "tables", None)
+    if tables is None or torch.cuda.is_current_stream_capturing():
+        return make()
+    key = key + (_stream(),)
+    if key not in tables:
+        tables[key] = make()
+    return tables[key]
+
+
 def _scan_tables(st, most):
     """[(lists, requests, blocks)] of each pass: int32 [4 requests + 2 blocks] as llark_seq_glr_chunks takes them, written by the device: no
-    copy, and nothing that a stream capture does not take. The layers of a step share them, but what a capture writes exists only in
-    its replays."""
-    tables = None if torch.cuda.is_current_stream_capturing() else getattr(st, "tables", None)
-    if tables is not None and ("scan", most) in tables:
-        return tables["scan", most]
-    out = []
-    for done, each, n, m in scan_passes(st.cu_host, most):
-        t = torch.empty(4 * n + 2 * m, device=st.device, dtype=torch.int32)
-        at = t.data_ptr()
-        check(lib().llark_seq_chunk_plan(_p(st.cu), st.n_seq, done, each, at, at + 16 * n, _stream()), "seq_chunk_plan")
-        out.append((t, n, m))
-    if tables is not None:
-        tables["scan", most] = out
-    return out
+    copy, and nothing that a stream capture does not take. The layers of a step share them."""
+    def make():
+        out = []
+        for done, each, n, m in scan_passes(st.cu_host, most):
+            t = torch.empty(4 * n + 2 * m, device=st.device, dtype=torch.int32)
+            at = t.data_ptr()
+            check(lib().llark_seq_chunk_plan(_p(st.cu), st.n_seq, done, each, at, at + 16 * n, _stream()), "seq_chunk_plan")
+            out.append((t, n, m))
+        return out
+
+    return _kept(st, ("scan", most), make)
 
 
 # What the walk costs more than the token-by-token scan before the first token, per head and block beyond the first of a request, and
@@ -1008,19 +1017,16 @@ def decay_powers(decay, device):
 
 def seq_rotary_table(freq, st):
     """(cos, sin) of position * frequency for every row of the step, fp32 [n_tok, n_freq, 2]; kept with the step for the other
-    layers (and heads, and passes) on this stream that rotate by the same tensor of frequencies."""
+    layers (and heads, and passes) on this stream that rotate by the same frequencies."""
     _req(freq, torch.float32)
-    key = freq.data_ptr(), _stream()
-    if key not in st.tables:
-        st.tables[key] = _rotary_table(freq, st)
-    return st.tables[key]
 
+    def make():
+        cs = torch.empty((st.n_tok, freq.numel(), 2), device=freq.device, dtype=torch.float32)
+        check(lib().llark_seq_rotary_table(_p(freq), freq.numel(), _p(st.tok_seq), _p(st.cu), _p(st.pos0), _p(cs), st.n_tok, _stream()),
+              "seq_rotary_table")
+        return freq, cs  # the frequencies too: their address is not another tensor's while the table is kept
 
-def _rotary_table(freq, st):
-    cs = torch.empty((st.n_tok, freq.numel(), 2), device=freq.device, dtype=torch.float32)
-    check(lib().llark_seq_rotary_table(_p(freq), freq.numel(), _p(st.tok_seq), _p(st.cu), _p(st.pos0), _p(cs), st.n_tok, _stream()),
-          "seq_rotary_table")
-    return cs
+    return _kept(st, ("rotary", freq.data_ptr(), freq.numel()), make)[1]
 
 
 def linear_qkv_rotary_takes(a, w, H, G, D, E, n_rot):
@@ -1033,17 +1039,14 @@ def linear_qkv_rotary_takes(a, w, H, G, D, E, n_rot):
 
 
 def linear_qkv_rotary(a, w, st, H, G, D, E, bias=None, freq=None):
-    """seq_qkv_rotary(linear(a, w, bias, out_dtype=float32), ..) of interleaved pairs without norms: q, k and v in bf16, from one launch. The
-    step's table of angles is kept with it, except in a capture: what that writes exists only in its replays."""
+    """seq_qkv_rotary(linear(a, w, bias, out_dtype=float32), ..) of interleaved pairs without norms: q, k and v in bf16, from one launch."""
     _req(a, BF16), _req(w, BF16)
     if bias is not None:
         _req(bias, torch.float32)
     if not _INITED:
         init()
     n = a.shape[0]
-    cs = None
-    if freq is not None:
-        cs = _rotary_table(freq, st) if torch.cuda.is_current_stream_capturing() else seq_rotary_table(freq, st)
+    cs = seq_rotary_table(freq, st) if freq is not None else None
     q, k, v = (torch.empty((n, c), device=a.device, dtype=BF16) for c in (H * D, G * D, G * E))
     LINEAR_STATS["tcgen05"] += 1
     check(lib().llark_linear_qkv_rotary(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), _p(bias), _p(cs), 2 * freq.numel() if cs is not None else 0,
@@ -1062,7 +1065,8 @@ def seq_decay_scan(src, q_off, k_off, v_off, powers, state, st, H, D, E, freq=No
     L = lib()
     o = torch.empty((st.n_tok, H * E), device=src.device, dtype=torch.float32)
     n_rot = 2 * freq.numel() if freq is not None else 0
-    cs = _p(seq_rotary_table(freq, st)) if n_rot else None
+    angles = seq_rotary_table(freq, st) if n_rot else None
+    cs = _p(angles)
     inter, ks, silu, pw, pl = int(interleaved), float(k_scale), int(silu), _p(powers), powers.shape[1]
     S = _p(state)
     if full_fp32 or st.max_len < DECAY_CHUNK_MIN_LEN or D > 128:

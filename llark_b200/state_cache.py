@@ -74,9 +74,14 @@ class _Chunks:
 def _step_chunks(self, length):
     """The step cut into work items of at most `length` consecutive rows of one request (for scans that run long
     prompts as independent chunks): row0 / n per item, index = 0 .. n_items-1, minus1 = -1 everywhere, last_slot = the
-    request's slot on its last item and -1 elsewhere, inner = index except -1 on a request's last item, seq_item0[b] = first item of request b. Built once per step."""
-    if length in self._chunks:
-        return self._chunks[length]
+    request's slot on its last item and -1 elsewhere, inner = index except -1 on a request's last item, seq_item0[b] = first item of request b. Built once per step
+    and stream; in a capture, whose copies exist only in its replays, each time."""
+    on_gpu = torch.device(self.device).type == "cuda"
+    key = length, torch.cuda.current_stream(self.device).cuda_stream if on_gpu else 0
+    if on_gpu and torch.cuda.is_current_stream_capturing():
+        key = length, "capture", len(self._chunks)  # not looked up again, but kept: the replays copy from its host buffer
+    if key in self._chunks:
+        return self._chunks[key]
     row0, n, last, inner, seq0 = [], [], [], [], [0]
     for b, ln in enumerate(self.lens):
         for lo in range(0, ln, length):
@@ -87,7 +92,7 @@ def _step_chunks(self, length):
         seq0.append(len(row0))
     k = len(row0)
     host = torch.tensor(row0 + n + list(range(k)) + [-1] * k + last + inner + seq0, dtype=torch.int32)
-    if torch.device(self.device).type == "cuda":
+    if on_gpu:
         host = host.pin_memory()
     dev = host.to(self.device, non_blocking=True)
     c = _Chunks()
@@ -95,7 +100,7 @@ def _step_chunks(self, length):
     c.n_items = k
     c.row0, c.n, c.index, c.minus1, c.last_slot, c.inner = (dev[i * k:(i + 1) * k] for i in range(6))
     c.seq_item0 = dev[6 * k:]
-    self._chunks[length] = c
+    self._chunks[key] = c
     return c
 
 

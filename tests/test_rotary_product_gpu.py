@@ -67,3 +67,57 @@ def test_a_stream_makes_its_own_table_of_angles():
     here = ops.seq_rotary_table(freq, st)
     torch.cuda.synchronize()
     assert here is not there and here is ops.seq_rotary_table(freq, st) and torch.equal(here, there)
+
+
+def test_a_stream_makes_its_own_lists_of_a_step():
+    """The lists of the block walk and of the scans' chunks, as the tables above: a stream does not read what another one may still be writing."""
+    from llark_b200 import ops
+    from llark_b200.state_cache import StepLayout
+
+    st = StepLayout([3, 170], [0, 5], [0, 1], torch.device("cuda"))
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    for make in (lambda: ops._scan_tables(st, 8), lambda: st.chunks(64)):
+        with torch.cuda.stream(side):
+            there = make()
+        here = make()
+        torch.cuda.synchronize()
+        assert here is not there and here is make()
+        values = lambda c: [t for t, _, _ in c] if isinstance(c, list) else [c.row0, c.n, c.index, c.minus1, c.last_slot, c.inner, c.seq_item0]  # noqa: E731
+        assert all(torch.equal(a, b) for a, b in zip(values(here), values(there), strict=True))
+
+
+def test_tables_of_a_step_are_those_of_their_frequencies():
+    from llark_b200 import ops
+    from llark_b200.state_cache import StepLayout
+
+    st, freq = StepLayout([3, 70], [0, 5], [0, 1], torch.device("cuda")), torch.rand(32, device="cuda")
+    wide, narrow = ops.seq_rotary_table(freq, st), ops.seq_rotary_table(freq[:16], st)  # the same address
+    assert narrow.shape == (73, 16, 2) and torch.equal(narrow, wide[:, :16])
+
+
+def test_what_a_capture_writes_is_not_kept_for_later_calls():
+    from llark_b200 import ops
+    from llark_b200.state_cache import StepLayout
+
+    n, H, D, E = 73, 2, 64, 64
+    g = torch.Generator(device="cuda").manual_seed(3)
+    src = torch.randn(n, H * (2 * D + E), device="cuda", generator=g)
+    freq, powers = torch.rand(32, device="cuda", generator=g), ops.decay_powers([0.9, 0.99], torch.device("cuda"))
+
+    def scan(st):
+        return ops.seq_decay_scan(src, 0, H * D, 2 * H * D, powers, torch.zeros(2, H, D, E, device="cuda"), st, H, D, E, freq=freq)
+
+    layout = lambda: StepLayout([3, 70], [0, 5], [0, 1], torch.device("cuda"))  # noqa: E731
+    want, st = scan(layout()), layout()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        got = scan(st)
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):  # the stream of the capture, which has not been replayed
+        assert torch.equal(scan(st), want)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
