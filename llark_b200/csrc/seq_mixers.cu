@@ -942,8 +942,8 @@ __global__ void head_rmsnorm_kernel(const float* __restrict__ x, const float* __
 // under 2.6), one request 7.0 -> 3.1, 64 requests 46.5 -> 25.1; D = 64, 8 requests 7.7 -> 4.4.
 template <typename T, int D>
 __global__ void __launch_bounds__(256)
-glr_step_kernel(const float* __restrict__ src, long long ld, int q_off, int f_off, int v_off, const float* __restrict__ lower,
-                float* __restrict__ state, const float* __restrict__ norm, T* __restrict__ out, const int* __restrict__ slot, int H, float eps) {
+glr_step_kernel(const float* src, long long ld, int q_off, int f_off, int v_off, const float* lower, float* __restrict__ state,
+                const float* norm, T* __restrict__ out, const int* slot, int H, float eps) {
     constexpr int E = 128, R = D / 8;  // rows of a warp
     __shared__ float sq[D], sf[D], part[8][E], red[4];
     const int h = blockIdx.x, b = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

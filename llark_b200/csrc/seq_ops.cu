@@ -298,9 +298,8 @@ __global__ void add_rmsnorm4_kernel(const float* __restrict__ x, const float* __
 // on): add_rmsnorm4_kernel and short_conv4_kernel in one launch, the same numbers. Latency bounds it. 4 taps of 2048 channels: 1 row 6.7 us ->
 // 4.8, 8 rows 7.0 -> 5.0, 64 rows 7.3 -> 5.6.
 template <typename T>
-__global__ void add_rmsnorm_conv4_kernel(const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ w,
-                                         float* __restrict__ x_out, const float* __restrict__ taps_w, float* __restrict__ tail,
-                                         const int* __restrict__ slot, T* __restrict__ out, int C, int taps, float eps) {
+__global__ void add_rmsnorm_conv4_kernel(const float* x, const float* y, const float* w, float* __restrict__ x_out, const float* taps_w,
+                                         float* __restrict__ tail, const int* slot, T* __restrict__ out, int C, int taps, float eps) {
     __shared__ float red[32];
     let_next_begin();
     wait_for_previous();

@@ -1,4 +1,4 @@
-"""What the Makefile and build.py rebuild after an edit."""
+"""What the Makefile and build.py rebuild after an edit, and what holds for all kernels of a kind."""
 import os
 import re
 import shutil
@@ -77,3 +77,16 @@ def test_a_tree_with_a_library_gets_its_native_functions(tmp_path, monkeypatch, 
     assert f"PYTHON={sys.executable}" in calls[0] and calls[0][-1] == os.path.relpath(build.calls_path(), str(tmp_path))
     assert os.path.basename(build.calls_path()) == "_calls" + build.sysconfig.get_config_var("EXT_SUFFIX")
     assert ("through ctypes" in capsys.readouterr().err) != made
+
+
+def test_kernels_launched_early_read_no_input_as_read_only():
+    """A kernel that lives beside the one before it may not use the loads for memory that nobody writes meanwhile."""
+    found = set()
+    for name in (n for n in os.listdir(CSRC) if n.endswith(".cu")):
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
+        for head, kernel, params, body in re.findall(r"__global__([^;{]*?)\b(\w+_kernel)\(([^{;]*)\)\s*\{(.*?)\n\}", text, re.S):
+            if "wait_for_previous()" in body:
+                found.add(kernel)
+                assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", params), kernel
+                assert not re.search(r"__ldg|ld_ahead|ld\.global\.nc", body), kernel
+    assert found == {"rmsnorm_fwd_kernel", "add_rmsnorm_conv4_kernel", "glr_step_kernel", "skinny_kernel", "skinny_tc_kernel"}

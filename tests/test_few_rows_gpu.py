@@ -203,3 +203,46 @@ def test_chains_over_k_are_short(M, N, K):
     x, w = torch.randn(M, K, device="cuda").to(BF16), (torch.randn(N, K, device="cuda") * K ** -0.5).to(BF16)
     chain = 320 if K == 2560 else 256
     assert _rel(ops.linear(x, w, out_dtype=F32), x.to(F64) @ w.to(F64).t()) < 1.5 * chain / 16 / 4 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("n", [1, 8, 40])
+def test_one_token_kernels_that_begin_early_see_what_was_written_before(n):
+    """The recurrence's step and the norm with the next convolution between products, each input written by the launch in front and each buffer
+    written again while the launch in front may still read it: against the same launches one at a time."""
+    from llark_b200 import ops
+    from llark_b200.state_cache import StepLayout
+
+    torch.manual_seed(n)
+    H, D, E, C, taps = 4, 128, 128, 512, 4
+    wide = [(torch.randn(3 * C, C, device="cuda") * C ** -0.5).to(BF16) for _ in range(2)]
+    square = [(torch.randn(C, C, device="cuda") * C ** -0.5).to(BF16) for _ in range(2)]
+    norm, row_norm, cw = torch.rand(E, device="cuda"), torch.rand(C, device="cuda"), torch.randn(C, taps, device="cuda") / 2
+    s0, t0, x0 = torch.randn(n, H, D, E, device="cuda"), torch.randn(n, taps - 1, C, device="cuda"), torch.randn(n, C, device="cuda")
+    src, y = torch.empty(n, 3 * C, device="cuda"), torch.empty(n, C, device="cuda")
+    w, low = norm.clone(), torch.empty(H * D, device="cuda")
+
+    def walk(wait):
+        state, tail, x = s0.clone(), t0.clone(), x0.clone()
+        st = StepLayout([1] * n, [0] * n, list(range(n))[::-1], torch.device("cuda"))
+        wait()
+        h = x.to(BF16)
+        wait()
+        for step in range(12):
+            ops.linear(h, wide[step % 2], out=src)
+            wait()
+            low.fill_(0.1 * (step % 3))
+            wait()
+            w.copy_(norm if step % 2 else 2 * norm)  # what the step right behind reads
+            wait()
+            o = ops.seq_glr_step(src, 0, H * D, 2 * H * D, low, state, st, H, D, E, w, 1e-5, BF16)
+            wait()
+            ops.linear(o, square[step % 2], out=y)
+            wait()
+            x, h = ops.seq_add_rmsnorm_conv(x, y, row_norm, 1e-5, cw, tail, st, BF16)
+            wait()
+        return x, h, state, tail
+
+    want = walk(torch.cuda.synchronize)
+    assert all(v.float().isfinite().all() for v in want)
+    for _ in range(20):
+        assert all(torch.equal(a, b) for a, b in zip(walk(lambda: None), want))
