@@ -171,7 +171,7 @@ __device__ __forceinline__ void epilogue(const Args& p, const float* red, int M,
                 y[e] = bf16_round(y[e]);
             }
             if (col < p.rope_cols) {  // the same for all four: whole heads are rotated
-                const long long at = (long long)(m % p.rope_S) * 128 + (col & 127);
+                const long long at = (long long)((p.first + m) % p.rope_S) * 128 + (col & 127);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const float c1 = __bfloat162float(p.rope_cos[at + e]), s1 = __bfloat162float(p.rope_sin[at + e]);
@@ -673,6 +673,20 @@ static Cut cut_of(const Args& a) {
     return cut;
 }
 
+static cudaError_t by_eights(const Args& a, cudaStream_t st) {
+    const int size = a.c_fp32 ? 4 : 2;
+    for (int m = 0; m < a.M; m += 8) {
+        Args b = a;
+        b.M = a.M - m < 8 ? a.M - m : 8;
+        b.first = a.first + m;
+        b.A += m * a.lda;
+        b.C = static_cast<char*>(a.C) + m * a.ldc * size;
+        if (a.R) b.R = static_cast<const char*>(a.R) + m * a.ldr * size;
+        const cudaError_t e = launch(b, st);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
 cudaError_t launch(const Args& a, cudaStream_t st) {
     const bool grouped = a.tiles != nullptr, two = paired(a);
     const int nch = (a.K + BK - 1) / BK, all = units_of(a);
@@ -686,6 +700,8 @@ cudaError_t launch(const Args& a, cudaStream_t st) {
         while (cs < 8 && tiles * cs * 2 <= 592 && nch / (cs * 2) >= 4) cs *= 2;
         return a.c_fp32 ? go_mma<float>(a, cs, tiles, st) : go_mma<bf16_t>(a, cs, tiles, st);
     }
+    // Rows closer to each other than K (one token's row for all tokens, windows of a sequence) are none that a tensor map is specified for
+    if (!grouped && (a.ldw < a.K || (a.lda < a.K && a.M > 32))) return by_eights(a, st);
     const Cut cut = cut_of(a);
 #define LLARK_SKINNY(N_, GR_, CH_) (a.c_fp32 ? go_tc<N_, float, GR_, CH_>(a, cut, st) : go_tc<N_, bf16_t, GR_, CH_>(a, cut, st))
     if (grouped) return LLARK_SKINNY(64, true, 1);

@@ -23,9 +23,9 @@ struct Args {
     int M, N, K;       // N: rows of W (kActSiluGlu, kActSwiglu: gate rows, then as many up rows: N counts both)
     int act;
     float limit, slope;
-    // kActRope: columns below rope_cols are rotated per 128-wide head, position = row % rope_S
+    // kActRope: columns below rope_cols are rotated per 128-wide head, position = (first + row) % rope_S
     const __nv_bfloat16 *rope_cos, *rope_sin;
-    int rope_S, rope_cols;
+    int rope_S, rope_cols, first;
     // Routed experts: tile list of (expert, first sorted row, rows <= 64), its length in meta[0] (at most max_tiles); rows of A
     // are perm[sorted row] / top (NULL: the sorted row itself), W holds one [N, K] block per expert, sums are multiplied by
     // in_wts[perm[sorted row]] when given. M is not used.

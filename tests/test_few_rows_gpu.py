@@ -246,3 +246,21 @@ def test_one_token_kernels_that_begin_early_see_what_was_written_before(n):
     assert all(v.float().isfinite().all() for v in want)
     for _ in range(20):
         assert all(torch.equal(a, b) for a, b in zip(walk(lambda: None), want))
+
+
+@pytest.mark.parametrize("M", [9, 33, 64])
+def test_rows_that_lie_in_each_other(M):
+    """One row for all tokens, and rows that begin 8 entries after each other, as tokens and as weights: the same as of copies of them."""
+    from llark_b200 import ops
+
+    torch.manual_seed(M)
+    K = N = 512
+    long, w, r = torch.randn(K + 8 * N, device="cuda").to(BF16), (torch.randn(N, K, device="cuda") * K ** -0.5).to(BF16), torch.randn(M, N, device="cuda").to(BF16)
+    cos, sin = (torch.rand(5, 128, device="cuda").to(BF16) for _ in range(2))
+    for x, v in ((long[:K].expand(M, K), w), (long.as_strided((M, K), (8, 1)), w), (w[:M], (long * K ** -0.5).as_strided((N, K), (8, 1)))):
+        z = x.to(F64) @ v.to(F64).t()
+        assert _rel(ops.gemm(x, v, out_dtype=F32), z) < 5e-6  # fp32 sums in any order, as above
+        assert _rel(ops.gemm(x, v, residual=r), z + r.to(F64)) < 2.0 ** -8  # one rounding of the result
+        want = ops.gemm(x.contiguous(), v.contiguous(), rope=(cos, sin, 5, 256))
+        # the same sums but for their order, which moves a rounding to bf16 here and there: sums, products and result are rounded
+        assert _rel(ops.gemm(x, v, rope=(cos, sin, 5, 256)), want.to(F64)) < 2.0 ** -8
