@@ -12,9 +12,9 @@
 //          0.002096 at 204 us instead of 224)
 //
 // What bounds it: the exponentials (16 per SM and clock) and the softmax around them; V and K are read from L2 by every head of a group.
-// Measured on a B200, 4 prompts of 2048 tokens, 32 heads over 8, window 1024: 182 us (565 TFLOP/s of visible pairs; 224 at first), seq_swa_mma.cu 722;
-// window 128: 99 against 253; 32 portions of 96 tokens behind 2000: 257 against 498. With the products issued by the warp together (see
-// warp_umma_f16), two numbers per instruction and a mask word for 32 keys, 4 prompts of 2048 to 1173 tokens: 184 -> 150.
+// Measured on a B200, 32 heads over 8, us: 4 prompts of 2048 tokens, window 1024, 184 (559 TFLOP/s of visible pairs; 224 at first; seq_swa_mma.cu 722), window
+// 128 90 (253); 32 portions of 96 tokens behind 2000 236 (498); 4 prompts of 2048, 1757, 1465 and 1173 tokens, window 1024, 148, which took 184 before the
+// products were issued by the warp together (see warp_umma_f16) and the softmax took two numbers per instruction and a mask word for 32 keys.
 #include "common.cuh"
 
 namespace llark {

@@ -11,7 +11,8 @@
 // 202 us of products for 163 us of bytes in a step of two layers and the head, one row, and 268 us for the whole step. So a CTA starts
 // while the kernel in front of it ends (launch_early): its weights are under way, or on their way to L2, before the tokens are there.
 // The next kernel is let in at once: after half of the slices or with the last ones asked for the step took 2 to 3 us longer.
-// Measured, a step of 1 / 8 / 32 rows: 269 -> 236, 297 -> 270, 560 -> 525 us (504 with the weights of 32 rows through TMA).
+// Measured, a step of 1 / 8 / 32 rows behind 1024 / 1024 / 1500 positions: 269 -> 236, 306 -> 280, 547 -> 485 us (the last with weights through TMA; 510
+// without).
 //
 // Measured on a B200, launches in a row on rotating weights (floor = the weights at 6.55 TB/s), against the 256-row tiles of the
 // tcgen05 GEMM core: N 4096 K 4096, 32 tokens 11.1 us (core 28.7, floor 5.1); N 22016 K 4096 33.0 (54.9, 27.5); N 4096 K 11008
